@@ -99,7 +99,7 @@ def draw(rng):
         case["cells"] = ",".join(str(s) for s in sides)
         case["drop"] = rng.randrange(0, max(1, sides[0] * sides[1] * sides[2] // 4) + 1)
     if arch == "medium" and rng.random() < 0.25:
-        case["channels"] = rng.choice((32, 64))
+        case["channels"] = 64
     case["options"] = rng.choice(("", "", "", "zbl", "agnesi", "scaled", "pairs", "agnesi,zbl,scaled"))
     if case["cells"].isdigit():
         case["options"] = rng.choice(("", "zbl"))       # tables of a hundred species pairs take long to make
