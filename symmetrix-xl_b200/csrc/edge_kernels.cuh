@@ -17,12 +17,43 @@
 // mace_kokkos_evaluate.cpp:92-106 and 157-186.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "generated/structures.h"
 
 namespace sxb {
 
 constexpr int kEdgeChunk = 64;
+
+// A receiver's edges can be dealt to several blocks (layer 1) or warps (layer 0): part p of n walks [x, y) of the
+// receiver's CSR range.  A receiver is a serial chain of about 75 edges at 0.5 to 1 us each, so with fewer receivers than
+// the chip holds blocks the whole kernel lasts as long as one chain; the host picks the number of parts (edge_parts and
+// cluster_parts in evaluator.cu).  Gradient parts are independent.  Forward parts are one thread-block cluster that adds
+// its sums up over distributed shared memory, in part order, so that the result has one order.
+__device__ __forceinline__ int2 edge_part(const int* __restrict__ first, int i, int part, int parts)
+{
+    const int begin = first[i], n = first[i + 1] - begin;
+    return make_int2(begin + static_cast<int>(static_cast<long>(n) * part / parts),
+                     begin + static_cast<int>(static_cast<long>(n) * (part + 1) / parts));
+}
+
+// Adds up `count` rows of `width` floats over the blocks of a cluster and hands every sum once to store(row, value);
+// `mine` is this block's copy in dynamic shared memory, written by its threads before the call.
+template <typename Store>
+__device__ __forceinline__ void cluster_sum_rows(float* mine, int count, int width, Store&& store)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int parts = static_cast<int>(cluster.num_blocks()), part = static_cast<int>(cluster.block_rank());
+    cluster.sync();
+    for (int q = part; q < count; q += parts) {
+        float sum = 0.0f;
+        for (int r = 0; r < parts; ++r) sum += cluster.map_shared_rank(mine, r)[q * width + threadIdx.x];
+        store(q, sum);
+    }
+    cluster.sync();   // no block leaves while another still reads its rows
+}
 
 // ---------------------------------------------------------------------------------------------
 // Real spherical harmonics up to l = 3 of a unit direction, model convention: the vector is
@@ -721,7 +752,9 @@ l0_reverse_kernel(int num_nodes, int node0, int C_runtime, const int* __restrict
 
 #define SXB_DEFINE_L1_KERNELS(NAME)                                                                                  \
     /* kGivenHarmonics: the caller passes Y_lm per edge [E][16] (the kernel-plugin interface) */                     \
-    template <int kC, bool kGivenHarmonics = false>                                                                  \
+    /* kParts: the parts of a receiver (blockIdx.y) are one cluster; a build of its own, because the code of the */  \
+    /* exchange costs the plain build a tenth of its speed */                                                        \
+    template <int kC, bool kGivenHarmonics = false, bool kParts = false>                                             \
     __global__ void __launch_bounds__(kC > 0 ? kC : 256)                                                             \
     l1_forward_kernel_##NAME(int num_nodes, int node0, int C_runtime, const int* __restrict__ first,                            \
                              const int* __restrict__ sources, const EdgeGeom* __restrict__ geom,                     \
@@ -738,7 +771,8 @@ l0_reverse_kernel(int num_nodes, int node0, int C_runtime, const int* __restrict
         const int local = blockIdx.x, i = node0 + local;                                                             \
         const int k = threadIdx.x;                                                                                   \
         const int F = NP * C;                                                                                        \
-        const int begin = first[i], end = first[i + 1];                                                              \
+        const int2 range = kParts ? edge_part(first, i, blockIdx.y, gridDim.y) : make_int2(first[i], first[i + 1]);  \
+        const int begin = range.x, end = range.y;                                                                    \
         float acc[NR];                                                                                               \
         _Pragma("unroll") for (int r_ = 0; r_ < NR; ++r_) acc[r_] = 0.0f;                                            \
         for (int chunk = begin; chunk < end; chunk += kEdgeChunk) {                                                  \
@@ -771,7 +805,13 @@ l0_reverse_kernel(int num_nodes, int node0, int C_runtime, const int* __restrict
         /* density scaling of A1 = Phi1 W (mace.cpp:2381-2403) commutes with the linear: scale Phi1 */              \
         const float scale = inv_scale != nullptr ? inv_scale[i] : 1.0f;                                              \
         float* out = Phi1 + static_cast<size_t>(local) * NE * C + k;                                                 \
-        _Pragma("unroll") for (int q = 0; q < NE; ++q) out[q * C] = out_lme[q] * scale;                              \
+        if constexpr (!kParts) {                                                                                     \
+            _Pragma("unroll") for (int q = 0; q < NE; ++q) out[q * C] = out_lme[q] * scale;                          \
+        } else {                                                                                                     \
+            extern __shared__ float part_rows[];                                                                     \
+            _Pragma("unroll") for (int q = 0; q < NE; ++q) part_rows[q * C + k] = out_lme[q];                        \
+            cluster_sum_rows(part_rows, NE, C, [&](int q, float sum) { out[q * C] = sum * scale; });                 \
+        }                                                                                                            \
     }                                                                                                                \
                                                                                                                      \
     /* kMinBlocks caps the registers of the 128-channel build: 3 blocks per SM = at most 170 registers */           \
@@ -794,7 +834,8 @@ l0_reverse_kernel(int num_nodes, int node0, int C_runtime, const int* __restrict
         const int k = threadIdx.x;                                                                                   \
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, num_warps = blockDim.x >> 5;                     \
         const int F = NP * C;                                                                                        \
-        const int begin = first[i], end = first[i + 1];                                                              \
+        const int2 range = edge_part(first, i, blockIdx.y, gridDim.y);                                               \
+        const int begin = range.x, end = range.y;                                                                    \
         if (threadIdx.x < 3) fs.receiver[threadIdx.x] = 0.0;                                                         \
         if (threadIdx.x < 9) fs.virial[threadIdx.x] = 0.0;                                                           \
         /* with density scaling dPhi1 holds the adjoint of the scaled Phi1: divide by 1 + rho_i once more */       \

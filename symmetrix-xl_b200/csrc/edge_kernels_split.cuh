@@ -15,7 +15,7 @@
 namespace sxb {
 
 #define SXB_DEFINE_L1_SPLIT_KERNELS(NAME, G)                                                                         \
-    template <int kC>                                                                                                \
+    template <int kC, bool kParts = false>                                                                           \
     __global__ void __launch_bounds__(kC)                                                                            \
     l1_forward_split_kernel_##NAME##_##G(int num_nodes, int node0, const int* __restrict__ first,                    \
                                          const int* __restrict__ sources, const EdgeGeom* __restrict__ geom,         \
@@ -34,7 +34,8 @@ namespace sxb {
         __shared__ ChunkState<false> s;                                                                              \
         const int local = blockIdx.x, i = node0 + local;                                                             \
         const int k = threadIdx.x;                                                                                   \
-        const int begin = first[i], end = first[i + 1];                                                              \
+        const int2 range = kParts ? edge_part(first, i, blockIdx.y, gridDim.y) : make_int2(first[i], first[i + 1]);  \
+        const int begin = range.x, end = range.y;                                                                    \
         float acc[NRG];                                                                                              \
         _Pragma("unroll") for (int r_ = 0; r_ < NRG; ++r_) acc[r_] = 0.0f;                                           \
         for (int chunk = begin; chunk < end; chunk += kEdgeChunk) {                                                  \
@@ -66,7 +67,13 @@ namespace sxb {
         SXB_##NAME##_##G##_TERMS(SXB_TERM_FORWARD)                                                                   \
         const float scale = inv_scale != nullptr ? inv_scale[i] : 1.0f;                                              \
         float* out = Phi1 + static_cast<size_t>(local) * NE * C + k;                                                 \
-        _Pragma("unroll") for (int q = 0; q < NEG; ++q) out[lme_of[q] * C] = out_lme[q] * scale;                     \
+        if constexpr (!kParts) {                                                                                     \
+            _Pragma("unroll") for (int q = 0; q < NEG; ++q) out[lme_of[q] * C] = out_lme[q] * scale;                          \
+        } else {                                                                                                     \
+            extern __shared__ float part_rows[];                                                                     \
+            _Pragma("unroll") for (int q = 0; q < NEG; ++q) part_rows[q * C + k] = out_lme[q];                        \
+            cluster_sum_rows(part_rows, NEG, C, [&](int q, float sum) { out[lme_of[q] * C] = sum * scale; });                 \
+        }                                                                                                            \
     }                                                                                                                \
                                                                                                                      \
     template <int kC>                                                                                                \
@@ -92,7 +99,8 @@ namespace sxb {
         const int local = blockIdx.x, i = node0 + local;                                                             \
         const int k = threadIdx.x;                                                                                   \
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;                                                  \
-        const int begin = first[i], end = first[i + 1];                                                              \
+        const int2 range = edge_part(first, i, blockIdx.y, gridDim.y);                                               \
+        const int begin = range.x, end = range.y;                                                                    \
         if (threadIdx.x < 3) fs.receiver[threadIdx.x] = 0.0;                                                         \
         if (threadIdx.x < 9) fs.virial[threadIdx.x] = 0.0;                                                           \
         const float scale = density.table != nullptr ? density.inv_scale[i] : 1.0f;                                  \

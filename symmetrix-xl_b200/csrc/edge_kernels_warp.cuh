@@ -95,7 +95,7 @@ struct VecLoad<4> {
 // ---------------------------------------------------------------------------------------------
 template <int kVec>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
-l0_forward_warp_kernel(int num_nodes, int node0, const int* __restrict__ first, const int* __restrict__ sources,
+l0_forward_warp_kernel(int num_nodes, int node0, int parts, const int* __restrict__ first, const int* __restrict__ sources,
                        const EdgeGeom* __restrict__ geom, const unsigned char* __restrict__ atype, int num_active,
                        SplineGrid grid, const float* __restrict__ table, float* __restrict__ A0,
                        const float* __restrict__ inv_scale)
@@ -103,13 +103,16 @@ l0_forward_warp_kernel(int num_nodes, int node0, const int* __restrict__ first, 
     constexpr int C = 32 * kVec, F = 4 * C;
     __shared__ WarpChunk<false> chunks[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int local = blockIdx.x * kWarpsPerBlock + warp;   // receiver inside the tile
-    if (local >= num_nodes) return;
+    // parts = 1: a warp per receiver; parts = kWarpsPerBlock: the block's warps share one receiver
+    const int slot = blockIdx.x * kWarpsPerBlock + warp;
+    const int local = slot / parts, part = slot % parts;    // receiver inside the tile
+    if (local >= num_nodes) return;                         // whole blocks when parts > 1
     const int i = node0 + local;                            // graph-wide receiver index
     WarpChunk<false>& s = chunks[warp];
     const int k = lane * kVec;
     const int type_i = atype[i];
-    const int begin = first[i], end = first[i + 1];
+    const int2 range = edge_part(first, i, part, parts);
+    const int begin = range.x, end = range.y;
     float acc[16][kVec];
 #pragma unroll
     for (int lm = 0; lm < 16; ++lm)
@@ -143,6 +146,29 @@ l0_forward_warp_kernel(int num_nodes, int node0, const int* __restrict__ first, 
             }
         }
     }
+    if (parts > 1) {
+        // every warp leaves its sums in shared memory; the warps of the receiver then add up a share of the rows each, in
+        // part order
+        extern __shared__ float part_rows[];                // [kWarpsPerBlock][16][C]
+#pragma unroll
+        for (int lm = 0; lm < 16; ++lm) VecLoad<kVec>::store(part_rows + (warp * 16 + lm) * C + k, acc[lm]);
+        __syncthreads();
+        const float scale = inv_scale != nullptr ? inv_scale[i] : 1.0f;
+        const float* rows = part_rows + (warp - part) * 16 * C + k;
+        for (int lm = part; lm < 16; lm += parts) {
+            float sum[kVec], v[kVec];
+            VecLoad<kVec>::load(rows + lm * C, sum);
+            for (int r = 1; r < parts; ++r) {
+                VecLoad<kVec>::load(rows + (r * 16 + lm) * C, v);
+#pragma unroll
+                for (int q = 0; q < kVec; ++q) sum[q] += v[q];
+            }
+#pragma unroll
+            for (int q = 0; q < kVec; ++q) sum[q] *= scale;
+            VecLoad<kVec>::store(A0 + (static_cast<size_t>(local) * 16 + lm) * C + k, sum);
+        }
+        return;
+    }
     if (inv_scale != nullptr) {   // density scaling, mace.cpp:1562-1584
         const float scale = inv_scale[i];
 #pragma unroll
@@ -158,7 +184,7 @@ l0_forward_warp_kernel(int num_nodes, int node0, const int* __restrict__ first, 
 // ---------------------------------------------------------------------------------------------
 template <int kVec>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
-l0_reverse_warp_kernel(int num_nodes, int node0, const int* __restrict__ first, const int* __restrict__ sources,
+l0_reverse_warp_kernel(int num_nodes, int node0, int parts, const int* __restrict__ first, const int* __restrict__ sources,
                        const EdgeGeom* __restrict__ geom, const unsigned char* __restrict__ atype, int num_active,
                        SplineGrid grid, const float* __restrict__ table, const float* __restrict__ A0_adj, ForceOutputs out,
                        DensityScale density)
@@ -166,13 +192,15 @@ l0_reverse_warp_kernel(int num_nodes, int node0, const int* __restrict__ first, 
     constexpr int C = 32 * kVec, F = 4 * C;
     __shared__ WarpChunk<true> chunks[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int local = blockIdx.x * kWarpsPerBlock + warp;   // receiver inside the tile
+    const int slot = blockIdx.x * kWarpsPerBlock + warp;
+    const int local = slot / parts;                         // receiver inside the tile
     if (local >= num_nodes) return;
     const int i = node0 + local;                            // graph-wide receiver index
     WarpChunk<true>& s = chunks[warp];
     const int k = lane * kVec;
     const int type_i = atype[i];
-    const int begin = first[i], end = first[i + 1];
+    const int2 range = edge_part(first, i, slot % parts, parts);
+    const int begin = range.x, end = range.y;
     float adj[16][kVec];
     {
         const float* in = A0_adj + static_cast<size_t>(local) * 16 * C + k;

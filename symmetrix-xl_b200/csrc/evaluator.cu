@@ -71,6 +71,69 @@ inline int blocks_for(long n, int threads) { return static_cast<int>((n + thread
         else KERNEL<0><<<(GRID), (C), 0, (STREAM)>>>(__VA_ARGS__);                    \
     } while (0)
 
+// How many parts to deal a receiver's edges to (edge_part in edge_kernels.cuh) in a gradient kernel.  `units` receivers of
+// `edges` list edges each run on `slots` resident blocks or warps; a part costs its edges plus `overhead` edges' worth of
+// prologue, chunk fill and reductions.  Up to a few rounds of the chip the last round is counted whole (a chain in it takes
+// as long as any other), beyond that half of it; a further part has to pay for itself by a twentieth.  Measured, 128
+// channels, 100 list edges, us at 1 / 2 / 4 / 8 parts: layer-1 gradient, 40 receivers 68 / 39 / 29 / 23, 317: 99 / 101 / 85 /
+// 91, 599: 177 / 146 / 150 / 162, 1080: 295 / 296 / 310 / 353; layer-0 gradient, 40: 81 / 45 / 29 / 21, 599: 88 / 58 / 60 /
+// 56, 2160: 182 / 149 / 146 / 161.
+int edge_parts(long units, double slots, double edges, double overhead, int most)
+{
+    int best = 1;
+    double best_cost = 0.0;
+    for (int parts = 1; parts <= most; parts *= 2) {
+        const double rounds = static_cast<double>(units) * parts / slots;
+        const double cost = (rounds < 4.0 ? std::ceil(rounds) : rounds + 0.5) * (edges / parts + overhead);
+        if (parts == 1 || cost < 0.95 * best_cost) {
+            best = parts;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+// The same for the layer-1 forward kernel, whose parts meet in a cluster: as many as fill the chip once.  Measured at 1 / 2 /
+// 4 / 8 parts: 40 receivers 37 / 34 / 23 / 18 us; 317 receivers (which fill it at one part and a half) 51 / 62 / 62 / 68 us.
+int cluster_parts(long units, double slots)
+{
+    int parts = 1;
+    while (parts < 8 && units * parts * 2 <= slots) parts *= 2;
+    return parts;
+}
+
+// Launches a kernel over (receivers, parts) with the parts of a receiver as one cluster, each with `row_bytes` of dynamic
+// shared memory.
+template <typename... Params, typename... Args>
+void launch_parts(void (*kernel)(Params...), int receivers, int parts, int threads, std::size_t row_bytes, cudaStream_t stream, Args&&... args)
+{
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(receivers, parts);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = row_bytes;
+    config.stream = stream;
+    cudaLaunchAttribute cluster = {};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = 1;
+    cluster.val.clusterDim.y = parts;
+    cluster.val.clusterDim.z = 1;
+    config.attrs = &cluster;
+    config.numAttrs = 1;
+    SXB_CUDA(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...));
+}
+// A layer-1 forward kernel: the plain build for one part, the cluster build for several.
+#define SXB_LAUNCH_PARTS(KERNEL, PART_KERNEL, RECEIVERS, PARTS, THREADS, ROW_BYTES, STREAM, ...)                        \
+    do {                                                                                                             \
+        if ((PARTS) == 1) KERNEL<<<(RECEIVERS), (THREADS), 0, (STREAM)>>>(__VA_ARGS__);                               \
+        else launch_parts(PART_KERNEL, (RECEIVERS), (PARTS), (THREADS), (ROW_BYTES), (STREAM), __VA_ARGS__);          \
+    } while (0)
+#define SXB_LAUNCH_PARTS_BY_CHANNELS(KERNEL, C, RECEIVERS, PARTS, ROW_BYTES, STREAM, ...)                              \
+    do {                                                                                                             \
+        if ((C) == 128) SXB_LAUNCH_PARTS(KERNEL<128>, (KERNEL<128, false, true>), RECEIVERS, PARTS, 128, ROW_BYTES, STREAM, __VA_ARGS__); \
+        else if ((C) == 32) SXB_LAUNCH_PARTS(KERNEL<32>, (KERNEL<32, false, true>), RECEIVERS, PARTS, 32, ROW_BYTES, STREAM, __VA_ARGS__); \
+        else SXB_LAUNCH_PARTS(KERNEL<0>, (KERNEL<0, false, true>), RECEIVERS, PARTS, C, ROW_BYTES, STREAM, __VA_ARGS__); \
+    } while (0)
+
 // Launches a symmetric-contraction kernel with G nodes per thread (G in {1, 2}); the dynamic
 // shared memory holds the [terms][32] weight slice of the block's element.
 #define SXB_LAUNCH_POLY(KERNEL, G, TERMS, T, C, STREAM, ...)                                                 \
@@ -951,14 +1014,23 @@ void Evaluator::run_pipeline(int phases)
     const float* inv1 = model_.a1_scaled ? inv_scale1_.ptr : nullptr;
     const DensityScale density0{model_.a0_scaled ? density0_table_.ptr : nullptr, inv_scale0_.ptr, dot0_.ptr, n_active};
     const DensityScale density1{model_.a1_scaled ? density1_table_.ptr : nullptr, inv_scale1_.ptr, dot1_.ptr, n_active};
+    // parts a receiver's edges are dealt to; resident warps per SM: 16 forward, 12 in the gradients (128 and 168 registers).
+    // Layer-0 forward has a build for one warp or a whole block per receiver: 40 receivers 46 -> 20 us, 599: 50 -> 38 us,
+    // 1080: 57 -> 47 us, 2160: 80 -> 86 us.
+    const double mean_edges = static_cast<double>(num_edges_) / std::max(1, R), block_warps = std::max(1, C / 32);
+    auto l1_forward_parts = [&](int T) { return cluster_parts(T, num_sms_ * std::floor(16.0 / block_warps)); };
+    auto l1_reverse_parts = [&](int T) { return edge_parts(T, num_sms_ * std::floor(12.0 / block_warps), mean_edges, 5.0, 8); };
+    auto l0_forward_parts = [&](int T) { return edge_parts(T, num_sms_ * 16.0, mean_edges, 6.0, kWarpsPerBlock) > 1 ? kWarpsPerBlock : 1; };
+    auto l0_reverse_parts = [&](int T) { return edge_parts(T, num_sms_ * 12.0, mean_edges, 4.0, 8); };
     auto l0_forward = [&](int t0, int T) {
-        const int warp_grid = blocks_for(T, kWarpsPerBlock);
+        const int parts = l0_forward_parts(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
+        const std::size_t part_bytes = parts > 1 ? static_cast<std::size_t>(kWarpsPerBlock) * 16 * C * sizeof(float) : 0;
         if (C == 128)
-            l0_forward_warp_kernel<4><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
+            l0_forward_warp_kernel<4><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         else if (C == 64)
-            l0_forward_warp_kernel<2><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
+            l0_forward_warp_kernel<2><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         else if (C == 32)
-            l0_forward_warp_kernel<1><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
+            l0_forward_warp_kernel<1><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         else
             l0_forward_kernel<0><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         launches_ += 1;
@@ -1054,17 +1126,19 @@ void Evaluator::run_pipeline(int phases)
                 launches_ += 1;
                 span_end();
             } else {
+            const int forward_parts = l1_forward_parts(T);
+            const std::size_t row_bytes = static_cast<std::size_t>(NE) * C * sizeof(float);   // S2: a set has fewer rows
             span_begin("l1_forward");
             if (model_.shape_id == 0)
-                SXB_LAUNCH_BY_CHANNELS(l1_forward_kernel_S0, C, T, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
-                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_);
+                SXB_LAUNCH_PARTS_BY_CHANNELS(l1_forward_kernel_S0, C, T, forward_parts, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr);
             else if (model_.shape_id == 1)
-                SXB_LAUNCH_BY_CHANNELS(l1_forward_kernel_S1, C, T, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
-                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_);
+                SXB_LAUNCH_PARTS_BY_CHANNELS(l1_forward_kernel_S1, C, T, forward_parts, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr);
             else {
                 // one launch per path set; the sets write disjoint components of Phi1
 #define SXB_SPLIT_FORWARD(SET)                                                                                            \
-                l1_forward_split_kernel_S2_##SET<128><<<T, 128, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, \
+                SXB_LAUNCH_PARTS(l1_forward_split_kernel_S2_##SET<128>, (l1_forward_split_kernel_S2_##SET<128, true>), T, forward_parts, 128, row_bytes, stream_, T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, \
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_)
                 SXB_SPLIT_FORWARD(G0);
                 SXB_SPLIT_FORWARD(G1);
@@ -1189,17 +1263,18 @@ void Evaluator::run_pipeline(int phases)
             }
             span_end();
             span_begin("l1_reverse");
+            const int reverse_parts = l1_reverse_parts(T);
             if (deterministic_ && model_.shape_id == 0)      // records instead of atomics: the build with the channel count at run time
-                l1_reverse_kernel_S0<0, 3, true><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                l1_reverse_kernel_S0<0, 3, true><<<dim3(T, reverse_parts), C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
             else if (deterministic_ && model_.shape_id == 1)
-                l1_reverse_kernel_S1<0, 3, true><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                l1_reverse_kernel_S1<0, 3, true><<<dim3(T, reverse_parts), C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
             else if (model_.shape_id == 0)
-                SXB_LAUNCH_BY_CHANNELS(l1_reverse_kernel_S0, C, T, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                SXB_LAUNCH_BY_CHANNELS(l1_reverse_kernel_S0, C, dim3(T, reverse_parts), stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                                        reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
             else if (model_.shape_id == 1)
-                SXB_LAUNCH_BY_CHANNELS(l1_reverse_kernel_S1, C, T, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                SXB_LAUNCH_BY_CHANNELS(l1_reverse_kernel_S1, C, dim3(T, reverse_parts), stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                                        reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
             else {
                 // one launch per path set; the sets add into the same edge forces, so those are cleared
@@ -1207,7 +1282,7 @@ void Evaluator::run_pipeline(int phases)
                 ForceOutputs split = fo;
                 split.accumulate_edge = 2;
 #define SXB_SPLIT_REVERSE(SET)                                                                                            \
-                l1_reverse_split_kernel_S2_##SET<128><<<T, 128, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, \
+                l1_reverse_split_kernel_S2_##SET<128><<<dim3(T, reverse_parts), 128, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, \
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, split, density1, r1_pair_types_)
                 SXB_SPLIT_REVERSE(G0);
                 SXB_SPLIT_REVERSE(G1);
@@ -1299,13 +1374,13 @@ void Evaluator::run_pipeline(int phases)
             span_end();
             span_begin("l0_reverse");
             {
-                const int warp_grid = blocks_for(T, kWarpsPerBlock);
+                const int parts = l0_reverse_parts(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
                 if (C == 128)
-                    l0_reverse_warp_kernel<4><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
+                    l0_reverse_warp_kernel<4><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else if (C == 64)
-                    l0_reverse_warp_kernel<2><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
+                    l0_reverse_warp_kernel<2><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else if (C == 32)
-                    l0_reverse_warp_kernel<1><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
+                    l0_reverse_warp_kernel<1><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else
                     l0_reverse_kernel<0><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
             }

@@ -497,3 +497,27 @@ def test_nve_energy_conservation(pkg, model_path):
     drift = np.abs(e - e[0]).max() / len(pos)
     assert drift < 2e-4, drift          # eV/atom over 20 fs
     assert md.kinetic() > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("arch,copies", [("medium", (2, 1, 1)), ("medium", (4, 2, 2)), ("small", (4, 2, 1)), ("large", (2, 2, 1))])
+def test_parts_of_a_receiver_add_up(pkg, model_path, arch, copies):
+    """A receiver's edges are dealt to more blocks and warps the fewer receivers there are: a cell of 38 atoms (most parts)
+    against the oracle, and its periodic copies (fewer parts, down to one) against the cell.  Bounds: those of the oracle
+    comparison; the copies differ from the cell by the order of float sums alone."""
+    from oracle import mace_numpy, neighbor
+
+    path = model_path(arch, 31)
+    pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 12)
+    pos, types = pos[2:], types[2:]
+    calc = pkg.Calculator(path, skin=0.5)
+    out = calc.calculate(pos, cell, types)
+    first, src, shifts = neighbor.build_neighbor_graph(pos, cell, calc.evaluator.r_cut + 0.5)
+    _e, energies, forces, _s = mace_numpy.NumpyMACE(str(path)).energy_forces_stress(types, pos, cell, first, src, shifts)
+    assert np.abs(out["energies"] - energies).max() <= TOL_E
+    assert np.abs(out["forces"] - forces).max() <= TOL_F
+    grid = np.stack(np.meshgrid(*[np.arange(c) for c in copies], indexing="ij"), axis=-1).reshape(-1, 3)
+    many = (pos[None] + (grid @ cell)[:, None]).reshape(-1, 3)
+    big = pkg.Calculator(path, skin=0.5).calculate(many, cell * np.array(copies)[:, None], np.tile(types, len(grid)))
+    assert np.abs(big["energies"].reshape(len(grid), -1) - out["energies"]).max() <= TOL_E
+    assert np.abs(big["forces"].reshape(len(grid), -1, 3) - out["forces"]).max() <= TOL_F
