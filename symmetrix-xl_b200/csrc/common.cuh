@@ -70,6 +70,36 @@ struct alignas(16) EdgeGeom {
     float ux, uy, uz, r;
 };
 
+// A pair of floats (two adjacent channels) in an aligned register pair, low word first, and the packed arithmetic of
+// sm_100a on it: each half rounds as the scalar instruction does, at one issue slot for both.  Measured with operands that
+// all differ: 44 TFLOP/s scalar (register ports), 67 TFLOP/s packed.
+using f2 = unsigned long long;
+
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
+{
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
+{
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
+{
+    f2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ float f2_sum(f2 v)
+{
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return lo + hi;
+}
+
 // Radial spline grid in the precision the kernels evaluate it in.
 struct SplineGrid {
     float x0, h, r_cut;

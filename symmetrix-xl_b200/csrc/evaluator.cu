@@ -134,23 +134,22 @@ void launch_parts(void (*kernel)(Params...), int receivers, int parts, int threa
         else SXB_LAUNCH_PARTS(KERNEL<0>, (KERNEL<0, false, true>), RECEIVERS, PARTS, C, ROW_BYTES, STREAM, __VA_ARGS__); \
     } while (0)
 
-// Launches a symmetric-contraction kernel with G nodes per thread (G in {1, 2}); the dynamic
-// shared memory holds the [terms][32] weight slice of the block's element.
-#define SXB_LAUNCH_POLY(KERNEL, G, TERMS, T, C, STREAM, ...)                                                 \
+// Launches a symmetric-contraction kernel; the dynamic shared memory holds the [terms][32] weight slice of the block's
+// element.  A pass of a block takes two nodes per warp; a block makes up to four passes with the slice it has staged, as
+// long as that leaves every SM four blocks.
+#define SXB_LAUNCH_POLY(KERNEL, NAME, TERMS, T, C, STREAM, ...)                                              \
     do {                                                                                                     \
-        const dim3 grid_(blocks_for((T), kPolyNodesPerBlock), (C) / 32);                                     \
+        int nodes_ = 2 * kPolyWarps##NAME;                                                                   \
+        while (nodes_ < 8 * kPolyWarps##NAME && blocks_for((T), 2 * nodes_) * ((C) / 32) >= 4 * num_sms_) nodes_ *= 2; \
+        const dim3 grid_(blocks_for((T), nodes_), (C) / 32);                                                 \
         const std::size_t smem_ = static_cast<std::size_t>(TERMS) * 32 * sizeof(float);                      \
-        if ((G) == 2) KERNEL<2><<<grid_, 32 * kPolyWarps, smem_, (STREAM)>>>(__VA_ARGS__);                   \
-        else KERNEL<1><<<grid_, 32 * kPolyWarps, smem_, (STREAM)>>>(__VA_ARGS__);                            \
+        KERNEL##_##NAME<<<grid_, 32 * kPolyWarps##NAME, smem_, (STREAM)>>>((T), nodes_, (C), __VA_ARGS__);    \
     } while (0)
 
 // Opts a contraction kernel into the dynamic shared memory its weight slice needs (once, at start-up).
 #define SXB_ALLOW_POLY_SMEM(KERNEL, TERMS)                                                                   \
-    do {                                                                                                     \
-        const int smem_ = static_cast<int>(static_cast<std::size_t>(TERMS) * 32 * sizeof(float));            \
-        SXB_CUDA(cudaFuncSetAttribute(KERNEL<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_));       \
-        SXB_CUDA(cudaFuncSetAttribute(KERNEL<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_));       \
-    } while (0)
+    SXB_CUDA(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,                       \
+                                  static_cast<int>(static_cast<std::size_t>(TERMS) * 32 * sizeof(float))))
 
 }  // namespace
 
@@ -190,10 +189,6 @@ Evaluator::Evaluator(const std::string& json_path, int device_ordinal, const std
     upload(atomic_energies_, model_.atomic_energies, stream_);
     if (const char* env = std::getenv("SXB_SIMT_LINEARS")) use_tensor_cores_ = !(env[0] == '1');
     if (const char* env = std::getenv("SXB_CUDA_GRAPHS")) use_graphs_ = env[0] != '0';
-    if (const char* env = std::getenv("SXB_POLY_GROUP")) {   // nodes per thread in the contraction kernels: "<forward><reverse>"
-        if (env[0] == '1' || env[0] == '2') poly_g_forward_ = env[0] - '0';
-        if (env[0] != 0 && (env[1] == '1' || env[1] == '2')) poly_g_reverse_ = env[1] - '0';
-    }
     for (int l = 0; l <= model_.hidden_l_max; ++l)
         upload_split(s_h1_[l], model_.w_h1.data() + static_cast<std::size_t>(l) * C * C, C, C);
     if (!model_.single_layer)
@@ -1073,11 +1068,11 @@ void Evaluator::run_pipeline(int phases)
             span_begin("m0_forward");
             float* m0 = M0_.ptr + t0 * rowH;
             if (model_.shape_id == 0)
-                SXB_LAUNCH_POLY(m0_forward_kernel_S0, poly_g_forward_, SXB_S0_M0_NUM_TERMS, T, C, stream_, T, C, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, m0);
+                SXB_LAUNCH_POLY(m0_forward_kernel, S0, SXB_S0_M0_NUM_TERMS, T, C, stream_, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, m0);
             else if (model_.shape_id == 1)
-                SXB_LAUNCH_POLY(m0_forward_kernel_S1, poly_g_forward_, SXB_S1_M0_NUM_TERMS, T, C, stream_, T, C, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, m0);
+                SXB_LAUNCH_POLY(m0_forward_kernel, S1, SXB_S1_M0_NUM_TERMS, T, C, stream_, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, m0);
             else
-                SXB_LAUNCH_POLY(m0_forward_kernel_S2, poly_g_forward_, SXB_S2_M0_NUM_TERMS, T, C, stream_, T, C, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, m0);
+                SXB_LAUNCH_POLY(m0_forward_kernel, S2, SXB_S2_M0_NUM_TERMS, T, C, stream_, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, m0);
             launches_ += 1;
             span_end();
             // H1_il = M0_il W_l
@@ -1163,11 +1158,11 @@ void Evaluator::run_pipeline(int phases)
             span_end();
             span_begin("m1_forward");
             if (model_.shape_id == 0)
-                SXB_LAUNCH_POLY(m1_forward_kernel_S0, poly_g_forward_, SXB_S0_M1_NUM_TERMS, T, C, stream_, T, C, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_.ptr);
+                SXB_LAUNCH_POLY(m1_forward_kernel, S0, SXB_S0_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_.ptr);
             else if (model_.shape_id == 1)
-                SXB_LAUNCH_POLY(m1_forward_kernel_S1, poly_g_forward_, SXB_S1_M1_NUM_TERMS, T, C, stream_, T, C, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_.ptr);
+                SXB_LAUNCH_POLY(m1_forward_kernel, S1, SXB_S1_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_.ptr);
             else
-                SXB_LAUNCH_POLY(m1_forward_kernel_S2, poly_g_forward_, SXB_S2_M1_NUM_TERMS, T, C, stream_, T, C, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_.ptr);
+                SXB_LAUNCH_POLY(m1_forward_kernel, S2, SXB_S2_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_.ptr);
             launches_ += 1;
             span_end();
             }
@@ -1243,11 +1238,11 @@ void Evaluator::run_pipeline(int phases)
             }
             span_begin("m1_reverse");
             if (model_.shape_id == 0)
-                SXB_LAUNCH_POLY(m1_reverse_kernel_S0, poly_g_reverse_, SXB_S0_M1_NUM_TERMS, T, C, stream_, T, C, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_adj_.ptr, A1_adj_.ptr, model_.a1_scaled ? dot1_.ptr + t0 : nullptr);
+                SXB_LAUNCH_POLY(m1_reverse_kernel, S0, SXB_S0_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_adj_.ptr, A1_adj_.ptr, model_.a1_scaled ? dot1_.ptr + t0 : nullptr);
             else if (model_.shape_id == 1)
-                SXB_LAUNCH_POLY(m1_reverse_kernel_S1, poly_g_reverse_, SXB_S1_M1_NUM_TERMS, T, C, stream_, T, C, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_adj_.ptr, A1_adj_.ptr, model_.a1_scaled ? dot1_.ptr + t0 : nullptr);
+                SXB_LAUNCH_POLY(m1_reverse_kernel, S1, SXB_S1_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_adj_.ptr, A1_adj_.ptr, model_.a1_scaled ? dot1_.ptr + t0 : nullptr);
             else
-                SXB_LAUNCH_POLY(m1_reverse_kernel_S2, poly_g_reverse_, SXB_S2_M1_NUM_TERMS, T, C, stream_, T, C, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_adj_.ptr, A1_adj_.ptr, model_.a1_scaled ? dot1_.ptr + t0 : nullptr);
+                SXB_LAUNCH_POLY(m1_reverse_kernel, S2, SXB_S2_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_adj_.ptr, A1_adj_.ptr, model_.a1_scaled ? dot1_.ptr + t0 : nullptr);
             launches_ += 1;
             span_end();
             span_begin("gemm_a1_reverse");
@@ -1365,11 +1360,11 @@ void Evaluator::run_pipeline(int phases)
             span_end();
             span_begin("m0_reverse");
             if (model_.shape_id == 0)
-                SXB_LAUNCH_POLY(m0_reverse_kernel_S0, poly_g_reverse_, SXB_S0_M0_NUM_TERMS, T, C, stream_, T, C, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, M0_adj_.ptr, A0_adj_.ptr, model_.a0_scaled ? dot0_.ptr + t0 : nullptr);
+                SXB_LAUNCH_POLY(m0_reverse_kernel, S0, SXB_S0_M0_NUM_TERMS, T, C, stream_, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, M0_adj_.ptr, A0_adj_.ptr, model_.a0_scaled ? dot0_.ptr + t0 : nullptr);
             else if (model_.shape_id == 1)
-                SXB_LAUNCH_POLY(m0_reverse_kernel_S1, poly_g_reverse_, SXB_S1_M0_NUM_TERMS, T, C, stream_, T, C, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, M0_adj_.ptr, A0_adj_.ptr, model_.a0_scaled ? dot0_.ptr + t0 : nullptr);
+                SXB_LAUNCH_POLY(m0_reverse_kernel, S1, SXB_S1_M0_NUM_TERMS, T, C, stream_, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, M0_adj_.ptr, A0_adj_.ptr, model_.a0_scaled ? dot0_.ptr + t0 : nullptr);
             else
-                SXB_LAUNCH_POLY(m0_reverse_kernel_S2, poly_g_reverse_, SXB_S2_M0_NUM_TERMS, T, C, stream_, T, C, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, M0_adj_.ptr, A0_adj_.ptr, model_.a0_scaled ? dot0_.ptr + t0 : nullptr);
+                SXB_LAUNCH_POLY(m0_reverse_kernel, S2, SXB_S2_M0_NUM_TERMS, T, C, stream_, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, M0_adj_.ptr, A0_adj_.ptr, model_.a0_scaled ? dot0_.ptr + t0 : nullptr);
             launches_ += 1;
             span_end();
             span_begin("l0_reverse");

@@ -176,7 +176,6 @@ private:
     DeviceBuffer<unsigned char> nb_temp_, ig_temp_;
     DeviceBuffer<float> zbl_pairs_;    // [active pair][4]: 1/a, 14.3996 Z_i Z_j, r_max, pad (models with ZBL)
     bool use_tma_activations_ = true;   // operand-streaming form of the tensor-core linears (N in {32, 64, 128})
-    int poly_g_forward_ = 1, poly_g_reverse_ = 1;   // nodes per thread in the symmetric-contraction kernels
     void upload_split(SplitWeight& out, const float* w, int rows, int cols);
     struct TcCall {
         const float* A; RowMap a_rows; const SplitWeight* w; bool reverse; float* C; RowMap c_rows;

@@ -74,6 +74,59 @@ def reverse_path_lines(p, q, l, l1, l2, base):
     return out
 
 
+def contraction_lines(terms):
+    """Straight-line bodies of a symmetric contraction, terms = [(out, term, monomial)], on channel pairs: W(t) weight of term
+    t, x[] inputs, o[] outputs (start at zero), adj[] output adjoints, g[] input adjoints (start at zero).
+
+    The monomials of degree 2 and 3 are grouped by their first two factors a, b, so that the products a b and the sums over
+    the third factor are formed once per group:
+      forward   o[out] += (x_a x_b) (sum_c w x_c + w_ab)                          one operation per term and one per group
+      reverse   s = sum_out w adj;  g_c += s x_a x_b;  v = sum_c s x_c + s_ab;  g_a += v x_b;  g_b += v x_a
+                                                                                  three per term, three per group
+    against three and seven operations for every term on its own."""
+    fwd, rev, pairs = [], [], {}
+    for out, t, mono in terms:
+        if len(mono) == 1:
+            fwd.append(f"      o[{out}] = f2_fma(W({t}), x[{mono[0]}], o[{out}]);")
+            rev.append(f"      g[{mono[0]}] = f2_fma(W({t}), adj[{out}], g[{mono[0]}]);")
+        else:
+            third = mono[2] if len(mono) == 3 else None
+            pairs.setdefault((mono[0], mono[1]), {}).setdefault(third, []).append((out, t))
+    for (a, b), group in sorted(pairs.items()):
+        fwd_group, rev_group = [], []     # a group is one line of the header
+        thirds = sorted(group, key=lambda c: (c is not None, c))
+        fwd_group.append(f"      {{ const unsigned long long p = f2_mul(x[{a}], x[{b}]);")
+        for out in sorted({o for c in thirds for o, _ in group[c]}):
+            expr = None
+            for c in thirds:
+                for o, t in group[c]:
+                    if o == out:
+                        if c is None:
+                            expr = f"W({t})" if expr is None else f"f2_add({expr}, W({t}))"
+                        else:
+                            expr = f"f2_mul(W({t}), x[{c}])" if expr is None else f"f2_fma(W({t}), x[{c}], {expr})"
+            fwd_group.append(f"        o[{out}] = f2_fma(p, {expr}, o[{out}]);")
+        fwd_group.append("      }")
+        cubic = any(c is not None for c in thirds)
+        rev_group.append("      {" + (f" const unsigned long long p = f2_mul(x[{a}], x[{b}]);" if cubic else "") + " unsigned long long v;")
+        first = True
+        for c in thirds:
+            expr = None
+            for o, t in group[c]:
+                expr = f"f2_mul(W({t}), adj[{o}])" if expr is None else f"f2_fma(W({t}), adj[{o}], {expr})"
+            if c is None:
+                rev_group.append(f"        v = {expr};")
+            else:
+                rev_group.append(f"        {{ const unsigned long long s = {expr}; g[{c}] = f2_fma(s, p, g[{c}]); "
+                           + (f"v = f2_mul(s, x[{c}]); }}" if first else f"v = f2_fma(s, x[{c}], v); }}"))
+            first = False
+        rev_group.append(f"        g[{a}] = f2_fma(v, x[{b}], g[{a}]); g[{b}] = f2_fma(v, x[{a}], g[{b}]);")
+        rev_group.append("      }")
+        fwd.append("      " + " ".join(part.strip() for part in fwd_group))
+        rev.append("      " + " ".join(part.strip() for part in rev_group))
+    return fwd, rev
+
+
 def emit_shape(name, l_max, L_max, tables, groups=1, by_edge_l=None):
     out = []
     paths = list(zip(tables["Phi1_l"], tables["Phi1_l1"], tables["Phi1_l2"]))
@@ -138,6 +191,13 @@ def emit_shape(name, l_max, L_max, tables, groups=1, by_edge_l=None):
             l3_.append(f"    X3(0, {t}, {mono[0]}, {mono[1]}, {mono[2]})")
     out.append(f"#define SXB_{name}_M1_TERMS(X1, X2, X3) \\")
     out.append(" \\\n".join(l1_ + l2_ + l3_))
+    m0 = [(LM, offs[LM] + t, mono) for LM in range(num_LM) for t, mono in enumerate(tables["M0_monomials"][str(LM)])]
+    for which, terms in (("M0", m0), ("M1", [(0, t, mono) for t, mono in enumerate(m1)])):
+        fwd, rev = contraction_lines(terms)
+        out.append(f"#define SXB_{name}_{which}_FORWARD_BODY \\")
+        out.append(" \\\n".join(fwd))
+        out.append(f"#define SXB_{name}_{which}_REVERSE_BODY \\")
+        out.append(" \\\n".join(rev))
     # straight-line bodies of the layer-1 edge kernels (one channel per thread):
     #   R[p], dR[p]: radial value / derivative of path p;  y[lm]: edge harmonics;
     #   h[lm2]: source features;  acc[row] / adj[row]: receiver row sums / row adjoints

@@ -249,6 +249,302 @@
     X3(0, 91, 8, 12, 14) \
     X3(0, 92, 8, 13, 13) \
     X3(0, 93, 8, 13, 15)
+#define SXB_S0_M0_FORWARD_BODY \
+      o[0] = f2_fma(W(0), x[0], o[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); o[0] = f2_fma(p, f2_fma(W(17), x[0], W(1)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); o[0] = f2_fma(p, f2_mul(W(18), x[1]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); o[0] = f2_fma(p, f2_mul(W(19), x[2]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); o[0] = f2_fma(p, f2_mul(W(20), x[3]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); o[0] = f2_fma(p, f2_mul(W(21), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); o[0] = f2_fma(p, f2_mul(W(22), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); o[0] = f2_fma(p, f2_mul(W(23), x[6]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); o[0] = f2_fma(p, f2_mul(W(24), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); o[0] = f2_fma(p, f2_mul(W(25), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); o[0] = f2_fma(p, f2_mul(W(26), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); o[0] = f2_fma(p, f2_mul(W(27), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); o[0] = f2_fma(p, f2_mul(W(28), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); o[0] = f2_fma(p, f2_mul(W(29), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); o[0] = f2_fma(p, f2_mul(W(30), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); o[0] = f2_fma(p, f2_mul(W(31), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); o[0] = f2_fma(p, f2_mul(W(32), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); o[0] = f2_fma(p, f2_fma(W(34), x[8], f2_fma(W(33), x[6], W(2))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); o[0] = f2_fma(p, f2_mul(W(35), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); o[0] = f2_fma(p, f2_mul(W(36), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); o[0] = f2_fma(p, f2_fma(W(38), x[15], f2_mul(W(37), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); o[0] = f2_fma(p, f2_fma(W(40), x[14], f2_mul(W(39), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); o[0] = f2_fma(p, f2_mul(W(41), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); o[0] = f2_fma(p, f2_mul(W(42), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); o[0] = f2_fma(p, f2_fma(W(44), x[11], f2_mul(W(43), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); o[0] = f2_fma(p, f2_fma(W(45), x[6], W(3)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); o[0] = f2_fma(p, f2_mul(W(46), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); o[0] = f2_fma(p, f2_mul(W(47), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); o[0] = f2_fma(p, f2_mul(W(48), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); o[0] = f2_fma(p, f2_mul(W(49), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); o[0] = f2_fma(p, f2_mul(W(50), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); o[0] = f2_fma(p, f2_mul(W(51), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); o[0] = f2_fma(p, f2_fma(W(53), x[8], f2_fma(W(52), x[6], W(4))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); o[0] = f2_fma(p, f2_fma(W(55), x[11], f2_mul(W(54), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); o[0] = f2_fma(p, f2_mul(W(56), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); o[0] = f2_fma(p, f2_mul(W(57), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); o[0] = f2_fma(p, f2_fma(W(59), x[14], f2_mul(W(58), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); o[0] = f2_fma(p, f2_fma(W(61), x[15], f2_mul(W(60), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); o[0] = f2_fma(p, f2_fma(W(62), x[6], W(5)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); o[0] = f2_fma(p, f2_mul(W(63), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); o[0] = f2_fma(p, f2_mul(W(64), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); o[0] = f2_fma(p, f2_mul(W(65), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); o[0] = f2_fma(p, f2_fma(W(67), x[15], f2_mul(W(66), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); o[0] = f2_fma(p, f2_fma(W(69), x[8], f2_fma(W(68), x[6], W(6))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); o[0] = f2_fma(p, f2_mul(W(70), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); o[0] = f2_fma(p, f2_fma(W(72), x[15], f2_mul(W(71), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); o[0] = f2_fma(p, f2_fma(W(74), x[14], f2_mul(W(73), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); o[0] = f2_fma(p, f2_fma(W(75), x[6], W(7)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); o[0] = f2_fma(p, f2_mul(W(76), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); o[0] = f2_fma(p, f2_mul(W(77), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); o[0] = f2_fma(p, f2_mul(W(78), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); o[0] = f2_fma(p, f2_mul(W(79), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); o[0] = f2_fma(p, f2_mul(W(80), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); o[0] = f2_fma(p, f2_mul(W(81), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); o[0] = f2_fma(p, f2_mul(W(82), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); o[0] = f2_fma(p, f2_fma(W(83), x[8], W(8)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); o[0] = f2_fma(p, f2_mul(W(84), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); o[0] = f2_fma(p, f2_mul(W(85), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); o[0] = f2_fma(p, f2_mul(W(86), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); o[0] = f2_fma(p, f2_mul(W(87), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); o[0] = f2_fma(p, f2_mul(W(88), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); o[0] = f2_fma(p, W(9), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); o[0] = f2_fma(p, f2_mul(W(89), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); o[0] = f2_fma(p, f2_mul(W(90), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); o[0] = f2_fma(p, f2_mul(W(91), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); o[0] = f2_fma(p, f2_fma(W(93), x[15], f2_mul(W(92), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); o[0] = f2_fma(p, W(10), o[0]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); o[0] = f2_fma(p, W(11), o[0]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); o[0] = f2_fma(p, W(12), o[0]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); o[0] = f2_fma(p, W(13), o[0]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); o[0] = f2_fma(p, W(14), o[0]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); o[0] = f2_fma(p, W(15), o[0]); } \
+      { const unsigned long long p = f2_mul(x[15], x[15]); o[0] = f2_fma(p, W(16), o[0]); }
+#define SXB_S0_M0_REVERSE_BODY \
+      g[0] = f2_fma(W(0), adj[0], g[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); unsigned long long v; v = f2_mul(W(1), adj[0]); { const unsigned long long s = f2_mul(W(17), adj[0]); g[0] = f2_fma(s, p, g[0]); v = f2_fma(s, x[0], v); } g[0] = f2_fma(v, x[0], g[0]); g[0] = f2_fma(v, x[0], g[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); unsigned long long v; { const unsigned long long s = f2_mul(W(18), adj[0]); g[1] = f2_fma(s, p, g[1]); v = f2_mul(s, x[1]); } g[0] = f2_fma(v, x[1], g[0]); g[1] = f2_fma(v, x[0], g[1]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(19), adj[0]); g[2] = f2_fma(s, p, g[2]); v = f2_mul(s, x[2]); } g[0] = f2_fma(v, x[2], g[0]); g[2] = f2_fma(v, x[0], g[2]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(20), adj[0]); g[3] = f2_fma(s, p, g[3]); v = f2_mul(s, x[3]); } g[0] = f2_fma(v, x[3], g[0]); g[3] = f2_fma(v, x[0], g[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(21), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[0] = f2_fma(v, x[4], g[0]); g[4] = f2_fma(v, x[0], g[4]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(22), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[0] = f2_fma(v, x[5], g[0]); g[5] = f2_fma(v, x[0], g[5]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(23), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_mul(s, x[6]); } g[0] = f2_fma(v, x[6], g[0]); g[6] = f2_fma(v, x[0], g[6]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(24), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[0] = f2_fma(v, x[7], g[0]); g[7] = f2_fma(v, x[0], g[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(25), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[0] = f2_fma(v, x[8], g[0]); g[8] = f2_fma(v, x[0], g[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(26), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[0] = f2_fma(v, x[9], g[0]); g[9] = f2_fma(v, x[0], g[9]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(27), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[0] = f2_fma(v, x[10], g[0]); g[10] = f2_fma(v, x[0], g[10]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(28), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[0] = f2_fma(v, x[11], g[0]); g[11] = f2_fma(v, x[0], g[11]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(29), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[0] = f2_fma(v, x[12], g[0]); g[12] = f2_fma(v, x[0], g[12]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(30), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[0] = f2_fma(v, x[13], g[0]); g[13] = f2_fma(v, x[0], g[13]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(31), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[0] = f2_fma(v, x[14], g[0]); g[14] = f2_fma(v, x[0], g[14]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(32), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[0] = f2_fma(v, x[15], g[0]); g[15] = f2_fma(v, x[0], g[15]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); unsigned long long v; v = f2_mul(W(2), adj[0]); { const unsigned long long s = f2_mul(W(33), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(34), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[1] = f2_fma(v, x[1], g[1]); g[1] = f2_fma(v, x[1], g[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(35), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[1] = f2_fma(v, x[2], g[1]); g[2] = f2_fma(v, x[1], g[2]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(36), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[1] = f2_fma(v, x[3], g[1]); g[3] = f2_fma(v, x[1], g[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(37), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(38), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[4], g[1]); g[4] = f2_fma(v, x[1], g[4]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(39), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(40), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[5], g[1]); g[5] = f2_fma(v, x[1], g[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(41), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[1] = f2_fma(v, x[6], g[1]); g[6] = f2_fma(v, x[1], g[6]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(42), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[1] = f2_fma(v, x[7], g[1]); g[7] = f2_fma(v, x[1], g[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(43), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(44), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[1] = f2_fma(v, x[8], g[1]); g[8] = f2_fma(v, x[1], g[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); unsigned long long v; v = f2_mul(W(3), adj[0]); { const unsigned long long s = f2_mul(W(45), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[2] = f2_fma(v, x[2], g[2]); g[2] = f2_fma(v, x[2], g[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(46), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[2] = f2_fma(v, x[3], g[2]); g[3] = f2_fma(v, x[2], g[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(47), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[2] = f2_fma(v, x[4], g[2]); g[4] = f2_fma(v, x[2], g[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(48), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[2] = f2_fma(v, x[5], g[2]); g[5] = f2_fma(v, x[2], g[5]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(49), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[2] = f2_fma(v, x[6], g[2]); g[6] = f2_fma(v, x[2], g[6]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(50), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[2] = f2_fma(v, x[7], g[2]); g[7] = f2_fma(v, x[2], g[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(51), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[2] = f2_fma(v, x[8], g[2]); g[8] = f2_fma(v, x[2], g[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); unsigned long long v; v = f2_mul(W(4), adj[0]); { const unsigned long long s = f2_mul(W(52), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(53), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[3] = f2_fma(v, x[3], g[3]); g[3] = f2_fma(v, x[3], g[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(54), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(55), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[3] = f2_fma(v, x[4], g[3]); g[4] = f2_fma(v, x[3], g[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(56), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[3] = f2_fma(v, x[5], g[3]); g[5] = f2_fma(v, x[3], g[5]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(57), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[3] = f2_fma(v, x[6], g[3]); g[6] = f2_fma(v, x[3], g[6]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(58), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(59), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[7], g[3]); g[7] = f2_fma(v, x[3], g[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(60), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(61), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[8], g[3]); g[8] = f2_fma(v, x[3], g[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); unsigned long long v; v = f2_mul(W(5), adj[0]); { const unsigned long long s = f2_mul(W(62), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[4] = f2_fma(v, x[4], g[4]); g[4] = f2_fma(v, x[4], g[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(63), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[4] = f2_fma(v, x[5], g[4]); g[5] = f2_fma(v, x[4], g[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(64), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[4] = f2_fma(v, x[9], g[4]); g[9] = f2_fma(v, x[4], g[9]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(65), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[4] = f2_fma(v, x[10], g[4]); g[10] = f2_fma(v, x[4], g[10]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(66), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(67), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[11], g[4]); g[11] = f2_fma(v, x[4], g[11]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); unsigned long long v; v = f2_mul(W(6), adj[0]); { const unsigned long long s = f2_mul(W(68), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(69), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[5] = f2_fma(v, x[5], g[5]); g[5] = f2_fma(v, x[5], g[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(70), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[5] = f2_fma(v, x[9], g[5]); g[9] = f2_fma(v, x[5], g[9]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(71), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(72), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[10], g[5]); g[10] = f2_fma(v, x[5], g[10]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(73), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(74), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[11], g[5]); g[11] = f2_fma(v, x[5], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); unsigned long long v; v = f2_mul(W(7), adj[0]); { const unsigned long long s = f2_mul(W(75), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[6] = f2_fma(v, x[6], g[6]); g[6] = f2_fma(v, x[6], g[6]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(76), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[6] = f2_fma(v, x[7], g[6]); g[7] = f2_fma(v, x[6], g[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(77), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[6] = f2_fma(v, x[8], g[6]); g[8] = f2_fma(v, x[6], g[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(78), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[6] = f2_fma(v, x[9], g[6]); g[9] = f2_fma(v, x[6], g[9]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(79), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[6] = f2_fma(v, x[11], g[6]); g[11] = f2_fma(v, x[6], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(80), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[6] = f2_fma(v, x[12], g[6]); g[12] = f2_fma(v, x[6], g[12]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(81), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[6] = f2_fma(v, x[13], g[6]); g[13] = f2_fma(v, x[6], g[13]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(82), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[6] = f2_fma(v, x[15], g[6]); g[15] = f2_fma(v, x[6], g[15]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); unsigned long long v; v = f2_mul(W(8), adj[0]); { const unsigned long long s = f2_mul(W(83), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[7] = f2_fma(v, x[7], g[7]); g[7] = f2_fma(v, x[7], g[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(84), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[7] = f2_fma(v, x[9], g[7]); g[9] = f2_fma(v, x[7], g[9]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(85), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[7] = f2_fma(v, x[10], g[7]); g[10] = f2_fma(v, x[7], g[10]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(86), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[7] = f2_fma(v, x[12], g[7]); g[12] = f2_fma(v, x[7], g[12]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(87), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[7] = f2_fma(v, x[13], g[7]); g[13] = f2_fma(v, x[7], g[13]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(88), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[7] = f2_fma(v, x[14], g[7]); g[14] = f2_fma(v, x[7], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(9), adj[0]); g[8] = f2_fma(v, x[8], g[8]); g[8] = f2_fma(v, x[8], g[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(89), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[9], g[8]); g[9] = f2_fma(v, x[8], g[9]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(90), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[11], g[8]); g[11] = f2_fma(v, x[8], g[11]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(91), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[8] = f2_fma(v, x[12], g[8]); g[12] = f2_fma(v, x[8], g[12]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(92), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(93), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[13], g[8]); g[13] = f2_fma(v, x[8], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(10), adj[0]); g[9] = f2_fma(v, x[9], g[9]); g[9] = f2_fma(v, x[9], g[9]); } \
+      { unsigned long long v; v = f2_mul(W(11), adj[0]); g[10] = f2_fma(v, x[10], g[10]); g[10] = f2_fma(v, x[10], g[10]); } \
+      { unsigned long long v; v = f2_mul(W(12), adj[0]); g[11] = f2_fma(v, x[11], g[11]); g[11] = f2_fma(v, x[11], g[11]); } \
+      { unsigned long long v; v = f2_mul(W(13), adj[0]); g[12] = f2_fma(v, x[12], g[12]); g[12] = f2_fma(v, x[12], g[12]); } \
+      { unsigned long long v; v = f2_mul(W(14), adj[0]); g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(15), adj[0]); g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(16), adj[0]); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
+#define SXB_S0_M1_FORWARD_BODY \
+      o[0] = f2_fma(W(0), x[0], o[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); o[0] = f2_fma(p, f2_fma(W(17), x[0], W(1)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); o[0] = f2_fma(p, f2_mul(W(18), x[1]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); o[0] = f2_fma(p, f2_mul(W(19), x[2]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); o[0] = f2_fma(p, f2_mul(W(20), x[3]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); o[0] = f2_fma(p, f2_mul(W(21), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); o[0] = f2_fma(p, f2_mul(W(22), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); o[0] = f2_fma(p, f2_mul(W(23), x[6]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); o[0] = f2_fma(p, f2_mul(W(24), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); o[0] = f2_fma(p, f2_mul(W(25), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); o[0] = f2_fma(p, f2_mul(W(26), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); o[0] = f2_fma(p, f2_mul(W(27), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); o[0] = f2_fma(p, f2_mul(W(28), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); o[0] = f2_fma(p, f2_mul(W(29), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); o[0] = f2_fma(p, f2_mul(W(30), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); o[0] = f2_fma(p, f2_mul(W(31), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); o[0] = f2_fma(p, f2_mul(W(32), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); o[0] = f2_fma(p, f2_fma(W(34), x[8], f2_fma(W(33), x[6], W(2))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); o[0] = f2_fma(p, f2_mul(W(35), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); o[0] = f2_fma(p, f2_mul(W(36), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); o[0] = f2_fma(p, f2_fma(W(38), x[15], f2_mul(W(37), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); o[0] = f2_fma(p, f2_fma(W(40), x[14], f2_mul(W(39), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); o[0] = f2_fma(p, f2_mul(W(41), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); o[0] = f2_fma(p, f2_mul(W(42), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); o[0] = f2_fma(p, f2_fma(W(44), x[11], f2_mul(W(43), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); o[0] = f2_fma(p, f2_fma(W(45), x[6], W(3)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); o[0] = f2_fma(p, f2_mul(W(46), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); o[0] = f2_fma(p, f2_mul(W(47), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); o[0] = f2_fma(p, f2_mul(W(48), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); o[0] = f2_fma(p, f2_mul(W(49), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); o[0] = f2_fma(p, f2_mul(W(50), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); o[0] = f2_fma(p, f2_mul(W(51), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); o[0] = f2_fma(p, f2_fma(W(53), x[8], f2_fma(W(52), x[6], W(4))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); o[0] = f2_fma(p, f2_fma(W(55), x[11], f2_mul(W(54), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); o[0] = f2_fma(p, f2_mul(W(56), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); o[0] = f2_fma(p, f2_mul(W(57), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); o[0] = f2_fma(p, f2_fma(W(59), x[14], f2_mul(W(58), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); o[0] = f2_fma(p, f2_fma(W(61), x[15], f2_mul(W(60), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); o[0] = f2_fma(p, f2_fma(W(62), x[6], W(5)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); o[0] = f2_fma(p, f2_mul(W(63), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); o[0] = f2_fma(p, f2_mul(W(64), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); o[0] = f2_fma(p, f2_mul(W(65), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); o[0] = f2_fma(p, f2_fma(W(67), x[15], f2_mul(W(66), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); o[0] = f2_fma(p, f2_fma(W(69), x[8], f2_fma(W(68), x[6], W(6))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); o[0] = f2_fma(p, f2_mul(W(70), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); o[0] = f2_fma(p, f2_fma(W(72), x[15], f2_mul(W(71), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); o[0] = f2_fma(p, f2_fma(W(74), x[14], f2_mul(W(73), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); o[0] = f2_fma(p, f2_fma(W(75), x[6], W(7)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); o[0] = f2_fma(p, f2_mul(W(76), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); o[0] = f2_fma(p, f2_mul(W(77), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); o[0] = f2_fma(p, f2_mul(W(78), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); o[0] = f2_fma(p, f2_mul(W(79), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); o[0] = f2_fma(p, f2_mul(W(80), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); o[0] = f2_fma(p, f2_mul(W(81), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); o[0] = f2_fma(p, f2_mul(W(82), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); o[0] = f2_fma(p, f2_fma(W(83), x[8], W(8)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); o[0] = f2_fma(p, f2_mul(W(84), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); o[0] = f2_fma(p, f2_mul(W(85), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); o[0] = f2_fma(p, f2_mul(W(86), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); o[0] = f2_fma(p, f2_mul(W(87), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); o[0] = f2_fma(p, f2_mul(W(88), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); o[0] = f2_fma(p, W(9), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); o[0] = f2_fma(p, f2_mul(W(89), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); o[0] = f2_fma(p, f2_mul(W(90), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); o[0] = f2_fma(p, f2_mul(W(91), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); o[0] = f2_fma(p, f2_fma(W(93), x[15], f2_mul(W(92), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); o[0] = f2_fma(p, W(10), o[0]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); o[0] = f2_fma(p, W(11), o[0]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); o[0] = f2_fma(p, W(12), o[0]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); o[0] = f2_fma(p, W(13), o[0]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); o[0] = f2_fma(p, W(14), o[0]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); o[0] = f2_fma(p, W(15), o[0]); } \
+      { const unsigned long long p = f2_mul(x[15], x[15]); o[0] = f2_fma(p, W(16), o[0]); }
+#define SXB_S0_M1_REVERSE_BODY \
+      g[0] = f2_fma(W(0), adj[0], g[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); unsigned long long v; v = f2_mul(W(1), adj[0]); { const unsigned long long s = f2_mul(W(17), adj[0]); g[0] = f2_fma(s, p, g[0]); v = f2_fma(s, x[0], v); } g[0] = f2_fma(v, x[0], g[0]); g[0] = f2_fma(v, x[0], g[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); unsigned long long v; { const unsigned long long s = f2_mul(W(18), adj[0]); g[1] = f2_fma(s, p, g[1]); v = f2_mul(s, x[1]); } g[0] = f2_fma(v, x[1], g[0]); g[1] = f2_fma(v, x[0], g[1]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(19), adj[0]); g[2] = f2_fma(s, p, g[2]); v = f2_mul(s, x[2]); } g[0] = f2_fma(v, x[2], g[0]); g[2] = f2_fma(v, x[0], g[2]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(20), adj[0]); g[3] = f2_fma(s, p, g[3]); v = f2_mul(s, x[3]); } g[0] = f2_fma(v, x[3], g[0]); g[3] = f2_fma(v, x[0], g[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(21), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[0] = f2_fma(v, x[4], g[0]); g[4] = f2_fma(v, x[0], g[4]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(22), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[0] = f2_fma(v, x[5], g[0]); g[5] = f2_fma(v, x[0], g[5]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(23), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_mul(s, x[6]); } g[0] = f2_fma(v, x[6], g[0]); g[6] = f2_fma(v, x[0], g[6]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(24), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[0] = f2_fma(v, x[7], g[0]); g[7] = f2_fma(v, x[0], g[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(25), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[0] = f2_fma(v, x[8], g[0]); g[8] = f2_fma(v, x[0], g[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(26), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[0] = f2_fma(v, x[9], g[0]); g[9] = f2_fma(v, x[0], g[9]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(27), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[0] = f2_fma(v, x[10], g[0]); g[10] = f2_fma(v, x[0], g[10]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(28), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[0] = f2_fma(v, x[11], g[0]); g[11] = f2_fma(v, x[0], g[11]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(29), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[0] = f2_fma(v, x[12], g[0]); g[12] = f2_fma(v, x[0], g[12]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(30), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[0] = f2_fma(v, x[13], g[0]); g[13] = f2_fma(v, x[0], g[13]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(31), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[0] = f2_fma(v, x[14], g[0]); g[14] = f2_fma(v, x[0], g[14]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(32), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[0] = f2_fma(v, x[15], g[0]); g[15] = f2_fma(v, x[0], g[15]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); unsigned long long v; v = f2_mul(W(2), adj[0]); { const unsigned long long s = f2_mul(W(33), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(34), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[1] = f2_fma(v, x[1], g[1]); g[1] = f2_fma(v, x[1], g[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(35), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[1] = f2_fma(v, x[2], g[1]); g[2] = f2_fma(v, x[1], g[2]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(36), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[1] = f2_fma(v, x[3], g[1]); g[3] = f2_fma(v, x[1], g[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(37), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(38), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[4], g[1]); g[4] = f2_fma(v, x[1], g[4]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(39), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(40), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[5], g[1]); g[5] = f2_fma(v, x[1], g[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(41), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[1] = f2_fma(v, x[6], g[1]); g[6] = f2_fma(v, x[1], g[6]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(42), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[1] = f2_fma(v, x[7], g[1]); g[7] = f2_fma(v, x[1], g[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(43), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(44), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[1] = f2_fma(v, x[8], g[1]); g[8] = f2_fma(v, x[1], g[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); unsigned long long v; v = f2_mul(W(3), adj[0]); { const unsigned long long s = f2_mul(W(45), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[2] = f2_fma(v, x[2], g[2]); g[2] = f2_fma(v, x[2], g[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(46), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[2] = f2_fma(v, x[3], g[2]); g[3] = f2_fma(v, x[2], g[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(47), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[2] = f2_fma(v, x[4], g[2]); g[4] = f2_fma(v, x[2], g[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(48), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[2] = f2_fma(v, x[5], g[2]); g[5] = f2_fma(v, x[2], g[5]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(49), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[2] = f2_fma(v, x[6], g[2]); g[6] = f2_fma(v, x[2], g[6]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(50), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[2] = f2_fma(v, x[7], g[2]); g[7] = f2_fma(v, x[2], g[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(51), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[2] = f2_fma(v, x[8], g[2]); g[8] = f2_fma(v, x[2], g[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); unsigned long long v; v = f2_mul(W(4), adj[0]); { const unsigned long long s = f2_mul(W(52), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(53), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[3] = f2_fma(v, x[3], g[3]); g[3] = f2_fma(v, x[3], g[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(54), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(55), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[3] = f2_fma(v, x[4], g[3]); g[4] = f2_fma(v, x[3], g[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(56), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[3] = f2_fma(v, x[5], g[3]); g[5] = f2_fma(v, x[3], g[5]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(57), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[3] = f2_fma(v, x[6], g[3]); g[6] = f2_fma(v, x[3], g[6]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(58), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(59), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[7], g[3]); g[7] = f2_fma(v, x[3], g[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(60), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(61), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[8], g[3]); g[8] = f2_fma(v, x[3], g[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); unsigned long long v; v = f2_mul(W(5), adj[0]); { const unsigned long long s = f2_mul(W(62), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[4] = f2_fma(v, x[4], g[4]); g[4] = f2_fma(v, x[4], g[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(63), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[4] = f2_fma(v, x[5], g[4]); g[5] = f2_fma(v, x[4], g[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(64), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[4] = f2_fma(v, x[9], g[4]); g[9] = f2_fma(v, x[4], g[9]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(65), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[4] = f2_fma(v, x[10], g[4]); g[10] = f2_fma(v, x[4], g[10]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(66), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(67), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[11], g[4]); g[11] = f2_fma(v, x[4], g[11]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); unsigned long long v; v = f2_mul(W(6), adj[0]); { const unsigned long long s = f2_mul(W(68), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(69), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[5] = f2_fma(v, x[5], g[5]); g[5] = f2_fma(v, x[5], g[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(70), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[5] = f2_fma(v, x[9], g[5]); g[9] = f2_fma(v, x[5], g[9]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(71), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(72), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[10], g[5]); g[10] = f2_fma(v, x[5], g[10]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(73), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(74), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[11], g[5]); g[11] = f2_fma(v, x[5], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); unsigned long long v; v = f2_mul(W(7), adj[0]); { const unsigned long long s = f2_mul(W(75), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[6] = f2_fma(v, x[6], g[6]); g[6] = f2_fma(v, x[6], g[6]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(76), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[6] = f2_fma(v, x[7], g[6]); g[7] = f2_fma(v, x[6], g[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(77), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[6] = f2_fma(v, x[8], g[6]); g[8] = f2_fma(v, x[6], g[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(78), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[6] = f2_fma(v, x[9], g[6]); g[9] = f2_fma(v, x[6], g[9]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(79), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[6] = f2_fma(v, x[11], g[6]); g[11] = f2_fma(v, x[6], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(80), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[6] = f2_fma(v, x[12], g[6]); g[12] = f2_fma(v, x[6], g[12]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(81), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[6] = f2_fma(v, x[13], g[6]); g[13] = f2_fma(v, x[6], g[13]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(82), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[6] = f2_fma(v, x[15], g[6]); g[15] = f2_fma(v, x[6], g[15]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); unsigned long long v; v = f2_mul(W(8), adj[0]); { const unsigned long long s = f2_mul(W(83), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[7] = f2_fma(v, x[7], g[7]); g[7] = f2_fma(v, x[7], g[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(84), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[7] = f2_fma(v, x[9], g[7]); g[9] = f2_fma(v, x[7], g[9]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(85), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[7] = f2_fma(v, x[10], g[7]); g[10] = f2_fma(v, x[7], g[10]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(86), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[7] = f2_fma(v, x[12], g[7]); g[12] = f2_fma(v, x[7], g[12]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(87), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[7] = f2_fma(v, x[13], g[7]); g[13] = f2_fma(v, x[7], g[13]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(88), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[7] = f2_fma(v, x[14], g[7]); g[14] = f2_fma(v, x[7], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(9), adj[0]); g[8] = f2_fma(v, x[8], g[8]); g[8] = f2_fma(v, x[8], g[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(89), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[9], g[8]); g[9] = f2_fma(v, x[8], g[9]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(90), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[11], g[8]); g[11] = f2_fma(v, x[8], g[11]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(91), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[8] = f2_fma(v, x[12], g[8]); g[12] = f2_fma(v, x[8], g[12]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(92), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(93), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[13], g[8]); g[13] = f2_fma(v, x[8], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(10), adj[0]); g[9] = f2_fma(v, x[9], g[9]); g[9] = f2_fma(v, x[9], g[9]); } \
+      { unsigned long long v; v = f2_mul(W(11), adj[0]); g[10] = f2_fma(v, x[10], g[10]); g[10] = f2_fma(v, x[10], g[10]); } \
+      { unsigned long long v; v = f2_mul(W(12), adj[0]); g[11] = f2_fma(v, x[11], g[11]); g[11] = f2_fma(v, x[11], g[11]); } \
+      { unsigned long long v; v = f2_mul(W(13), adj[0]); g[12] = f2_fma(v, x[12], g[12]); g[12] = f2_fma(v, x[12], g[12]); } \
+      { unsigned long long v; v = f2_mul(W(14), adj[0]); g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(15), adj[0]); g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(16), adj[0]); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
 #define SXB_S0_L1_FORWARD_BODY \
     { /* path 0: edge l=0, source l=0 -> l=0 */ \
       const float t0 = R[0] * h[0]; \
@@ -1047,6 +1343,412 @@
     X3(0, 91, 8, 12, 14) \
     X3(0, 92, 8, 13, 13) \
     X3(0, 93, 8, 13, 15)
+#define SXB_S1_M0_FORWARD_BODY \
+      o[0] = f2_fma(W(0), x[0], o[0]); \
+      o[1] = f2_fma(W(94), x[1], o[1]); \
+      o[2] = f2_fma(W(212), x[2], o[2]); \
+      o[3] = f2_fma(W(304), x[3], o[3]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); o[0] = f2_fma(p, f2_fma(W(17), x[0], W(1)), o[0]); o[1] = f2_fma(p, f2_mul(W(108), x[1]), o[1]); o[2] = f2_fma(p, f2_mul(W(222), x[2]), o[2]); o[3] = f2_fma(p, f2_mul(W(318), x[3]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); o[0] = f2_fma(p, f2_mul(W(18), x[1]), o[0]); o[1] = f2_fma(p, f2_fma(W(110), x[8], f2_fma(W(109), x[6], W(95))), o[1]); o[2] = f2_fma(p, f2_mul(W(223), x[5]), o[2]); o[3] = f2_fma(p, f2_mul(W(319), x[4]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); o[0] = f2_fma(p, f2_mul(W(19), x[2]), o[0]); o[1] = f2_fma(p, f2_mul(W(111), x[5]), o[1]); o[2] = f2_fma(p, f2_fma(W(224), x[6], W(213)), o[2]); o[3] = f2_fma(p, f2_mul(W(320), x[7]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); o[0] = f2_fma(p, f2_mul(W(20), x[3]), o[0]); o[1] = f2_fma(p, f2_mul(W(112), x[4]), o[1]); o[2] = f2_fma(p, f2_mul(W(225), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(322), x[8], f2_fma(W(321), x[6], W(305))), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); o[0] = f2_fma(p, f2_mul(W(21), x[4]), o[0]); o[1] = f2_fma(p, f2_fma(W(114), x[15], f2_mul(W(113), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(226), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(324), x[11], f2_mul(W(323), x[9])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); o[0] = f2_fma(p, f2_mul(W(22), x[5]), o[0]); o[1] = f2_fma(p, f2_fma(W(116), x[14], f2_mul(W(115), x[12])), o[1]); o[2] = f2_fma(p, f2_mul(W(227), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(325), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); o[0] = f2_fma(p, f2_mul(W(23), x[6]), o[0]); o[1] = f2_fma(p, f2_mul(W(117), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(228), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(326), x[13]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); o[0] = f2_fma(p, f2_mul(W(24), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(118), x[10]), o[1]); o[2] = f2_fma(p, f2_mul(W(229), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(328), x[14], f2_mul(W(327), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); o[0] = f2_fma(p, f2_mul(W(25), x[8]), o[0]); o[1] = f2_fma(p, f2_fma(W(120), x[11], f2_mul(W(119), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(230), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(330), x[15], f2_mul(W(329), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); o[0] = f2_fma(p, f2_mul(W(26), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); o[0] = f2_fma(p, f2_mul(W(27), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); o[0] = f2_fma(p, f2_mul(W(28), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); o[0] = f2_fma(p, f2_mul(W(29), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); o[0] = f2_fma(p, f2_mul(W(30), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); o[0] = f2_fma(p, f2_mul(W(31), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); o[0] = f2_fma(p, f2_mul(W(32), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); o[0] = f2_fma(p, f2_fma(W(34), x[8], f2_fma(W(33), x[6], W(2))), o[0]); o[1] = f2_fma(p, f2_fma(W(123), x[11], f2_fma(W(122), x[9], f2_mul(W(121), x[1]))), o[1]); o[2] = f2_fma(p, f2_fma(W(233), x[14], f2_fma(W(232), x[12], f2_mul(W(231), x[2]))), o[2]); o[3] = f2_fma(p, f2_fma(W(333), x[15], f2_fma(W(332), x[13], f2_mul(W(331), x[3]))), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); o[0] = f2_fma(p, f2_mul(W(35), x[5]), o[0]); o[1] = f2_fma(p, f2_fma(W(126), x[14], f2_fma(W(125), x[12], f2_mul(W(124), x[2]))), o[1]); o[2] = f2_fma(p, f2_mul(W(234), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(334), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); o[0] = f2_fma(p, f2_mul(W(36), x[4]), o[0]); o[1] = f2_fma(p, f2_fma(W(129), x[15], f2_fma(W(128), x[13], f2_mul(W(127), x[3]))), o[1]); o[2] = f2_fma(p, f2_mul(W(235), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(336), x[11], f2_mul(W(335), x[9])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); o[0] = f2_fma(p, f2_fma(W(38), x[15], f2_mul(W(37), x[13])), o[0]); o[1] = f2_fma(p, f2_mul(W(130), x[4]), o[1]); o[2] = f2_fma(p, f2_mul(W(236), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(338), x[8], f2_fma(W(337), x[6], W(306))), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); o[0] = f2_fma(p, f2_fma(W(40), x[14], f2_mul(W(39), x[12])), o[0]); o[1] = f2_fma(p, f2_mul(W(131), x[5]), o[1]); o[2] = f2_fma(p, f2_fma(W(238), x[8], f2_fma(W(237), x[6], W(214))), o[2]); o[3] = f2_fma(p, f2_mul(W(339), x[7]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); o[0] = f2_fma(p, f2_mul(W(41), x[11]), o[0]); o[1] = f2_fma(p, f2_fma(W(133), x[8], f2_fma(W(132), x[6], W(96))), o[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); o[0] = f2_fma(p, f2_mul(W(42), x[10]), o[0]); o[1] = f2_fma(p, f2_mul(W(134), x[7]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); o[0] = f2_fma(p, f2_fma(W(44), x[11], f2_mul(W(43), x[9])), o[0]); o[1] = f2_fma(p, f2_fma(W(135), x[8], W(97)), o[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[9]); o[1] = f2_fma(p, f2_fma(W(137), x[11], f2_mul(W(136), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(239), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(341), x[15], f2_mul(W(340), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[10]); o[1] = f2_fma(p, f2_mul(W(138), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(241), x[15], f2_mul(W(240), x[13])), o[2]); o[3] = f2_fma(p, f2_fma(W(343), x[14], f2_mul(W(342), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[11]); o[1] = f2_fma(p, f2_mul(W(139), x[11]), o[1]); o[2] = f2_fma(p, f2_fma(W(243), x[14], f2_mul(W(242), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(345), x[15], f2_mul(W(344), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[12]); o[1] = f2_fma(p, f2_fma(W(141), x[14], f2_mul(W(140), x[12])), o[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[13]); o[1] = f2_fma(p, f2_fma(W(143), x[15], f2_mul(W(142), x[13])), o[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[14]); o[1] = f2_fma(p, f2_mul(W(144), x[14]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[15]); o[1] = f2_fma(p, f2_mul(W(145), x[15]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); o[0] = f2_fma(p, f2_fma(W(45), x[6], W(3)), o[0]); o[1] = f2_fma(p, f2_mul(W(146), x[11]), o[1]); o[2] = f2_fma(p, f2_fma(W(245), x[12], f2_mul(W(244), x[2])), o[2]); o[3] = f2_fma(p, f2_fma(W(347), x[13], f2_mul(W(346), x[3])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); o[0] = f2_fma(p, f2_mul(W(46), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(147), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(247), x[13], f2_mul(W(246), x[3])), o[2]); o[3] = f2_fma(p, f2_fma(W(349), x[14], f2_mul(W(348), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); o[0] = f2_fma(p, f2_mul(W(47), x[10]), o[0]); o[1] = f2_fma(p, f2_mul(W(148), x[7]), o[1]); o[2] = f2_fma(p, f2_mul(W(248), x[4]), o[2]); o[3] = f2_fma(p, f2_mul(W(350), x[5]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); o[0] = f2_fma(p, f2_mul(W(48), x[11]), o[0]); o[1] = f2_fma(p, f2_fma(W(150), x[8], f2_fma(W(149), x[6], W(98))), o[1]); o[2] = f2_fma(p, f2_mul(W(249), x[5]), o[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); o[0] = f2_fma(p, f2_mul(W(49), x[12]), o[0]); o[2] = f2_fma(p, f2_fma(W(250), x[6], W(215)), o[2]); o[3] = f2_fma(p, f2_mul(W(351), x[7]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); o[0] = f2_fma(p, f2_mul(W(50), x[13]), o[0]); o[2] = f2_fma(p, f2_mul(W(251), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(352), x[8], W(307)), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); o[0] = f2_fma(p, f2_mul(W(51), x[14]), o[0]); o[2] = f2_fma(p, f2_mul(W(252), x[8]), o[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[9]); o[1] = f2_fma(p, f2_mul(W(151), x[14]), o[1]); o[2] = f2_fma(p, f2_mul(W(253), x[9]), o[2]); o[3] = f2_fma(p, f2_mul(W(353), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[10]); o[1] = f2_fma(p, f2_fma(W(153), x[15], f2_mul(W(152), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(254), x[10]), o[2]); o[3] = f2_fma(p, f2_mul(W(354), x[11]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[11]); o[1] = f2_fma(p, f2_fma(W(155), x[14], f2_mul(W(154), x[12])), o[1]); o[2] = f2_fma(p, f2_mul(W(255), x[11]), o[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[12]); o[2] = f2_fma(p, f2_mul(W(256), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(355), x[13]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[13]); o[2] = f2_fma(p, f2_mul(W(257), x[13]), o[2]); o[3] = f2_fma(p, f2_mul(W(356), x[14]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[14]); o[2] = f2_fma(p, f2_mul(W(258), x[14]), o[2]); o[3] = f2_fma(p, f2_mul(W(357), x[15]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[15]); o[2] = f2_fma(p, f2_mul(W(259), x[15]), o[2]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); o[0] = f2_fma(p, f2_fma(W(53), x[8], f2_fma(W(52), x[6], W(4))), o[0]); o[1] = f2_fma(p, f2_fma(W(157), x[11], f2_mul(W(156), x[9])), o[1]); o[2] = f2_fma(p, f2_fma(W(261), x[14], f2_mul(W(260), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(360), x[15], f2_fma(W(359), x[13], f2_mul(W(358), x[3]))), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); o[0] = f2_fma(p, f2_fma(W(55), x[11], f2_mul(W(54), x[9])), o[0]); o[1] = f2_fma(p, f2_fma(W(159), x[8], f2_fma(W(158), x[6], W(99))), o[1]); o[2] = f2_fma(p, f2_mul(W(262), x[5]), o[2]); o[3] = f2_fma(p, f2_mul(W(361), x[4]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); o[0] = f2_fma(p, f2_mul(W(56), x[10]), o[0]); o[1] = f2_fma(p, f2_mul(W(160), x[7]), o[1]); o[3] = f2_fma(p, f2_mul(W(362), x[5]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); o[0] = f2_fma(p, f2_mul(W(57), x[13]), o[0]); o[2] = f2_fma(p, f2_mul(W(263), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(364), x[8], f2_fma(W(363), x[6], W(308))), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); o[0] = f2_fma(p, f2_fma(W(59), x[14], f2_mul(W(58), x[12])), o[0]); o[2] = f2_fma(p, f2_fma(W(264), x[8], W(216)), o[2]); o[3] = f2_fma(p, f2_mul(W(365), x[7]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); o[0] = f2_fma(p, f2_fma(W(61), x[15], f2_mul(W(60), x[13])), o[0]); o[3] = f2_fma(p, f2_fma(W(366), x[8], W(309)), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[9]); o[1] = f2_fma(p, f2_fma(W(162), x[15], f2_mul(W(161), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(265), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(368), x[11], f2_mul(W(367), x[9])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[10]); o[1] = f2_fma(p, f2_fma(W(164), x[14], f2_mul(W(163), x[12])), o[1]); o[2] = f2_fma(p, f2_mul(W(266), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(369), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[11]); o[1] = f2_fma(p, f2_fma(W(166), x[15], f2_mul(W(165), x[13])), o[1]); o[3] = f2_fma(p, f2_mul(W(370), x[11]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[12]); o[2] = f2_fma(p, f2_mul(W(267), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(372), x[14], f2_mul(W(371), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[13]); o[2] = f2_fma(p, f2_mul(W(268), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(374), x[15], f2_mul(W(373), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[14]); o[2] = f2_fma(p, f2_mul(W(269), x[15]), o[2]); o[3] = f2_fma(p, f2_mul(W(375), x[14]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[15]); o[3] = f2_fma(p, f2_mul(W(376), x[15]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); o[0] = f2_fma(p, f2_fma(W(62), x[6], W(5)), o[0]); o[1] = f2_fma(p, f2_fma(W(168), x[11], f2_mul(W(167), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(270), x[12]), o[2]); o[3] = f2_fma(p, f2_fma(W(378), x[15], f2_mul(W(377), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); o[0] = f2_fma(p, f2_mul(W(63), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(169), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(272), x[15], f2_mul(W(271), x[13])), o[2]); o[3] = f2_fma(p, f2_fma(W(380), x[14], f2_mul(W(379), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[6]); o[1] = f2_fma(p, f2_fma(W(171), x[15], f2_mul(W(170), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(273), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(382), x[11], f2_mul(W(381), x[9])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[7]); o[1] = f2_fma(p, f2_fma(W(173), x[14], f2_mul(W(172), x[12])), o[1]); o[2] = f2_fma(p, f2_fma(W(275), x[11], f2_mul(W(274), x[9])), o[2]); o[3] = f2_fma(p, f2_mul(W(383), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[8]); o[1] = f2_fma(p, f2_fma(W(175), x[15], f2_mul(W(174), x[13])), o[1]); o[3] = f2_fma(p, f2_fma(W(385), x[11], f2_mul(W(384), x[9])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); o[0] = f2_fma(p, f2_mul(W(64), x[13]), o[0]); o[3] = f2_fma(p, W(310), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); o[0] = f2_fma(p, f2_mul(W(65), x[12]), o[0]); o[2] = f2_fma(p, W(217), o[2]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); o[0] = f2_fma(p, f2_fma(W(67), x[15], f2_mul(W(66), x[13])), o[0]); o[3] = f2_fma(p, W(311), o[3]); } \
+      { const unsigned long long p = f2_mul(x[4], x[13]); o[1] = f2_fma(p, W(100), o[1]); } \
+      { const unsigned long long p = f2_mul(x[4], x[15]); o[1] = f2_fma(p, W(101), o[1]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); o[0] = f2_fma(p, f2_fma(W(69), x[8], f2_fma(W(68), x[6], W(6))), o[0]); o[1] = f2_fma(p, f2_fma(W(177), x[11], f2_mul(W(176), x[9])), o[1]); o[2] = f2_fma(p, f2_fma(W(277), x[14], f2_mul(W(276), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(387), x[15], f2_mul(W(386), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[5], x[6]); o[1] = f2_fma(p, f2_fma(W(179), x[14], f2_mul(W(178), x[12])), o[1]); o[2] = f2_fma(p, f2_mul(W(278), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(388), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[5], x[7]); o[1] = f2_fma(p, f2_fma(W(181), x[15], f2_mul(W(180), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(279), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(390), x[11], f2_mul(W(389), x[9])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[5], x[8]); o[1] = f2_fma(p, f2_fma(W(183), x[14], f2_mul(W(182), x[12])), o[1]); o[2] = f2_fma(p, f2_fma(W(281), x[11], f2_mul(W(280), x[9])), o[2]); o[3] = f2_fma(p, f2_mul(W(391), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); o[0] = f2_fma(p, f2_mul(W(70), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); o[0] = f2_fma(p, f2_fma(W(72), x[15], f2_mul(W(71), x[13])), o[0]); o[3] = f2_fma(p, W(312), o[3]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); o[0] = f2_fma(p, f2_fma(W(74), x[14], f2_mul(W(73), x[12])), o[0]); o[2] = f2_fma(p, W(218), o[2]); } \
+      { const unsigned long long p = f2_mul(x[5], x[12]); o[1] = f2_fma(p, W(102), o[1]); } \
+      { const unsigned long long p = f2_mul(x[5], x[14]); o[1] = f2_fma(p, W(103), o[1]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); o[0] = f2_fma(p, f2_fma(W(75), x[6], W(7)), o[0]); o[1] = f2_fma(p, f2_mul(W(184), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(282), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(392), x[13]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); o[0] = f2_fma(p, f2_mul(W(76), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(185), x[10]), o[1]); o[2] = f2_fma(p, f2_mul(W(283), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(394), x[14], f2_mul(W(393), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); o[0] = f2_fma(p, f2_mul(W(77), x[8]), o[0]); o[1] = f2_fma(p, f2_fma(W(187), x[11], f2_mul(W(186), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(284), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(396), x[15], f2_mul(W(395), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); o[0] = f2_fma(p, f2_mul(W(78), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); o[0] = f2_fma(p, f2_mul(W(79), x[11]), o[0]); o[1] = f2_fma(p, W(104), o[1]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); o[0] = f2_fma(p, f2_mul(W(80), x[12]), o[0]); o[2] = f2_fma(p, W(219), o[2]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); o[0] = f2_fma(p, f2_mul(W(81), x[13]), o[0]); o[3] = f2_fma(p, W(313), o[3]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); o[0] = f2_fma(p, f2_mul(W(82), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); o[0] = f2_fma(p, f2_fma(W(83), x[8], W(8)), o[0]); o[1] = f2_fma(p, f2_fma(W(189), x[11], f2_mul(W(188), x[9])), o[1]); o[2] = f2_fma(p, f2_fma(W(286), x[14], f2_mul(W(285), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(398), x[15], f2_mul(W(397), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[7], x[8]); o[1] = f2_fma(p, f2_mul(W(190), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(288), x[15], f2_mul(W(287), x[13])), o[2]); o[3] = f2_fma(p, f2_fma(W(400), x[14], f2_mul(W(399), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); o[0] = f2_fma(p, f2_mul(W(84), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); o[0] = f2_fma(p, f2_mul(W(85), x[11]), o[0]); o[1] = f2_fma(p, W(105), o[1]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); o[0] = f2_fma(p, f2_mul(W(86), x[13]), o[0]); o[3] = f2_fma(p, W(314), o[3]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); o[0] = f2_fma(p, f2_mul(W(87), x[14]), o[0]); o[2] = f2_fma(p, W(220), o[2]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); o[0] = f2_fma(p, f2_mul(W(88), x[15]), o[0]); o[3] = f2_fma(p, W(315), o[3]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); o[0] = f2_fma(p, W(9), o[0]); o[1] = f2_fma(p, f2_fma(W(192), x[11], f2_mul(W(191), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(289), x[12]), o[2]); o[3] = f2_fma(p, f2_fma(W(402), x[15], f2_mul(W(401), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); o[0] = f2_fma(p, f2_mul(W(89), x[11]), o[0]); o[1] = f2_fma(p, W(106), o[1]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); o[0] = f2_fma(p, f2_mul(W(90), x[11]), o[0]); o[1] = f2_fma(p, W(107), o[1]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); o[0] = f2_fma(p, f2_mul(W(91), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); o[0] = f2_fma(p, f2_fma(W(93), x[15], f2_mul(W(92), x[13])), o[0]); o[3] = f2_fma(p, W(316), o[3]); } \
+      { const unsigned long long p = f2_mul(x[8], x[14]); o[2] = f2_fma(p, W(221), o[2]); } \
+      { const unsigned long long p = f2_mul(x[8], x[15]); o[3] = f2_fma(p, W(317), o[3]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); o[0] = f2_fma(p, W(10), o[0]); o[1] = f2_fma(p, f2_mul(W(193), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(290), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(403), x[13]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[9], x[10]); o[1] = f2_fma(p, f2_mul(W(194), x[10]), o[1]); o[2] = f2_fma(p, f2_mul(W(291), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(405), x[14], f2_mul(W(404), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[9], x[11]); o[1] = f2_fma(p, f2_mul(W(195), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(292), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(407), x[15], f2_mul(W(406), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[9], x[12]); o[1] = f2_fma(p, f2_mul(W(196), x[14]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[9], x[13]); o[1] = f2_fma(p, f2_fma(W(198), x[15], f2_mul(W(197), x[13])), o[1]); } \
+      { const unsigned long long p = f2_mul(x[9], x[14]); o[1] = f2_fma(p, f2_mul(W(199), x[14]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); o[0] = f2_fma(p, W(11), o[0]); o[1] = f2_fma(p, f2_mul(W(200), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(293), x[12]), o[2]); o[3] = f2_fma(p, f2_fma(W(409), x[15], f2_mul(W(408), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[10], x[11]); o[2] = f2_fma(p, f2_fma(W(295), x[15], f2_mul(W(294), x[13])), o[2]); o[3] = f2_fma(p, f2_fma(W(411), x[14], f2_mul(W(410), x[12])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[10], x[12]); o[1] = f2_fma(p, f2_fma(W(202), x[15], f2_mul(W(201), x[13])), o[1]); } \
+      { const unsigned long long p = f2_mul(x[10], x[13]); o[1] = f2_fma(p, f2_mul(W(203), x[14]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[10], x[14]); o[1] = f2_fma(p, f2_mul(W(204), x[15]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); o[0] = f2_fma(p, W(12), o[0]); o[1] = f2_fma(p, f2_mul(W(205), x[11]), o[1]); o[2] = f2_fma(p, f2_fma(W(297), x[14], f2_mul(W(296), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(413), x[15], f2_mul(W(412), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[11], x[12]); o[1] = f2_fma(p, f2_fma(W(207), x[14], f2_mul(W(206), x[12])), o[1]); } \
+      { const unsigned long long p = f2_mul(x[11], x[13]); o[1] = f2_fma(p, f2_fma(W(209), x[15], f2_mul(W(208), x[13])), o[1]); } \
+      { const unsigned long long p = f2_mul(x[11], x[14]); o[1] = f2_fma(p, f2_mul(W(210), x[14]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[11], x[15]); o[1] = f2_fma(p, f2_mul(W(211), x[15]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); o[0] = f2_fma(p, W(13), o[0]); o[2] = f2_fma(p, f2_mul(W(298), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(414), x[13]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[12], x[13]); o[2] = f2_fma(p, f2_mul(W(299), x[13]), o[2]); o[3] = f2_fma(p, f2_mul(W(415), x[14]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[12], x[14]); o[2] = f2_fma(p, f2_mul(W(300), x[14]), o[2]); o[3] = f2_fma(p, f2_mul(W(416), x[15]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[12], x[15]); o[2] = f2_fma(p, f2_mul(W(301), x[15]), o[2]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); o[0] = f2_fma(p, W(14), o[0]); o[2] = f2_fma(p, f2_mul(W(302), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(418), x[15], f2_mul(W(417), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[13], x[14]); o[2] = f2_fma(p, f2_mul(W(303), x[15]), o[2]); o[3] = f2_fma(p, f2_mul(W(419), x[14]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[13], x[15]); o[3] = f2_fma(p, f2_mul(W(420), x[15]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); o[0] = f2_fma(p, W(15), o[0]); o[3] = f2_fma(p, f2_mul(W(421), x[15]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[15], x[15]); o[0] = f2_fma(p, W(16), o[0]); }
+#define SXB_S1_M0_REVERSE_BODY \
+      g[0] = f2_fma(W(0), adj[0], g[0]); \
+      g[1] = f2_fma(W(94), adj[1], g[1]); \
+      g[2] = f2_fma(W(212), adj[2], g[2]); \
+      g[3] = f2_fma(W(304), adj[3], g[3]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); unsigned long long v; v = f2_mul(W(1), adj[0]); { const unsigned long long s = f2_mul(W(17), adj[0]); g[0] = f2_fma(s, p, g[0]); v = f2_fma(s, x[0], v); } { const unsigned long long s = f2_mul(W(108), adj[1]); g[1] = f2_fma(s, p, g[1]); v = f2_fma(s, x[1], v); } { const unsigned long long s = f2_mul(W(222), adj[2]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(318), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } g[0] = f2_fma(v, x[0], g[0]); g[0] = f2_fma(v, x[0], g[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); unsigned long long v; v = f2_mul(W(95), adj[1]); { const unsigned long long s = f2_mul(W(18), adj[0]); g[1] = f2_fma(s, p, g[1]); v = f2_fma(s, x[1], v); } { const unsigned long long s = f2_mul(W(319), adj[3]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(223), adj[2]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(109), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(110), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[0] = f2_fma(v, x[1], g[0]); g[1] = f2_fma(v, x[0], g[1]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); unsigned long long v; v = f2_mul(W(213), adj[2]); { const unsigned long long s = f2_mul(W(19), adj[0]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(111), adj[1]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(224), adj[2]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(320), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } g[0] = f2_fma(v, x[2], g[0]); g[2] = f2_fma(v, x[0], g[2]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); unsigned long long v; v = f2_mul(W(305), adj[3]); { const unsigned long long s = f2_mul(W(20), adj[0]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(112), adj[1]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(321), adj[3]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(225), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(322), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[0] = f2_fma(v, x[3], g[0]); g[3] = f2_fma(v, x[0], g[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(21), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } { const unsigned long long s = f2_mul(W(323), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(226), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(324), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(113), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(114), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[4], g[0]); g[4] = f2_fma(v, x[0], g[4]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(22), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } { const unsigned long long s = f2_mul(W(325), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(227), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(115), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(116), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[0] = f2_fma(v, x[5], g[0]); g[5] = f2_fma(v, x[0], g[5]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(23), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_mul(s, x[6]); } { const unsigned long long s = f2_mul(W(117), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(228), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(326), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[0] = f2_fma(v, x[6], g[0]); g[6] = f2_fma(v, x[0], g[6]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(24), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } { const unsigned long long s = f2_mul(W(118), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(327), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(229), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(328), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[0] = f2_fma(v, x[7], g[0]); g[7] = f2_fma(v, x[0], g[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(25), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } { const unsigned long long s = f2_mul(W(119), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(120), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(329), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(230), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(330), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[8], g[0]); g[8] = f2_fma(v, x[0], g[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(26), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[0] = f2_fma(v, x[9], g[0]); g[9] = f2_fma(v, x[0], g[9]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(27), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[0] = f2_fma(v, x[10], g[0]); g[10] = f2_fma(v, x[0], g[10]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(28), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[0] = f2_fma(v, x[11], g[0]); g[11] = f2_fma(v, x[0], g[11]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(29), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[0] = f2_fma(v, x[12], g[0]); g[12] = f2_fma(v, x[0], g[12]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(30), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[0] = f2_fma(v, x[13], g[0]); g[13] = f2_fma(v, x[0], g[13]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(31), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[0] = f2_fma(v, x[14], g[0]); g[14] = f2_fma(v, x[0], g[14]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(32), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[0] = f2_fma(v, x[15], g[0]); g[15] = f2_fma(v, x[0], g[15]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); unsigned long long v; v = f2_mul(W(2), adj[0]); { const unsigned long long s = f2_mul(W(121), adj[1]); g[1] = f2_fma(s, p, g[1]); v = f2_fma(s, x[1], v); } { const unsigned long long s = f2_mul(W(231), adj[2]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(331), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(33), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(34), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(122), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(123), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(232), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(332), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(233), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(333), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[1], g[1]); g[1] = f2_fma(v, x[1], g[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(124), adj[1]); g[2] = f2_fma(s, p, g[2]); v = f2_mul(s, x[2]); } { const unsigned long long s = f2_mul(W(35), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(334), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(234), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(125), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(126), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[2], g[1]); g[2] = f2_fma(v, x[1], g[2]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(127), adj[1]); g[3] = f2_fma(s, p, g[3]); v = f2_mul(s, x[3]); } { const unsigned long long s = f2_mul(W(36), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(335), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(235), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(336), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(128), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(129), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[3], g[1]); g[3] = f2_fma(v, x[1], g[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); unsigned long long v; v = f2_mul(W(306), adj[3]); { const unsigned long long s = f2_mul(W(130), adj[1]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(337), adj[3]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(236), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(338), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(37), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(38), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[4], g[1]); g[4] = f2_fma(v, x[1], g[4]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); unsigned long long v; v = f2_mul(W(214), adj[2]); { const unsigned long long s = f2_mul(W(131), adj[1]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(237), adj[2]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(339), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(238), adj[2]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(39), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(40), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[5], g[1]); g[5] = f2_fma(v, x[1], g[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); unsigned long long v; v = f2_mul(W(96), adj[1]); { const unsigned long long s = f2_mul(W(132), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(133), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(41), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[1] = f2_fma(v, x[6], g[1]); g[6] = f2_fma(v, x[1], g[6]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(134), adj[1]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } { const unsigned long long s = f2_mul(W(42), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } g[1] = f2_fma(v, x[7], g[1]); g[7] = f2_fma(v, x[1], g[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); unsigned long long v; v = f2_mul(W(97), adj[1]); { const unsigned long long s = f2_mul(W(135), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(43), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(44), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[1] = f2_fma(v, x[8], g[1]); g[8] = f2_fma(v, x[1], g[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(136), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(137), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(340), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(239), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(341), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[9], g[1]); g[9] = f2_fma(v, x[1], g[9]); } \
+      { const unsigned long long p = f2_mul(x[1], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(138), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(342), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(240), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(343), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(241), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[10], g[1]); g[10] = f2_fma(v, x[1], g[10]); } \
+      { const unsigned long long p = f2_mul(x[1], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(139), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } { const unsigned long long s = f2_mul(W(242), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(344), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(243), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(345), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[11], g[1]); g[11] = f2_fma(v, x[1], g[11]); } \
+      { const unsigned long long p = f2_mul(x[1], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(140), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(141), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[12], g[1]); g[12] = f2_fma(v, x[1], g[12]); } \
+      { const unsigned long long p = f2_mul(x[1], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(142), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(143), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[13], g[1]); g[13] = f2_fma(v, x[1], g[13]); } \
+      { const unsigned long long p = f2_mul(x[1], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(144), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[1] = f2_fma(v, x[14], g[1]); g[14] = f2_fma(v, x[1], g[14]); } \
+      { const unsigned long long p = f2_mul(x[1], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(145), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[1] = f2_fma(v, x[15], g[1]); g[15] = f2_fma(v, x[1], g[15]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); unsigned long long v; v = f2_mul(W(3), adj[0]); { const unsigned long long s = f2_mul(W(244), adj[2]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(346), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(45), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(146), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(245), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(347), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[2] = f2_fma(v, x[2], g[2]); g[2] = f2_fma(v, x[2], g[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(246), adj[2]); g[3] = f2_fma(s, p, g[3]); v = f2_mul(s, x[3]); } { const unsigned long long s = f2_mul(W(46), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(147), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(348), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(247), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(349), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[3], g[2]); g[3] = f2_fma(v, x[2], g[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(248), adj[2]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } { const unsigned long long s = f2_mul(W(350), adj[3]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(148), adj[1]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(47), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } g[2] = f2_fma(v, x[4], g[2]); g[4] = f2_fma(v, x[2], g[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); unsigned long long v; v = f2_mul(W(98), adj[1]); { const unsigned long long s = f2_mul(W(249), adj[2]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(149), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(150), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(48), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[2] = f2_fma(v, x[5], g[2]); g[5] = f2_fma(v, x[2], g[5]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); unsigned long long v; v = f2_mul(W(215), adj[2]); { const unsigned long long s = f2_mul(W(250), adj[2]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(351), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(49), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } g[2] = f2_fma(v, x[6], g[2]); g[6] = f2_fma(v, x[2], g[6]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); unsigned long long v; v = f2_mul(W(307), adj[3]); { const unsigned long long s = f2_mul(W(251), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(352), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(50), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[2] = f2_fma(v, x[7], g[2]); g[7] = f2_fma(v, x[2], g[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(252), adj[2]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } { const unsigned long long s = f2_mul(W(51), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[8], g[2]); g[8] = f2_fma(v, x[2], g[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(253), adj[2]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(353), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(151), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[9], g[2]); g[9] = f2_fma(v, x[2], g[9]); } \
+      { const unsigned long long p = f2_mul(x[2], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(254), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(354), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(152), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(153), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[10], g[2]); g[10] = f2_fma(v, x[2], g[10]); } \
+      { const unsigned long long p = f2_mul(x[2], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(255), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } { const unsigned long long s = f2_mul(W(154), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(155), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[11], g[2]); g[11] = f2_fma(v, x[2], g[11]); } \
+      { const unsigned long long p = f2_mul(x[2], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(256), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(355), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[2] = f2_fma(v, x[12], g[2]); g[12] = f2_fma(v, x[2], g[12]); } \
+      { const unsigned long long p = f2_mul(x[2], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(257), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(356), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[13], g[2]); g[13] = f2_fma(v, x[2], g[13]); } \
+      { const unsigned long long p = f2_mul(x[2], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(258), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } { const unsigned long long s = f2_mul(W(357), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[14], g[2]); g[14] = f2_fma(v, x[2], g[14]); } \
+      { const unsigned long long p = f2_mul(x[2], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(259), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[2] = f2_fma(v, x[15], g[2]); g[15] = f2_fma(v, x[2], g[15]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); unsigned long long v; v = f2_mul(W(4), adj[0]); { const unsigned long long s = f2_mul(W(358), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(52), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(53), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(156), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(157), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(260), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(359), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(261), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(360), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[3], g[3]); g[3] = f2_fma(v, x[3], g[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); unsigned long long v; v = f2_mul(W(99), adj[1]); { const unsigned long long s = f2_mul(W(361), adj[3]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(262), adj[2]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(158), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(159), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(54), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(55), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[3] = f2_fma(v, x[4], g[3]); g[4] = f2_fma(v, x[3], g[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(362), adj[3]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } { const unsigned long long s = f2_mul(W(160), adj[1]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(56), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } g[3] = f2_fma(v, x[5], g[3]); g[5] = f2_fma(v, x[3], g[5]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); unsigned long long v; v = f2_mul(W(308), adj[3]); { const unsigned long long s = f2_mul(W(363), adj[3]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(263), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(364), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(57), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[3] = f2_fma(v, x[6], g[3]); g[6] = f2_fma(v, x[3], g[6]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); unsigned long long v; v = f2_mul(W(216), adj[2]); { const unsigned long long s = f2_mul(W(365), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(264), adj[2]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(58), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(59), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[7], g[3]); g[7] = f2_fma(v, x[3], g[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); unsigned long long v; v = f2_mul(W(309), adj[3]); { const unsigned long long s = f2_mul(W(366), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(60), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(61), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[8], g[3]); g[8] = f2_fma(v, x[3], g[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(367), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(265), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(368), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(161), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(162), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[9], g[3]); g[9] = f2_fma(v, x[3], g[9]); } \
+      { const unsigned long long p = f2_mul(x[3], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(369), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(266), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(163), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(164), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[10], g[3]); g[10] = f2_fma(v, x[3], g[10]); } \
+      { const unsigned long long p = f2_mul(x[3], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(370), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } { const unsigned long long s = f2_mul(W(165), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(166), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[11], g[3]); g[11] = f2_fma(v, x[3], g[11]); } \
+      { const unsigned long long p = f2_mul(x[3], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(371), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(267), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(372), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[12], g[3]); g[12] = f2_fma(v, x[3], g[12]); } \
+      { const unsigned long long p = f2_mul(x[3], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(373), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(268), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(374), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[13], g[3]); g[13] = f2_fma(v, x[3], g[13]); } \
+      { const unsigned long long p = f2_mul(x[3], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(375), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } { const unsigned long long s = f2_mul(W(269), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[14], g[3]); g[14] = f2_fma(v, x[3], g[14]); } \
+      { const unsigned long long p = f2_mul(x[3], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(376), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[3] = f2_fma(v, x[15], g[3]); g[15] = f2_fma(v, x[3], g[15]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); unsigned long long v; v = f2_mul(W(5), adj[0]); { const unsigned long long s = f2_mul(W(62), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(167), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(168), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(270), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(377), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(378), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[4], g[4]); g[4] = f2_fma(v, x[4], g[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(63), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } { const unsigned long long s = f2_mul(W(169), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(379), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(271), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(380), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(272), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[5], g[4]); g[5] = f2_fma(v, x[4], g[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(381), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(273), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(382), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(170), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(171), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[6], g[4]); g[6] = f2_fma(v, x[4], g[6]); } \
+      { const unsigned long long p = f2_mul(x[4], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(274), adj[2]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(383), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(275), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(172), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(173), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[4] = f2_fma(v, x[7], g[4]); g[7] = f2_fma(v, x[4], g[7]); } \
+      { const unsigned long long p = f2_mul(x[4], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(384), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(385), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(174), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(175), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[8], g[4]); g[8] = f2_fma(v, x[4], g[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); unsigned long long v; v = f2_mul(W(310), adj[3]); { const unsigned long long s = f2_mul(W(64), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[4] = f2_fma(v, x[9], g[4]); g[9] = f2_fma(v, x[4], g[9]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); unsigned long long v; v = f2_mul(W(217), adj[2]); { const unsigned long long s = f2_mul(W(65), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } g[4] = f2_fma(v, x[10], g[4]); g[10] = f2_fma(v, x[4], g[10]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); unsigned long long v; v = f2_mul(W(311), adj[3]); { const unsigned long long s = f2_mul(W(66), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(67), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[11], g[4]); g[11] = f2_fma(v, x[4], g[11]); } \
+      { unsigned long long v; v = f2_mul(W(100), adj[1]); g[4] = f2_fma(v, x[13], g[4]); g[13] = f2_fma(v, x[4], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(101), adj[1]); g[4] = f2_fma(v, x[15], g[4]); g[15] = f2_fma(v, x[4], g[15]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); unsigned long long v; v = f2_mul(W(6), adj[0]); { const unsigned long long s = f2_mul(W(68), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(69), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(176), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(177), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(276), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(386), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(277), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(387), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[5], g[5]); g[5] = f2_fma(v, x[5], g[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(388), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(278), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(178), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(179), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[6], g[5]); g[6] = f2_fma(v, x[5], g[6]); } \
+      { const unsigned long long p = f2_mul(x[5], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(389), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(279), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(390), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(180), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(181), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[7], g[5]); g[7] = f2_fma(v, x[5], g[7]); } \
+      { const unsigned long long p = f2_mul(x[5], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(280), adj[2]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(391), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(281), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(182), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(183), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[8], g[5]); g[8] = f2_fma(v, x[5], g[8]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(70), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[5] = f2_fma(v, x[9], g[5]); g[9] = f2_fma(v, x[5], g[9]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); unsigned long long v; v = f2_mul(W(312), adj[3]); { const unsigned long long s = f2_mul(W(71), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(72), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[10], g[5]); g[10] = f2_fma(v, x[5], g[10]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); unsigned long long v; v = f2_mul(W(218), adj[2]); { const unsigned long long s = f2_mul(W(73), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(74), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[11], g[5]); g[11] = f2_fma(v, x[5], g[11]); } \
+      { unsigned long long v; v = f2_mul(W(102), adj[1]); g[5] = f2_fma(v, x[12], g[5]); g[12] = f2_fma(v, x[5], g[12]); } \
+      { unsigned long long v; v = f2_mul(W(103), adj[1]); g[5] = f2_fma(v, x[14], g[5]); g[14] = f2_fma(v, x[5], g[14]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); unsigned long long v; v = f2_mul(W(7), adj[0]); { const unsigned long long s = f2_mul(W(75), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(184), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(282), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(392), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[6] = f2_fma(v, x[6], g[6]); g[6] = f2_fma(v, x[6], g[6]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(76), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } { const unsigned long long s = f2_mul(W(185), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(393), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(283), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(394), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[6] = f2_fma(v, x[7], g[6]); g[7] = f2_fma(v, x[6], g[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(77), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } { const unsigned long long s = f2_mul(W(186), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(187), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(395), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(284), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(396), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[6] = f2_fma(v, x[8], g[6]); g[8] = f2_fma(v, x[6], g[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(78), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[6] = f2_fma(v, x[9], g[6]); g[9] = f2_fma(v, x[6], g[9]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); unsigned long long v; v = f2_mul(W(104), adj[1]); { const unsigned long long s = f2_mul(W(79), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[6] = f2_fma(v, x[11], g[6]); g[11] = f2_fma(v, x[6], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); unsigned long long v; v = f2_mul(W(219), adj[2]); { const unsigned long long s = f2_mul(W(80), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } g[6] = f2_fma(v, x[12], g[6]); g[12] = f2_fma(v, x[6], g[12]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); unsigned long long v; v = f2_mul(W(313), adj[3]); { const unsigned long long s = f2_mul(W(81), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[6] = f2_fma(v, x[13], g[6]); g[13] = f2_fma(v, x[6], g[13]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(82), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[6] = f2_fma(v, x[15], g[6]); g[15] = f2_fma(v, x[6], g[15]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); unsigned long long v; v = f2_mul(W(8), adj[0]); { const unsigned long long s = f2_mul(W(83), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(188), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(189), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(285), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(397), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(286), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(398), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[7], g[7]); g[7] = f2_fma(v, x[7], g[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(190), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(399), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(287), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(400), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(288), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[8], g[7]); g[8] = f2_fma(v, x[7], g[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(84), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[7] = f2_fma(v, x[9], g[7]); g[9] = f2_fma(v, x[7], g[9]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); unsigned long long v; v = f2_mul(W(105), adj[1]); { const unsigned long long s = f2_mul(W(85), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[7] = f2_fma(v, x[10], g[7]); g[10] = f2_fma(v, x[7], g[10]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); unsigned long long v; v = f2_mul(W(314), adj[3]); { const unsigned long long s = f2_mul(W(86), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[7] = f2_fma(v, x[12], g[7]); g[12] = f2_fma(v, x[7], g[12]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); unsigned long long v; v = f2_mul(W(220), adj[2]); { const unsigned long long s = f2_mul(W(87), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[7] = f2_fma(v, x[13], g[7]); g[13] = f2_fma(v, x[7], g[13]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); unsigned long long v; v = f2_mul(W(315), adj[3]); { const unsigned long long s = f2_mul(W(88), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[14], g[7]); g[14] = f2_fma(v, x[7], g[14]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); unsigned long long v; v = f2_mul(W(9), adj[0]); { const unsigned long long s = f2_mul(W(191), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(192), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(289), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(401), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(402), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[8], g[8]); g[8] = f2_fma(v, x[8], g[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); unsigned long long v; v = f2_mul(W(106), adj[1]); { const unsigned long long s = f2_mul(W(89), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[8] = f2_fma(v, x[9], g[8]); g[9] = f2_fma(v, x[8], g[9]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); unsigned long long v; v = f2_mul(W(107), adj[1]); { const unsigned long long s = f2_mul(W(90), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[8] = f2_fma(v, x[11], g[8]); g[11] = f2_fma(v, x[8], g[11]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(91), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[8] = f2_fma(v, x[12], g[8]); g[12] = f2_fma(v, x[8], g[12]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); unsigned long long v; v = f2_mul(W(316), adj[3]); { const unsigned long long s = f2_mul(W(92), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(93), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[13], g[8]); g[13] = f2_fma(v, x[8], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(221), adj[2]); g[8] = f2_fma(v, x[14], g[8]); g[14] = f2_fma(v, x[8], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(317), adj[3]); g[8] = f2_fma(v, x[15], g[8]); g[15] = f2_fma(v, x[8], g[15]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); unsigned long long v; v = f2_mul(W(10), adj[0]); { const unsigned long long s = f2_mul(W(193), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(290), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(403), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[9] = f2_fma(v, x[9], g[9]); g[9] = f2_fma(v, x[9], g[9]); } \
+      { const unsigned long long p = f2_mul(x[9], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(194), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(404), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(291), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(405), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[9] = f2_fma(v, x[10], g[9]); g[10] = f2_fma(v, x[9], g[10]); } \
+      { const unsigned long long p = f2_mul(x[9], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(195), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } { const unsigned long long s = f2_mul(W(406), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(292), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(407), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[9] = f2_fma(v, x[11], g[9]); g[11] = f2_fma(v, x[9], g[11]); } \
+      { const unsigned long long p = f2_mul(x[9], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(196), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[9] = f2_fma(v, x[12], g[9]); g[12] = f2_fma(v, x[9], g[12]); } \
+      { const unsigned long long p = f2_mul(x[9], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(197), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(198), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[9] = f2_fma(v, x[13], g[9]); g[13] = f2_fma(v, x[9], g[13]); } \
+      { const unsigned long long p = f2_mul(x[9], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(199), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[9] = f2_fma(v, x[14], g[9]); g[14] = f2_fma(v, x[9], g[14]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); unsigned long long v; v = f2_mul(W(11), adj[0]); { const unsigned long long s = f2_mul(W(200), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(293), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(408), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(409), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[10] = f2_fma(v, x[10], g[10]); g[10] = f2_fma(v, x[10], g[10]); } \
+      { const unsigned long long p = f2_mul(x[10], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(410), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(294), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(411), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(295), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[10] = f2_fma(v, x[11], g[10]); g[11] = f2_fma(v, x[10], g[11]); } \
+      { const unsigned long long p = f2_mul(x[10], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(201), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(202), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[10] = f2_fma(v, x[12], g[10]); g[12] = f2_fma(v, x[10], g[12]); } \
+      { const unsigned long long p = f2_mul(x[10], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(203), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[10] = f2_fma(v, x[13], g[10]); g[13] = f2_fma(v, x[10], g[13]); } \
+      { const unsigned long long p = f2_mul(x[10], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(204), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[10] = f2_fma(v, x[14], g[10]); g[14] = f2_fma(v, x[10], g[14]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); unsigned long long v; v = f2_mul(W(12), adj[0]); { const unsigned long long s = f2_mul(W(205), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(296), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(412), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(297), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(413), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[11] = f2_fma(v, x[11], g[11]); g[11] = f2_fma(v, x[11], g[11]); } \
+      { const unsigned long long p = f2_mul(x[11], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(206), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(207), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[11] = f2_fma(v, x[12], g[11]); g[12] = f2_fma(v, x[11], g[12]); } \
+      { const unsigned long long p = f2_mul(x[11], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(208), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(209), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[11] = f2_fma(v, x[13], g[11]); g[13] = f2_fma(v, x[11], g[13]); } \
+      { const unsigned long long p = f2_mul(x[11], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(210), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[11] = f2_fma(v, x[14], g[11]); g[14] = f2_fma(v, x[11], g[14]); } \
+      { const unsigned long long p = f2_mul(x[11], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(211), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[11] = f2_fma(v, x[15], g[11]); g[15] = f2_fma(v, x[11], g[15]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); unsigned long long v; v = f2_mul(W(13), adj[0]); { const unsigned long long s = f2_mul(W(298), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(414), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[12] = f2_fma(v, x[12], g[12]); g[12] = f2_fma(v, x[12], g[12]); } \
+      { const unsigned long long p = f2_mul(x[12], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(299), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(415), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[12] = f2_fma(v, x[13], g[12]); g[13] = f2_fma(v, x[12], g[13]); } \
+      { const unsigned long long p = f2_mul(x[12], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(300), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } { const unsigned long long s = f2_mul(W(416), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[12] = f2_fma(v, x[14], g[12]); g[14] = f2_fma(v, x[12], g[14]); } \
+      { const unsigned long long p = f2_mul(x[12], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(301), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[12] = f2_fma(v, x[15], g[12]); g[15] = f2_fma(v, x[12], g[15]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); unsigned long long v; v = f2_mul(W(14), adj[0]); { const unsigned long long s = f2_mul(W(417), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(302), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(418), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
+      { const unsigned long long p = f2_mul(x[13], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(419), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } { const unsigned long long s = f2_mul(W(303), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[13] = f2_fma(v, x[14], g[13]); g[14] = f2_fma(v, x[13], g[14]); } \
+      { const unsigned long long p = f2_mul(x[13], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(420), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[13] = f2_fma(v, x[15], g[13]); g[15] = f2_fma(v, x[13], g[15]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); unsigned long long v; v = f2_mul(W(15), adj[0]); { const unsigned long long s = f2_mul(W(421), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(16), adj[0]); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
+#define SXB_S1_M1_FORWARD_BODY \
+      o[0] = f2_fma(W(0), x[0], o[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); o[0] = f2_fma(p, f2_fma(W(17), x[0], W(1)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); o[0] = f2_fma(p, f2_mul(W(18), x[1]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); o[0] = f2_fma(p, f2_mul(W(19), x[2]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); o[0] = f2_fma(p, f2_mul(W(20), x[3]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); o[0] = f2_fma(p, f2_mul(W(21), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); o[0] = f2_fma(p, f2_mul(W(22), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); o[0] = f2_fma(p, f2_mul(W(23), x[6]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); o[0] = f2_fma(p, f2_mul(W(24), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); o[0] = f2_fma(p, f2_mul(W(25), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); o[0] = f2_fma(p, f2_mul(W(26), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); o[0] = f2_fma(p, f2_mul(W(27), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); o[0] = f2_fma(p, f2_mul(W(28), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); o[0] = f2_fma(p, f2_mul(W(29), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); o[0] = f2_fma(p, f2_mul(W(30), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); o[0] = f2_fma(p, f2_mul(W(31), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); o[0] = f2_fma(p, f2_mul(W(32), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); o[0] = f2_fma(p, f2_fma(W(34), x[8], f2_fma(W(33), x[6], W(2))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); o[0] = f2_fma(p, f2_mul(W(35), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); o[0] = f2_fma(p, f2_mul(W(36), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); o[0] = f2_fma(p, f2_fma(W(38), x[15], f2_mul(W(37), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); o[0] = f2_fma(p, f2_fma(W(40), x[14], f2_mul(W(39), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); o[0] = f2_fma(p, f2_mul(W(41), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); o[0] = f2_fma(p, f2_mul(W(42), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); o[0] = f2_fma(p, f2_fma(W(44), x[11], f2_mul(W(43), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); o[0] = f2_fma(p, f2_fma(W(45), x[6], W(3)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); o[0] = f2_fma(p, f2_mul(W(46), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); o[0] = f2_fma(p, f2_mul(W(47), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); o[0] = f2_fma(p, f2_mul(W(48), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); o[0] = f2_fma(p, f2_mul(W(49), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); o[0] = f2_fma(p, f2_mul(W(50), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); o[0] = f2_fma(p, f2_mul(W(51), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); o[0] = f2_fma(p, f2_fma(W(53), x[8], f2_fma(W(52), x[6], W(4))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); o[0] = f2_fma(p, f2_fma(W(55), x[11], f2_mul(W(54), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); o[0] = f2_fma(p, f2_mul(W(56), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); o[0] = f2_fma(p, f2_mul(W(57), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); o[0] = f2_fma(p, f2_fma(W(59), x[14], f2_mul(W(58), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); o[0] = f2_fma(p, f2_fma(W(61), x[15], f2_mul(W(60), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); o[0] = f2_fma(p, f2_fma(W(62), x[6], W(5)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); o[0] = f2_fma(p, f2_mul(W(63), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); o[0] = f2_fma(p, f2_mul(W(64), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); o[0] = f2_fma(p, f2_mul(W(65), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); o[0] = f2_fma(p, f2_fma(W(67), x[15], f2_mul(W(66), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); o[0] = f2_fma(p, f2_fma(W(69), x[8], f2_fma(W(68), x[6], W(6))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); o[0] = f2_fma(p, f2_mul(W(70), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); o[0] = f2_fma(p, f2_fma(W(72), x[15], f2_mul(W(71), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); o[0] = f2_fma(p, f2_fma(W(74), x[14], f2_mul(W(73), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); o[0] = f2_fma(p, f2_fma(W(75), x[6], W(7)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); o[0] = f2_fma(p, f2_mul(W(76), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); o[0] = f2_fma(p, f2_mul(W(77), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); o[0] = f2_fma(p, f2_mul(W(78), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); o[0] = f2_fma(p, f2_mul(W(79), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); o[0] = f2_fma(p, f2_mul(W(80), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); o[0] = f2_fma(p, f2_mul(W(81), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); o[0] = f2_fma(p, f2_mul(W(82), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); o[0] = f2_fma(p, f2_fma(W(83), x[8], W(8)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); o[0] = f2_fma(p, f2_mul(W(84), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); o[0] = f2_fma(p, f2_mul(W(85), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); o[0] = f2_fma(p, f2_mul(W(86), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); o[0] = f2_fma(p, f2_mul(W(87), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); o[0] = f2_fma(p, f2_mul(W(88), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); o[0] = f2_fma(p, W(9), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); o[0] = f2_fma(p, f2_mul(W(89), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); o[0] = f2_fma(p, f2_mul(W(90), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); o[0] = f2_fma(p, f2_mul(W(91), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); o[0] = f2_fma(p, f2_fma(W(93), x[15], f2_mul(W(92), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); o[0] = f2_fma(p, W(10), o[0]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); o[0] = f2_fma(p, W(11), o[0]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); o[0] = f2_fma(p, W(12), o[0]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); o[0] = f2_fma(p, W(13), o[0]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); o[0] = f2_fma(p, W(14), o[0]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); o[0] = f2_fma(p, W(15), o[0]); } \
+      { const unsigned long long p = f2_mul(x[15], x[15]); o[0] = f2_fma(p, W(16), o[0]); }
+#define SXB_S1_M1_REVERSE_BODY \
+      g[0] = f2_fma(W(0), adj[0], g[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); unsigned long long v; v = f2_mul(W(1), adj[0]); { const unsigned long long s = f2_mul(W(17), adj[0]); g[0] = f2_fma(s, p, g[0]); v = f2_fma(s, x[0], v); } g[0] = f2_fma(v, x[0], g[0]); g[0] = f2_fma(v, x[0], g[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); unsigned long long v; { const unsigned long long s = f2_mul(W(18), adj[0]); g[1] = f2_fma(s, p, g[1]); v = f2_mul(s, x[1]); } g[0] = f2_fma(v, x[1], g[0]); g[1] = f2_fma(v, x[0], g[1]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(19), adj[0]); g[2] = f2_fma(s, p, g[2]); v = f2_mul(s, x[2]); } g[0] = f2_fma(v, x[2], g[0]); g[2] = f2_fma(v, x[0], g[2]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(20), adj[0]); g[3] = f2_fma(s, p, g[3]); v = f2_mul(s, x[3]); } g[0] = f2_fma(v, x[3], g[0]); g[3] = f2_fma(v, x[0], g[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(21), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[0] = f2_fma(v, x[4], g[0]); g[4] = f2_fma(v, x[0], g[4]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(22), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[0] = f2_fma(v, x[5], g[0]); g[5] = f2_fma(v, x[0], g[5]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(23), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_mul(s, x[6]); } g[0] = f2_fma(v, x[6], g[0]); g[6] = f2_fma(v, x[0], g[6]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(24), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[0] = f2_fma(v, x[7], g[0]); g[7] = f2_fma(v, x[0], g[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(25), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[0] = f2_fma(v, x[8], g[0]); g[8] = f2_fma(v, x[0], g[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(26), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[0] = f2_fma(v, x[9], g[0]); g[9] = f2_fma(v, x[0], g[9]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(27), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[0] = f2_fma(v, x[10], g[0]); g[10] = f2_fma(v, x[0], g[10]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(28), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[0] = f2_fma(v, x[11], g[0]); g[11] = f2_fma(v, x[0], g[11]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(29), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[0] = f2_fma(v, x[12], g[0]); g[12] = f2_fma(v, x[0], g[12]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(30), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[0] = f2_fma(v, x[13], g[0]); g[13] = f2_fma(v, x[0], g[13]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(31), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[0] = f2_fma(v, x[14], g[0]); g[14] = f2_fma(v, x[0], g[14]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(32), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[0] = f2_fma(v, x[15], g[0]); g[15] = f2_fma(v, x[0], g[15]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); unsigned long long v; v = f2_mul(W(2), adj[0]); { const unsigned long long s = f2_mul(W(33), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(34), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[1] = f2_fma(v, x[1], g[1]); g[1] = f2_fma(v, x[1], g[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(35), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[1] = f2_fma(v, x[2], g[1]); g[2] = f2_fma(v, x[1], g[2]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(36), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[1] = f2_fma(v, x[3], g[1]); g[3] = f2_fma(v, x[1], g[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(37), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(38), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[4], g[1]); g[4] = f2_fma(v, x[1], g[4]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(39), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(40), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[5], g[1]); g[5] = f2_fma(v, x[1], g[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(41), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[1] = f2_fma(v, x[6], g[1]); g[6] = f2_fma(v, x[1], g[6]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(42), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[1] = f2_fma(v, x[7], g[1]); g[7] = f2_fma(v, x[1], g[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(43), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(44), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[1] = f2_fma(v, x[8], g[1]); g[8] = f2_fma(v, x[1], g[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); unsigned long long v; v = f2_mul(W(3), adj[0]); { const unsigned long long s = f2_mul(W(45), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[2] = f2_fma(v, x[2], g[2]); g[2] = f2_fma(v, x[2], g[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(46), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[2] = f2_fma(v, x[3], g[2]); g[3] = f2_fma(v, x[2], g[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(47), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[2] = f2_fma(v, x[4], g[2]); g[4] = f2_fma(v, x[2], g[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(48), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[2] = f2_fma(v, x[5], g[2]); g[5] = f2_fma(v, x[2], g[5]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(49), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[2] = f2_fma(v, x[6], g[2]); g[6] = f2_fma(v, x[2], g[6]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(50), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[2] = f2_fma(v, x[7], g[2]); g[7] = f2_fma(v, x[2], g[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(51), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[2] = f2_fma(v, x[8], g[2]); g[8] = f2_fma(v, x[2], g[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); unsigned long long v; v = f2_mul(W(4), adj[0]); { const unsigned long long s = f2_mul(W(52), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(53), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[3] = f2_fma(v, x[3], g[3]); g[3] = f2_fma(v, x[3], g[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(54), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(55), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[3] = f2_fma(v, x[4], g[3]); g[4] = f2_fma(v, x[3], g[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(56), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[3] = f2_fma(v, x[5], g[3]); g[5] = f2_fma(v, x[3], g[5]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(57), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[3] = f2_fma(v, x[6], g[3]); g[6] = f2_fma(v, x[3], g[6]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(58), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(59), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[7], g[3]); g[7] = f2_fma(v, x[3], g[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(60), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(61), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[8], g[3]); g[8] = f2_fma(v, x[3], g[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); unsigned long long v; v = f2_mul(W(5), adj[0]); { const unsigned long long s = f2_mul(W(62), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[4] = f2_fma(v, x[4], g[4]); g[4] = f2_fma(v, x[4], g[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(63), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[4] = f2_fma(v, x[5], g[4]); g[5] = f2_fma(v, x[4], g[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(64), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[4] = f2_fma(v, x[9], g[4]); g[9] = f2_fma(v, x[4], g[9]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(65), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[4] = f2_fma(v, x[10], g[4]); g[10] = f2_fma(v, x[4], g[10]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(66), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(67), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[11], g[4]); g[11] = f2_fma(v, x[4], g[11]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); unsigned long long v; v = f2_mul(W(6), adj[0]); { const unsigned long long s = f2_mul(W(68), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(69), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[5] = f2_fma(v, x[5], g[5]); g[5] = f2_fma(v, x[5], g[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(70), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[5] = f2_fma(v, x[9], g[5]); g[9] = f2_fma(v, x[5], g[9]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(71), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(72), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[10], g[5]); g[10] = f2_fma(v, x[5], g[10]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(73), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(74), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[11], g[5]); g[11] = f2_fma(v, x[5], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); unsigned long long v; v = f2_mul(W(7), adj[0]); { const unsigned long long s = f2_mul(W(75), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[6] = f2_fma(v, x[6], g[6]); g[6] = f2_fma(v, x[6], g[6]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(76), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[6] = f2_fma(v, x[7], g[6]); g[7] = f2_fma(v, x[6], g[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(77), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[6] = f2_fma(v, x[8], g[6]); g[8] = f2_fma(v, x[6], g[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(78), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[6] = f2_fma(v, x[9], g[6]); g[9] = f2_fma(v, x[6], g[9]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(79), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[6] = f2_fma(v, x[11], g[6]); g[11] = f2_fma(v, x[6], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(80), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[6] = f2_fma(v, x[12], g[6]); g[12] = f2_fma(v, x[6], g[12]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(81), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[6] = f2_fma(v, x[13], g[6]); g[13] = f2_fma(v, x[6], g[13]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(82), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[6] = f2_fma(v, x[15], g[6]); g[15] = f2_fma(v, x[6], g[15]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); unsigned long long v; v = f2_mul(W(8), adj[0]); { const unsigned long long s = f2_mul(W(83), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[7] = f2_fma(v, x[7], g[7]); g[7] = f2_fma(v, x[7], g[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(84), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[7] = f2_fma(v, x[9], g[7]); g[9] = f2_fma(v, x[7], g[9]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(85), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[7] = f2_fma(v, x[10], g[7]); g[10] = f2_fma(v, x[7], g[10]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(86), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[7] = f2_fma(v, x[12], g[7]); g[12] = f2_fma(v, x[7], g[12]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(87), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[7] = f2_fma(v, x[13], g[7]); g[13] = f2_fma(v, x[7], g[13]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(88), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[7] = f2_fma(v, x[14], g[7]); g[14] = f2_fma(v, x[7], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(9), adj[0]); g[8] = f2_fma(v, x[8], g[8]); g[8] = f2_fma(v, x[8], g[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(89), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[9], g[8]); g[9] = f2_fma(v, x[8], g[9]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(90), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[11], g[8]); g[11] = f2_fma(v, x[8], g[11]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(91), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[8] = f2_fma(v, x[12], g[8]); g[12] = f2_fma(v, x[8], g[12]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(92), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(93), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[13], g[8]); g[13] = f2_fma(v, x[8], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(10), adj[0]); g[9] = f2_fma(v, x[9], g[9]); g[9] = f2_fma(v, x[9], g[9]); } \
+      { unsigned long long v; v = f2_mul(W(11), adj[0]); g[10] = f2_fma(v, x[10], g[10]); g[10] = f2_fma(v, x[10], g[10]); } \
+      { unsigned long long v; v = f2_mul(W(12), adj[0]); g[11] = f2_fma(v, x[11], g[11]); g[11] = f2_fma(v, x[11], g[11]); } \
+      { unsigned long long v; v = f2_mul(W(13), adj[0]); g[12] = f2_fma(v, x[12], g[12]); g[12] = f2_fma(v, x[12], g[12]); } \
+      { unsigned long long v; v = f2_mul(W(14), adj[0]); g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(15), adj[0]); g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(16), adj[0]); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
 #define SXB_S1_L1_FORWARD_BODY \
     { /* path 0: edge l=0, source l=0 -> l=0 */ \
       const float t0 = R[0] * h[0]; \
@@ -2847,6 +3549,444 @@
     X3(0, 91, 8, 12, 14) \
     X3(0, 92, 8, 13, 13) \
     X3(0, 93, 8, 13, 15)
+#define SXB_S2_M0_FORWARD_BODY \
+      o[0] = f2_fma(W(0), x[0], o[0]); \
+      o[1] = f2_fma(W(94), x[1], o[1]); \
+      o[2] = f2_fma(W(206), x[2], o[2]); \
+      o[3] = f2_fma(W(298), x[3], o[3]); \
+      o[4] = f2_fma(W(410), x[4], o[4]); \
+      o[5] = f2_fma(W(500), x[5], o[5]); \
+      o[6] = f2_fma(W(597), x[6], o[6]); \
+      o[7] = f2_fma(W(692), x[7], o[7]); \
+      o[8] = f2_fma(W(789), x[8], o[8]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); o[0] = f2_fma(p, f2_fma(W(17), x[0], W(1)), o[0]); o[1] = f2_fma(p, f2_mul(W(108), x[1]), o[1]); o[2] = f2_fma(p, f2_mul(W(216), x[2]), o[2]); o[3] = f2_fma(p, f2_mul(W(312), x[3]), o[3]); o[4] = f2_fma(p, f2_mul(W(424), x[4]), o[4]); o[5] = f2_fma(p, f2_mul(W(515), x[5]), o[5]); o[6] = f2_fma(p, f2_mul(W(615), x[6]), o[6]); o[7] = f2_fma(p, f2_mul(W(707), x[7]), o[7]); o[8] = f2_fma(p, f2_mul(W(806), x[8]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); o[0] = f2_fma(p, f2_mul(W(18), x[1]), o[0]); o[1] = f2_fma(p, f2_fma(W(110), x[8], f2_fma(W(109), x[6], W(95))), o[1]); o[2] = f2_fma(p, f2_mul(W(217), x[5]), o[2]); o[3] = f2_fma(p, f2_mul(W(313), x[4]), o[3]); o[4] = f2_fma(p, f2_fma(W(427), x[15], f2_fma(W(426), x[13], f2_mul(W(425), x[3]))), o[4]); o[5] = f2_fma(p, f2_fma(W(518), x[14], f2_fma(W(517), x[12], f2_mul(W(516), x[2]))), o[5]); o[6] = f2_fma(p, f2_fma(W(617), x[11], f2_mul(W(616), x[1])), o[6]); o[7] = f2_fma(p, f2_mul(W(708), x[10]), o[7]); o[8] = f2_fma(p, f2_fma(W(809), x[11], f2_fma(W(808), x[9], f2_mul(W(807), x[1]))), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); o[0] = f2_fma(p, f2_mul(W(19), x[2]), o[0]); o[1] = f2_fma(p, f2_mul(W(111), x[5]), o[1]); o[2] = f2_fma(p, f2_fma(W(218), x[6], W(207)), o[2]); o[3] = f2_fma(p, f2_mul(W(314), x[7]), o[3]); o[4] = f2_fma(p, f2_mul(W(428), x[10]), o[4]); o[5] = f2_fma(p, f2_mul(W(519), x[11]), o[5]); o[6] = f2_fma(p, f2_fma(W(619), x[12], f2_mul(W(618), x[2])), o[6]); o[7] = f2_fma(p, f2_fma(W(710), x[13], f2_mul(W(709), x[3])), o[7]); o[8] = f2_fma(p, f2_mul(W(810), x[14]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); o[0] = f2_fma(p, f2_mul(W(20), x[3]), o[0]); o[1] = f2_fma(p, f2_mul(W(112), x[4]), o[1]); o[2] = f2_fma(p, f2_mul(W(219), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(316), x[8], f2_fma(W(315), x[6], W(299))), o[3]); o[4] = f2_fma(p, f2_fma(W(430), x[11], f2_mul(W(429), x[9])), o[4]); o[5] = f2_fma(p, f2_mul(W(520), x[10]), o[5]); o[6] = f2_fma(p, f2_fma(W(621), x[13], f2_mul(W(620), x[3])), o[6]); o[7] = f2_fma(p, f2_fma(W(712), x[14], f2_mul(W(711), x[12])), o[7]); o[8] = f2_fma(p, f2_fma(W(813), x[15], f2_fma(W(812), x[13], f2_mul(W(811), x[3]))), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); o[0] = f2_fma(p, f2_mul(W(21), x[4]), o[0]); o[1] = f2_fma(p, f2_fma(W(114), x[15], f2_mul(W(113), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(220), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(318), x[11], f2_mul(W(317), x[9])), o[3]); o[4] = f2_fma(p, f2_fma(W(431), x[6], W(411)), o[4]); o[5] = f2_fma(p, f2_mul(W(521), x[7]), o[5]); o[6] = f2_fma(p, f2_mul(W(622), x[4]), o[6]); o[7] = f2_fma(p, f2_mul(W(713), x[5]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); o[0] = f2_fma(p, f2_mul(W(22), x[5]), o[0]); o[1] = f2_fma(p, f2_fma(W(116), x[14], f2_mul(W(115), x[12])), o[1]); o[2] = f2_fma(p, f2_mul(W(221), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(319), x[10]), o[3]); o[4] = f2_fma(p, f2_mul(W(432), x[7]), o[4]); o[5] = f2_fma(p, f2_fma(W(523), x[8], f2_fma(W(522), x[6], W(501))), o[5]); o[6] = f2_fma(p, f2_mul(W(623), x[5]), o[6]); o[8] = f2_fma(p, f2_mul(W(814), x[5]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); o[0] = f2_fma(p, f2_mul(W(23), x[6]), o[0]); o[1] = f2_fma(p, f2_mul(W(117), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(222), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(320), x[13]), o[3]); o[6] = f2_fma(p, f2_fma(W(624), x[6], W(598)), o[6]); o[7] = f2_fma(p, f2_mul(W(714), x[7]), o[7]); o[8] = f2_fma(p, f2_mul(W(815), x[8]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); o[0] = f2_fma(p, f2_mul(W(24), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(118), x[10]), o[1]); o[2] = f2_fma(p, f2_mul(W(223), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(322), x[14], f2_mul(W(321), x[12])), o[3]); o[6] = f2_fma(p, f2_mul(W(625), x[7]), o[6]); o[7] = f2_fma(p, f2_fma(W(715), x[8], W(693)), o[7]); o[8] = f2_fma(p, f2_mul(W(816), x[7]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); o[0] = f2_fma(p, f2_mul(W(25), x[8]), o[0]); o[1] = f2_fma(p, f2_fma(W(120), x[11], f2_mul(W(119), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(224), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(324), x[15], f2_mul(W(323), x[13])), o[3]); o[6] = f2_fma(p, f2_mul(W(626), x[8]), o[6]); o[8] = f2_fma(p, W(790), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); o[0] = f2_fma(p, f2_mul(W(26), x[9]), o[0]); o[4] = f2_fma(p, f2_mul(W(433), x[13]), o[4]); o[5] = f2_fma(p, f2_mul(W(524), x[14]), o[5]); o[6] = f2_fma(p, f2_mul(W(627), x[9]), o[6]); o[7] = f2_fma(p, f2_mul(W(716), x[10]), o[7]); o[8] = f2_fma(p, f2_mul(W(817), x[11]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); o[0] = f2_fma(p, f2_mul(W(27), x[10]), o[0]); o[4] = f2_fma(p, f2_mul(W(434), x[12]), o[4]); o[5] = f2_fma(p, f2_fma(W(526), x[15], f2_mul(W(525), x[13])), o[5]); o[7] = f2_fma(p, f2_mul(W(717), x[11]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); o[0] = f2_fma(p, f2_mul(W(28), x[11]), o[0]); o[4] = f2_fma(p, f2_fma(W(436), x[15], f2_mul(W(435), x[13])), o[4]); o[5] = f2_fma(p, f2_fma(W(528), x[14], f2_mul(W(527), x[12])), o[5]); o[6] = f2_fma(p, f2_mul(W(628), x[11]), o[6]); o[8] = f2_fma(p, f2_mul(W(818), x[11]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); o[0] = f2_fma(p, f2_mul(W(29), x[12]), o[0]); o[6] = f2_fma(p, f2_mul(W(629), x[12]), o[6]); o[7] = f2_fma(p, f2_mul(W(718), x[13]), o[7]); o[8] = f2_fma(p, f2_mul(W(819), x[14]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); o[0] = f2_fma(p, f2_mul(W(30), x[13]), o[0]); o[6] = f2_fma(p, f2_mul(W(630), x[13]), o[6]); o[7] = f2_fma(p, f2_mul(W(719), x[14]), o[7]); o[8] = f2_fma(p, f2_fma(W(821), x[15], f2_mul(W(820), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); o[0] = f2_fma(p, f2_mul(W(31), x[14]), o[0]); o[7] = f2_fma(p, f2_mul(W(720), x[15]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); o[0] = f2_fma(p, f2_mul(W(32), x[15]), o[0]); o[6] = f2_fma(p, f2_mul(W(631), x[15]), o[6]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); o[0] = f2_fma(p, f2_fma(W(34), x[8], f2_fma(W(33), x[6], W(2))), o[0]); o[1] = f2_fma(p, f2_fma(W(123), x[11], f2_fma(W(122), x[9], f2_mul(W(121), x[1]))), o[1]); o[2] = f2_fma(p, f2_fma(W(227), x[14], f2_fma(W(226), x[12], f2_mul(W(225), x[2]))), o[2]); o[3] = f2_fma(p, f2_fma(W(327), x[15], f2_fma(W(326), x[13], f2_mul(W(325), x[3]))), o[3]); o[4] = f2_fma(p, f2_mul(W(437), x[4]), o[4]); o[5] = f2_fma(p, f2_mul(W(529), x[5]), o[5]); o[6] = f2_fma(p, f2_fma(W(633), x[8], f2_fma(W(632), x[6], W(599))), o[6]); o[7] = f2_fma(p, f2_mul(W(721), x[7]), o[7]); o[8] = f2_fma(p, f2_fma(W(823), x[8], f2_fma(W(822), x[6], W(791))), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); o[0] = f2_fma(p, f2_mul(W(35), x[5]), o[0]); o[1] = f2_fma(p, f2_fma(W(126), x[14], f2_fma(W(125), x[12], f2_mul(W(124), x[2]))), o[1]); o[2] = f2_fma(p, f2_mul(W(228), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(328), x[10]), o[3]); o[4] = f2_fma(p, f2_mul(W(438), x[7]), o[4]); o[5] = f2_fma(p, f2_fma(W(531), x[8], f2_fma(W(530), x[6], W(502))), o[5]); o[6] = f2_fma(p, f2_mul(W(634), x[5]), o[6]); o[7] = f2_fma(p, f2_mul(W(722), x[4]), o[7]); o[8] = f2_fma(p, f2_mul(W(824), x[5]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); o[0] = f2_fma(p, f2_mul(W(36), x[4]), o[0]); o[1] = f2_fma(p, f2_fma(W(129), x[15], f2_fma(W(128), x[13], f2_mul(W(127), x[3]))), o[1]); o[2] = f2_fma(p, f2_mul(W(229), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(330), x[11], f2_mul(W(329), x[9])), o[3]); o[4] = f2_fma(p, f2_fma(W(439), x[6], W(412)), o[4]); o[5] = f2_fma(p, f2_mul(W(532), x[7]), o[5]); o[6] = f2_fma(p, f2_mul(W(635), x[4]), o[6]); o[7] = f2_fma(p, f2_mul(W(723), x[5]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); o[0] = f2_fma(p, f2_fma(W(38), x[15], f2_mul(W(37), x[13])), o[0]); o[1] = f2_fma(p, f2_mul(W(130), x[4]), o[1]); o[2] = f2_fma(p, f2_mul(W(230), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(331), x[6], W(300)), o[3]); o[4] = f2_fma(p, f2_fma(W(441), x[11], f2_mul(W(440), x[9])), o[4]); o[5] = f2_fma(p, f2_mul(W(533), x[10]), o[5]); o[6] = f2_fma(p, f2_fma(W(637), x[15], f2_mul(W(636), x[13])), o[6]); o[7] = f2_fma(p, f2_fma(W(725), x[14], f2_mul(W(724), x[12])), o[7]); o[8] = f2_fma(p, f2_fma(W(826), x[15], f2_mul(W(825), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); o[0] = f2_fma(p, f2_fma(W(40), x[14], f2_mul(W(39), x[12])), o[0]); o[1] = f2_fma(p, f2_mul(W(131), x[5]), o[1]); o[2] = f2_fma(p, f2_fma(W(232), x[8], f2_fma(W(231), x[6], W(208))), o[2]); o[3] = f2_fma(p, f2_mul(W(332), x[7]), o[3]); o[4] = f2_fma(p, f2_mul(W(442), x[10]), o[4]); o[5] = f2_fma(p, f2_fma(W(535), x[11], f2_mul(W(534), x[9])), o[5]); o[6] = f2_fma(p, f2_fma(W(639), x[14], f2_mul(W(638), x[12])), o[6]); o[7] = f2_fma(p, f2_fma(W(727), x[15], f2_mul(W(726), x[13])), o[7]); o[8] = f2_fma(p, f2_fma(W(828), x[14], f2_mul(W(827), x[12])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); o[0] = f2_fma(p, f2_mul(W(41), x[11]), o[0]); o[1] = f2_fma(p, f2_fma(W(133), x[8], f2_fma(W(132), x[6], W(96))), o[1]); o[4] = f2_fma(p, f2_fma(W(444), x[15], f2_mul(W(443), x[13])), o[4]); o[5] = f2_fma(p, f2_fma(W(537), x[14], f2_mul(W(536), x[12])), o[5]); o[6] = f2_fma(p, f2_mul(W(640), x[11]), o[6]); o[7] = f2_fma(p, f2_mul(W(728), x[10]), o[7]); o[8] = f2_fma(p, f2_fma(W(830), x[11], f2_mul(W(829), x[9])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); o[0] = f2_fma(p, f2_mul(W(42), x[10]), o[0]); o[1] = f2_fma(p, f2_mul(W(134), x[7]), o[1]); o[4] = f2_fma(p, f2_fma(W(446), x[14], f2_mul(W(445), x[12])), o[4]); o[5] = f2_fma(p, f2_fma(W(539), x[15], f2_mul(W(538), x[13])), o[5]); o[6] = f2_fma(p, f2_mul(W(641), x[10]), o[6]); o[7] = f2_fma(p, f2_fma(W(730), x[11], f2_mul(W(729), x[9])), o[7]); o[8] = f2_fma(p, f2_mul(W(831), x[10]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); o[0] = f2_fma(p, f2_fma(W(44), x[11], f2_mul(W(43), x[9])), o[0]); o[1] = f2_fma(p, f2_fma(W(135), x[8], W(97)), o[1]); o[4] = f2_fma(p, f2_fma(W(448), x[15], f2_mul(W(447), x[13])), o[4]); o[5] = f2_fma(p, f2_fma(W(541), x[14], f2_mul(W(540), x[12])), o[5]); o[6] = f2_fma(p, f2_fma(W(643), x[11], f2_mul(W(642), x[9])), o[6]); o[7] = f2_fma(p, f2_mul(W(731), x[10]), o[7]); o[8] = f2_fma(p, f2_fma(W(833), x[11], f2_mul(W(832), x[9])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[9]); o[1] = f2_fma(p, f2_fma(W(137), x[11], f2_mul(W(136), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(233), x[14]), o[2]); o[3] = f2_fma(p, f2_mul(W(333), x[13]), o[3]); o[8] = f2_fma(p, W(792), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[10]); o[1] = f2_fma(p, f2_mul(W(138), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(235), x[15], f2_mul(W(234), x[13])), o[2]); o[3] = f2_fma(p, f2_mul(W(334), x[12]), o[3]); o[7] = f2_fma(p, W(694), o[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[11]); o[1] = f2_fma(p, f2_mul(W(139), x[11]), o[1]); o[2] = f2_fma(p, f2_fma(W(237), x[14], f2_mul(W(236), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(336), x[15], f2_mul(W(335), x[13])), o[3]); o[6] = f2_fma(p, W(600), o[6]); o[8] = f2_fma(p, W(793), o[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[12]); o[1] = f2_fma(p, f2_fma(W(141), x[14], f2_mul(W(140), x[12])), o[1]); o[5] = f2_fma(p, W(503), o[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[13]); o[1] = f2_fma(p, f2_fma(W(143), x[15], f2_mul(W(142), x[13])), o[1]); o[4] = f2_fma(p, W(413), o[4]); } \
+      { const unsigned long long p = f2_mul(x[1], x[14]); o[1] = f2_fma(p, f2_mul(W(144), x[14]), o[1]); o[5] = f2_fma(p, W(504), o[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[15]); o[1] = f2_fma(p, f2_mul(W(145), x[15]), o[1]); o[4] = f2_fma(p, W(414), o[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); o[0] = f2_fma(p, f2_fma(W(45), x[6], W(3)), o[0]); o[1] = f2_fma(p, f2_mul(W(146), x[11]), o[1]); o[2] = f2_fma(p, f2_fma(W(239), x[12], f2_mul(W(238), x[2])), o[2]); o[3] = f2_fma(p, f2_fma(W(338), x[13], f2_mul(W(337), x[3])), o[3]); o[4] = f2_fma(p, f2_mul(W(449), x[4]), o[4]); o[5] = f2_fma(p, f2_mul(W(542), x[5]), o[5]); o[6] = f2_fma(p, f2_fma(W(644), x[6], W(601)), o[6]); o[7] = f2_fma(p, f2_mul(W(732), x[7]), o[7]); o[8] = f2_fma(p, f2_mul(W(834), x[8]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); o[0] = f2_fma(p, f2_mul(W(46), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(147), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(241), x[13], f2_mul(W(240), x[3])), o[2]); o[3] = f2_fma(p, f2_fma(W(340), x[14], f2_mul(W(339), x[12])), o[3]); o[4] = f2_fma(p, f2_mul(W(450), x[5]), o[4]); o[5] = f2_fma(p, f2_mul(W(543), x[4]), o[5]); o[6] = f2_fma(p, f2_mul(W(645), x[7]), o[6]); o[7] = f2_fma(p, f2_fma(W(734), x[8], f2_fma(W(733), x[6], W(695))), o[7]); o[8] = f2_fma(p, f2_mul(W(835), x[7]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); o[0] = f2_fma(p, f2_mul(W(47), x[10]), o[0]); o[1] = f2_fma(p, f2_mul(W(148), x[7]), o[1]); o[2] = f2_fma(p, f2_mul(W(242), x[4]), o[2]); o[3] = f2_fma(p, f2_mul(W(341), x[5]), o[3]); o[4] = f2_fma(p, f2_mul(W(451), x[12]), o[4]); o[5] = f2_fma(p, f2_fma(W(545), x[15], f2_mul(W(544), x[13])), o[5]); o[6] = f2_fma(p, f2_mul(W(646), x[10]), o[6]); o[7] = f2_fma(p, f2_fma(W(736), x[11], f2_mul(W(735), x[9])), o[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); o[0] = f2_fma(p, f2_mul(W(48), x[11]), o[0]); o[1] = f2_fma(p, f2_fma(W(150), x[8], f2_fma(W(149), x[6], W(98))), o[1]); o[2] = f2_fma(p, f2_mul(W(243), x[5]), o[2]); o[4] = f2_fma(p, f2_fma(W(453), x[15], f2_mul(W(452), x[13])), o[4]); o[5] = f2_fma(p, f2_fma(W(547), x[14], f2_mul(W(546), x[12])), o[5]); o[6] = f2_fma(p, f2_mul(W(647), x[11]), o[6]); o[7] = f2_fma(p, f2_mul(W(737), x[10]), o[7]); o[8] = f2_fma(p, f2_fma(W(837), x[11], f2_mul(W(836), x[9])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); o[0] = f2_fma(p, f2_mul(W(49), x[12]), o[0]); o[2] = f2_fma(p, f2_fma(W(244), x[6], W(209)), o[2]); o[3] = f2_fma(p, f2_mul(W(342), x[7]), o[3]); o[4] = f2_fma(p, f2_mul(W(454), x[10]), o[4]); o[5] = f2_fma(p, f2_mul(W(548), x[11]), o[5]); o[6] = f2_fma(p, f2_mul(W(648), x[12]), o[6]); o[7] = f2_fma(p, f2_mul(W(738), x[13]), o[7]); o[8] = f2_fma(p, f2_mul(W(838), x[14]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); o[0] = f2_fma(p, f2_mul(W(50), x[13]), o[0]); o[2] = f2_fma(p, f2_mul(W(245), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(343), x[8], W(301)), o[3]); o[4] = f2_fma(p, f2_fma(W(456), x[11], f2_mul(W(455), x[9])), o[4]); o[5] = f2_fma(p, f2_mul(W(549), x[10]), o[5]); o[6] = f2_fma(p, f2_mul(W(649), x[13]), o[6]); o[7] = f2_fma(p, f2_fma(W(740), x[14], f2_mul(W(739), x[12])), o[7]); o[8] = f2_fma(p, f2_fma(W(840), x[15], f2_mul(W(839), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); o[0] = f2_fma(p, f2_mul(W(51), x[14]), o[0]); o[2] = f2_fma(p, f2_mul(W(246), x[8]), o[2]); o[5] = f2_fma(p, f2_fma(W(551), x[11], f2_mul(W(550), x[9])), o[5]); o[6] = f2_fma(p, f2_mul(W(650), x[14]), o[6]); o[7] = f2_fma(p, f2_fma(W(742), x[15], f2_mul(W(741), x[13])), o[7]); o[8] = f2_fma(p, f2_mul(W(841), x[12]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[9]); o[1] = f2_fma(p, f2_mul(W(151), x[14]), o[1]); o[2] = f2_fma(p, f2_mul(W(247), x[9]), o[2]); o[3] = f2_fma(p, f2_mul(W(344), x[10]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[10]); o[1] = f2_fma(p, f2_fma(W(153), x[15], f2_mul(W(152), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(248), x[10]), o[2]); o[3] = f2_fma(p, f2_mul(W(345), x[11]), o[3]); o[4] = f2_fma(p, W(415), o[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[11]); o[1] = f2_fma(p, f2_fma(W(155), x[14], f2_mul(W(154), x[12])), o[1]); o[2] = f2_fma(p, f2_mul(W(249), x[11]), o[2]); o[5] = f2_fma(p, W(505), o[5]); } \
+      { const unsigned long long p = f2_mul(x[2], x[12]); o[2] = f2_fma(p, f2_mul(W(250), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(346), x[13]), o[3]); o[6] = f2_fma(p, W(602), o[6]); } \
+      { const unsigned long long p = f2_mul(x[2], x[13]); o[2] = f2_fma(p, f2_mul(W(251), x[13]), o[2]); o[3] = f2_fma(p, f2_mul(W(347), x[14]), o[3]); o[7] = f2_fma(p, W(696), o[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[14]); o[2] = f2_fma(p, f2_mul(W(252), x[14]), o[2]); o[3] = f2_fma(p, f2_mul(W(348), x[15]), o[3]); o[8] = f2_fma(p, W(794), o[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[15]); o[2] = f2_fma(p, f2_mul(W(253), x[15]), o[2]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); o[0] = f2_fma(p, f2_fma(W(53), x[8], f2_fma(W(52), x[6], W(4))), o[0]); o[1] = f2_fma(p, f2_fma(W(157), x[11], f2_mul(W(156), x[9])), o[1]); o[2] = f2_fma(p, f2_fma(W(255), x[14], f2_mul(W(254), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(351), x[15], f2_fma(W(350), x[13], f2_mul(W(349), x[3]))), o[3]); o[4] = f2_fma(p, f2_mul(W(457), x[4]), o[4]); o[5] = f2_fma(p, f2_mul(W(552), x[5]), o[5]); o[6] = f2_fma(p, f2_fma(W(652), x[8], f2_fma(W(651), x[6], W(603))), o[6]); o[7] = f2_fma(p, f2_mul(W(743), x[7]), o[7]); o[8] = f2_fma(p, f2_fma(W(843), x[8], f2_fma(W(842), x[6], W(795))), o[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); o[0] = f2_fma(p, f2_fma(W(55), x[11], f2_mul(W(54), x[9])), o[0]); o[1] = f2_fma(p, f2_fma(W(158), x[6], W(99)), o[1]); o[2] = f2_fma(p, f2_mul(W(256), x[5]), o[2]); o[3] = f2_fma(p, f2_mul(W(352), x[4]), o[3]); o[4] = f2_fma(p, f2_fma(W(459), x[15], f2_mul(W(458), x[13])), o[4]); o[5] = f2_fma(p, f2_fma(W(554), x[14], f2_mul(W(553), x[12])), o[5]); o[6] = f2_fma(p, f2_fma(W(654), x[11], f2_mul(W(653), x[9])), o[6]); o[7] = f2_fma(p, f2_mul(W(744), x[10]), o[7]); o[8] = f2_fma(p, f2_fma(W(845), x[11], f2_mul(W(844), x[9])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); o[0] = f2_fma(p, f2_mul(W(56), x[10]), o[0]); o[1] = f2_fma(p, f2_mul(W(159), x[7]), o[1]); o[3] = f2_fma(p, f2_mul(W(353), x[5]), o[3]); o[4] = f2_fma(p, f2_fma(W(461), x[14], f2_mul(W(460), x[12])), o[4]); o[5] = f2_fma(p, f2_fma(W(556), x[15], f2_mul(W(555), x[13])), o[5]); o[6] = f2_fma(p, f2_mul(W(655), x[10]), o[6]); o[7] = f2_fma(p, f2_fma(W(746), x[11], f2_mul(W(745), x[9])), o[7]); o[8] = f2_fma(p, f2_mul(W(846), x[10]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); o[0] = f2_fma(p, f2_mul(W(57), x[13]), o[0]); o[2] = f2_fma(p, f2_mul(W(257), x[7]), o[2]); o[3] = f2_fma(p, f2_fma(W(355), x[8], f2_fma(W(354), x[6], W(302))), o[3]); o[4] = f2_fma(p, f2_fma(W(463), x[11], f2_mul(W(462), x[9])), o[4]); o[5] = f2_fma(p, f2_mul(W(557), x[10]), o[5]); o[6] = f2_fma(p, f2_mul(W(656), x[13]), o[6]); o[7] = f2_fma(p, f2_fma(W(748), x[14], f2_mul(W(747), x[12])), o[7]); o[8] = f2_fma(p, f2_fma(W(848), x[15], f2_mul(W(847), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); o[0] = f2_fma(p, f2_fma(W(59), x[14], f2_mul(W(58), x[12])), o[0]); o[2] = f2_fma(p, f2_fma(W(258), x[8], W(210)), o[2]); o[3] = f2_fma(p, f2_mul(W(356), x[7]), o[3]); o[4] = f2_fma(p, f2_mul(W(464), x[10]), o[4]); o[5] = f2_fma(p, f2_fma(W(559), x[11], f2_mul(W(558), x[9])), o[5]); o[6] = f2_fma(p, f2_fma(W(658), x[14], f2_mul(W(657), x[12])), o[6]); o[7] = f2_fma(p, f2_fma(W(750), x[15], f2_mul(W(749), x[13])), o[7]); o[8] = f2_fma(p, f2_fma(W(850), x[14], f2_mul(W(849), x[12])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); o[0] = f2_fma(p, f2_fma(W(61), x[15], f2_mul(W(60), x[13])), o[0]); o[3] = f2_fma(p, f2_fma(W(357), x[8], W(303)), o[3]); o[4] = f2_fma(p, f2_fma(W(466), x[11], f2_mul(W(465), x[9])), o[4]); o[5] = f2_fma(p, f2_mul(W(560), x[10]), o[5]); o[6] = f2_fma(p, f2_fma(W(660), x[15], f2_mul(W(659), x[13])), o[6]); o[7] = f2_fma(p, f2_fma(W(752), x[14], f2_mul(W(751), x[12])), o[7]); o[8] = f2_fma(p, f2_fma(W(852), x[15], f2_mul(W(851), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[9]); o[1] = f2_fma(p, f2_mul(W(160), x[13]), o[1]); o[2] = f2_fma(p, f2_mul(W(259), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(359), x[11], f2_mul(W(358), x[9])), o[3]); o[4] = f2_fma(p, W(416), o[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[10]); o[1] = f2_fma(p, f2_mul(W(161), x[12]), o[1]); o[2] = f2_fma(p, f2_mul(W(260), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(360), x[10]), o[3]); o[5] = f2_fma(p, W(506), o[5]); } \
+      { const unsigned long long p = f2_mul(x[3], x[11]); o[1] = f2_fma(p, f2_fma(W(163), x[15], f2_mul(W(162), x[13])), o[1]); o[3] = f2_fma(p, f2_mul(W(361), x[11]), o[3]); o[4] = f2_fma(p, W(417), o[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[12]); o[2] = f2_fma(p, f2_mul(W(261), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(363), x[14], f2_mul(W(362), x[12])), o[3]); o[7] = f2_fma(p, W(697), o[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[13]); o[2] = f2_fma(p, f2_mul(W(262), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(365), x[15], f2_mul(W(364), x[13])), o[3]); o[6] = f2_fma(p, W(604), o[6]); o[8] = f2_fma(p, W(796), o[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[14]); o[2] = f2_fma(p, f2_mul(W(263), x[15]), o[2]); o[3] = f2_fma(p, f2_mul(W(366), x[14]), o[3]); o[7] = f2_fma(p, W(698), o[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[15]); o[3] = f2_fma(p, f2_mul(W(367), x[15]), o[3]); o[8] = f2_fma(p, W(797), o[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); o[0] = f2_fma(p, f2_fma(W(62), x[6], W(5)), o[0]); o[1] = f2_fma(p, f2_fma(W(165), x[11], f2_mul(W(164), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(264), x[12]), o[2]); o[3] = f2_fma(p, f2_fma(W(369), x[15], f2_mul(W(368), x[13])), o[3]); o[4] = f2_fma(p, f2_mul(W(467), x[4]), o[4]); o[5] = f2_fma(p, f2_mul(W(561), x[5]), o[5]); o[6] = f2_fma(p, f2_fma(W(661), x[6], W(605)), o[6]); o[7] = f2_fma(p, f2_mul(W(753), x[7]), o[7]); o[8] = f2_fma(p, f2_mul(W(853), x[8]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); o[0] = f2_fma(p, f2_mul(W(63), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(166), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(266), x[15], f2_mul(W(265), x[13])), o[2]); o[3] = f2_fma(p, f2_fma(W(371), x[14], f2_mul(W(370), x[12])), o[3]); o[4] = f2_fma(p, f2_mul(W(468), x[5]), o[4]); o[7] = f2_fma(p, W(699), o[7]); } \
+      { const unsigned long long p = f2_mul(x[4], x[6]); o[1] = f2_fma(p, f2_fma(W(168), x[15], f2_mul(W(167), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(267), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(373), x[11], f2_mul(W(372), x[9])), o[3]); o[4] = f2_fma(p, f2_fma(W(469), x[6], W(418)), o[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[7]); o[1] = f2_fma(p, f2_fma(W(170), x[14], f2_mul(W(169), x[12])), o[1]); o[2] = f2_fma(p, f2_fma(W(269), x[11], f2_mul(W(268), x[9])), o[2]); o[3] = f2_fma(p, f2_mul(W(374), x[10]), o[3]); o[4] = f2_fma(p, f2_mul(W(470), x[7]), o[4]); o[5] = f2_fma(p, W(507), o[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[8]); o[1] = f2_fma(p, f2_mul(W(171), x[15]), o[1]); o[3] = f2_fma(p, f2_mul(W(375), x[9]), o[3]); o[4] = f2_fma(p, f2_mul(W(471), x[8]), o[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); o[0] = f2_fma(p, f2_mul(W(64), x[13]), o[0]); o[3] = f2_fma(p, W(304), o[3]); o[4] = f2_fma(p, f2_fma(W(473), x[11], f2_mul(W(472), x[9])), o[4]); o[5] = f2_fma(p, f2_mul(W(562), x[10]), o[5]); o[6] = f2_fma(p, f2_mul(W(662), x[13]), o[6]); o[7] = f2_fma(p, f2_fma(W(755), x[14], f2_mul(W(754), x[12])), o[7]); o[8] = f2_fma(p, f2_mul(W(854), x[13]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); o[0] = f2_fma(p, f2_mul(W(65), x[12]), o[0]); o[2] = f2_fma(p, W(211), o[2]); o[4] = f2_fma(p, f2_mul(W(474), x[10]), o[4]); o[5] = f2_fma(p, f2_mul(W(563), x[11]), o[5]); o[6] = f2_fma(p, f2_mul(W(663), x[12]), o[6]); o[7] = f2_fma(p, f2_fma(W(757), x[15], f2_mul(W(756), x[13])), o[7]); o[8] = f2_fma(p, f2_mul(W(855), x[14]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); o[0] = f2_fma(p, f2_fma(W(67), x[15], f2_mul(W(66), x[13])), o[0]); o[3] = f2_fma(p, W(305), o[3]); o[4] = f2_fma(p, f2_mul(W(475), x[11]), o[4]); o[6] = f2_fma(p, f2_fma(W(665), x[15], f2_mul(W(664), x[13])), o[6]); o[7] = f2_fma(p, f2_fma(W(759), x[14], f2_mul(W(758), x[12])), o[7]); o[8] = f2_fma(p, f2_mul(W(856), x[15]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[12]); o[4] = f2_fma(p, f2_mul(W(476), x[12]), o[4]); o[5] = f2_fma(p, f2_fma(W(565), x[15], f2_mul(W(564), x[13])), o[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[13]); o[1] = f2_fma(p, W(100), o[1]); o[4] = f2_fma(p, f2_fma(W(478), x[15], f2_mul(W(477), x[13])), o[4]); o[5] = f2_fma(p, f2_mul(W(566), x[14]), o[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[14]); o[4] = f2_fma(p, f2_mul(W(479), x[14]), o[4]); o[5] = f2_fma(p, f2_mul(W(567), x[15]), o[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[15]); o[1] = f2_fma(p, W(101), o[1]); o[4] = f2_fma(p, f2_mul(W(480), x[15]), o[4]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); o[0] = f2_fma(p, f2_fma(W(69), x[8], f2_fma(W(68), x[6], W(6))), o[0]); o[1] = f2_fma(p, f2_fma(W(173), x[11], f2_mul(W(172), x[9])), o[1]); o[2] = f2_fma(p, f2_fma(W(271), x[14], f2_mul(W(270), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(377), x[15], f2_mul(W(376), x[13])), o[3]); o[5] = f2_fma(p, f2_mul(W(568), x[5]), o[5]); o[6] = f2_fma(p, f2_fma(W(666), x[6], W(606)), o[6]); o[7] = f2_fma(p, f2_mul(W(760), x[7]), o[7]); o[8] = f2_fma(p, f2_fma(W(857), x[8], W(798)), o[8]); } \
+      { const unsigned long long p = f2_mul(x[5], x[6]); o[1] = f2_fma(p, f2_fma(W(175), x[14], f2_mul(W(174), x[12])), o[1]); o[2] = f2_fma(p, f2_mul(W(272), x[11]), o[2]); o[3] = f2_fma(p, f2_mul(W(378), x[10]), o[3]); o[5] = f2_fma(p, f2_fma(W(569), x[6], W(508)), o[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[7]); o[1] = f2_fma(p, f2_fma(W(177), x[15], f2_mul(W(176), x[13])), o[1]); o[2] = f2_fma(p, f2_mul(W(273), x[10]), o[2]); o[3] = f2_fma(p, f2_fma(W(380), x[11], f2_mul(W(379), x[9])), o[3]); o[4] = f2_fma(p, W(419), o[4]); o[5] = f2_fma(p, f2_mul(W(570), x[7]), o[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[8]); o[1] = f2_fma(p, f2_fma(W(179), x[14], f2_mul(W(178), x[12])), o[1]); o[2] = f2_fma(p, f2_fma(W(275), x[11], f2_mul(W(274), x[9])), o[2]); o[3] = f2_fma(p, f2_mul(W(381), x[10]), o[3]); o[5] = f2_fma(p, f2_fma(W(571), x[8], W(509)), o[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); o[0] = f2_fma(p, f2_mul(W(70), x[14]), o[0]); o[4] = f2_fma(p, f2_mul(W(481), x[10]), o[4]); o[5] = f2_fma(p, f2_fma(W(573), x[11], f2_mul(W(572), x[9])), o[5]); o[6] = f2_fma(p, f2_mul(W(667), x[14]), o[6]); o[7] = f2_fma(p, f2_mul(W(761), x[13]), o[7]); o[8] = f2_fma(p, f2_fma(W(859), x[14], f2_mul(W(858), x[12])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); o[0] = f2_fma(p, f2_fma(W(72), x[15], f2_mul(W(71), x[13])), o[0]); o[3] = f2_fma(p, W(306), o[3]); o[4] = f2_fma(p, f2_mul(W(482), x[11]), o[4]); o[5] = f2_fma(p, f2_mul(W(574), x[10]), o[5]); o[6] = f2_fma(p, f2_fma(W(669), x[15], f2_mul(W(668), x[13])), o[6]); o[7] = f2_fma(p, f2_mul(W(762), x[12]), o[7]); o[8] = f2_fma(p, f2_fma(W(861), x[15], f2_mul(W(860), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); o[0] = f2_fma(p, f2_fma(W(74), x[14], f2_mul(W(73), x[12])), o[0]); o[2] = f2_fma(p, W(212), o[2]); o[5] = f2_fma(p, f2_mul(W(575), x[11]), o[5]); o[6] = f2_fma(p, f2_fma(W(671), x[14], f2_mul(W(670), x[12])), o[6]); o[7] = f2_fma(p, f2_fma(W(764), x[15], f2_mul(W(763), x[13])), o[7]); o[8] = f2_fma(p, f2_fma(W(863), x[14], f2_mul(W(862), x[12])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[5], x[12]); o[1] = f2_fma(p, W(102), o[1]); o[4] = f2_fma(p, f2_fma(W(484), x[15], f2_mul(W(483), x[13])), o[4]); o[5] = f2_fma(p, f2_fma(W(577), x[14], f2_mul(W(576), x[12])), o[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[13]); o[4] = f2_fma(p, f2_mul(W(485), x[14]), o[4]); o[5] = f2_fma(p, f2_fma(W(579), x[15], f2_mul(W(578), x[13])), o[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[14]); o[1] = f2_fma(p, W(103), o[1]); o[4] = f2_fma(p, f2_mul(W(486), x[15]), o[4]); o[5] = f2_fma(p, f2_mul(W(580), x[14]), o[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[15]); o[5] = f2_fma(p, f2_mul(W(581), x[15]), o[5]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); o[0] = f2_fma(p, f2_fma(W(75), x[6], W(7)), o[0]); o[1] = f2_fma(p, f2_mul(W(180), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(276), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(382), x[13]), o[3]); o[6] = f2_fma(p, f2_fma(W(672), x[6], W(607)), o[6]); o[7] = f2_fma(p, f2_mul(W(765), x[7]), o[7]); o[8] = f2_fma(p, f2_mul(W(864), x[8]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); o[0] = f2_fma(p, f2_mul(W(76), x[7]), o[0]); o[1] = f2_fma(p, f2_mul(W(181), x[10]), o[1]); o[2] = f2_fma(p, f2_mul(W(277), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(384), x[14], f2_mul(W(383), x[12])), o[3]); o[6] = f2_fma(p, f2_mul(W(673), x[7]), o[6]); o[7] = f2_fma(p, W(700), o[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); o[0] = f2_fma(p, f2_mul(W(77), x[8]), o[0]); o[1] = f2_fma(p, f2_fma(W(183), x[11], f2_mul(W(182), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(278), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(386), x[15], f2_mul(W(385), x[13])), o[3]); o[6] = f2_fma(p, f2_mul(W(674), x[8]), o[6]); o[8] = f2_fma(p, W(799), o[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); o[0] = f2_fma(p, f2_mul(W(78), x[9]), o[0]); o[4] = f2_fma(p, f2_mul(W(487), x[13]), o[4]); o[5] = f2_fma(p, f2_mul(W(582), x[14]), o[5]); o[6] = f2_fma(p, f2_mul(W(675), x[9]), o[6]); o[7] = f2_fma(p, f2_mul(W(766), x[10]), o[7]); o[8] = f2_fma(p, f2_mul(W(865), x[11]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[10]); o[4] = f2_fma(p, f2_mul(W(488), x[12]), o[4]); o[5] = f2_fma(p, f2_fma(W(584), x[15], f2_mul(W(583), x[13])), o[5]); o[6] = f2_fma(p, f2_mul(W(676), x[10]), o[6]); o[7] = f2_fma(p, f2_mul(W(767), x[11]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); o[0] = f2_fma(p, f2_mul(W(79), x[11]), o[0]); o[1] = f2_fma(p, W(104), o[1]); o[4] = f2_fma(p, f2_fma(W(490), x[15], f2_mul(W(489), x[13])), o[4]); o[5] = f2_fma(p, f2_fma(W(586), x[14], f2_mul(W(585), x[12])), o[5]); o[6] = f2_fma(p, f2_mul(W(677), x[11]), o[6]); o[8] = f2_fma(p, f2_mul(W(866), x[11]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); o[0] = f2_fma(p, f2_mul(W(80), x[12]), o[0]); o[2] = f2_fma(p, W(213), o[2]); o[6] = f2_fma(p, f2_mul(W(678), x[12]), o[6]); o[7] = f2_fma(p, f2_mul(W(768), x[13]), o[7]); o[8] = f2_fma(p, f2_mul(W(867), x[14]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); o[0] = f2_fma(p, f2_mul(W(81), x[13]), o[0]); o[3] = f2_fma(p, W(307), o[3]); o[6] = f2_fma(p, f2_mul(W(679), x[13]), o[6]); o[7] = f2_fma(p, f2_mul(W(769), x[14]), o[7]); o[8] = f2_fma(p, f2_fma(W(869), x[15], f2_mul(W(868), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[14]); o[6] = f2_fma(p, f2_mul(W(680), x[14]), o[6]); o[7] = f2_fma(p, f2_mul(W(770), x[15]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); o[0] = f2_fma(p, f2_mul(W(82), x[15]), o[0]); o[6] = f2_fma(p, f2_mul(W(681), x[15]), o[6]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); o[0] = f2_fma(p, f2_fma(W(83), x[8], W(8)), o[0]); o[1] = f2_fma(p, f2_fma(W(185), x[11], f2_mul(W(184), x[9])), o[1]); o[2] = f2_fma(p, f2_fma(W(280), x[14], f2_mul(W(279), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(388), x[15], f2_mul(W(387), x[13])), o[3]); o[6] = f2_fma(p, W(608), o[6]); o[7] = f2_fma(p, f2_mul(W(771), x[7]), o[7]); o[8] = f2_fma(p, f2_fma(W(870), x[8], W(800)), o[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[8]); o[1] = f2_fma(p, f2_mul(W(186), x[10]), o[1]); o[2] = f2_fma(p, f2_fma(W(282), x[15], f2_mul(W(281), x[13])), o[2]); o[3] = f2_fma(p, f2_fma(W(390), x[14], f2_mul(W(389), x[12])), o[3]); o[7] = f2_fma(p, f2_fma(W(772), x[8], W(701)), o[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); o[0] = f2_fma(p, f2_mul(W(84), x[10]), o[0]); o[4] = f2_fma(p, f2_fma(W(492), x[14], f2_mul(W(491), x[12])), o[4]); o[5] = f2_fma(p, f2_mul(W(587), x[13]), o[5]); o[6] = f2_fma(p, f2_mul(W(682), x[10]), o[6]); o[7] = f2_fma(p, f2_fma(W(774), x[11], f2_mul(W(773), x[9])), o[7]); o[8] = f2_fma(p, f2_mul(W(871), x[10]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); o[0] = f2_fma(p, f2_mul(W(85), x[11]), o[0]); o[1] = f2_fma(p, W(105), o[1]); o[4] = f2_fma(p, f2_fma(W(494), x[15], f2_mul(W(493), x[13])), o[4]); o[5] = f2_fma(p, f2_mul(W(588), x[12]), o[5]); o[6] = f2_fma(p, f2_mul(W(683), x[11]), o[6]); o[7] = f2_fma(p, f2_mul(W(775), x[10]), o[7]); o[8] = f2_fma(p, f2_mul(W(872), x[11]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[11]); o[4] = f2_fma(p, f2_fma(W(496), x[14], f2_mul(W(495), x[12])), o[4]); o[5] = f2_fma(p, f2_fma(W(590), x[15], f2_mul(W(589), x[13])), o[5]); o[7] = f2_fma(p, f2_mul(W(776), x[11]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); o[0] = f2_fma(p, f2_mul(W(86), x[13]), o[0]); o[3] = f2_fma(p, W(308), o[3]); o[6] = f2_fma(p, f2_mul(W(684), x[13]), o[6]); o[7] = f2_fma(p, f2_fma(W(778), x[14], f2_mul(W(777), x[12])), o[7]); o[8] = f2_fma(p, f2_fma(W(874), x[15], f2_mul(W(873), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); o[0] = f2_fma(p, f2_mul(W(87), x[14]), o[0]); o[2] = f2_fma(p, W(214), o[2]); o[6] = f2_fma(p, f2_mul(W(685), x[14]), o[6]); o[7] = f2_fma(p, f2_fma(W(780), x[15], f2_mul(W(779), x[13])), o[7]); o[8] = f2_fma(p, f2_mul(W(875), x[14]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); o[0] = f2_fma(p, f2_mul(W(88), x[15]), o[0]); o[3] = f2_fma(p, W(309), o[3]); o[6] = f2_fma(p, f2_mul(W(686), x[15]), o[6]); o[7] = f2_fma(p, f2_mul(W(781), x[14]), o[7]); o[8] = f2_fma(p, f2_mul(W(876), x[15]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[15]); o[7] = f2_fma(p, f2_mul(W(782), x[15]), o[7]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); o[0] = f2_fma(p, W(9), o[0]); o[1] = f2_fma(p, f2_fma(W(188), x[11], f2_mul(W(187), x[9])), o[1]); o[2] = f2_fma(p, f2_mul(W(283), x[12]), o[2]); o[3] = f2_fma(p, f2_fma(W(392), x[15], f2_mul(W(391), x[13])), o[3]); o[6] = f2_fma(p, W(609), o[6]); o[8] = f2_fma(p, f2_mul(W(877), x[8]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); o[0] = f2_fma(p, f2_mul(W(89), x[11]), o[0]); o[1] = f2_fma(p, W(106), o[1]); o[4] = f2_fma(p, f2_mul(W(497), x[13]), o[4]); o[5] = f2_fma(p, f2_fma(W(592), x[14], f2_mul(W(591), x[12])), o[5]); o[6] = f2_fma(p, f2_mul(W(687), x[11]), o[6]); o[7] = f2_fma(p, f2_mul(W(783), x[10]), o[7]); o[8] = f2_fma(p, f2_fma(W(879), x[11], f2_mul(W(878), x[9])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[10]); o[4] = f2_fma(p, f2_mul(W(498), x[14]), o[4]); o[5] = f2_fma(p, f2_fma(W(594), x[15], f2_mul(W(593), x[13])), o[5]); o[7] = f2_fma(p, f2_mul(W(784), x[11]), o[7]); o[8] = f2_fma(p, f2_mul(W(880), x[10]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); o[0] = f2_fma(p, f2_mul(W(90), x[11]), o[0]); o[1] = f2_fma(p, W(107), o[1]); o[4] = f2_fma(p, f2_mul(W(499), x[15]), o[4]); o[5] = f2_fma(p, f2_fma(W(596), x[14], f2_mul(W(595), x[12])), o[5]); o[6] = f2_fma(p, f2_mul(W(688), x[11]), o[6]); o[8] = f2_fma(p, f2_mul(W(881), x[11]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); o[0] = f2_fma(p, f2_mul(W(91), x[14]), o[0]); o[6] = f2_fma(p, f2_mul(W(689), x[14]), o[6]); o[7] = f2_fma(p, f2_fma(W(786), x[15], f2_mul(W(785), x[13])), o[7]); o[8] = f2_fma(p, f2_mul(W(882), x[12]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); o[0] = f2_fma(p, f2_fma(W(93), x[15], f2_mul(W(92), x[13])), o[0]); o[3] = f2_fma(p, W(310), o[3]); o[6] = f2_fma(p, f2_fma(W(691), x[15], f2_mul(W(690), x[13])), o[6]); o[7] = f2_fma(p, f2_mul(W(787), x[14]), o[7]); o[8] = f2_fma(p, f2_fma(W(884), x[15], f2_mul(W(883), x[13])), o[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[14]); o[2] = f2_fma(p, W(215), o[2]); o[7] = f2_fma(p, f2_mul(W(788), x[15]), o[7]); o[8] = f2_fma(p, f2_mul(W(885), x[14]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[15]); o[3] = f2_fma(p, W(311), o[3]); o[8] = f2_fma(p, f2_mul(W(886), x[15]), o[8]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); o[0] = f2_fma(p, W(10), o[0]); o[1] = f2_fma(p, f2_mul(W(189), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(284), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(393), x[13]), o[3]); o[6] = f2_fma(p, W(610), o[6]); } \
+      { const unsigned long long p = f2_mul(x[9], x[10]); o[1] = f2_fma(p, f2_mul(W(190), x[10]), o[1]); o[2] = f2_fma(p, f2_mul(W(285), x[13]), o[2]); o[3] = f2_fma(p, f2_fma(W(395), x[14], f2_mul(W(394), x[12])), o[3]); o[7] = f2_fma(p, W(702), o[7]); } \
+      { const unsigned long long p = f2_mul(x[9], x[11]); o[1] = f2_fma(p, f2_mul(W(191), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(286), x[14]), o[2]); o[3] = f2_fma(p, f2_mul(W(396), x[13]), o[3]); o[8] = f2_fma(p, W(801), o[8]); } \
+      { const unsigned long long p = f2_mul(x[9], x[12]); o[1] = f2_fma(p, f2_mul(W(192), x[14]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[9], x[13]); o[1] = f2_fma(p, f2_mul(W(193), x[13]), o[1]); o[4] = f2_fma(p, W(420), o[4]); } \
+      { const unsigned long long p = f2_mul(x[9], x[14]); o[1] = f2_fma(p, f2_mul(W(194), x[14]), o[1]); o[5] = f2_fma(p, W(510), o[5]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); o[0] = f2_fma(p, W(11), o[0]); o[1] = f2_fma(p, f2_mul(W(195), x[11]), o[1]); o[2] = f2_fma(p, f2_mul(W(287), x[12]), o[2]); o[3] = f2_fma(p, f2_fma(W(398), x[15], f2_mul(W(397), x[13])), o[3]); } \
+      { const unsigned long long p = f2_mul(x[10], x[11]); o[2] = f2_fma(p, f2_fma(W(289), x[15], f2_mul(W(288), x[13])), o[2]); o[3] = f2_fma(p, f2_mul(W(399), x[12]), o[3]); o[7] = f2_fma(p, W(703), o[7]); } \
+      { const unsigned long long p = f2_mul(x[10], x[12]); o[1] = f2_fma(p, f2_fma(W(197), x[15], f2_mul(W(196), x[13])), o[1]); o[4] = f2_fma(p, W(421), o[4]); } \
+      { const unsigned long long p = f2_mul(x[10], x[13]); o[5] = f2_fma(p, W(511), o[5]); } \
+      { const unsigned long long p = f2_mul(x[10], x[14]); o[1] = f2_fma(p, f2_mul(W(198), x[15]), o[1]); } \
+      { const unsigned long long p = f2_mul(x[10], x[15]); o[5] = f2_fma(p, W(512), o[5]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); o[0] = f2_fma(p, W(12), o[0]); o[1] = f2_fma(p, f2_mul(W(199), x[11]), o[1]); o[2] = f2_fma(p, f2_fma(W(291), x[14], f2_mul(W(290), x[12])), o[2]); o[3] = f2_fma(p, f2_fma(W(401), x[15], f2_mul(W(400), x[13])), o[3]); o[6] = f2_fma(p, W(611), o[6]); o[8] = f2_fma(p, W(802), o[8]); } \
+      { const unsigned long long p = f2_mul(x[11], x[12]); o[1] = f2_fma(p, f2_fma(W(201), x[14], f2_mul(W(200), x[12])), o[1]); o[5] = f2_fma(p, W(513), o[5]); } \
+      { const unsigned long long p = f2_mul(x[11], x[13]); o[1] = f2_fma(p, f2_fma(W(203), x[15], f2_mul(W(202), x[13])), o[1]); o[4] = f2_fma(p, W(422), o[4]); } \
+      { const unsigned long long p = f2_mul(x[11], x[14]); o[1] = f2_fma(p, f2_mul(W(204), x[14]), o[1]); o[5] = f2_fma(p, W(514), o[5]); } \
+      { const unsigned long long p = f2_mul(x[11], x[15]); o[1] = f2_fma(p, f2_mul(W(205), x[15]), o[1]); o[4] = f2_fma(p, W(423), o[4]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); o[0] = f2_fma(p, W(13), o[0]); o[2] = f2_fma(p, f2_mul(W(292), x[12]), o[2]); o[3] = f2_fma(p, f2_mul(W(402), x[13]), o[3]); o[6] = f2_fma(p, W(612), o[6]); } \
+      { const unsigned long long p = f2_mul(x[12], x[13]); o[2] = f2_fma(p, f2_mul(W(293), x[13]), o[2]); o[3] = f2_fma(p, f2_mul(W(403), x[14]), o[3]); o[7] = f2_fma(p, W(704), o[7]); } \
+      { const unsigned long long p = f2_mul(x[12], x[14]); o[2] = f2_fma(p, f2_mul(W(294), x[14]), o[2]); o[3] = f2_fma(p, f2_mul(W(404), x[15]), o[3]); o[8] = f2_fma(p, W(803), o[8]); } \
+      { const unsigned long long p = f2_mul(x[12], x[15]); o[2] = f2_fma(p, f2_mul(W(295), x[15]), o[2]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); o[0] = f2_fma(p, W(14), o[0]); o[2] = f2_fma(p, f2_mul(W(296), x[14]), o[2]); o[3] = f2_fma(p, f2_fma(W(406), x[15], f2_mul(W(405), x[13])), o[3]); o[6] = f2_fma(p, W(613), o[6]); o[8] = f2_fma(p, W(804), o[8]); } \
+      { const unsigned long long p = f2_mul(x[13], x[14]); o[2] = f2_fma(p, f2_mul(W(297), x[15]), o[2]); o[3] = f2_fma(p, f2_mul(W(407), x[14]), o[3]); o[7] = f2_fma(p, W(705), o[7]); } \
+      { const unsigned long long p = f2_mul(x[13], x[15]); o[3] = f2_fma(p, f2_mul(W(408), x[15]), o[3]); o[8] = f2_fma(p, W(805), o[8]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); o[0] = f2_fma(p, W(15), o[0]); o[3] = f2_fma(p, f2_mul(W(409), x[15]), o[3]); } \
+      { const unsigned long long p = f2_mul(x[14], x[15]); o[7] = f2_fma(p, W(706), o[7]); } \
+      { const unsigned long long p = f2_mul(x[15], x[15]); o[0] = f2_fma(p, W(16), o[0]); o[6] = f2_fma(p, W(614), o[6]); }
+#define SXB_S2_M0_REVERSE_BODY \
+      g[0] = f2_fma(W(0), adj[0], g[0]); \
+      g[1] = f2_fma(W(94), adj[1], g[1]); \
+      g[2] = f2_fma(W(206), adj[2], g[2]); \
+      g[3] = f2_fma(W(298), adj[3], g[3]); \
+      g[4] = f2_fma(W(410), adj[4], g[4]); \
+      g[5] = f2_fma(W(500), adj[5], g[5]); \
+      g[6] = f2_fma(W(597), adj[6], g[6]); \
+      g[7] = f2_fma(W(692), adj[7], g[7]); \
+      g[8] = f2_fma(W(789), adj[8], g[8]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); unsigned long long v; v = f2_mul(W(1), adj[0]); { const unsigned long long s = f2_mul(W(17), adj[0]); g[0] = f2_fma(s, p, g[0]); v = f2_fma(s, x[0], v); } { const unsigned long long s = f2_mul(W(108), adj[1]); g[1] = f2_fma(s, p, g[1]); v = f2_fma(s, x[1], v); } { const unsigned long long s = f2_mul(W(216), adj[2]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(312), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(424), adj[4]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(515), adj[5]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(615), adj[6]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(707), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(806), adj[8]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[0] = f2_fma(v, x[0], g[0]); g[0] = f2_fma(v, x[0], g[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); unsigned long long v; v = f2_mul(W(95), adj[1]); { const unsigned long long s = f2_fma(W(807), adj[8], f2_fma(W(616), adj[6], f2_mul(W(18), adj[0]))); g[1] = f2_fma(s, p, g[1]); v = f2_fma(s, x[1], v); } { const unsigned long long s = f2_mul(W(516), adj[5]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(425), adj[4]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(313), adj[3]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(217), adj[2]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(109), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(110), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(808), adj[8]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(708), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_fma(W(809), adj[8], f2_mul(W(617), adj[6])); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(517), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(426), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(518), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(427), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[1], g[0]); g[1] = f2_fma(v, x[0], g[1]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); unsigned long long v; v = f2_mul(W(207), adj[2]); { const unsigned long long s = f2_fma(W(618), adj[6], f2_mul(W(19), adj[0])); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(709), adj[7]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(111), adj[1]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(218), adj[2]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(314), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(428), adj[4]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(519), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(619), adj[6]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(710), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(810), adj[8]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[0] = f2_fma(v, x[2], g[0]); g[2] = f2_fma(v, x[0], g[2]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); unsigned long long v; v = f2_mul(W(299), adj[3]); { const unsigned long long s = f2_fma(W(811), adj[8], f2_fma(W(620), adj[6], f2_mul(W(20), adj[0]))); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(112), adj[1]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(315), adj[3]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(219), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(316), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(429), adj[4]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(520), adj[5]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(430), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(711), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(812), adj[8], f2_mul(W(621), adj[6])); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(712), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(813), adj[8]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[3], g[0]); g[3] = f2_fma(v, x[0], g[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); unsigned long long v; v = f2_mul(W(411), adj[4]); { const unsigned long long s = f2_fma(W(622), adj[6], f2_mul(W(21), adj[0])); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(713), adj[7]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(431), adj[4]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(521), adj[5]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(317), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(220), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(318), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(113), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(114), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[4], g[0]); g[4] = f2_fma(v, x[0], g[4]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); unsigned long long v; v = f2_mul(W(501), adj[5]); { const unsigned long long s = f2_fma(W(814), adj[8], f2_fma(W(623), adj[6], f2_mul(W(22), adj[0]))); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(522), adj[5]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(432), adj[4]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(523), adj[5]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(319), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(221), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(115), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(116), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[0] = f2_fma(v, x[5], g[0]); g[5] = f2_fma(v, x[0], g[5]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); unsigned long long v; v = f2_mul(W(598), adj[6]); { const unsigned long long s = f2_fma(W(624), adj[6], f2_mul(W(23), adj[0])); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(714), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(815), adj[8]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(117), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(222), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(320), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[0] = f2_fma(v, x[6], g[0]); g[6] = f2_fma(v, x[0], g[6]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); unsigned long long v; v = f2_mul(W(693), adj[7]); { const unsigned long long s = f2_fma(W(816), adj[8], f2_fma(W(625), adj[6], f2_mul(W(24), adj[0]))); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(715), adj[7]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(118), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(321), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(223), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(322), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[0] = f2_fma(v, x[7], g[0]); g[7] = f2_fma(v, x[0], g[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); unsigned long long v; v = f2_mul(W(790), adj[8]); { const unsigned long long s = f2_fma(W(626), adj[6], f2_mul(W(25), adj[0])); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(119), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(120), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(323), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(224), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(324), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[8], g[0]); g[8] = f2_fma(v, x[0], g[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); unsigned long long v; { const unsigned long long s = f2_fma(W(627), adj[6], f2_mul(W(26), adj[0])); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(716), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(817), adj[8]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(433), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(524), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[0] = f2_fma(v, x[9], g[0]); g[9] = f2_fma(v, x[0], g[9]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(27), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(717), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(434), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(525), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(526), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[10], g[0]); g[10] = f2_fma(v, x[0], g[10]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); unsigned long long v; { const unsigned long long s = f2_fma(W(818), adj[8], f2_fma(W(628), adj[6], f2_mul(W(28), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } { const unsigned long long s = f2_mul(W(527), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(435), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(528), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(436), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[11], g[0]); g[11] = f2_fma(v, x[0], g[11]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); unsigned long long v; { const unsigned long long s = f2_fma(W(629), adj[6], f2_mul(W(29), adj[0])); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(718), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(819), adj[8]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[0] = f2_fma(v, x[12], g[0]); g[12] = f2_fma(v, x[0], g[12]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); unsigned long long v; { const unsigned long long s = f2_fma(W(820), adj[8], f2_fma(W(630), adj[6], f2_mul(W(30), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(719), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(821), adj[8]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[13], g[0]); g[13] = f2_fma(v, x[0], g[13]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(31), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } { const unsigned long long s = f2_mul(W(720), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[0] = f2_fma(v, x[14], g[0]); g[14] = f2_fma(v, x[0], g[14]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); unsigned long long v; { const unsigned long long s = f2_fma(W(631), adj[6], f2_mul(W(32), adj[0])); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[0] = f2_fma(v, x[15], g[0]); g[15] = f2_fma(v, x[0], g[15]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); unsigned long long v; v = f2_fma(W(791), adj[8], f2_fma(W(599), adj[6], f2_mul(W(2), adj[0]))); { const unsigned long long s = f2_mul(W(121), adj[1]); g[1] = f2_fma(s, p, g[1]); v = f2_fma(s, x[1], v); } { const unsigned long long s = f2_mul(W(225), adj[2]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(325), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(437), adj[4]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(529), adj[5]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_fma(W(822), adj[8], f2_fma(W(632), adj[6], f2_mul(W(33), adj[0]))); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(721), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_fma(W(823), adj[8], f2_fma(W(633), adj[6], f2_mul(W(34), adj[0]))); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(122), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(123), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(226), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(326), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(227), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(327), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[1], g[1]); g[1] = f2_fma(v, x[1], g[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); unsigned long long v; v = f2_mul(W(502), adj[5]); { const unsigned long long s = f2_mul(W(124), adj[1]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(722), adj[7]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_fma(W(824), adj[8], f2_fma(W(634), adj[6], f2_mul(W(35), adj[0]))); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(530), adj[5]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(438), adj[4]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(531), adj[5]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(328), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(228), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(125), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(126), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[2], g[1]); g[2] = f2_fma(v, x[1], g[2]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); unsigned long long v; v = f2_mul(W(412), adj[4]); { const unsigned long long s = f2_mul(W(127), adj[1]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_fma(W(635), adj[6], f2_mul(W(36), adj[0])); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(723), adj[7]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(439), adj[4]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(532), adj[5]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(329), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(229), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(330), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(128), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(129), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[3], g[1]); g[3] = f2_fma(v, x[1], g[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); unsigned long long v; v = f2_mul(W(300), adj[3]); { const unsigned long long s = f2_mul(W(130), adj[1]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(331), adj[3]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(230), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(440), adj[4]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(533), adj[5]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(441), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(724), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(825), adj[8], f2_fma(W(636), adj[6], f2_mul(W(37), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(725), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_fma(W(826), adj[8], f2_fma(W(637), adj[6], f2_mul(W(38), adj[0]))); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[4], g[1]); g[4] = f2_fma(v, x[1], g[4]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); unsigned long long v; v = f2_mul(W(208), adj[2]); { const unsigned long long s = f2_mul(W(131), adj[1]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(231), adj[2]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(332), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(232), adj[2]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(534), adj[5]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(442), adj[4]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(535), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_fma(W(827), adj[8], f2_fma(W(638), adj[6], f2_mul(W(39), adj[0]))); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(726), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(828), adj[8], f2_fma(W(639), adj[6], f2_mul(W(40), adj[0]))); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(727), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[5], g[1]); g[5] = f2_fma(v, x[1], g[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); unsigned long long v; v = f2_mul(W(96), adj[1]); { const unsigned long long s = f2_mul(W(132), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(133), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(829), adj[8]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(728), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_fma(W(830), adj[8], f2_fma(W(640), adj[6], f2_mul(W(41), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(536), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(443), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(537), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(444), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[6], g[1]); g[6] = f2_fma(v, x[1], g[6]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(134), adj[1]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } { const unsigned long long s = f2_mul(W(729), adj[7]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_fma(W(831), adj[8], f2_fma(W(641), adj[6], f2_mul(W(42), adj[0]))); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(730), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(445), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(538), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(446), adj[4]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(539), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[7], g[1]); g[7] = f2_fma(v, x[1], g[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); unsigned long long v; v = f2_mul(W(97), adj[1]); { const unsigned long long s = f2_mul(W(135), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_fma(W(832), adj[8], f2_fma(W(642), adj[6], f2_mul(W(43), adj[0]))); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(731), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_fma(W(833), adj[8], f2_fma(W(643), adj[6], f2_mul(W(44), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(540), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(447), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(541), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(448), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[8], g[1]); g[8] = f2_fma(v, x[1], g[8]); } \
+      { const unsigned long long p = f2_mul(x[1], x[9]); unsigned long long v; v = f2_mul(W(792), adj[8]); { const unsigned long long s = f2_mul(W(136), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(137), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(333), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(233), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[9], g[1]); g[9] = f2_fma(v, x[1], g[9]); } \
+      { const unsigned long long p = f2_mul(x[1], x[10]); unsigned long long v; v = f2_mul(W(694), adj[7]); { const unsigned long long s = f2_mul(W(138), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(334), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(234), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(235), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[10], g[1]); g[10] = f2_fma(v, x[1], g[10]); } \
+      { const unsigned long long p = f2_mul(x[1], x[11]); unsigned long long v; v = f2_fma(W(793), adj[8], f2_mul(W(600), adj[6])); { const unsigned long long s = f2_mul(W(139), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(236), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(335), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(237), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(336), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[11], g[1]); g[11] = f2_fma(v, x[1], g[11]); } \
+      { const unsigned long long p = f2_mul(x[1], x[12]); unsigned long long v; v = f2_mul(W(503), adj[5]); { const unsigned long long s = f2_mul(W(140), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(141), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[12], g[1]); g[12] = f2_fma(v, x[1], g[12]); } \
+      { const unsigned long long p = f2_mul(x[1], x[13]); unsigned long long v; v = f2_mul(W(413), adj[4]); { const unsigned long long s = f2_mul(W(142), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(143), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[13], g[1]); g[13] = f2_fma(v, x[1], g[13]); } \
+      { const unsigned long long p = f2_mul(x[1], x[14]); unsigned long long v; v = f2_mul(W(504), adj[5]); { const unsigned long long s = f2_mul(W(144), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[14], g[1]); g[14] = f2_fma(v, x[1], g[14]); } \
+      { const unsigned long long p = f2_mul(x[1], x[15]); unsigned long long v; v = f2_mul(W(414), adj[4]); { const unsigned long long s = f2_mul(W(145), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[15], g[1]); g[15] = f2_fma(v, x[1], g[15]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); unsigned long long v; v = f2_fma(W(601), adj[6], f2_mul(W(3), adj[0])); { const unsigned long long s = f2_mul(W(238), adj[2]); g[2] = f2_fma(s, p, g[2]); v = f2_fma(s, x[2], v); } { const unsigned long long s = f2_mul(W(337), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(449), adj[4]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(542), adj[5]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_fma(W(644), adj[6], f2_mul(W(45), adj[0])); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(732), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(834), adj[8]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(146), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(239), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(338), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[2] = f2_fma(v, x[2], g[2]); g[2] = f2_fma(v, x[2], g[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); unsigned long long v; v = f2_mul(W(695), adj[7]); { const unsigned long long s = f2_mul(W(240), adj[2]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(543), adj[5]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(450), adj[4]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(733), adj[7]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_fma(W(835), adj[8], f2_fma(W(645), adj[6], f2_mul(W(46), adj[0]))); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(734), adj[7]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(147), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(339), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(241), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(340), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[3], g[2]); g[3] = f2_fma(v, x[2], g[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(242), adj[2]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } { const unsigned long long s = f2_mul(W(341), adj[3]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(148), adj[1]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(735), adj[7]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_fma(W(646), adj[6], f2_mul(W(47), adj[0])); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(736), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(451), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(544), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(545), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[4], g[2]); g[4] = f2_fma(v, x[2], g[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); unsigned long long v; v = f2_mul(W(98), adj[1]); { const unsigned long long s = f2_mul(W(243), adj[2]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(149), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(150), adj[1]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(836), adj[8]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(737), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_fma(W(837), adj[8], f2_fma(W(647), adj[6], f2_mul(W(48), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(546), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(452), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(547), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(453), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[5], g[2]); g[5] = f2_fma(v, x[2], g[5]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); unsigned long long v; v = f2_mul(W(209), adj[2]); { const unsigned long long s = f2_mul(W(244), adj[2]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(342), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(454), adj[4]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(548), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_fma(W(648), adj[6], f2_mul(W(49), adj[0])); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(738), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(838), adj[8]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[6], g[2]); g[6] = f2_fma(v, x[2], g[6]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); unsigned long long v; v = f2_mul(W(301), adj[3]); { const unsigned long long s = f2_mul(W(245), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(343), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(455), adj[4]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(549), adj[5]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(456), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(739), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(839), adj[8], f2_fma(W(649), adj[6], f2_mul(W(50), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(740), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(840), adj[8]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[7], g[2]); g[7] = f2_fma(v, x[2], g[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(246), adj[2]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } { const unsigned long long s = f2_mul(W(550), adj[5]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(551), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(841), adj[8]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(741), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(650), adj[6], f2_mul(W(51), adj[0])); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(742), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[8], g[2]); g[8] = f2_fma(v, x[2], g[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(247), adj[2]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(344), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(151), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[9], g[2]); g[9] = f2_fma(v, x[2], g[9]); } \
+      { const unsigned long long p = f2_mul(x[2], x[10]); unsigned long long v; v = f2_mul(W(415), adj[4]); { const unsigned long long s = f2_mul(W(248), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(345), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(152), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(153), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[10], g[2]); g[10] = f2_fma(v, x[2], g[10]); } \
+      { const unsigned long long p = f2_mul(x[2], x[11]); unsigned long long v; v = f2_mul(W(505), adj[5]); { const unsigned long long s = f2_mul(W(249), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(154), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(155), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[11], g[2]); g[11] = f2_fma(v, x[2], g[11]); } \
+      { const unsigned long long p = f2_mul(x[2], x[12]); unsigned long long v; v = f2_mul(W(602), adj[6]); { const unsigned long long s = f2_mul(W(250), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(346), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[2] = f2_fma(v, x[12], g[2]); g[12] = f2_fma(v, x[2], g[12]); } \
+      { const unsigned long long p = f2_mul(x[2], x[13]); unsigned long long v; v = f2_mul(W(696), adj[7]); { const unsigned long long s = f2_mul(W(251), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(347), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[2] = f2_fma(v, x[13], g[2]); g[13] = f2_fma(v, x[2], g[13]); } \
+      { const unsigned long long p = f2_mul(x[2], x[14]); unsigned long long v; v = f2_mul(W(794), adj[8]); { const unsigned long long s = f2_mul(W(252), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(348), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[2] = f2_fma(v, x[14], g[2]); g[14] = f2_fma(v, x[2], g[14]); } \
+      { const unsigned long long p = f2_mul(x[2], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(253), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[2] = f2_fma(v, x[15], g[2]); g[15] = f2_fma(v, x[2], g[15]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); unsigned long long v; v = f2_fma(W(795), adj[8], f2_fma(W(603), adj[6], f2_mul(W(4), adj[0]))); { const unsigned long long s = f2_mul(W(349), adj[3]); g[3] = f2_fma(s, p, g[3]); v = f2_fma(s, x[3], v); } { const unsigned long long s = f2_mul(W(457), adj[4]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(552), adj[5]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_fma(W(842), adj[8], f2_fma(W(651), adj[6], f2_mul(W(52), adj[0]))); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(743), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_fma(W(843), adj[8], f2_fma(W(652), adj[6], f2_mul(W(53), adj[0]))); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(156), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(157), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(254), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(350), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(255), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(351), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[3], g[3]); g[3] = f2_fma(v, x[3], g[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); unsigned long long v; v = f2_mul(W(99), adj[1]); { const unsigned long long s = f2_mul(W(352), adj[3]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(256), adj[2]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(158), adj[1]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_fma(W(844), adj[8], f2_fma(W(653), adj[6], f2_mul(W(54), adj[0]))); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(744), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_fma(W(845), adj[8], f2_fma(W(654), adj[6], f2_mul(W(55), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(553), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(458), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(554), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(459), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[4], g[3]); g[4] = f2_fma(v, x[3], g[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(353), adj[3]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } { const unsigned long long s = f2_mul(W(159), adj[1]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(745), adj[7]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_fma(W(846), adj[8], f2_fma(W(655), adj[6], f2_mul(W(56), adj[0]))); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(746), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(460), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(555), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(461), adj[4]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(556), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[5], g[3]); g[5] = f2_fma(v, x[3], g[5]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); unsigned long long v; v = f2_mul(W(302), adj[3]); { const unsigned long long s = f2_mul(W(354), adj[3]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(257), adj[2]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(355), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(462), adj[4]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(557), adj[5]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(463), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(747), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(847), adj[8], f2_fma(W(656), adj[6], f2_mul(W(57), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(748), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(848), adj[8]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[6], g[3]); g[6] = f2_fma(v, x[3], g[6]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); unsigned long long v; v = f2_mul(W(210), adj[2]); { const unsigned long long s = f2_mul(W(356), adj[3]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(258), adj[2]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(558), adj[5]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(464), adj[4]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(559), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_fma(W(849), adj[8], f2_fma(W(657), adj[6], f2_mul(W(58), adj[0]))); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(749), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(850), adj[8], f2_fma(W(658), adj[6], f2_mul(W(59), adj[0]))); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(750), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[7], g[3]); g[7] = f2_fma(v, x[3], g[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); unsigned long long v; v = f2_mul(W(303), adj[3]); { const unsigned long long s = f2_mul(W(357), adj[3]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(465), adj[4]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(560), adj[5]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(466), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(751), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(851), adj[8], f2_fma(W(659), adj[6], f2_mul(W(60), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(752), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_fma(W(852), adj[8], f2_fma(W(660), adj[6], f2_mul(W(61), adj[0]))); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[8], g[3]); g[8] = f2_fma(v, x[3], g[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[9]); unsigned long long v; v = f2_mul(W(416), adj[4]); { const unsigned long long s = f2_mul(W(358), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(259), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(359), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(160), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[3] = f2_fma(v, x[9], g[3]); g[9] = f2_fma(v, x[3], g[9]); } \
+      { const unsigned long long p = f2_mul(x[3], x[10]); unsigned long long v; v = f2_mul(W(506), adj[5]); { const unsigned long long s = f2_mul(W(360), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(260), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(161), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } g[3] = f2_fma(v, x[10], g[3]); g[10] = f2_fma(v, x[3], g[10]); } \
+      { const unsigned long long p = f2_mul(x[3], x[11]); unsigned long long v; v = f2_mul(W(417), adj[4]); { const unsigned long long s = f2_mul(W(361), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(162), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(163), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[11], g[3]); g[11] = f2_fma(v, x[3], g[11]); } \
+      { const unsigned long long p = f2_mul(x[3], x[12]); unsigned long long v; v = f2_mul(W(697), adj[7]); { const unsigned long long s = f2_mul(W(362), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(261), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(363), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[12], g[3]); g[12] = f2_fma(v, x[3], g[12]); } \
+      { const unsigned long long p = f2_mul(x[3], x[13]); unsigned long long v; v = f2_fma(W(796), adj[8], f2_mul(W(604), adj[6])); { const unsigned long long s = f2_mul(W(364), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(262), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(365), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[13], g[3]); g[13] = f2_fma(v, x[3], g[13]); } \
+      { const unsigned long long p = f2_mul(x[3], x[14]); unsigned long long v; v = f2_mul(W(698), adj[7]); { const unsigned long long s = f2_mul(W(366), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(263), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[14], g[3]); g[14] = f2_fma(v, x[3], g[14]); } \
+      { const unsigned long long p = f2_mul(x[3], x[15]); unsigned long long v; v = f2_mul(W(797), adj[8]); { const unsigned long long s = f2_mul(W(367), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[15], g[3]); g[15] = f2_fma(v, x[3], g[15]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); unsigned long long v; v = f2_fma(W(605), adj[6], f2_mul(W(5), adj[0])); { const unsigned long long s = f2_mul(W(467), adj[4]); g[4] = f2_fma(s, p, g[4]); v = f2_fma(s, x[4], v); } { const unsigned long long s = f2_mul(W(561), adj[5]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_fma(W(661), adj[6], f2_mul(W(62), adj[0])); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(753), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(853), adj[8]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(164), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(165), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(264), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(368), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(369), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[4], g[4]); g[4] = f2_fma(v, x[4], g[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); unsigned long long v; v = f2_mul(W(699), adj[7]); { const unsigned long long s = f2_mul(W(468), adj[4]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_mul(W(63), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(166), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(370), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(265), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(371), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(266), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[5], g[4]); g[5] = f2_fma(v, x[4], g[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[6]); unsigned long long v; v = f2_mul(W(418), adj[4]); { const unsigned long long s = f2_mul(W(469), adj[4]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(372), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(267), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(373), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(167), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(168), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[6], g[4]); g[6] = f2_fma(v, x[4], g[6]); } \
+      { const unsigned long long p = f2_mul(x[4], x[7]); unsigned long long v; v = f2_mul(W(507), adj[5]); { const unsigned long long s = f2_mul(W(470), adj[4]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(268), adj[2]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(374), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(269), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(169), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(170), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[4] = f2_fma(v, x[7], g[4]); g[7] = f2_fma(v, x[4], g[7]); } \
+      { const unsigned long long p = f2_mul(x[4], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(471), adj[4]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } { const unsigned long long s = f2_mul(W(375), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(171), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[8], g[4]); g[8] = f2_fma(v, x[4], g[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); unsigned long long v; v = f2_mul(W(304), adj[3]); { const unsigned long long s = f2_mul(W(472), adj[4]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(562), adj[5]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(473), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(754), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(854), adj[8], f2_fma(W(662), adj[6], f2_mul(W(64), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(755), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[4] = f2_fma(v, x[9], g[4]); g[9] = f2_fma(v, x[4], g[9]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); unsigned long long v; v = f2_mul(W(211), adj[2]); { const unsigned long long s = f2_mul(W(474), adj[4]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(563), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_fma(W(663), adj[6], f2_mul(W(65), adj[0])); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(756), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(855), adj[8]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(757), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[10], g[4]); g[10] = f2_fma(v, x[4], g[10]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); unsigned long long v; v = f2_mul(W(305), adj[3]); { const unsigned long long s = f2_mul(W(475), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(758), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(664), adj[6], f2_mul(W(66), adj[0])); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(759), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_fma(W(856), adj[8], f2_fma(W(665), adj[6], f2_mul(W(67), adj[0]))); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[11], g[4]); g[11] = f2_fma(v, x[4], g[11]); } \
+      { const unsigned long long p = f2_mul(x[4], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(476), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(564), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(565), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[12], g[4]); g[12] = f2_fma(v, x[4], g[12]); } \
+      { const unsigned long long p = f2_mul(x[4], x[13]); unsigned long long v; v = f2_mul(W(100), adj[1]); { const unsigned long long s = f2_mul(W(477), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(566), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(478), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[13], g[4]); g[13] = f2_fma(v, x[4], g[13]); } \
+      { const unsigned long long p = f2_mul(x[4], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(479), adj[4]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } { const unsigned long long s = f2_mul(W(567), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[14], g[4]); g[14] = f2_fma(v, x[4], g[14]); } \
+      { const unsigned long long p = f2_mul(x[4], x[15]); unsigned long long v; v = f2_mul(W(101), adj[1]); { const unsigned long long s = f2_mul(W(480), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[15], g[4]); g[15] = f2_fma(v, x[4], g[15]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); unsigned long long v; v = f2_fma(W(798), adj[8], f2_fma(W(606), adj[6], f2_mul(W(6), adj[0]))); { const unsigned long long s = f2_mul(W(568), adj[5]); g[5] = f2_fma(s, p, g[5]); v = f2_fma(s, x[5], v); } { const unsigned long long s = f2_fma(W(666), adj[6], f2_mul(W(68), adj[0])); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(760), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_fma(W(857), adj[8], f2_mul(W(69), adj[0])); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(172), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(173), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(270), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(376), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(271), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(377), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[5], g[5]); g[5] = f2_fma(v, x[5], g[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[6]); unsigned long long v; v = f2_mul(W(508), adj[5]); { const unsigned long long s = f2_mul(W(569), adj[5]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(378), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(272), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(174), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(175), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[6], g[5]); g[6] = f2_fma(v, x[5], g[6]); } \
+      { const unsigned long long p = f2_mul(x[5], x[7]); unsigned long long v; v = f2_mul(W(419), adj[4]); { const unsigned long long s = f2_mul(W(570), adj[5]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(379), adj[3]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(273), adj[2]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(380), adj[3]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(176), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(177), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[7], g[5]); g[7] = f2_fma(v, x[5], g[7]); } \
+      { const unsigned long long p = f2_mul(x[5], x[8]); unsigned long long v; v = f2_mul(W(509), adj[5]); { const unsigned long long s = f2_mul(W(571), adj[5]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(274), adj[2]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(381), adj[3]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(275), adj[2]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(178), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(179), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[8], g[5]); g[8] = f2_fma(v, x[5], g[8]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(572), adj[5]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(481), adj[4]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(573), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(858), adj[8]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(761), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(859), adj[8], f2_fma(W(667), adj[6], f2_mul(W(70), adj[0]))); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[9], g[5]); g[9] = f2_fma(v, x[5], g[9]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); unsigned long long v; v = f2_mul(W(306), adj[3]); { const unsigned long long s = f2_mul(W(574), adj[5]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(482), adj[4]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(762), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(860), adj[8], f2_fma(W(668), adj[6], f2_mul(W(71), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(861), adj[8], f2_fma(W(669), adj[6], f2_mul(W(72), adj[0]))); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[10], g[5]); g[10] = f2_fma(v, x[5], g[10]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); unsigned long long v; v = f2_mul(W(212), adj[2]); { const unsigned long long s = f2_mul(W(575), adj[5]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_fma(W(862), adj[8], f2_fma(W(670), adj[6], f2_mul(W(73), adj[0]))); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(763), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(863), adj[8], f2_fma(W(671), adj[6], f2_mul(W(74), adj[0]))); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(764), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[11], g[5]); g[11] = f2_fma(v, x[5], g[11]); } \
+      { const unsigned long long p = f2_mul(x[5], x[12]); unsigned long long v; v = f2_mul(W(102), adj[1]); { const unsigned long long s = f2_mul(W(576), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(483), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(577), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(484), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[12], g[5]); g[12] = f2_fma(v, x[5], g[12]); } \
+      { const unsigned long long p = f2_mul(x[5], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(578), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(485), adj[4]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(579), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[13], g[5]); g[13] = f2_fma(v, x[5], g[13]); } \
+      { const unsigned long long p = f2_mul(x[5], x[14]); unsigned long long v; v = f2_mul(W(103), adj[1]); { const unsigned long long s = f2_mul(W(580), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(486), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[14], g[5]); g[14] = f2_fma(v, x[5], g[14]); } \
+      { const unsigned long long p = f2_mul(x[5], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(581), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[5] = f2_fma(v, x[15], g[5]); g[15] = f2_fma(v, x[5], g[15]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); unsigned long long v; v = f2_fma(W(607), adj[6], f2_mul(W(7), adj[0])); { const unsigned long long s = f2_fma(W(672), adj[6], f2_mul(W(75), adj[0])); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(765), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(864), adj[8]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(180), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(276), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(382), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[6] = f2_fma(v, x[6], g[6]); g[6] = f2_fma(v, x[6], g[6]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); unsigned long long v; v = f2_mul(W(700), adj[7]); { const unsigned long long s = f2_fma(W(673), adj[6], f2_mul(W(76), adj[0])); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_mul(W(181), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(383), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(277), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(384), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[6] = f2_fma(v, x[7], g[6]); g[7] = f2_fma(v, x[6], g[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); unsigned long long v; v = f2_mul(W(799), adj[8]); { const unsigned long long s = f2_fma(W(674), adj[6], f2_mul(W(77), adj[0])); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(182), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(183), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(385), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(278), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(386), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[6] = f2_fma(v, x[8], g[6]); g[8] = f2_fma(v, x[6], g[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); unsigned long long v; { const unsigned long long s = f2_fma(W(675), adj[6], f2_mul(W(78), adj[0])); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(766), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(865), adj[8]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(487), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(582), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[6] = f2_fma(v, x[9], g[6]); g[9] = f2_fma(v, x[6], g[9]); } \
+      { const unsigned long long p = f2_mul(x[6], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(676), adj[6]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(767), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(488), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(583), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(584), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[6] = f2_fma(v, x[10], g[6]); g[10] = f2_fma(v, x[6], g[10]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); unsigned long long v; v = f2_mul(W(104), adj[1]); { const unsigned long long s = f2_fma(W(866), adj[8], f2_fma(W(677), adj[6], f2_mul(W(79), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(585), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(489), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(586), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(490), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[6] = f2_fma(v, x[11], g[6]); g[11] = f2_fma(v, x[6], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); unsigned long long v; v = f2_mul(W(213), adj[2]); { const unsigned long long s = f2_fma(W(678), adj[6], f2_mul(W(80), adj[0])); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(768), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(867), adj[8]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[6] = f2_fma(v, x[12], g[6]); g[12] = f2_fma(v, x[6], g[12]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); unsigned long long v; v = f2_mul(W(307), adj[3]); { const unsigned long long s = f2_fma(W(868), adj[8], f2_fma(W(679), adj[6], f2_mul(W(81), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(769), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(869), adj[8]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[6] = f2_fma(v, x[13], g[6]); g[13] = f2_fma(v, x[6], g[13]); } \
+      { const unsigned long long p = f2_mul(x[6], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(680), adj[6]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } { const unsigned long long s = f2_mul(W(770), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[6] = f2_fma(v, x[14], g[6]); g[14] = f2_fma(v, x[6], g[14]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); unsigned long long v; { const unsigned long long s = f2_fma(W(681), adj[6], f2_mul(W(82), adj[0])); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[6] = f2_fma(v, x[15], g[6]); g[15] = f2_fma(v, x[6], g[15]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); unsigned long long v; v = f2_fma(W(800), adj[8], f2_fma(W(608), adj[6], f2_mul(W(8), adj[0]))); { const unsigned long long s = f2_mul(W(771), adj[7]); g[7] = f2_fma(s, p, g[7]); v = f2_fma(s, x[7], v); } { const unsigned long long s = f2_fma(W(870), adj[8], f2_mul(W(83), adj[0])); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(184), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(185), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(279), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(387), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(280), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(388), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[7], g[7]); g[7] = f2_fma(v, x[7], g[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[8]); unsigned long long v; v = f2_mul(W(701), adj[7]); { const unsigned long long s = f2_mul(W(772), adj[7]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(186), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(389), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(281), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(390), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(282), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[8], g[7]); g[8] = f2_fma(v, x[7], g[8]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(773), adj[7]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_fma(W(871), adj[8], f2_fma(W(682), adj[6], f2_mul(W(84), adj[0]))); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(774), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(491), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(587), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(492), adj[4]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[7] = f2_fma(v, x[9], g[7]); g[9] = f2_fma(v, x[7], g[9]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); unsigned long long v; v = f2_mul(W(105), adj[1]); { const unsigned long long s = f2_mul(W(775), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_fma(W(872), adj[8], f2_fma(W(683), adj[6], f2_mul(W(85), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(588), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(493), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(494), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[10], g[7]); g[10] = f2_fma(v, x[7], g[10]); } \
+      { const unsigned long long p = f2_mul(x[7], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(776), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } { const unsigned long long s = f2_mul(W(495), adj[4]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(589), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(496), adj[4]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(590), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[11], g[7]); g[11] = f2_fma(v, x[7], g[11]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); unsigned long long v; v = f2_mul(W(308), adj[3]); { const unsigned long long s = f2_mul(W(777), adj[7]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_fma(W(873), adj[8], f2_fma(W(684), adj[6], f2_mul(W(86), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(778), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(874), adj[8]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[12], g[7]); g[12] = f2_fma(v, x[7], g[12]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); unsigned long long v; v = f2_mul(W(214), adj[2]); { const unsigned long long s = f2_mul(W(779), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(875), adj[8], f2_fma(W(685), adj[6], f2_mul(W(87), adj[0]))); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(780), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[13], g[7]); g[13] = f2_fma(v, x[7], g[13]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); unsigned long long v; v = f2_mul(W(309), adj[3]); { const unsigned long long s = f2_mul(W(781), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_fma(W(876), adj[8], f2_fma(W(686), adj[6], f2_mul(W(88), adj[0]))); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[7] = f2_fma(v, x[14], g[7]); g[14] = f2_fma(v, x[7], g[14]); } \
+      { const unsigned long long p = f2_mul(x[7], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(782), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[7] = f2_fma(v, x[15], g[7]); g[15] = f2_fma(v, x[7], g[15]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); unsigned long long v; v = f2_fma(W(609), adj[6], f2_mul(W(9), adj[0])); { const unsigned long long s = f2_mul(W(877), adj[8]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } { const unsigned long long s = f2_mul(W(187), adj[1]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(188), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(283), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(391), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(392), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[8], g[8]); g[8] = f2_fma(v, x[8], g[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); unsigned long long v; v = f2_mul(W(106), adj[1]); { const unsigned long long s = f2_mul(W(878), adj[8]); g[9] = f2_fma(s, p, g[9]); v = f2_fma(s, x[9], v); } { const unsigned long long s = f2_mul(W(783), adj[7]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_fma(W(879), adj[8], f2_fma(W(687), adj[6], f2_mul(W(89), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(591), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(497), adj[4]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(592), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[8] = f2_fma(v, x[9], g[8]); g[9] = f2_fma(v, x[8], g[9]); } \
+      { const unsigned long long p = f2_mul(x[8], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(880), adj[8]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } { const unsigned long long s = f2_mul(W(784), adj[7]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(593), adj[5]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(498), adj[4]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(594), adj[5]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[10], g[8]); g[10] = f2_fma(v, x[8], g[10]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); unsigned long long v; v = f2_mul(W(107), adj[1]); { const unsigned long long s = f2_fma(W(881), adj[8], f2_fma(W(688), adj[6], f2_mul(W(90), adj[0]))); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(595), adj[5]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(596), adj[5]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(499), adj[4]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[11], g[8]); g[11] = f2_fma(v, x[8], g[11]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(882), adj[8]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(785), adj[7]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_fma(W(689), adj[6], f2_mul(W(91), adj[0])); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(786), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[12], g[8]); g[12] = f2_fma(v, x[8], g[12]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); unsigned long long v; v = f2_mul(W(310), adj[3]); { const unsigned long long s = f2_fma(W(883), adj[8], f2_fma(W(690), adj[6], f2_mul(W(92), adj[0]))); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(787), adj[7]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_fma(W(884), adj[8], f2_fma(W(691), adj[6], f2_mul(W(93), adj[0]))); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[13], g[8]); g[13] = f2_fma(v, x[8], g[13]); } \
+      { const unsigned long long p = f2_mul(x[8], x[14]); unsigned long long v; v = f2_mul(W(215), adj[2]); { const unsigned long long s = f2_mul(W(885), adj[8]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(788), adj[7]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[14], g[8]); g[14] = f2_fma(v, x[8], g[14]); } \
+      { const unsigned long long p = f2_mul(x[8], x[15]); unsigned long long v; v = f2_mul(W(311), adj[3]); { const unsigned long long s = f2_mul(W(886), adj[8]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[15], g[8]); g[15] = f2_fma(v, x[8], g[15]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); unsigned long long v; v = f2_fma(W(610), adj[6], f2_mul(W(10), adj[0])); { const unsigned long long s = f2_mul(W(189), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(284), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(393), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[9] = f2_fma(v, x[9], g[9]); g[9] = f2_fma(v, x[9], g[9]); } \
+      { const unsigned long long p = f2_mul(x[9], x[10]); unsigned long long v; v = f2_mul(W(702), adj[7]); { const unsigned long long s = f2_mul(W(190), adj[1]); g[10] = f2_fma(s, p, g[10]); v = f2_fma(s, x[10], v); } { const unsigned long long s = f2_mul(W(394), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(285), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(395), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[9] = f2_fma(v, x[10], g[9]); g[10] = f2_fma(v, x[9], g[10]); } \
+      { const unsigned long long p = f2_mul(x[9], x[11]); unsigned long long v; v = f2_mul(W(801), adj[8]); { const unsigned long long s = f2_mul(W(191), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(396), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(286), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[9] = f2_fma(v, x[11], g[9]); g[11] = f2_fma(v, x[9], g[11]); } \
+      { const unsigned long long p = f2_mul(x[9], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(192), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[9] = f2_fma(v, x[12], g[9]); g[12] = f2_fma(v, x[9], g[12]); } \
+      { const unsigned long long p = f2_mul(x[9], x[13]); unsigned long long v; v = f2_mul(W(420), adj[4]); { const unsigned long long s = f2_mul(W(193), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[9] = f2_fma(v, x[13], g[9]); g[13] = f2_fma(v, x[9], g[13]); } \
+      { const unsigned long long p = f2_mul(x[9], x[14]); unsigned long long v; v = f2_mul(W(510), adj[5]); { const unsigned long long s = f2_mul(W(194), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[9] = f2_fma(v, x[14], g[9]); g[14] = f2_fma(v, x[9], g[14]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); unsigned long long v; v = f2_mul(W(11), adj[0]); { const unsigned long long s = f2_mul(W(195), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(287), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(397), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(398), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[10] = f2_fma(v, x[10], g[10]); g[10] = f2_fma(v, x[10], g[10]); } \
+      { const unsigned long long p = f2_mul(x[10], x[11]); unsigned long long v; v = f2_mul(W(703), adj[7]); { const unsigned long long s = f2_mul(W(399), adj[3]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(288), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(289), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[10] = f2_fma(v, x[11], g[10]); g[11] = f2_fma(v, x[10], g[11]); } \
+      { const unsigned long long p = f2_mul(x[10], x[12]); unsigned long long v; v = f2_mul(W(421), adj[4]); { const unsigned long long s = f2_mul(W(196), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(197), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[10] = f2_fma(v, x[12], g[10]); g[12] = f2_fma(v, x[10], g[12]); } \
+      { unsigned long long v; v = f2_mul(W(511), adj[5]); g[10] = f2_fma(v, x[13], g[10]); g[13] = f2_fma(v, x[10], g[13]); } \
+      { const unsigned long long p = f2_mul(x[10], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(198), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[10] = f2_fma(v, x[14], g[10]); g[14] = f2_fma(v, x[10], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(512), adj[5]); g[10] = f2_fma(v, x[15], g[10]); g[15] = f2_fma(v, x[10], g[15]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); unsigned long long v; v = f2_fma(W(802), adj[8], f2_fma(W(611), adj[6], f2_mul(W(12), adj[0]))); { const unsigned long long s = f2_mul(W(199), adj[1]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } { const unsigned long long s = f2_mul(W(290), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(400), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(291), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(401), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[11] = f2_fma(v, x[11], g[11]); g[11] = f2_fma(v, x[11], g[11]); } \
+      { const unsigned long long p = f2_mul(x[11], x[12]); unsigned long long v; v = f2_mul(W(513), adj[5]); { const unsigned long long s = f2_mul(W(200), adj[1]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(201), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[11] = f2_fma(v, x[12], g[11]); g[12] = f2_fma(v, x[11], g[12]); } \
+      { const unsigned long long p = f2_mul(x[11], x[13]); unsigned long long v; v = f2_mul(W(422), adj[4]); { const unsigned long long s = f2_mul(W(202), adj[1]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(203), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[11] = f2_fma(v, x[13], g[11]); g[13] = f2_fma(v, x[11], g[13]); } \
+      { const unsigned long long p = f2_mul(x[11], x[14]); unsigned long long v; v = f2_mul(W(514), adj[5]); { const unsigned long long s = f2_mul(W(204), adj[1]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[11] = f2_fma(v, x[14], g[11]); g[14] = f2_fma(v, x[11], g[14]); } \
+      { const unsigned long long p = f2_mul(x[11], x[15]); unsigned long long v; v = f2_mul(W(423), adj[4]); { const unsigned long long s = f2_mul(W(205), adj[1]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[11] = f2_fma(v, x[15], g[11]); g[15] = f2_fma(v, x[11], g[15]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); unsigned long long v; v = f2_fma(W(612), adj[6], f2_mul(W(13), adj[0])); { const unsigned long long s = f2_mul(W(292), adj[2]); g[12] = f2_fma(s, p, g[12]); v = f2_fma(s, x[12], v); } { const unsigned long long s = f2_mul(W(402), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } g[12] = f2_fma(v, x[12], g[12]); g[12] = f2_fma(v, x[12], g[12]); } \
+      { const unsigned long long p = f2_mul(x[12], x[13]); unsigned long long v; v = f2_mul(W(704), adj[7]); { const unsigned long long s = f2_mul(W(293), adj[2]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(403), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[12] = f2_fma(v, x[13], g[12]); g[13] = f2_fma(v, x[12], g[13]); } \
+      { const unsigned long long p = f2_mul(x[12], x[14]); unsigned long long v; v = f2_mul(W(803), adj[8]); { const unsigned long long s = f2_mul(W(294), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(404), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[12] = f2_fma(v, x[14], g[12]); g[14] = f2_fma(v, x[12], g[14]); } \
+      { const unsigned long long p = f2_mul(x[12], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(295), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[12] = f2_fma(v, x[15], g[12]); g[15] = f2_fma(v, x[12], g[15]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); unsigned long long v; v = f2_fma(W(804), adj[8], f2_fma(W(613), adj[6], f2_mul(W(14), adj[0]))); { const unsigned long long s = f2_mul(W(405), adj[3]); g[13] = f2_fma(s, p, g[13]); v = f2_fma(s, x[13], v); } { const unsigned long long s = f2_mul(W(296), adj[2]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(406), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
+      { const unsigned long long p = f2_mul(x[13], x[14]); unsigned long long v; v = f2_mul(W(705), adj[7]); { const unsigned long long s = f2_mul(W(407), adj[3]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } { const unsigned long long s = f2_mul(W(297), adj[2]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[13] = f2_fma(v, x[14], g[13]); g[14] = f2_fma(v, x[13], g[14]); } \
+      { const unsigned long long p = f2_mul(x[13], x[15]); unsigned long long v; v = f2_mul(W(805), adj[8]); { const unsigned long long s = f2_mul(W(408), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[13] = f2_fma(v, x[15], g[13]); g[15] = f2_fma(v, x[13], g[15]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); unsigned long long v; v = f2_mul(W(15), adj[0]); { const unsigned long long s = f2_mul(W(409), adj[3]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(706), adj[7]); g[14] = f2_fma(v, x[15], g[14]); g[15] = f2_fma(v, x[14], g[15]); } \
+      { unsigned long long v; v = f2_fma(W(614), adj[6], f2_mul(W(16), adj[0])); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
+#define SXB_S2_M1_FORWARD_BODY \
+      o[0] = f2_fma(W(0), x[0], o[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); o[0] = f2_fma(p, f2_fma(W(17), x[0], W(1)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); o[0] = f2_fma(p, f2_mul(W(18), x[1]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); o[0] = f2_fma(p, f2_mul(W(19), x[2]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); o[0] = f2_fma(p, f2_mul(W(20), x[3]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); o[0] = f2_fma(p, f2_mul(W(21), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); o[0] = f2_fma(p, f2_mul(W(22), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); o[0] = f2_fma(p, f2_mul(W(23), x[6]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); o[0] = f2_fma(p, f2_mul(W(24), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); o[0] = f2_fma(p, f2_mul(W(25), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); o[0] = f2_fma(p, f2_mul(W(26), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); o[0] = f2_fma(p, f2_mul(W(27), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); o[0] = f2_fma(p, f2_mul(W(28), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); o[0] = f2_fma(p, f2_mul(W(29), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); o[0] = f2_fma(p, f2_mul(W(30), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); o[0] = f2_fma(p, f2_mul(W(31), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); o[0] = f2_fma(p, f2_mul(W(32), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); o[0] = f2_fma(p, f2_fma(W(34), x[8], f2_fma(W(33), x[6], W(2))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); o[0] = f2_fma(p, f2_mul(W(35), x[5]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); o[0] = f2_fma(p, f2_mul(W(36), x[4]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); o[0] = f2_fma(p, f2_fma(W(38), x[15], f2_mul(W(37), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); o[0] = f2_fma(p, f2_fma(W(40), x[14], f2_mul(W(39), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); o[0] = f2_fma(p, f2_mul(W(41), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); o[0] = f2_fma(p, f2_mul(W(42), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); o[0] = f2_fma(p, f2_fma(W(44), x[11], f2_mul(W(43), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); o[0] = f2_fma(p, f2_fma(W(45), x[6], W(3)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); o[0] = f2_fma(p, f2_mul(W(46), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); o[0] = f2_fma(p, f2_mul(W(47), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); o[0] = f2_fma(p, f2_mul(W(48), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); o[0] = f2_fma(p, f2_mul(W(49), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); o[0] = f2_fma(p, f2_mul(W(50), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); o[0] = f2_fma(p, f2_mul(W(51), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); o[0] = f2_fma(p, f2_fma(W(53), x[8], f2_fma(W(52), x[6], W(4))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); o[0] = f2_fma(p, f2_fma(W(55), x[11], f2_mul(W(54), x[9])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); o[0] = f2_fma(p, f2_mul(W(56), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); o[0] = f2_fma(p, f2_mul(W(57), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); o[0] = f2_fma(p, f2_fma(W(59), x[14], f2_mul(W(58), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); o[0] = f2_fma(p, f2_fma(W(61), x[15], f2_mul(W(60), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); o[0] = f2_fma(p, f2_fma(W(62), x[6], W(5)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); o[0] = f2_fma(p, f2_mul(W(63), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); o[0] = f2_fma(p, f2_mul(W(64), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); o[0] = f2_fma(p, f2_mul(W(65), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); o[0] = f2_fma(p, f2_fma(W(67), x[15], f2_mul(W(66), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); o[0] = f2_fma(p, f2_fma(W(69), x[8], f2_fma(W(68), x[6], W(6))), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); o[0] = f2_fma(p, f2_mul(W(70), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); o[0] = f2_fma(p, f2_fma(W(72), x[15], f2_mul(W(71), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); o[0] = f2_fma(p, f2_fma(W(74), x[14], f2_mul(W(73), x[12])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); o[0] = f2_fma(p, f2_fma(W(75), x[6], W(7)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); o[0] = f2_fma(p, f2_mul(W(76), x[7]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); o[0] = f2_fma(p, f2_mul(W(77), x[8]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); o[0] = f2_fma(p, f2_mul(W(78), x[9]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); o[0] = f2_fma(p, f2_mul(W(79), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); o[0] = f2_fma(p, f2_mul(W(80), x[12]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); o[0] = f2_fma(p, f2_mul(W(81), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); o[0] = f2_fma(p, f2_mul(W(82), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); o[0] = f2_fma(p, f2_fma(W(83), x[8], W(8)), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); o[0] = f2_fma(p, f2_mul(W(84), x[10]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); o[0] = f2_fma(p, f2_mul(W(85), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); o[0] = f2_fma(p, f2_mul(W(86), x[13]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); o[0] = f2_fma(p, f2_mul(W(87), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); o[0] = f2_fma(p, f2_mul(W(88), x[15]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[8]); o[0] = f2_fma(p, W(9), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); o[0] = f2_fma(p, f2_mul(W(89), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); o[0] = f2_fma(p, f2_mul(W(90), x[11]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); o[0] = f2_fma(p, f2_mul(W(91), x[14]), o[0]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); o[0] = f2_fma(p, f2_fma(W(93), x[15], f2_mul(W(92), x[13])), o[0]); } \
+      { const unsigned long long p = f2_mul(x[9], x[9]); o[0] = f2_fma(p, W(10), o[0]); } \
+      { const unsigned long long p = f2_mul(x[10], x[10]); o[0] = f2_fma(p, W(11), o[0]); } \
+      { const unsigned long long p = f2_mul(x[11], x[11]); o[0] = f2_fma(p, W(12), o[0]); } \
+      { const unsigned long long p = f2_mul(x[12], x[12]); o[0] = f2_fma(p, W(13), o[0]); } \
+      { const unsigned long long p = f2_mul(x[13], x[13]); o[0] = f2_fma(p, W(14), o[0]); } \
+      { const unsigned long long p = f2_mul(x[14], x[14]); o[0] = f2_fma(p, W(15), o[0]); } \
+      { const unsigned long long p = f2_mul(x[15], x[15]); o[0] = f2_fma(p, W(16), o[0]); }
+#define SXB_S2_M1_REVERSE_BODY \
+      g[0] = f2_fma(W(0), adj[0], g[0]); \
+      { const unsigned long long p = f2_mul(x[0], x[0]); unsigned long long v; v = f2_mul(W(1), adj[0]); { const unsigned long long s = f2_mul(W(17), adj[0]); g[0] = f2_fma(s, p, g[0]); v = f2_fma(s, x[0], v); } g[0] = f2_fma(v, x[0], g[0]); g[0] = f2_fma(v, x[0], g[0]); } \
+      { const unsigned long long p = f2_mul(x[0], x[1]); unsigned long long v; { const unsigned long long s = f2_mul(W(18), adj[0]); g[1] = f2_fma(s, p, g[1]); v = f2_mul(s, x[1]); } g[0] = f2_fma(v, x[1], g[0]); g[1] = f2_fma(v, x[0], g[1]); } \
+      { const unsigned long long p = f2_mul(x[0], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(19), adj[0]); g[2] = f2_fma(s, p, g[2]); v = f2_mul(s, x[2]); } g[0] = f2_fma(v, x[2], g[0]); g[2] = f2_fma(v, x[0], g[2]); } \
+      { const unsigned long long p = f2_mul(x[0], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(20), adj[0]); g[3] = f2_fma(s, p, g[3]); v = f2_mul(s, x[3]); } g[0] = f2_fma(v, x[3], g[0]); g[3] = f2_fma(v, x[0], g[3]); } \
+      { const unsigned long long p = f2_mul(x[0], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(21), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[0] = f2_fma(v, x[4], g[0]); g[4] = f2_fma(v, x[0], g[4]); } \
+      { const unsigned long long p = f2_mul(x[0], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(22), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[0] = f2_fma(v, x[5], g[0]); g[5] = f2_fma(v, x[0], g[5]); } \
+      { const unsigned long long p = f2_mul(x[0], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(23), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_mul(s, x[6]); } g[0] = f2_fma(v, x[6], g[0]); g[6] = f2_fma(v, x[0], g[6]); } \
+      { const unsigned long long p = f2_mul(x[0], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(24), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[0] = f2_fma(v, x[7], g[0]); g[7] = f2_fma(v, x[0], g[7]); } \
+      { const unsigned long long p = f2_mul(x[0], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(25), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[0] = f2_fma(v, x[8], g[0]); g[8] = f2_fma(v, x[0], g[8]); } \
+      { const unsigned long long p = f2_mul(x[0], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(26), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[0] = f2_fma(v, x[9], g[0]); g[9] = f2_fma(v, x[0], g[9]); } \
+      { const unsigned long long p = f2_mul(x[0], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(27), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[0] = f2_fma(v, x[10], g[0]); g[10] = f2_fma(v, x[0], g[10]); } \
+      { const unsigned long long p = f2_mul(x[0], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(28), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[0] = f2_fma(v, x[11], g[0]); g[11] = f2_fma(v, x[0], g[11]); } \
+      { const unsigned long long p = f2_mul(x[0], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(29), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[0] = f2_fma(v, x[12], g[0]); g[12] = f2_fma(v, x[0], g[12]); } \
+      { const unsigned long long p = f2_mul(x[0], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(30), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[0] = f2_fma(v, x[13], g[0]); g[13] = f2_fma(v, x[0], g[13]); } \
+      { const unsigned long long p = f2_mul(x[0], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(31), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[0] = f2_fma(v, x[14], g[0]); g[14] = f2_fma(v, x[0], g[14]); } \
+      { const unsigned long long p = f2_mul(x[0], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(32), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[0] = f2_fma(v, x[15], g[0]); g[15] = f2_fma(v, x[0], g[15]); } \
+      { const unsigned long long p = f2_mul(x[1], x[1]); unsigned long long v; v = f2_mul(W(2), adj[0]); { const unsigned long long s = f2_mul(W(33), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(34), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[1] = f2_fma(v, x[1], g[1]); g[1] = f2_fma(v, x[1], g[1]); } \
+      { const unsigned long long p = f2_mul(x[1], x[2]); unsigned long long v; { const unsigned long long s = f2_mul(W(35), adj[0]); g[5] = f2_fma(s, p, g[5]); v = f2_mul(s, x[5]); } g[1] = f2_fma(v, x[2], g[1]); g[2] = f2_fma(v, x[1], g[2]); } \
+      { const unsigned long long p = f2_mul(x[1], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(36), adj[0]); g[4] = f2_fma(s, p, g[4]); v = f2_mul(s, x[4]); } g[1] = f2_fma(v, x[3], g[1]); g[3] = f2_fma(v, x[1], g[3]); } \
+      { const unsigned long long p = f2_mul(x[1], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(37), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(38), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[1] = f2_fma(v, x[4], g[1]); g[4] = f2_fma(v, x[1], g[4]); } \
+      { const unsigned long long p = f2_mul(x[1], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(39), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(40), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[1] = f2_fma(v, x[5], g[1]); g[5] = f2_fma(v, x[1], g[5]); } \
+      { const unsigned long long p = f2_mul(x[1], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(41), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[1] = f2_fma(v, x[6], g[1]); g[6] = f2_fma(v, x[1], g[6]); } \
+      { const unsigned long long p = f2_mul(x[1], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(42), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[1] = f2_fma(v, x[7], g[1]); g[7] = f2_fma(v, x[1], g[7]); } \
+      { const unsigned long long p = f2_mul(x[1], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(43), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(44), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[1] = f2_fma(v, x[8], g[1]); g[8] = f2_fma(v, x[1], g[8]); } \
+      { const unsigned long long p = f2_mul(x[2], x[2]); unsigned long long v; v = f2_mul(W(3), adj[0]); { const unsigned long long s = f2_mul(W(45), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[2] = f2_fma(v, x[2], g[2]); g[2] = f2_fma(v, x[2], g[2]); } \
+      { const unsigned long long p = f2_mul(x[2], x[3]); unsigned long long v; { const unsigned long long s = f2_mul(W(46), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[2] = f2_fma(v, x[3], g[2]); g[3] = f2_fma(v, x[2], g[3]); } \
+      { const unsigned long long p = f2_mul(x[2], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(47), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[2] = f2_fma(v, x[4], g[2]); g[4] = f2_fma(v, x[2], g[4]); } \
+      { const unsigned long long p = f2_mul(x[2], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(48), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[2] = f2_fma(v, x[5], g[2]); g[5] = f2_fma(v, x[2], g[5]); } \
+      { const unsigned long long p = f2_mul(x[2], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(49), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[2] = f2_fma(v, x[6], g[2]); g[6] = f2_fma(v, x[2], g[6]); } \
+      { const unsigned long long p = f2_mul(x[2], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(50), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[2] = f2_fma(v, x[7], g[2]); g[7] = f2_fma(v, x[2], g[7]); } \
+      { const unsigned long long p = f2_mul(x[2], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(51), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[2] = f2_fma(v, x[8], g[2]); g[8] = f2_fma(v, x[2], g[8]); } \
+      { const unsigned long long p = f2_mul(x[3], x[3]); unsigned long long v; v = f2_mul(W(4), adj[0]); { const unsigned long long s = f2_mul(W(52), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(53), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[3] = f2_fma(v, x[3], g[3]); g[3] = f2_fma(v, x[3], g[3]); } \
+      { const unsigned long long p = f2_mul(x[3], x[4]); unsigned long long v; { const unsigned long long s = f2_mul(W(54), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } { const unsigned long long s = f2_mul(W(55), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_fma(s, x[11], v); } g[3] = f2_fma(v, x[4], g[3]); g[4] = f2_fma(v, x[3], g[4]); } \
+      { const unsigned long long p = f2_mul(x[3], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(56), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[3] = f2_fma(v, x[5], g[3]); g[5] = f2_fma(v, x[3], g[5]); } \
+      { const unsigned long long p = f2_mul(x[3], x[6]); unsigned long long v; { const unsigned long long s = f2_mul(W(57), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[3] = f2_fma(v, x[6], g[3]); g[6] = f2_fma(v, x[3], g[6]); } \
+      { const unsigned long long p = f2_mul(x[3], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(58), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(59), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[3] = f2_fma(v, x[7], g[3]); g[7] = f2_fma(v, x[3], g[7]); } \
+      { const unsigned long long p = f2_mul(x[3], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(60), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(61), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[3] = f2_fma(v, x[8], g[3]); g[8] = f2_fma(v, x[3], g[8]); } \
+      { const unsigned long long p = f2_mul(x[4], x[4]); unsigned long long v; v = f2_mul(W(5), adj[0]); { const unsigned long long s = f2_mul(W(62), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[4] = f2_fma(v, x[4], g[4]); g[4] = f2_fma(v, x[4], g[4]); } \
+      { const unsigned long long p = f2_mul(x[4], x[5]); unsigned long long v; { const unsigned long long s = f2_mul(W(63), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[4] = f2_fma(v, x[5], g[4]); g[5] = f2_fma(v, x[4], g[5]); } \
+      { const unsigned long long p = f2_mul(x[4], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(64), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[4] = f2_fma(v, x[9], g[4]); g[9] = f2_fma(v, x[4], g[9]); } \
+      { const unsigned long long p = f2_mul(x[4], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(65), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[4] = f2_fma(v, x[10], g[4]); g[10] = f2_fma(v, x[4], g[10]); } \
+      { const unsigned long long p = f2_mul(x[4], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(66), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(67), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[4] = f2_fma(v, x[11], g[4]); g[11] = f2_fma(v, x[4], g[11]); } \
+      { const unsigned long long p = f2_mul(x[5], x[5]); unsigned long long v; v = f2_mul(W(6), adj[0]); { const unsigned long long s = f2_mul(W(68), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } { const unsigned long long s = f2_mul(W(69), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[5] = f2_fma(v, x[5], g[5]); g[5] = f2_fma(v, x[5], g[5]); } \
+      { const unsigned long long p = f2_mul(x[5], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(70), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[5] = f2_fma(v, x[9], g[5]); g[9] = f2_fma(v, x[5], g[9]); } \
+      { const unsigned long long p = f2_mul(x[5], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(71), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(72), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[5] = f2_fma(v, x[10], g[5]); g[10] = f2_fma(v, x[5], g[10]); } \
+      { const unsigned long long p = f2_mul(x[5], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(73), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } { const unsigned long long s = f2_mul(W(74), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_fma(s, x[14], v); } g[5] = f2_fma(v, x[11], g[5]); g[11] = f2_fma(v, x[5], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[6]); unsigned long long v; v = f2_mul(W(7), adj[0]); { const unsigned long long s = f2_mul(W(75), adj[0]); g[6] = f2_fma(s, p, g[6]); v = f2_fma(s, x[6], v); } g[6] = f2_fma(v, x[6], g[6]); g[6] = f2_fma(v, x[6], g[6]); } \
+      { const unsigned long long p = f2_mul(x[6], x[7]); unsigned long long v; { const unsigned long long s = f2_mul(W(76), adj[0]); g[7] = f2_fma(s, p, g[7]); v = f2_mul(s, x[7]); } g[6] = f2_fma(v, x[7], g[6]); g[7] = f2_fma(v, x[6], g[7]); } \
+      { const unsigned long long p = f2_mul(x[6], x[8]); unsigned long long v; { const unsigned long long s = f2_mul(W(77), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_mul(s, x[8]); } g[6] = f2_fma(v, x[8], g[6]); g[8] = f2_fma(v, x[6], g[8]); } \
+      { const unsigned long long p = f2_mul(x[6], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(78), adj[0]); g[9] = f2_fma(s, p, g[9]); v = f2_mul(s, x[9]); } g[6] = f2_fma(v, x[9], g[6]); g[9] = f2_fma(v, x[6], g[9]); } \
+      { const unsigned long long p = f2_mul(x[6], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(79), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[6] = f2_fma(v, x[11], g[6]); g[11] = f2_fma(v, x[6], g[11]); } \
+      { const unsigned long long p = f2_mul(x[6], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(80), adj[0]); g[12] = f2_fma(s, p, g[12]); v = f2_mul(s, x[12]); } g[6] = f2_fma(v, x[12], g[6]); g[12] = f2_fma(v, x[6], g[12]); } \
+      { const unsigned long long p = f2_mul(x[6], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(81), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[6] = f2_fma(v, x[13], g[6]); g[13] = f2_fma(v, x[6], g[13]); } \
+      { const unsigned long long p = f2_mul(x[6], x[15]); unsigned long long v; { const unsigned long long s = f2_mul(W(82), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[6] = f2_fma(v, x[15], g[6]); g[15] = f2_fma(v, x[6], g[15]); } \
+      { const unsigned long long p = f2_mul(x[7], x[7]); unsigned long long v; v = f2_mul(W(8), adj[0]); { const unsigned long long s = f2_mul(W(83), adj[0]); g[8] = f2_fma(s, p, g[8]); v = f2_fma(s, x[8], v); } g[7] = f2_fma(v, x[7], g[7]); g[7] = f2_fma(v, x[7], g[7]); } \
+      { const unsigned long long p = f2_mul(x[7], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(84), adj[0]); g[10] = f2_fma(s, p, g[10]); v = f2_mul(s, x[10]); } g[7] = f2_fma(v, x[9], g[7]); g[9] = f2_fma(v, x[7], g[9]); } \
+      { const unsigned long long p = f2_mul(x[7], x[10]); unsigned long long v; { const unsigned long long s = f2_mul(W(85), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[7] = f2_fma(v, x[10], g[7]); g[10] = f2_fma(v, x[7], g[10]); } \
+      { const unsigned long long p = f2_mul(x[7], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(86), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } g[7] = f2_fma(v, x[12], g[7]); g[12] = f2_fma(v, x[7], g[12]); } \
+      { const unsigned long long p = f2_mul(x[7], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(87), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[7] = f2_fma(v, x[13], g[7]); g[13] = f2_fma(v, x[7], g[13]); } \
+      { const unsigned long long p = f2_mul(x[7], x[14]); unsigned long long v; { const unsigned long long s = f2_mul(W(88), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_mul(s, x[15]); } g[7] = f2_fma(v, x[14], g[7]); g[14] = f2_fma(v, x[7], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(9), adj[0]); g[8] = f2_fma(v, x[8], g[8]); g[8] = f2_fma(v, x[8], g[8]); } \
+      { const unsigned long long p = f2_mul(x[8], x[9]); unsigned long long v; { const unsigned long long s = f2_mul(W(89), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[9], g[8]); g[9] = f2_fma(v, x[8], g[9]); } \
+      { const unsigned long long p = f2_mul(x[8], x[11]); unsigned long long v; { const unsigned long long s = f2_mul(W(90), adj[0]); g[11] = f2_fma(s, p, g[11]); v = f2_mul(s, x[11]); } g[8] = f2_fma(v, x[11], g[8]); g[11] = f2_fma(v, x[8], g[11]); } \
+      { const unsigned long long p = f2_mul(x[8], x[12]); unsigned long long v; { const unsigned long long s = f2_mul(W(91), adj[0]); g[14] = f2_fma(s, p, g[14]); v = f2_mul(s, x[14]); } g[8] = f2_fma(v, x[12], g[8]); g[12] = f2_fma(v, x[8], g[12]); } \
+      { const unsigned long long p = f2_mul(x[8], x[13]); unsigned long long v; { const unsigned long long s = f2_mul(W(92), adj[0]); g[13] = f2_fma(s, p, g[13]); v = f2_mul(s, x[13]); } { const unsigned long long s = f2_mul(W(93), adj[0]); g[15] = f2_fma(s, p, g[15]); v = f2_fma(s, x[15], v); } g[8] = f2_fma(v, x[13], g[8]); g[13] = f2_fma(v, x[8], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(10), adj[0]); g[9] = f2_fma(v, x[9], g[9]); g[9] = f2_fma(v, x[9], g[9]); } \
+      { unsigned long long v; v = f2_mul(W(11), adj[0]); g[10] = f2_fma(v, x[10], g[10]); g[10] = f2_fma(v, x[10], g[10]); } \
+      { unsigned long long v; v = f2_mul(W(12), adj[0]); g[11] = f2_fma(v, x[11], g[11]); g[11] = f2_fma(v, x[11], g[11]); } \
+      { unsigned long long v; v = f2_mul(W(13), adj[0]); g[12] = f2_fma(v, x[12], g[12]); g[12] = f2_fma(v, x[12], g[12]); } \
+      { unsigned long long v; v = f2_mul(W(14), adj[0]); g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
+      { unsigned long long v; v = f2_mul(W(15), adj[0]); g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
+      { unsigned long long v; v = f2_mul(W(16), adj[0]); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
 #define SXB_S2_L1_FORWARD_BODY \
     { /* path 0: edge l=0, source l=0 -> l=0 */ \
       const float t0 = R[0] * h[0]; \

@@ -521,3 +521,29 @@ def test_parts_of_a_receiver_add_up(pkg, model_path, arch, copies):
     big = pkg.Calculator(path, skin=0.5).calculate(many, cell * np.array(copies)[:, None], np.tile(types, len(grid)))
     assert np.abs(big["energies"].reshape(len(grid), -1) - out["energies"]).max() <= TOL_E
     assert np.abs(big["forces"].reshape(len(grid), -1, 3) - out["forces"]).max() <= TOL_F
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("arch,counts", [("medium", (1, 1, 1)), ("medium", (3, 17, 15)), ("small", (33, 1, 2)), ("large", (31, 2, 34))])
+def test_contraction_runs_of_elements(pkg, model_path, arch, counts):
+    """The contraction kernels walk runs of equal elements, two nodes per warp: runs of one, odd runs, runs that end inside a
+    block and runs that fill it exactly, for stage tensors against the oracle (bounds of the stage comparison)."""
+    from oracle import mace_numpy, neighbor
+
+    path = model_path(arch, 33)
+    rng = np.random.default_rng(5)
+    n = sum(counts)
+    side = int(np.ceil(n ** (1 / 3)))
+    grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)[:n]
+    pos = 2.4 * grid + rng.uniform(-0.2, 0.2, (n, 3))
+    cell = np.eye(3) * max(2.4 * side, 4.8)
+    types = np.repeat(np.arange(3), counts).astype(np.int32)
+    ev = pkg.MACEB200(path)
+    res = ev._prepare_periodic_factorized_graph(types, pos, cell, np.linalg.inv(cell), ev.r_cut)
+    ev._compute_prepared_factorized_positions(res["generation"], pos)
+    first, src, shifts = neighbor.build_neighbor_graph(pos, cell, ev.r_cut)
+    oracle = mace_numpy.NumpyMACE(str(path))
+    _e, energies, forces, _s = oracle.energy_forces_stress(types, pos, cell, first, src, shifts)
+    assert np.abs(ev.node_energies - energies).max() <= TOL_E
+    got = ev._reduce_atom_forces(n, execution_graph_generation=res["generation"])
+    assert np.abs(got - forces).max() <= TOL_F * max(1.0, np.abs(forces).max())
