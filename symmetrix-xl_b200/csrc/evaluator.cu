@@ -16,6 +16,7 @@
 
 #include "deterministic_kernels.cuh"
 #include "edge_kernels.cuh"
+#include "edge_kernels_shared.cuh"
 #include "edge_kernels_split.cuh"
 #include "edge_kernels_warp.cuh"
 #include "graph_kernels.cuh"
@@ -208,6 +209,13 @@ Evaluator::Evaluator(const std::string& json_path, int device_ordinal, const std
     SXB_ALLOW_POLY_SMEM(m1_forward_kernel_S0, SXB_S0_M1_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_S0, SXB_S0_M1_NUM_TERMS);
     SXB_ALLOW_POLY_SMEM(m1_forward_kernel_S1, SXB_S1_M1_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_S1, SXB_S1_M1_NUM_TERMS);
     SXB_ALLOW_POLY_SMEM(m1_forward_kernel_S2, SXB_S2_M1_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_S2, SXB_S2_M1_NUM_TERMS);
+#define SXB_ALLOW_SHARED_ROWS(NAME, WIDTH)                                                                               \
+    SXB_CUDA(cudaFuncSetAttribute(l1_reverse_shared_kernel_##NAME<WIDTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                  static_cast<int>(shared_rows_bytes(SXB_##NAME##_NUM_ROWS, WIDTH))))
+    SXB_ALLOW_SHARED_ROWS(S1, 128);
+    SXB_ALLOW_SHARED_ROWS(S1, 64);
+    SXB_ALLOW_SHARED_ROWS(S2, 128);
+#undef SXB_ALLOW_SHARED_ROWS
     SXB_CUDA(cudaFuncSetAttribute(tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes));
     SXB_CUDA(cudaFuncSetAttribute(tc_gemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kT3SmemBytes));
     SXB_CUDA(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device_));
@@ -1014,7 +1022,6 @@ void Evaluator::run_pipeline(int phases)
     // 1080: 57 -> 47 us, 2160: 80 -> 86 us.
     const double mean_edges = static_cast<double>(num_edges_) / std::max(1, R), block_warps = std::max(1, C / 32);
     auto l1_forward_parts = [&](int T) { return cluster_parts(T, num_sms_ * std::floor(16.0 / block_warps)); };
-    auto l1_reverse_parts = [&](int T) { return edge_parts(T, num_sms_ * std::floor(12.0 / block_warps), mean_edges, 5.0, 8); };
     auto l0_forward_parts = [&](int T) { return edge_parts(T, num_sms_ * 16.0, mean_edges, 6.0, kWarpsPerBlock) > 1 ? kWarpsPerBlock : 1; };
     auto l0_reverse_parts = [&](int T) { return edge_parts(T, num_sms_ * 12.0, mean_edges, 4.0, 8); };
     auto l0_forward = [&](int t0, int T) {
@@ -1108,8 +1115,6 @@ void Evaluator::run_pipeline(int phases)
         }
     }
     if (phases & 2) {
-        if (model_.shape_id == 2 && fo.edge_forces != nullptr)   // the split gradient kernels accumulate into it
-            SXB_CUDA(cudaMemsetAsync(fo.edge_forces, 0, sizeof(double) * 3 * static_cast<std::size_t>(num_edges_), stream_));
         for (int t0 = 0; t0 < R; t0 += tile_cap) {
             const int T = std::min(tile_cap, R - t0);
             if (model_.single_layer) {
@@ -1258,33 +1263,34 @@ void Evaluator::run_pipeline(int phases)
             }
             span_end();
             span_begin("l1_reverse");
-            const int reverse_parts = l1_reverse_parts(T);
-            if (deterministic_ && model_.shape_id == 0)      // records instead of atomics: the build with the channel count at run time
-                l1_reverse_kernel_S0<0, 3, true><<<dim3(T, reverse_parts), C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+            // hidden l > 0 at the common widths: row adjoints in shared memory; otherwise one channel per thread with the
+            // adjoints in registers (16 rows for hidden 0e), which also leaves the records of the reproducible mode.
+            const bool shared_rows = !deterministic_ && (model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64)));
+            const int reverse_parts = shared_rows ? edge_parts(T, model_.shape_id == 2 ? num_sms_ : num_sms_ * 3 * 128 / C, mean_edges, 8.0, 8)
+                                                  : edge_parts(T, num_sms_ * std::floor(12.0 / block_warps), mean_edges, 5.0, 8);
+            const dim3 reverse_grid(T, reverse_parts);
+#define SXB_SHARED_REVERSE(NAME, WIDTH)                                                                                   \
+            l1_reverse_shared_kernel_##NAME<WIDTH><<<reverse_grid, WIDTH / 2 * kSharedTeams##NAME,                         \
+                                                     shared_rows_bytes(SXB_##NAME##_NUM_ROWS, WIDTH), stream_>>>(          \
+                t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, reinterpret_cast<const float4*>(r1_table_.ptr), \
+                H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_)
+            if (shared_rows) {
+                if (model_.shape_id == 2) SXB_SHARED_REVERSE(S2, 128);
+                else if (C == 128) SXB_SHARED_REVERSE(S1, 128);
+                else SXB_SHARED_REVERSE(S1, 64);
+            } else if (deterministic_ && model_.shape_id == 0)
+                l1_reverse_kernel_S0<0, 3, true><<<reverse_grid, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
-            else if (deterministic_ && model_.shape_id == 1)
-                l1_reverse_kernel_S1<0, 3, true><<<dim3(T, reverse_parts), C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+            else if (deterministic_)
+                l1_reverse_kernel_S1<0, 3, true><<<reverse_grid, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
             else if (model_.shape_id == 0)
-                SXB_LAUNCH_BY_CHANNELS(l1_reverse_kernel_S0, C, dim3(T, reverse_parts), stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                SXB_LAUNCH_BY_CHANNELS(l1_reverse_kernel_S0, C, reverse_grid, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                                        reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
-            else if (model_.shape_id == 1)
-                SXB_LAUNCH_BY_CHANNELS(l1_reverse_kernel_S1, C, dim3(T, reverse_parts), stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
-                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
-            else {
-                // one launch per path set; the sets add into the same edge forces, so those are cleared
-                // first and accumulated atomically
-                ForceOutputs split = fo;
-                split.accumulate_edge = 2;
-#define SXB_SPLIT_REVERSE(SET)                                                                                            \
-                l1_reverse_split_kernel_S2_##SET<128><<<dim3(T, reverse_parts), 128, 0, stream_>>>(T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, \
-                    reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, split, density1, r1_pair_types_)
-                SXB_SPLIT_REVERSE(G0);
-                SXB_SPLIT_REVERSE(G1);
-                SXB_SPLIT_REVERSE(G2);
-#undef SXB_SPLIT_REVERSE
-                launches_ += 2;
-            }
+            else
+                l1_reverse_kernel_S1<0><<<reverse_grid, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                    reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
+#undef SXB_SHARED_REVERSE
             launches_ += 1;
             span_end();
         }

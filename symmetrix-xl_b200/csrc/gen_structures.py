@@ -127,6 +127,70 @@ def contraction_lines(terms):
     return fwd, rev
 
 
+def reverse_edges_lines(paths, row_begin, fed):
+    """Straight-line layer-1 gradient of kEdges edges at once on channel pairs (edge_kernels_shared.cuh).  ADJ(row) reads a
+    row adjoint from shared memory; every value it returns feeds two operations per edge.  EACH(statement) repeats the
+    statement for every edge e.  Names: h[e][lm2], hadj[e][lm2] source features and their adjoint, R[e], dR[e] radial value
+    and slope of the path at hand (RADIAL(p) fetches them), y[e][], ang[e][] the harmonics and the angular adjoint of the
+    edge l at hand, radial[e].  Per path the same contractions as reverse_path_lines; rows that no coupling term feeds (their
+    adjoint is zero: 12 of 88 for hidden 0e+1o, 56 of 243 for 0e+1o+2e) are left out."""
+    out, used = [], set()
+
+    def put(target, a, b):
+        out[-1] += f" EACH({target} = f2_fma({a}, {b}, {target});)" if target in used else f" EACH({target} = f2_mul({a}, {b});)"
+        used.add(target)
+
+    for l1 in sorted({path[1] for path in paths}):
+        n1 = 2 * l1 + 1
+        out.append(f"    {{ f2 y[kEdges][{n1}]{f', ang[kEdges][{n1}]' if l1 else ''}; EACH(load_pair_harmonics<{l1}>(yrow[e], y[e]);)")
+        used -= {f"ang[e][{a}]" for a in range(16)}
+        for p, (l, _, l2) in [(p, path) for p, path in enumerate(paths) if path[1] == l1]:
+            n2 = 2 * l2 + 1
+            out.append(f"    {{ /* path {p}: edge l={l1}, source l={l2} -> l={l} */ RADIAL({p}) f2 yw[kEdges], t[kEdges][{n2}], v[kEdges][{n2}];")
+            used -= {"yw[e]"} | {f"{k}[e][{q}]" for k in "tv" for q in range(16)}
+            if n2 < n1:
+                for b in range(n2):
+                    out.append("     ")
+                    put(f"t[e][{b}]", "R[e]", f"h[e][{l2 * l2 + b}]")
+                for a in range(n1):
+                    for b in range(n2):
+                        if row_begin[p] + a * n2 + b not in fed:
+                            continue
+                        out.append(f"      {{ const f2 w = ADJ({row_begin[p] + a * n2 + b});")
+                        put(f"ang[e][{a}]", f"t[e][{b}]", "w")
+                        put(f"v[e][{b}]", f"y[e][{a}]", "w")
+                        out[-1] += " }"
+                for b in range(n2):
+                    out.append("     ")
+                    put(f"hadj[e][{l2 * l2 + b}]", "R[e]", f"v[e][{b}]")
+                    put("yw[e]", f"h[e][{l2 * l2 + b}]", f"v[e][{b}]")
+            else:
+                for a in range(n1):
+                    row = row_begin[p] + a * n2
+                    if not fed.intersection(range(row, row + n2)):
+                        continue
+                    out.append(f"      EACH(t[e][0] = f2_mul(R[e], y[e][{a}]);)")
+                    used -= {"v[e][0]"}
+                    for b in range(n2):
+                        if row + b not in fed:
+                            continue
+                        out.append(f"      {{ const f2 w = ADJ({row + b});")
+                        put("v[e][0]", f"h[e][{l2 * l2 + b}]", "w")
+                        put(f"hadj[e][{l2 * l2 + b}]", "t[e][0]", "w")
+                        out[-1] += " }"
+                    out.append("     ")
+                    if l1:
+                        put(f"ang[e][{a}]", "R[e]", "v[e][0]")
+                    put("yw[e]", f"y[e][{a}]", "v[e][0]")
+            out.append("     ")
+            put("radial[e]", "dR[e]", "yw[e]")
+            out.append("    }")
+        if l1:
+            out.append(f"      EACH(add_angular_force<{l1}>(grow[e], ang[e], fx[e], fy[e], fz[e]);)")
+        out.append("    }")
+    return out
+
+
 def emit_shape(name, l_max, L_max, tables, groups=1, by_edge_l=None):
     out = []
     paths = list(zip(tables["Phi1_l"], tables["Phi1_l1"], tables["Phi1_l2"]))
@@ -217,6 +281,9 @@ def emit_shape(name, l_max, L_max, tables, groups=1, by_edge_l=None):
     out.append(" \\\n".join(fwd))
     out.append(f"#define SXB_{name}_L1_REVERSE_BODY \\")
     out.append(" \\\n".join(rev))
+    if L_max > 0:
+        out.append(f"#define SXB_{name}_L1_REVERSE_EDGES_BODY \\")
+        out.append(" \\\n".join(reverse_edges_lines(paths, row_begin, set(tables["Phi1_lelm1lm2"]))))
     if groups > 1:
         out.extend(emit_path_groups(name, paths, row_begin, tables, groups, by_edge_l))
     out.append("")
@@ -257,13 +324,11 @@ def emit_path_groups(name, paths, row_begin, tables, groups, by_edge_l=None):
                 rows_g += 1
         lmes = sorted(lme for lme, p in lme_path.items() if p in plist)
         local_lme = {lme: i for i, lme in enumerate(lmes)}
-        hmask, emask = 0, 0
+        hmask = 0
         for p in plist:
-            l1, l2 = paths[p][1], paths[p][2]
+            l2 = paths[p][2]
             for b in range(l2 * l2, (l2 + 1) ** 2):
                 hmask |= 1 << b
-            for a in range(l1 * l1, (l1 + 1) ** 2):
-                emask |= 1 << a
         pre = f"SXB_{name}_G{g}"
         out.append(f"#define {pre}_NUM_PATHS {len(plist)}")
         out.append(f"#define {pre}_NUM_ROWS {rows_g}")
@@ -271,13 +336,11 @@ def emit_path_groups(name, paths, row_begin, tables, groups, by_edge_l=None):
         out.append(f"#define {pre}_PATH_LIST {{{', '.join(map(str, plist))}}}")
         out.append(f"#define {pre}_LME_LIST {{{', '.join(map(str, lmes))}}}")
         out.append(f"#define {pre}_SOURCE_MASK {hmask}u   // source components lm2 the set touches")
-        out.append(f"#define {pre}_EDGE_MASK {emask}u   // edge harmonics lm1 the set touches")
-        out.append(f"#define {pre}_HAS_PATH0 {1 if 0 in plist else 0}")
         out.append(f"// X(term, row inside the set, output inside the set)")
         out.append(f"#define {pre}_TERMS(X) \\")
         out.append(" \\\n".join(f"    X({t}, {local_row[row]}, {local_lme[lme]})" for t, (row, lme) in
                                 enumerate(zip(tables["Phi1_lelm1lm2"], tables["Phi1_lme"])) if row in local_row))
-        fwd, rev = [], []
+        fwd = []
         for q, p in enumerate(plist):
             l, l1, l2 = paths[p]
             n1, n2 = 2 * l1 + 1, 2 * l2 + 1
@@ -290,11 +353,8 @@ def emit_path_groups(name, paths, row_begin, tables, groups, by_edge_l=None):
                     row = base + a * n2 + b
                     fwd.append(f"      acc[{row}] = fmaf(t{b}, y[{l1 * l1 + a}], acc[{row}]);")
             fwd.append("    }")
-            rev.extend(reverse_path_lines(p, q, l, l1, l2, base))
         out.append(f"#define {pre}_FORWARD_BODY \\")
         out.append(" \\\n".join(fwd))
-        out.append(f"#define {pre}_REVERSE_BODY \\")
-        out.append(" \\\n".join(rev))
     return out
 
 

@@ -2069,6 +2069,164 @@
         hadj[3] = fmaf(R[9], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
       radial = fmaf(dR[9], yw, radial); \
     }
+#define SXB_S1_L1_REVERSE_EDGES_BODY \
+    { f2 y[kEdges][1]; EACH(load_pair_harmonics<0>(yrow[e], y[e]);) \
+    { /* path 0: edge l=0, source l=0 -> l=0 */ RADIAL(0) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(0); EACH(v[e][0] = f2_mul(h[e][0], w);) EACH(hadj[e][0] = f2_mul(t[e][0], w);) } \
+      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_mul(dR[e], yw[e]);) \
+    } \
+    { /* path 3: edge l=0, source l=1 -> l=1 */ RADIAL(3) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(13); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(14); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(15); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_mul(t[e][0], w);) } \
+      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    } \
+    { f2 y[kEdges][3], ang[kEdges][3]; EACH(load_pair_harmonics<1>(yrow[e], y[e]);) \
+    { /* path 1: edge l=1, source l=1 -> l=0 */ RADIAL(1) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(1); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      EACH(ang[e][0] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(5); EACH(v[e][0] = f2_mul(h[e][2], w);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      EACH(ang[e][1] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(9); EACH(v[e][0] = f2_mul(h[e][3], w);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][2] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 2: edge l=1, source l=0 -> l=1 */ RADIAL(2) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
+      { const f2 w = ADJ(10); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(11); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(12); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 6: edge l=1, source l=1 -> l=2 */ RADIAL(6) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(36); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      { const f2 w = ADJ(37); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      { const f2 w = ADJ(38); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(39); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      { const f2 w = ADJ(40); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      { const f2 w = ADJ(41); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(42); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      { const f2 w = ADJ(43); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      { const f2 w = ADJ(44); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+      EACH(add_angular_force<1>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+    } \
+    { f2 y[kEdges][5], ang[kEdges][5]; EACH(load_pair_harmonics<2>(yrow[e], y[e]);) \
+    { /* path 4: edge l=2, source l=1 -> l=1 */ RADIAL(4) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
+      { const f2 w = ADJ(16); EACH(ang[e][0] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(18); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(19); EACH(ang[e][1] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(20); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
+      { const f2 w = ADJ(22); EACH(ang[e][2] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(23); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(24); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
+      { const f2 w = ADJ(26); EACH(ang[e][3] = f2_mul(t[e][1], w);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(27); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(28); EACH(ang[e][4] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(30); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
+      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
+      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 5: edge l=2, source l=0 -> l=2 */ RADIAL(5) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
+      { const f2 w = ADJ(31); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(32); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(33); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(34); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(35); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 9: edge l=2, source l=1 -> l=3 */ RADIAL(9) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
+      { const f2 w = ADJ(73); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(74); EACH(ang[e][0] = f2_fma(t[e][1], w, ang[e][0]);) EACH(v[e][1] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(75); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(76); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(77); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_fma(y[e][1], w, v[e][1]);) } \
+      { const f2 w = ADJ(78); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
+      { const f2 w = ADJ(79); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(80); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(81); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
+      { const f2 w = ADJ(82); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(83); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(84); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(85); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(86); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
+      { const f2 w = ADJ(87); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
+      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
+      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+      EACH(add_angular_force<2>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+    } \
+    { f2 y[kEdges][7], ang[kEdges][7]; EACH(load_pair_harmonics<3>(yrow[e], y[e]);) \
+    { /* path 7: edge l=3, source l=1 -> l=2 */ RADIAL(7) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
+      { const f2 w = ADJ(45); EACH(ang[e][0] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(47); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(48); EACH(ang[e][1] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(49); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
+      { const f2 w = ADJ(50); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
+      { const f2 w = ADJ(51); EACH(ang[e][2] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(52); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(53); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
+      { const f2 w = ADJ(54); EACH(ang[e][3] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(55); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(56); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(57); EACH(ang[e][4] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(58); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
+      { const f2 w = ADJ(59); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      { const f2 w = ADJ(60); EACH(ang[e][5] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
+      { const f2 w = ADJ(61); EACH(ang[e][5] = f2_fma(t[e][1], w, ang[e][5]);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
+      { const f2 w = ADJ(62); EACH(ang[e][5] = f2_fma(t[e][2], w, ang[e][5]);) EACH(v[e][2] = f2_fma(y[e][5], w, v[e][2]);) } \
+      { const f2 w = ADJ(63); EACH(ang[e][6] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
+      { const f2 w = ADJ(65); EACH(ang[e][6] = f2_fma(t[e][2], w, ang[e][6]);) EACH(v[e][2] = f2_fma(y[e][6], w, v[e][2]);) } \
+      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
+      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
+      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 8: edge l=3, source l=0 -> l=3 */ RADIAL(8) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
+      { const f2 w = ADJ(66); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(67); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(68); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(69); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(70); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(71); EACH(ang[e][5] = f2_fma(t[e][0], w, ang[e][5]);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
+      { const f2 w = ADJ(72); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
+      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+      EACH(add_angular_force<3>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+    }
 
 // ---- shape S2: edge l_max=3, hidden L_max=2
 #define SXB_S2_LMAX 3
@@ -4775,6 +4933,350 @@
         hadj[8] = fmaf(R[16], s_, hadj[8]); yw = fmaf(h[8], s_, yw); } \
       radial = fmaf(dR[16], yw, radial); \
     }
+#define SXB_S2_L1_REVERSE_EDGES_BODY \
+    { f2 y[kEdges][1]; EACH(load_pair_harmonics<0>(yrow[e], y[e]);) \
+    { /* path 0: edge l=0, source l=0 -> l=0 */ RADIAL(0) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(0); EACH(v[e][0] = f2_mul(h[e][0], w);) EACH(hadj[e][0] = f2_mul(t[e][0], w);) } \
+      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_mul(dR[e], yw[e]);) \
+    } \
+    { /* path 4: edge l=0, source l=1 -> l=1 */ RADIAL(4) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(38); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(39); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(40); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_mul(t[e][0], w);) } \
+      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 11: edge l=0, source l=2 -> l=2 */ RADIAL(11) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(141); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(142); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(143); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(144); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_mul(t[e][0], w);) } \
+      { const f2 w = ADJ(145); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_mul(t[e][0], w);) } \
+      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    } \
+    { f2 y[kEdges][3], ang[kEdges][3]; EACH(load_pair_harmonics<1>(yrow[e], y[e]);) \
+    { /* path 1: edge l=1, source l=1 -> l=0 */ RADIAL(1) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(1); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      EACH(ang[e][0] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(5); EACH(v[e][0] = f2_mul(h[e][2], w);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      EACH(ang[e][1] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(9); EACH(v[e][0] = f2_mul(h[e][3], w);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][2] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 3: edge l=1, source l=0 -> l=1 */ RADIAL(3) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
+      { const f2 w = ADJ(35); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(36); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(37); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 6: edge l=1, source l=2 -> l=1 */ RADIAL(6) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(56); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(57); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(58); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(60); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(62); EACH(v[e][0] = f2_mul(h[e][5], w);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(63); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(64); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(66); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(68); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(69); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(70); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 9: edge l=1, source l=1 -> l=2 */ RADIAL(9) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(111); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      { const f2 w = ADJ(112); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      { const f2 w = ADJ(113); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(114); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      { const f2 w = ADJ(115); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      { const f2 w = ADJ(116); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(117); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
+      { const f2 w = ADJ(118); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
+      { const f2 w = ADJ(119); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
+      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 15: edge l=1, source l=2 -> l=3 */ RADIAL(15) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(193); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(194); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(195); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(196); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(197); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(198); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(199); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(200); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(201); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(202); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(203); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(204); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(205); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(206); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(207); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+      EACH(add_angular_force<1>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+    } \
+    { f2 y[kEdges][5], ang[kEdges][5]; EACH(load_pair_harmonics<2>(yrow[e], y[e]);) \
+    { /* path 2: edge l=2, source l=2 -> l=0 */ RADIAL(2) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(10); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      EACH(ang[e][0] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(16); EACH(v[e][0] = f2_mul(h[e][5], w);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      EACH(ang[e][1] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(22); EACH(v[e][0] = f2_mul(h[e][6], w);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      EACH(ang[e][2] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][3]);) \
+      { const f2 w = ADJ(28); EACH(v[e][0] = f2_mul(h[e][7], w);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      EACH(ang[e][3] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][3], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][4]);) \
+      { const f2 w = ADJ(34); EACH(v[e][0] = f2_mul(h[e][8], w);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][4] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][4], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 5: edge l=2, source l=1 -> l=1 */ RADIAL(5) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
+      { const f2 w = ADJ(41); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(43); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(44); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(45); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
+      { const f2 w = ADJ(47); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(48); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(49); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
+      { const f2 w = ADJ(51); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(52); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(53); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(55); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
+      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
+      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 8: edge l=2, source l=0 -> l=2 */ RADIAL(8) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
+      { const f2 w = ADJ(106); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(107); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(108); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(109); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(110); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 12: edge l=2, source l=2 -> l=2 */ RADIAL(12) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
+      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
+      { const f2 w = ADJ(146); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(147); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(148); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(149); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
+      { const f2 w = ADJ(151); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(152); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(153); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(154); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(155); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
+      { const f2 w = ADJ(156); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(157); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(158); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(159); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(160); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][3]);) \
+      { const f2 w = ADJ(161); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
+      { const f2 w = ADJ(162); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(163); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(164); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(165); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][3] = f2_fma(R[e], v[e][0], ang[e][3]);) EACH(yw[e] = f2_fma(y[e][3], v[e][0], yw[e]);) \
+      EACH(t[e][0] = f2_mul(R[e], y[e][4]);) \
+      { const f2 w = ADJ(167); EACH(v[e][0] = f2_mul(h[e][5], w);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
+      { const f2 w = ADJ(168); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
+      { const f2 w = ADJ(169); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
+      { const f2 w = ADJ(170); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
+      EACH(ang[e][4] = f2_fma(R[e], v[e][0], ang[e][4]);) EACH(yw[e] = f2_fma(y[e][4], v[e][0], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 14: edge l=2, source l=1 -> l=3 */ RADIAL(14) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
+      { const f2 w = ADJ(178); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(179); EACH(ang[e][0] = f2_fma(t[e][1], w, ang[e][0]);) EACH(v[e][1] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(180); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(181); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(182); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_fma(y[e][1], w, v[e][1]);) } \
+      { const f2 w = ADJ(183); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
+      { const f2 w = ADJ(184); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(185); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(186); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
+      { const f2 w = ADJ(187); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(188); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(189); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(190); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(191); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
+      { const f2 w = ADJ(192); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
+      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
+      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+      EACH(add_angular_force<2>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+    } \
+    { f2 y[kEdges][7], ang[kEdges][7]; EACH(load_pair_harmonics<3>(yrow[e], y[e]);) \
+    { /* path 7: edge l=3, source l=2 -> l=1 */ RADIAL(7) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][4]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][5]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][6]);) \
+      EACH(t[e][3] = f2_mul(R[e], h[e][7]);) \
+      EACH(t[e][4] = f2_mul(R[e], h[e][8]);) \
+      { const f2 w = ADJ(71); EACH(ang[e][0] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(75); EACH(ang[e][0] = f2_fma(t[e][4], w, ang[e][0]);) EACH(v[e][4] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(76); EACH(ang[e][1] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(77); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
+      { const f2 w = ADJ(79); EACH(ang[e][1] = f2_fma(t[e][3], w, ang[e][1]);) EACH(v[e][3] = f2_mul(y[e][1], w);) } \
+      { const f2 w = ADJ(81); EACH(ang[e][2] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(82); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(83); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_mul(y[e][2], w);) } \
+      { const f2 w = ADJ(85); EACH(ang[e][2] = f2_fma(t[e][4], w, ang[e][2]);) EACH(v[e][4] = f2_fma(y[e][2], w, v[e][4]);) } \
+      { const f2 w = ADJ(87); EACH(ang[e][3] = f2_mul(t[e][1], w);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(88); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(89); EACH(ang[e][3] = f2_fma(t[e][3], w, ang[e][3]);) EACH(v[e][3] = f2_fma(y[e][3], w, v[e][3]);) } \
+      { const f2 w = ADJ(91); EACH(ang[e][4] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(93); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      { const f2 w = ADJ(94); EACH(ang[e][4] = f2_fma(t[e][3], w, ang[e][4]);) EACH(v[e][3] = f2_fma(y[e][4], w, v[e][3]);) } \
+      { const f2 w = ADJ(95); EACH(ang[e][4] = f2_fma(t[e][4], w, ang[e][4]);) EACH(v[e][4] = f2_fma(y[e][4], w, v[e][4]);) } \
+      { const f2 w = ADJ(97); EACH(ang[e][5] = f2_mul(t[e][1], w);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
+      { const f2 w = ADJ(99); EACH(ang[e][5] = f2_fma(t[e][3], w, ang[e][5]);) EACH(v[e][3] = f2_fma(y[e][5], w, v[e][3]);) } \
+      { const f2 w = ADJ(100); EACH(ang[e][5] = f2_fma(t[e][4], w, ang[e][5]);) EACH(v[e][4] = f2_fma(y[e][5], w, v[e][4]);) } \
+      { const f2 w = ADJ(101); EACH(ang[e][6] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
+      { const f2 w = ADJ(105); EACH(ang[e][6] = f2_fma(t[e][4], w, ang[e][6]);) EACH(v[e][4] = f2_fma(y[e][6], w, v[e][4]);) } \
+      EACH(hadj[e][4] = f2_fma(R[e], v[e][0], hadj[e][4]);) EACH(yw[e] = f2_mul(h[e][4], v[e][0]);) \
+      EACH(hadj[e][5] = f2_fma(R[e], v[e][1], hadj[e][5]);) EACH(yw[e] = f2_fma(h[e][5], v[e][1], yw[e]);) \
+      EACH(hadj[e][6] = f2_fma(R[e], v[e][2], hadj[e][6]);) EACH(yw[e] = f2_fma(h[e][6], v[e][2], yw[e]);) \
+      EACH(hadj[e][7] = f2_fma(R[e], v[e][3], hadj[e][7]);) EACH(yw[e] = f2_fma(h[e][7], v[e][3], yw[e]);) \
+      EACH(hadj[e][8] = f2_fma(R[e], v[e][4], hadj[e][8]);) EACH(yw[e] = f2_fma(h[e][8], v[e][4], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 10: edge l=3, source l=1 -> l=2 */ RADIAL(10) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
+      { const f2 w = ADJ(120); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(122); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(123); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(124); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
+      { const f2 w = ADJ(125); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
+      { const f2 w = ADJ(126); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(127); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(128); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
+      { const f2 w = ADJ(129); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(130); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(131); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(132); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(133); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
+      { const f2 w = ADJ(134); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      { const f2 w = ADJ(135); EACH(ang[e][5] = f2_fma(t[e][0], w, ang[e][5]);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
+      { const f2 w = ADJ(136); EACH(ang[e][5] = f2_fma(t[e][1], w, ang[e][5]);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
+      { const f2 w = ADJ(137); EACH(ang[e][5] = f2_fma(t[e][2], w, ang[e][5]);) EACH(v[e][2] = f2_fma(y[e][5], w, v[e][2]);) } \
+      { const f2 w = ADJ(138); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
+      { const f2 w = ADJ(140); EACH(ang[e][6] = f2_fma(t[e][2], w, ang[e][6]);) EACH(v[e][2] = f2_fma(y[e][6], w, v[e][2]);) } \
+      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
+      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
+      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 13: edge l=3, source l=0 -> l=3 */ RADIAL(13) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
+      { const f2 w = ADJ(171); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(172); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(173); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(174); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(175); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(176); EACH(ang[e][5] = f2_fma(t[e][0], w, ang[e][5]);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
+      { const f2 w = ADJ(177); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
+      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+    { /* path 16: edge l=3, source l=2 -> l=3 */ RADIAL(16) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
+      EACH(t[e][0] = f2_mul(R[e], h[e][4]);) \
+      EACH(t[e][1] = f2_mul(R[e], h[e][5]);) \
+      EACH(t[e][2] = f2_mul(R[e], h[e][6]);) \
+      EACH(t[e][3] = f2_mul(R[e], h[e][7]);) \
+      EACH(t[e][4] = f2_mul(R[e], h[e][8]);) \
+      { const f2 w = ADJ(208); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(209); EACH(ang[e][0] = f2_fma(t[e][1], w, ang[e][0]);) EACH(v[e][1] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(210); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(211); EACH(ang[e][0] = f2_fma(t[e][3], w, ang[e][0]);) EACH(v[e][3] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(212); EACH(ang[e][0] = f2_fma(t[e][4], w, ang[e][0]);) EACH(v[e][4] = f2_mul(y[e][0], w);) } \
+      { const f2 w = ADJ(213); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
+      { const f2 w = ADJ(214); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_fma(y[e][1], w, v[e][1]);) } \
+      { const f2 w = ADJ(216); EACH(ang[e][1] = f2_fma(t[e][3], w, ang[e][1]);) EACH(v[e][3] = f2_fma(y[e][1], w, v[e][3]);) } \
+      { const f2 w = ADJ(218); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
+      { const f2 w = ADJ(219); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
+      { const f2 w = ADJ(220); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
+      { const f2 w = ADJ(221); EACH(ang[e][2] = f2_fma(t[e][3], w, ang[e][2]);) EACH(v[e][3] = f2_fma(y[e][2], w, v[e][3]);) } \
+      { const f2 w = ADJ(222); EACH(ang[e][2] = f2_fma(t[e][4], w, ang[e][2]);) EACH(v[e][4] = f2_fma(y[e][2], w, v[e][4]);) } \
+      { const f2 w = ADJ(223); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
+      { const f2 w = ADJ(224); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
+      { const f2 w = ADJ(225); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
+      { const f2 w = ADJ(226); EACH(ang[e][3] = f2_fma(t[e][3], w, ang[e][3]);) EACH(v[e][3] = f2_fma(y[e][3], w, v[e][3]);) } \
+      { const f2 w = ADJ(227); EACH(ang[e][3] = f2_fma(t[e][4], w, ang[e][3]);) EACH(v[e][4] = f2_fma(y[e][3], w, v[e][4]);) } \
+      { const f2 w = ADJ(228); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
+      { const f2 w = ADJ(229); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
+      { const f2 w = ADJ(230); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
+      { const f2 w = ADJ(231); EACH(ang[e][4] = f2_fma(t[e][3], w, ang[e][4]);) EACH(v[e][3] = f2_fma(y[e][4], w, v[e][3]);) } \
+      { const f2 w = ADJ(232); EACH(ang[e][4] = f2_fma(t[e][4], w, ang[e][4]);) EACH(v[e][4] = f2_fma(y[e][4], w, v[e][4]);) } \
+      { const f2 w = ADJ(234); EACH(ang[e][5] = f2_fma(t[e][1], w, ang[e][5]);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
+      { const f2 w = ADJ(236); EACH(ang[e][5] = f2_fma(t[e][3], w, ang[e][5]);) EACH(v[e][3] = f2_fma(y[e][5], w, v[e][3]);) } \
+      { const f2 w = ADJ(237); EACH(ang[e][5] = f2_fma(t[e][4], w, ang[e][5]);) EACH(v[e][4] = f2_fma(y[e][5], w, v[e][4]);) } \
+      { const f2 w = ADJ(238); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
+      { const f2 w = ADJ(239); EACH(ang[e][6] = f2_fma(t[e][1], w, ang[e][6]);) EACH(v[e][1] = f2_fma(y[e][6], w, v[e][1]);) } \
+      { const f2 w = ADJ(240); EACH(ang[e][6] = f2_fma(t[e][2], w, ang[e][6]);) EACH(v[e][2] = f2_fma(y[e][6], w, v[e][2]);) } \
+      { const f2 w = ADJ(241); EACH(ang[e][6] = f2_fma(t[e][3], w, ang[e][6]);) EACH(v[e][3] = f2_fma(y[e][6], w, v[e][3]);) } \
+      { const f2 w = ADJ(242); EACH(ang[e][6] = f2_fma(t[e][4], w, ang[e][6]);) EACH(v[e][4] = f2_fma(y[e][6], w, v[e][4]);) } \
+      EACH(hadj[e][4] = f2_fma(R[e], v[e][0], hadj[e][4]);) EACH(yw[e] = f2_mul(h[e][4], v[e][0]);) \
+      EACH(hadj[e][5] = f2_fma(R[e], v[e][1], hadj[e][5]);) EACH(yw[e] = f2_fma(h[e][5], v[e][1], yw[e]);) \
+      EACH(hadj[e][6] = f2_fma(R[e], v[e][2], hadj[e][6]);) EACH(yw[e] = f2_fma(h[e][6], v[e][2], yw[e]);) \
+      EACH(hadj[e][7] = f2_fma(R[e], v[e][3], hadj[e][7]);) EACH(yw[e] = f2_fma(h[e][7], v[e][3], yw[e]);) \
+      EACH(hadj[e][8] = f2_fma(R[e], v[e][4], hadj[e][8]);) EACH(yw[e] = f2_fma(h[e][8], v[e][4], yw[e]);) \
+      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    } \
+      EACH(add_angular_force<3>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+    }
 #define SXB_S2_NUM_GROUPS 3
 #define SXB_S2_G0_NUM_PATHS 10
 #define SXB_S2_G0_NUM_ROWS 88
@@ -4782,8 +5284,6 @@
 #define SXB_S2_G0_PATH_LIST {0, 1, 3, 4, 5, 8, 9, 10, 13, 14}
 #define SXB_S2_G0_LME_LIST {0, 1, 3, 4, 5, 8, 9, 10, 13, 14, 15, 18, 19, 20, 23, 24, 25, 28, 29, 30, 33, 34, 35, 38, 39, 40, 43, 44, 47, 48, 51, 52, 55, 56, 59, 60, 63, 64, 67, 68}
 #define SXB_S2_G0_SOURCE_MASK 15u   // source components lm2 the set touches
-#define SXB_S2_G0_EDGE_MASK 65535u   // edge harmonics lm1 the set touches
-#define SXB_S2_G0_HAS_PATH0 1
 // X(term, row inside the set, output inside the set)
 #define SXB_S2_G0_TERMS(X) \
     X(0, 0, 0) \
@@ -5003,203 +5503,12 @@
       acc[86] = fmaf(t1, y[8], acc[86]); \
       acc[87] = fmaf(t2, y[8], acc[87]); \
     }
-#define SXB_S2_G0_REVERSE_BODY \
-    { /* path 0: edge l=0, source l=0 -> l=0 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[0] * y[0]; \
-      { const float w = h[0] * adj[0]; \
-        ang[0] = fmaf(R[0], w, ang[0]); yw = fmaf(y[0], w, yw); } \
-      hadj[0] = fmaf(ry0, adj[0], hadj[0]); \
-      radial = fmaf(dR[0], yw, radial); \
-    } \
-    { /* path 1: edge l=1, source l=1 -> l=0 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[1] * y[1]; \
-      const float ry1 = R[1] * y[2]; \
-      const float ry2 = R[1] * y[3]; \
-      { const float w = fmaf(h[3], adj[3], fmaf(h[2], adj[2], h[1] * adj[1])); \
-        ang[1] = fmaf(R[1], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[3], adj[6], fmaf(h[2], adj[5], h[1] * adj[4])); \
-        ang[2] = fmaf(R[1], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[3], adj[9], fmaf(h[2], adj[8], h[1] * adj[7])); \
-        ang[3] = fmaf(R[1], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[1] = fmaf(ry0, adj[1], hadj[1]); \
-      hadj[1] = fmaf(ry1, adj[4], hadj[1]); \
-      hadj[1] = fmaf(ry2, adj[7], hadj[1]); \
-      hadj[2] = fmaf(ry0, adj[2], hadj[2]); \
-      hadj[2] = fmaf(ry1, adj[5], hadj[2]); \
-      hadj[2] = fmaf(ry2, adj[8], hadj[2]); \
-      hadj[3] = fmaf(ry0, adj[3], hadj[3]); \
-      hadj[3] = fmaf(ry1, adj[6], hadj[3]); \
-      hadj[3] = fmaf(ry2, adj[9], hadj[3]); \
-      radial = fmaf(dR[1], yw, radial); \
-    } \
-    { /* path 3: edge l=1, source l=0 -> l=1 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[2] * h[0]; \
-      ang[1] = fmaf(rh0, adj[10], ang[1]); \
-      ang[2] = fmaf(rh0, adj[11], ang[2]); \
-      ang[3] = fmaf(rh0, adj[12], ang[3]); \
-      { const float s_ = fmaf(y[3], adj[12], fmaf(y[2], adj[11], y[1] * adj[10])); \
-        hadj[0] = fmaf(R[2], s_, hadj[0]); yw = fmaf(h[0], s_, yw); } \
-      radial = fmaf(dR[2], yw, radial); \
-    } \
-    { /* path 4: edge l=0, source l=1 -> l=1 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[3] * y[0]; \
-      { const float w = fmaf(h[3], adj[15], fmaf(h[2], adj[14], h[1] * adj[13])); \
-        ang[0] = fmaf(R[3], w, ang[0]); yw = fmaf(y[0], w, yw); } \
-      hadj[1] = fmaf(ry0, adj[13], hadj[1]); \
-      hadj[2] = fmaf(ry0, adj[14], hadj[2]); \
-      hadj[3] = fmaf(ry0, adj[15], hadj[3]); \
-      radial = fmaf(dR[3], yw, radial); \
-    } \
-    { /* path 5: edge l=2, source l=1 -> l=1 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[4] * h[1]; \
-      const float rh1 = R[4] * h[2]; \
-      const float rh2 = R[4] * h[3]; \
-      ang[4] = fmaf(rh0, adj[16], ang[4]); \
-      ang[4] = fmaf(rh1, adj[17], ang[4]); \
-      ang[4] = fmaf(rh2, adj[18], ang[4]); \
-      ang[5] = fmaf(rh0, adj[19], ang[5]); \
-      ang[5] = fmaf(rh1, adj[20], ang[5]); \
-      ang[5] = fmaf(rh2, adj[21], ang[5]); \
-      ang[6] = fmaf(rh0, adj[22], ang[6]); \
-      ang[6] = fmaf(rh1, adj[23], ang[6]); \
-      ang[6] = fmaf(rh2, adj[24], ang[6]); \
-      ang[7] = fmaf(rh0, adj[25], ang[7]); \
-      ang[7] = fmaf(rh1, adj[26], ang[7]); \
-      ang[7] = fmaf(rh2, adj[27], ang[7]); \
-      ang[8] = fmaf(rh0, adj[28], ang[8]); \
-      ang[8] = fmaf(rh1, adj[29], ang[8]); \
-      ang[8] = fmaf(rh2, adj[30], ang[8]); \
-      { const float s_ = fmaf(y[8], adj[28], fmaf(y[7], adj[25], fmaf(y[6], adj[22], fmaf(y[5], adj[19], y[4] * adj[16])))); \
-        hadj[1] = fmaf(R[4], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[29], fmaf(y[7], adj[26], fmaf(y[6], adj[23], fmaf(y[5], adj[20], y[4] * adj[17])))); \
-        hadj[2] = fmaf(R[4], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[30], fmaf(y[7], adj[27], fmaf(y[6], adj[24], fmaf(y[5], adj[21], y[4] * adj[18])))); \
-        hadj[3] = fmaf(R[4], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
-      radial = fmaf(dR[4], yw, radial); \
-    } \
-    { /* path 8: edge l=2, source l=0 -> l=2 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[5] * h[0]; \
-      ang[4] = fmaf(rh0, adj[31], ang[4]); \
-      ang[5] = fmaf(rh0, adj[32], ang[5]); \
-      ang[6] = fmaf(rh0, adj[33], ang[6]); \
-      ang[7] = fmaf(rh0, adj[34], ang[7]); \
-      ang[8] = fmaf(rh0, adj[35], ang[8]); \
-      { const float s_ = fmaf(y[8], adj[35], fmaf(y[7], adj[34], fmaf(y[6], adj[33], fmaf(y[5], adj[32], y[4] * adj[31])))); \
-        hadj[0] = fmaf(R[5], s_, hadj[0]); yw = fmaf(h[0], s_, yw); } \
-      radial = fmaf(dR[5], yw, radial); \
-    } \
-    { /* path 9: edge l=1, source l=1 -> l=2 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[6] * y[1]; \
-      const float ry1 = R[6] * y[2]; \
-      const float ry2 = R[6] * y[3]; \
-      { const float w = fmaf(h[3], adj[38], fmaf(h[2], adj[37], h[1] * adj[36])); \
-        ang[1] = fmaf(R[6], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[3], adj[41], fmaf(h[2], adj[40], h[1] * adj[39])); \
-        ang[2] = fmaf(R[6], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[3], adj[44], fmaf(h[2], adj[43], h[1] * adj[42])); \
-        ang[3] = fmaf(R[6], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[1] = fmaf(ry0, adj[36], hadj[1]); \
-      hadj[1] = fmaf(ry1, adj[39], hadj[1]); \
-      hadj[1] = fmaf(ry2, adj[42], hadj[1]); \
-      hadj[2] = fmaf(ry0, adj[37], hadj[2]); \
-      hadj[2] = fmaf(ry1, adj[40], hadj[2]); \
-      hadj[2] = fmaf(ry2, adj[43], hadj[2]); \
-      hadj[3] = fmaf(ry0, adj[38], hadj[3]); \
-      hadj[3] = fmaf(ry1, adj[41], hadj[3]); \
-      hadj[3] = fmaf(ry2, adj[44], hadj[3]); \
-      radial = fmaf(dR[6], yw, radial); \
-    } \
-    { /* path 10: edge l=3, source l=1 -> l=2 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[7] * h[1]; \
-      const float rh1 = R[7] * h[2]; \
-      const float rh2 = R[7] * h[3]; \
-      ang[9] = fmaf(rh0, adj[45], ang[9]); \
-      ang[9] = fmaf(rh1, adj[46], ang[9]); \
-      ang[9] = fmaf(rh2, adj[47], ang[9]); \
-      ang[10] = fmaf(rh0, adj[48], ang[10]); \
-      ang[10] = fmaf(rh1, adj[49], ang[10]); \
-      ang[10] = fmaf(rh2, adj[50], ang[10]); \
-      ang[11] = fmaf(rh0, adj[51], ang[11]); \
-      ang[11] = fmaf(rh1, adj[52], ang[11]); \
-      ang[11] = fmaf(rh2, adj[53], ang[11]); \
-      ang[12] = fmaf(rh0, adj[54], ang[12]); \
-      ang[12] = fmaf(rh1, adj[55], ang[12]); \
-      ang[12] = fmaf(rh2, adj[56], ang[12]); \
-      ang[13] = fmaf(rh0, adj[57], ang[13]); \
-      ang[13] = fmaf(rh1, adj[58], ang[13]); \
-      ang[13] = fmaf(rh2, adj[59], ang[13]); \
-      ang[14] = fmaf(rh0, adj[60], ang[14]); \
-      ang[14] = fmaf(rh1, adj[61], ang[14]); \
-      ang[14] = fmaf(rh2, adj[62], ang[14]); \
-      ang[15] = fmaf(rh0, adj[63], ang[15]); \
-      ang[15] = fmaf(rh1, adj[64], ang[15]); \
-      ang[15] = fmaf(rh2, adj[65], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[63], fmaf(y[14], adj[60], fmaf(y[13], adj[57], fmaf(y[12], adj[54], fmaf(y[11], adj[51], fmaf(y[10], adj[48], y[9] * adj[45])))))); \
-        hadj[1] = fmaf(R[7], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[64], fmaf(y[14], adj[61], fmaf(y[13], adj[58], fmaf(y[12], adj[55], fmaf(y[11], adj[52], fmaf(y[10], adj[49], y[9] * adj[46])))))); \
-        hadj[2] = fmaf(R[7], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[65], fmaf(y[14], adj[62], fmaf(y[13], adj[59], fmaf(y[12], adj[56], fmaf(y[11], adj[53], fmaf(y[10], adj[50], y[9] * adj[47])))))); \
-        hadj[3] = fmaf(R[7], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
-      radial = fmaf(dR[7], yw, radial); \
-    } \
-    { /* path 13: edge l=3, source l=0 -> l=3 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[8] * h[0]; \
-      ang[9] = fmaf(rh0, adj[66], ang[9]); \
-      ang[10] = fmaf(rh0, adj[67], ang[10]); \
-      ang[11] = fmaf(rh0, adj[68], ang[11]); \
-      ang[12] = fmaf(rh0, adj[69], ang[12]); \
-      ang[13] = fmaf(rh0, adj[70], ang[13]); \
-      ang[14] = fmaf(rh0, adj[71], ang[14]); \
-      ang[15] = fmaf(rh0, adj[72], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[72], fmaf(y[14], adj[71], fmaf(y[13], adj[70], fmaf(y[12], adj[69], fmaf(y[11], adj[68], fmaf(y[10], adj[67], y[9] * adj[66])))))); \
-        hadj[0] = fmaf(R[8], s_, hadj[0]); yw = fmaf(h[0], s_, yw); } \
-      radial = fmaf(dR[8], yw, radial); \
-    } \
-    { /* path 14: edge l=2, source l=1 -> l=3 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[9] * h[1]; \
-      const float rh1 = R[9] * h[2]; \
-      const float rh2 = R[9] * h[3]; \
-      ang[4] = fmaf(rh0, adj[73], ang[4]); \
-      ang[4] = fmaf(rh1, adj[74], ang[4]); \
-      ang[4] = fmaf(rh2, adj[75], ang[4]); \
-      ang[5] = fmaf(rh0, adj[76], ang[5]); \
-      ang[5] = fmaf(rh1, adj[77], ang[5]); \
-      ang[5] = fmaf(rh2, adj[78], ang[5]); \
-      ang[6] = fmaf(rh0, adj[79], ang[6]); \
-      ang[6] = fmaf(rh1, adj[80], ang[6]); \
-      ang[6] = fmaf(rh2, adj[81], ang[6]); \
-      ang[7] = fmaf(rh0, adj[82], ang[7]); \
-      ang[7] = fmaf(rh1, adj[83], ang[7]); \
-      ang[7] = fmaf(rh2, adj[84], ang[7]); \
-      ang[8] = fmaf(rh0, adj[85], ang[8]); \
-      ang[8] = fmaf(rh1, adj[86], ang[8]); \
-      ang[8] = fmaf(rh2, adj[87], ang[8]); \
-      { const float s_ = fmaf(y[8], adj[85], fmaf(y[7], adj[82], fmaf(y[6], adj[79], fmaf(y[5], adj[76], y[4] * adj[73])))); \
-        hadj[1] = fmaf(R[9], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[86], fmaf(y[7], adj[83], fmaf(y[6], adj[80], fmaf(y[5], adj[77], y[4] * adj[74])))); \
-        hadj[2] = fmaf(R[9], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[87], fmaf(y[7], adj[84], fmaf(y[6], adj[81], fmaf(y[5], adj[78], y[4] * adj[75])))); \
-        hadj[3] = fmaf(R[9], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
-      radial = fmaf(dR[9], yw, radial); \
-    }
 #define SXB_S2_G1_NUM_PATHS 4
 #define SXB_S2_G1_NUM_ROWS 80
 #define SXB_S2_G1_NUM_LME 12
 #define SXB_S2_G1_PATH_LIST {2, 6, 7, 11}
 #define SXB_S2_G1_LME_LIST {2, 6, 7, 11, 12, 16, 17, 21, 26, 31, 36, 41}
 #define SXB_S2_G1_SOURCE_MASK 496u   // source components lm2 the set touches
-#define SXB_S2_G1_EDGE_MASK 65535u   // edge harmonics lm1 the set touches
-#define SXB_S2_G1_HAS_PATH0 0
 // X(term, row inside the set, output inside the set)
 #define SXB_S2_G1_TERMS(X) \
     X(4, 75, 7) \
@@ -5353,153 +5662,12 @@
       acc[78] = fmaf(t3, y[0], acc[78]); \
       acc[79] = fmaf(t4, y[0], acc[79]); \
     }
-#define SXB_S2_G1_REVERSE_BODY \
-    { /* path 2: edge l=2, source l=2 -> l=0 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[0] * y[4]; \
-      const float ry1 = R[0] * y[5]; \
-      const float ry2 = R[0] * y[6]; \
-      const float ry3 = R[0] * y[7]; \
-      const float ry4 = R[0] * y[8]; \
-      { const float w = fmaf(h[8], adj[4], fmaf(h[7], adj[3], fmaf(h[6], adj[2], fmaf(h[5], adj[1], h[4] * adj[0])))); \
-        ang[4] = fmaf(R[0], w, ang[4]); yw = fmaf(y[4], w, yw); } \
-      { const float w = fmaf(h[8], adj[9], fmaf(h[7], adj[8], fmaf(h[6], adj[7], fmaf(h[5], adj[6], h[4] * adj[5])))); \
-        ang[5] = fmaf(R[0], w, ang[5]); yw = fmaf(y[5], w, yw); } \
-      { const float w = fmaf(h[8], adj[14], fmaf(h[7], adj[13], fmaf(h[6], adj[12], fmaf(h[5], adj[11], h[4] * adj[10])))); \
-        ang[6] = fmaf(R[0], w, ang[6]); yw = fmaf(y[6], w, yw); } \
-      { const float w = fmaf(h[8], adj[19], fmaf(h[7], adj[18], fmaf(h[6], adj[17], fmaf(h[5], adj[16], h[4] * adj[15])))); \
-        ang[7] = fmaf(R[0], w, ang[7]); yw = fmaf(y[7], w, yw); } \
-      { const float w = fmaf(h[8], adj[24], fmaf(h[7], adj[23], fmaf(h[6], adj[22], fmaf(h[5], adj[21], h[4] * adj[20])))); \
-        ang[8] = fmaf(R[0], w, ang[8]); yw = fmaf(y[8], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[0], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[5], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[10], hadj[4]); \
-      hadj[4] = fmaf(ry3, adj[15], hadj[4]); \
-      hadj[4] = fmaf(ry4, adj[20], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[1], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[6], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[11], hadj[5]); \
-      hadj[5] = fmaf(ry3, adj[16], hadj[5]); \
-      hadj[5] = fmaf(ry4, adj[21], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[2], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[7], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[12], hadj[6]); \
-      hadj[6] = fmaf(ry3, adj[17], hadj[6]); \
-      hadj[6] = fmaf(ry4, adj[22], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[3], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[8], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[13], hadj[7]); \
-      hadj[7] = fmaf(ry3, adj[18], hadj[7]); \
-      hadj[7] = fmaf(ry4, adj[23], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[4], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[9], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[14], hadj[8]); \
-      hadj[8] = fmaf(ry3, adj[19], hadj[8]); \
-      hadj[8] = fmaf(ry4, adj[24], hadj[8]); \
-      radial = fmaf(dR[0], yw, radial); \
-    } \
-    { /* path 6: edge l=1, source l=2 -> l=1 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[1] * y[1]; \
-      const float ry1 = R[1] * y[2]; \
-      const float ry2 = R[1] * y[3]; \
-      { const float w = fmaf(h[8], adj[29], fmaf(h[7], adj[28], fmaf(h[6], adj[27], fmaf(h[5], adj[26], h[4] * adj[25])))); \
-        ang[1] = fmaf(R[1], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[8], adj[34], fmaf(h[7], adj[33], fmaf(h[6], adj[32], fmaf(h[5], adj[31], h[4] * adj[30])))); \
-        ang[2] = fmaf(R[1], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[8], adj[39], fmaf(h[7], adj[38], fmaf(h[6], adj[37], fmaf(h[5], adj[36], h[4] * adj[35])))); \
-        ang[3] = fmaf(R[1], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[25], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[30], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[35], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[26], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[31], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[36], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[27], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[32], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[37], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[28], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[33], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[38], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[29], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[34], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[39], hadj[8]); \
-      radial = fmaf(dR[1], yw, radial); \
-    } \
-    { /* path 7: edge l=3, source l=2 -> l=1 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[2] * h[4]; \
-      const float rh1 = R[2] * h[5]; \
-      const float rh2 = R[2] * h[6]; \
-      const float rh3 = R[2] * h[7]; \
-      const float rh4 = R[2] * h[8]; \
-      ang[9] = fmaf(rh0, adj[40], ang[9]); \
-      ang[9] = fmaf(rh1, adj[41], ang[9]); \
-      ang[9] = fmaf(rh2, adj[42], ang[9]); \
-      ang[9] = fmaf(rh3, adj[43], ang[9]); \
-      ang[9] = fmaf(rh4, adj[44], ang[9]); \
-      ang[10] = fmaf(rh0, adj[45], ang[10]); \
-      ang[10] = fmaf(rh1, adj[46], ang[10]); \
-      ang[10] = fmaf(rh2, adj[47], ang[10]); \
-      ang[10] = fmaf(rh3, adj[48], ang[10]); \
-      ang[10] = fmaf(rh4, adj[49], ang[10]); \
-      ang[11] = fmaf(rh0, adj[50], ang[11]); \
-      ang[11] = fmaf(rh1, adj[51], ang[11]); \
-      ang[11] = fmaf(rh2, adj[52], ang[11]); \
-      ang[11] = fmaf(rh3, adj[53], ang[11]); \
-      ang[11] = fmaf(rh4, adj[54], ang[11]); \
-      ang[12] = fmaf(rh0, adj[55], ang[12]); \
-      ang[12] = fmaf(rh1, adj[56], ang[12]); \
-      ang[12] = fmaf(rh2, adj[57], ang[12]); \
-      ang[12] = fmaf(rh3, adj[58], ang[12]); \
-      ang[12] = fmaf(rh4, adj[59], ang[12]); \
-      ang[13] = fmaf(rh0, adj[60], ang[13]); \
-      ang[13] = fmaf(rh1, adj[61], ang[13]); \
-      ang[13] = fmaf(rh2, adj[62], ang[13]); \
-      ang[13] = fmaf(rh3, adj[63], ang[13]); \
-      ang[13] = fmaf(rh4, adj[64], ang[13]); \
-      ang[14] = fmaf(rh0, adj[65], ang[14]); \
-      ang[14] = fmaf(rh1, adj[66], ang[14]); \
-      ang[14] = fmaf(rh2, adj[67], ang[14]); \
-      ang[14] = fmaf(rh3, adj[68], ang[14]); \
-      ang[14] = fmaf(rh4, adj[69], ang[14]); \
-      ang[15] = fmaf(rh0, adj[70], ang[15]); \
-      ang[15] = fmaf(rh1, adj[71], ang[15]); \
-      ang[15] = fmaf(rh2, adj[72], ang[15]); \
-      ang[15] = fmaf(rh3, adj[73], ang[15]); \
-      ang[15] = fmaf(rh4, adj[74], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[70], fmaf(y[14], adj[65], fmaf(y[13], adj[60], fmaf(y[12], adj[55], fmaf(y[11], adj[50], fmaf(y[10], adj[45], y[9] * adj[40])))))); \
-        hadj[4] = fmaf(R[2], s_, hadj[4]); yw = fmaf(h[4], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[71], fmaf(y[14], adj[66], fmaf(y[13], adj[61], fmaf(y[12], adj[56], fmaf(y[11], adj[51], fmaf(y[10], adj[46], y[9] * adj[41])))))); \
-        hadj[5] = fmaf(R[2], s_, hadj[5]); yw = fmaf(h[5], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[72], fmaf(y[14], adj[67], fmaf(y[13], adj[62], fmaf(y[12], adj[57], fmaf(y[11], adj[52], fmaf(y[10], adj[47], y[9] * adj[42])))))); \
-        hadj[6] = fmaf(R[2], s_, hadj[6]); yw = fmaf(h[6], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[73], fmaf(y[14], adj[68], fmaf(y[13], adj[63], fmaf(y[12], adj[58], fmaf(y[11], adj[53], fmaf(y[10], adj[48], y[9] * adj[43])))))); \
-        hadj[7] = fmaf(R[2], s_, hadj[7]); yw = fmaf(h[7], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[74], fmaf(y[14], adj[69], fmaf(y[13], adj[64], fmaf(y[12], adj[59], fmaf(y[11], adj[54], fmaf(y[10], adj[49], y[9] * adj[44])))))); \
-        hadj[8] = fmaf(R[2], s_, hadj[8]); yw = fmaf(h[8], s_, yw); } \
-      radial = fmaf(dR[2], yw, radial); \
-    } \
-    { /* path 11: edge l=0, source l=2 -> l=2 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[3] * y[0]; \
-      { const float w = fmaf(h[8], adj[79], fmaf(h[7], adj[78], fmaf(h[6], adj[77], fmaf(h[5], adj[76], h[4] * adj[75])))); \
-        ang[0] = fmaf(R[3], w, ang[0]); yw = fmaf(y[0], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[75], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[76], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[77], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[78], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[79], hadj[8]); \
-      radial = fmaf(dR[3], yw, radial); \
-    }
 #define SXB_S2_G2_NUM_PATHS 3
 #define SXB_S2_G2_NUM_ROWS 75
 #define SXB_S2_G2_NUM_LME 19
 #define SXB_S2_G2_PATH_LIST {12, 15, 16}
 #define SXB_S2_G2_LME_LIST {22, 27, 32, 37, 42, 45, 46, 49, 50, 53, 54, 57, 58, 61, 62, 65, 66, 69, 70}
 #define SXB_S2_G2_SOURCE_MASK 496u   // source components lm2 the set touches
-#define SXB_S2_G2_EDGE_MASK 65534u   // edge harmonics lm1 the set touches
-#define SXB_S2_G2_HAS_PATH0 0
 // X(term, row inside the set, output inside the set)
 #define SXB_S2_G2_TERMS(X) \
     X(16, 25, 13) \
@@ -5685,131 +5853,4 @@
       acc[72] = fmaf(t2, y[15], acc[72]); \
       acc[73] = fmaf(t3, y[15], acc[73]); \
       acc[74] = fmaf(t4, y[15], acc[74]); \
-    }
-#define SXB_S2_G2_REVERSE_BODY \
-    { /* path 12: edge l=2, source l=2 -> l=2 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[0] * y[4]; \
-      const float ry1 = R[0] * y[5]; \
-      const float ry2 = R[0] * y[6]; \
-      const float ry3 = R[0] * y[7]; \
-      const float ry4 = R[0] * y[8]; \
-      { const float w = fmaf(h[8], adj[4], fmaf(h[7], adj[3], fmaf(h[6], adj[2], fmaf(h[5], adj[1], h[4] * adj[0])))); \
-        ang[4] = fmaf(R[0], w, ang[4]); yw = fmaf(y[4], w, yw); } \
-      { const float w = fmaf(h[8], adj[9], fmaf(h[7], adj[8], fmaf(h[6], adj[7], fmaf(h[5], adj[6], h[4] * adj[5])))); \
-        ang[5] = fmaf(R[0], w, ang[5]); yw = fmaf(y[5], w, yw); } \
-      { const float w = fmaf(h[8], adj[14], fmaf(h[7], adj[13], fmaf(h[6], adj[12], fmaf(h[5], adj[11], h[4] * adj[10])))); \
-        ang[6] = fmaf(R[0], w, ang[6]); yw = fmaf(y[6], w, yw); } \
-      { const float w = fmaf(h[8], adj[19], fmaf(h[7], adj[18], fmaf(h[6], adj[17], fmaf(h[5], adj[16], h[4] * adj[15])))); \
-        ang[7] = fmaf(R[0], w, ang[7]); yw = fmaf(y[7], w, yw); } \
-      { const float w = fmaf(h[8], adj[24], fmaf(h[7], adj[23], fmaf(h[6], adj[22], fmaf(h[5], adj[21], h[4] * adj[20])))); \
-        ang[8] = fmaf(R[0], w, ang[8]); yw = fmaf(y[8], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[0], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[5], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[10], hadj[4]); \
-      hadj[4] = fmaf(ry3, adj[15], hadj[4]); \
-      hadj[4] = fmaf(ry4, adj[20], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[1], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[6], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[11], hadj[5]); \
-      hadj[5] = fmaf(ry3, adj[16], hadj[5]); \
-      hadj[5] = fmaf(ry4, adj[21], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[2], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[7], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[12], hadj[6]); \
-      hadj[6] = fmaf(ry3, adj[17], hadj[6]); \
-      hadj[6] = fmaf(ry4, adj[22], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[3], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[8], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[13], hadj[7]); \
-      hadj[7] = fmaf(ry3, adj[18], hadj[7]); \
-      hadj[7] = fmaf(ry4, adj[23], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[4], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[9], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[14], hadj[8]); \
-      hadj[8] = fmaf(ry3, adj[19], hadj[8]); \
-      hadj[8] = fmaf(ry4, adj[24], hadj[8]); \
-      radial = fmaf(dR[0], yw, radial); \
-    } \
-    { /* path 15: edge l=1, source l=2 -> l=3 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[1] * y[1]; \
-      const float ry1 = R[1] * y[2]; \
-      const float ry2 = R[1] * y[3]; \
-      { const float w = fmaf(h[8], adj[29], fmaf(h[7], adj[28], fmaf(h[6], adj[27], fmaf(h[5], adj[26], h[4] * adj[25])))); \
-        ang[1] = fmaf(R[1], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[8], adj[34], fmaf(h[7], adj[33], fmaf(h[6], adj[32], fmaf(h[5], adj[31], h[4] * adj[30])))); \
-        ang[2] = fmaf(R[1], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[8], adj[39], fmaf(h[7], adj[38], fmaf(h[6], adj[37], fmaf(h[5], adj[36], h[4] * adj[35])))); \
-        ang[3] = fmaf(R[1], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[25], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[30], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[35], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[26], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[31], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[36], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[27], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[32], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[37], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[28], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[33], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[38], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[29], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[34], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[39], hadj[8]); \
-      radial = fmaf(dR[1], yw, radial); \
-    } \
-    { /* path 16: edge l=3, source l=2 -> l=3 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[2] * h[4]; \
-      const float rh1 = R[2] * h[5]; \
-      const float rh2 = R[2] * h[6]; \
-      const float rh3 = R[2] * h[7]; \
-      const float rh4 = R[2] * h[8]; \
-      ang[9] = fmaf(rh0, adj[40], ang[9]); \
-      ang[9] = fmaf(rh1, adj[41], ang[9]); \
-      ang[9] = fmaf(rh2, adj[42], ang[9]); \
-      ang[9] = fmaf(rh3, adj[43], ang[9]); \
-      ang[9] = fmaf(rh4, adj[44], ang[9]); \
-      ang[10] = fmaf(rh0, adj[45], ang[10]); \
-      ang[10] = fmaf(rh1, adj[46], ang[10]); \
-      ang[10] = fmaf(rh2, adj[47], ang[10]); \
-      ang[10] = fmaf(rh3, adj[48], ang[10]); \
-      ang[10] = fmaf(rh4, adj[49], ang[10]); \
-      ang[11] = fmaf(rh0, adj[50], ang[11]); \
-      ang[11] = fmaf(rh1, adj[51], ang[11]); \
-      ang[11] = fmaf(rh2, adj[52], ang[11]); \
-      ang[11] = fmaf(rh3, adj[53], ang[11]); \
-      ang[11] = fmaf(rh4, adj[54], ang[11]); \
-      ang[12] = fmaf(rh0, adj[55], ang[12]); \
-      ang[12] = fmaf(rh1, adj[56], ang[12]); \
-      ang[12] = fmaf(rh2, adj[57], ang[12]); \
-      ang[12] = fmaf(rh3, adj[58], ang[12]); \
-      ang[12] = fmaf(rh4, adj[59], ang[12]); \
-      ang[13] = fmaf(rh0, adj[60], ang[13]); \
-      ang[13] = fmaf(rh1, adj[61], ang[13]); \
-      ang[13] = fmaf(rh2, adj[62], ang[13]); \
-      ang[13] = fmaf(rh3, adj[63], ang[13]); \
-      ang[13] = fmaf(rh4, adj[64], ang[13]); \
-      ang[14] = fmaf(rh0, adj[65], ang[14]); \
-      ang[14] = fmaf(rh1, adj[66], ang[14]); \
-      ang[14] = fmaf(rh2, adj[67], ang[14]); \
-      ang[14] = fmaf(rh3, adj[68], ang[14]); \
-      ang[14] = fmaf(rh4, adj[69], ang[14]); \
-      ang[15] = fmaf(rh0, adj[70], ang[15]); \
-      ang[15] = fmaf(rh1, adj[71], ang[15]); \
-      ang[15] = fmaf(rh2, adj[72], ang[15]); \
-      ang[15] = fmaf(rh3, adj[73], ang[15]); \
-      ang[15] = fmaf(rh4, adj[74], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[70], fmaf(y[14], adj[65], fmaf(y[13], adj[60], fmaf(y[12], adj[55], fmaf(y[11], adj[50], fmaf(y[10], adj[45], y[9] * adj[40])))))); \
-        hadj[4] = fmaf(R[2], s_, hadj[4]); yw = fmaf(h[4], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[71], fmaf(y[14], adj[66], fmaf(y[13], adj[61], fmaf(y[12], adj[56], fmaf(y[11], adj[51], fmaf(y[10], adj[46], y[9] * adj[41])))))); \
-        hadj[5] = fmaf(R[2], s_, hadj[5]); yw = fmaf(h[5], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[72], fmaf(y[14], adj[67], fmaf(y[13], adj[62], fmaf(y[12], adj[57], fmaf(y[11], adj[52], fmaf(y[10], adj[47], y[9] * adj[42])))))); \
-        hadj[6] = fmaf(R[2], s_, hadj[6]); yw = fmaf(h[6], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[73], fmaf(y[14], adj[68], fmaf(y[13], adj[63], fmaf(y[12], adj[58], fmaf(y[11], adj[53], fmaf(y[10], adj[48], y[9] * adj[43])))))); \
-        hadj[7] = fmaf(R[2], s_, hadj[7]); yw = fmaf(h[7], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[74], fmaf(y[14], adj[69], fmaf(y[13], adj[64], fmaf(y[12], adj[59], fmaf(y[11], adj[54], fmaf(y[10], adj[49], y[9] * adj[44])))))); \
-        hadj[8] = fmaf(R[2], s_, hadj[8]); yw = fmaf(h[8], s_, yw); } \
-      radial = fmaf(dR[2], yw, radial); \
     }

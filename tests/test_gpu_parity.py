@@ -547,3 +547,30 @@ def test_contraction_runs_of_elements(pkg, model_path, arch, counts):
     assert np.abs(ev.node_energies - energies).max() <= TOL_E
     got = ev._reduce_atom_forces(n, execution_graph_generation=res["generation"])
     assert np.abs(got - forces).max() <= TOL_F * max(1.0, np.abs(forces).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,options", [(128, {}), (64, {}), (64, {"a0_scaled": True, "a1_scaled": True}), (128, {"agnesi": True})])
+def test_layer1_gradient_widths_and_odd_edge_counts(pkg, model_path, channels, options):
+    """The layer-1 gradient takes two edges at a time from chunks of 64 list edges: receivers without, with one, with an odd
+    number and with more than a chunk of active edges, at both compiled widths, against the oracle."""
+    from oracle import mace_numpy, neighbor
+
+    path = model_path("medium", 35, channels=channels, **options)
+    rng = np.random.default_rng(9)
+    blob = rng.uniform(0.0, 1.0, (26, 3)) * np.array([9.0, 9.0, 4.0])
+    keep = [0]
+    for i in range(1, len(blob)):
+        if all(np.linalg.norm(blob[i] - blob[j]) > 1.6 for j in keep):
+            keep.append(i)
+    pos = np.concatenate([blob[keep], [[30.0, 30.0, 30.0], [45.0, 30.0, 30.0], [45.0, 33.0, 30.0]]])
+    cell = np.eye(3) * 60.0
+    types = (np.arange(len(pos)) % 3).astype(np.int32)
+    dense_pos, dense_cell, dense_types = pkg.modelgen.srtio3(2, 0.05, 3)
+    calc = pkg.Calculator(path, skin=0.5)
+    for p, c, t in ((pos, cell, types), (dense_pos, dense_cell * 0.93, dense_types)):
+        out = calc.calculate(p, c, t)
+        first, src, shifts = neighbor.build_neighbor_graph(p, c, calc.evaluator.r_cut + 0.5)
+        _e, energies, forces, _s = mace_numpy.NumpyMACE(str(path)).energy_forces_stress(t, p, c, first, src, shifts)
+        assert np.abs(out["energies"] - energies).max() <= TOL_E
+        assert np.abs(out["forces"] - forces).max() <= TOL_F * max(1.0, np.abs(forces).max())
