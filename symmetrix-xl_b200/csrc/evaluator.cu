@@ -1296,7 +1296,7 @@ void Evaluator::run_pipeline(int phases)
         }
         if (deterministic_ && !model_.single_layer) {
             span_begin("source_adjoint_schedule");
-            reduce_source_adjoint_kernel<<<ALL, 128, 0, stream_>>>(NH * C, source_offsets_.ptr, source_edges_.ptr, geom_.ptr, grid_.r_cut,
+            reduce_source_adjoint_kernel<<<ALL, kScheduleChunk, 0, stream_>>>(NH * C, source_offsets_.ptr, source_edges_.ptr, geom_.ptr, grid_.r_cut,
                                                                   edge_source_adjoint_.ptr, H1_adj_.ptr);
             launches_ += 1;
             span_end();
@@ -1402,11 +1402,11 @@ void Evaluator::run_pipeline(int phases)
         span_begin("finalize");
         if (deterministic_) {
             const long blocks = std::max<long>(blocks_for(std::max<long>(num_edges_, 1), kTotalsThreads), blocks_for(R, kTotalsThreads));
-            reduce_node_forces_kernel<<<blocks_for(ALL, 128), 128, 0, stream_>>>(ALL, R, first_.ptr, source_offsets_.ptr, source_edges_.ptr,
+            reduce_node_forces_kernel<<<blocks_for(static_cast<long>(ALL) * 32, 128), 128, 0, stream_>>>(ALL, R, first_.ptr, source_offsets_.ptr, source_edges_.ptr,
                                                                                   edge_forces_.ptr, forces_.ptr);
             partial_totals_kernel<<<blocks, kTotalsThreads, 0, stream_>>>(num_edges_, R, geom_.ptr, edge_forces_.ptr, node_energies_.ptr,
                                                                           det_partials_.ptr);
-            final_totals_kernel<<<1, 32, 0, stream_>>>(static_cast<int>(blocks), det_partials_.ptr, energy_slots_.ptr, virial_slots_.ptr);
+            final_totals_kernel<<<1, 320, 0, stream_>>>(static_cast<int>(blocks), det_partials_.ptr, energy_slots_.ptr, virial_slots_.ptr);
             launches_ += 3;
         }
         publish_results_kernel<<<blocks_for(11 + static_cast<long>(R) + 3 * static_cast<long>(ALL), 256), 256, 0, stream_>>>(
