@@ -81,6 +81,22 @@ __device__ __forceinline__ void add_angular_force(const float* __restrict__ row,
     }
 }
 
+// Writes the harmonics and gradients of an edge in that layout.
+__device__ __forceinline__ void fill_pair_harmonics(const EdgeGeom& g, float2* __restrict__ y, float* __restrict__ grad)
+{
+    float Y[16], gX[16], gY[16], gZ[16];
+    harmonics16<true>(g.ux, g.uy, g.uz, 1.0f / g.r, Y, gX, gY, gZ);
+#pragma unroll
+    for (int lm = 0; lm < 16; ++lm) {
+        const int l = lm < 1 ? 0 : lm < 4 ? 1 : lm < 9 ? 2 : 3, m = lm - l * l;
+        y[(l == 0 ? 0 : l == 1 ? 2 : l == 2 ? 6 : 12) + m] = make_float2(Y[lm], Y[lm]);
+        if (l > 0) {
+            float* o = grad + (l == 1 ? 0 : l == 2 ? 12 : 28) + 3 * m;
+            o[0] = gX[lm]; o[1] = gY[lm]; o[2] = gZ[lm];
+        }
+    }
+}
+
 // Fills the chunk with the active ones of the edges [begin, begin + count) of one receiver, count <= 64: the first two
 // warps, one edge per lane, in edge order.  `words` 16-byte words per (pair, interval) of the table.
 __device__ __forceinline__ void fill_active_chunk(ActiveChunk& s, int begin, int count, const int* __restrict__ sources,
@@ -118,17 +134,7 @@ __device__ __forceinline__ void fill_active_chunk(ActiveChunk& s, int begin, int
     }
     s.index[slot] = make_int4((pair * grid.intervals + interval) * words, j, e, 0);
     s.misc[slot] = make_float4(x, g.ux, g.uy, g.uz);
-    float Y[16], gX[16], gY[16], gZ[16];
-    harmonics16<true>(g.ux, g.uy, g.uz, 1.0f / g.r, Y, gX, gY, gZ);
-#pragma unroll
-    for (int lm = 0; lm < 16; ++lm) {
-        const int l = lm < 1 ? 0 : lm < 4 ? 1 : lm < 9 ? 2 : 3, m = lm - l * l;
-        s.y[slot][(l == 0 ? 0 : l == 1 ? 2 : l == 2 ? 6 : 12) + m] = make_float2(Y[lm], Y[lm]);
-        if (l > 0) {
-            float* o = &s.g[slot][(l == 1 ? 0 : l == 2 ? 12 : 28) + 3 * m];
-            o[0] = gX[lm]; o[1] = gY[lm]; o[2] = gZ[lm];
-        }
-    }
+    fill_pair_harmonics(g, s.y[slot], s.g[slot]);
     s.len[slot] = make_float2(g.r, density_table != nullptr
         ? scalar_spline_derivative(density_table, (type_i * density_types + (density_types > 1 ? atype[j] : 0)) * grid.intervals + interval, x) : 0.0f);
 }

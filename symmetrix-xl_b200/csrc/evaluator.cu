@@ -216,6 +216,8 @@ Evaluator::Evaluator(const std::string& json_path, int device_ordinal, const std
     SXB_ALLOW_SHARED_ROWS(S1, 64);
     SXB_ALLOW_SHARED_ROWS(S2, 128);
 #undef SXB_ALLOW_SHARED_ROWS
+    SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpsPerBlock * sizeof(WarpPairChunk)));
+    SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpsPerBlock * sizeof(WarpPairChunk)));
     SXB_CUDA(cudaFuncSetAttribute(tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes));
     SXB_CUDA(cudaFuncSetAttribute(tc_gemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kT3SmemBytes));
     SXB_CUDA(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device_));
@@ -1377,9 +1379,9 @@ void Evaluator::run_pipeline(int phases)
             {
                 const int parts = l0_reverse_parts(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
                 if (C == 128)
-                    l0_reverse_warp_kernel<4><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
+                    l0_reverse_pair_kernel<4><<<warp_grid, warp_threads, kWarpsPerBlock * sizeof(WarpPairChunk), stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else if (C == 64)
-                    l0_reverse_warp_kernel<2><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
+                    l0_reverse_pair_kernel<2><<<warp_grid, warp_threads, kWarpsPerBlock * sizeof(WarpPairChunk), stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else if (C == 32)
                     l0_reverse_warp_kernel<1><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else
