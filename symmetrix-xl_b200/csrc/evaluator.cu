@@ -862,14 +862,13 @@ void Evaluator::upload_split(SplitWeight& out, const float* w, int rows, int col
     // forward product: N = cols, K = rows; reverse product: N = rows, K = cols
     if (rows % kTcChunk != 0 || cols % kTcChunk != 0)
         throw std::invalid_argument("Linear extents must be multiples of 32 for the tensor-core kernel.");
-    out.map_fwd_hi = make_weight_map(out.fwd_hi.ptr, cols, rows, std::min(cols, kTcNTile));
-    out.map_fwd_lo = make_weight_map(out.fwd_lo.ptr, cols, rows, std::min(cols, kTcNTile));
-    out.map_rev_hi = make_weight_map(out.rev_hi.ptr, rows, cols, std::min(rows, kTcNTile));
-    out.map_rev_lo = make_weight_map(out.rev_lo.ptr, rows, cols, std::min(rows, kTcNTile));
-    out.wide_fwd_hi = make_weight_map(out.fwd_hi.ptr, cols, rows, std::min(cols, 128));
-    out.wide_fwd_lo = make_weight_map(out.fwd_lo.ptr, cols, rows, std::min(cols, 128));
-    out.wide_rev_hi = make_weight_map(out.rev_hi.ptr, rows, cols, std::min(rows, 128));
-    out.wide_rev_lo = make_weight_map(out.rev_lo.ptr, rows, cols, std::min(rows, 128));
+    for (int w = 0; w < 3; ++w) {
+        const int width = 32 << w;
+        out.map_fwd_hi[w] = make_weight_map(out.fwd_hi.ptr, cols, rows, std::min(cols, width));
+        out.map_fwd_lo[w] = make_weight_map(out.fwd_lo.ptr, cols, rows, std::min(cols, width));
+        out.map_rev_hi[w] = make_weight_map(out.rev_hi.ptr, rows, cols, std::min(rows, width));
+        out.map_rev_lo[w] = make_weight_map(out.rev_lo.ptr, rows, cols, std::min(rows, width));
+    }
 }
 
 // Runs a group of independent linears as one tensor-core launch (or as FP32 SIMT launches when the
@@ -905,12 +904,31 @@ void Evaluator::launch_tc(const std::vector<TcCall>& calls)
         }
         return;
     }
+    // Widest column tile of {128, 64, 32} not above `width` that divides N, as an index into the tensor maps; -1: none
+    // (N = 32 or a multiple of 64 has one, other widths go to the first tcgen05 kernel and its checks).
+    auto tile_index = [](int N, int width) {
+        if (N != 32 && N % 64 != 0) return -1;
+        for (int w = 2; w >= 0; --w)
+            if ((32 << w) <= width && N % (32 << w) == 0) return w;
+        return -1;
+    };
+    auto work_items = [&](int width) {
+        long items = 0;
+        for (const auto& c : calls) {
+            const int N = c.reverse ? c.w->rows : c.w->cols, nodes = kTcRows / c.a_rows.components;
+            items += static_cast<long>((std::max(c.num_nodes, 0) + nodes - 1) / nodes) * (N / (32 << tile_index(N, width)));
+        }
+        return items;
+    };
     bool streaming = use_tma_activations_;
-    for (const auto& c : calls) {
-        const int N = c.reverse ? c.w->rows : c.w->cols;
-        const int n_tile = std::min(N, 128);
-        if ((n_tile != 32 && n_tile != 64 && n_tile != 128) || N % n_tile != 0) streaming = false;
-    }
+    for (const auto& c : calls)
+        if (tile_index(c.reverse ? c.w->rows : c.w->cols, 128) < 0) streaming = false;
+    // Few rows leave most SMs without a work item, and an item's time goes with its width (0.8 us per 32 of K at 128
+    // columns): narrower tiles until half the SMs have one.  40 atoms, 128 channels, six launches: 15, 21, 15, 15, 15,
+    // 15 us at 128 columns, 13, 18, 11, 13, 13, 13 us at 32.
+    int width = 128;
+    if (streaming)
+        while (width > 32 && 2 * work_items(width) <= num_sms_) width /= 2;
     if (streaming) {
         std::size_t next = 0;
         while (next < calls.size()) {
@@ -924,13 +942,14 @@ void Evaluator::launch_tc(const std::vector<TcCall>& calls)
                 p.N = c.reverse ? c.w->rows : c.w->cols;
                 p.K = c.reverse ? c.w->cols : c.w->rows;
                 if (p.K % kTcChunk != 0) throw std::invalid_argument("Linear extents are not supported by the tensor-core kernel.");
-                p.n_tile = std::min(p.N, 128);
+                const int w = tile_index(p.N, width);
+                p.n_tile = 32 << w;
                 p.n_tiles = p.N / p.n_tile;
                 p.nodes_per_tile = kTcRows / c.a_rows.components;
                 p.rows_per_tile = p.nodes_per_tile * c.a_rows.components;
                 p.map_a = make_activation_map(c.A, c.a_rows, c.first_node, c.num_nodes, p.K, p.nodes_per_tile);
-                p.map_hi = c.reverse ? c.w->wide_rev_hi : c.w->wide_fwd_hi;
-                p.map_lo = c.reverse ? c.w->wide_rev_lo : c.w->wide_fwd_lo;
+                p.map_hi = c.reverse ? c.w->map_rev_hi[w] : c.w->map_fwd_hi[w];
+                p.map_lo = c.reverse ? c.w->map_rev_lo[w] : c.w->map_fwd_lo[w];
                 p.C = c.C;
                 p.bias = c.bias;
                 p.c_rows = c.c_rows;
@@ -960,8 +979,8 @@ void Evaluator::launch_tc(const std::vector<TcCall>& calls)
             if (c.num_nodes <= 0) continue;
             TcProblem& p = batch.problem[count];
             p.A = c.A;
-            p.map_hi = c.reverse ? c.w->map_rev_hi : c.w->map_fwd_hi;
-            p.map_lo = c.reverse ? c.w->map_rev_lo : c.w->map_fwd_lo;
+            p.map_hi = c.reverse ? c.w->map_rev_hi[1] : c.w->map_fwd_hi[1];
+            p.map_lo = c.reverse ? c.w->map_rev_lo[1] : c.w->map_fwd_lo[1];
             p.C = c.C;
             p.bias = c.bias;
             p.a_rows = c.a_rows;

@@ -160,8 +160,8 @@ private:
     struct SplitWeight {
         DeviceBuffer<float> fwd_hi, fwd_lo, rev_hi, rev_lo, full;
         int rows = 0, cols = 0;   // W is [rows = K of fwd][cols = N of fwd]
-        CUtensorMap map_fwd_hi, map_fwd_lo, map_rev_hi, map_rev_lo;   // [N][K] tensors, box [n_tile][32]
-        CUtensorMap wide_fwd_hi, wide_fwd_lo, wide_rev_hi, wide_rev_lo;   // the same with box [min(N, 128)][32]
+        // tensor maps of the four matrices, box [min(N, width)][32]; width 32, 64, 128 at index 0, 1, 2
+        CUtensorMap map_fwd_hi[3], map_fwd_lo[3], map_rev_hi[3], map_rev_lo[3];
     };
     SplitWeight s_h1_[4], s_a1_[4], s_h2_m1_;
     std::vector<SplitWeight> s_h2_skip_;

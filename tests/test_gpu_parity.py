@@ -502,7 +502,8 @@ def test_nve_energy_conservation(pkg, model_path):
 @pytest.mark.gpu
 @pytest.mark.parametrize("arch,copies", [("medium", (2, 1, 1)), ("medium", (4, 2, 2)), ("small", (4, 2, 1)), ("large", (2, 2, 1))])
 def test_parts_of_a_receiver_add_up(pkg, model_path, arch, copies):
-    """A receiver's edges are dealt to more blocks and warps the fewer receivers there are: a cell of 38 atoms (most parts)
+    """A receiver's edges are dealt to more blocks and warps, and the linears' column tiles get narrower, the fewer receivers
+    there are: a cell of 38 atoms (most parts)
     against the oracle, and its periodic copies (fewer parts, down to one) against the cell.  Bounds: those of the oracle
     comparison; the copies differ from the cell by the order of float sums alone."""
     from oracle import mace_numpy, neighbor
