@@ -9,7 +9,7 @@
 // Teams of kC / 64 warps share a receiver.  5,000 receivers, 500,000 list edges, 128 channels, this / the register form:
 // hidden 0e+1o 0.941 / 1.060 ms, 0e+1o+2e 2.16 / 2.57 ms (three launches).  Shapes tried for 0e+1o, (teams, blocks per SM,
 // edges): (2, 3, 2) 0.941, (4, 2, 1) 1.005, (4, 1, 2) 1.089; for 0e+1o+2e: (6, 1, 1) 2.157, (4, 1, 2) 2.153, (8, 1, 1) 2.23.
-// Now bound by latency at twelve warps per SM and by shared-memory reads.  The reproducible mode keeps the register form,
+// Now bound by the shared-memory data pipe (77 % of its wavefronts at twelve warps per SM).  The reproducible mode keeps the register form,
 // which leaves its records faster (1,080 receivers: 0.295 against 0.469 ms).
 //
 // Math and reference citations: see edge_kernels.cuh (layer 1 reverse).
