@@ -32,43 +32,48 @@ SHAPES = [("S0", 3, 0, 1, None), ("S1", 3, 1, 1, None),
           ("S2", 3, 2, 3, [[0, 3, 8, 13, 1, 4, 5, 9, 10, 14], [7, 2, 6, 11], [16, 12, 15]])]
 
 
-def reverse_path_lines(p, q, l, l1, l2, base):
+def reverse_path_lines(p, q, l, l1, l2, base, fed):
     """Straight-line gradient code of one path for one (edge, channel): q = index of the path's radial
     function in R[] / dR[], base = first row adjoint of the path in adj[].  With w_a = sum_b h_b adj_ab and
     s_b = sum_a y_a adj_ab the path contributes
       ang_a += R w_a   (angular part of the force),   hadj_b += R s_b   (source adjoint),
       radial += dR * sum_a y_a w_a,   and   sum_a y_a w_a = sum_b h_b s_b.
     The radial sum runs over the shorter index set, and R is folded into that set's vector first, so
-    that the other contraction accumulates straight into its target."""
+    that the other contraction accumulates straight into its target.  Rows outside `fed` have no coupling
+    term (their adjoint is zero: 12 of 88 for hidden 0e+1o) and are left out."""
     n1, n2 = 2 * l1 + 1, 2 * l2 + 1
     out = [f"    {{ /* path {p}: edge l={l1}, source l={l2} -> l={l} */"]
     out.append("      float yw = 0.0f;")
+
+    def rows(pairs):
+        return [(a, b, base + a * n2 + b) for a, b in pairs if base + a * n2 + b in fed]
+
+    def nested(terms):
+        expr = f"{terms[0][0]} * {terms[0][1]}"
+        for x, adj in terms[1:]:
+            expr = f"fmaf({x}, {adj}, {expr})"
+        return expr
+
     if n2 < n1:
         for b in range(n2):
             out.append(f"      const float rh{b} = R[{q}] * h[{l2 * l2 + b}];")
-        for a in range(n1):
-            for b in range(n2):
-                out.append(f"      ang[{l1 * l1 + a}] = fmaf(rh{b}, adj[{base + a * n2 + b}], ang[{l1 * l1 + a}]);")
+        for a, b, row in rows((a, b) for a in range(n1) for b in range(n2)):
+            out.append(f"      ang[{l1 * l1 + a}] = fmaf(rh{b}, adj[{row}], ang[{l1 * l1 + a}]);")
         for b in range(n2):
-            terms_ = [(f"y[{l1 * l1 + a}]", f"adj[{base + a * n2 + b}]") for a in range(n1)]
-            expr = f"{terms_[0][0]} * {terms_[0][1]}"
-            for yy, aa in terms_[1:]:
-                expr = f"fmaf({yy}, {aa}, {expr})"
-            out.append(f"      {{ const float s_ = {expr};")
-            out.append(f"        hadj[{l2 * l2 + b}] = fmaf(R[{q}], s_, hadj[{l2 * l2 + b}]); yw = fmaf(h[{l2 * l2 + b}], s_, yw); }}")
+            terms = [(f"y[{l1 * l1 + a}]", f"adj[{row}]") for a, _, row in rows((a, b) for a in range(n1))]
+            if terms:
+                out.append(f"      {{ const float s_ = {nested(terms)};")
+                out.append(f"        hadj[{l2 * l2 + b}] = fmaf(R[{q}], s_, hadj[{l2 * l2 + b}]); yw = fmaf(h[{l2 * l2 + b}], s_, yw); }}")
     else:
         for a in range(n1):
             out.append(f"      const float ry{a} = R[{q}] * y[{l1 * l1 + a}];")
         for a in range(n1):
-            terms_ = [(f"h[{l2 * l2 + b}]", f"adj[{base + a * n2 + b}]") for b in range(n2)]
-            expr = f"{terms_[0][0]} * {terms_[0][1]}"
-            for hh, aa in terms_[1:]:
-                expr = f"fmaf({hh}, {aa}, {expr})"
-            out.append(f"      {{ const float w = {expr};")
-            out.append(f"        ang[{l1 * l1 + a}] = fmaf(R[{q}], w, ang[{l1 * l1 + a}]); yw = fmaf(y[{l1 * l1 + a}], w, yw); }}")
-        for b in range(n2):
-            for a in range(n1):
-                out.append(f"      hadj[{l2 * l2 + b}] = fmaf(ry{a}, adj[{base + a * n2 + b}], hadj[{l2 * l2 + b}]);")
+            terms = [(f"h[{l2 * l2 + b}]", f"adj[{row}]") for _, b, row in rows((a, b) for b in range(n2))]
+            if terms:
+                out.append(f"      {{ const float w = {nested(terms)};")
+                out.append(f"        ang[{l1 * l1 + a}] = fmaf(R[{q}], w, ang[{l1 * l1 + a}]); yw = fmaf(y[{l1 * l1 + a}], w, yw); }}")
+        for a, b, row in rows((a, b) for b in range(n2) for a in range(n1)):
+            out.append(f"      hadj[{l2 * l2 + b}] = fmaf(ry{a}, adj[{row}], hadj[{l2 * l2 + b}]);")
     out.append(f"      radial = fmaf(dR[{q}], yw, radial);")
     out.append("    }")
     return out
@@ -276,11 +281,12 @@ def emit_shape(name, l_max, L_max, tables, groups=1, by_edge_l=None):
                 row = row_begin[p] + a * n2 + b
                 fwd.append(f"      acc[{row}] = fmaf(t{b}, y[{l1 * l1 + a}], acc[{row}]);")
         fwd.append("    }")
-        rev.extend(reverse_path_lines(p, p, l, l1, l2, row_begin[p]))
-    out.append(f"#define SXB_{name}_L1_FORWARD_BODY \\")
-    out.append(" \\\n".join(fwd))
-    out.append(f"#define SXB_{name}_L1_REVERSE_BODY \\")
-    out.append(" \\\n".join(rev))
+        rev.extend(reverse_path_lines(p, p, l, l1, l2, row_begin[p], set(tables["Phi1_lelm1lm2"])))
+    if groups == 1:      # shapes with path sets have no kernel that holds all rows in registers
+        out.append(f"#define SXB_{name}_L1_FORWARD_BODY \\")
+        out.append(" \\\n".join(fwd))
+        out.append(f"#define SXB_{name}_L1_REVERSE_BODY \\")
+        out.append(" \\\n".join(rev))
     if L_max > 0:
         out.append(f"#define SXB_{name}_L1_REVERSE_EDGES_BODY \\")
         out.append(" \\\n".join(reverse_edges_lines(paths, row_begin, set(tables["Phi1_lelm1lm2"]))))

@@ -1894,20 +1894,14 @@
       const float ry0 = R[1] * y[1]; \
       const float ry1 = R[1] * y[2]; \
       const float ry2 = R[1] * y[3]; \
-      { const float w = fmaf(h[3], adj[3], fmaf(h[2], adj[2], h[1] * adj[1])); \
+      { const float w = h[1] * adj[1]; \
         ang[1] = fmaf(R[1], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[3], adj[6], fmaf(h[2], adj[5], h[1] * adj[4])); \
+      { const float w = h[2] * adj[5]; \
         ang[2] = fmaf(R[1], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[3], adj[9], fmaf(h[2], adj[8], h[1] * adj[7])); \
+      { const float w = h[3] * adj[9]; \
         ang[3] = fmaf(R[1], w, ang[3]); yw = fmaf(y[3], w, yw); } \
       hadj[1] = fmaf(ry0, adj[1], hadj[1]); \
-      hadj[1] = fmaf(ry1, adj[4], hadj[1]); \
-      hadj[1] = fmaf(ry2, adj[7], hadj[1]); \
-      hadj[2] = fmaf(ry0, adj[2], hadj[2]); \
       hadj[2] = fmaf(ry1, adj[5], hadj[2]); \
-      hadj[2] = fmaf(ry2, adj[8], hadj[2]); \
-      hadj[3] = fmaf(ry0, adj[3], hadj[3]); \
-      hadj[3] = fmaf(ry1, adj[6], hadj[3]); \
       hadj[3] = fmaf(ry2, adj[9], hadj[3]); \
       radial = fmaf(dR[1], yw, radial); \
     } \
@@ -1937,25 +1931,21 @@
       const float rh1 = R[4] * h[2]; \
       const float rh2 = R[4] * h[3]; \
       ang[4] = fmaf(rh0, adj[16], ang[4]); \
-      ang[4] = fmaf(rh1, adj[17], ang[4]); \
       ang[4] = fmaf(rh2, adj[18], ang[4]); \
       ang[5] = fmaf(rh0, adj[19], ang[5]); \
       ang[5] = fmaf(rh1, adj[20], ang[5]); \
-      ang[5] = fmaf(rh2, adj[21], ang[5]); \
       ang[6] = fmaf(rh0, adj[22], ang[6]); \
       ang[6] = fmaf(rh1, adj[23], ang[6]); \
       ang[6] = fmaf(rh2, adj[24], ang[6]); \
-      ang[7] = fmaf(rh0, adj[25], ang[7]); \
       ang[7] = fmaf(rh1, adj[26], ang[7]); \
       ang[7] = fmaf(rh2, adj[27], ang[7]); \
       ang[8] = fmaf(rh0, adj[28], ang[8]); \
-      ang[8] = fmaf(rh1, adj[29], ang[8]); \
       ang[8] = fmaf(rh2, adj[30], ang[8]); \
-      { const float s_ = fmaf(y[8], adj[28], fmaf(y[7], adj[25], fmaf(y[6], adj[22], fmaf(y[5], adj[19], y[4] * adj[16])))); \
+      { const float s_ = fmaf(y[8], adj[28], fmaf(y[6], adj[22], fmaf(y[5], adj[19], y[4] * adj[16]))); \
         hadj[1] = fmaf(R[4], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[29], fmaf(y[7], adj[26], fmaf(y[6], adj[23], fmaf(y[5], adj[20], y[4] * adj[17])))); \
+      { const float s_ = fmaf(y[7], adj[26], fmaf(y[6], adj[23], y[5] * adj[20])); \
         hadj[2] = fmaf(R[4], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[30], fmaf(y[7], adj[27], fmaf(y[6], adj[24], fmaf(y[5], adj[21], y[4] * adj[18])))); \
+      { const float s_ = fmaf(y[8], adj[30], fmaf(y[7], adj[27], fmaf(y[6], adj[24], y[4] * adj[18]))); \
         hadj[3] = fmaf(R[4], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
       radial = fmaf(dR[4], yw, radial); \
     } \
@@ -1999,7 +1989,6 @@
       const float rh1 = R[7] * h[2]; \
       const float rh2 = R[7] * h[3]; \
       ang[9] = fmaf(rh0, adj[45], ang[9]); \
-      ang[9] = fmaf(rh1, adj[46], ang[9]); \
       ang[9] = fmaf(rh2, adj[47], ang[9]); \
       ang[10] = fmaf(rh0, adj[48], ang[10]); \
       ang[10] = fmaf(rh1, adj[49], ang[10]); \
@@ -2017,11 +2006,10 @@
       ang[14] = fmaf(rh1, adj[61], ang[14]); \
       ang[14] = fmaf(rh2, adj[62], ang[14]); \
       ang[15] = fmaf(rh0, adj[63], ang[15]); \
-      ang[15] = fmaf(rh1, adj[64], ang[15]); \
       ang[15] = fmaf(rh2, adj[65], ang[15]); \
       { const float s_ = fmaf(y[15], adj[63], fmaf(y[14], adj[60], fmaf(y[13], adj[57], fmaf(y[12], adj[54], fmaf(y[11], adj[51], fmaf(y[10], adj[48], y[9] * adj[45])))))); \
         hadj[1] = fmaf(R[7], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[64], fmaf(y[14], adj[61], fmaf(y[13], adj[58], fmaf(y[12], adj[55], fmaf(y[11], adj[52], fmaf(y[10], adj[49], y[9] * adj[46])))))); \
+      { const float s_ = fmaf(y[14], adj[61], fmaf(y[13], adj[58], fmaf(y[12], adj[55], fmaf(y[11], adj[52], y[10] * adj[49])))); \
         hadj[2] = fmaf(R[7], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
       { const float s_ = fmaf(y[15], adj[65], fmaf(y[14], adj[62], fmaf(y[13], adj[59], fmaf(y[12], adj[56], fmaf(y[11], adj[53], fmaf(y[10], adj[50], y[9] * adj[47])))))); \
         hadj[3] = fmaf(R[7], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
@@ -4145,794 +4133,6 @@
       { unsigned long long v; v = f2_mul(W(14), adj[0]); g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
       { unsigned long long v; v = f2_mul(W(15), adj[0]); g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
       { unsigned long long v; v = f2_mul(W(16), adj[0]); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
-#define SXB_S2_L1_FORWARD_BODY \
-    { /* path 0: edge l=0, source l=0 -> l=0 */ \
-      const float t0 = R[0] * h[0]; \
-      acc[0] = fmaf(t0, y[0], acc[0]); \
-    } \
-    { /* path 1: edge l=1, source l=1 -> l=0 */ \
-      const float t0 = R[1] * h[1]; \
-      const float t1 = R[1] * h[2]; \
-      const float t2 = R[1] * h[3]; \
-      acc[1] = fmaf(t0, y[1], acc[1]); \
-      acc[2] = fmaf(t1, y[1], acc[2]); \
-      acc[3] = fmaf(t2, y[1], acc[3]); \
-      acc[4] = fmaf(t0, y[2], acc[4]); \
-      acc[5] = fmaf(t1, y[2], acc[5]); \
-      acc[6] = fmaf(t2, y[2], acc[6]); \
-      acc[7] = fmaf(t0, y[3], acc[7]); \
-      acc[8] = fmaf(t1, y[3], acc[8]); \
-      acc[9] = fmaf(t2, y[3], acc[9]); \
-    } \
-    { /* path 2: edge l=2, source l=2 -> l=0 */ \
-      const float t0 = R[2] * h[4]; \
-      const float t1 = R[2] * h[5]; \
-      const float t2 = R[2] * h[6]; \
-      const float t3 = R[2] * h[7]; \
-      const float t4 = R[2] * h[8]; \
-      acc[10] = fmaf(t0, y[4], acc[10]); \
-      acc[11] = fmaf(t1, y[4], acc[11]); \
-      acc[12] = fmaf(t2, y[4], acc[12]); \
-      acc[13] = fmaf(t3, y[4], acc[13]); \
-      acc[14] = fmaf(t4, y[4], acc[14]); \
-      acc[15] = fmaf(t0, y[5], acc[15]); \
-      acc[16] = fmaf(t1, y[5], acc[16]); \
-      acc[17] = fmaf(t2, y[5], acc[17]); \
-      acc[18] = fmaf(t3, y[5], acc[18]); \
-      acc[19] = fmaf(t4, y[5], acc[19]); \
-      acc[20] = fmaf(t0, y[6], acc[20]); \
-      acc[21] = fmaf(t1, y[6], acc[21]); \
-      acc[22] = fmaf(t2, y[6], acc[22]); \
-      acc[23] = fmaf(t3, y[6], acc[23]); \
-      acc[24] = fmaf(t4, y[6], acc[24]); \
-      acc[25] = fmaf(t0, y[7], acc[25]); \
-      acc[26] = fmaf(t1, y[7], acc[26]); \
-      acc[27] = fmaf(t2, y[7], acc[27]); \
-      acc[28] = fmaf(t3, y[7], acc[28]); \
-      acc[29] = fmaf(t4, y[7], acc[29]); \
-      acc[30] = fmaf(t0, y[8], acc[30]); \
-      acc[31] = fmaf(t1, y[8], acc[31]); \
-      acc[32] = fmaf(t2, y[8], acc[32]); \
-      acc[33] = fmaf(t3, y[8], acc[33]); \
-      acc[34] = fmaf(t4, y[8], acc[34]); \
-    } \
-    { /* path 3: edge l=1, source l=0 -> l=1 */ \
-      const float t0 = R[3] * h[0]; \
-      acc[35] = fmaf(t0, y[1], acc[35]); \
-      acc[36] = fmaf(t0, y[2], acc[36]); \
-      acc[37] = fmaf(t0, y[3], acc[37]); \
-    } \
-    { /* path 4: edge l=0, source l=1 -> l=1 */ \
-      const float t0 = R[4] * h[1]; \
-      const float t1 = R[4] * h[2]; \
-      const float t2 = R[4] * h[3]; \
-      acc[38] = fmaf(t0, y[0], acc[38]); \
-      acc[39] = fmaf(t1, y[0], acc[39]); \
-      acc[40] = fmaf(t2, y[0], acc[40]); \
-    } \
-    { /* path 5: edge l=2, source l=1 -> l=1 */ \
-      const float t0 = R[5] * h[1]; \
-      const float t1 = R[5] * h[2]; \
-      const float t2 = R[5] * h[3]; \
-      acc[41] = fmaf(t0, y[4], acc[41]); \
-      acc[42] = fmaf(t1, y[4], acc[42]); \
-      acc[43] = fmaf(t2, y[4], acc[43]); \
-      acc[44] = fmaf(t0, y[5], acc[44]); \
-      acc[45] = fmaf(t1, y[5], acc[45]); \
-      acc[46] = fmaf(t2, y[5], acc[46]); \
-      acc[47] = fmaf(t0, y[6], acc[47]); \
-      acc[48] = fmaf(t1, y[6], acc[48]); \
-      acc[49] = fmaf(t2, y[6], acc[49]); \
-      acc[50] = fmaf(t0, y[7], acc[50]); \
-      acc[51] = fmaf(t1, y[7], acc[51]); \
-      acc[52] = fmaf(t2, y[7], acc[52]); \
-      acc[53] = fmaf(t0, y[8], acc[53]); \
-      acc[54] = fmaf(t1, y[8], acc[54]); \
-      acc[55] = fmaf(t2, y[8], acc[55]); \
-    } \
-    { /* path 6: edge l=1, source l=2 -> l=1 */ \
-      const float t0 = R[6] * h[4]; \
-      const float t1 = R[6] * h[5]; \
-      const float t2 = R[6] * h[6]; \
-      const float t3 = R[6] * h[7]; \
-      const float t4 = R[6] * h[8]; \
-      acc[56] = fmaf(t0, y[1], acc[56]); \
-      acc[57] = fmaf(t1, y[1], acc[57]); \
-      acc[58] = fmaf(t2, y[1], acc[58]); \
-      acc[59] = fmaf(t3, y[1], acc[59]); \
-      acc[60] = fmaf(t4, y[1], acc[60]); \
-      acc[61] = fmaf(t0, y[2], acc[61]); \
-      acc[62] = fmaf(t1, y[2], acc[62]); \
-      acc[63] = fmaf(t2, y[2], acc[63]); \
-      acc[64] = fmaf(t3, y[2], acc[64]); \
-      acc[65] = fmaf(t4, y[2], acc[65]); \
-      acc[66] = fmaf(t0, y[3], acc[66]); \
-      acc[67] = fmaf(t1, y[3], acc[67]); \
-      acc[68] = fmaf(t2, y[3], acc[68]); \
-      acc[69] = fmaf(t3, y[3], acc[69]); \
-      acc[70] = fmaf(t4, y[3], acc[70]); \
-    } \
-    { /* path 7: edge l=3, source l=2 -> l=1 */ \
-      const float t0 = R[7] * h[4]; \
-      const float t1 = R[7] * h[5]; \
-      const float t2 = R[7] * h[6]; \
-      const float t3 = R[7] * h[7]; \
-      const float t4 = R[7] * h[8]; \
-      acc[71] = fmaf(t0, y[9], acc[71]); \
-      acc[72] = fmaf(t1, y[9], acc[72]); \
-      acc[73] = fmaf(t2, y[9], acc[73]); \
-      acc[74] = fmaf(t3, y[9], acc[74]); \
-      acc[75] = fmaf(t4, y[9], acc[75]); \
-      acc[76] = fmaf(t0, y[10], acc[76]); \
-      acc[77] = fmaf(t1, y[10], acc[77]); \
-      acc[78] = fmaf(t2, y[10], acc[78]); \
-      acc[79] = fmaf(t3, y[10], acc[79]); \
-      acc[80] = fmaf(t4, y[10], acc[80]); \
-      acc[81] = fmaf(t0, y[11], acc[81]); \
-      acc[82] = fmaf(t1, y[11], acc[82]); \
-      acc[83] = fmaf(t2, y[11], acc[83]); \
-      acc[84] = fmaf(t3, y[11], acc[84]); \
-      acc[85] = fmaf(t4, y[11], acc[85]); \
-      acc[86] = fmaf(t0, y[12], acc[86]); \
-      acc[87] = fmaf(t1, y[12], acc[87]); \
-      acc[88] = fmaf(t2, y[12], acc[88]); \
-      acc[89] = fmaf(t3, y[12], acc[89]); \
-      acc[90] = fmaf(t4, y[12], acc[90]); \
-      acc[91] = fmaf(t0, y[13], acc[91]); \
-      acc[92] = fmaf(t1, y[13], acc[92]); \
-      acc[93] = fmaf(t2, y[13], acc[93]); \
-      acc[94] = fmaf(t3, y[13], acc[94]); \
-      acc[95] = fmaf(t4, y[13], acc[95]); \
-      acc[96] = fmaf(t0, y[14], acc[96]); \
-      acc[97] = fmaf(t1, y[14], acc[97]); \
-      acc[98] = fmaf(t2, y[14], acc[98]); \
-      acc[99] = fmaf(t3, y[14], acc[99]); \
-      acc[100] = fmaf(t4, y[14], acc[100]); \
-      acc[101] = fmaf(t0, y[15], acc[101]); \
-      acc[102] = fmaf(t1, y[15], acc[102]); \
-      acc[103] = fmaf(t2, y[15], acc[103]); \
-      acc[104] = fmaf(t3, y[15], acc[104]); \
-      acc[105] = fmaf(t4, y[15], acc[105]); \
-    } \
-    { /* path 8: edge l=2, source l=0 -> l=2 */ \
-      const float t0 = R[8] * h[0]; \
-      acc[106] = fmaf(t0, y[4], acc[106]); \
-      acc[107] = fmaf(t0, y[5], acc[107]); \
-      acc[108] = fmaf(t0, y[6], acc[108]); \
-      acc[109] = fmaf(t0, y[7], acc[109]); \
-      acc[110] = fmaf(t0, y[8], acc[110]); \
-    } \
-    { /* path 9: edge l=1, source l=1 -> l=2 */ \
-      const float t0 = R[9] * h[1]; \
-      const float t1 = R[9] * h[2]; \
-      const float t2 = R[9] * h[3]; \
-      acc[111] = fmaf(t0, y[1], acc[111]); \
-      acc[112] = fmaf(t1, y[1], acc[112]); \
-      acc[113] = fmaf(t2, y[1], acc[113]); \
-      acc[114] = fmaf(t0, y[2], acc[114]); \
-      acc[115] = fmaf(t1, y[2], acc[115]); \
-      acc[116] = fmaf(t2, y[2], acc[116]); \
-      acc[117] = fmaf(t0, y[3], acc[117]); \
-      acc[118] = fmaf(t1, y[3], acc[118]); \
-      acc[119] = fmaf(t2, y[3], acc[119]); \
-    } \
-    { /* path 10: edge l=3, source l=1 -> l=2 */ \
-      const float t0 = R[10] * h[1]; \
-      const float t1 = R[10] * h[2]; \
-      const float t2 = R[10] * h[3]; \
-      acc[120] = fmaf(t0, y[9], acc[120]); \
-      acc[121] = fmaf(t1, y[9], acc[121]); \
-      acc[122] = fmaf(t2, y[9], acc[122]); \
-      acc[123] = fmaf(t0, y[10], acc[123]); \
-      acc[124] = fmaf(t1, y[10], acc[124]); \
-      acc[125] = fmaf(t2, y[10], acc[125]); \
-      acc[126] = fmaf(t0, y[11], acc[126]); \
-      acc[127] = fmaf(t1, y[11], acc[127]); \
-      acc[128] = fmaf(t2, y[11], acc[128]); \
-      acc[129] = fmaf(t0, y[12], acc[129]); \
-      acc[130] = fmaf(t1, y[12], acc[130]); \
-      acc[131] = fmaf(t2, y[12], acc[131]); \
-      acc[132] = fmaf(t0, y[13], acc[132]); \
-      acc[133] = fmaf(t1, y[13], acc[133]); \
-      acc[134] = fmaf(t2, y[13], acc[134]); \
-      acc[135] = fmaf(t0, y[14], acc[135]); \
-      acc[136] = fmaf(t1, y[14], acc[136]); \
-      acc[137] = fmaf(t2, y[14], acc[137]); \
-      acc[138] = fmaf(t0, y[15], acc[138]); \
-      acc[139] = fmaf(t1, y[15], acc[139]); \
-      acc[140] = fmaf(t2, y[15], acc[140]); \
-    } \
-    { /* path 11: edge l=0, source l=2 -> l=2 */ \
-      const float t0 = R[11] * h[4]; \
-      const float t1 = R[11] * h[5]; \
-      const float t2 = R[11] * h[6]; \
-      const float t3 = R[11] * h[7]; \
-      const float t4 = R[11] * h[8]; \
-      acc[141] = fmaf(t0, y[0], acc[141]); \
-      acc[142] = fmaf(t1, y[0], acc[142]); \
-      acc[143] = fmaf(t2, y[0], acc[143]); \
-      acc[144] = fmaf(t3, y[0], acc[144]); \
-      acc[145] = fmaf(t4, y[0], acc[145]); \
-    } \
-    { /* path 12: edge l=2, source l=2 -> l=2 */ \
-      const float t0 = R[12] * h[4]; \
-      const float t1 = R[12] * h[5]; \
-      const float t2 = R[12] * h[6]; \
-      const float t3 = R[12] * h[7]; \
-      const float t4 = R[12] * h[8]; \
-      acc[146] = fmaf(t0, y[4], acc[146]); \
-      acc[147] = fmaf(t1, y[4], acc[147]); \
-      acc[148] = fmaf(t2, y[4], acc[148]); \
-      acc[149] = fmaf(t3, y[4], acc[149]); \
-      acc[150] = fmaf(t4, y[4], acc[150]); \
-      acc[151] = fmaf(t0, y[5], acc[151]); \
-      acc[152] = fmaf(t1, y[5], acc[152]); \
-      acc[153] = fmaf(t2, y[5], acc[153]); \
-      acc[154] = fmaf(t3, y[5], acc[154]); \
-      acc[155] = fmaf(t4, y[5], acc[155]); \
-      acc[156] = fmaf(t0, y[6], acc[156]); \
-      acc[157] = fmaf(t1, y[6], acc[157]); \
-      acc[158] = fmaf(t2, y[6], acc[158]); \
-      acc[159] = fmaf(t3, y[6], acc[159]); \
-      acc[160] = fmaf(t4, y[6], acc[160]); \
-      acc[161] = fmaf(t0, y[7], acc[161]); \
-      acc[162] = fmaf(t1, y[7], acc[162]); \
-      acc[163] = fmaf(t2, y[7], acc[163]); \
-      acc[164] = fmaf(t3, y[7], acc[164]); \
-      acc[165] = fmaf(t4, y[7], acc[165]); \
-      acc[166] = fmaf(t0, y[8], acc[166]); \
-      acc[167] = fmaf(t1, y[8], acc[167]); \
-      acc[168] = fmaf(t2, y[8], acc[168]); \
-      acc[169] = fmaf(t3, y[8], acc[169]); \
-      acc[170] = fmaf(t4, y[8], acc[170]); \
-    } \
-    { /* path 13: edge l=3, source l=0 -> l=3 */ \
-      const float t0 = R[13] * h[0]; \
-      acc[171] = fmaf(t0, y[9], acc[171]); \
-      acc[172] = fmaf(t0, y[10], acc[172]); \
-      acc[173] = fmaf(t0, y[11], acc[173]); \
-      acc[174] = fmaf(t0, y[12], acc[174]); \
-      acc[175] = fmaf(t0, y[13], acc[175]); \
-      acc[176] = fmaf(t0, y[14], acc[176]); \
-      acc[177] = fmaf(t0, y[15], acc[177]); \
-    } \
-    { /* path 14: edge l=2, source l=1 -> l=3 */ \
-      const float t0 = R[14] * h[1]; \
-      const float t1 = R[14] * h[2]; \
-      const float t2 = R[14] * h[3]; \
-      acc[178] = fmaf(t0, y[4], acc[178]); \
-      acc[179] = fmaf(t1, y[4], acc[179]); \
-      acc[180] = fmaf(t2, y[4], acc[180]); \
-      acc[181] = fmaf(t0, y[5], acc[181]); \
-      acc[182] = fmaf(t1, y[5], acc[182]); \
-      acc[183] = fmaf(t2, y[5], acc[183]); \
-      acc[184] = fmaf(t0, y[6], acc[184]); \
-      acc[185] = fmaf(t1, y[6], acc[185]); \
-      acc[186] = fmaf(t2, y[6], acc[186]); \
-      acc[187] = fmaf(t0, y[7], acc[187]); \
-      acc[188] = fmaf(t1, y[7], acc[188]); \
-      acc[189] = fmaf(t2, y[7], acc[189]); \
-      acc[190] = fmaf(t0, y[8], acc[190]); \
-      acc[191] = fmaf(t1, y[8], acc[191]); \
-      acc[192] = fmaf(t2, y[8], acc[192]); \
-    } \
-    { /* path 15: edge l=1, source l=2 -> l=3 */ \
-      const float t0 = R[15] * h[4]; \
-      const float t1 = R[15] * h[5]; \
-      const float t2 = R[15] * h[6]; \
-      const float t3 = R[15] * h[7]; \
-      const float t4 = R[15] * h[8]; \
-      acc[193] = fmaf(t0, y[1], acc[193]); \
-      acc[194] = fmaf(t1, y[1], acc[194]); \
-      acc[195] = fmaf(t2, y[1], acc[195]); \
-      acc[196] = fmaf(t3, y[1], acc[196]); \
-      acc[197] = fmaf(t4, y[1], acc[197]); \
-      acc[198] = fmaf(t0, y[2], acc[198]); \
-      acc[199] = fmaf(t1, y[2], acc[199]); \
-      acc[200] = fmaf(t2, y[2], acc[200]); \
-      acc[201] = fmaf(t3, y[2], acc[201]); \
-      acc[202] = fmaf(t4, y[2], acc[202]); \
-      acc[203] = fmaf(t0, y[3], acc[203]); \
-      acc[204] = fmaf(t1, y[3], acc[204]); \
-      acc[205] = fmaf(t2, y[3], acc[205]); \
-      acc[206] = fmaf(t3, y[3], acc[206]); \
-      acc[207] = fmaf(t4, y[3], acc[207]); \
-    } \
-    { /* path 16: edge l=3, source l=2 -> l=3 */ \
-      const float t0 = R[16] * h[4]; \
-      const float t1 = R[16] * h[5]; \
-      const float t2 = R[16] * h[6]; \
-      const float t3 = R[16] * h[7]; \
-      const float t4 = R[16] * h[8]; \
-      acc[208] = fmaf(t0, y[9], acc[208]); \
-      acc[209] = fmaf(t1, y[9], acc[209]); \
-      acc[210] = fmaf(t2, y[9], acc[210]); \
-      acc[211] = fmaf(t3, y[9], acc[211]); \
-      acc[212] = fmaf(t4, y[9], acc[212]); \
-      acc[213] = fmaf(t0, y[10], acc[213]); \
-      acc[214] = fmaf(t1, y[10], acc[214]); \
-      acc[215] = fmaf(t2, y[10], acc[215]); \
-      acc[216] = fmaf(t3, y[10], acc[216]); \
-      acc[217] = fmaf(t4, y[10], acc[217]); \
-      acc[218] = fmaf(t0, y[11], acc[218]); \
-      acc[219] = fmaf(t1, y[11], acc[219]); \
-      acc[220] = fmaf(t2, y[11], acc[220]); \
-      acc[221] = fmaf(t3, y[11], acc[221]); \
-      acc[222] = fmaf(t4, y[11], acc[222]); \
-      acc[223] = fmaf(t0, y[12], acc[223]); \
-      acc[224] = fmaf(t1, y[12], acc[224]); \
-      acc[225] = fmaf(t2, y[12], acc[225]); \
-      acc[226] = fmaf(t3, y[12], acc[226]); \
-      acc[227] = fmaf(t4, y[12], acc[227]); \
-      acc[228] = fmaf(t0, y[13], acc[228]); \
-      acc[229] = fmaf(t1, y[13], acc[229]); \
-      acc[230] = fmaf(t2, y[13], acc[230]); \
-      acc[231] = fmaf(t3, y[13], acc[231]); \
-      acc[232] = fmaf(t4, y[13], acc[232]); \
-      acc[233] = fmaf(t0, y[14], acc[233]); \
-      acc[234] = fmaf(t1, y[14], acc[234]); \
-      acc[235] = fmaf(t2, y[14], acc[235]); \
-      acc[236] = fmaf(t3, y[14], acc[236]); \
-      acc[237] = fmaf(t4, y[14], acc[237]); \
-      acc[238] = fmaf(t0, y[15], acc[238]); \
-      acc[239] = fmaf(t1, y[15], acc[239]); \
-      acc[240] = fmaf(t2, y[15], acc[240]); \
-      acc[241] = fmaf(t3, y[15], acc[241]); \
-      acc[242] = fmaf(t4, y[15], acc[242]); \
-    }
-#define SXB_S2_L1_REVERSE_BODY \
-    { /* path 0: edge l=0, source l=0 -> l=0 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[0] * y[0]; \
-      { const float w = h[0] * adj[0]; \
-        ang[0] = fmaf(R[0], w, ang[0]); yw = fmaf(y[0], w, yw); } \
-      hadj[0] = fmaf(ry0, adj[0], hadj[0]); \
-      radial = fmaf(dR[0], yw, radial); \
-    } \
-    { /* path 1: edge l=1, source l=1 -> l=0 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[1] * y[1]; \
-      const float ry1 = R[1] * y[2]; \
-      const float ry2 = R[1] * y[3]; \
-      { const float w = fmaf(h[3], adj[3], fmaf(h[2], adj[2], h[1] * adj[1])); \
-        ang[1] = fmaf(R[1], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[3], adj[6], fmaf(h[2], adj[5], h[1] * adj[4])); \
-        ang[2] = fmaf(R[1], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[3], adj[9], fmaf(h[2], adj[8], h[1] * adj[7])); \
-        ang[3] = fmaf(R[1], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[1] = fmaf(ry0, adj[1], hadj[1]); \
-      hadj[1] = fmaf(ry1, adj[4], hadj[1]); \
-      hadj[1] = fmaf(ry2, adj[7], hadj[1]); \
-      hadj[2] = fmaf(ry0, adj[2], hadj[2]); \
-      hadj[2] = fmaf(ry1, adj[5], hadj[2]); \
-      hadj[2] = fmaf(ry2, adj[8], hadj[2]); \
-      hadj[3] = fmaf(ry0, adj[3], hadj[3]); \
-      hadj[3] = fmaf(ry1, adj[6], hadj[3]); \
-      hadj[3] = fmaf(ry2, adj[9], hadj[3]); \
-      radial = fmaf(dR[1], yw, radial); \
-    } \
-    { /* path 2: edge l=2, source l=2 -> l=0 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[2] * y[4]; \
-      const float ry1 = R[2] * y[5]; \
-      const float ry2 = R[2] * y[6]; \
-      const float ry3 = R[2] * y[7]; \
-      const float ry4 = R[2] * y[8]; \
-      { const float w = fmaf(h[8], adj[14], fmaf(h[7], adj[13], fmaf(h[6], adj[12], fmaf(h[5], adj[11], h[4] * adj[10])))); \
-        ang[4] = fmaf(R[2], w, ang[4]); yw = fmaf(y[4], w, yw); } \
-      { const float w = fmaf(h[8], adj[19], fmaf(h[7], adj[18], fmaf(h[6], adj[17], fmaf(h[5], adj[16], h[4] * adj[15])))); \
-        ang[5] = fmaf(R[2], w, ang[5]); yw = fmaf(y[5], w, yw); } \
-      { const float w = fmaf(h[8], adj[24], fmaf(h[7], adj[23], fmaf(h[6], adj[22], fmaf(h[5], adj[21], h[4] * adj[20])))); \
-        ang[6] = fmaf(R[2], w, ang[6]); yw = fmaf(y[6], w, yw); } \
-      { const float w = fmaf(h[8], adj[29], fmaf(h[7], adj[28], fmaf(h[6], adj[27], fmaf(h[5], adj[26], h[4] * adj[25])))); \
-        ang[7] = fmaf(R[2], w, ang[7]); yw = fmaf(y[7], w, yw); } \
-      { const float w = fmaf(h[8], adj[34], fmaf(h[7], adj[33], fmaf(h[6], adj[32], fmaf(h[5], adj[31], h[4] * adj[30])))); \
-        ang[8] = fmaf(R[2], w, ang[8]); yw = fmaf(y[8], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[10], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[15], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[20], hadj[4]); \
-      hadj[4] = fmaf(ry3, adj[25], hadj[4]); \
-      hadj[4] = fmaf(ry4, adj[30], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[11], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[16], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[21], hadj[5]); \
-      hadj[5] = fmaf(ry3, adj[26], hadj[5]); \
-      hadj[5] = fmaf(ry4, adj[31], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[12], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[17], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[22], hadj[6]); \
-      hadj[6] = fmaf(ry3, adj[27], hadj[6]); \
-      hadj[6] = fmaf(ry4, adj[32], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[13], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[18], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[23], hadj[7]); \
-      hadj[7] = fmaf(ry3, adj[28], hadj[7]); \
-      hadj[7] = fmaf(ry4, adj[33], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[14], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[19], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[24], hadj[8]); \
-      hadj[8] = fmaf(ry3, adj[29], hadj[8]); \
-      hadj[8] = fmaf(ry4, adj[34], hadj[8]); \
-      radial = fmaf(dR[2], yw, radial); \
-    } \
-    { /* path 3: edge l=1, source l=0 -> l=1 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[3] * h[0]; \
-      ang[1] = fmaf(rh0, adj[35], ang[1]); \
-      ang[2] = fmaf(rh0, adj[36], ang[2]); \
-      ang[3] = fmaf(rh0, adj[37], ang[3]); \
-      { const float s_ = fmaf(y[3], adj[37], fmaf(y[2], adj[36], y[1] * adj[35])); \
-        hadj[0] = fmaf(R[3], s_, hadj[0]); yw = fmaf(h[0], s_, yw); } \
-      radial = fmaf(dR[3], yw, radial); \
-    } \
-    { /* path 4: edge l=0, source l=1 -> l=1 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[4] * y[0]; \
-      { const float w = fmaf(h[3], adj[40], fmaf(h[2], adj[39], h[1] * adj[38])); \
-        ang[0] = fmaf(R[4], w, ang[0]); yw = fmaf(y[0], w, yw); } \
-      hadj[1] = fmaf(ry0, adj[38], hadj[1]); \
-      hadj[2] = fmaf(ry0, adj[39], hadj[2]); \
-      hadj[3] = fmaf(ry0, adj[40], hadj[3]); \
-      radial = fmaf(dR[4], yw, radial); \
-    } \
-    { /* path 5: edge l=2, source l=1 -> l=1 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[5] * h[1]; \
-      const float rh1 = R[5] * h[2]; \
-      const float rh2 = R[5] * h[3]; \
-      ang[4] = fmaf(rh0, adj[41], ang[4]); \
-      ang[4] = fmaf(rh1, adj[42], ang[4]); \
-      ang[4] = fmaf(rh2, adj[43], ang[4]); \
-      ang[5] = fmaf(rh0, adj[44], ang[5]); \
-      ang[5] = fmaf(rh1, adj[45], ang[5]); \
-      ang[5] = fmaf(rh2, adj[46], ang[5]); \
-      ang[6] = fmaf(rh0, adj[47], ang[6]); \
-      ang[6] = fmaf(rh1, adj[48], ang[6]); \
-      ang[6] = fmaf(rh2, adj[49], ang[6]); \
-      ang[7] = fmaf(rh0, adj[50], ang[7]); \
-      ang[7] = fmaf(rh1, adj[51], ang[7]); \
-      ang[7] = fmaf(rh2, adj[52], ang[7]); \
-      ang[8] = fmaf(rh0, adj[53], ang[8]); \
-      ang[8] = fmaf(rh1, adj[54], ang[8]); \
-      ang[8] = fmaf(rh2, adj[55], ang[8]); \
-      { const float s_ = fmaf(y[8], adj[53], fmaf(y[7], adj[50], fmaf(y[6], adj[47], fmaf(y[5], adj[44], y[4] * adj[41])))); \
-        hadj[1] = fmaf(R[5], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[54], fmaf(y[7], adj[51], fmaf(y[6], adj[48], fmaf(y[5], adj[45], y[4] * adj[42])))); \
-        hadj[2] = fmaf(R[5], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[55], fmaf(y[7], adj[52], fmaf(y[6], adj[49], fmaf(y[5], adj[46], y[4] * adj[43])))); \
-        hadj[3] = fmaf(R[5], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
-      radial = fmaf(dR[5], yw, radial); \
-    } \
-    { /* path 6: edge l=1, source l=2 -> l=1 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[6] * y[1]; \
-      const float ry1 = R[6] * y[2]; \
-      const float ry2 = R[6] * y[3]; \
-      { const float w = fmaf(h[8], adj[60], fmaf(h[7], adj[59], fmaf(h[6], adj[58], fmaf(h[5], adj[57], h[4] * adj[56])))); \
-        ang[1] = fmaf(R[6], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[8], adj[65], fmaf(h[7], adj[64], fmaf(h[6], adj[63], fmaf(h[5], adj[62], h[4] * adj[61])))); \
-        ang[2] = fmaf(R[6], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[8], adj[70], fmaf(h[7], adj[69], fmaf(h[6], adj[68], fmaf(h[5], adj[67], h[4] * adj[66])))); \
-        ang[3] = fmaf(R[6], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[56], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[61], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[66], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[57], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[62], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[67], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[58], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[63], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[68], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[59], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[64], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[69], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[60], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[65], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[70], hadj[8]); \
-      radial = fmaf(dR[6], yw, radial); \
-    } \
-    { /* path 7: edge l=3, source l=2 -> l=1 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[7] * h[4]; \
-      const float rh1 = R[7] * h[5]; \
-      const float rh2 = R[7] * h[6]; \
-      const float rh3 = R[7] * h[7]; \
-      const float rh4 = R[7] * h[8]; \
-      ang[9] = fmaf(rh0, adj[71], ang[9]); \
-      ang[9] = fmaf(rh1, adj[72], ang[9]); \
-      ang[9] = fmaf(rh2, adj[73], ang[9]); \
-      ang[9] = fmaf(rh3, adj[74], ang[9]); \
-      ang[9] = fmaf(rh4, adj[75], ang[9]); \
-      ang[10] = fmaf(rh0, adj[76], ang[10]); \
-      ang[10] = fmaf(rh1, adj[77], ang[10]); \
-      ang[10] = fmaf(rh2, adj[78], ang[10]); \
-      ang[10] = fmaf(rh3, adj[79], ang[10]); \
-      ang[10] = fmaf(rh4, adj[80], ang[10]); \
-      ang[11] = fmaf(rh0, adj[81], ang[11]); \
-      ang[11] = fmaf(rh1, adj[82], ang[11]); \
-      ang[11] = fmaf(rh2, adj[83], ang[11]); \
-      ang[11] = fmaf(rh3, adj[84], ang[11]); \
-      ang[11] = fmaf(rh4, adj[85], ang[11]); \
-      ang[12] = fmaf(rh0, adj[86], ang[12]); \
-      ang[12] = fmaf(rh1, adj[87], ang[12]); \
-      ang[12] = fmaf(rh2, adj[88], ang[12]); \
-      ang[12] = fmaf(rh3, adj[89], ang[12]); \
-      ang[12] = fmaf(rh4, adj[90], ang[12]); \
-      ang[13] = fmaf(rh0, adj[91], ang[13]); \
-      ang[13] = fmaf(rh1, adj[92], ang[13]); \
-      ang[13] = fmaf(rh2, adj[93], ang[13]); \
-      ang[13] = fmaf(rh3, adj[94], ang[13]); \
-      ang[13] = fmaf(rh4, adj[95], ang[13]); \
-      ang[14] = fmaf(rh0, adj[96], ang[14]); \
-      ang[14] = fmaf(rh1, adj[97], ang[14]); \
-      ang[14] = fmaf(rh2, adj[98], ang[14]); \
-      ang[14] = fmaf(rh3, adj[99], ang[14]); \
-      ang[14] = fmaf(rh4, adj[100], ang[14]); \
-      ang[15] = fmaf(rh0, adj[101], ang[15]); \
-      ang[15] = fmaf(rh1, adj[102], ang[15]); \
-      ang[15] = fmaf(rh2, adj[103], ang[15]); \
-      ang[15] = fmaf(rh3, adj[104], ang[15]); \
-      ang[15] = fmaf(rh4, adj[105], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[101], fmaf(y[14], adj[96], fmaf(y[13], adj[91], fmaf(y[12], adj[86], fmaf(y[11], adj[81], fmaf(y[10], adj[76], y[9] * adj[71])))))); \
-        hadj[4] = fmaf(R[7], s_, hadj[4]); yw = fmaf(h[4], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[102], fmaf(y[14], adj[97], fmaf(y[13], adj[92], fmaf(y[12], adj[87], fmaf(y[11], adj[82], fmaf(y[10], adj[77], y[9] * adj[72])))))); \
-        hadj[5] = fmaf(R[7], s_, hadj[5]); yw = fmaf(h[5], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[103], fmaf(y[14], adj[98], fmaf(y[13], adj[93], fmaf(y[12], adj[88], fmaf(y[11], adj[83], fmaf(y[10], adj[78], y[9] * adj[73])))))); \
-        hadj[6] = fmaf(R[7], s_, hadj[6]); yw = fmaf(h[6], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[104], fmaf(y[14], adj[99], fmaf(y[13], adj[94], fmaf(y[12], adj[89], fmaf(y[11], adj[84], fmaf(y[10], adj[79], y[9] * adj[74])))))); \
-        hadj[7] = fmaf(R[7], s_, hadj[7]); yw = fmaf(h[7], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[105], fmaf(y[14], adj[100], fmaf(y[13], adj[95], fmaf(y[12], adj[90], fmaf(y[11], adj[85], fmaf(y[10], adj[80], y[9] * adj[75])))))); \
-        hadj[8] = fmaf(R[7], s_, hadj[8]); yw = fmaf(h[8], s_, yw); } \
-      radial = fmaf(dR[7], yw, radial); \
-    } \
-    { /* path 8: edge l=2, source l=0 -> l=2 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[8] * h[0]; \
-      ang[4] = fmaf(rh0, adj[106], ang[4]); \
-      ang[5] = fmaf(rh0, adj[107], ang[5]); \
-      ang[6] = fmaf(rh0, adj[108], ang[6]); \
-      ang[7] = fmaf(rh0, adj[109], ang[7]); \
-      ang[8] = fmaf(rh0, adj[110], ang[8]); \
-      { const float s_ = fmaf(y[8], adj[110], fmaf(y[7], adj[109], fmaf(y[6], adj[108], fmaf(y[5], adj[107], y[4] * adj[106])))); \
-        hadj[0] = fmaf(R[8], s_, hadj[0]); yw = fmaf(h[0], s_, yw); } \
-      radial = fmaf(dR[8], yw, radial); \
-    } \
-    { /* path 9: edge l=1, source l=1 -> l=2 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[9] * y[1]; \
-      const float ry1 = R[9] * y[2]; \
-      const float ry2 = R[9] * y[3]; \
-      { const float w = fmaf(h[3], adj[113], fmaf(h[2], adj[112], h[1] * adj[111])); \
-        ang[1] = fmaf(R[9], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[3], adj[116], fmaf(h[2], adj[115], h[1] * adj[114])); \
-        ang[2] = fmaf(R[9], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[3], adj[119], fmaf(h[2], adj[118], h[1] * adj[117])); \
-        ang[3] = fmaf(R[9], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[1] = fmaf(ry0, adj[111], hadj[1]); \
-      hadj[1] = fmaf(ry1, adj[114], hadj[1]); \
-      hadj[1] = fmaf(ry2, adj[117], hadj[1]); \
-      hadj[2] = fmaf(ry0, adj[112], hadj[2]); \
-      hadj[2] = fmaf(ry1, adj[115], hadj[2]); \
-      hadj[2] = fmaf(ry2, adj[118], hadj[2]); \
-      hadj[3] = fmaf(ry0, adj[113], hadj[3]); \
-      hadj[3] = fmaf(ry1, adj[116], hadj[3]); \
-      hadj[3] = fmaf(ry2, adj[119], hadj[3]); \
-      radial = fmaf(dR[9], yw, radial); \
-    } \
-    { /* path 10: edge l=3, source l=1 -> l=2 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[10] * h[1]; \
-      const float rh1 = R[10] * h[2]; \
-      const float rh2 = R[10] * h[3]; \
-      ang[9] = fmaf(rh0, adj[120], ang[9]); \
-      ang[9] = fmaf(rh1, adj[121], ang[9]); \
-      ang[9] = fmaf(rh2, adj[122], ang[9]); \
-      ang[10] = fmaf(rh0, adj[123], ang[10]); \
-      ang[10] = fmaf(rh1, adj[124], ang[10]); \
-      ang[10] = fmaf(rh2, adj[125], ang[10]); \
-      ang[11] = fmaf(rh0, adj[126], ang[11]); \
-      ang[11] = fmaf(rh1, adj[127], ang[11]); \
-      ang[11] = fmaf(rh2, adj[128], ang[11]); \
-      ang[12] = fmaf(rh0, adj[129], ang[12]); \
-      ang[12] = fmaf(rh1, adj[130], ang[12]); \
-      ang[12] = fmaf(rh2, adj[131], ang[12]); \
-      ang[13] = fmaf(rh0, adj[132], ang[13]); \
-      ang[13] = fmaf(rh1, adj[133], ang[13]); \
-      ang[13] = fmaf(rh2, adj[134], ang[13]); \
-      ang[14] = fmaf(rh0, adj[135], ang[14]); \
-      ang[14] = fmaf(rh1, adj[136], ang[14]); \
-      ang[14] = fmaf(rh2, adj[137], ang[14]); \
-      ang[15] = fmaf(rh0, adj[138], ang[15]); \
-      ang[15] = fmaf(rh1, adj[139], ang[15]); \
-      ang[15] = fmaf(rh2, adj[140], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[138], fmaf(y[14], adj[135], fmaf(y[13], adj[132], fmaf(y[12], adj[129], fmaf(y[11], adj[126], fmaf(y[10], adj[123], y[9] * adj[120])))))); \
-        hadj[1] = fmaf(R[10], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[139], fmaf(y[14], adj[136], fmaf(y[13], adj[133], fmaf(y[12], adj[130], fmaf(y[11], adj[127], fmaf(y[10], adj[124], y[9] * adj[121])))))); \
-        hadj[2] = fmaf(R[10], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[140], fmaf(y[14], adj[137], fmaf(y[13], adj[134], fmaf(y[12], adj[131], fmaf(y[11], adj[128], fmaf(y[10], adj[125], y[9] * adj[122])))))); \
-        hadj[3] = fmaf(R[10], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
-      radial = fmaf(dR[10], yw, radial); \
-    } \
-    { /* path 11: edge l=0, source l=2 -> l=2 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[11] * y[0]; \
-      { const float w = fmaf(h[8], adj[145], fmaf(h[7], adj[144], fmaf(h[6], adj[143], fmaf(h[5], adj[142], h[4] * adj[141])))); \
-        ang[0] = fmaf(R[11], w, ang[0]); yw = fmaf(y[0], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[141], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[142], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[143], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[144], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[145], hadj[8]); \
-      radial = fmaf(dR[11], yw, radial); \
-    } \
-    { /* path 12: edge l=2, source l=2 -> l=2 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[12] * y[4]; \
-      const float ry1 = R[12] * y[5]; \
-      const float ry2 = R[12] * y[6]; \
-      const float ry3 = R[12] * y[7]; \
-      const float ry4 = R[12] * y[8]; \
-      { const float w = fmaf(h[8], adj[150], fmaf(h[7], adj[149], fmaf(h[6], adj[148], fmaf(h[5], adj[147], h[4] * adj[146])))); \
-        ang[4] = fmaf(R[12], w, ang[4]); yw = fmaf(y[4], w, yw); } \
-      { const float w = fmaf(h[8], adj[155], fmaf(h[7], adj[154], fmaf(h[6], adj[153], fmaf(h[5], adj[152], h[4] * adj[151])))); \
-        ang[5] = fmaf(R[12], w, ang[5]); yw = fmaf(y[5], w, yw); } \
-      { const float w = fmaf(h[8], adj[160], fmaf(h[7], adj[159], fmaf(h[6], adj[158], fmaf(h[5], adj[157], h[4] * adj[156])))); \
-        ang[6] = fmaf(R[12], w, ang[6]); yw = fmaf(y[6], w, yw); } \
-      { const float w = fmaf(h[8], adj[165], fmaf(h[7], adj[164], fmaf(h[6], adj[163], fmaf(h[5], adj[162], h[4] * adj[161])))); \
-        ang[7] = fmaf(R[12], w, ang[7]); yw = fmaf(y[7], w, yw); } \
-      { const float w = fmaf(h[8], adj[170], fmaf(h[7], adj[169], fmaf(h[6], adj[168], fmaf(h[5], adj[167], h[4] * adj[166])))); \
-        ang[8] = fmaf(R[12], w, ang[8]); yw = fmaf(y[8], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[146], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[151], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[156], hadj[4]); \
-      hadj[4] = fmaf(ry3, adj[161], hadj[4]); \
-      hadj[4] = fmaf(ry4, adj[166], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[147], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[152], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[157], hadj[5]); \
-      hadj[5] = fmaf(ry3, adj[162], hadj[5]); \
-      hadj[5] = fmaf(ry4, adj[167], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[148], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[153], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[158], hadj[6]); \
-      hadj[6] = fmaf(ry3, adj[163], hadj[6]); \
-      hadj[6] = fmaf(ry4, adj[168], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[149], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[154], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[159], hadj[7]); \
-      hadj[7] = fmaf(ry3, adj[164], hadj[7]); \
-      hadj[7] = fmaf(ry4, adj[169], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[150], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[155], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[160], hadj[8]); \
-      hadj[8] = fmaf(ry3, adj[165], hadj[8]); \
-      hadj[8] = fmaf(ry4, adj[170], hadj[8]); \
-      radial = fmaf(dR[12], yw, radial); \
-    } \
-    { /* path 13: edge l=3, source l=0 -> l=3 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[13] * h[0]; \
-      ang[9] = fmaf(rh0, adj[171], ang[9]); \
-      ang[10] = fmaf(rh0, adj[172], ang[10]); \
-      ang[11] = fmaf(rh0, adj[173], ang[11]); \
-      ang[12] = fmaf(rh0, adj[174], ang[12]); \
-      ang[13] = fmaf(rh0, adj[175], ang[13]); \
-      ang[14] = fmaf(rh0, adj[176], ang[14]); \
-      ang[15] = fmaf(rh0, adj[177], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[177], fmaf(y[14], adj[176], fmaf(y[13], adj[175], fmaf(y[12], adj[174], fmaf(y[11], adj[173], fmaf(y[10], adj[172], y[9] * adj[171])))))); \
-        hadj[0] = fmaf(R[13], s_, hadj[0]); yw = fmaf(h[0], s_, yw); } \
-      radial = fmaf(dR[13], yw, radial); \
-    } \
-    { /* path 14: edge l=2, source l=1 -> l=3 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[14] * h[1]; \
-      const float rh1 = R[14] * h[2]; \
-      const float rh2 = R[14] * h[3]; \
-      ang[4] = fmaf(rh0, adj[178], ang[4]); \
-      ang[4] = fmaf(rh1, adj[179], ang[4]); \
-      ang[4] = fmaf(rh2, adj[180], ang[4]); \
-      ang[5] = fmaf(rh0, adj[181], ang[5]); \
-      ang[5] = fmaf(rh1, adj[182], ang[5]); \
-      ang[5] = fmaf(rh2, adj[183], ang[5]); \
-      ang[6] = fmaf(rh0, adj[184], ang[6]); \
-      ang[6] = fmaf(rh1, adj[185], ang[6]); \
-      ang[6] = fmaf(rh2, adj[186], ang[6]); \
-      ang[7] = fmaf(rh0, adj[187], ang[7]); \
-      ang[7] = fmaf(rh1, adj[188], ang[7]); \
-      ang[7] = fmaf(rh2, adj[189], ang[7]); \
-      ang[8] = fmaf(rh0, adj[190], ang[8]); \
-      ang[8] = fmaf(rh1, adj[191], ang[8]); \
-      ang[8] = fmaf(rh2, adj[192], ang[8]); \
-      { const float s_ = fmaf(y[8], adj[190], fmaf(y[7], adj[187], fmaf(y[6], adj[184], fmaf(y[5], adj[181], y[4] * adj[178])))); \
-        hadj[1] = fmaf(R[14], s_, hadj[1]); yw = fmaf(h[1], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[191], fmaf(y[7], adj[188], fmaf(y[6], adj[185], fmaf(y[5], adj[182], y[4] * adj[179])))); \
-        hadj[2] = fmaf(R[14], s_, hadj[2]); yw = fmaf(h[2], s_, yw); } \
-      { const float s_ = fmaf(y[8], adj[192], fmaf(y[7], adj[189], fmaf(y[6], adj[186], fmaf(y[5], adj[183], y[4] * adj[180])))); \
-        hadj[3] = fmaf(R[14], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
-      radial = fmaf(dR[14], yw, radial); \
-    } \
-    { /* path 15: edge l=1, source l=2 -> l=3 */ \
-      float yw = 0.0f; \
-      const float ry0 = R[15] * y[1]; \
-      const float ry1 = R[15] * y[2]; \
-      const float ry2 = R[15] * y[3]; \
-      { const float w = fmaf(h[8], adj[197], fmaf(h[7], adj[196], fmaf(h[6], adj[195], fmaf(h[5], adj[194], h[4] * adj[193])))); \
-        ang[1] = fmaf(R[15], w, ang[1]); yw = fmaf(y[1], w, yw); } \
-      { const float w = fmaf(h[8], adj[202], fmaf(h[7], adj[201], fmaf(h[6], adj[200], fmaf(h[5], adj[199], h[4] * adj[198])))); \
-        ang[2] = fmaf(R[15], w, ang[2]); yw = fmaf(y[2], w, yw); } \
-      { const float w = fmaf(h[8], adj[207], fmaf(h[7], adj[206], fmaf(h[6], adj[205], fmaf(h[5], adj[204], h[4] * adj[203])))); \
-        ang[3] = fmaf(R[15], w, ang[3]); yw = fmaf(y[3], w, yw); } \
-      hadj[4] = fmaf(ry0, adj[193], hadj[4]); \
-      hadj[4] = fmaf(ry1, adj[198], hadj[4]); \
-      hadj[4] = fmaf(ry2, adj[203], hadj[4]); \
-      hadj[5] = fmaf(ry0, adj[194], hadj[5]); \
-      hadj[5] = fmaf(ry1, adj[199], hadj[5]); \
-      hadj[5] = fmaf(ry2, adj[204], hadj[5]); \
-      hadj[6] = fmaf(ry0, adj[195], hadj[6]); \
-      hadj[6] = fmaf(ry1, adj[200], hadj[6]); \
-      hadj[6] = fmaf(ry2, adj[205], hadj[6]); \
-      hadj[7] = fmaf(ry0, adj[196], hadj[7]); \
-      hadj[7] = fmaf(ry1, adj[201], hadj[7]); \
-      hadj[7] = fmaf(ry2, adj[206], hadj[7]); \
-      hadj[8] = fmaf(ry0, adj[197], hadj[8]); \
-      hadj[8] = fmaf(ry1, adj[202], hadj[8]); \
-      hadj[8] = fmaf(ry2, adj[207], hadj[8]); \
-      radial = fmaf(dR[15], yw, radial); \
-    } \
-    { /* path 16: edge l=3, source l=2 -> l=3 */ \
-      float yw = 0.0f; \
-      const float rh0 = R[16] * h[4]; \
-      const float rh1 = R[16] * h[5]; \
-      const float rh2 = R[16] * h[6]; \
-      const float rh3 = R[16] * h[7]; \
-      const float rh4 = R[16] * h[8]; \
-      ang[9] = fmaf(rh0, adj[208], ang[9]); \
-      ang[9] = fmaf(rh1, adj[209], ang[9]); \
-      ang[9] = fmaf(rh2, adj[210], ang[9]); \
-      ang[9] = fmaf(rh3, adj[211], ang[9]); \
-      ang[9] = fmaf(rh4, adj[212], ang[9]); \
-      ang[10] = fmaf(rh0, adj[213], ang[10]); \
-      ang[10] = fmaf(rh1, adj[214], ang[10]); \
-      ang[10] = fmaf(rh2, adj[215], ang[10]); \
-      ang[10] = fmaf(rh3, adj[216], ang[10]); \
-      ang[10] = fmaf(rh4, adj[217], ang[10]); \
-      ang[11] = fmaf(rh0, adj[218], ang[11]); \
-      ang[11] = fmaf(rh1, adj[219], ang[11]); \
-      ang[11] = fmaf(rh2, adj[220], ang[11]); \
-      ang[11] = fmaf(rh3, adj[221], ang[11]); \
-      ang[11] = fmaf(rh4, adj[222], ang[11]); \
-      ang[12] = fmaf(rh0, adj[223], ang[12]); \
-      ang[12] = fmaf(rh1, adj[224], ang[12]); \
-      ang[12] = fmaf(rh2, adj[225], ang[12]); \
-      ang[12] = fmaf(rh3, adj[226], ang[12]); \
-      ang[12] = fmaf(rh4, adj[227], ang[12]); \
-      ang[13] = fmaf(rh0, adj[228], ang[13]); \
-      ang[13] = fmaf(rh1, adj[229], ang[13]); \
-      ang[13] = fmaf(rh2, adj[230], ang[13]); \
-      ang[13] = fmaf(rh3, adj[231], ang[13]); \
-      ang[13] = fmaf(rh4, adj[232], ang[13]); \
-      ang[14] = fmaf(rh0, adj[233], ang[14]); \
-      ang[14] = fmaf(rh1, adj[234], ang[14]); \
-      ang[14] = fmaf(rh2, adj[235], ang[14]); \
-      ang[14] = fmaf(rh3, adj[236], ang[14]); \
-      ang[14] = fmaf(rh4, adj[237], ang[14]); \
-      ang[15] = fmaf(rh0, adj[238], ang[15]); \
-      ang[15] = fmaf(rh1, adj[239], ang[15]); \
-      ang[15] = fmaf(rh2, adj[240], ang[15]); \
-      ang[15] = fmaf(rh3, adj[241], ang[15]); \
-      ang[15] = fmaf(rh4, adj[242], ang[15]); \
-      { const float s_ = fmaf(y[15], adj[238], fmaf(y[14], adj[233], fmaf(y[13], adj[228], fmaf(y[12], adj[223], fmaf(y[11], adj[218], fmaf(y[10], adj[213], y[9] * adj[208])))))); \
-        hadj[4] = fmaf(R[16], s_, hadj[4]); yw = fmaf(h[4], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[239], fmaf(y[14], adj[234], fmaf(y[13], adj[229], fmaf(y[12], adj[224], fmaf(y[11], adj[219], fmaf(y[10], adj[214], y[9] * adj[209])))))); \
-        hadj[5] = fmaf(R[16], s_, hadj[5]); yw = fmaf(h[5], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[240], fmaf(y[14], adj[235], fmaf(y[13], adj[230], fmaf(y[12], adj[225], fmaf(y[11], adj[220], fmaf(y[10], adj[215], y[9] * adj[210])))))); \
-        hadj[6] = fmaf(R[16], s_, hadj[6]); yw = fmaf(h[6], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[241], fmaf(y[14], adj[236], fmaf(y[13], adj[231], fmaf(y[12], adj[226], fmaf(y[11], adj[221], fmaf(y[10], adj[216], y[9] * adj[211])))))); \
-        hadj[7] = fmaf(R[16], s_, hadj[7]); yw = fmaf(h[7], s_, yw); } \
-      { const float s_ = fmaf(y[15], adj[242], fmaf(y[14], adj[237], fmaf(y[13], adj[232], fmaf(y[12], adj[227], fmaf(y[11], adj[222], fmaf(y[10], adj[217], y[9] * adj[212])))))); \
-        hadj[8] = fmaf(R[16], s_, hadj[8]); yw = fmaf(h[8], s_, yw); } \
-      radial = fmaf(dR[16], yw, radial); \
-    }
 #define SXB_S2_L1_REVERSE_EDGES_BODY \
     { f2 y[kEdges][1]; EACH(load_pair_harmonics<0>(yrow[e], y[e]);) \
     { /* path 0: edge l=0, source l=0 -> l=0 */ RADIAL(0) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
