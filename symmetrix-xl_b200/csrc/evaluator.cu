@@ -203,21 +203,30 @@ Evaluator::Evaluator(const std::string& json_path, int device_ordinal, const std
         upload(residual_fused_, model_.residual_fused, stream_);
         upload(residual_scalar_, model_.residual_scalar, stream_);
     }
-    SXB_ALLOW_POLY_SMEM(m0_forward_kernel_S0, SXB_S0_M0_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m0_reverse_kernel_S0, SXB_S0_M0_NUM_TERMS);
-    SXB_ALLOW_POLY_SMEM(m0_forward_kernel_S1, SXB_S1_M0_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m0_reverse_kernel_S1, SXB_S1_M0_NUM_TERMS);
-    SXB_ALLOW_POLY_SMEM(m0_forward_kernel_S2, SXB_S2_M0_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m0_reverse_kernel_S2, SXB_S2_M0_NUM_TERMS);
-    SXB_ALLOW_POLY_SMEM(m1_forward_kernel_S0, SXB_S0_M1_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_S0, SXB_S0_M1_NUM_TERMS);
-    SXB_ALLOW_POLY_SMEM(m1_forward_kernel_S1, SXB_S1_M1_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_S1, SXB_S1_M1_NUM_TERMS);
-    SXB_ALLOW_POLY_SMEM(m1_forward_kernel_S2, SXB_S2_M1_NUM_TERMS); SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_S2, SXB_S2_M1_NUM_TERMS);
+    // shared-memory limits of the model's own structure only: setting one loads the kernel
+#define SXB_ALLOW_POLY_SMEM_SHAPE(NAME)                                                                                  \
+    SXB_ALLOW_POLY_SMEM(m0_forward_kernel_##NAME, SXB_##NAME##_M0_NUM_TERMS);                                           \
+    SXB_ALLOW_POLY_SMEM(m0_reverse_kernel_##NAME, SXB_##NAME##_M0_NUM_TERMS);                                           \
+    SXB_ALLOW_POLY_SMEM(m1_forward_kernel_##NAME, SXB_##NAME##_M1_NUM_TERMS);                                           \
+    SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_##NAME, SXB_##NAME##_M1_NUM_TERMS)
 #define SXB_ALLOW_SHARED_ROWS(NAME, WIDTH)                                                                               \
     SXB_CUDA(cudaFuncSetAttribute(l1_reverse_shared_kernel_##NAME<WIDTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                   static_cast<int>(shared_rows_bytes(SXB_##NAME##_NUM_ROWS, WIDTH))))
-    SXB_ALLOW_SHARED_ROWS(S1, 128);
-    SXB_ALLOW_SHARED_ROWS(S1, 64);
-    SXB_ALLOW_SHARED_ROWS(S2, 128);
+    if (model_.shape_id == 0) {
+        SXB_ALLOW_POLY_SMEM_SHAPE(S0);
+    } else if (model_.shape_id == 1) {
+        SXB_ALLOW_POLY_SMEM_SHAPE(S1);
+        if (C == 128) SXB_ALLOW_SHARED_ROWS(S1, 128);
+        if (C == 64) SXB_ALLOW_SHARED_ROWS(S1, 64);
+    } else {
+        SXB_ALLOW_POLY_SMEM_SHAPE(S2);
+        SXB_ALLOW_SHARED_ROWS(S2, 128);
+    }
+#undef SXB_ALLOW_POLY_SMEM_SHAPE
 #undef SXB_ALLOW_SHARED_ROWS
-    SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpsPerBlock * sizeof(WarpPairChunk)));
-    SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpsPerBlock * sizeof(WarpPairChunk)));
+    constexpr int pair_chunk_bytes = kWarpsPerBlock * sizeof(WarpPairChunk);
+    if (C == 128) SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_chunk_bytes));
+    if (C == 64) SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_chunk_bytes));
     SXB_CUDA(cudaFuncSetAttribute(tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes));
     SXB_CUDA(cudaFuncSetAttribute(tc_gemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kT3SmemBytes));
     SXB_CUDA(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device_));
