@@ -10,7 +10,9 @@
 // hidden 0e+1o 0.941 / 1.060 ms, 0e+1o+2e 2.16 / 2.57 ms (three launches).  Shapes tried for 0e+1o, (teams, blocks per SM,
 // edges): (2, 3, 2) 0.941, (4, 2, 1) 1.005, (4, 1, 2) 1.089; for 0e+1o+2e: (6, 1, 1) 2.157, (4, 1, 2) 2.153, (8, 1, 1) 2.23.
 // Now bound by the shared-memory data pipe (77 % of its wavefronts at twelve warps per SM).  The reproducible mode keeps the register form,
-// which leaves its records faster (1,080 receivers: 0.295 against 0.469 ms).
+// which leaves its records faster (1,080 receivers: 0.295 against 0.469 ms).  Registers: 168 at 128 channels (24 bytes spilled),
+// three blocks of four warps; at 64 channels the edge state, which does not shrink with the width, leaves room for four blocks
+// of two warps, so a thread may have 248: 5,000 receivers 0.451 ms, with the 168 of six blocks that never fit 0.599 ms.
 //
 // Math and reference citations: see edge_kernels.cuh (layer 1 reverse).
 #pragma once
@@ -198,9 +200,30 @@ __device__ __forceinline__ void flush_active_chunk(const ActiveChunk& s, const f
 
 #define SXB_SHARED_TRANSPOSE(term, row, lme) if ((row) % kShares == share) rows[(row) * kC + column] += cgc.cg[term] * dphi[lme];
 
-#define SXB_DEFINE_L1_SHARED_KERNEL(NAME, TEAMS, BLOCKS, EDGES)                                                     \
+constexpr std::size_t shared_rows_bytes(int rows, int channels) { return static_cast<std::size_t>(rows) * channels * sizeof(float); }
+// Shared memory of a block with `channels` channels: row adjoints, edge state, partial forces and sums, and the kilobyte that
+// the system keeps.  The edge state is the same at every width, so halving the channels does not double the blocks per SM.
+constexpr std::size_t shared_block_bytes(int rows, int channels)
+{
+    return shared_rows_bytes(rows, channels) + sizeof(ActiveChunk) + kEdgeChunk * (channels / 64) * 3 * sizeof(float)
+           + 2 * kForceSums * sizeof(double) + 1024;
+}
+constexpr std::size_t kSharedPerSM = 228 * 1024;
+
+// threads of a block per 64 channels, in warps, and resident blocks of an SM: what the launch bounds ask for and what the part
+// rule counts with
+constexpr int kSharedTeamsS1 = 2, kSharedTeamsS2 = 6;
+template <int kC>
+constexpr int kSharedBlocksS1 = kC == 128 ? 3 : 4;
+template <int kC>
+constexpr int kSharedBlocksS2 = 1;
+static_assert(kSharedBlocksS1<128> * shared_block_bytes(SXB_S1_NUM_ROWS, 128) <= kSharedPerSM, "0e+1o, 128 channels");
+static_assert(kSharedBlocksS1<64> * shared_block_bytes(SXB_S1_NUM_ROWS, 64) <= kSharedPerSM, "0e+1o, 64 channels");
+static_assert(kSharedBlocksS2<128> * shared_block_bytes(SXB_S2_NUM_ROWS, 128) <= kSharedPerSM, "0e+1o+2e, 128 channels");
+
+#define SXB_DEFINE_L1_SHARED_KERNEL(NAME, TEAMS, EDGES)                                                             \
 template <int kC>                                                                                                   \
-__global__ void __launch_bounds__(kC / 2 * TEAMS, BLOCKS * 128 / kC)                                                \
+__global__ void __launch_bounds__(kC / 2 * TEAMS, kSharedBlocks##NAME<kC>)                                          \
 l1_reverse_shared_kernel_##NAME(int node0, const int* __restrict__ first, const int* __restrict__ sources,          \
                                 const EdgeGeom* __restrict__ geom, const unsigned char* __restrict__ atype, SplineGrid grid,\
                                 const float4* __restrict__ table, const float* __restrict__ H1,                     \
@@ -269,12 +292,8 @@ l1_reverse_shared_kernel_##NAME(int node0, const int* __restrict__ first, const 
     }                                                                                                               \
 }
 
-SXB_DEFINE_L1_SHARED_KERNEL(S1, 2, 3, 2)
-SXB_DEFINE_L1_SHARED_KERNEL(S2, 6, 1, 1)
-
-// threads of a block and dynamic shared memory
-constexpr int kSharedTeamsS1 = 2, kSharedTeamsS2 = 6;
-constexpr std::size_t shared_rows_bytes(int rows, int channels) { return static_cast<std::size_t>(rows) * channels * sizeof(float); }
+SXB_DEFINE_L1_SHARED_KERNEL(S1, 2, 2)
+SXB_DEFINE_L1_SHARED_KERNEL(S2, 6, 1)
 
 #undef EACH
 #undef ADJ

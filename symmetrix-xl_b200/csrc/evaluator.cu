@@ -1296,7 +1296,8 @@ void Evaluator::run_pipeline(int phases)
             // hidden l > 0 at the common widths: row adjoints in shared memory; otherwise one channel per thread with the
             // adjoints in registers (16 rows for hidden 0e), which also leaves the records of the reproducible mode.
             const bool shared_rows = !deterministic_ && (model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64)));
-            const int reverse_parts = shared_rows ? edge_parts(T, model_.shape_id == 2 ? num_sms_ : num_sms_ * 3 * 128 / C, mean_edges, 8.0, 8)
+            const int shared_blocks = model_.shape_id == 2 ? kSharedBlocksS2<128> : C == 64 ? kSharedBlocksS1<64> : kSharedBlocksS1<128>;
+            const int reverse_parts = shared_rows ? edge_parts(T, num_sms_ * shared_blocks, mean_edges, 8.0, 8)
                                                   : edge_parts(T, num_sms_ * std::floor(12.0 / block_warps), mean_edges, 5.0, 8);
             const dim3 reverse_grid(T, reverse_parts);
 #define SXB_SHARED_REVERSE(NAME, WIDTH)                                                                                   \

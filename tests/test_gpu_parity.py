@@ -575,3 +575,22 @@ def test_layer1_gradient_widths_and_odd_edge_counts(pkg, model_path, channels, o
         _e, energies, forces, _s = mace_numpy.NumpyMACE(str(path)).energy_forces_stress(t, p, c, first, src, shifts)
         assert np.abs(out["energies"] - energies).max() <= TOL_E
         assert np.abs(out["forces"] - forces).max() <= TOL_F * max(1.0, np.abs(forces).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("arch,channels,copies", [("medium", 128, (3, 3, 3)), ("medium", 64, (3, 3, 3)), ("large", 128, (3, 3, 2))])
+def test_receivers_of_several_edge_chunks(pkg, model_path, arch, channels, copies):
+    """Receivers enough that their 97 list edges are not dealt out, so that a block of the layer-1 gradient fills its 64-edge
+    chunk a second time, at every compiled width: periodic copies of a 40-atom cell, atom by atom against the oracle of the
+    cell (bounds of the oracle comparison)."""
+    path = model_path(arch, 37, channels=channels)
+    pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 14)
+    r_cut = pkg.MACEB200(path).r_cut
+    first, src, shifts = neighbor.build_neighbor_graph(pos, cell, r_cut + 0.5)
+    _e, energies, forces, _s = mace_numpy.NumpyMACE(str(path)).energy_forces_stress(types, pos, cell, first, src, shifts)
+    grid = np.stack(np.meshgrid(*[np.arange(c) for c in copies], indexing="ij"), axis=-1).reshape(-1, 3)
+    many = (pos[None] + (grid @ cell)[:, None]).reshape(-1, 3)
+    calc = pkg.Calculator(path, skin=0.5)
+    out = calc.calculate(many, cell * np.array(copies)[:, None], np.tile(types, len(grid)))
+    assert np.abs(out["energies"].reshape(len(grid), -1) - energies).max() <= TOL_E
+    assert np.abs(out["forces"].reshape(len(grid), -1, 3) - forces).max() <= TOL_F
