@@ -28,8 +28,8 @@ constexpr int kEdgeChunk = 64;
 
 // A receiver's edges can be dealt to several blocks (layer 1) or warps (layer 0): part p of n walks [x, y) of the
 // receiver's CSR range.  A receiver is a serial chain of about 75 edges at 0.5 to 1 us each, so with fewer receivers than
-// the chip holds blocks the whole kernel lasts as long as one chain; the host picks the number of parts (edge_parts and
-// cluster_parts in evaluator.cu).  Gradient parts are independent.  Forward parts are one thread-block cluster that adds
+// the chip holds blocks the whole kernel lasts as long as one chain; the host picks the number of parts
+// (part_rules.hpp).  Gradient parts are independent.  Forward parts are one thread-block cluster that adds
 // its sums up over distributed shared memory, in part order, so that the result has one order.
 __device__ __forceinline__ int2 edge_part(const int* __restrict__ first, int i, int part, int parts)
 {

@@ -21,6 +21,7 @@
 #include "edge_kernels_warp.cuh"
 #include "graph_kernels.cuh"
 #include "node_kernels.cuh"
+#include "part_rules.hpp"
 #include "tc_gemm.cuh"
 #include "tc_gemm_tma.cuh"
 
@@ -71,37 +72,6 @@ inline int blocks_for(long n, int threads) { return static_cast<int>((n + thread
         else if ((C) == 32) KERNEL<32><<<(GRID), 32, 0, (STREAM)>>>(__VA_ARGS__);     \
         else KERNEL<0><<<(GRID), (C), 0, (STREAM)>>>(__VA_ARGS__);                    \
     } while (0)
-
-// How many parts to deal a receiver's edges to (edge_part in edge_kernels.cuh) in a gradient kernel.  `units` receivers of
-// `edges` list edges each run on `slots` resident blocks or warps; a part costs its edges plus `overhead` edges' worth of
-// prologue, chunk fill and reductions.  Up to a few rounds of the chip the last round is counted whole (a chain in it takes
-// as long as any other), beyond that half of it; a further part has to pay for itself by a twentieth.  Measured, 128
-// channels, 100 list edges, us at 1 / 2 / 4 / 8 parts: layer-1 gradient, 40 receivers 68 / 39 / 29 / 23, 317: 99 / 101 / 85 /
-// 91, 599: 177 / 146 / 150 / 162, 1080: 295 / 296 / 310 / 353; layer-0 gradient, 40: 81 / 45 / 29 / 21, 599: 88 / 58 / 60 /
-// 56, 2160: 182 / 149 / 146 / 161.
-int edge_parts(long units, double slots, double edges, double overhead, int most)
-{
-    int best = 1;
-    double best_cost = 0.0;
-    for (int parts = 1; parts <= most; parts *= 2) {
-        const double rounds = static_cast<double>(units) * parts / slots;
-        const double cost = (rounds < 4.0 ? std::ceil(rounds) : rounds + 0.5) * (edges / parts + overhead);
-        if (parts == 1 || cost < 0.95 * best_cost) {
-            best = parts;
-            best_cost = cost;
-        }
-    }
-    return best;
-}
-
-// The same for the layer-1 forward kernel, whose parts meet in a cluster: as many as fill the chip once.  Measured at 1 / 2 /
-// 4 / 8 parts: 40 receivers 37 / 34 / 23 / 18 us; 317 receivers (which fill it at one part and a half) 51 / 62 / 62 / 68 us.
-int cluster_parts(long units, double slots)
-{
-    int parts = 1;
-    while (parts < 8 && units * parts * 2 <= slots) parts *= 2;
-    return parts;
-}
 
 // Launches a kernel over (receivers, parts) with the parts of a receiver as one cluster, each with `row_bytes` of dynamic
 // shared memory.
@@ -1047,15 +1017,9 @@ void Evaluator::run_pipeline(int phases)
     const float* inv1 = model_.a1_scaled ? inv_scale1_.ptr : nullptr;
     const DensityScale density0{model_.a0_scaled ? density0_table_.ptr : nullptr, inv_scale0_.ptr, dot0_.ptr, n_active};
     const DensityScale density1{model_.a1_scaled ? density1_table_.ptr : nullptr, inv_scale1_.ptr, dot1_.ptr, n_active};
-    // parts a receiver's edges are dealt to; resident warps per SM: 16 forward, 12 in the gradients (128 and 168 registers).
-    // Layer-0 forward has a build for one warp or a whole block per receiver: 40 receivers 46 -> 20 us, 599: 50 -> 38 us,
-    // 1080: 57 -> 47 us, 2160: 80 -> 86 us.
-    const double mean_edges = static_cast<double>(num_edges_) / std::max(1, R), block_warps = std::max(1, C / 32);
-    auto l1_forward_parts = [&](int T) { return cluster_parts(T, num_sms_ * std::floor(16.0 / block_warps)); };
-    auto l0_forward_parts = [&](int T) { return edge_parts(T, num_sms_ * 16.0, mean_edges, 6.0, kWarpsPerBlock) > 1 ? kWarpsPerBlock : 1; };
-    auto l0_reverse_parts = [&](int T) { return edge_parts(T, num_sms_ * 12.0, mean_edges, 4.0, 8); };
+    const PartRules rules{num_sms_, C, model_.shape_id, static_cast<double>(num_edges_) / std::max(1, R)};
     auto l0_forward = [&](int t0, int T) {
-        const int parts = l0_forward_parts(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
+        const int parts = rules.l0_forward(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
         const std::size_t part_bytes = parts > 1 ? static_cast<std::size_t>(kWarpsPerBlock) * 16 * C * sizeof(float) : 0;
         if (C == 128)
             l0_forward_warp_kernel<4><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
@@ -1156,7 +1120,7 @@ void Evaluator::run_pipeline(int phases)
                 launches_ += 1;
                 span_end();
             } else {
-            const int forward_parts = l1_forward_parts(T);
+            const int forward_parts = rules.l1_forward(T);
             const std::size_t row_bytes = static_cast<std::size_t>(NE) * C * sizeof(float);   // S2: a set has fewer rows
             span_begin("l1_forward");
             if (model_.shape_id == 0)
@@ -1297,8 +1261,7 @@ void Evaluator::run_pipeline(int phases)
             // adjoints in registers (16 rows for hidden 0e), which also leaves the records of the reproducible mode.
             const bool shared_rows = !deterministic_ && (model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64)));
             const int shared_blocks = model_.shape_id == 2 ? kSharedBlocksS2<128> : C == 64 ? kSharedBlocksS1<64> : kSharedBlocksS1<128>;
-            const int reverse_parts = shared_rows ? edge_parts(T, num_sms_ * shared_blocks, mean_edges, 8.0, 8)
-                                                  : edge_parts(T, num_sms_ * std::floor(12.0 / block_warps), mean_edges, 5.0, 8);
+            const int reverse_parts = shared_rows ? rules.l1_reverse_shared(T, shared_blocks) : rules.l1_reverse(T);
             const dim3 reverse_grid(T, reverse_parts);
 #define SXB_SHARED_REVERSE(NAME, WIDTH)                                                                                   \
             l1_reverse_shared_kernel_##NAME<WIDTH><<<reverse_grid, WIDTH / 2 * kSharedTeams##NAME,                         \
@@ -1406,7 +1369,7 @@ void Evaluator::run_pipeline(int phases)
             span_end();
             span_begin("l0_reverse");
             {
-                const int parts = l0_reverse_parts(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
+                const int parts = rules.l0_reverse(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
                 if (C == 128)
                     l0_reverse_pair_kernel<4><<<warp_grid, warp_threads, kWarpsPerBlock * sizeof(WarpPairChunk), stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else if (C == 64)

@@ -1,0 +1,90 @@
+// How many parts the edge kernels deal a receiver's edges to (edge_part in edge_kernels.cuh).  Host arithmetic without CUDA.
+//
+// A receiver is a serial chain of its edges, so with fewer receivers than the chip holds blocks (or warps) a kernel lasts as
+// long as one chain.  What a rule needs of its kernel is how many blocks or warps of it are resident on an SM, by registers
+// (65,536), shared memory (228 KB) and blocks (32).  Times below: us a launch, B200, medium model (97 list edges a receiver)
+// unless said otherwise.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+
+namespace sxb {
+
+// Time of `units` receivers of `edges` list edges each in `parts` parts on `slots` resident blocks or warps, in edges: a part
+// costs its edges plus `overhead` edges' worth of prologue, chunk fill and reductions.  Up to a few rounds of the chip the last
+// round is counted whole (a chain in it takes as long as any other), beyond that half of it.
+inline double parts_cost(long units, double slots, double edges, double overhead, int parts)
+{
+    const double rounds = static_cast<double>(units) * parts / slots;
+    return (rounds < 4.0 ? std::ceil(rounds) : rounds + 0.5) * (edges / parts + overhead);
+}
+
+// The best of 1, step, step^2, ... `most` parts; more parts have to bring the cost below `gain` of what it was.
+inline int edge_parts(long units, double slots, double edges, double overhead, double gain, int step, int most)
+{
+    int best = 1;
+    for (int parts = step; parts <= most; parts *= step)
+        if (parts_cost(units, slots, edges, overhead, parts) < gain * parts_cost(units, slots, edges, overhead, best)) best = parts;
+    return best;
+}
+
+struct PartRules {
+    int num_sms, channels, shape;      // shape: 0 hidden 0e, 1 0e+1o, 2 0e+1o+2e
+    double edges;                      // mean list edges of a receiver
+
+    int block_warps() const { return std::max(1, channels / 32); }
+
+    // Layer-0 sums: a build for one warp and one for the four warps of a block per receiver, and nothing between them.  Resident
+    // warps 16, 32 and 40 at 128, 64 and 32 channels (128, 64 and 48 registers).  One / four, 128 channels: 40 receivers 46 / 20,
+    // 1,080: 59 / 46, 2,160: 76 / 82, 2,560: 109 / 97, 5,000: 176 / 174, 7,200: 222 / 238; 64 channels, where a part costs more
+    // beside its edges: 2,160: 72 / 64, 3,240: 77 / 85, 7,560: 137 / 166.
+    int l0_forward(long receivers) const
+    {
+        const int resident = channels == 128 ? 16 : channels == 64 ? 32 : 40;
+        return edge_parts(receivers, 1.0 * num_sms * resident, edges, channels == 64 ? 11.0 : 5.0, 0.9, 4, 4);
+    }
+
+    // Layer-0 gradient: resident warps 12, 16 and 20 at 128, 64 and 32 channels (168 registers; 54 and 39 KB a block of four).
+    // 1 / 2 / 4 / 8 parts, 128 channels: 40 receivers 66 / 39 / 25 / 17, 600: 72 / 48 / 50 / 48, 2,160: 138 / 119 / 123 / 142,
+    // 5,000: 243 / 248 / 271 / 312; 64 channels, 1,500: 68 / 68 / 64 / 70; 32 channels (hidden 0e, 58 edges), 1,080: 35 / 29 /
+    // 31 / 33.
+    int l0_reverse(long receivers) const
+    {
+        const int resident = channels == 128 ? 12 : channels == 64 ? 16 : 20;
+        return edge_parts(receivers, 1.0 * num_sms * resident, edges, 4.0, 0.95, 2, 8);
+    }
+
+    // Layer-1 sums, whose parts meet in a cluster: as many as fill the chip once, at most five blocks on an SM (placing the
+    // blocks of more clusters takes longer than the chains they shorten).  1 / 2 / 4 / 8 parts, 128 channels: 40 receivers 39 /
+    // 35 / 23 / 18, 320: 51 / 64 / 64 / 70; 64 channels, 160: 39 / 37 / 27 / 31; hidden 0e (58 edges) at 32 channels, 160: 21 /
+    // 17 / 13 / 15, 600: 21 / 27 / 27 / 31, at 128 channels, 160: 27 / 21 / 17 / 21.
+    int l1_forward(long receivers) const
+    {
+        const long slots = static_cast<long>(num_sms) * std::min(5, (shape == 0 ? 32 : 16) / block_warps());
+        int parts = 1;
+        while (parts < 8 && receivers * parts * 2 <= slots) parts *= 2;
+        return parts;
+    }
+
+    // Layer-1 gradient with the row adjoints in shared memory, `resident` blocks of it on an SM.  1 / 2 / 4 / 8 parts, 128
+    // channels: 40 receivers 64 / 37 / 29 / 25, 320: 91 / 84 / 84 / 101, 600: 148 / 134 / 142 / 175, 1,080: 224 / 220 / 246 /
+    // 308, 5,000: 900 / 934 / 1,092 / 1,422; 64 channels, 320: 54 / 50 / 50 / 58, 1,080: 115 / 117 / 130 / 162; 0e+1o+2e, 40: 74 /
+    // 44 / 44 / 46, 160: 111 / 99 / 105 / 132, 600: 293 / 297 / 347 / 457.
+    int l1_reverse_shared(long receivers, int resident) const
+    {
+        return edge_parts(receivers, 1.0 * num_sms * resident, edges, 8.0, 0.95, 2, 8);
+    }
+
+    // Layer-1 gradient with the row adjoints in registers.  Hidden 0e: 128 registers and 26 KB a block, eight blocks of up to two
+    // warps, four of four.  1 / 2 / 4 / 8 parts, 32 channels (58 edges), 40 receivers: 31 / 21 / 15 / 13, 600: 35 / 33 / 33 / 35,
+    // 1,080: 37 / 39 / 45 / 56, 1,500: 60 / 54 / 60 / 72.  0e+1o (other widths, records): counted with 12 warps; records at 128
+    // channels, 40: 68 / 39 / 29 / 27, 600: 201 / 177 / 176 / 199, 1,080: 293 / 293 / 308 / 353.
+    int l1_reverse(long receivers) const
+    {
+        const int resident = shape == 0 ? std::min(8, 16 / block_warps()) : 12 / block_warps();
+        return edge_parts(receivers, 1.0 * num_sms * std::max(1, resident), edges, 5.0, 0.95, 2, 8);
+    }
+};
+
+}  // namespace sxb

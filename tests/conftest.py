@@ -1,3 +1,5 @@
+import ctypes
+import subprocess
 import sys
 from pathlib import Path
 
@@ -39,6 +41,25 @@ def model_path(pkg, model_dir):
         return cache[key]
 
     return get
+
+
+@pytest.fixture(scope="session")
+def part_rule(tmp_path_factory):
+    """rule(kernel, sms, channels, shape, edges, receivers, resident) -> parts, compiled from the library's header."""
+    folder = tmp_path_factory.mktemp("part_rules")
+    header = ROOT / "symmetrix-xl_b200" / "csrc" / "part_rules.hpp"
+    (folder / "rules.cpp").write_text(
+        f'#include "{header}"\n'
+        'extern "C" int rule(int kernel, int sms, int channels, int shape, double edges, long receivers, int resident)\n'
+        "{\n    const sxb::PartRules r{sms, channels, shape, edges};\n"
+        "    return kernel == 0 ? r.l0_forward(receivers) : kernel == 1 ? r.l1_forward(receivers) : kernel == 3 ? r.l0_reverse(receivers)\n"
+        "           : resident ? r.l1_reverse_shared(receivers, resident) : r.l1_reverse(receivers);\n}\n")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-o", str(folder / "rules.so"),
+                    str(folder / "rules.cpp")], check=True)
+    lib = ctypes.CDLL(str(folder / "rules.so"))
+    lib.rule.argtypes = [ctypes.c_int] * 4 + [ctypes.c_double, ctypes.c_long, ctypes.c_int]
+    kernels = ("l0_forward", "l1_forward", "l1_reverse", "l0_reverse")
+    return lambda kernel, *args: lib.rule(kernels.index(kernel), *args)
 
 
 def csr_from_positions(positions, cell, cutoff):

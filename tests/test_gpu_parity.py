@@ -578,19 +578,41 @@ def test_layer1_gradient_widths_and_odd_edge_counts(pkg, model_path, channels, o
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("arch,channels,copies", [("medium", 128, (3, 3, 3)), ("medium", 64, (3, 3, 3)), ("large", 128, (3, 3, 2))])
-def test_receivers_of_several_edge_chunks(pkg, model_path, arch, channels, copies):
-    """Receivers enough that their 97 list edges are not dealt out, so that a block of the layer-1 gradient fills its 64-edge
-    chunk a second time, at every compiled width: periodic copies of a 40-atom cell, atom by atom against the oracle of the
-    cell (bounds of the oracle comparison)."""
-    path = model_path(arch, 37, channels=channels)
+@pytest.mark.parametrize("arch,channels,options,copies,parts", [
+    # parts of a receiver in the layer-0 sums, the layer-1 sums, the layer-1 and the layer-0 gradient
+    ("medium", 128, {}, (1, 1, 1), (4, 8, 8, 8)),
+    ("medium", 128, {}, (2, 2, 2), (4, 1, 4, 4)),
+    ("medium", 128, {}, (3, 3, 3), (4, 1, 1, 4)),
+    ("medium", 128, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 4), (4, 1, 2, 1)),
+    ("medium", 128, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 6), (1, 1, 1, 2)),
+    ("medium", 64, {}, (1, 1, 1), (4, 8, 8, 8)),
+    ("medium", 64, {}, (3, 3, 3), (4, 1, 1, 2)),
+    ("medium", 64, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 9), (1, 1, 1, 2)),
+    ("large", 128, {}, (1, 1, 1), (4, 8, 2, 8)),
+    ("large", 128, {}, (3, 3, 2), (4, 1, 1, 2)),
+    ("small", 32, {}, (1, 1, 1), (4, 8, 8, 8)),
+    ("small", 32, {}, (4, 3, 3), (4, 1, 2, 2)),
+    ("small", 32, {}, (6, 5, 4), (1, 1, 1, 1)),
+])
+def test_every_division_of_receivers(pkg, model_path, part_rule, arch, channels, options, copies, parts):
+    """Each build that the part rules can choose, from the most parts to undivided receivers whose 97 list edges (small: 58)
+    fill the 64-edge chunks of the layer-1 kernels and the 32-edge ones of layer 0 more than once: periodic copies of a 40-atom
+    cell, atom by atom against the oracle of the cell (bounds of the oracle comparison).  The parts are asserted, so that a
+    changed rule cannot leave a build out unnoticed."""
+    import torch
+
+    path = model_path(arch, 37, channels=channels, **options)
     pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 14)
-    r_cut = pkg.MACEB200(path).r_cut
-    first, src, shifts = neighbor.build_neighbor_graph(pos, cell, r_cut + 0.5)
+    calc = pkg.Calculator(path, skin=0.5)
+    first, src, shifts = neighbor.build_neighbor_graph(pos, cell, calc.evaluator.r_cut + 0.5)
     _e, energies, forces, _s = mace_numpy.NumpyMACE(str(path)).energy_forces_stress(types, pos, cell, first, src, shifts)
     grid = np.stack(np.meshgrid(*[np.arange(c) for c in copies], indexing="ij"), axis=-1).reshape(-1, 3)
     many = (pos[None] + (grid @ cell)[:, None]).reshape(-1, 3)
-    calc = pkg.Calculator(path, skin=0.5)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    shape = {"small": 0, "medium": 1, "large": 2}[arch]
+    resident = {(1, 128): 3, (1, 64): 4, (2, 128): 1}.get((shape, channels), 0)
+    assert parts == tuple(part_rule(kernel, sms, channels, shape, len(src) / len(pos), len(many), resident if kernel == "l1_reverse" else 0)
+                          for kernel in ("l0_forward", "l1_forward", "l1_reverse", "l0_reverse"))
     out = calc.calculate(many, cell * np.array(copies)[:, None], np.tile(types, len(grid)))
     assert np.abs(out["energies"].reshape(len(grid), -1) - energies).max() <= TOL_E
     assert np.abs(out["forces"].reshape(len(grid), -1, 3) - forces).max() <= TOL_F
