@@ -555,6 +555,7 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
     SXB_CUDA(cudaMemcpyAsync(&status, error_flag_.ptr, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     SXB_CUDA(cudaStreamSynchronize(stream_));
     if (status & 4) throw std::invalid_argument("Neighbor graph positions must be finite.");
+    if (status & 32) throw std::invalid_argument("Neighbor graph positions lie too many cells away from the periodic cell.");
     if (total > static_cast<long long>(std::numeric_limits<int>::max()))
         throw std::length_error("Neighbor graph exceeds 32-bit edge indexing.");
     first_caller_.reserve(nr + 1);

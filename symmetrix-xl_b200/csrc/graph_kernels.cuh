@@ -24,7 +24,8 @@ struct CellGrid {
 };
 
 // Fractional coordinates wrapped into [0, 1), the wrap count per axis, the wrapped Cartesian position
-// and the atom's bin; a non-finite coordinate raises bit 2 of the status word.
+// and the atom's bin; a non-finite coordinate raises bit 2 of the status word, one more than 2^31 - 1 cells
+// away bit 5.
 __global__ void wrap_and_bin_kernel(int n, CellGrid grid, const double* __restrict__ positions,
                                     const double* __restrict__ inv_cell, const double* __restrict__ cell,
                                     double* __restrict__ wrapped_pos, int* __restrict__ wrap_count,
@@ -52,6 +53,10 @@ __global__ void wrap_and_bin_kernel(int n, CellGrid grid, const double* __restri
         double s = __dmul_rn(p[0], inv_cell[axis]);
         s = __dadd_rn(s, __dmul_rn(p[1], inv_cell[3 + axis]));
         s = __dadd_rn(s, __dmul_rn(p[2], inv_cell[6 + axis]));
+        if (!(fabs(s) < 2147483647.0)) {   // the count of cells does not fit an int (nor, below, a bin that is made from it)
+            atomicOr(status, 32);
+            s = 0.0;
+        }
         const int w = static_cast<int>(floor(s));
         f[axis] = __dadd_rn(s, -static_cast<double>(w));
         wrap_count[3 * atom + axis] = w;

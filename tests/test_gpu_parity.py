@@ -53,6 +53,22 @@ def test_neighbor_graph_triclinic_and_wrapped(pkg, model_path):
     assert mine == brute
 
 
+@pytest.mark.parametrize("far", [1e12, -1e12, 1e300, -1e300, float("nan"), float("-inf")])
+def test_neighbor_graph_refuses_positions_it_cannot_wrap(pkg, model_path, far):
+    """A coordinate whose count of cells does not fit 32 bits (a diverged trajectory is full of them) is an error like one that
+    is not finite, on either side of the cell; the evaluator stays usable.  A million cells away is still the same crystal."""
+    pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 4)
+    ev = pkg.MACEB200(model_path("small"))
+    inverse = np.linalg.inv(cell)
+    bad = pos.copy()
+    bad[7, 1] = far
+    with pytest.raises(ValueError, match="positions"):
+        ev._prepare_periodic_factorized_graph(types, bad, cell, inverse, 5.5)
+    edges = ev._prepare_periodic_factorized_graph(types, pos, cell, inverse, 5.5)["num_edges"]
+    moved = pos + np.array([1e6, -1e6, 0.0]) @ cell
+    assert abs(ev._prepare_periodic_factorized_graph(types, moved, cell, inverse, 5.5)["num_edges"] - edges) <= 2
+
+
 # with density scaling the device keeps Phi1 already divided by 1 + rho and A1_adj / dPhi1 / A0_adj
 # not yet divided (the division is folded into the next kernel's load), so those stages differ by
 # design from the serial evaluator's intermediates and are left to the energy / force comparison
