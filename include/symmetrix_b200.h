@@ -364,7 +364,11 @@ int sxb_set_tile_size(sxb_evaluator* evaluator, int32_t receivers_per_tile);
  * source-sorted schedule, the device counterpart of the reference's source schedule and source-owner
  * accumulation (source_offsets / source_edges, libsymmetrix/source/mace_kokkos_factorized_lifecycle.cpp:
  * 2133-2195; symmetrix/source/symmetrix/jit_codegen.py:1018-1109): two evaluations of one input give
- * identical bits.  Costs 4*num_hidden*num_channels bytes per edge (refused above 16 GB), so it is meant
+ * identical bits.  Energies and forces are sums over the edges inside the cutoff in list order: lists of
+ * another skin give the same bits as long as they have those edges in the same order, and so do tiles of
+ * another size (forces of tiled and untiled evaluations differ in the order of one sum).  The virial is
+ * summed over blocks of the whole list and repeats on the same list.  Costs 4*num_hidden*num_channels
+ * bytes per edge (refused above 16 GB), so it is meant
  * for small and medium systems; not available for hidden irreps 0e+1o+2e or density-scaled models.
  * The setting invalidates the prepared graph; prepare again afterwards. */
 int sxb_set_deterministic(sxb_evaluator* evaluator, int32_t enabled);

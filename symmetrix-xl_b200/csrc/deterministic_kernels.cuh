@@ -65,35 +65,54 @@ __device__ __forceinline__ double warp_total(double v)
     return v;
 }
 
-// forces[node] = - sum over the node's own edges (it is their receiver) + sum over the edges it is the source of.  One warp
-// per node: every lane takes each 32nd edge of either list in ascending order, the lanes meet in a fixed tree.  (One thread
-// per node left 1,080 atoms on nine blocks; this and the last stage below: 105 -> 33 us.)
-__global__ void reduce_node_forces_kernel(int num_nodes, int num_receivers, const int* __restrict__ first,
-                                          const int* __restrict__ source_offsets, const int* __restrict__ source_edges,
-                                          const double* __restrict__ edge_forces, double* __restrict__ forces)
+// Adds the lanes' force vectors to the warp's running sums: the n-th vector that is not zero goes to lane n % 32, whatever
+// number of zero vectors (edges in the list's skin) lies between them.  `rank` counts them; `slots` is the warp's exchange area.
+__device__ __forceinline__ void add_by_rank(const double (&f)[3], double (*__restrict__ slots)[3], int lane, int& rank, double (&sum)[3])
 {
-    const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const bool given = f[0] != 0.0 || f[1] != 0.0 || f[2] != 0.0;
+    const unsigned mask = __ballot_sync(0xffffffffu, given);
+    if (given)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) slots[(rank + __popc(mask & ((1u << lane) - 1u))) & 31][q] = f[q];
+    __syncwarp();
+    if (((lane - rank) & 31) < __popc(mask))
+#pragma unroll
+        for (int q = 0; q < 3; ++q) sum[q] += slots[lane][q];
+    __syncwarp();
+    rank += __popc(mask);
+}
+
+// forces[node] = - sum over the node's own edges (it is their receiver) + sum over the edges it is the source of.  One warp
+// per node: the edges of either list that carry a force are dealt to the lanes in ascending order, the lanes meet in a fixed
+// tree.  (One thread per node left 1,080 atoms on nine blocks; this and the last stage below: 105 -> 33 us.)
+constexpr int kNodeForceWarps = 4;
+__global__ void __launch_bounds__(32 * kNodeForceWarps)
+reduce_node_forces_kernel(int num_nodes, int num_receivers, const int* __restrict__ first, const int* __restrict__ source_offsets,
+                          const int* __restrict__ source_edges, const double* __restrict__ edge_forces, double* __restrict__ forces)
+{
+    __shared__ double slots[kNodeForceWarps][32][3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, node = blockIdx.x * kNodeForceWarps + warp;
     if (node >= num_nodes) return;
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    if (node < num_receivers)
-        for (int e = first[node] + lane; e < first[node + 1]; e += 32) {
-            fx -= edge_forces[3 * static_cast<size_t>(e)];
-            fy -= edge_forces[3 * static_cast<size_t>(e) + 1];
-            fz -= edge_forces[3 * static_cast<size_t>(e) + 2];
-        }
-    for (int k = source_offsets[node] + lane; k < source_offsets[node + 1]; k += 32) {
-        const size_t e = static_cast<size_t>(source_edges[k]);
-        fx += edge_forces[3 * e];
-        fy += edge_forces[3 * e + 1];
-        fz += edge_forces[3 * e + 2];
+    double own[3] = {0.0, 0.0, 0.0}, f[3];
+    int rank = 0;
+    const int own_end = node < num_receivers ? first[node + 1] : 0;
+    for (int e0 = node < num_receivers ? first[node] : 0; e0 < own_end; e0 += 32) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) f[q] = e0 + lane < own_end ? -edge_forces[3 * static_cast<size_t>(e0 + lane) + q] : 0.0;
+        add_by_rank(f, slots[warp], lane, rank, own);
     }
-    fx = warp_total(fx);
-    fy = warp_total(fy);
-    fz = warp_total(fz);
-    if (lane == 0) {
-        forces[3 * static_cast<size_t>(node)] = fx;
-        forces[3 * static_cast<size_t>(node) + 1] = fy;
-        forces[3 * static_cast<size_t>(node) + 2] = fz;
+    rank = 0;
+    const int end = source_offsets[node + 1];
+    for (int k0 = source_offsets[node]; k0 < end; k0 += 32) {
+        const size_t e = k0 + lane < end ? source_edges[k0 + lane] : 0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) f[q] = k0 + lane < end ? edge_forces[3 * e + q] : 0.0;
+        add_by_rank(f, slots[warp], lane, rank, own);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double total = warp_total(own[q]);
+        if (lane == 0) forces[3 * static_cast<size_t>(node) + q] = total;
     }
 }
 

@@ -38,6 +38,29 @@ __device__ __forceinline__ int2 edge_part(const int* __restrict__ first, int i, 
                      begin + static_cast<int>(static_cast<long>(n) * (part + 1) / parts));
 }
 
+// The same with the cuts counted in edges inside the cutoff, for the forward sums of the reproducible mode: which edges meet in
+// a part, and so the order of the sum, is then a matter of those edges alone and not of how many skin edges the list at hand
+// carries between them.  Every warp of the block walks the list by itself.
+__device__ __forceinline__ int2 active_edge_part(const int* __restrict__ first, const EdgeGeom* __restrict__ geom, float r_cut, int i,
+                                                 int part, int parts)
+{
+    const int begin = first[i], end = first[i + 1], lane = threadIdx.x & 31;
+    int active = 0;
+    for (int e = begin; e < end; e += 32) active += __popc(__ballot_sync(0xffffffffu, e + lane < end && geom[e + lane].r < r_cut));
+    const int from = static_cast<int>(static_cast<long>(active) * part / parts);
+    const int to = static_cast<int>(static_cast<long>(active) * (part + 1) / parts);
+    int2 range = make_int2(end, end);
+    for (int e = begin, before = 0; e < end; e += 32) {
+        const unsigned mask = __ballot_sync(0xffffffffu, e + lane < end && geom[e + lane].r < r_cut);
+        const int rank = (mask >> lane) & 1u ? before + __popc(mask & ((1u << lane) - 1u)) : -1;
+        const unsigned at_from = __ballot_sync(0xffffffffu, rank == from), at_to = __ballot_sync(0xffffffffu, rank == to);
+        if (at_from) range.x = e + __ffs(at_from) - 1;
+        if (at_to) range.y = e + __ffs(at_to) - 1;
+        before += __popc(mask);
+    }
+    return range;
+}
+
 // Adds up `count` rows of `width` floats over the blocks of a cluster and hands every sum once to store(row, value);
 // `mine` is this block's copy in dynamic shared memory, written by its threads before the call.
 template <typename Store>
@@ -761,7 +784,7 @@ l0_reverse_kernel(int num_nodes, int node0, int C_runtime, const int* __restrict
                              const float4* __restrict__ table4, const float* __restrict__ H1,                        \
                              const __grid_constant__ CouplingConstants cgc, float* __restrict__ Phi1,                \
                              const float* __restrict__ inv_scale, int pair_types,                                    \
-                             const float* __restrict__ given_harmonics = nullptr)                                    \
+                             const float* __restrict__ given_harmonics = nullptr, bool parts_by_active = false)      \
     {                                                                                                                \
         constexpr int NP = SXB_##NAME##_NUM_PATHS, NR = SXB_##NAME##_NUM_ROWS, NH = SXB_##NAME##_NUM_HIDDEN;          \
         constexpr int NE = SXB_##NAME##_NUM_LME;                                                                     \
@@ -770,7 +793,9 @@ l0_reverse_kernel(int num_nodes, int node0, int C_runtime, const int* __restrict
         const int local = blockIdx.x, i = node0 + local;                                                             \
         const int k = threadIdx.x;                                                                                   \
         const int F = NP * C;                                                                                        \
-        const int2 range = kParts ? edge_part(first, i, blockIdx.y, gridDim.y) : make_int2(first[i], first[i + 1]);  \
+        const int2 range = !kParts ? make_int2(first[i], first[i + 1])                                               \
+                           : parts_by_active ? active_edge_part(first, geom, grid.r_cut, i, blockIdx.y, gridDim.y)   \
+                                             : edge_part(first, i, blockIdx.y, gridDim.y);                           \
         const int begin = range.x, end = range.y;                                                                    \
         float acc[NR];                                                                                               \
         _Pragma("unroll") for (int r_ = 0; r_ < NR; ++r_) acc[r_] = 0.0f;                                            \

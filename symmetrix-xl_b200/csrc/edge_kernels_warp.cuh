@@ -113,9 +113,9 @@ struct PairLoad<2> {
 // ---------------------------------------------------------------------------------------------
 template <int kVec>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
-l0_forward_warp_kernel(int num_nodes, int node0, int parts, const int* __restrict__ first, const int* __restrict__ sources,
-                       const EdgeGeom* __restrict__ geom, const unsigned char* __restrict__ atype, int num_active,
-                       SplineGrid grid, const float* __restrict__ table, float* __restrict__ A0,
+l0_forward_warp_kernel(int num_nodes, int node0, int parts, bool parts_by_active, const int* __restrict__ first,
+                       const int* __restrict__ sources, const EdgeGeom* __restrict__ geom, const unsigned char* __restrict__ atype,
+                       int num_active, SplineGrid grid, const float* __restrict__ table, float* __restrict__ A0,
                        const float* __restrict__ inv_scale)
 {
     constexpr int C = 32 * kVec, F = 4 * C;
@@ -129,7 +129,8 @@ l0_forward_warp_kernel(int num_nodes, int node0, int parts, const int* __restric
     WarpChunk<false>& s = chunks[warp];
     const int k = lane * kVec;
     const int type_i = atype[i];
-    const int2 range = edge_part(first, i, part, parts);
+    const int2 range = parts_by_active && parts > 1 ? active_edge_part(first, geom, grid.r_cut, i, part, parts)
+                                                    : edge_part(first, i, part, parts);
     const int begin = range.x, end = range.y;
     float acc[16][kVec];
 #pragma unroll

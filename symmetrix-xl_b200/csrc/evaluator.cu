@@ -1018,16 +1018,20 @@ void Evaluator::run_pipeline(int phases)
     const float* inv1 = model_.a1_scaled ? inv_scale1_.ptr : nullptr;
     const DensityScale density0{model_.a0_scaled ? density0_table_.ptr : nullptr, inv_scale0_.ptr, dot0_.ptr, n_active};
     const DensityScale density1{model_.a1_scaled ? density1_table_.ptr : nullptr, inv_scale1_.ptr, dot1_.ptr, n_active};
-    const PartRules rules{num_sms_, C, model_.shape_id, static_cast<double>(num_edges_) / std::max(1, R)};
+    // The reproducible mode deals forward sums out by the receivers of the graph and a fixed list length, and by edges inside the
+    // cutoff (active_edge_part): neither the tile size nor the skin edges of the list at hand change the order of a sum.
+    const double mean_edges = static_cast<double>(num_edges_) / std::max(1, R);
+    const PartRules rules{num_sms_, C, model_.shape_id, mean_edges}, sum_rules{num_sms_, C, model_.shape_id, deterministic_ ? 100.0 : mean_edges};
+    auto sum_receivers = [&](int T) { return deterministic_ ? R : T; };
     auto l0_forward = [&](int t0, int T) {
-        const int parts = rules.l0_forward(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
+        const int parts = sum_rules.l0_forward(sum_receivers(T)), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
         const std::size_t part_bytes = parts > 1 ? static_cast<std::size_t>(kWarpsPerBlock) * 16 * C * sizeof(float) : 0;
         if (C == 128)
-            l0_forward_warp_kernel<4><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
+            l0_forward_warp_kernel<4><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, deterministic_, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         else if (C == 64)
-            l0_forward_warp_kernel<2><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
+            l0_forward_warp_kernel<2><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, deterministic_, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         else if (C == 32)
-            l0_forward_warp_kernel<1><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
+            l0_forward_warp_kernel<1><<<warp_grid, warp_threads, part_bytes, stream_>>>(T, t0, parts, deterministic_, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         else
             l0_forward_kernel<0><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         launches_ += 1;
@@ -1121,15 +1125,15 @@ void Evaluator::run_pipeline(int phases)
                 launches_ += 1;
                 span_end();
             } else {
-            const int forward_parts = rules.l1_forward(T);
+            const int forward_parts = sum_rules.l1_forward(sum_receivers(T));
             const std::size_t row_bytes = static_cast<std::size_t>(NE) * C * sizeof(float);   // S2: a set has fewer rows
             span_begin("l1_forward");
             if (model_.shape_id == 0)
                 SXB_LAUNCH_PARTS_BY_CHANNELS(l1_forward_kernel_S0, C, T, forward_parts, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
-                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr);
+                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr, deterministic_);
             else if (model_.shape_id == 1)
                 SXB_LAUNCH_PARTS_BY_CHANNELS(l1_forward_kernel_S1, C, T, forward_parts, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
-                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr);
+                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr, deterministic_);
             else {
                 // one launch per path set; the sets write disjoint components of Phi1
 #define SXB_SPLIT_FORWARD(SET)                                                                                            \
@@ -1397,8 +1401,8 @@ void Evaluator::run_pipeline(int phases)
         span_begin("finalize");
         if (deterministic_) {
             const long blocks = std::max<long>(blocks_for(std::max<long>(num_edges_, 1), kTotalsThreads), blocks_for(R, kTotalsThreads));
-            reduce_node_forces_kernel<<<blocks_for(static_cast<long>(ALL) * 32, 128), 128, 0, stream_>>>(ALL, R, first_.ptr, source_offsets_.ptr, source_edges_.ptr,
-                                                                                  edge_forces_.ptr, forces_.ptr);
+            reduce_node_forces_kernel<<<blocks_for(ALL, kNodeForceWarps), 32 * kNodeForceWarps, 0, stream_>>>(
+                ALL, R, first_.ptr, source_offsets_.ptr, source_edges_.ptr, edge_forces_.ptr, forces_.ptr);
             partial_totals_kernel<<<blocks, kTotalsThreads, 0, stream_>>>(num_edges_, R, geom_.ptr, edge_forces_.ptr, node_energies_.ptr,
                                                                           det_partials_.ptr);
             final_totals_kernel<<<1, 320, 0, stream_>>>(static_cast<int>(blocks), det_partials_.ptr, energy_slots_.ptr, virial_slots_.ptr);

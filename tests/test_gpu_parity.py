@@ -500,6 +500,34 @@ def test_reproducible_mode_gives_identical_bits(pkg, model_path, arch, zbl):
         scaled.calculate(pos, cell, types)
 
 
+@pytest.mark.parametrize("arch,channels", [("medium", 128), ("medium", 64), ("small", 32)])
+def test_reproducible_bits_do_not_depend_on_tiles_or_skin(pkg, model_path, arch, channels):
+    """Energies and forces of the reproducible mode are sums over the edges inside the cutoff, in list order: the number of
+    skin edges between them and the size of the tiles change no bit (one bin along each axis, so that every list has its edges
+    in the same order).  Tiled evaluations add the direct adjoint of M0 last and the untiled one first: their forces are
+    compared among themselves.  40 atoms are dealt out to parts."""
+    path = model_path(arch, seed=12, channels=channels)
+    pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 31)
+    pos = pos + 0.25 * cell.sum(axis=0) / 2
+    edges, results = set(), {}
+    for tile, skin in ((0, 0.5), (0, 0.0), (0, 0.9), (7, 0.5), (16, 0.2), (20, 0.5), (1, 0.0)):
+        ev = pkg.MACEB200(path)
+        ev.set_deterministic(True)
+        ev.set_tile_size(tile)
+        res = ev._prepare_periodic_factorized_graph(types, pos, cell, np.linalg.inv(cell), ev.r_cut + skin)
+        ev._compute_prepared_factorized_positions(res["generation"], pos)
+        edges.add(res["num_edges"])
+        forces = ev._reduce_atom_forces(len(pos), execution_graph_generation=res["generation"]).copy()
+        results.setdefault(tile > 0, []).append((ev.node_energies.copy(), ev.energy, ev.stage("H1_adj").copy(), forces))
+    assert len(edges) > 2
+    first = results[False][0]
+    for run in results[False] + results[True]:
+        assert np.array_equal(run[0], first[0]) and run[1] == first[1] and np.array_equal(run[2], first[2])
+    for runs in results.values():
+        for run in runs:
+            assert np.array_equal(run[3], runs[0][3])
+
+
 def test_nve_energy_conservation(pkg, model_path):
     """20 velocity-Verlet steps of 1 fs at 300 K: total energy is conserved to integrator accuracy."""
     path = model_path("small")
