@@ -377,15 +377,14 @@ l0_reverse_pair_kernel(int num_nodes, int node0, int parts, const int* __restric
     finish_warp_receiver(lane, i, out, rfx, rfy, rfz, vir);
 }
 
-// The same with one channel per lane (32 channels), in single floats.
-template <int kVec>
+// The same for 32 channels: one per lane, in single floats.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
 l0_reverse_warp_kernel(int num_nodes, int node0, int parts, const int* __restrict__ first, const int* __restrict__ sources,
                        const EdgeGeom* __restrict__ geom, const unsigned char* __restrict__ atype, int num_active,
                        SplineGrid grid, const float* __restrict__ table, const float* __restrict__ A0_adj, ForceOutputs out,
                        DensityScale density)
 {
-    constexpr int C = 32 * kVec, F = 4 * C;
+    constexpr int C = 32, F = 4 * C;
     __shared__ WarpChunk<true> chunks[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = blockIdx.x * kWarpsPerBlock + warp;
@@ -393,15 +392,14 @@ l0_reverse_warp_kernel(int num_nodes, int node0, int parts, const int* __restric
     if (local >= num_nodes) return;
     const int i = node0 + local;                            // graph-wide receiver index
     WarpChunk<true>& s = chunks[warp];
-    const int k = lane * kVec;
     const int type_i = atype[i];
     const int2 range = edge_part(first, i, slot % parts, parts);
     const int begin = range.x, end = range.y;
-    float adj[16][kVec];
+    float adj[16];
     {
-        const float* in = A0_adj + static_cast<size_t>(local) * 16 * C + k;
+        const float* in = A0_adj + static_cast<size_t>(local) * 16 * C + lane;
 #pragma unroll
-        for (int lm = 0; lm < 16; ++lm) VecLoad<kVec>::load(in + lm * C, adj[lm]);
+        for (int lm = 0; lm < 16; ++lm) adj[lm] = in[lm * C];
     }
     // with density scaling the stored adjoint refers to the scaled A0: dE/dA0_unscaled = adj / (1 + rho_i)
     float density_coef = 0.0f;
@@ -409,9 +407,7 @@ l0_reverse_warp_kernel(int num_nodes, int node0, int parts, const int* __restric
         const float scale = density.inv_scale[i];
         density_coef = density.dot[i] * scale;
 #pragma unroll
-        for (int lm = 0; lm < 16; ++lm)
-#pragma unroll
-            for (int v = 0; v < kVec; ++v) adj[lm][v] *= scale;
+        for (int lm = 0; lm < 16; ++lm) adj[lm] *= scale;
     }
     // per-lane partial sums over the edges this lane finishes (lane t owns edge t of every chunk)
     double rfx = 0.0, rfy = 0.0, rfz = 0.0;
@@ -426,31 +422,21 @@ l0_reverse_warp_kernel(int num_nodes, int node0, int parts, const int* __restric
             if (base < 0) continue;
             const float4 m = s.misc[t];
             const float x = m.x, xx = x * x, xxx = xx * x, x2 = 2.0f * x, xx3 = 3.0f * xx;
-            const float* c = table + base + k;
+            const float* c = table + base + lane;
             float y[16], ang[16];
             load16(s.y[t], y);
             float radial = 0.0f;
 #pragma unroll
             for (int l = 0; l < 4; ++l) {
-                float c0[kVec], c1[kVec], c2[kVec], c3[kVec];
-                VecLoad<kVec>::load(c + l * C, c0);
-                VecLoad<kVec>::load(c + F + l * C, c1);
-                VecLoad<kVec>::load(c + 2 * F + l * C, c2);
-                VecLoad<kVec>::load(c + 3 * F + l * C, c3);
+                const float c0 = c[l * C], c1 = c[F + l * C], c2 = c[2 * F + l * C], c3 = c[3 * F + l * C];
+                const float R = cubic(c0, c1, c2, c3, x, xx, xxx), dR = cubic_derivative(c1, c2, c3, x2, xx3);
+                float ya = 0.0f;
 #pragma unroll
-                for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) ang[lm] = 0.0f;
-#pragma unroll
-                for (int v = 0; v < kVec; ++v) {
-                    const float R = cubic(c0[v], c1[v], c2[v], c3[v], x, xx, xxx);
-                    const float dR = cubic_derivative(c1[v], c2[v], c3[v], x2, xx3);
-                    float ya = 0.0f;
-#pragma unroll
-                    for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) {
-                        ya = fmaf(y[lm], adj[lm][v], ya);
-                        ang[lm] = fmaf(R, adj[lm][v], ang[lm]);
-                    }
-                    radial = fmaf(dR, ya, radial);
+                for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) {
+                    ya = fmaf(y[lm], adj[lm], ya);
+                    ang[lm] = R * adj[lm];
                 }
+                radial = fmaf(dR, ya, radial);
             }
             float fx = radial * m.y, fy = radial * m.z, fz = radial * m.w;
             {

@@ -1131,10 +1131,15 @@ void Evaluator::run_pipeline(int phases)
             if (model_.shape_id == 0)
                 SXB_LAUNCH_PARTS_BY_CHANNELS(l1_forward_kernel_S0, C, T, forward_parts, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                                        reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr, deterministic_);
-            else if (model_.shape_id == 1)
-                SXB_LAUNCH_PARTS_BY_CHANNELS(l1_forward_kernel_S1, C, T, forward_parts, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
-                                       reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr, deterministic_);
-            else {
+            else if (model_.shape_id == 1) {
+                // hidden 0e+1o has no 32-channel build: its linears of 96 columns run on the FP32 fallback only
+                if (C == 128)
+                    SXB_LAUNCH_PARTS(l1_forward_kernel_S1<128>, (l1_forward_kernel_S1<128, false, true>), T, forward_parts, 128, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr, deterministic_);
+                else
+                    SXB_LAUNCH_PARTS(l1_forward_kernel_S1<0>, (l1_forward_kernel_S1<0, false, true>), T, forward_parts, C, row_bytes, stream_, T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
+                                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, coupling_, Phi1_.ptr, inv1, r1_pair_types_, nullptr, deterministic_);
+            } else {
                 // one launch per path set; the sets write disjoint components of Phi1
 #define SXB_SPLIT_FORWARD(SET)                                                                                            \
                 SXB_LAUNCH_PARTS(l1_forward_split_kernel_S2_##SET<128>, (l1_forward_split_kernel_S2_##SET<128, true>), T, forward_parts, 128, row_bytes, stream_, T, t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, \
@@ -1380,7 +1385,7 @@ void Evaluator::run_pipeline(int phases)
                 else if (C == 64)
                     l0_reverse_pair_kernel<2><<<warp_grid, warp_threads, kWarpsPerBlock * sizeof(WarpPairChunk), stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else if (C == 32)
-                    l0_reverse_warp_kernel<1><<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
+                    l0_reverse_warp_kernel<<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else
                     l0_reverse_kernel<0><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
             }
