@@ -547,9 +547,9 @@ def test_nve_energy_conservation(pkg, model_path):
 @pytest.mark.parametrize("arch,copies", [("medium", (2, 1, 1)), ("medium", (4, 2, 2)), ("small", (4, 2, 1)), ("large", (2, 2, 1))])
 def test_parts_of_a_receiver_add_up(pkg, model_path, arch, copies):
     """A receiver's edges are dealt to more blocks and warps, and the linears' column tiles get narrower, the fewer receivers
-    there are: a cell of 38 atoms (most parts)
-    against the oracle, and its periodic copies (fewer parts, down to one) against the cell.  Bounds: those of the oracle
-    comparison; the copies differ from the cell by the order of float sums alone."""
+    there are: a cell of 38 atoms (most parts) against the oracle, and its periodic copies (fewer parts; undivided receivers
+    are in test_every_division_of_receivers) against the cell.  Bounds: those of the oracle comparison; the copies differ from
+    the cell by the order of float sums alone."""
     from oracle import mace_numpy, neighbor
 
     path = model_path(arch, 31)
@@ -592,13 +592,17 @@ def test_contraction_runs_of_elements(pkg, model_path, arch, counts):
     assert np.abs(ev.node_energies - energies).max() <= TOL_E
     got = ev._reduce_atom_forces(n, execution_graph_generation=res["generation"])
     assert np.abs(got - forces).max() <= TOL_F * max(1.0, np.abs(forces).max())
+    for name in ("M0", "M1", "A1_adj", "A0_adj"):      # what the four contraction kernels leave
+        want = oracle.stage[name]
+        assert np.abs(ev.stage(name).reshape(want.shape) - want).max() <= 2e-5 * max(1.0, np.abs(want).max()), name
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("channels,options", [(128, {}), (64, {}), (64, {"a0_scaled": True, "a1_scaled": True}), (128, {"agnesi": True})])
 def test_layer1_gradient_widths_and_odd_edge_counts(pkg, model_path, channels, options):
-    """The layer-1 gradient takes two edges at a time from chunks of 64 list edges: receivers without, with one, with an odd
-    number and with more than a chunk of active edges, at both compiled widths, against the oracle."""
+    """The layer-1 gradient takes two edges at a time: receivers without, with one and with an odd number of active edges, and a
+    dense cell whose 120 list edges a receiver are dealt to eight parts, at both compiled widths, against the oracle.  (Chunks
+    filled more than once: test_every_division_of_receivers.)"""
     from oracle import mace_numpy, neighbor
 
     path = model_path("medium", 35, channels=channels, **options)
