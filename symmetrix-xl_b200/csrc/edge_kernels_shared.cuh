@@ -6,11 +6,11 @@
 // packed instructions of sm_100a and kEdges edges of the receiver at a time, and every adjoint it reads feeds two operations
 // per edge.  All paths of a structure fit one kernel, whatever their number of rows, so the source features, the edge state
 // and the force reduction are paid once per edge instead of once per path set.  Rows without a coupling term are left out.
-// Teams of kC / 64 warps share a receiver.  5,000 receivers, 500,000 list edges, 128 channels, this / the register form:
-// hidden 0e+1o 0.941 / 1.060 ms, 0e+1o+2e 2.16 / 2.57 ms (three launches).  Shapes tried for 0e+1o, (teams, blocks per SM,
-// edges): (2, 3, 2) 0.941, (4, 2, 1) 1.005, (4, 1, 2) 1.089; for 0e+1o+2e: (6, 1, 1) 2.157, (4, 1, 2) 2.153, (8, 1, 1) 2.23.
-// Now bound by the shared-memory data pipe (77 % of its wavefronts at twelve warps per SM).  The reproducible mode keeps the register form,
-// which leaves its records faster (1,080 receivers: 0.295 against 0.469 ms).  Registers: 168 at 128 channels (24 bytes spilled),
+// Teams of kC / 64 warps share a receiver.  Register form / this, 128 channels: hidden 0e+1o, 5,000 atoms 1.003 / 0.898 ms;
+// 0e+1o+2e, 20,000 atoms 10.47 (three launches) / 8.88 ms.  Other shapes (teams, blocks per SM, edges) against (2, 3, 2) for
+// 0e+1o: (4, 2, 1) +7 %, (4, 1, 2) +16 %; against (6, 1, 1) for 0e+1o+2e: (4, 1, 2) 0 %, (8, 1, 1) +3 %.
+// Now bound by the shared-memory data pipe (77 % of its wavefronts at twelve warps per SM).  The reproducible mode keeps the
+// register form, which leaves its records faster (1,080 receivers: 0.295 against 0.469 ms).  Registers: 168 at 128 channels (24 bytes spilled),
 // three blocks of four warps; at 64 channels the edge state, which does not shrink with the width, leaves room for four blocks
 // of two warps, so a thread may have 248: 5,000 receivers 0.451 ms, with the 168 of six blocks that never fit 0.599 ms.
 //

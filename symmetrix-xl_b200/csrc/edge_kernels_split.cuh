@@ -5,7 +5,9 @@
 // registers and writes only the outputs that set feeds - every output component belongs to exactly
 // one path, so the sets write disjoint parts of Phi1.
 // Thread mapping, edge chunking and the math are those of edge_kernels.cuh (layer 1 forward,
-// libsymmetrix/source/mace.cpp:2023-2083).
+// libsymmetrix/source/mace.cpp:2023-2083).  The cluster builds (kParts) index lme_of at run time in their store, which keeps it
+// in local memory (48 to 160 bytes a thread); the three launches take 101 / 45 us at 1 / 8 parts for 40 receivers, 105 / 101 at
+// 1 / 2 for 160.
 #pragma once
 
 #include "edge_kernels.cuh"

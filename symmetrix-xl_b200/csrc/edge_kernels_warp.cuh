@@ -268,9 +268,9 @@ struct alignas(16) WarpPairChunk {
     float force[kWarpChunk][3];
 };
 
-// Layer-0 gradient, kVec channels per lane as kVec / 2 pairs in the packed instructions of sm_100a.  Bound by instruction
-// issue (380 instructions per edge in the one-float form); 5,000 receivers,
-// 128 channels: 286 / 243 us, 40 receivers 21 / 18 us.  Kernel time goes with the coefficient rows (8 KB per edge) and issue.
+// Layer-0 gradient, kVec channels per lane as kVec / 2 pairs in the packed instructions of sm_100a.  Waits on its coefficient
+// rows (8 KB per edge from L2) at 2.8 warps per scheduler, 0.41 instructions per cycle.  One-float form / pairs, 128 channels:
+// 5,000 receivers 286 / 243 us, 40 receivers 21 / 18 us.
 template <int kVec>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
 l0_reverse_pair_kernel(int num_nodes, int node0, int parts, const int* __restrict__ first, const int* __restrict__ sources,

@@ -16,7 +16,8 @@ namespace sxb {
 // channel pairs and the compiled structure is straight-line code on them (contraction_lines in gen_structures.py: monomials
 // grouped by their first two factors).  Weights are laid out [element][term][channel].  A block covers consecutive nodes and
 // 32 channels, half a warp per node; it first copies the [term][32] weight slice of its nodes' element to shared
-// memory.  Bound by instruction issue.  5,000 nodes, 128 channels, hidden 0e+1o, one channel per thread with every monomial on
+// memory.  Bound by the FMA pipe in turn with the weight reads (gradient of M0: 0.42 instructions per cycle and scheduler, the
+// math pipe its first stall).  5,000 nodes, 128 channels, hidden 0e+1o, one channel per thread with every monomial on
 // its own / this form: M0 62 / 48, its gradient 118 / 62, M1 27 / 22, its gradient 36 / 27 us; 40 nodes: gradient of M0 27 / 15.
 
 // Density-scaled models: dot[node] += sum over (lm, channels of this half warp) of A_adj * A, the quantity
@@ -43,8 +44,9 @@ __device__ __forceinline__ void stage_poly_weights(float4* __restrict__ dst, con
     __syncthreads();
 }
 
-// Walks the nodes of one block, two per warp and pass, one run of equal elements after the other (nodes are sorted by
-// element: most blocks are one run).  CALL sees node, valid (false for the lanes of a node past the end, which repeat the
+// Walks the nodes of one block, two per warp and pass, one run of equal elements after the other.  Receivers are sorted by
+// element (the counting sort of Evaluator::install_graph), so most blocks are one run, and the count of equal elements is the
+// length of the run.  CALL sees node, valid (false for the lanes of a node past the end, which repeat the
 // last one), k (first channel of the pair) and w (weight pairs of a term at w[term * 16]).
 #define SXB_POLY_WALK(NT, CALL)                                                                                     \
     extern __shared__ float4 w_s[];                                                                                 \

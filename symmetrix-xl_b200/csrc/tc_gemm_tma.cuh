@@ -14,7 +14,7 @@
 //     write tile i (tensor memory -> registers -> a small transposing tile in shared memory ->
 //     whole 128-byte row segments) while the tensor core already works on tile i + 1.
 // A row tile holds floor(128 / components) whole nodes (128, 126, 125 or 126 rows); the remaining
-// accumulator lanes are never stored.  A column tile is min(N, 128) wide.
+// accumulator lanes are never stored.  A column tile is 128, 64 or 32 columns wide, as the launch chooses.
 // Thread roles: warps 0-3 residual, warps 4-7 epilogue, warp 8 lane 0 tcgen05.mma issue (warp 8 also
 // owns the tensor-memory allocation), warp 9 lane 0 weight TMA, warp 10 lane 0 activation TMA.  The
 // issuing thread is the narrow point of such a pipeline (every mbarrier or tcgen05 instruction costs
@@ -48,7 +48,7 @@ struct alignas(64) Tc3Problem {
     int M, N, K;             // logical rows (nodes x components), outputs, K % 32 == 0
     int accumulate;
     int rows_per_tile, nodes_per_tile;
-    int n_tile, n_tiles;     // min(N, 128) in {32, 64, 128}; N % n_tile == 0
+    int n_tile, n_tiles;     // 32, 64 or 128; N % n_tile == 0
     int m_tiles;
     int tile_begin;          // first work item of this problem (items are m-major: m_tile * n_tiles + n)
 };
