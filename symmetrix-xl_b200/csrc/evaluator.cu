@@ -807,6 +807,9 @@ CUtensorMap make_weight_map(const float* device_ptr, int n, int k, int n_tile)
 }
 }  // namespace
 
+namespace {
+constexpr int tc_width(int index) { return 32 * (index + 1); }   // columns of a tile: 32, 64, 96, 128
+}
 // Splits W [rows][cols] into a TF32-exact high part (low 13 mantissa bits cleared) and the
 // residual, in both orientations the tensor-core kernel needs ([N][K], K contiguous).
 void Evaluator::upload_split(SplitWeight& out, const float* w, int rows, int cols)
@@ -842,8 +845,8 @@ void Evaluator::upload_split(SplitWeight& out, const float* w, int rows, int col
     // forward product: N = cols, K = rows; reverse product: N = rows, K = cols
     if (rows % kTcChunk != 0 || cols % kTcChunk != 0)
         throw std::invalid_argument("Linear extents must be multiples of 32 for the tensor-core kernel.");
-    for (int w = 0; w < 3; ++w) {
-        const int width = 32 << w;
+    for (int w = 0; w < kTcWidths; ++w) {
+        const int width = tc_width(w);
         out.map_fwd_hi[w] = make_weight_map(out.fwd_hi.ptr, cols, rows, std::min(cols, width));
         out.map_fwd_lo[w] = make_weight_map(out.fwd_lo.ptr, cols, rows, std::min(cols, width));
         out.map_rev_hi[w] = make_weight_map(out.rev_hi.ptr, rows, cols, std::min(rows, width));
@@ -884,19 +887,19 @@ void Evaluator::launch_tc(const std::vector<TcCall>& calls)
         }
         return;
     }
-    // Widest column tile of {128, 64, 32} not above `width` that divides N, as an index into the tensor maps; -1: none
+    // Widest column tile of {128, 96, 64, 32} not above `width` that divides N, as an index into the tensor maps; -1: none
     // (N = 32 or a multiple of 64 has one, other widths go to the first tcgen05 kernel and its checks).
     auto tile_index = [](int N, int width) {
         if (N != 32 && N % 64 != 0) return -1;
-        for (int w = 2; w >= 0; --w)
-            if ((32 << w) <= width && N % (32 << w) == 0) return w;
+        for (int w = kTcWidths - 1; w >= 0; --w)
+            if (tc_width(w) <= width && N % tc_width(w) == 0) return w;
         return -1;
     };
     auto work_items = [&](int width) {
         long items = 0;
         for (const auto& c : calls) {
             const int N = c.reverse ? c.w->rows : c.w->cols, nodes = kTcRows / c.a_rows.components;
-            items += static_cast<long>((std::max(c.num_nodes, 0) + nodes - 1) / nodes) * (N / (32 << tile_index(N, width)));
+            items += static_cast<long>((std::max(c.num_nodes, 0) + nodes - 1) / nodes) * (N / tc_width(tile_index(N, width)));
         }
         return items;
     };
@@ -919,22 +922,19 @@ void Evaluator::launch_tc(const std::vector<TcCall>& calls)
                 const auto& c = calls[next];
                 if (c.num_nodes <= 0) continue;
                 Tc3Problem& p = batch.problem[count];
-                p.N = c.reverse ? c.w->rows : c.w->cols;
+                const int N = c.reverse ? c.w->rows : c.w->cols;
                 p.K = c.reverse ? c.w->cols : c.w->rows;
                 if (p.K % kTcChunk != 0) throw std::invalid_argument("Linear extents are not supported by the tensor-core kernel.");
-                const int w = tile_index(p.N, width);
-                p.n_tile = 32 << w;
-                p.n_tiles = p.N / p.n_tile;
+                const int w = tile_index(N, width);
+                p.n_tile = tc_width(w);
+                p.n_tiles = N / p.n_tile;
                 p.nodes_per_tile = kTcRows / c.a_rows.components;
                 p.rows_per_tile = p.nodes_per_tile * c.a_rows.components;
                 p.map_a = make_activation_map(c.A, c.a_rows, c.first_node, c.num_nodes, p.K, p.nodes_per_tile);
                 p.map_hi = c.reverse ? c.w->map_rev_hi[w] : c.w->map_fwd_hi[w];
                 p.map_lo = c.reverse ? c.w->map_rev_lo[w] : c.w->map_fwd_lo[w];
-                p.C = c.C;
-                p.bias = c.bias;
-                p.c_rows = c.c_rows;
-                p.first_node = c.first_node;
-                p.M = c.num_nodes * c.a_rows.components;
+                p.map_c = make_activation_map(c.C, c.c_rows, c.first_node, c.num_nodes, N, p.nodes_per_tile);
+                p.bias = c.accumulate ? nullptr : c.bias;
                 p.accumulate = c.accumulate ? 1 : 0;
                 p.m_tiles = (c.num_nodes + p.nodes_per_tile - 1) / p.nodes_per_tile;
                 p.tile_begin = tiles;

@@ -157,11 +157,12 @@ private:
     DeviceBuffer<float> readout1_, readout2_w1_, readout2_w2_;
     // the same weights split into TF32-exact high part and residual, stored [N][K] (K contiguous)
     // for the product with W ("fwd", C = A W) and with W^T ("rev", C = A W^T)
+    static constexpr int kTcWidths = 4;
     struct SplitWeight {
         DeviceBuffer<float> fwd_hi, fwd_lo, rev_hi, rev_lo, full;
         int rows = 0, cols = 0;   // W is [rows = K of fwd][cols = N of fwd]
-        // tensor maps of the four matrices, box [min(N, width)][32]; width 32, 64, 128 at index 0, 1, 2
-        CUtensorMap map_fwd_hi[3], map_fwd_lo[3], map_rev_hi[3], map_rev_lo[3];
+        // tensor maps of the four matrices, box [min(N, width)][32]; width 32, 64, 96, 128 at index 0 to 3
+        CUtensorMap map_fwd_hi[kTcWidths], map_fwd_lo[kTcWidths], map_rev_hi[kTcWidths], map_rev_lo[kTcWidths];
     };
     SplitWeight s_h1_[4], s_a1_[4], s_h2_m1_;
     std::vector<SplitWeight> s_h2_skip_;
