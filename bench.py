@@ -39,6 +39,10 @@ PARITY_ATOM_LIMIT = 1_500_000   # largest system the N > 1 runs re-evaluate on o
 SEED = 17
 # algorithmic work of the reference's formulation per (edge, channel)
 FLOP_PER_EDGE_CHANNEL = {"l0_forward": 56, "l0_reverse": 284, "l1_forward": 408, "l1_reverse": 850}
+# layer 0 on the 64 functions of the radial network's last hidden layer, per (edge, function): value and 16 harmonics; value, slope and
+# the two products with 16 adjoints (the linears to and from A0 are the stages gemm_a0 and gemm_a0_reverse)
+BASIS_FUNCTIONS = 64
+FLOP_PER_EDGE_FUNCTION = {"l0_forward": 38, "l0_reverse": 74}
 
 
 def _peaks():
@@ -138,12 +142,17 @@ def edge_kernel_roofline(ev, stage_ms, num_edges, active_edges, n, measured, hbm
     l2_bytes_per_edge = {"l0_forward": 16 * 4 * C, "l0_reverse": 16 * 4 * C,
                          "l1_forward": 16 * ev.num_paths * C + 4 * num_hidden * C,
                          "l1_reverse": 16 * ev.num_paths * C + 8 * num_hidden * C}
+    flops_per_edge = {name: flop * C for name, flop in FLOP_PER_EDGE_CHANNEL.items()}
+    if "gemm_a0" in stage_ms:
+        for name, flop in FLOP_PER_EDGE_FUNCTION.items():
+            flops_per_edge[name] = flop * BASIS_FUNCTIONS
+            l2_bytes_per_edge[name] = 16 * BASIS_FUNCTIONS
     kernels = {}
     for name in FLOP_PER_EDGE_CHANNEL:
         if name not in stage_ms:
             continue
         seconds = stage_ms[name] * 1e-3
-        flops = FLOP_PER_EDGE_CHANNEL[name] * active_edges * C
+        flops = flops_per_edge[name] * active_edges
         hbm_bytes = num_edges * 20 + n * node_rows[name] * C * 4
         l2_bytes = l2_bytes_per_edge[name] * active_edges
         kernels[name] = {"ms": stage_ms[name], "fp32_tflops": flops / seconds / 1e12,
@@ -152,7 +161,7 @@ def edge_kernel_roofline(ev, stage_ms, num_edges, active_edges, n, measured, hbm
                          "l2_gbs": l2_bytes / seconds / 1e9, "l2_frac": l2_bytes / seconds / 1e9 / measured["l2_read_gbs"]}
     dom = kernels[dominant]
     alg_bytes = num_edges * 20 + n * node_rows[dominant] * C * 4
-    alg_flops = FLOP_PER_EDGE_CHANNEL[dominant] * active_edges * C
+    alg_flops = flops_per_edge[dominant] * active_edges
     # DRAM bytes of one launch (dram__bytes_read.sum + dram__bytes_write.sum) from the tracked ncu
     # summary of this kernel and workload, when one exists
     traffic = None

@@ -154,6 +154,63 @@ __device__ __forceinline__ void spline_point(const SplineGrid& g, float r, int& 
     }
 }
 
+// The edges of every receiver inside the cutoff, written by the geometry kernels along with the records: edges[first[i] ..] in
+// list order, which is by source type where the graph distinguishes types; ends[i * types + a] is the end of type a's run.
+// The list's skin is a quarter of its edges; a kernel that deals edges to lanes wants to know the others beforehand.
+struct ActiveEdges {
+    int* edges;
+    int* ends;
+    int types;                        // at most 32
+    const unsigned char* atype;
+    float cutoff;
+};
+
+// A warp's place in the lists of its receiver: add() for every 32 edges of the list in order, all lanes together.
+struct ActiveEdgeWriter {
+    const ActiveEdges& out;
+    int receiver, begin, lane, total = 0, mine = 0;   // lane a < types counts the edges of type a
+    __device__ __forceinline__ void add(bool active, int e, int source)
+    {
+        const unsigned mask = __ballot_sync(0xffffffffu, active);
+        if (active) out.edges[begin + total + __popc(mask & ((1u << lane) - 1u))] = e;
+        total += __popc(mask);
+        if (out.types > 1) {
+            const int type = active ? out.atype[source] : -1;
+            for (int a = 0; a < out.types; ++a) {
+                const unsigned of_type = __ballot_sync(0xffffffffu, type == a);
+                if (lane == a) mine += __popc(of_type);
+            }
+        }
+    }
+    __device__ __forceinline__ void finish()
+    {
+        int sum = out.types > 1 ? mine : total;
+        if (out.types > 1)
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, sum, offset);
+                if (lane >= offset) sum += below;
+            }
+        if (lane < out.types) out.ends[static_cast<size_t>(receiver) * out.types + lane] = begin + sum;
+    }
+};
+
+// The lists alone, from the records of caller-supplied edge vectors.  One warp per receiver.
+static __global__ void active_edges_kernel(int num_nodes, const int* __restrict__ first, const int* __restrict__ sources,
+                                           const EdgeGeom* __restrict__ geom, const ActiveEdges active)
+{
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (warp >= num_nodes) return;
+    const int begin = first[warp], end = first[warp + 1];
+    ActiveEdgeWriter writer{active, warp, begin, lane};
+    for (int e0 = begin; e0 < end; e0 += 32) {
+        const int e = e0 + lane;
+        writer.add(e < end && geom[e].r < active.cutoff, e, e < end ? sources[e] : 0);
+    }
+    writer.finish();
+}
+
 // ---------------------------------------------------------------------------------------------
 // Per-step geometry: xyz_ij = r_j - r_i + shift * cell in double, then the float record.
 // One warp per receiver, lanes over its edges.
@@ -161,7 +218,7 @@ static __global__ void geometry_from_positions_kernel(int num_nodes, const int* 
                                                const int* __restrict__ sources, const int* __restrict__ shifts,
                                                const double* __restrict__ positions, const int* __restrict__ original,
                                                const double* __restrict__ cell, EdgeGeom* __restrict__ geom,
-                                               int* __restrict__ error_flag)
+                                               int* __restrict__ error_flag, const ActiveEdges active)
 {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -169,8 +226,10 @@ static __global__ void geometry_from_positions_kernel(int num_nodes, const int* 
     const int oi = original[warp];
     const double xi = positions[3 * oi], yi = positions[3 * oi + 1], zi = positions[3 * oi + 2];
     const int begin = first[warp], end = first[warp + 1];
-    for (int e = begin + lane; e < end; e += 32) {
-        const int oj = original[sources[e]];
+    ActiveEdgeWriter writer{active, warp, begin, lane};
+    for (int e0 = begin; e0 < end; e0 += 32) {
+        const int e = min(e0 + lane, end - 1), source = sources[e];   // the lanes beyond the end repeat its last edge
+        const int oj = original[source];
         double dx = positions[3 * oj] - xi, dy = positions[3 * oj + 1] - yi, dz = positions[3 * oj + 2] - zi;
         if (shifts != nullptr) {   // graphs without periodic shifts (explicit ghost atoms, open systems): plain differences
             const size_t se = 3 * static_cast<size_t>(e);
@@ -187,7 +246,9 @@ static __global__ void geometry_from_positions_kernel(int num_nodes, const int* 
         g.uz = static_cast<float>(dz / r);
         g.r = static_cast<float>(r);
         geom[e] = g;
+        writer.add(e0 + lane < end && g.r < active.cutoff, e, source);
     }
+    writer.finish();
 }
 
 // Per-step geometry from a reference state (graphs built by the caller without integer shifts):
@@ -202,7 +263,7 @@ __global__ void geometry_from_reference_kernel(int num_nodes, const int* __restr
                                                const double* __restrict__ reference, const double* __restrict__ reference_xyz,
                                                const int* __restrict__ edge_map, const double* __restrict__ cell,
                                                const double* __restrict__ inv_cell, int pbc_mask, EdgeGeom* __restrict__ geom,
-                                               int* __restrict__ error_flag)
+                                               int* __restrict__ error_flag, const ActiveEdges active)
 {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -222,9 +283,11 @@ __global__ void geometry_from_reference_kernel(int num_nodes, const int* __restr
     double fi[3];
     displacement(original[warp], fi);
     const int begin = first[warp], end = first[warp + 1];
-    for (int e = begin + lane; e < end; e += 32) {
+    ActiveEdgeWriter writer{active, warp, begin, lane};
+    for (int e0 = begin; e0 < end; e0 += 32) {
+        const int e = min(e0 + lane, end - 1), source = sources[e];
         double fj[3];
-        displacement(original[sources[e]], fj);
+        displacement(original[source], fj);
         const size_t o = 3 * static_cast<size_t>(edge_map[e]);
         double dx, dy, dz;
         if (kFractional) {
@@ -247,7 +310,9 @@ __global__ void geometry_from_reference_kernel(int num_nodes, const int* __restr
         g.uz = static_cast<float>(dz / r);
         g.r = static_cast<float>(r);
         geom[e] = g;
+        writer.add(e0 + lane < end && g.r < active.cutoff, e, source);
     }
+    writer.finish();
 }
 
 // Geometry from caller-supplied edge vectors (original edge order == internal edge order of

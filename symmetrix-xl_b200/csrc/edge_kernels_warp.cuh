@@ -10,7 +10,7 @@
 
 #include <type_traits>
 
-#include "edge_kernels_shared.cuh"
+#include "edge_kernels_pairs.cuh"
 
 namespace sxb {
 
@@ -257,7 +257,7 @@ __device__ __forceinline__ void finish_warp_receiver(int lane, int i, const Forc
 }
 
 // ---------------------------------------------------------------------------------------------
-// Edge state of the gradient: harmonics as pairs (Y, Y) and gradients per component, the layout of edge_kernels_shared.cuh.
+// Edge state of the gradient: harmonics as pairs (Y, Y) and gradients per component, the layout of edge_kernels_pairs.cuh.
 struct alignas(16) WarpPairChunk {
     float2 y[kWarpChunk][kPairSlots];
     float g[kWarpChunk][kGradSlots];
@@ -319,7 +319,7 @@ l0_reverse_pair_kernel(int num_nodes, int node0, int parts, const int* __restric
                 const int type_j = atype[j];
                 base = ((type_i * num_active + type_j) * grid.intervals + interval) * 4 * F;
                 s.misc[lane] = make_float4(x, g.ux, g.uy, g.uz);
-                fill_pair_harmonics(g, s.y[lane], s.g[lane]);
+                fill_pair_harmonics<true>(g, s.y[lane], s.g[lane]);
                 s.len[lane] = g.r;
                 s.dens[lane] = density.table != nullptr
                                    ? scalar_spline_derivative(density.table, (type_i * density.types + (density.types > 1 ? type_j : 0)) * grid.intervals + interval, x)

@@ -16,9 +16,9 @@
 
 #include "deterministic_kernels.cuh"
 #include "edge_kernels.cuh"
-#include "edge_kernels_shared.cuh"
+#include "edge_kernels_pairs.cuh"
 #include "edge_kernels_split.cuh"
-#include "edge_kernels_warp.cuh"
+#include "edge_kernels_basis.cuh"
 #include "graph_kernels.cuh"
 #include "node_kernels.cuh"
 #include "part_rules.hpp"
@@ -179,21 +179,20 @@ Evaluator::Evaluator(const std::string& json_path, int device_ordinal, const std
     SXB_ALLOW_POLY_SMEM(m0_reverse_kernel_##NAME, SXB_##NAME##_M0_NUM_TERMS);                                           \
     SXB_ALLOW_POLY_SMEM(m1_forward_kernel_##NAME, SXB_##NAME##_M1_NUM_TERMS);                                           \
     SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_##NAME, SXB_##NAME##_M1_NUM_TERMS)
-#define SXB_ALLOW_SHARED_ROWS(NAME, WIDTH)                                                                               \
-    SXB_CUDA(cudaFuncSetAttribute(l1_reverse_shared_kernel_##NAME<WIDTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                  static_cast<int>(shared_rows_bytes(SXB_##NAME##_NUM_ROWS, WIDTH))))
+#define SXB_ALLOW_PAIR_CHUNK(NAME, WIDTH)                                                                                \
+    SXB_CUDA(cudaFuncSetAttribute(l1_reverse_pair_kernel_##NAME<WIDTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pair_dynamic_bytes(WIDTH))))
     if (model_.shape_id == 0) {
         SXB_ALLOW_POLY_SMEM_SHAPE(S0);
     } else if (model_.shape_id == 1) {
         SXB_ALLOW_POLY_SMEM_SHAPE(S1);
-        if (C == 128) SXB_ALLOW_SHARED_ROWS(S1, 128);
-        if (C == 64) SXB_ALLOW_SHARED_ROWS(S1, 64);
+        if (C == 128) SXB_ALLOW_PAIR_CHUNK(S1, 128);
+        if (C == 64) SXB_ALLOW_PAIR_CHUNK(S1, 64);
     } else {
         SXB_ALLOW_POLY_SMEM_SHAPE(S2);
-        SXB_ALLOW_SHARED_ROWS(S2, 128);
+        SXB_ALLOW_PAIR_CHUNK(S2, 128);
     }
 #undef SXB_ALLOW_POLY_SMEM_SHAPE
-#undef SXB_ALLOW_SHARED_ROWS
+#undef SXB_ALLOW_PAIR_CHUNK
     constexpr int pair_chunk_bytes = kWarpsPerBlock * sizeof(WarpPairChunk);
     if (C == 128) SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_chunk_bytes));
     if (C == 64) SXB_CUDA(cudaFuncSetAttribute(l0_reverse_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_chunk_bytes));
@@ -230,7 +229,7 @@ Evaluator::~Evaluator()
     if (host_stage_) cudaFreeHost(host_stage_);
 }
 
-void Evaluator::prepare_active_types(const std::vector<int>& node_types)
+void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num_receivers)
 {
     std::vector<int> requested(node_types);
     std::sort(requested.begin(), requested.end());
@@ -239,12 +238,36 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types)
     for (int t : requested)
         if (t < 0 || t >= model_.num_elements) throw std::invalid_argument("MACE active type index is out of range.");
     if (requested.size() > 255) throw std::invalid_argument("More than 255 active element types.");
-    if (requested == active_types_) return;
-    active_types_ = requested;
-    const auto table = fold_r0_table(model_, active_types_);
-    if (table.size() > static_cast<std::size_t>(std::numeric_limits<int>::max()))
-        throw std::length_error("Layer-0 spline table exceeds 32-bit indexing; too many active element types.");
-    upload(r0_table_, table, stream_);
+    const int types = static_cast<int>(requested.size()), L = model_.l_max + 1;
+    const bool changed = requested != active_types_;
+    if (changed) {
+        active_types_ = requested;
+        basis_ready_ = table_ready_ = false;
+    }
+    // layer 0 on the functions of the radial network's last hidden layer, or on the folded table of every ordered pair: each
+    // built when a graph first asks for it
+    basis_layer0_ = (model_.channels == 128 || model_.channels == 64) && radial_basis_width(model_, "R0") == kBasis
+                    && PartRules{num_sms_, model_.channels, model_.shape_id, 0.0}.layer0_on_basis(num_receivers, types);
+    if (basis_layer0_ && !basis_ready_) {
+        upload(basis_table_, build_r0_basis(model_, active_types_, &basis_pair_types_, false), stream_);
+        upload(basis_steps_, build_r0_basis(model_, active_types_, &basis_pair_types_, true), stream_);
+        s_a0_.resize(static_cast<std::size_t>(types) * L);
+        for (int a = 0; a < types; ++a)
+            for (int l = 0; l < L; ++l)
+                upload_split(s_a0_[a * L + l], fold_r0_mixing(model_, active_types_, a, l).data(), types * kBasis, model_.channels);
+        basis_ready_ = true;
+    }
+    if (!basis_layer0_ && !table_ready_) {
+        const auto table = fold_r0_table(model_, active_types_);
+        if (table.size() > static_cast<std::size_t>(std::numeric_limits<int>::max()))
+            throw std::length_error("Layer-0 spline table exceeds 32-bit indexing; too many active element types.");
+        upload(r0_table_, table, stream_);
+        table_ready_ = true;
+    }
+    if (!changed) {
+        SXB_CUDA(cudaStreamSynchronize(stream_));
+        return;
+    }
     {
         if (!model_.single_layer) {
             int pairs = 1;
@@ -290,7 +313,7 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     num_nodes_ = num_nodes;
     num_edges_ = num_edges;
     has_shifts_ = has_shifts;
-    prepare_active_types(node_types);
+    prepare_active_types(node_types, num_receivers);
     std::vector<int> type_to_active(model_.num_elements, -1);
     for (std::size_t a = 0; a < active_types_.size(); ++a) type_to_active[active_types_[a]] = static_cast<int>(a);
     // internal order: receivers stably grouped by element (a counting sort), feature-only nodes after them
@@ -335,7 +358,7 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     temp.reserve(temp_bytes);
     cub::DeviceScan::ExclusiveSum(temp.ptr, temp_bytes, counts.ptr, first_.ptr, R + 1, stream_);
     permute_graph_kernel<<<blocks_for(static_cast<long>(R) * 32, 256), 256, 0, stream_>>>(
-        R, original_.ptr, internal_of_.ptr, first_caller_.ptr, sources_caller_.ptr,
+        R, edge_types(), atype_.ptr, original_.ptr, internal_of_.ptr, first_caller_.ptr, sources_caller_.ptr,
         has_shifts ? shifts_caller_.ptr : nullptr, first_.ptr, sources_.ptr, has_shifts ? shifts_.ptr : nullptr, edge_map_.ptr);
     launches_ += 1;
     SXB_CUDA(cudaGetLastError());
@@ -346,8 +369,11 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     const std::size_t N = num_receivers, ALL = num_nodes, C = model_.channels, NH = model_.num_hidden, NE = model_.num_lme;
     const std::size_t T = static_cast<std::size_t>(tile_capacity());
     geom_.reserve_with_slack(num_edges);
+    active_edges_.reserve_with_slack(num_edges);
+    active_ends_.reserve(N * edge_types());
     A0_.reserve(T * 16 * C);
     A0_adj_.reserve(T * 16 * C);
+    if (basis_layer0_) moments_.reserve(static_cast<std::size_t>(moment_receivers()) * 16 * kBasis * active_types_.size());
     M0_.reserve(N * NH * C);
     M0_adj_.reserve(T * NH * C);
     H1_.reserve(ALL * NH * C);
@@ -991,6 +1017,11 @@ void Evaluator::launch_tc(const std::vector<TcCall>& calls)
 // bit 2 = the rest of the reverse pass.  Between the phases a domain-decomposed run exchanges the
 // H1 rows and then the H1_adj rows of its ghost nodes (reference: begin / continue /
 // finish_factorized_distributed_evaluation, libsymmetrix/source/mace_kokkos_evaluate.cpp:1658-2101).
+ActiveEdges Evaluator::active_edges() const
+{
+    return {active_edges_.ptr, active_ends_.ptr, edge_types(), atype_.ptr, grid_.r_cut};
+}
+
 void Evaluator::run_pipeline(int phases)
 {
     const int R = num_receivers_, ALL = num_nodes_, C = model_.channels, NH = model_.num_hidden, NE = model_.num_lme;
@@ -1023,7 +1054,50 @@ void Evaluator::run_pipeline(int phases)
     const double mean_edges = static_cast<double>(num_edges_) / std::max(1, R);
     const PartRules rules{num_sms_, C, model_.shape_id, mean_edges}, sum_rules{num_sms_, C, model_.shape_id, deterministic_ ? 100.0 : mean_edges};
     auto sum_receivers = [&](int T) { return deterministic_ ? R : T; };
+    // per-element node ranges intersected with the tile
+    auto for_type_ranges = [&](int t0, int T, auto&& body) {
+        for (int a = 0; a < n_active; ++a) {
+            const int begin = std::max(type_begin_[a], t0), end = std::min(type_begin_[a + 1], t0 + T);
+            if (end > begin) body(a, begin, end - begin);
+        }
+    };
+    // the sums over the radial functions live for a slice of the receivers at a time
+    auto for_moment_slices = [&](int t0, int T, auto&& body) {
+        for (int begin = t0; begin < t0 + T; begin += moment_receivers()) body(begin, std::min(moment_receivers(), t0 + T - begin));
+    };
+    // A0 (or its adjoint) of a slice from the sums (or to their adjoint): one linear per (receiver type, l); t0: first receiver of
+    // the tile
+    auto basis_linears = [&](int slice, int receivers, int t0, bool reverse) {
+        const long width = static_cast<long>(kBasis) * n_active;
+        std::vector<TcCall> calls;
+        for_type_ranges(slice, receivers, [&](int a, int begin, int count) {
+            float* const moments = moments_.ptr + static_cast<std::size_t>(begin - slice) * 16 * width;
+            float* const nodes = (reverse ? A0_adj_.ptr : A0_.ptr) + static_cast<std::size_t>(begin - t0) * 16 * C;
+            for (int l = 0; l <= model_.l_max; ++l) {
+                const RowMap moment_rows{16 * width, width, l * l * width, 2 * l + 1}, node_rows{16L * C, C, static_cast<long>(l) * l * C, 2 * l + 1};
+                const SplitWeight* w = &s_a0_[a * (model_.l_max + 1) + l];
+                if (reverse) calls.push_back({nodes, node_rows, w, true, moments, moment_rows, 0, count, false, nullptr});
+                else calls.push_back({moments, moment_rows, w, false, nodes, node_rows, 0, count, false, nullptr});
+            }
+        });
+        launch_tc(calls);
+    };
     auto l0_forward = [&](int t0, int T) {
+        if (basis_layer0_) {
+            for_moment_slices(t0, T, [&](int begin, int count) {
+                span_begin("l0_forward");
+                l0_moments_kernel<<<count * n_active, 32, 0, stream_>>>(
+                    begin, n_active, first_.ptr, geom_.ptr, active_edges(), basis_pair_types_, grid_,
+                    reinterpret_cast<const float4*>(basis_table_.ptr), moments_.ptr, inv0);
+                launches_ += 1;
+                span_end();
+                span_begin("gemm_a0");
+                basis_linears(begin, count, t0, false);
+                span_end();
+            });
+            return;
+        }
+        span_begin("l0_forward");
         const int parts = sum_rules.l0_forward(sum_receivers(T)), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
         const std::size_t part_bytes = parts > 1 ? static_cast<std::size_t>(kWarpsPerBlock) * 16 * C * sizeof(float) : 0;
         if (C == 128)
@@ -1035,13 +1109,7 @@ void Evaluator::run_pipeline(int phases)
         else
             l0_forward_kernel<0><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_.ptr, inv0);
         launches_ += 1;
-    };
-    // per-element node ranges intersected with the tile
-    auto for_type_ranges = [&](int t0, int T, auto&& body) {
-        for (int a = 0; a < n_active; ++a) {
-            const int begin = std::max(type_begin_[a], t0), end = std::min(type_begin_[a + 1], t0 + T);
-            if (end > begin) body(a, begin, end - begin);
-        }
+        span_end();
     };
 
     if (phases & 1) {
@@ -1068,9 +1136,7 @@ void Evaluator::run_pipeline(int phases)
         }
         for (int t0 = 0; t0 < R; t0 += tile_cap) {
             const int T = std::min(tile_cap, R - t0);
-            span_begin("l0_forward");
             l0_forward(t0, T);
-            span_end();
             span_begin("m0_forward");
             float* m0 = M0_.ptr + t0 * rowH;
             if (model_.shape_id == 0)
@@ -1266,22 +1332,23 @@ void Evaluator::run_pipeline(int phases)
                 launch_tc(calls);
             }
             span_end();
+            // hidden l > 0 at the common widths: channel pairs with the row adjoints in tensor memory; otherwise one channel per thread
+            // with the adjoints in registers (16 rows for hidden 0e), which also leaves the records of the reproducible mode.
+            const bool paired = !deterministic_ && (model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64)));
             span_begin("l1_reverse");
-            // hidden l > 0 at the common widths: row adjoints in shared memory; otherwise one channel per thread with the
-            // adjoints in registers (16 rows for hidden 0e), which also leaves the records of the reproducible mode.
-            const bool shared_rows = !deterministic_ && (model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64)));
-            const int shared_blocks = model_.shape_id == 2 ? kSharedBlocksS2<128> : C == 64 ? kSharedBlocksS1<64> : kSharedBlocksS1<128>;
-            const int reverse_parts = shared_rows ? rules.l1_reverse_shared(T, shared_blocks) : rules.l1_reverse(T);
+            if (paired && fo.edge_forces != nullptr && t0 == 0)   // edges at or beyond the cutoff are not visited
+                SXB_CUDA(cudaMemsetAsync(fo.edge_forces, 0, sizeof(double) * 3 * num_edges_, stream_));
+            const int pair_blocks = model_.shape_id == 2 ? kPairBlocksS2 : kPairBlocksS1;
+            const int reverse_parts = paired ? rules.l1_reverse_pairs(T, pair_blocks) : rules.l1_reverse(T);
             const dim3 reverse_grid(T, reverse_parts);
-#define SXB_SHARED_REVERSE(NAME, WIDTH)                                                                                   \
-            l1_reverse_shared_kernel_##NAME<WIDTH><<<reverse_grid, WIDTH / 2 * kSharedTeams##NAME,                         \
-                                                     shared_rows_bytes(SXB_##NAME##_NUM_ROWS, WIDTH), stream_>>>(          \
-                t0, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_, reinterpret_cast<const float4*>(r1_table_.ptr), \
+#define SXB_PAIR_REVERSE(NAME, WIDTH)                                                                                     \
+            l1_reverse_pair_kernel_##NAME<WIDTH><<<reverse_grid, 32 * kPairWarps##NAME, pair_dynamic_bytes(WIDTH), stream_>>>(  \
+                t0, first_.ptr, sources_.ptr, geom_.ptr, active_edges(), grid_, reinterpret_cast<const float4*>(r1_table_.ptr), \
                 H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_)
-            if (shared_rows) {
-                if (model_.shape_id == 2) SXB_SHARED_REVERSE(S2, 128);
-                else if (C == 128) SXB_SHARED_REVERSE(S1, 128);
-                else SXB_SHARED_REVERSE(S1, 64);
+            if (paired) {
+                if (model_.shape_id == 2) SXB_PAIR_REVERSE(S2, 128);
+                else if (C == 128) SXB_PAIR_REVERSE(S1, 128);
+                else SXB_PAIR_REVERSE(S1, 64);
             } else if (deterministic_ && model_.shape_id == 0)
                 l1_reverse_kernel_S0<0, 3, true><<<reverse_grid, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
@@ -1294,7 +1361,7 @@ void Evaluator::run_pipeline(int phases)
             else
                 l1_reverse_kernel_S1<0><<<reverse_grid, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,
                     reinterpret_cast<const float4*>(r1_table_.ptr), H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_);
-#undef SXB_SHARED_REVERSE
+#undef SXB_PAIR_REVERSE
             launches_ += 1;
             span_end();
         }
@@ -1308,6 +1375,8 @@ void Evaluator::run_pipeline(int phases)
     }
     if (phases & 4) {
         fo.accumulate_edge = model_.single_layer ? 0 : 1;   // the layer-1 gradient wrote the edge forces first
+        if (basis_layer0_ && fo.edge_forces != nullptr && !fo.accumulate_edge)   // edges at or beyond the cutoff are not visited
+            SXB_CUDA(cudaMemsetAsync(fo.edge_forces, 0, sizeof(double) * 3 * num_edges_, stream_));
         if (phases != 7 && halo_plan_.active && halo_plan_.received_rows != nullptr) {   // reverse halo: adjoints my atoms collected as ghosts of the peers
             span_begin("halo_unpack");
             unpack_rows(1, halo_plan_.send_indices, halo_plan_.num_send, halo_plan_.received_rows, true);
@@ -1317,9 +1386,7 @@ void Evaluator::run_pipeline(int phases)
             const int T = std::min(tile_cap, R - t0);
             if (tiled) {
                 // the tile workspace no longer holds this tile's A0: regenerate it
-                span_begin("l0_forward_recompute");
                 l0_forward(t0, T);
-                span_end();
             }
             span_begin("gemm_h1_reverse");
             // M0_adj_il = H1_adj_il W_l^T, then the direct adjoint q + T_element H2_adj on the scalar block
@@ -1377,8 +1444,20 @@ void Evaluator::run_pipeline(int phases)
                 SXB_LAUNCH_POLY(m0_reverse_kernel, S2, SXB_S2_M0_NUM_TERMS, T, C, stream_, A0_.ptr, element_.ptr + t0, m0_weights_.ptr, M0_adj_.ptr, A0_adj_.ptr, model_.a0_scaled ? dot0_.ptr + t0 : nullptr);
             launches_ += 1;
             span_end();
-            span_begin("l0_reverse");
-            {
+            if (basis_layer0_) {
+                for_moment_slices(t0, T, [&](int begin, int count) {
+                    span_begin("gemm_a0_reverse");
+                    basis_linears(begin, count, t0, true);
+                    span_end();
+                    span_begin("l0_reverse");
+                    l0_moments_reverse_kernel<<<dim3(count, rules.l0_moments_reverse(count, n_active)), 32, 0, stream_>>>(
+                        begin, n_active, first_.ptr, sources_.ptr, geom_.ptr, active_edges(), basis_pair_types_, grid_,
+                        reinterpret_cast<const float4*>(basis_steps_.ptr), moments_.ptr, fo, density0);
+                    launches_ += 1;
+                    span_end();
+                });
+            } else {
+                span_begin("l0_reverse");
                 const int parts = rules.l0_reverse(T), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
                 if (C == 128)
                     l0_reverse_pair_kernel<4><<<warp_grid, warp_threads, kWarpsPerBlock * sizeof(WarpPairChunk), stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
@@ -1388,9 +1467,9 @@ void Evaluator::run_pipeline(int phases)
                     l0_reverse_warp_kernel<<<warp_grid, warp_threads, 0, stream_>>>(T, t0, parts, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
                 else
                     l0_reverse_kernel<0><<<T, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, r0_table_.ptr, A0_adj_.ptr, fo, density0);
+                launches_ += 1;
+                span_end();
             }
-            launches_ += 1;
-            span_end();
         }
         if (model_.has_zbl) {
             span_begin("zbl");
@@ -1443,15 +1522,15 @@ void Evaluator::enqueue_phases(int phases, const double* positions, bool upload_
             if (geometry_mode_ == 1)
                 geometry_from_reference_kernel<false><<<grid, 256, 0, stream_>>>(
                     num_receivers_, first_.ptr, sources_.ptr, positions, original_.ptr, reference_positions_.ptr, reference_xyz_.ptr,
-                    edge_map_.ptr, cell_.ptr, inv_cell_.ptr, pbc_mask_, geom_.ptr, error_flag_.ptr);
+                    edge_map_.ptr, cell_.ptr, inv_cell_.ptr, pbc_mask_, geom_.ptr, error_flag_.ptr, active_edges());
             else if (geometry_mode_ == 2)
                 geometry_from_reference_kernel<true><<<grid, 256, 0, stream_>>>(
                     num_receivers_, first_.ptr, sources_.ptr, positions, original_.ptr, reference_positions_.ptr, reference_xyz_.ptr,
-                    edge_map_.ptr, cell_.ptr, inv_cell_.ptr, pbc_mask_, geom_.ptr, error_flag_.ptr);
+                    edge_map_.ptr, cell_.ptr, inv_cell_.ptr, pbc_mask_, geom_.ptr, error_flag_.ptr, active_edges());
             else
                 geometry_from_positions_kernel<<<grid, 256, 0, stream_>>>(
                     num_receivers_, first_.ptr, sources_.ptr, has_shifts_ ? shifts_.ptr : nullptr, positions, original_.ptr, cell_.ptr,
-                    geom_.ptr, error_flag_.ptr);
+                    geom_.ptr, error_flag_.ptr, active_edges());
             launches_ += 1;
         }
         run_pipeline(phases);
@@ -1576,7 +1655,8 @@ void Evaluator::compute_edge_vectors(std::uint64_t generation, const double* xyz
     SXB_CUDA(cudaMemcpyAsync(dxyz.ptr, xyz, sizeof(double) * 3 * num_edges_, cudaMemcpyHostToDevice, stream_));
     SXB_CUDA(cudaMemsetAsync(error_flag_.ptr, 0, sizeof(int), stream_));
     geometry_from_vectors_kernel<<<blocks_for(num_edges_, 256), 256, 0, stream_>>>(num_edges_, dxyz.ptr, edge_map_.ptr, geom_.ptr, error_flag_.ptr);
-    launches_ += 1;
+    active_edges_kernel<<<blocks_for(static_cast<long>(num_receivers_) * 32, 256), 256, 0, stream_>>>(num_receivers_, first_.ptr, sources_.ptr, geom_.ptr, active_edges());
+    launches_ += 2;
     enqueue_phases(7, nullptr, false);
     finish_compute();
 }
@@ -1616,7 +1696,8 @@ void Evaluator::distributed_begin_edge_vectors(std::uint64_t generation, const d
     if (num_edges_ > 0)
         geometry_from_vectors_kernel<<<blocks_for(num_edges_, 256), 256, 0, stream_>>>(num_edges_, device_xyz, edge_map_.ptr, geom_.ptr,
                                                                                       error_flag_.ptr);
-    launches_ += 1;
+    active_edges_kernel<<<blocks_for(static_cast<long>(num_receivers_) * 32, 256), 256, 0, stream_>>>(num_receivers_, first_.ptr, sources_.ptr, geom_.ptr, active_edges());
+    launches_ += 2;
     enqueue_phases(1, nullptr, false);
     phase_ = 1;
 }

@@ -1,6 +1,7 @@
 // Evaluator class behind the C ABI (include/symmetrix_b200.h).
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <stdexcept>
@@ -16,6 +17,7 @@
 
 namespace sxb {
 
+struct ActiveEdges;
 
 struct StaleGraph : std::invalid_argument {
     using std::invalid_argument::invalid_argument;
@@ -94,11 +96,11 @@ public:
     long launches() const { return launches_; }
     std::size_t workspace_bytes() const
     {
-        return geom_.bytes() + A0_.bytes() + A0_adj_.bytes() + M0_.bytes() + M0_adj_.bytes() + H1_.bytes() + H1_adj_.bytes() + Phi1_.bytes()
+        return geom_.bytes() + active_edges_.bytes() + active_ends_.bytes() + A0_.bytes() + A0_adj_.bytes() + M0_.bytes() + M0_adj_.bytes() + H1_.bytes() + H1_adj_.bytes() + Phi1_.bytes()
                + dPhi1_.bytes() + A1_.bytes() + A1_adj_.bytes() + M1_.bytes() + M1_adj_.bytes() + H2_.bytes() + H2_adj_.bytes()
                + first_.bytes() + sources_.bytes() + shifts_.bytes() + edge_map_.bytes() + first_caller_.bytes() + sources_caller_.bytes()
                + shifts_caller_.bytes() + forces_.bytes() + forces_out_.bytes() + positions_.bytes() + edge_forces_.bytes()
-               + r0_table_.bytes() + r1_table_.bytes();
+               + r0_table_.bytes() + r1_table_.bytes() + basis_table_.bytes() + basis_steps_.bytes() + moments_.bytes();
     }
     // Per-kernel device times of the last compute (CUDA events on the evaluator's stream), only
     // collected while profiling is switched on.
@@ -109,8 +111,26 @@ public:
     void require_results() const;
 
 private:
-    void prepare_active_types(const std::vector<int>& node_types);
+    void prepare_active_types(const std::vector<int>& node_types, int num_receivers);
     void install_graph(int num_receivers, int num_nodes, const std::vector<int>& node_types, long num_edges, bool has_shifts);
+    ActiveEdges active_edges() const;
+    // receivers whose sums over the radial functions are kept at a time: 96 MB of them stay in L2 between their kernels
+    int moment_receivers() const
+    {
+        const long fit = (96l << 20) / (16l * 64 * static_cast<long>(sizeof(float)) * static_cast<long>(std::max<std::size_t>(1, active_types_.size())));
+        return static_cast<int>(std::min<long>(tile_capacity(), std::max(1024l, fit)));
+    }
+    int edge_types() const { return basis_layer0_ ? static_cast<int>(active_types_.size()) : 1; }   // types a receiver's edges are grouped by
+    // M1 to readout and back in one kernel (node_readout_kernel_*): the model has that form, and the graph is so small that short
+    // dependent kernels cost more than the tensor cores gain.  By the receivers of the graph and not of the tile, so that tiles do
+    // not change the arithmetic.  Five launches / one, us, 128 channels: 40 receivers 47 / 19, 320: 48 / 19, 1,080: 55 / 31, 5,000: 88 /
+    // 99; 64 channels, 1,080: 60 / 17; hidden 0e at 32 channels, 320: 43 / 15.
+    bool fused_readout_model() const
+    {
+        const int C = model_.channels;
+        return model_.readout2_hidden == 16 && (C == 128 || C == 64 || C == 32) && !model_.single_layer && !model_.legacy_h1_basis && !model_.pre_linear_up;
+    }
+    bool fused_readout() const { return fused_readout_model() && static_cast<long>(num_receivers_) * model_.channels <= 3000l * 128; }
     void run_pipeline(int phases);
     void enqueue_phases(int phases, const double* positions, bool upload_staged);
     void drop_step_graphs();
@@ -149,7 +169,7 @@ private:
 
     // model tables on the device
     DeviceBuffer<float> density0_table_, density1_table_, inv_scale0_, inv_scale1_, dot0_, dot1_;
-    DeviceBuffer<float> r0_table_, r1_table_, m0_weights_, m1_weights_, w_h1_, w_a1_[4], h2_skip_, h2_m1_;
+    DeviceBuffer<float> r0_table_, r1_table_, m0_weights_, m1_weights_, w_h1_, w_a1_[4], h2_skip_, h2_m1_, h2_skip_t_, h2_m1_t_;
     // pre_linear_up basis: x = M0[l=0] P0 (+ residual) and its adjoint per receiver; residual-first constants per element
     DeviceBuffer<float> scalar_input_, scalar_adjoint_, residual_fused_, residual_scalar_;
     DeviceBuffer<int> hidden_poly_terms_;          // single-layer models: monomials of the readout polynomial over H1
@@ -166,6 +186,11 @@ private:
     };
     SplitWeight s_h1_[4], s_a1_[4], s_h2_m1_;
     std::vector<SplitWeight> s_h2_skip_;
+    std::vector<SplitWeight> s_a0_;   // [active type of the receiver][l]: radial functions of the network's last hidden layer to A0
+    DeviceBuffer<float> basis_table_, basis_steps_, moments_;   // their splines in the order of either kernel; [slice][16][types * 64] sums over the edges, or their adjoints
+    bool basis_layer0_ = false;       // layer 0 runs on those functions (chosen per graph)
+    bool basis_ready_ = false, table_ready_ = false;   // which of the two tables stands for the active types
+    int basis_pair_types_ = 1;
     SplitWeight s_product0_;          // P0 of the pre_linear_up basis
     bool use_tensor_cores_ = true;
     int num_sms_ = 148;
@@ -206,6 +231,7 @@ private:
 
     // work buffers
     DeviceBuffer<EdgeGeom> geom_;
+    DeviceBuffer<int> active_edges_, active_ends_;   // edges inside the cutoff and the ends of their runs by source type (ActiveEdges)
     DeviceBuffer<float> A0_, A0_adj_, M0_, M0_adj_, H1_, H1_adj_, Phi1_, dPhi1_, A1_, A1_adj_, M1_, M1_adj_, H2_, H2_adj_;
     DeviceBuffer<double> node_energies_, node_energies_out_, forces_, forces_out_, edge_forces_;
     DeviceBuffer<double> totals_, energy_slots_, virial_slots_;

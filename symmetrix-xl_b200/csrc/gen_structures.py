@@ -132,27 +132,37 @@ def contraction_lines(terms):
     return fwd, rev
 
 
+ROW_BATCH = 8      # kRowBatch of edge_kernels_pairs.cuh
+
+
 def reverse_edges_lines(paths, row_begin, fed):
-    """Straight-line layer-1 gradient of kEdges edges at once on channel pairs (edge_kernels_shared.cuh).  ADJ(row) reads a
-    row adjoint from shared memory; every value it returns feeds two operations per edge.  EACH(statement) repeats the
-    statement for every edge e.  Names: h[e][lm2], hadj[e][lm2] source features and their adjoint, R[e], dR[e] radial value
-    and slope of the path at hand (RADIAL(p) fetches them), y[e][], ang[e][] the harmonics and the angular adjoint of the
-    edge l at hand, radial[e].  Per path the same contractions as reverse_path_lines; rows that no coupling term feeds (their
-    adjoint is zero: 12 of 88 for hidden 0e+1o, 56 of 243 for 0e+1o+2e) are left out."""
-    out, used = [], set()
+    """Straight-line layer-1 gradient of one edge on channel pairs (edge_kernels_pairs.cuh) and the rows in the order it uses
+    them.  Row adjoints come kRowBatch at a time: ROWS(batch) brings the batch into w[], every value of which feeds two
+    operations.  Names: h[lm2], hadj[lm2] source features and their adjoint, R, dR radial value and slope of the path at hand
+    (RADIAL(p) fetches them), y[], ang[] the harmonics and the angular adjoint of the edge l at hand (f[lm]: of both channels),
+    radial.  Per path the same
+    contractions as reverse_path_lines; rows that no coupling term feeds (their adjoint is zero: 12 of 88 for hidden 0e+1o, 56
+    of 243 for 0e+1o+2e) are left out."""
+    out, used, order = [], set(), []
 
     def put(target, a, b):
-        out[-1] += f" EACH({target} = f2_fma({a}, {b}, {target});)" if target in used else f" EACH({target} = f2_mul({a}, {b});)"
+        target, a, b = target.replace("[e]", ""), a.replace("[e]", ""), b.replace("[e]", "")
+        out[-1] += f" {target} = f2_fma({a}, {b}, {target});" if target in used else f" {target} = f2_mul({a}, {b});"
         used.add(target)
+
+    def take(row):
+        slot = len(order)
+        order.append(row)
+        out.append(f"      {f'ROWS({slot // ROW_BATCH}) ' if slot % ROW_BATCH == 0 else ''}{{ const f2 w = rows[{slot % ROW_BATCH}];")
 
     for l1 in sorted({path[1] for path in paths}):
         n1 = 2 * l1 + 1
-        out.append(f"    {{ f2 y[kEdges][{n1}]{f', ang[kEdges][{n1}]' if l1 else ''}; EACH(load_pair_harmonics<{l1}>(yrow[e], y[e]);)")
-        used -= {f"ang[e][{a}]" for a in range(16)}
+        out.append(f"    {{ f2 y[{n1}]{f', ang[{n1}]' if l1 else ''}; load_pair_harmonics<{l1}>(yrow, y);")
+        used -= {f"ang[{a}]" for a in range(16)}
         for p, (l, _, l2) in [(p, path) for p, path in enumerate(paths) if path[1] == l1]:
             n2 = 2 * l2 + 1
-            out.append(f"    {{ /* path {p}: edge l={l1}, source l={l2} -> l={l} */ RADIAL({p}) f2 yw[kEdges], t[kEdges][{n2}], v[kEdges][{n2}];")
-            used -= {"yw[e]"} | {f"{k}[e][{q}]" for k in "tv" for q in range(16)}
+            out.append(f"    {{ /* path {p}: edge l={l1}, source l={l2} -> l={l} */ RADIAL({p}) f2 yw, t[{n2}], v[{n2}];")
+            used -= {"yw"} | {f"{k}[{q}]" for k in "tv" for q in range(16)}
             if n2 < n1:
                 for b in range(n2):
                     out.append("     ")
@@ -161,7 +171,7 @@ def reverse_edges_lines(paths, row_begin, fed):
                     for b in range(n2):
                         if row_begin[p] + a * n2 + b not in fed:
                             continue
-                        out.append(f"      {{ const f2 w = ADJ({row_begin[p] + a * n2 + b});")
+                        take(row_begin[p] + a * n2 + b)
                         put(f"ang[e][{a}]", f"t[e][{b}]", "w")
                         put(f"v[e][{b}]", f"y[e][{a}]", "w")
                         out[-1] += " }"
@@ -174,12 +184,12 @@ def reverse_edges_lines(paths, row_begin, fed):
                     row = row_begin[p] + a * n2
                     if not fed.intersection(range(row, row + n2)):
                         continue
-                    out.append(f"      EACH(t[e][0] = f2_mul(R[e], y[e][{a}]);)")
-                    used -= {"v[e][0]"}
+                    out.append(f"      t[0] = f2_mul(R, y[{a}]);")
+                    used -= {"v[0]"}
                     for b in range(n2):
                         if row + b not in fed:
                             continue
-                        out.append(f"      {{ const f2 w = ADJ({row + b});")
+                        take(row + b)
                         put("v[e][0]", f"h[e][{l2 * l2 + b}]", "w")
                         put(f"hadj[e][{l2 * l2 + b}]", "t[e][0]", "w")
                         out[-1] += " }"
@@ -191,8 +201,22 @@ def reverse_edges_lines(paths, row_begin, fed):
             put("radial[e]", "dR[e]", "yw[e]")
             out.append("    }")
         if l1:
-            out.append(f"      EACH(add_angular_force<{l1}>(grow[e], ang[e], fx[e], fy[e], fz[e]);)")
+            out.append("     " + "".join(f" f[{l1 * l1 + a}] = f2_sum(ang[{a}]);" for a in range(n1)))
         out.append("    }")
+    return out, order
+
+
+def adjoint_rows_lines(order, term_row, term_lme):
+    """The row adjoints in that order, kRowBatch at a time: TERM(slot, term, lme) / TERM_ADD for a row's first / further coupling
+    terms, STORE(batch) hands a full batch (the last one padded with zeros) over."""
+    out = []
+    for slot, row in enumerate(order + [None] * (-len(order) % ROW_BATCH)):
+        terms = [(t, lme) for t, (r, lme) in enumerate(zip(term_row, term_lme)) if r == row]
+        line = "    " + (" ".join(f"TERM{'_ADD' if n else ''}({slot % ROW_BATCH}, {t}, {lme})" for n, (t, lme) in enumerate(terms))
+                         if terms else f"v[{slot % ROW_BATCH}] = 0ull;")
+        if slot % ROW_BATCH == ROW_BATCH - 1:
+            line += f" STORE({slot // ROW_BATCH})"
+        out.append(line)
     return out
 
 
@@ -288,8 +312,12 @@ def emit_shape(name, l_max, L_max, tables, groups=1, by_edge_l=None):
         out.append(f"#define SXB_{name}_L1_REVERSE_BODY \\")
         out.append(" \\\n".join(rev))
     if L_max > 0:
-        out.append(f"#define SXB_{name}_L1_REVERSE_EDGES_BODY \\")
-        out.append(" \\\n".join(reverse_edges_lines(paths, row_begin, set(tables["Phi1_lelm1lm2"]))))
+        body, order = reverse_edges_lines(paths, row_begin, set(tables["Phi1_lelm1lm2"]))
+        out.append(f"#define SXB_{name}_ROW_BATCHES {(len(order) + ROW_BATCH - 1) // ROW_BATCH}")
+        out.append(f"#define SXB_{name}_L1_REVERSE_EDGE_BODY \\")
+        out.append(" \\\n".join(body))
+        out.append(f"#define SXB_{name}_L1_ADJOINT_ROWS \\")
+        out.append(" \\\n".join(adjoint_rows_lines(order, tables["Phi1_lelm1lm2"], tables["Phi1_lme"])))
     if groups > 1:
         out.extend(emit_path_groups(name, paths, row_begin, tables, groups, by_edge_l))
     out.append("")

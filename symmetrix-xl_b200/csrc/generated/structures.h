@@ -2057,164 +2057,246 @@
         hadj[3] = fmaf(R[9], s_, hadj[3]); yw = fmaf(h[3], s_, yw); } \
       radial = fmaf(dR[9], yw, radial); \
     }
-#define SXB_S1_L1_REVERSE_EDGES_BODY \
-    { f2 y[kEdges][1]; EACH(load_pair_harmonics<0>(yrow[e], y[e]);) \
-    { /* path 0: edge l=0, source l=0 -> l=0 */ RADIAL(0) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(0); EACH(v[e][0] = f2_mul(h[e][0], w);) EACH(hadj[e][0] = f2_mul(t[e][0], w);) } \
-      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_mul(dR[e], yw[e]);) \
+#define SXB_S1_ROW_BATCHES 10
+#define SXB_S1_L1_REVERSE_EDGE_BODY \
+    { f2 y[1]; load_pair_harmonics<0>(yrow, y); \
+    { /* path 0: edge l=0, source l=0 -> l=0 */ RADIAL(0) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, y[0]); \
+      ROWS(0) { const f2 w = rows[0]; v[0] = f2_mul(h[0], w); hadj[0] = f2_mul(t[0], w); } \
+      yw = f2_mul(y[0], v[0]); \
+      radial = f2_mul(dR, yw); \
     } \
-    { /* path 3: edge l=0, source l=1 -> l=1 */ RADIAL(3) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(13); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(14); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(15); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_mul(t[e][0], w);) } \
-      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 3: edge l=0, source l=1 -> l=1 */ RADIAL(3) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[1]; v[0] = f2_mul(h[1], w); hadj[1] = f2_mul(t[0], w); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_mul(t[0], w); } \
+      { const f2 w = rows[3]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_mul(t[0], w); } \
+      yw = f2_mul(y[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
     } \
-    { f2 y[kEdges][3], ang[kEdges][3]; EACH(load_pair_harmonics<1>(yrow[e], y[e]);) \
-    { /* path 1: edge l=1, source l=1 -> l=0 */ RADIAL(1) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(1); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      EACH(ang[e][0] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(5); EACH(v[e][0] = f2_mul(h[e][2], w);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      EACH(ang[e][1] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(9); EACH(v[e][0] = f2_mul(h[e][3], w);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][2] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { f2 y[3], ang[3]; load_pair_harmonics<1>(yrow, y); \
+    { /* path 1: edge l=1, source l=1 -> l=0 */ RADIAL(1) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[4]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      ang[0] = f2_mul(R, v[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      { const f2 w = rows[5]; v[0] = f2_mul(h[2], w); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      ang[1] = f2_mul(R, v[0]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      { const f2 w = rows[6]; v[0] = f2_mul(h[3], w); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[2] = f2_mul(R, v[0]); yw = f2_fma(y[2], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 2: edge l=1, source l=0 -> l=1 */ RADIAL(2) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
-      { const f2 w = ADJ(10); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(11); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(12); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 2: edge l=1, source l=0 -> l=1 */ RADIAL(2) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, h[0]); \
+      { const f2 w = rows[7]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      ROWS(1) { const f2 w = rows[0]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[1]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      hadj[0] = f2_fma(R, v[0], hadj[0]); yw = f2_mul(h[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 6: edge l=1, source l=1 -> l=2 */ RADIAL(6) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(36); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      { const f2 w = ADJ(37); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      { const f2 w = ADJ(38); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(39); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      { const f2 w = ADJ(40); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      { const f2 w = ADJ(41); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(42); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      { const f2 w = ADJ(43); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      { const f2 w = ADJ(44); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 6: edge l=1, source l=1 -> l=2 */ RADIAL(6) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[2]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      { const f2 w = rows[3]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[0] = f2_fma(R, v[0], ang[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      { const f2 w = rows[5]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      { const f2 w = rows[6]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[1] = f2_fma(R, v[0], ang[1]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      ROWS(2) { const f2 w = rows[0]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[2] = f2_fma(R, v[0], ang[2]); yw = f2_fma(y[2], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-      EACH(add_angular_force<1>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+      f[1] = f2_sum(ang[0]); f[2] = f2_sum(ang[1]); f[3] = f2_sum(ang[2]); \
     } \
-    { f2 y[kEdges][5], ang[kEdges][5]; EACH(load_pair_harmonics<2>(yrow[e], y[e]);) \
-    { /* path 4: edge l=2, source l=1 -> l=1 */ RADIAL(4) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
-      { const f2 w = ADJ(16); EACH(ang[e][0] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(18); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(19); EACH(ang[e][1] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(20); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
-      { const f2 w = ADJ(22); EACH(ang[e][2] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(23); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(24); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
-      { const f2 w = ADJ(26); EACH(ang[e][3] = f2_mul(t[e][1], w);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(27); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(28); EACH(ang[e][4] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(30); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
-      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
-      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { f2 y[5], ang[5]; load_pair_harmonics<2>(yrow, y); \
+    { /* path 4: edge l=2, source l=1 -> l=1 */ RADIAL(4) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, h[1]); \
+      t[1] = f2_mul(R, h[2]); \
+      t[2] = f2_mul(R, h[3]); \
+      { const f2 w = rows[3]; ang[0] = f2_mul(t[0], w); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[4]; ang[0] = f2_fma(t[2], w, ang[0]); v[2] = f2_mul(y[0], w); } \
+      { const f2 w = rows[5]; ang[1] = f2_mul(t[0], w); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[6]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_mul(y[1], w); } \
+      { const f2 w = rows[7]; ang[2] = f2_mul(t[0], w); v[0] = f2_fma(y[2], w, v[0]); } \
+      ROWS(3) { const f2 w = rows[0]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[1]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_fma(y[2], w, v[2]); } \
+      { const f2 w = rows[2]; ang[3] = f2_mul(t[1], w); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[3]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      { const f2 w = rows[4]; ang[4] = f2_mul(t[0], w); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[5]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      hadj[1] = f2_fma(R, v[0], hadj[1]); yw = f2_mul(h[1], v[0]); \
+      hadj[2] = f2_fma(R, v[1], hadj[2]); yw = f2_fma(h[2], v[1], yw); \
+      hadj[3] = f2_fma(R, v[2], hadj[3]); yw = f2_fma(h[3], v[2], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 5: edge l=2, source l=0 -> l=2 */ RADIAL(5) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
-      { const f2 w = ADJ(31); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(32); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(33); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(34); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(35); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 5: edge l=2, source l=0 -> l=2 */ RADIAL(5) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, h[0]); \
+      { const f2 w = rows[6]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[7]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      ROWS(4) { const f2 w = rows[0]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      { const f2 w = rows[1]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[2]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      hadj[0] = f2_fma(R, v[0], hadj[0]); yw = f2_mul(h[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 9: edge l=2, source l=1 -> l=3 */ RADIAL(9) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
-      { const f2 w = ADJ(73); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(74); EACH(ang[e][0] = f2_fma(t[e][1], w, ang[e][0]);) EACH(v[e][1] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(75); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(76); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(77); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_fma(y[e][1], w, v[e][1]);) } \
-      { const f2 w = ADJ(78); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
-      { const f2 w = ADJ(79); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(80); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(81); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
-      { const f2 w = ADJ(82); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(83); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(84); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(85); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(86); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
-      { const f2 w = ADJ(87); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
-      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
-      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 9: edge l=2, source l=1 -> l=3 */ RADIAL(9) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, h[1]); \
+      t[1] = f2_mul(R, h[2]); \
+      t[2] = f2_mul(R, h[3]); \
+      { const f2 w = rows[3]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[4]; ang[0] = f2_fma(t[1], w, ang[0]); v[1] = f2_mul(y[0], w); } \
+      { const f2 w = rows[5]; ang[0] = f2_fma(t[2], w, ang[0]); v[2] = f2_mul(y[0], w); } \
+      { const f2 w = rows[6]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[7]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_fma(y[1], w, v[1]); } \
+      ROWS(5) { const f2 w = rows[0]; ang[1] = f2_fma(t[2], w, ang[1]); v[2] = f2_fma(y[1], w, v[2]); } \
+      { const f2 w = rows[1]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      { const f2 w = rows[2]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[3]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_fma(y[2], w, v[2]); } \
+      { const f2 w = rows[4]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[5]; ang[3] = f2_fma(t[1], w, ang[3]); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[6]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      { const f2 w = rows[7]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      ROWS(6) { const f2 w = rows[0]; ang[4] = f2_fma(t[1], w, ang[4]); v[1] = f2_fma(y[4], w, v[1]); } \
+      { const f2 w = rows[1]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      hadj[1] = f2_fma(R, v[0], hadj[1]); yw = f2_mul(h[1], v[0]); \
+      hadj[2] = f2_fma(R, v[1], hadj[2]); yw = f2_fma(h[2], v[1], yw); \
+      hadj[3] = f2_fma(R, v[2], hadj[3]); yw = f2_fma(h[3], v[2], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-      EACH(add_angular_force<2>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+      f[4] = f2_sum(ang[0]); f[5] = f2_sum(ang[1]); f[6] = f2_sum(ang[2]); f[7] = f2_sum(ang[3]); f[8] = f2_sum(ang[4]); \
     } \
-    { f2 y[kEdges][7], ang[kEdges][7]; EACH(load_pair_harmonics<3>(yrow[e], y[e]);) \
-    { /* path 7: edge l=3, source l=1 -> l=2 */ RADIAL(7) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
-      { const f2 w = ADJ(45); EACH(ang[e][0] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(47); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(48); EACH(ang[e][1] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(49); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
-      { const f2 w = ADJ(50); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
-      { const f2 w = ADJ(51); EACH(ang[e][2] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(52); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(53); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
-      { const f2 w = ADJ(54); EACH(ang[e][3] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(55); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(56); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(57); EACH(ang[e][4] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(58); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
-      { const f2 w = ADJ(59); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      { const f2 w = ADJ(60); EACH(ang[e][5] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
-      { const f2 w = ADJ(61); EACH(ang[e][5] = f2_fma(t[e][1], w, ang[e][5]);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
-      { const f2 w = ADJ(62); EACH(ang[e][5] = f2_fma(t[e][2], w, ang[e][5]);) EACH(v[e][2] = f2_fma(y[e][5], w, v[e][2]);) } \
-      { const f2 w = ADJ(63); EACH(ang[e][6] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
-      { const f2 w = ADJ(65); EACH(ang[e][6] = f2_fma(t[e][2], w, ang[e][6]);) EACH(v[e][2] = f2_fma(y[e][6], w, v[e][2]);) } \
-      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
-      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
-      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { f2 y[7], ang[7]; load_pair_harmonics<3>(yrow, y); \
+    { /* path 7: edge l=3, source l=1 -> l=2 */ RADIAL(7) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, h[1]); \
+      t[1] = f2_mul(R, h[2]); \
+      t[2] = f2_mul(R, h[3]); \
+      { const f2 w = rows[2]; ang[0] = f2_mul(t[0], w); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[3]; ang[0] = f2_fma(t[2], w, ang[0]); v[2] = f2_mul(y[0], w); } \
+      { const f2 w = rows[4]; ang[1] = f2_mul(t[0], w); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[5]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_mul(y[1], w); } \
+      { const f2 w = rows[6]; ang[1] = f2_fma(t[2], w, ang[1]); v[2] = f2_fma(y[1], w, v[2]); } \
+      { const f2 w = rows[7]; ang[2] = f2_mul(t[0], w); v[0] = f2_fma(y[2], w, v[0]); } \
+      ROWS(7) { const f2 w = rows[0]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[1]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_fma(y[2], w, v[2]); } \
+      { const f2 w = rows[2]; ang[3] = f2_mul(t[0], w); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[3]; ang[3] = f2_fma(t[1], w, ang[3]); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[4]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      { const f2 w = rows[5]; ang[4] = f2_mul(t[0], w); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[6]; ang[4] = f2_fma(t[1], w, ang[4]); v[1] = f2_fma(y[4], w, v[1]); } \
+      { const f2 w = rows[7]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      ROWS(8) { const f2 w = rows[0]; ang[5] = f2_mul(t[0], w); v[0] = f2_fma(y[5], w, v[0]); } \
+      { const f2 w = rows[1]; ang[5] = f2_fma(t[1], w, ang[5]); v[1] = f2_fma(y[5], w, v[1]); } \
+      { const f2 w = rows[2]; ang[5] = f2_fma(t[2], w, ang[5]); v[2] = f2_fma(y[5], w, v[2]); } \
+      { const f2 w = rows[3]; ang[6] = f2_mul(t[0], w); v[0] = f2_fma(y[6], w, v[0]); } \
+      { const f2 w = rows[4]; ang[6] = f2_fma(t[2], w, ang[6]); v[2] = f2_fma(y[6], w, v[2]); } \
+      hadj[1] = f2_fma(R, v[0], hadj[1]); yw = f2_mul(h[1], v[0]); \
+      hadj[2] = f2_fma(R, v[1], hadj[2]); yw = f2_fma(h[2], v[1], yw); \
+      hadj[3] = f2_fma(R, v[2], hadj[3]); yw = f2_fma(h[3], v[2], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 8: edge l=3, source l=0 -> l=3 */ RADIAL(8) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
-      { const f2 w = ADJ(66); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(67); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(68); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(69); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(70); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(71); EACH(ang[e][5] = f2_fma(t[e][0], w, ang[e][5]);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
-      { const f2 w = ADJ(72); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
-      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 8: edge l=3, source l=0 -> l=3 */ RADIAL(8) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, h[0]); \
+      { const f2 w = rows[5]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[6]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[7]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      ROWS(9) { const f2 w = rows[0]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[1]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[2]; ang[5] = f2_fma(t[0], w, ang[5]); v[0] = f2_fma(y[5], w, v[0]); } \
+      { const f2 w = rows[3]; ang[6] = f2_fma(t[0], w, ang[6]); v[0] = f2_fma(y[6], w, v[0]); } \
+      hadj[0] = f2_fma(R, v[0], hadj[0]); yw = f2_mul(h[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-      EACH(add_angular_force<3>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+      f[9] = f2_sum(ang[0]); f[10] = f2_sum(ang[1]); f[11] = f2_sum(ang[2]); f[12] = f2_sum(ang[3]); f[13] = f2_sum(ang[4]); f[14] = f2_sum(ang[5]); f[15] = f2_sum(ang[6]); \
     }
+#define SXB_S1_L1_ADJOINT_ROWS \
+    TERM(0, 0, 0) \
+    TERM(1, 1, 3) \
+    TERM(2, 2, 6) \
+    TERM(3, 3, 9) \
+    TERM(4, 5, 1) \
+    TERM(5, 12, 1) \
+    TERM(6, 18, 1) \
+    TERM(7, 4, 2) STORE(0) \
+    TERM(0, 10, 5) \
+    TERM(1, 15, 8) \
+    TERM(2, 6, 18) TERM_ADD(2, 7, 24) \
+    TERM(3, 8, 15) \
+    TERM(4, 9, 12) \
+    TERM(5, 11, 15) \
+    TERM(6, 13, 18) \
+    TERM(7, 14, 21) STORE(1) \
+    TERM(0, 16, 12) \
+    TERM(1, 17, 21) \
+    TERM(2, 19, 18) TERM_ADD(2, 20, 24) \
+    TERM(3, 22, 10) \
+    TERM(4, 26, 4) \
+    TERM(5, 30, 7) \
+    TERM(6, 33, 4) \
+    TERM(7, 37, 4) STORE(2) \
+    TERM(0, 39, 7) \
+    TERM(1, 41, 10) \
+    TERM(2, 45, 10) \
+    TERM(3, 47, 7) \
+    TERM(4, 51, 4) \
+    TERM(5, 55, 10) \
+    TERM(6, 21, 11) \
+    TERM(7, 29, 14) STORE(3) \
+    TERM(0, 36, 17) \
+    TERM(1, 43, 20) \
+    TERM(2, 50, 23) \
+    TERM(3, 23, 35) TERM_ADD(3, 24, 39) \
+    TERM(4, 25, 29) \
+    TERM(5, 27, 27) TERM_ADD(5, 28, 31) \
+    TERM(6, 31, 33) TERM_ADD(6, 32, 37) \
+    TERM(7, 34, 31) STORE(4) \
+    TERM(0, 35, 29) \
+    TERM(1, 38, 31) \
+    TERM(2, 40, 33) \
+    TERM(3, 42, 35) \
+    TERM(4, 44, 29) \
+    TERM(5, 46, 35) \
+    TERM(6, 48, 33) TERM_ADD(6, 49, 37) \
+    TERM(7, 52, 27) TERM_ADD(7, 53, 31) STORE(5) \
+    TERM(0, 54, 37) \
+    TERM(1, 56, 35) TERM_ADD(1, 57, 39) \
+    TERM(2, 59, 25) \
+    TERM(3, 60, 13) \
+    TERM(4, 62, 22) \
+    TERM(5, 63, 13) \
+    TERM(6, 64, 16) \
+    TERM(7, 66, 19) TERM_ADD(7, 67, 25) STORE(6) \
+    TERM(0, 68, 16) \
+    TERM(1, 69, 13) \
+    TERM(2, 71, 16) \
+    TERM(3, 72, 19) \
+    TERM(4, 73, 22) \
+    TERM(5, 75, 13) \
+    TERM(6, 76, 22) \
+    TERM(7, 77, 19) TERM_ADD(7, 78, 25) STORE(7) \
+    TERM(0, 80, 16) \
+    TERM(1, 81, 25) \
+    TERM(2, 82, 22) \
+    TERM(3, 84, 13) \
+    TERM(4, 85, 25) \
+    TERM(5, 58, 26) \
+    TERM(6, 61, 28) \
+    TERM(7, 65, 30) STORE(8) \
+    TERM(0, 70, 32) \
+    TERM(1, 74, 34) \
+    TERM(2, 79, 36) \
+    TERM(3, 83, 38) \
+    v[4] = 0ull; \
+    v[5] = 0ull; \
+    v[6] = 0ull; \
+    v[7] = 0ull; STORE(9)
 
 // ---- shape S2: edge l_max=3, hidden L_max=2
 #define SXB_S2_LMAX 3
@@ -4133,350 +4215,544 @@
       { unsigned long long v; v = f2_mul(W(14), adj[0]); g[13] = f2_fma(v, x[13], g[13]); g[13] = f2_fma(v, x[13], g[13]); } \
       { unsigned long long v; v = f2_mul(W(15), adj[0]); g[14] = f2_fma(v, x[14], g[14]); g[14] = f2_fma(v, x[14], g[14]); } \
       { unsigned long long v; v = f2_mul(W(16), adj[0]); g[15] = f2_fma(v, x[15], g[15]); g[15] = f2_fma(v, x[15], g[15]); }
-#define SXB_S2_L1_REVERSE_EDGES_BODY \
-    { f2 y[kEdges][1]; EACH(load_pair_harmonics<0>(yrow[e], y[e]);) \
-    { /* path 0: edge l=0, source l=0 -> l=0 */ RADIAL(0) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(0); EACH(v[e][0] = f2_mul(h[e][0], w);) EACH(hadj[e][0] = f2_mul(t[e][0], w);) } \
-      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_mul(dR[e], yw[e]);) \
+#define SXB_S2_ROW_BATCHES 24
+#define SXB_S2_L1_REVERSE_EDGE_BODY \
+    { f2 y[1]; load_pair_harmonics<0>(yrow, y); \
+    { /* path 0: edge l=0, source l=0 -> l=0 */ RADIAL(0) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, y[0]); \
+      ROWS(0) { const f2 w = rows[0]; v[0] = f2_mul(h[0], w); hadj[0] = f2_mul(t[0], w); } \
+      yw = f2_mul(y[0], v[0]); \
+      radial = f2_mul(dR, yw); \
     } \
-    { /* path 4: edge l=0, source l=1 -> l=1 */ RADIAL(4) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(38); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(39); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(40); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_mul(t[e][0], w);) } \
-      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 4: edge l=0, source l=1 -> l=1 */ RADIAL(4) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[1]; v[0] = f2_mul(h[1], w); hadj[1] = f2_mul(t[0], w); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_mul(t[0], w); } \
+      { const f2 w = rows[3]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_mul(t[0], w); } \
+      yw = f2_mul(y[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 11: edge l=0, source l=2 -> l=2 */ RADIAL(11) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(141); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(142); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(143); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(144); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_mul(t[e][0], w);) } \
-      { const f2 w = ADJ(145); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_mul(t[e][0], w);) } \
-      EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 11: edge l=0, source l=2 -> l=2 */ RADIAL(11) f2 yw, t[5], v[5]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[4]; v[0] = f2_mul(h[4], w); hadj[4] = f2_mul(t[0], w); } \
+      { const f2 w = rows[5]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_mul(t[0], w); } \
+      { const f2 w = rows[6]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_mul(t[0], w); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_mul(t[0], w); } \
+      ROWS(1) { const f2 w = rows[0]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_mul(t[0], w); } \
+      yw = f2_mul(y[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
     } \
-    { f2 y[kEdges][3], ang[kEdges][3]; EACH(load_pair_harmonics<1>(yrow[e], y[e]);) \
-    { /* path 1: edge l=1, source l=1 -> l=0 */ RADIAL(1) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(1); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      EACH(ang[e][0] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(5); EACH(v[e][0] = f2_mul(h[e][2], w);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      EACH(ang[e][1] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(9); EACH(v[e][0] = f2_mul(h[e][3], w);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][2] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { f2 y[3], ang[3]; load_pair_harmonics<1>(yrow, y); \
+    { /* path 1: edge l=1, source l=1 -> l=0 */ RADIAL(1) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[1]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      ang[0] = f2_mul(R, v[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      { const f2 w = rows[2]; v[0] = f2_mul(h[2], w); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      ang[1] = f2_mul(R, v[0]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      { const f2 w = rows[3]; v[0] = f2_mul(h[3], w); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[2] = f2_mul(R, v[0]); yw = f2_fma(y[2], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 3: edge l=1, source l=0 -> l=1 */ RADIAL(3) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
-      { const f2 w = ADJ(35); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(36); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(37); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 3: edge l=1, source l=0 -> l=1 */ RADIAL(3) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, h[0]); \
+      { const f2 w = rows[4]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[5]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[6]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      hadj[0] = f2_fma(R, v[0], hadj[0]); yw = f2_mul(h[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 6: edge l=1, source l=2 -> l=1 */ RADIAL(6) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(56); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(57); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(58); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(60); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(62); EACH(v[e][0] = f2_mul(h[e][5], w);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(63); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(64); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(66); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(68); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(69); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(70); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 6: edge l=1, source l=2 -> l=1 */ RADIAL(6) f2 yw, t[5], v[5]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[7]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      ROWS(2) { const f2 w = rows[0]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[0] = f2_fma(R, v[0], ang[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      { const f2 w = rows[3]; v[0] = f2_mul(h[5], w); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[5]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      ang[1] = f2_fma(R, v[0], ang[1]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      { const f2 w = rows[6]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      ROWS(3) { const f2 w = rows[0]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[2] = f2_fma(R, v[0], ang[2]); yw = f2_fma(y[2], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 9: edge l=1, source l=1 -> l=2 */ RADIAL(9) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(111); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      { const f2 w = ADJ(112); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      { const f2 w = ADJ(113); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(114); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      { const f2 w = ADJ(115); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      { const f2 w = ADJ(116); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(117); EACH(v[e][0] = f2_mul(h[e][1], w);) EACH(hadj[e][1] = f2_fma(t[e][0], w, hadj[e][1]);) } \
-      { const f2 w = ADJ(118); EACH(v[e][0] = f2_fma(h[e][2], w, v[e][0]);) EACH(hadj[e][2] = f2_fma(t[e][0], w, hadj[e][2]);) } \
-      { const f2 w = ADJ(119); EACH(v[e][0] = f2_fma(h[e][3], w, v[e][0]);) EACH(hadj[e][3] = f2_fma(t[e][0], w, hadj[e][3]);) } \
-      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 9: edge l=1, source l=1 -> l=2 */ RADIAL(9) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[2]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      { const f2 w = rows[3]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[0] = f2_fma(R, v[0], ang[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      { const f2 w = rows[5]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      { const f2 w = rows[6]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[1] = f2_fma(R, v[0], ang[1]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      ROWS(4) { const f2 w = rows[0]; v[0] = f2_mul(h[1], w); hadj[1] = f2_fma(t[0], w, hadj[1]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[2], w, v[0]); hadj[2] = f2_fma(t[0], w, hadj[2]); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[3], w, v[0]); hadj[3] = f2_fma(t[0], w, hadj[3]); } \
+      ang[2] = f2_fma(R, v[0], ang[2]); yw = f2_fma(y[2], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 15: edge l=1, source l=2 -> l=3 */ RADIAL(15) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(193); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(194); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(195); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(196); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(197); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(198); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(199); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(200); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(201); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(202); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(203); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(204); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(205); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(206); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(207); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 15: edge l=1, source l=2 -> l=3 */ RADIAL(15) f2 yw, t[5], v[5]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[3]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[5]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[6]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[0] = f2_fma(R, v[0], ang[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      ROWS(5) { const f2 w = rows[0]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[3]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[1] = f2_fma(R, v[0], ang[1]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      { const f2 w = rows[5]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      { const f2 w = rows[6]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      ROWS(6) { const f2 w = rows[0]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[2] = f2_fma(R, v[0], ang[2]); yw = f2_fma(y[2], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-      EACH(add_angular_force<1>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+      f[1] = f2_sum(ang[0]); f[2] = f2_sum(ang[1]); f[3] = f2_sum(ang[2]); \
     } \
-    { f2 y[kEdges][5], ang[kEdges][5]; EACH(load_pair_harmonics<2>(yrow[e], y[e]);) \
-    { /* path 2: edge l=2, source l=2 -> l=0 */ RADIAL(2) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(10); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      EACH(ang[e][0] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(16); EACH(v[e][0] = f2_mul(h[e][5], w);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      EACH(ang[e][1] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(22); EACH(v[e][0] = f2_mul(h[e][6], w);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      EACH(ang[e][2] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][3]);) \
-      { const f2 w = ADJ(28); EACH(v[e][0] = f2_mul(h[e][7], w);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      EACH(ang[e][3] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][3], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][4]);) \
-      { const f2 w = ADJ(34); EACH(v[e][0] = f2_mul(h[e][8], w);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][4] = f2_mul(R[e], v[e][0]);) EACH(yw[e] = f2_fma(y[e][4], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { f2 y[5], ang[5]; load_pair_harmonics<2>(yrow, y); \
+    { /* path 2: edge l=2, source l=2 -> l=0 */ RADIAL(2) f2 yw, t[5], v[5]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[2]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      ang[0] = f2_mul(R, v[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      { const f2 w = rows[3]; v[0] = f2_mul(h[5], w); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      ang[1] = f2_mul(R, v[0]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      { const f2 w = rows[4]; v[0] = f2_mul(h[6], w); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      ang[2] = f2_mul(R, v[0]); yw = f2_fma(y[2], v[0], yw); \
+      t[0] = f2_mul(R, y[3]); \
+      { const f2 w = rows[5]; v[0] = f2_mul(h[7], w); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      ang[3] = f2_mul(R, v[0]); yw = f2_fma(y[3], v[0], yw); \
+      t[0] = f2_mul(R, y[4]); \
+      { const f2 w = rows[6]; v[0] = f2_mul(h[8], w); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[4] = f2_mul(R, v[0]); yw = f2_fma(y[4], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 5: edge l=2, source l=1 -> l=1 */ RADIAL(5) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
-      { const f2 w = ADJ(41); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(43); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(44); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(45); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
-      { const f2 w = ADJ(47); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(48); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(49); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
-      { const f2 w = ADJ(51); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(52); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(53); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(55); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
-      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
-      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 5: edge l=2, source l=1 -> l=1 */ RADIAL(5) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, h[1]); \
+      t[1] = f2_mul(R, h[2]); \
+      t[2] = f2_mul(R, h[3]); \
+      { const f2 w = rows[7]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      ROWS(7) { const f2 w = rows[0]; ang[0] = f2_fma(t[2], w, ang[0]); v[2] = f2_mul(y[0], w); } \
+      { const f2 w = rows[1]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[2]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_mul(y[1], w); } \
+      { const f2 w = rows[3]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      { const f2 w = rows[4]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[5]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_fma(y[2], w, v[2]); } \
+      { const f2 w = rows[6]; ang[3] = f2_fma(t[1], w, ang[3]); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[7]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      ROWS(8) { const f2 w = rows[0]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[1]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      hadj[1] = f2_fma(R, v[0], hadj[1]); yw = f2_mul(h[1], v[0]); \
+      hadj[2] = f2_fma(R, v[1], hadj[2]); yw = f2_fma(h[2], v[1], yw); \
+      hadj[3] = f2_fma(R, v[2], hadj[3]); yw = f2_fma(h[3], v[2], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 8: edge l=2, source l=0 -> l=2 */ RADIAL(8) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
-      { const f2 w = ADJ(106); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(107); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(108); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(109); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(110); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 8: edge l=2, source l=0 -> l=2 */ RADIAL(8) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, h[0]); \
+      { const f2 w = rows[2]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[3]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[4]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      { const f2 w = rows[5]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[6]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      hadj[0] = f2_fma(R, v[0], hadj[0]); yw = f2_mul(h[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 12: edge l=2, source l=2 -> l=2 */ RADIAL(12) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
-      EACH(t[e][0] = f2_mul(R[e], y[e][0]);) \
-      { const f2 w = ADJ(146); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(147); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(148); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(149); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      EACH(ang[e][0] = f2_fma(R[e], v[e][0], ang[e][0]);) EACH(yw[e] = f2_mul(y[e][0], v[e][0]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][1]);) \
-      { const f2 w = ADJ(151); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(152); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(153); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(154); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(155); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][1] = f2_fma(R[e], v[e][0], ang[e][1]);) EACH(yw[e] = f2_fma(y[e][1], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][2]);) \
-      { const f2 w = ADJ(156); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(157); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(158); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(159); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(160); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][2] = f2_fma(R[e], v[e][0], ang[e][2]);) EACH(yw[e] = f2_fma(y[e][2], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][3]);) \
-      { const f2 w = ADJ(161); EACH(v[e][0] = f2_mul(h[e][4], w);) EACH(hadj[e][4] = f2_fma(t[e][0], w, hadj[e][4]);) } \
-      { const f2 w = ADJ(162); EACH(v[e][0] = f2_fma(h[e][5], w, v[e][0]);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(163); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(164); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(165); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][3] = f2_fma(R[e], v[e][0], ang[e][3]);) EACH(yw[e] = f2_fma(y[e][3], v[e][0], yw[e]);) \
-      EACH(t[e][0] = f2_mul(R[e], y[e][4]);) \
-      { const f2 w = ADJ(167); EACH(v[e][0] = f2_mul(h[e][5], w);) EACH(hadj[e][5] = f2_fma(t[e][0], w, hadj[e][5]);) } \
-      { const f2 w = ADJ(168); EACH(v[e][0] = f2_fma(h[e][6], w, v[e][0]);) EACH(hadj[e][6] = f2_fma(t[e][0], w, hadj[e][6]);) } \
-      { const f2 w = ADJ(169); EACH(v[e][0] = f2_fma(h[e][7], w, v[e][0]);) EACH(hadj[e][7] = f2_fma(t[e][0], w, hadj[e][7]);) } \
-      { const f2 w = ADJ(170); EACH(v[e][0] = f2_fma(h[e][8], w, v[e][0]);) EACH(hadj[e][8] = f2_fma(t[e][0], w, hadj[e][8]);) } \
-      EACH(ang[e][4] = f2_fma(R[e], v[e][0], ang[e][4]);) EACH(yw[e] = f2_fma(y[e][4], v[e][0], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 12: edge l=2, source l=2 -> l=2 */ RADIAL(12) f2 yw, t[5], v[5]; \
+      t[0] = f2_mul(R, y[0]); \
+      { const f2 w = rows[7]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      ROWS(9) { const f2 w = rows[0]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      ang[0] = f2_fma(R, v[0], ang[0]); yw = f2_mul(y[0], v[0]); \
+      t[0] = f2_mul(R, y[1]); \
+      { const f2 w = rows[3]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[5]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[6]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[1] = f2_fma(R, v[0], ang[1]); yw = f2_fma(y[1], v[0], yw); \
+      t[0] = f2_mul(R, y[2]); \
+      ROWS(10) { const f2 w = rows[0]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[2]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[3]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[2] = f2_fma(R, v[0], ang[2]); yw = f2_fma(y[2], v[0], yw); \
+      t[0] = f2_mul(R, y[3]); \
+      { const f2 w = rows[5]; v[0] = f2_mul(h[4], w); hadj[4] = f2_fma(t[0], w, hadj[4]); } \
+      { const f2 w = rows[6]; v[0] = f2_fma(h[5], w, v[0]); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[7]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      ROWS(11) { const f2 w = rows[0]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[1]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[3] = f2_fma(R, v[0], ang[3]); yw = f2_fma(y[3], v[0], yw); \
+      t[0] = f2_mul(R, y[4]); \
+      { const f2 w = rows[2]; v[0] = f2_mul(h[5], w); hadj[5] = f2_fma(t[0], w, hadj[5]); } \
+      { const f2 w = rows[3]; v[0] = f2_fma(h[6], w, v[0]); hadj[6] = f2_fma(t[0], w, hadj[6]); } \
+      { const f2 w = rows[4]; v[0] = f2_fma(h[7], w, v[0]); hadj[7] = f2_fma(t[0], w, hadj[7]); } \
+      { const f2 w = rows[5]; v[0] = f2_fma(h[8], w, v[0]); hadj[8] = f2_fma(t[0], w, hadj[8]); } \
+      ang[4] = f2_fma(R, v[0], ang[4]); yw = f2_fma(y[4], v[0], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 14: edge l=2, source l=1 -> l=3 */ RADIAL(14) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
-      { const f2 w = ADJ(178); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(179); EACH(ang[e][0] = f2_fma(t[e][1], w, ang[e][0]);) EACH(v[e][1] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(180); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(181); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(182); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_fma(y[e][1], w, v[e][1]);) } \
-      { const f2 w = ADJ(183); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
-      { const f2 w = ADJ(184); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(185); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(186); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
-      { const f2 w = ADJ(187); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(188); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(189); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(190); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(191); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
-      { const f2 w = ADJ(192); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
-      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
-      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 14: edge l=2, source l=1 -> l=3 */ RADIAL(14) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, h[1]); \
+      t[1] = f2_mul(R, h[2]); \
+      t[2] = f2_mul(R, h[3]); \
+      { const f2 w = rows[6]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[7]; ang[0] = f2_fma(t[1], w, ang[0]); v[1] = f2_mul(y[0], w); } \
+      ROWS(12) { const f2 w = rows[0]; ang[0] = f2_fma(t[2], w, ang[0]); v[2] = f2_mul(y[0], w); } \
+      { const f2 w = rows[1]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[2]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_fma(y[1], w, v[1]); } \
+      { const f2 w = rows[3]; ang[1] = f2_fma(t[2], w, ang[1]); v[2] = f2_fma(y[1], w, v[2]); } \
+      { const f2 w = rows[4]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      { const f2 w = rows[5]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[6]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_fma(y[2], w, v[2]); } \
+      { const f2 w = rows[7]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      ROWS(13) { const f2 w = rows[0]; ang[3] = f2_fma(t[1], w, ang[3]); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[1]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      { const f2 w = rows[2]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[3]; ang[4] = f2_fma(t[1], w, ang[4]); v[1] = f2_fma(y[4], w, v[1]); } \
+      { const f2 w = rows[4]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      hadj[1] = f2_fma(R, v[0], hadj[1]); yw = f2_mul(h[1], v[0]); \
+      hadj[2] = f2_fma(R, v[1], hadj[2]); yw = f2_fma(h[2], v[1], yw); \
+      hadj[3] = f2_fma(R, v[2], hadj[3]); yw = f2_fma(h[3], v[2], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-      EACH(add_angular_force<2>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+      f[4] = f2_sum(ang[0]); f[5] = f2_sum(ang[1]); f[6] = f2_sum(ang[2]); f[7] = f2_sum(ang[3]); f[8] = f2_sum(ang[4]); \
     } \
-    { f2 y[kEdges][7], ang[kEdges][7]; EACH(load_pair_harmonics<3>(yrow[e], y[e]);) \
-    { /* path 7: edge l=3, source l=2 -> l=1 */ RADIAL(7) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][4]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][5]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][6]);) \
-      EACH(t[e][3] = f2_mul(R[e], h[e][7]);) \
-      EACH(t[e][4] = f2_mul(R[e], h[e][8]);) \
-      { const f2 w = ADJ(71); EACH(ang[e][0] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(75); EACH(ang[e][0] = f2_fma(t[e][4], w, ang[e][0]);) EACH(v[e][4] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(76); EACH(ang[e][1] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(77); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
-      { const f2 w = ADJ(79); EACH(ang[e][1] = f2_fma(t[e][3], w, ang[e][1]);) EACH(v[e][3] = f2_mul(y[e][1], w);) } \
-      { const f2 w = ADJ(81); EACH(ang[e][2] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(82); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(83); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_mul(y[e][2], w);) } \
-      { const f2 w = ADJ(85); EACH(ang[e][2] = f2_fma(t[e][4], w, ang[e][2]);) EACH(v[e][4] = f2_fma(y[e][2], w, v[e][4]);) } \
-      { const f2 w = ADJ(87); EACH(ang[e][3] = f2_mul(t[e][1], w);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(88); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(89); EACH(ang[e][3] = f2_fma(t[e][3], w, ang[e][3]);) EACH(v[e][3] = f2_fma(y[e][3], w, v[e][3]);) } \
-      { const f2 w = ADJ(91); EACH(ang[e][4] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(93); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      { const f2 w = ADJ(94); EACH(ang[e][4] = f2_fma(t[e][3], w, ang[e][4]);) EACH(v[e][3] = f2_fma(y[e][4], w, v[e][3]);) } \
-      { const f2 w = ADJ(95); EACH(ang[e][4] = f2_fma(t[e][4], w, ang[e][4]);) EACH(v[e][4] = f2_fma(y[e][4], w, v[e][4]);) } \
-      { const f2 w = ADJ(97); EACH(ang[e][5] = f2_mul(t[e][1], w);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
-      { const f2 w = ADJ(99); EACH(ang[e][5] = f2_fma(t[e][3], w, ang[e][5]);) EACH(v[e][3] = f2_fma(y[e][5], w, v[e][3]);) } \
-      { const f2 w = ADJ(100); EACH(ang[e][5] = f2_fma(t[e][4], w, ang[e][5]);) EACH(v[e][4] = f2_fma(y[e][5], w, v[e][4]);) } \
-      { const f2 w = ADJ(101); EACH(ang[e][6] = f2_mul(t[e][0], w);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
-      { const f2 w = ADJ(105); EACH(ang[e][6] = f2_fma(t[e][4], w, ang[e][6]);) EACH(v[e][4] = f2_fma(y[e][6], w, v[e][4]);) } \
-      EACH(hadj[e][4] = f2_fma(R[e], v[e][0], hadj[e][4]);) EACH(yw[e] = f2_mul(h[e][4], v[e][0]);) \
-      EACH(hadj[e][5] = f2_fma(R[e], v[e][1], hadj[e][5]);) EACH(yw[e] = f2_fma(h[e][5], v[e][1], yw[e]);) \
-      EACH(hadj[e][6] = f2_fma(R[e], v[e][2], hadj[e][6]);) EACH(yw[e] = f2_fma(h[e][6], v[e][2], yw[e]);) \
-      EACH(hadj[e][7] = f2_fma(R[e], v[e][3], hadj[e][7]);) EACH(yw[e] = f2_fma(h[e][7], v[e][3], yw[e]);) \
-      EACH(hadj[e][8] = f2_fma(R[e], v[e][4], hadj[e][8]);) EACH(yw[e] = f2_fma(h[e][8], v[e][4], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { f2 y[7], ang[7]; load_pair_harmonics<3>(yrow, y); \
+    { /* path 7: edge l=3, source l=2 -> l=1 */ RADIAL(7) f2 yw, t[5], v[5]; \
+      t[0] = f2_mul(R, h[4]); \
+      t[1] = f2_mul(R, h[5]); \
+      t[2] = f2_mul(R, h[6]); \
+      t[3] = f2_mul(R, h[7]); \
+      t[4] = f2_mul(R, h[8]); \
+      { const f2 w = rows[5]; ang[0] = f2_mul(t[0], w); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[6]; ang[0] = f2_fma(t[4], w, ang[0]); v[4] = f2_mul(y[0], w); } \
+      { const f2 w = rows[7]; ang[1] = f2_mul(t[0], w); v[0] = f2_fma(y[1], w, v[0]); } \
+      ROWS(14) { const f2 w = rows[0]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_mul(y[1], w); } \
+      { const f2 w = rows[1]; ang[1] = f2_fma(t[3], w, ang[1]); v[3] = f2_mul(y[1], w); } \
+      { const f2 w = rows[2]; ang[2] = f2_mul(t[0], w); v[0] = f2_fma(y[2], w, v[0]); } \
+      { const f2 w = rows[3]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[4]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_mul(y[2], w); } \
+      { const f2 w = rows[5]; ang[2] = f2_fma(t[4], w, ang[2]); v[4] = f2_fma(y[2], w, v[4]); } \
+      { const f2 w = rows[6]; ang[3] = f2_mul(t[1], w); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[7]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      ROWS(15) { const f2 w = rows[0]; ang[3] = f2_fma(t[3], w, ang[3]); v[3] = f2_fma(y[3], w, v[3]); } \
+      { const f2 w = rows[1]; ang[4] = f2_mul(t[0], w); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[2]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      { const f2 w = rows[3]; ang[4] = f2_fma(t[3], w, ang[4]); v[3] = f2_fma(y[4], w, v[3]); } \
+      { const f2 w = rows[4]; ang[4] = f2_fma(t[4], w, ang[4]); v[4] = f2_fma(y[4], w, v[4]); } \
+      { const f2 w = rows[5]; ang[5] = f2_mul(t[1], w); v[1] = f2_fma(y[5], w, v[1]); } \
+      { const f2 w = rows[6]; ang[5] = f2_fma(t[3], w, ang[5]); v[3] = f2_fma(y[5], w, v[3]); } \
+      { const f2 w = rows[7]; ang[5] = f2_fma(t[4], w, ang[5]); v[4] = f2_fma(y[5], w, v[4]); } \
+      ROWS(16) { const f2 w = rows[0]; ang[6] = f2_mul(t[0], w); v[0] = f2_fma(y[6], w, v[0]); } \
+      { const f2 w = rows[1]; ang[6] = f2_fma(t[4], w, ang[6]); v[4] = f2_fma(y[6], w, v[4]); } \
+      hadj[4] = f2_fma(R, v[0], hadj[4]); yw = f2_mul(h[4], v[0]); \
+      hadj[5] = f2_fma(R, v[1], hadj[5]); yw = f2_fma(h[5], v[1], yw); \
+      hadj[6] = f2_fma(R, v[2], hadj[6]); yw = f2_fma(h[6], v[2], yw); \
+      hadj[7] = f2_fma(R, v[3], hadj[7]); yw = f2_fma(h[7], v[3], yw); \
+      hadj[8] = f2_fma(R, v[4], hadj[8]); yw = f2_fma(h[8], v[4], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 10: edge l=3, source l=1 -> l=2 */ RADIAL(10) f2 yw[kEdges], t[kEdges][3], v[kEdges][3]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][1]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][2]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][3]);) \
-      { const f2 w = ADJ(120); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(122); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(123); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(124); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_mul(y[e][1], w);) } \
-      { const f2 w = ADJ(125); EACH(ang[e][1] = f2_fma(t[e][2], w, ang[e][1]);) EACH(v[e][2] = f2_fma(y[e][1], w, v[e][2]);) } \
-      { const f2 w = ADJ(126); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(127); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(128); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
-      { const f2 w = ADJ(129); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(130); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(131); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(132); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(133); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
-      { const f2 w = ADJ(134); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      { const f2 w = ADJ(135); EACH(ang[e][5] = f2_fma(t[e][0], w, ang[e][5]);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
-      { const f2 w = ADJ(136); EACH(ang[e][5] = f2_fma(t[e][1], w, ang[e][5]);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
-      { const f2 w = ADJ(137); EACH(ang[e][5] = f2_fma(t[e][2], w, ang[e][5]);) EACH(v[e][2] = f2_fma(y[e][5], w, v[e][2]);) } \
-      { const f2 w = ADJ(138); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
-      { const f2 w = ADJ(140); EACH(ang[e][6] = f2_fma(t[e][2], w, ang[e][6]);) EACH(v[e][2] = f2_fma(y[e][6], w, v[e][2]);) } \
-      EACH(hadj[e][1] = f2_fma(R[e], v[e][0], hadj[e][1]);) EACH(yw[e] = f2_mul(h[e][1], v[e][0]);) \
-      EACH(hadj[e][2] = f2_fma(R[e], v[e][1], hadj[e][2]);) EACH(yw[e] = f2_fma(h[e][2], v[e][1], yw[e]);) \
-      EACH(hadj[e][3] = f2_fma(R[e], v[e][2], hadj[e][3]);) EACH(yw[e] = f2_fma(h[e][3], v[e][2], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 10: edge l=3, source l=1 -> l=2 */ RADIAL(10) f2 yw, t[3], v[3]; \
+      t[0] = f2_mul(R, h[1]); \
+      t[1] = f2_mul(R, h[2]); \
+      t[2] = f2_mul(R, h[3]); \
+      { const f2 w = rows[2]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[3]; ang[0] = f2_fma(t[2], w, ang[0]); v[2] = f2_mul(y[0], w); } \
+      { const f2 w = rows[4]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[5]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_mul(y[1], w); } \
+      { const f2 w = rows[6]; ang[1] = f2_fma(t[2], w, ang[1]); v[2] = f2_fma(y[1], w, v[2]); } \
+      { const f2 w = rows[7]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      ROWS(17) { const f2 w = rows[0]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[1]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_fma(y[2], w, v[2]); } \
+      { const f2 w = rows[2]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[3]; ang[3] = f2_fma(t[1], w, ang[3]); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[4]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      { const f2 w = rows[5]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[6]; ang[4] = f2_fma(t[1], w, ang[4]); v[1] = f2_fma(y[4], w, v[1]); } \
+      { const f2 w = rows[7]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      ROWS(18) { const f2 w = rows[0]; ang[5] = f2_fma(t[0], w, ang[5]); v[0] = f2_fma(y[5], w, v[0]); } \
+      { const f2 w = rows[1]; ang[5] = f2_fma(t[1], w, ang[5]); v[1] = f2_fma(y[5], w, v[1]); } \
+      { const f2 w = rows[2]; ang[5] = f2_fma(t[2], w, ang[5]); v[2] = f2_fma(y[5], w, v[2]); } \
+      { const f2 w = rows[3]; ang[6] = f2_fma(t[0], w, ang[6]); v[0] = f2_fma(y[6], w, v[0]); } \
+      { const f2 w = rows[4]; ang[6] = f2_fma(t[2], w, ang[6]); v[2] = f2_fma(y[6], w, v[2]); } \
+      hadj[1] = f2_fma(R, v[0], hadj[1]); yw = f2_mul(h[1], v[0]); \
+      hadj[2] = f2_fma(R, v[1], hadj[2]); yw = f2_fma(h[2], v[1], yw); \
+      hadj[3] = f2_fma(R, v[2], hadj[3]); yw = f2_fma(h[3], v[2], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 13: edge l=3, source l=0 -> l=3 */ RADIAL(13) f2 yw[kEdges], t[kEdges][1], v[kEdges][1]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][0]);) \
-      { const f2 w = ADJ(171); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(172); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(173); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(174); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(175); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(176); EACH(ang[e][5] = f2_fma(t[e][0], w, ang[e][5]);) EACH(v[e][0] = f2_fma(y[e][5], w, v[e][0]);) } \
-      { const f2 w = ADJ(177); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
-      EACH(hadj[e][0] = f2_fma(R[e], v[e][0], hadj[e][0]);) EACH(yw[e] = f2_mul(h[e][0], v[e][0]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 13: edge l=3, source l=0 -> l=3 */ RADIAL(13) f2 yw, t[1], v[1]; \
+      t[0] = f2_mul(R, h[0]); \
+      { const f2 w = rows[5]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[6]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[7]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      ROWS(19) { const f2 w = rows[0]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[1]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[2]; ang[5] = f2_fma(t[0], w, ang[5]); v[0] = f2_fma(y[5], w, v[0]); } \
+      { const f2 w = rows[3]; ang[6] = f2_fma(t[0], w, ang[6]); v[0] = f2_fma(y[6], w, v[0]); } \
+      hadj[0] = f2_fma(R, v[0], hadj[0]); yw = f2_mul(h[0], v[0]); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-    { /* path 16: edge l=3, source l=2 -> l=3 */ RADIAL(16) f2 yw[kEdges], t[kEdges][5], v[kEdges][5]; \
-      EACH(t[e][0] = f2_mul(R[e], h[e][4]);) \
-      EACH(t[e][1] = f2_mul(R[e], h[e][5]);) \
-      EACH(t[e][2] = f2_mul(R[e], h[e][6]);) \
-      EACH(t[e][3] = f2_mul(R[e], h[e][7]);) \
-      EACH(t[e][4] = f2_mul(R[e], h[e][8]);) \
-      { const f2 w = ADJ(208); EACH(ang[e][0] = f2_fma(t[e][0], w, ang[e][0]);) EACH(v[e][0] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(209); EACH(ang[e][0] = f2_fma(t[e][1], w, ang[e][0]);) EACH(v[e][1] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(210); EACH(ang[e][0] = f2_fma(t[e][2], w, ang[e][0]);) EACH(v[e][2] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(211); EACH(ang[e][0] = f2_fma(t[e][3], w, ang[e][0]);) EACH(v[e][3] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(212); EACH(ang[e][0] = f2_fma(t[e][4], w, ang[e][0]);) EACH(v[e][4] = f2_mul(y[e][0], w);) } \
-      { const f2 w = ADJ(213); EACH(ang[e][1] = f2_fma(t[e][0], w, ang[e][1]);) EACH(v[e][0] = f2_fma(y[e][1], w, v[e][0]);) } \
-      { const f2 w = ADJ(214); EACH(ang[e][1] = f2_fma(t[e][1], w, ang[e][1]);) EACH(v[e][1] = f2_fma(y[e][1], w, v[e][1]);) } \
-      { const f2 w = ADJ(216); EACH(ang[e][1] = f2_fma(t[e][3], w, ang[e][1]);) EACH(v[e][3] = f2_fma(y[e][1], w, v[e][3]);) } \
-      { const f2 w = ADJ(218); EACH(ang[e][2] = f2_fma(t[e][0], w, ang[e][2]);) EACH(v[e][0] = f2_fma(y[e][2], w, v[e][0]);) } \
-      { const f2 w = ADJ(219); EACH(ang[e][2] = f2_fma(t[e][1], w, ang[e][2]);) EACH(v[e][1] = f2_fma(y[e][2], w, v[e][1]);) } \
-      { const f2 w = ADJ(220); EACH(ang[e][2] = f2_fma(t[e][2], w, ang[e][2]);) EACH(v[e][2] = f2_fma(y[e][2], w, v[e][2]);) } \
-      { const f2 w = ADJ(221); EACH(ang[e][2] = f2_fma(t[e][3], w, ang[e][2]);) EACH(v[e][3] = f2_fma(y[e][2], w, v[e][3]);) } \
-      { const f2 w = ADJ(222); EACH(ang[e][2] = f2_fma(t[e][4], w, ang[e][2]);) EACH(v[e][4] = f2_fma(y[e][2], w, v[e][4]);) } \
-      { const f2 w = ADJ(223); EACH(ang[e][3] = f2_fma(t[e][0], w, ang[e][3]);) EACH(v[e][0] = f2_fma(y[e][3], w, v[e][0]);) } \
-      { const f2 w = ADJ(224); EACH(ang[e][3] = f2_fma(t[e][1], w, ang[e][3]);) EACH(v[e][1] = f2_fma(y[e][3], w, v[e][1]);) } \
-      { const f2 w = ADJ(225); EACH(ang[e][3] = f2_fma(t[e][2], w, ang[e][3]);) EACH(v[e][2] = f2_fma(y[e][3], w, v[e][2]);) } \
-      { const f2 w = ADJ(226); EACH(ang[e][3] = f2_fma(t[e][3], w, ang[e][3]);) EACH(v[e][3] = f2_fma(y[e][3], w, v[e][3]);) } \
-      { const f2 w = ADJ(227); EACH(ang[e][3] = f2_fma(t[e][4], w, ang[e][3]);) EACH(v[e][4] = f2_fma(y[e][3], w, v[e][4]);) } \
-      { const f2 w = ADJ(228); EACH(ang[e][4] = f2_fma(t[e][0], w, ang[e][4]);) EACH(v[e][0] = f2_fma(y[e][4], w, v[e][0]);) } \
-      { const f2 w = ADJ(229); EACH(ang[e][4] = f2_fma(t[e][1], w, ang[e][4]);) EACH(v[e][1] = f2_fma(y[e][4], w, v[e][1]);) } \
-      { const f2 w = ADJ(230); EACH(ang[e][4] = f2_fma(t[e][2], w, ang[e][4]);) EACH(v[e][2] = f2_fma(y[e][4], w, v[e][2]);) } \
-      { const f2 w = ADJ(231); EACH(ang[e][4] = f2_fma(t[e][3], w, ang[e][4]);) EACH(v[e][3] = f2_fma(y[e][4], w, v[e][3]);) } \
-      { const f2 w = ADJ(232); EACH(ang[e][4] = f2_fma(t[e][4], w, ang[e][4]);) EACH(v[e][4] = f2_fma(y[e][4], w, v[e][4]);) } \
-      { const f2 w = ADJ(234); EACH(ang[e][5] = f2_fma(t[e][1], w, ang[e][5]);) EACH(v[e][1] = f2_fma(y[e][5], w, v[e][1]);) } \
-      { const f2 w = ADJ(236); EACH(ang[e][5] = f2_fma(t[e][3], w, ang[e][5]);) EACH(v[e][3] = f2_fma(y[e][5], w, v[e][3]);) } \
-      { const f2 w = ADJ(237); EACH(ang[e][5] = f2_fma(t[e][4], w, ang[e][5]);) EACH(v[e][4] = f2_fma(y[e][5], w, v[e][4]);) } \
-      { const f2 w = ADJ(238); EACH(ang[e][6] = f2_fma(t[e][0], w, ang[e][6]);) EACH(v[e][0] = f2_fma(y[e][6], w, v[e][0]);) } \
-      { const f2 w = ADJ(239); EACH(ang[e][6] = f2_fma(t[e][1], w, ang[e][6]);) EACH(v[e][1] = f2_fma(y[e][6], w, v[e][1]);) } \
-      { const f2 w = ADJ(240); EACH(ang[e][6] = f2_fma(t[e][2], w, ang[e][6]);) EACH(v[e][2] = f2_fma(y[e][6], w, v[e][2]);) } \
-      { const f2 w = ADJ(241); EACH(ang[e][6] = f2_fma(t[e][3], w, ang[e][6]);) EACH(v[e][3] = f2_fma(y[e][6], w, v[e][3]);) } \
-      { const f2 w = ADJ(242); EACH(ang[e][6] = f2_fma(t[e][4], w, ang[e][6]);) EACH(v[e][4] = f2_fma(y[e][6], w, v[e][4]);) } \
-      EACH(hadj[e][4] = f2_fma(R[e], v[e][0], hadj[e][4]);) EACH(yw[e] = f2_mul(h[e][4], v[e][0]);) \
-      EACH(hadj[e][5] = f2_fma(R[e], v[e][1], hadj[e][5]);) EACH(yw[e] = f2_fma(h[e][5], v[e][1], yw[e]);) \
-      EACH(hadj[e][6] = f2_fma(R[e], v[e][2], hadj[e][6]);) EACH(yw[e] = f2_fma(h[e][6], v[e][2], yw[e]);) \
-      EACH(hadj[e][7] = f2_fma(R[e], v[e][3], hadj[e][7]);) EACH(yw[e] = f2_fma(h[e][7], v[e][3], yw[e]);) \
-      EACH(hadj[e][8] = f2_fma(R[e], v[e][4], hadj[e][8]);) EACH(yw[e] = f2_fma(h[e][8], v[e][4], yw[e]);) \
-      EACH(radial[e] = f2_fma(dR[e], yw[e], radial[e]);) \
+    { /* path 16: edge l=3, source l=2 -> l=3 */ RADIAL(16) f2 yw, t[5], v[5]; \
+      t[0] = f2_mul(R, h[4]); \
+      t[1] = f2_mul(R, h[5]); \
+      t[2] = f2_mul(R, h[6]); \
+      t[3] = f2_mul(R, h[7]); \
+      t[4] = f2_mul(R, h[8]); \
+      { const f2 w = rows[4]; ang[0] = f2_fma(t[0], w, ang[0]); v[0] = f2_mul(y[0], w); } \
+      { const f2 w = rows[5]; ang[0] = f2_fma(t[1], w, ang[0]); v[1] = f2_mul(y[0], w); } \
+      { const f2 w = rows[6]; ang[0] = f2_fma(t[2], w, ang[0]); v[2] = f2_mul(y[0], w); } \
+      { const f2 w = rows[7]; ang[0] = f2_fma(t[3], w, ang[0]); v[3] = f2_mul(y[0], w); } \
+      ROWS(20) { const f2 w = rows[0]; ang[0] = f2_fma(t[4], w, ang[0]); v[4] = f2_mul(y[0], w); } \
+      { const f2 w = rows[1]; ang[1] = f2_fma(t[0], w, ang[1]); v[0] = f2_fma(y[1], w, v[0]); } \
+      { const f2 w = rows[2]; ang[1] = f2_fma(t[1], w, ang[1]); v[1] = f2_fma(y[1], w, v[1]); } \
+      { const f2 w = rows[3]; ang[1] = f2_fma(t[3], w, ang[1]); v[3] = f2_fma(y[1], w, v[3]); } \
+      { const f2 w = rows[4]; ang[2] = f2_fma(t[0], w, ang[2]); v[0] = f2_fma(y[2], w, v[0]); } \
+      { const f2 w = rows[5]; ang[2] = f2_fma(t[1], w, ang[2]); v[1] = f2_fma(y[2], w, v[1]); } \
+      { const f2 w = rows[6]; ang[2] = f2_fma(t[2], w, ang[2]); v[2] = f2_fma(y[2], w, v[2]); } \
+      { const f2 w = rows[7]; ang[2] = f2_fma(t[3], w, ang[2]); v[3] = f2_fma(y[2], w, v[3]); } \
+      ROWS(21) { const f2 w = rows[0]; ang[2] = f2_fma(t[4], w, ang[2]); v[4] = f2_fma(y[2], w, v[4]); } \
+      { const f2 w = rows[1]; ang[3] = f2_fma(t[0], w, ang[3]); v[0] = f2_fma(y[3], w, v[0]); } \
+      { const f2 w = rows[2]; ang[3] = f2_fma(t[1], w, ang[3]); v[1] = f2_fma(y[3], w, v[1]); } \
+      { const f2 w = rows[3]; ang[3] = f2_fma(t[2], w, ang[3]); v[2] = f2_fma(y[3], w, v[2]); } \
+      { const f2 w = rows[4]; ang[3] = f2_fma(t[3], w, ang[3]); v[3] = f2_fma(y[3], w, v[3]); } \
+      { const f2 w = rows[5]; ang[3] = f2_fma(t[4], w, ang[3]); v[4] = f2_fma(y[3], w, v[4]); } \
+      { const f2 w = rows[6]; ang[4] = f2_fma(t[0], w, ang[4]); v[0] = f2_fma(y[4], w, v[0]); } \
+      { const f2 w = rows[7]; ang[4] = f2_fma(t[1], w, ang[4]); v[1] = f2_fma(y[4], w, v[1]); } \
+      ROWS(22) { const f2 w = rows[0]; ang[4] = f2_fma(t[2], w, ang[4]); v[2] = f2_fma(y[4], w, v[2]); } \
+      { const f2 w = rows[1]; ang[4] = f2_fma(t[3], w, ang[4]); v[3] = f2_fma(y[4], w, v[3]); } \
+      { const f2 w = rows[2]; ang[4] = f2_fma(t[4], w, ang[4]); v[4] = f2_fma(y[4], w, v[4]); } \
+      { const f2 w = rows[3]; ang[5] = f2_fma(t[1], w, ang[5]); v[1] = f2_fma(y[5], w, v[1]); } \
+      { const f2 w = rows[4]; ang[5] = f2_fma(t[3], w, ang[5]); v[3] = f2_fma(y[5], w, v[3]); } \
+      { const f2 w = rows[5]; ang[5] = f2_fma(t[4], w, ang[5]); v[4] = f2_fma(y[5], w, v[4]); } \
+      { const f2 w = rows[6]; ang[6] = f2_fma(t[0], w, ang[6]); v[0] = f2_fma(y[6], w, v[0]); } \
+      { const f2 w = rows[7]; ang[6] = f2_fma(t[1], w, ang[6]); v[1] = f2_fma(y[6], w, v[1]); } \
+      ROWS(23) { const f2 w = rows[0]; ang[6] = f2_fma(t[2], w, ang[6]); v[2] = f2_fma(y[6], w, v[2]); } \
+      { const f2 w = rows[1]; ang[6] = f2_fma(t[3], w, ang[6]); v[3] = f2_fma(y[6], w, v[3]); } \
+      { const f2 w = rows[2]; ang[6] = f2_fma(t[4], w, ang[6]); v[4] = f2_fma(y[6], w, v[4]); } \
+      hadj[4] = f2_fma(R, v[0], hadj[4]); yw = f2_mul(h[4], v[0]); \
+      hadj[5] = f2_fma(R, v[1], hadj[5]); yw = f2_fma(h[5], v[1], yw); \
+      hadj[6] = f2_fma(R, v[2], hadj[6]); yw = f2_fma(h[6], v[2], yw); \
+      hadj[7] = f2_fma(R, v[3], hadj[7]); yw = f2_fma(h[7], v[3], yw); \
+      hadj[8] = f2_fma(R, v[4], hadj[8]); yw = f2_fma(h[8], v[4], yw); \
+      radial = f2_fma(dR, yw, radial); \
     } \
-      EACH(add_angular_force<3>(grow[e], ang[e], fx[e], fy[e], fz[e]);) \
+      f[9] = f2_sum(ang[0]); f[10] = f2_sum(ang[1]); f[11] = f2_sum(ang[2]); f[12] = f2_sum(ang[3]); f[13] = f2_sum(ang[4]); f[14] = f2_sum(ang[5]); f[15] = f2_sum(ang[6]); \
     }
+#define SXB_S2_L1_ADJOINT_ROWS \
+    TERM(0, 0, 0) \
+    TERM(1, 1, 4) \
+    TERM(2, 2, 9) \
+    TERM(3, 3, 14) \
+    TERM(4, 4, 21) \
+    TERM(5, 5, 26) \
+    TERM(6, 6, 31) \
+    TERM(7, 7, 36) STORE(0) \
+    TERM(0, 8, 41) \
+    TERM(1, 10, 1) \
+    TERM(2, 29, 1) \
+    TERM(3, 43, 1) \
+    TERM(4, 9, 3) \
+    TERM(5, 27, 8) \
+    TERM(6, 40, 13) \
+    TERM(7, 15, 16) STORE(1) \
+    TERM(0, 18, 11) \
+    TERM(1, 21, 6) \
+    TERM(2, 24, 6) \
+    TERM(3, 33, 6) \
+    TERM(4, 35, 11) \
+    TERM(5, 37, 16) \
+    TERM(6, 46, 6) \
+    TERM(7, 50, 16) STORE(2) \
+    TERM(0, 52, 11) \
+    TERM(1, 55, 16) \
+    TERM(2, 11, 29) TERM_ADD(2, 12, 39) \
+    TERM(3, 13, 24) \
+    TERM(4, 14, 19) \
+    TERM(5, 28, 24) \
+    TERM(6, 30, 29) \
+    TERM(7, 31, 34) STORE(3) \
+    TERM(0, 41, 19) \
+    TERM(1, 42, 34) \
+    TERM(2, 44, 29) TERM_ADD(2, 45, 39) \
+    TERM(3, 16, 61) TERM_ADD(3, 17, 69) \
+    TERM(4, 19, 57) TERM_ADD(4, 20, 65) \
+    TERM(5, 22, 53) \
+    TERM(6, 23, 49) \
+    TERM(7, 25, 45) TERM_ADD(7, 26, 53) STORE(4) \
+    TERM(0, 32, 49) \
+    TERM(1, 34, 53) \
+    TERM(2, 36, 57) \
+    TERM(3, 38, 61) \
+    TERM(4, 39, 65) \
+    TERM(5, 47, 45) TERM_ADD(5, 48, 53) \
+    TERM(6, 49, 49) \
+    TERM(7, 51, 61) STORE(5) \
+    TERM(0, 53, 57) TERM_ADD(0, 54, 65) \
+    TERM(1, 56, 61) TERM_ADD(1, 57, 69) \
+    TERM(2, 66, 2) \
+    TERM(3, 79, 2) \
+    TERM(4, 94, 2) \
+    TERM(5, 108, 2) \
+    TERM(6, 123, 2) \
+    TERM(7, 59, 15) STORE(6) \
+    TERM(0, 63, 5) \
+    TERM(1, 72, 10) \
+    TERM(2, 75, 5) \
+    TERM(3, 86, 5) \
+    TERM(4, 88, 10) \
+    TERM(5, 90, 15) \
+    TERM(6, 100, 15) \
+    TERM(7, 102, 10) STORE(7) \
+    TERM(0, 113, 5) \
+    TERM(1, 117, 15) \
+    TERM(2, 58, 18) \
+    TERM(3, 71, 23) \
+    TERM(4, 85, 28) \
+    TERM(5, 98, 33) \
+    TERM(6, 112, 38) \
+    TERM(7, 67, 32) STORE(8) \
+    TERM(0, 68, 37) \
+    TERM(1, 69, 22) \
+    TERM(2, 70, 27) \
+    TERM(3, 78, 37) \
+    TERM(4, 80, 32) TERM_ADD(4, 81, 42) \
+    TERM(5, 82, 27) \
+    TERM(6, 83, 22) \
+    TERM(7, 84, 27) STORE(9) \
+    TERM(0, 92, 22) \
+    TERM(1, 93, 27) \
+    TERM(2, 95, 32) \
+    TERM(3, 96, 37) \
+    TERM(4, 97, 42) \
+    TERM(5, 105, 27) \
+    TERM(6, 106, 22) \
+    TERM(7, 107, 37) STORE(10) \
+    TERM(0, 109, 32) TERM_ADD(0, 110, 42) \
+    TERM(1, 111, 37) \
+    TERM(2, 120, 27) \
+    TERM(3, 121, 42) \
+    TERM(4, 122, 37) \
+    TERM(5, 124, 32) \
+    TERM(6, 60, 60) TERM_ADD(6, 61, 68) \
+    TERM(7, 62, 48) STORE(11) \
+    TERM(0, 64, 44) TERM_ADD(0, 65, 52) \
+    TERM(1, 73, 56) TERM_ADD(1, 74, 64) \
+    TERM(2, 76, 52) \
+    TERM(3, 77, 48) \
+    TERM(4, 87, 52) \
+    TERM(5, 89, 56) \
+    TERM(6, 91, 60) \
+    TERM(7, 99, 48) STORE(12) \
+    TERM(0, 101, 60) \
+    TERM(1, 103, 56) TERM_ADD(1, 104, 64) \
+    TERM(2, 114, 44) TERM_ADD(2, 115, 52) \
+    TERM(3, 116, 64) \
+    TERM(4, 118, 60) TERM_ADD(4, 119, 68) \
+    TERM(5, 128, 17) \
+    TERM(6, 133, 7) \
+    TERM(7, 139, 12) STORE(13) \
+    TERM(0, 141, 17) \
+    TERM(1, 144, 7) \
+    TERM(2, 152, 17) \
+    TERM(3, 155, 12) \
+    TERM(4, 158, 7) \
+    TERM(5, 161, 7) \
+    TERM(6, 169, 7) \
+    TERM(7, 171, 12) STORE(14) \
+    TERM(0, 173, 17) \
+    TERM(1, 181, 7) \
+    TERM(2, 185, 17) \
+    TERM(3, 187, 12) \
+    TERM(4, 190, 17) \
+    TERM(5, 197, 7) \
+    TERM(6, 200, 17) \
+    TERM(7, 203, 12) STORE(15) \
+    TERM(0, 208, 7) \
+    TERM(1, 213, 17) \
+    TERM(2, 126, 40) \
+    TERM(3, 127, 20) \
+    TERM(4, 136, 35) \
+    TERM(5, 137, 20) \
+    TERM(6, 138, 25) \
+    TERM(7, 148, 30) TERM_ADD(7, 149, 40) STORE(16) \
+    TERM(0, 150, 25) \
+    TERM(1, 151, 20) \
+    TERM(2, 165, 25) \
+    TERM(3, 166, 30) \
+    TERM(4, 167, 35) \
+    TERM(5, 177, 20) \
+    TERM(6, 178, 35) \
+    TERM(7, 179, 30) TERM_ADD(7, 180, 40) STORE(17) \
+    TERM(0, 194, 25) \
+    TERM(1, 195, 40) \
+    TERM(2, 196, 35) \
+    TERM(3, 206, 20) \
+    TERM(4, 207, 40) \
+    TERM(5, 125, 43) \
+    TERM(6, 135, 47) \
+    TERM(7, 147, 51) STORE(18) \
+    TERM(0, 164, 55) \
+    TERM(1, 176, 59) \
+    TERM(2, 193, 63) \
+    TERM(3, 205, 67) \
+    TERM(4, 129, 62) \
+    TERM(5, 130, 66) \
+    TERM(6, 131, 46) \
+    TERM(7, 132, 50) STORE(19) \
+    TERM(0, 134, 54) \
+    TERM(1, 140, 58) \
+    TERM(2, 142, 62) TERM_ADD(2, 143, 70) \
+    TERM(3, 145, 46) TERM_ADD(3, 146, 54) \
+    TERM(4, 153, 62) TERM_ADD(4, 154, 70) \
+    TERM(5, 156, 58) TERM_ADD(5, 157, 66) \
+    TERM(6, 159, 54) \
+    TERM(7, 160, 50) STORE(20) \
+    TERM(0, 162, 46) TERM_ADD(0, 163, 54) \
+    TERM(1, 168, 50) \
+    TERM(2, 170, 54) \
+    TERM(3, 172, 58) \
+    TERM(4, 174, 62) \
+    TERM(5, 175, 66) \
+    TERM(6, 182, 46) TERM_ADD(6, 183, 54) \
+    TERM(7, 184, 50) STORE(21) \
+    TERM(0, 186, 62) \
+    TERM(1, 188, 58) TERM_ADD(1, 189, 66) \
+    TERM(2, 191, 62) TERM_ADD(2, 192, 70) \
+    TERM(3, 198, 46) TERM_ADD(3, 199, 54) \
+    TERM(4, 201, 62) TERM_ADD(4, 202, 70) \
+    TERM(5, 204, 58) \
+    TERM(6, 209, 54) \
+    TERM(7, 210, 50) STORE(22) \
+    TERM(0, 211, 70) \
+    TERM(1, 212, 66) \
+    TERM(2, 214, 62) \
+    v[3] = 0ull; \
+    v[4] = 0ull; \
+    v[5] = 0ull; \
+    v[6] = 0ull; \
+    v[7] = 0ull; STORE(23)
 #define SXB_S2_NUM_GROUPS 3
 #define SXB_S2_G0_NUM_PATHS 10
 #define SXB_S2_G0_NUM_ROWS 88

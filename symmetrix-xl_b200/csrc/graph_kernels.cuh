@@ -176,8 +176,10 @@ receiver_edges_kernel(int num_receivers, CellGrid grid, const int* __restrict__ 
 
 // Re-expresses a CSR graph given in caller node order in the internal order (nodes grouped by
 // element): receiver ``new`` is caller node ``original[new]``; its edge list keeps its order and
-// its sources are renumbered.  ``edge_map[new_edge]`` = caller edge index.
-__global__ void permute_graph_kernel(int n, const int* __restrict__ original, const int* __restrict__ internal_of,
+// its sources are renumbered.  ``edge_map[new_edge]`` = caller edge index.  With types > 1 the edges of a receiver are
+// stably grouped by the active type of their source.
+__global__ void permute_graph_kernel(int n, int types, const unsigned char* __restrict__ atype, const int* __restrict__ original,
+                                     const int* __restrict__ internal_of,
                                      const int* __restrict__ old_first, const int* __restrict__ old_sources,
                                      const int* __restrict__ old_shifts, const int* __restrict__ new_first,
                                      int* __restrict__ new_sources, int* __restrict__ new_shifts, int* __restrict__ edge_map)
@@ -188,16 +190,25 @@ __global__ void permute_graph_kernel(int n, const int* __restrict__ original, co
     const int old_node = original[warp];
     const int ob = old_first[old_node], count = old_first[old_node + 1] - ob;
     const int nb = new_first[warp];
-    for (int t = lane; t < count; t += 32) {
-        new_sources[nb + t] = internal_of[old_sources[ob + t]];
-        edge_map[nb + t] = ob + t;
-        if (old_shifts != nullptr) {
-            const size_t to = 3 * static_cast<size_t>(nb + t), from = 3 * static_cast<size_t>(ob + t);
-            new_shifts[to] = old_shifts[from];
-            new_shifts[to + 1] = old_shifts[from + 1];
-            new_shifts[to + 2] = old_shifts[from + 2];
+    int written = 0;
+    for (int a = 0; a < types; ++a)
+        for (int t0 = 0; t0 < count; t0 += 32) {
+            const int t = t0 + lane, source = t < count ? internal_of[old_sources[ob + t]] : -1;
+            const bool take = source >= 0 && (types == 1 || atype[source] == a);
+            const unsigned mask = __ballot_sync(0xffffffffu, take);
+            if (take) {
+                const int e = nb + written + __popc(mask & ((1u << lane) - 1u));
+                new_sources[e] = source;
+                edge_map[e] = ob + t;
+                if (old_shifts != nullptr) {
+                    const size_t to = 3 * static_cast<size_t>(e), from = 3 * static_cast<size_t>(ob + t);
+                    new_shifts[to] = old_shifts[from];
+                    new_shifts[to + 1] = old_shifts[from + 1];
+                    new_shifts[to + 2] = old_shifts[from + 2];
+                }
+            }
+            written += __popc(mask);
         }
-    }
 }
 
 __global__ void gather_counts_kernel(int n, const int* __restrict__ original, const int* __restrict__ old_first,

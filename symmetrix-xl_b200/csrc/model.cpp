@@ -86,11 +86,12 @@ Network parse_network(const json& def, const std::string& name)
     return n;
 }
 
-// values[node][out] for a batch of feature rows (weights are [out][in] row-major)
-std::vector<double> run_network(const Network& n, const std::vector<double>& features, int batch)
+// values[node][out] for a batch of feature rows (weights are [out][in] row-major); hidden_only stops after the last hidden layer
+std::vector<double> run_network(const Network& n, const std::vector<double>& features, int batch, bool hidden_only = false)
 {
     std::vector<double> x = features;
-    for (std::size_t layer = 0; layer + 1 < n.shape.size(); ++layer) {
+    const std::size_t layers = n.shape.size() - (hidden_only ? 2 : 1);
+    for (std::size_t layer = 0; layer < layers; ++layer) {
         const int in = n.shape[layer], out = n.shape[layer + 1];
         const bool last = layer + 2 == n.shape.size();
         std::vector<double> y(static_cast<std::size_t>(batch) * out);
@@ -728,6 +729,68 @@ const std::vector<double>& radial_coefficients(const HostModel& m, const std::st
     const Network& net = d.networks.at(name);
     const auto values = run_network(net, radial_features(d, a, b), d.points);
     return d.cache.emplace(key, spline_coefficients(values, d.points, net.shape.back(), d.h)).first->second;
+}
+
+int radial_basis_width(const HostModel& m, const std::string& name)
+{
+    const auto& d = *static_cast<const RadialDefinition*>(m.radial.get());
+    if (d.stored_pairs) return 0;
+    const Network& net = d.networks.at(name);
+    return net.shape.size() >= 3 && !net.tanh_square ? net.shape[net.shape.size() - 2] : 0;
+}
+
+std::vector<float> build_r0_basis(const HostModel& m, const std::vector<int>& active_types, int* pair_types, bool stepped)
+{
+    const auto& d = *static_cast<const RadialDefinition*>(m.radial.get());
+    const Network& net = d.networks.at("R0");
+    const int H = radial_basis_width(m, "R0"), n = m.agnesi ? static_cast<int>(active_types.size()) : 1;
+    *pair_types = n;
+    const std::size_t intervals = static_cast<std::size_t>(m.spline_points - 1);
+    std::vector<float> out(static_cast<std::size_t>(n) * (n + 1) / 2 * intervals * 4 * H);
+    float* o = out.data();
+    for (int a = 0; a < n; ++a)
+        for (int b = a; b < n; ++b) {   // pair index a*(2n-a-1)/2 + b
+            const auto values = run_network(net, radial_features(d, m.agnesi ? active_types[a] : 0, m.agnesi ? active_types[b] : 0), d.points, true);
+            const auto c = spline_coefficients(values, d.points, H, d.h);
+            for (std::size_t i = 0; i < intervals; ++i) {
+                if (stepped) {
+                    for (int j = 0; j < H / 4; ++j)
+                        for (int t = 0; t < 4; ++t)
+                            for (int q = 0; q < 4; ++q) *o++ = static_cast<float>(c[(i * 4 + q) * H + H / 4 * t + j]);
+                    continue;
+                }
+                for (int half = 0; half < 2; ++half)
+                    for (int h = 0; h < H; h += 2)
+                        for (int q = 2 * half; q < 2 * half + 2; ++q)
+                            for (int k = 0; k < 2; ++k) *o++ = static_cast<float>(c[(i * 4 + q) * H + h + k]);
+            }
+        }
+    return out;
+}
+
+std::vector<float> fold_r0_mixing(const HostModel& m, const std::vector<int>& active_types, int ai, int l)
+{
+    const auto& d = *static_cast<const RadialDefinition*>(m.radial.get());
+    const Network& net = d.networks.at("R0");
+    const int H = radial_basis_width(m, "R0"), n = static_cast<int>(active_types.size()), C = m.channels, L = m.l_max + 1;
+    const std::vector<double>& last = net.weights.back();   // [l * C + k][h]
+    const double* w = m.w_a0.data() + (static_cast<std::size_t>(active_types[ai]) * L + l) * C * C;
+    std::vector<float> out(static_cast<std::size_t>(n) * H * C);
+    std::vector<double> acc(C);
+    for (int aj = 0; aj < n; ++aj) {
+        const double* h0 = m.h0.data() + static_cast<std::size_t>(active_types[aj]) * C;
+        for (int h = 0; h < H; ++h) {
+            std::fill(acc.begin(), acc.end(), 0.0);
+            for (int k = 0; k < C; ++k) {
+                const double s = last[(static_cast<std::size_t>(l) * C + k) * H + h] * h0[k];
+                const double* wk = w + static_cast<std::size_t>(k) * C;
+                for (int j = 0; j < C; ++j) acc[j] += s * wk[j];
+            }
+            float* o = out.data() + (static_cast<std::size_t>(aj) * H + h) * C;
+            for (int j = 0; j < C; ++j) o[j] = static_cast<float>(acc[j]);
+        }
+    }
+    return out;
 }
 
 std::vector<float> build_r1_table(const HostModel& m, const std::vector<int>& active_types, int* num_pairs)

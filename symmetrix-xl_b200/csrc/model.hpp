@@ -103,6 +103,19 @@ std::vector<float> build_r1_table(const HostModel& model, const std::vector<int>
 // Density table [ordered pair ai*n+aj][interval][4] in float of network "A0" or "A1".
 std::vector<float> build_density_table(const HostModel& model, const std::string& name, const std::vector<int>& active_types);
 
+// Width of the last hidden layer of radial network ``name``, 0 when its functions are not a linear map of that layer (stored pair
+// splines, a network without hidden layers or with postprocessing).
+int radial_basis_width(const HostModel& model, const std::string& name);
+
+// Splines of the last hidden layer of network "R0": [unordered pair][interval][2][H / 2][4] in float, (c0, c0', c1, c1') and then
+// (c2, c2', c3, c3') of two neighbouring functions, or stepped [unordered pair][interval][H / 4][4][4], the four coefficients of
+// function H / 4 * t + j at [j][t]; one pair (pair_types = 1) when the model has no distance transform.
+std::vector<float> build_r0_basis(const HostModel& model, const std::vector<int>& active_types, int* pair_types, bool stepped);
+
+// The map from those functions to A0 for receivers of active type ai: [type_j * H + h][C], with the network's last layer,
+// H0[type_j] and W_A0[type_i][l] folded in double and rounded once to float.
+std::vector<float> fold_r0_mixing(const HostModel& model, const std::vector<int>& active_types, int ai, int l);
+
 // Folds H0[type_j] and W_A0[type_i][l] into the layer-0 spline coefficients for the
 // given active types (the reference does the same per ordered species pair,
 // mace_kokkos_factorized_lifecycle.cpp:3988-4047), in double, rounded once to float.

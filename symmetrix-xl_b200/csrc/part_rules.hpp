@@ -55,6 +55,21 @@ struct PartRules {
         return edge_parts(receivers, 1.0 * num_sms * resident, edges, 4.0, 0.95, 2, 8);
     }
 
+    // Layer 0 on the radial functions (edge_kernels_basis.cuh, two kernels more than on the folded table) or on the table: sums and
+    // gradient together, us, table / functions, 128 channels, three types: 320 receivers 54 / 63, 500: 73 / 68, 720: 96 / 75, 1,260:
+    // 137 / 97, 5,000: 415 / 220; 64 channels: 500: 56 / 63, 600: 66 / 67, 720: 70 / 70, 1,260: 106 / 92.  The work of the functions grows
+    // with the types: 5,000 receivers with 4, 6 and 8 types 457 / 257, 464 / 345, 468 / 411, 20,000 with ten 1,731 / 1,675.
+    bool layer0_on_basis(long receivers, int types) const { return types <= 10 && receivers >= (channels == 128 ? 150l : 230l) * types; }
+
+    // Layer-0 gradient on the radial functions: a warp per receiver (1) when that fills the twelve resident warps of every SM,
+    // otherwise one per (receiver, source type) and part of whole steps of 16 edges (a run has 15 to 45 edges in the medium model).
+    int l0_moments_reverse(long receivers, int types) const
+    {
+        const long slots = 12l * num_sms;
+        if (receivers >= slots) return 1;
+        return types * static_cast<int>(std::max(1l, std::min(4l, slots / std::max(1l, receivers * types))));
+    }
+
     // Layer-1 sums, whose parts meet in a cluster: as many as fill the chip once, at most five blocks on an SM (placing the
     // blocks of more clusters takes longer than the chains they shorten).  1 / 2 / 4 / 8 parts, 128 channels: 40 receivers 39 /
     // 35 / 23 / 18, 320: 51 / 64 / 64 / 70; 64 channels, 160: 39 / 37 / 27 / 31; hidden 0e (58 edges) at 32 channels, 160: 21 /
@@ -67,13 +82,22 @@ struct PartRules {
         return parts;
     }
 
-    // Layer-1 gradient with the row adjoints in shared memory, `resident` blocks of it on an SM.  1 / 2 / 4 / 8 parts, 128
-    // channels: 40 receivers 64 / 37 / 29 / 25, 320: 91 / 84 / 84 / 101, 600: 148 / 134 / 142 / 175, 1,080: 224 / 220 / 246 /
-    // 308, 5,000: 900 / 934 / 1,092 / 1,422; 64 channels, 320: 54 / 50 / 50 / 58, 1,080: 115 / 117 / 130 / 162; 0e+1o+2e, 40: 74 /
-    // 44 / 44 / 46, 160: 111 / 99 / 105 / 132, 600: 293 / 297 / 347 / 457.
+    // Blocks that hold a receiver's row adjoints (the layer-1 gradient on channel pairs), `resident` of them on an SM.
     int l1_reverse_shared(long receivers, int resident) const
     {
         return edge_parts(receivers, 1.0 * num_sms * resident, edges, 8.0, 0.95, 2, 8);
+    }
+
+    // Layer-1 gradient with the row adjoints in tensor memory.  A block of it has eight or twelve warps, a part costs more beside its
+    // edges than with a few warps: no more blocks than fill the chip about twice.  1 / 2 / 4 / 8 parts, 128 channels: 40 receivers
+    // 38 / 25 / 23 / 23, 160: 50 / 44 / 44 / 50, 320: 72 / 66 / 70 / 87, 600: 111 / 109 / 119 / 154, 1,080: 173 / 179 / 204 / 267, 5,000: 699 /
+    // 762 / 904 / 1,308; 64 channels, 40: 23 / 17 / 17 / 19, 320: 44 / 42 / 50 / 68, 1,080: 97 / 105 / 136 / 199; 0e+1o+2e, 40: 56 / 35 / 37 / 38,
+    // 160: 85 / 80 / 83 / 103, 600: 220 / 236 / 275 / 359.
+    int l1_reverse_pairs(long receivers, int resident) const
+    {
+        int parts = l1_reverse_shared(receivers, resident);
+        while (parts > 1 && 1.0 * receivers * parts > 2.2 * num_sms * resident) parts /= 2;
+        return parts;
     }
 
     // Layer-1 gradient with the row adjoints in registers.  Hidden 0e: 128 registers and 26 KB a block, eight blocks of up to two
