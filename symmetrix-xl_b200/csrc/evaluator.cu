@@ -154,6 +154,17 @@ Evaluator::Evaluator(const std::string& json_path, int device_ordinal, const std
     }
     upload(h2_skip_, model_.h2_skip, stream_);
     upload(h2_m1_, model_.h2_m1, stream_);
+    if (fused_readout_model()) {   // the same weights [element][out][in]
+        auto transposed = [C](const std::vector<float>& w) {
+            std::vector<float> t(w.size());
+            for (std::size_t m = 0; m < w.size(); m += static_cast<std::size_t>(C) * C)
+                for (int i = 0; i < C; ++i)
+                    for (int j = 0; j < C; ++j) t[m + static_cast<std::size_t>(j) * C + i] = w[m + static_cast<std::size_t>(i) * C + j];
+            return t;
+        };
+        upload(h2_skip_t_, transposed(model_.h2_skip), stream_);
+        upload(h2_m1_t_, transposed(model_.h2_m1), stream_);
+    }
     upload(readout1_, model_.readout1, stream_);
     upload(readout2_w1_, model_.readout2_w1, stream_);
     upload(readout2_w2_, model_.readout2_w2, stream_);
@@ -386,6 +397,7 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     M1_adj_.reserve(T * C);
     H2_.reserve(T * C);
     H2_adj_.reserve(N * C);
+    if (fused_readout() && static_cast<std::size_t>(tile_capacity()) < N) scalar_adjoint_.reserve(N * C);   // direct adjoint of M0's scalar block
     if (model_.pre_linear_up) {   // scalar input of the first readout and the skip, and its adjoint, for every receiver
         scalar_input_.reserve(N * C);
         scalar_adjoint_.reserve(N * C);
@@ -1028,6 +1040,7 @@ void Evaluator::run_pipeline(int phases)
     const int n_active = static_cast<int>(active_types_.size());
     const int tile_cap = tile_capacity();
     const bool tiled = tile_cap < R;
+    const bool fused = fused_readout();
     const std::size_t rowH = static_cast<std::size_t>(NH) * C;
     const RowMap scalar_rows{static_cast<long>(NH) * C, C, 0, 1};
     const RowMap flat_rows{static_cast<long>(C), C, 0, 1};
@@ -1155,7 +1168,7 @@ void Evaluator::run_pipeline(int phases)
                 calls.push_back({m0, rows, &s_h1_[l], false, H1_.ptr + t0 * rowH, rows, 0, T, false, nullptr});
             }
             // one tile: the element-dependent skip term of H2 (x_i T_element) only needs M0, so it rides in this launch
-            if (!tiled && !model_.legacy_h1_basis && !model_.pre_linear_up)
+            if (!fused && !tiled && !model_.legacy_h1_basis && !model_.pre_linear_up)
                 for_type_ranges(t0, T, [&](int a, int begin, int count) {
                     calls.push_back({M0_.ptr + begin * rowH, scalar_rows, &s_h2_skip_[active_types_[a]], false,
                                      H2_.ptr + static_cast<std::size_t>(begin - t0) * C, flat_rows, 0, count, false, nullptr});
@@ -1231,6 +1244,23 @@ void Evaluator::run_pipeline(int phases)
                 launch_tc(calls);
             }
             span_end();
+            if (fused) {
+                span_begin("node_readout");
+                const NodeReadoutArgs args{T, model_.readout2_scale, element_.ptr + t0, A1_.ptr, M0_.ptr + t0 * rowH, m1_weights_.ptr,
+                                           h2_m1_.ptr, h2_m1_t_.ptr, h2_skip_.ptr, h2_skip_t_.ptr, readout1_.ptr, readout2_w1_.ptr, readout2_w2_.ptr,
+                                           atomic_energies_.ptr, M1_.ptr, H2_.ptr, H2_adj_.ptr + static_cast<std::size_t>(t0) * C, M1_adj_.ptr,
+                                           A1_adj_.ptr, tiled ? scalar_adjoint_.ptr + static_cast<std::size_t>(t0) * C : M0_adj_.ptr,
+                                           tiled ? C : static_cast<int>(rowH), model_.a1_scaled ? dot1_.ptr + t0 : nullptr, node_energies_.ptr + t0, energy_slots};
+#define SXB_NODE_READOUT(NAME)                                                                                            \
+                (C == 128 ? node_readout_kernel_##NAME<128> : C == 64 ? node_readout_kernel_##NAME<64> : node_readout_kernel_##NAME<32>) \
+                    <<<blocks_for(T, 512 / C), 256, 0, stream_>>>(args)
+                if (model_.shape_id == 0) SXB_NODE_READOUT(S0);
+                else if (model_.shape_id == 1) SXB_NODE_READOUT(S1);
+                else node_readout_kernel_S2<128><<<blocks_for(T, 4), 256, 0, stream_>>>(args);
+#undef SXB_NODE_READOUT
+                launches_ += 1;
+                span_end();
+            } else {
             span_begin("m1_forward");
             if (model_.shape_id == 0)
                 SXB_LAUNCH_POLY(m1_forward_kernel, S0, SXB_S0_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_.ptr);
@@ -1241,6 +1271,8 @@ void Evaluator::run_pipeline(int phases)
             launches_ += 1;
             span_end();
             }
+            }
+            if (!fused) {
             // H2 = xs T_element + M1 W
             span_begin("gemm_h2");
             {
@@ -1320,6 +1352,7 @@ void Evaluator::run_pipeline(int phases)
                 SXB_LAUNCH_POLY(m1_reverse_kernel, S2, SXB_S2_M1_NUM_TERMS, T, C, stream_, A1_.ptr, element_.ptr + t0, m1_weights_.ptr, M1_adj_.ptr, A1_adj_.ptr, model_.a1_scaled ? dot1_.ptr + t0 : nullptr);
             launches_ += 1;
             span_end();
+            }
             span_begin("gemm_a1_reverse");
             {
                 std::vector<TcCall> calls;
@@ -1415,17 +1448,20 @@ void Evaluator::run_pipeline(int phases)
                 }
                 launch_tc(calls);
             } else {
+                if (tiled && fused)   // the direct adjoint of the scalar block, kept from the second sweep
+                    SXB_CUDA(cudaMemcpy2DAsync(M0_adj_.ptr, rowH * sizeof(float), scalar_adjoint_.ptr + static_cast<std::size_t>(t0) * C, C * sizeof(float),
+                                               C * sizeof(float), T, cudaMemcpyDeviceToDevice, stream_));
                 std::vector<TcCall> calls;
                 for (int l = 0; l <= model_.hidden_l_max; ++l) {
                     const RowMap rows{static_cast<long>(NH) * C, C, static_cast<long>(l) * l * C, 2 * l + 1};
-                    if (tiled)
+                    if (tiled && !fused)
                         calls.push_back({H1_adj_.ptr + t0 * rowH, rows, &s_h1_[l], true, M0_adj_.ptr, rows, 0, T, false,
                                          l == 0 ? readout1_.ptr : nullptr});
                     else   // the scalar block already holds the direct adjoint (written with the H2 reverse linear)
                         calls.push_back({H1_adj_.ptr + t0 * rowH, rows, &s_h1_[l], true, M0_adj_.ptr, rows, 0, T, l == 0, nullptr});
                 }
                 launch_tc(calls);
-                if (tiled) {
+                if (tiled && !fused) {
                     calls.clear();
                     for_type_ranges(t0, T, [&](int a, int begin, int count) {
                         calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[active_types_[a]], true,

@@ -352,21 +352,14 @@ readout_kernel(int num_nodes, int C, int hidden, float act_scale, const float* _
 // The same readout for the common head shape (16 hidden units, C a multiple of 32, at most 256): the 16
 // pre-activations of a node are formed together, each lane holding its channels' partial sums, and
 // summed over the warp by a butterfly that halves the number of live values at every step (16 shuffles
-// instead of 80); lane L ends up with hidden unit L / 2.  No per-thread array is indexed at run time.
+// instead of 80); lane L ends up with hidden unit L / 2.  No per-thread array is indexed at run time.  Returns the node's
+// energy without E0 (in lane 0); g is the adjoint of H2, channels lane + 32 j.
 template <int kChunks>   // C / 32
-__global__ void __launch_bounds__(256)
-readout16_kernel(int num_nodes, float act_scale, const float* __restrict__ M0, int num_hidden_lm,
-                 const float* __restrict__ H2, const unsigned char* __restrict__ element,
-                 const double* __restrict__ atomic_energies, const float* __restrict__ q,
-                 const float* __restrict__ W1 /*[16][C]*/, const float* __restrict__ W2 /*[16]*/,
-                 double* __restrict__ node_energies, float* __restrict__ H2_adj, double* __restrict__ energy_slots)
+__device__ __forceinline__ double readout16_node(int lane, float act_scale, const float* __restrict__ xs, const float* __restrict__ h2,
+                                                 const float* __restrict__ q, const float* __restrict__ W1 /*[16][C]*/,
+                                                 const float* __restrict__ W2 /*[16]*/, float (&g)[kChunks])
 {
     constexpr int C = 32 * kChunks, kHidden = 16;
-    const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (node >= num_nodes) return;
-    const float* xs = M0 + static_cast<size_t>(node) * num_hidden_lm * C;   // scalar block of M0
-    const float* h2 = H2 + static_cast<size_t>(node) * C;
     float hv[kChunks];
     float e1 = 0.0f;
 #pragma unroll
@@ -406,7 +399,6 @@ readout16_kernel(int num_nodes, float act_scale, const float* __restrict__ M0, i
         e1 += __shfl_xor_sync(0xffffffffu, e1, offset);
         e2 += __shfl_xor_sync(0xffffffffu, e2, offset);
     }
-    float g[kChunks];
 #pragma unroll
     for (int j = 0; j < kChunks; ++j) g[j] = 0.0f;
 #pragma unroll
@@ -415,14 +407,170 @@ readout16_kernel(int num_nodes, float act_scale, const float* __restrict__ M0, i
 #pragma unroll
         for (int j = 0; j < kChunks; ++j) g[j] = fmaf(c, W1[h * C + lane + 32 * j], g[j]);
     }
+    return static_cast<double>(e1) + static_cast<double>(e2);
+}
+
+template <int kChunks>
+__global__ void __launch_bounds__(256)
+readout16_kernel(int num_nodes, float act_scale, const float* __restrict__ M0, int num_hidden_lm,
+                 const float* __restrict__ H2, const unsigned char* __restrict__ element,
+                 const double* __restrict__ atomic_energies, const float* __restrict__ q,
+                 const float* __restrict__ W1, const float* __restrict__ W2,
+                 double* __restrict__ node_energies, float* __restrict__ H2_adj, double* __restrict__ energy_slots)
+{
+    constexpr int C = 32 * kChunks;
+    const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (node >= num_nodes) return;
+    float g[kChunks];
+    const double e = atomic_energies[element[node]]
+                     + readout16_node<kChunks>(lane, act_scale, M0 + static_cast<size_t>(node) * num_hidden_lm * C, H2 + static_cast<size_t>(node) * C, q, W1, W2, g);
 #pragma unroll
     for (int j = 0; j < kChunks; ++j) H2_adj[static_cast<size_t>(node) * C + lane + 32 * j] = g[j];
     if (lane == 0) {
-        const double e = atomic_energies[element[node]] + static_cast<double>(e1) + static_cast<double>(e2);
         node_energies[node] = e;
         if (energy_slots != nullptr) atomicAdd(energy_slots + (node % kVirialSlots), e);
     }
 }
+
+// ---------------------------------------------------------------------------------------------
+// Everything between A1 and its adjoint in one launch: contraction M1, H2 = x T_element + M1 W with x the scalar block of M0,
+// readout, and their adjoints back to A1_adj and to the scalar block of M0_adj (readout weights + T_element H2_adj).  All of it is
+// local to a node, and as five launches it lasts as long as five short dependent kernels (9 to 13 us each up to a thousand nodes).
+// A block takes 512 / kC nodes; the linears run in FP32 on the vectors in shared memory, a thread per output column and part of
+// the sum, the weights once per block.
+struct NodeReadoutArgs {
+    int num_nodes;
+    float act_scale;
+    const unsigned char* element;
+    const float *A1, *M0, *m1_weights;             // [node][16][kC], [node][NH][kC], [element][term][kC]
+    const float *W, *Wt, *T, *Tt;                  // [in][out], [out][in], the same per element
+    const float *q, *W1, *W2;
+    const double* atomic_energies;
+    float *M1, *H2, *H2_adj, *M1_adj, *A1_adj, *M0_adj;
+    int M0_adj_stride;                             // floats between the nodes' scalar blocks
+    float* dot;
+    double *node_energies, *energy_slots;
+};
+
+#define W(t) w[(t) * (kC / 2)]
+#define SXB_DEFINE_NODE_READOUT(NAME)                                                                               \
+template <int kC>                                                                                                   \
+__global__ void __launch_bounds__(256, 2) node_readout_kernel_##NAME(const NodeReadoutArgs a)                       \
+{                                                                                                                   \
+    constexpr int NH = SXB_##NAME##_NUM_HIDDEN, NT = SXB_##NAME##_M1_NUM_TERMS, G = 512 / kC, kParts = 256 / kC;    \
+    __shared__ float m1[kC][G], xs[kC][G], adj_s[kC][G], h2[G][kC], sums[2][kParts][G][kC];                         \
+    __shared__ unsigned char types[G];                                                                              \
+    const int tid = threadIdx.x, base = blockIdx.x * G;                                                             \
+    const int n = tid / (kC / 2), k = 2 * (tid % (kC / 2));             /* node and channel pair of the contractions */ \
+    const bool valid = base + n < a.num_nodes;                                                                      \
+    const size_t node = valid ? base + n : a.num_nodes - 1;             /* a place past the end repeats the last node */ \
+    const int column = tid % kC, part = tid / kC;                       /* output and part of the sum of the linears */ \
+    const int type = a.element[node];                                                                               \
+    const f2* const w = reinterpret_cast<const f2*>(a.m1_weights + static_cast<size_t>(type) * NT * kC + k);        \
+    const float* const in = a.A1 + node * 16 * kC + k;                                                              \
+    {                                                                                                               \
+        f2 x[16], o[1];                                                                                             \
+        _Pragma("unroll") for (int r = 0; r < 16; ++r) x[r] = *reinterpret_cast<const f2*>(in + r * kC);            \
+        o[0] = 0ull;                                                                                                \
+        SXB_##NAME##_M1_FORWARD_BODY                                                                                \
+        const float2 value = *reinterpret_cast<const float2*>(&o[0]);                                               \
+        const float2 scalar = *reinterpret_cast<const float2*>(a.M0 + node * NH * kC + k);                          \
+        m1[k][n] = value.x; m1[k + 1][n] = value.y;                                                                 \
+        xs[k][n] = scalar.x; xs[k + 1][n] = scalar.y;                                                               \
+        if (valid) *reinterpret_cast<float2*>(a.M1 + node * kC + k) = value;                                        \
+        if (k == 0) types[n] = static_cast<unsigned char>(type);                                                    \
+    }                                                                                                               \
+    __syncthreads();                                                                                                \
+    {                                                                                                               \
+        float acc[G];                                                                                               \
+        _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = 0.0f;                                                \
+        _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {               \
+            const float wv = a.W[c * kC + column];                                                                  \
+            _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(m1[c][r], wv, acc[r]);                      \
+        }                                                                                                           \
+        for (int r0 = 0; r0 < G;) {   /* runs of equal elements: one in most blocks, receivers are sorted by element */ \
+            const int run = types[r0];                                                                              \
+            int r1 = r0 + 1;                                                                                        \
+            while (r1 < G && types[r1] == run) ++r1;                                                                \
+            const float* const T = a.T + static_cast<size_t>(run) * kC * kC + column;                               \
+            _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {           \
+                const float tv = T[c * kC];                                                                         \
+                _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(r >= r0 && r < r1 ? xs[c][r] : 0.0f, tv, acc[r]); \
+            }                                                                                                       \
+            r0 = r1;                                                                                                \
+        }                                                                                                           \
+        _Pragma("unroll") for (int r = 0; r < G; ++r) sums[0][part][r][column] = acc[r];                            \
+    }                                                                                                               \
+    __syncthreads();                                                                                                \
+    for (int idx = tid; idx < G * kC; idx += 256) {                                                                 \
+        const int r = idx / kC, c = idx % kC;                                                                       \
+        float total = 0.0f;                                                                                         \
+        _Pragma("unroll") for (int p = 0; p < kParts; ++p) total += sums[0][p][r][c];                               \
+        h2[r][c] = total;                                                                                           \
+        if (base + r < a.num_nodes) a.H2[static_cast<size_t>(base + r) * kC + c] = total;                           \
+    }                                                                                                               \
+    __syncthreads();                                                                                                \
+    for (int r = tid >> 5; r < G; r += 8) {                                                                         \
+        const int lane = tid & 31;                                                                                  \
+        const size_t at = min(base + r, a.num_nodes - 1);                                                           \
+        float g[kC / 32];                                                                                           \
+        const double e = a.atomic_energies[types[r]]                                                                \
+                         + readout16_node<kC / 32>(lane, a.act_scale, a.M0 + at * NH * kC, h2[r], a.q, a.W1, a.W2, g); \
+        _Pragma("unroll") for (int c = 0; c < kC / 32; ++c) {                                                       \
+            adj_s[lane + 32 * c][r] = g[c];                                                                         \
+            if (base + r < a.num_nodes) a.H2_adj[at * kC + lane + 32 * c] = g[c];                                   \
+        }                                                                                                           \
+        if (lane == 0 && base + r < a.num_nodes) {                                                                  \
+            a.node_energies[at] = e;                                                                                \
+            if (a.energy_slots != nullptr) atomicAdd(a.energy_slots + (at % kVirialSlots), e);                      \
+        }                                                                                                           \
+    }                                                                                                               \
+    __syncthreads();                                                                                                \
+    {                                                                                                               \
+        float acc[G], skip[G];                                                                                      \
+        _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = skip[r] = 0.0f;                                      \
+        _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {               \
+            const float wv = a.Wt[c * kC + column];                                                                 \
+            _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(adj_s[c][r], wv, acc[r]);                   \
+        }                                                                                                           \
+        for (int r0 = 0; r0 < G;) {                                                                                 \
+            const int run = types[r0];                                                                              \
+            int r1 = r0 + 1;                                                                                        \
+            while (r1 < G && types[r1] == run) ++r1;                                                                \
+            const float* const T = a.Tt + static_cast<size_t>(run) * kC * kC + column;                              \
+            _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {           \
+                const float tv = T[c * kC];                                                                         \
+                _Pragma("unroll") for (int r = 0; r < G; ++r) skip[r] = fmaf(r >= r0 && r < r1 ? adj_s[c][r] : 0.0f, tv, skip[r]); \
+            }                                                                                                       \
+            r0 = r1;                                                                                                \
+        }                                                                                                           \
+        _Pragma("unroll") for (int r = 0; r < G; ++r) { sums[0][part][r][column] = acc[r]; sums[1][part][r][column] = skip[r]; } \
+    }                                                                                                               \
+    __syncthreads();                                                                                                \
+    {                                                                                                               \
+        f2 x[16], g[16], adj[1];                                                                                    \
+        float2 m1_adj = make_float2(0.0f, 0.0f), m0_adj = *reinterpret_cast<const float2*>(a.q + k);                \
+        _Pragma("unroll") for (int p = 0; p < kParts; ++p) {                                                        \
+            const float2 u = *reinterpret_cast<const float2*>(&sums[0][p][n][k]), v = *reinterpret_cast<const float2*>(&sums[1][p][n][k]); \
+            m1_adj.x += u.x; m1_adj.y += u.y; m0_adj.x += v.x; m0_adj.y += v.y;                                     \
+        }                                                                                                           \
+        if (valid) {                                                                                                \
+            *reinterpret_cast<float2*>(a.M1_adj + node * kC + k) = m1_adj;                                          \
+            *reinterpret_cast<float2*>(a.M0_adj + node * a.M0_adj_stride + k) = m0_adj;                                    \
+        }                                                                                                           \
+        _Pragma("unroll") for (int r = 0; r < 16; ++r) { x[r] = *reinterpret_cast<const f2*>(in + r * kC); g[r] = 0ull; } \
+        adj[0] = *reinterpret_cast<const f2*>(&m1_adj);                                                             \
+        SXB_##NAME##_M1_REVERSE_BODY                                                                                \
+        float* out = a.A1_adj + node * 16 * kC + k;                                                                 \
+        if (valid) { _Pragma("unroll") for (int r = 0; r < 16; ++r) *reinterpret_cast<f2*>(out + r * kC) = g[r]; }  \
+        if (a.dot != nullptr) poly_accumulate_dot(g, x, a.dot, static_cast<int>(node), valid);                      \
+    }                                                                                                               \
+}
+SXB_DEFINE_NODE_READOUT(S0)
+SXB_DEFINE_NODE_READOUT(S1)
+SXB_DEFINE_NODE_READOUT(S2)
+#undef W
 
 // tensor[node][0][k] = values[k] for the first num_nodes nodes of a (node, component, channel) tensor.
 __global__ void fill_scalar_block_kernel(int num_nodes, int C, long node_stride, const float* __restrict__ values,
