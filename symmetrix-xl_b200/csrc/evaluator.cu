@@ -473,6 +473,8 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
         host_results_capacity_ = 0;
     }
     generation_ += 1;
+    if (evaluations_ > 0) last_evaluations_ = evaluations_;
+    evaluations_ = 0;
     have_results_ = false;
     mirror_valid_ = false;
     phase_ = 0;
@@ -1546,7 +1548,8 @@ void Evaluator::run_pipeline(int phases)
 // Enqueues the geometry kernel (when `positions` is given) and the pipeline phases on the stream.
 // Outside profiling the sequence is captured once per (phases, graph generation, position buffer)
 // into a CUDA graph and replayed afterwards: every kernel argument is fixed for a prepared graph, so
-// a step costs one graph launch instead of some twenty kernel launches.
+// a step costs one graph launch instead of some twenty kernel launches.  Not for graphs that are
+// expected to be short-lived (kReplaysToPay).
 void Evaluator::enqueue_phases(int phases, const double* positions, bool upload_staged)
 {
     auto enqueue = [&] {
@@ -1571,9 +1574,11 @@ void Evaluator::enqueue_phases(int phases, const double* positions, bool upload_
         }
         run_pipeline(phases);
     };
+    if (phases & 1) ++evaluations_;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (stream_ != nullptr && cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess) cudaGetLastError();
-    if (!use_graphs_ || profiling_ || stream_ == nullptr || capturing != cudaStreamCaptureStatusNone) {
+    const bool short_lived = last_evaluations_ < kReplaysToPay && evaluations_ < kReplaysToPay;
+    if (!use_graphs_ || short_lived || profiling_ || stream_ == nullptr || capturing != cudaStreamCaptureStatusNone) {
         enqueue();      // also when the caller is capturing this stream itself: the kernels then join its graph
         return;
     }

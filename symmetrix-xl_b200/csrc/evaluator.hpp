@@ -114,10 +114,11 @@ private:
     void prepare_active_types(const std::vector<int>& node_types, int num_receivers);
     void install_graph(int num_receivers, int num_nodes, const std::vector<int>& node_types, long num_edges, bool has_shifts);
     ActiveEdges active_edges() const;
-    // receivers whose sums over the radial functions are kept at a time: 96 MB of them stay in L2 between their kernels
+    // receivers whose sums over the radial functions are kept at a time, 1 GB of them: 135,000 receivers, three types, in slices of 96 MB
+    // (which stay in L2) / 0.8 GB: layer 0 7.9 / 6.8 ms; 20,000 with ten types 2.4 / 1.8 ms
     int moment_receivers() const
     {
-        const long fit = (96l << 20) / (16l * 64 * static_cast<long>(sizeof(float)) * static_cast<long>(std::max<std::size_t>(1, active_types_.size())));
+        const long fit = (1l << 30) / (16l * 64 * static_cast<long>(sizeof(float)) * static_cast<long>(std::max<std::size_t>(1, active_types_.size())));
         return static_cast<int>(std::min<long>(tile_capacity(), std::max(1024l, fit)));
     }
     int edge_types() const { return basis_layer0_ ? static_cast<int>(active_types_.size()) : 1; }   // types a receiver's edges are grouped by
@@ -144,6 +145,11 @@ private:
         long launches = 0;
     };
     std::map<int, StepGraph> step_graphs_;
+    // A program that takes a new neighbor list every few evaluations (a list of structures, hot dynamics) never earns back what
+    // capturing and instantiating a step costs: 160 us against 5 to 20 us saved per replay.  When the last graph was given up before
+    // kReplaysToPay evaluations, this one's steps are launched kernel by kernel until it has had as many.
+    static constexpr long kReplaysToPay = 8;
+    long evaluations_ = 0, last_evaluations_ = kReplaysToPay;   // begun on this graph and on the one before it
     struct HaloPlan {
         bool active = false;
         const int* send_indices = nullptr;
