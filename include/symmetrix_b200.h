@@ -135,6 +135,14 @@ int sxb_compute_positions(sxb_evaluator* evaluator, uint64_t generation, const d
  * pair_symmetrix/pair_symmetrix_mace_kokkos.cpp:1532-1568). */
 int sxb_compute_positions_device(sxb_evaluator* evaluator, uint64_t generation, const double* device_positions);
 
+/* sxb_compute_positions in two halves, so that several evaluators can be in flight at once from one thread
+ * (a committee: SymmetrixEnsemble, symmetrix/source/symmetrix/ensemble.py:166-212).  begin copies the
+ * positions and enqueues the evaluation on the evaluator's stream; finish waits for it and reads status and
+ * totals.  Between the two there are no results (the getters report that), and any other computation or a new
+ * graph on this evaluator drops what was begun. */
+int sxb_begin_positions(sxb_evaluator* evaluator, uint64_t generation, const double* positions);
+int sxb_finish_positions(sxb_evaluator* evaluator, uint64_t generation);
+
 /* Replaces _compute_prepared_factorized(generation, xyz, r) and the one-shot
  * compute_node_energies_forces(num_nodes, node_types, num_neigh, neigh_indices, neigh_types, xyz, r)
  * (symmetrix/source/cpp/mace_kokkos.cpp:1817-1827, 2169-2204): edge vectors xyz f64[3*num_edges] in

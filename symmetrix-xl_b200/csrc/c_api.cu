@@ -287,6 +287,22 @@ int sxb_compute_positions_device(sxb_evaluator* ev, uint64_t generation, const d
     });
 }
 
+int sxb_begin_positions(sxb_evaluator* ev, uint64_t generation, const double* positions)
+{
+    return guarded([&] {
+        require(ev, "evaluator"); require(positions, "positions");
+        ev->impl.begin_positions(generation, positions, false);
+    });
+}
+
+int sxb_finish_positions(sxb_evaluator* ev, uint64_t generation)
+{
+    return guarded([&] {
+        require(ev, "evaluator");
+        ev->impl.finish_positions(generation);
+    });
+}
+
 int sxb_compute_edge_vectors(sxb_evaluator* ev, uint64_t generation, const double* xyz)
 {
     return guarded([&] {

@@ -51,6 +51,8 @@ public:
     void check_generation(std::uint64_t generation) const;
 
     void compute_positions(std::uint64_t generation, const double* positions, bool on_device);
+    void begin_positions(std::uint64_t generation, const double* positions, bool on_device);   // enqueues, does not wait
+    void finish_positions(std::uint64_t generation);                                           // waits and collects
     void compute_edge_vectors(std::uint64_t generation, const double* xyz);
     void synchronize();
     void distributed_begin(std::uint64_t generation, const double* device_positions);
@@ -163,6 +165,8 @@ private:
     HaloPlan halo_plan_;
     bool use_graphs_ = true;
     void finish_compute();
+    void collect_compute();     // waits for the evaluation whose end has been recorded, and reads status and totals
+    void settle();              // waits for an evaluation that was begun and never finished
     void launch_gemm(const float* A, const RowMap& a_rows, const float* B, int ldb, bool b_transposed, float* C,
                      const RowMap& c_rows, int first_node, int num_nodes, int N, int K, bool accumulate, const float* bias);
 
@@ -258,6 +262,7 @@ private:
     bool mirror_valid_ = false;
     bool keep_edge_forces_ = false;
     bool have_results_ = false;
+    bool pending_ = false;      // an evaluation has been begun and its results have not been collected
     long launches_ = 0;
     float last_ms_ = 0.0f;
     bool profiling_ = false;

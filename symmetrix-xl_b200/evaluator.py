@@ -63,6 +63,8 @@ SIGNATURES = {
     "sxb_get_graph": (ctypes.c_int, [_P, ctypes.c_uint64, _P, _P, _P]),
     "sxb_compute_positions": (ctypes.c_int, [_P, ctypes.c_uint64, _P]),
     "sxb_compute_positions_device": (ctypes.c_int, [_P, ctypes.c_uint64, _P]),
+    "sxb_begin_positions": (ctypes.c_int, [_P, ctypes.c_uint64, _P]),
+    "sxb_finish_positions": (ctypes.c_int, [_P, ctypes.c_uint64]),
     "sxb_compute_edge_vectors": (ctypes.c_int, [_P, ctypes.c_uint64, _P]),
     "sxb_synchronize": (ctypes.c_int, [_P]),
     "sxb_get_node_energies": (ctypes.c_int, [_P, _P, ctypes.c_int64]),
@@ -493,6 +495,17 @@ class MACEB200:
             raise ValueError("positions extent does not match the prepared graph.")
         _check(self._lib.sxb_compute_positions(self._h, int(graph_generation), positions.ctypes.data))
 
+    def _begin_prepared_factorized_positions(self, graph_generation, positions):
+        """First half of ``_compute_prepared_factorized_positions``: enqueues the evaluation and does not wait."""
+        positions = _f64(positions).reshape(-1)
+        if positions.size != 3 * self._num_nodes:
+            raise ValueError("positions extent does not match the prepared graph.")
+        _check(self._lib.sxb_begin_positions(self._h, int(graph_generation), positions.ctypes.data))
+
+    def _finish_prepared_factorized_positions(self, graph_generation):
+        """Second half: waits for the evaluation and collects its results."""
+        _check(self._lib.sxb_finish_positions(self._h, int(graph_generation)))
+
     def compute_positions_device(self, graph_generation, device_pointer: int):
         """Evaluation from float64 positions already resident on the evaluator's device."""
         _check(self._lib.sxb_compute_positions_device(self._h, int(graph_generation), ctypes.c_void_p(device_pointer)))
@@ -703,6 +716,12 @@ class Calculator:
         return moved + strain * reach <= 0.5 * self.skin, True
 
     def calculate(self, positions, cell, node_types, pbc=(True, True, True)):
+        positions, cell, node_types, pbc = self._prepare(positions, cell, node_types, pbc)
+        self.evaluator._compute_prepared_factorized_positions(self._generation, positions)
+        return self._results(cell, node_types, pbc)
+
+    def _prepare(self, positions, cell, node_types, pbc):
+        """The arguments in their canonical form, with the neighbor list reused or built for them."""
         positions = _f64(positions).reshape(-1, 3)
         cell = _f64(cell).reshape(3, 3)
         node_types = _i32(node_types)
@@ -737,7 +756,10 @@ class Calculator:
             self._types = node_types.copy()
             self._pbc = pbc
             self.rebuilds += 1
-        ev._compute_prepared_factorized_positions(self._generation, positions)
+        return positions, cell, node_types, pbc
+
+    def _results(self, cell, node_types, pbc):
+        ev = self.evaluator
         n = len(node_types)
         energies = ev.node_energies
         out = {"energy": float(energies.sum()), "energies": energies,
@@ -749,8 +771,8 @@ class Calculator:
 
 class EnsembleCalculator:
     """Same-process committee of calculators, after the reference's ``SymmetrixEnsemble``
-    (symmetrix/source/symmetrix/ensemble.py:65-212): members are evaluated one after the other on the same
-    input; every property ``x`` is returned as the member mean under ``x``, the stacked member values under
+    (symmetrix/source/symmetrix/ensemble.py:65-212): members are evaluated on the same input, each on its
+    evaluator's stream and all of them in flight before the first is waited for; every property ``x`` is returned as the member mean under ``x``, the stacked member values under
     ``x_comm`` and the population variance under ``x_var``.  Members must agree on cutoff, element list and
     skin (the reference's compatibility check, :133-144).  Exactly one of ``model_files`` / ``calculators``."""
 
@@ -783,7 +805,7 @@ class EnsembleCalculator:
         self.num_models = len(members)
 
     def calculate(self, positions, cell, node_types, pbc=(True, True, True)):
-        outputs = [member.calculate(positions, cell, node_types, pbc) for member in self.calculators]
+        outputs = self._member_results(positions, cell, node_types, pbc)
         results = {}
         for name in outputs[0]:
             committee = np.stack([np.asarray(out[name], dtype=np.float64) for out in outputs], axis=0)
@@ -792,3 +814,28 @@ class EnsembleCalculator:
             results[name + "_var"] = float(variance) if variance.ndim == 0 else variance
             results[name + "_comm"] = committee
         return results
+
+    def _member_results(self, positions, cell, node_types, pbc):
+        # a member that is listed twice, or whose class computes in its own way, is called as it stands
+        if len({id(m.evaluator) for m in self.calculators}) < self.num_models \
+                or any(type(m).calculate is not Calculator.calculate for m in self.calculators):
+            return [member.calculate(positions, cell, node_types, pbc) for member in self.calculators]
+        begun, outputs = [], []
+        try:
+            for member in self.calculators:
+                inputs = member._prepare(positions, cell, node_types, pbc)
+                member.evaluator._begin_prepared_factorized_positions(member._generation, inputs[0])
+                begun.append((member, inputs[1:]))
+        finally:
+            # whatever was begun is waited for, also when a later member refuses the input
+            failure = None
+            for member, inputs in begun:
+                try:
+                    member.evaluator._finish_prepared_factorized_positions(member._generation)
+                    if failure is None:
+                        outputs.append(member._results(*inputs))
+                except Exception as error:
+                    failure = failure or error
+            if failure is not None:
+                raise failure
+        return outputs

@@ -131,6 +131,42 @@ def test_affine_cell_change_reuses_the_neighbor_list(pkg, model_path):
     assert calc.rebuilds == 2                      # a large strain rebuilds
 
 
+def test_members_in_flight_together_match_members_called_alone(pkg, model_path):
+    """Members are begun before any is waited for: moving atoms, a member listed twice, and an input that the last
+    step refuses (two atoms on one spot) leave every member usable.  The bound covers the order of the atomic sums
+    alone: 128 channels of FP32 partial sums, at most 2^-24 * sqrt(edges) relative each."""
+    pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 8)
+    members = [pkg.Calculator(model_path("small", seed=s), skin=0.5) for s in (31, 32, 33)]
+    alone = [pkg.Calculator(model_path("small", seed=s), skin=0.5) for s in (31, 32, 33)]
+    ensemble = pkg.EnsembleCalculator(calculators=members)
+    twice = pkg.EnsembleCalculator(calculators=[members[0], members[0]])
+    rng = np.random.default_rng(4)
+    for _ in range(12):                                # past the point where a list's step is captured and replayed
+        pos = pos + rng.normal(scale=0.003, size=pos.shape)
+        out, double = ensemble.calculate(pos, cell, types), twice.calculate(pos, cell, types)
+        for m, member in enumerate(alone):
+            want = member.calculate(pos, cell, types)
+            for name, bound in (("energies", 2e-6), ("forces", 2e-5), ("stress", 1e-7)):
+                assert np.abs(out[name + "_comm"][m] - want[name]).max() <= bound, (m, name)
+            if m == 0:
+                assert np.abs(double["forces_comm"] - want["forces"][None]).max() <= 2e-5
+    bad = pos.copy()
+    bad[1] = bad[0]
+    with pytest.raises(ValueError):
+        ensemble.calculate(bad, cell, types)
+    again = ensemble.calculate(pos, cell, types)
+    assert np.abs(again["forces_comm"] - out["forces_comm"]).max() <= 2e-5
+    ev, generation = members[0].evaluator, members[0]._generation
+    with pytest.raises(ValueError):
+        ev._finish_prepared_factorized_positions(generation)          # nothing was begun
+    ev._begin_prepared_factorized_positions(generation, pos)
+    with pytest.raises(RuntimeError):
+        ev.node_energies                                              # no results between the two halves
+    ev._begin_prepared_factorized_positions(generation, pos)          # drops the first
+    ev._finish_prepared_factorized_positions(generation)
+    assert np.abs(ev.node_energies - again["energies_comm"][0]).max() <= 2e-6
+
+
 def test_ensemble_returns_mean_committee_and_variance(pkg, model_path):
     """Committee of models evaluated in one process (symmetrix/source/symmetrix/ensemble.py:166-212)."""
     paths = [model_path("small", seed=s) for s in (31, 32, 33)]
