@@ -143,6 +143,16 @@ int sxb_compute_positions_device(sxb_evaluator* evaluator, uint64_t generation, 
 int sxb_begin_positions(sxb_evaluator* evaluator, uint64_t generation, const double* positions);
 int sxb_finish_positions(sxb_evaluator* evaluator, uint64_t generation);
 
+/* One velocity-Verlet step around an evaluation, on arrays in device memory (f64: x, v, f, f_out, x_ref [3*n], m [n]), each
+ * half in one kernel on the caller's stream (a cudaStream_t; both calls wait for it).
+ * advance: v += half * f / m, x += dt * v; *moved = the largest squared distance of an atom from x_ref (NaN if one is NaN).
+ * finish: f_out = the forces of the last evaluation, which has to be of n atoms; v += half * f_out / m;
+ * *twice_kinetic = sum(m v^2). */
+int sxb_md_advance(sxb_evaluator* evaluator, void* stream, int32_t n, double dt, double half, double* x, double* v,
+                   const double* f, const double* m, const double* x_ref, double* moved);
+int sxb_md_finish(sxb_evaluator* evaluator, void* stream, int32_t n, double half, double* v, const double* m, double* f_out,
+                  double* twice_kinetic);
+
 /* Replaces _compute_prepared_factorized(generation, xyz, r) and the one-shot
  * compute_node_energies_forces(num_nodes, node_types, num_neigh, neigh_indices, neigh_types, xyz, r)
  * (symmetrix/source/cpp/mace_kokkos.cpp:1817-1827, 2169-2204): edge vectors xyz f64[3*num_edges] in

@@ -303,6 +303,26 @@ int sxb_finish_positions(sxb_evaluator* ev, uint64_t generation)
     });
 }
 
+int sxb_md_advance(sxb_evaluator* ev, void* stream, int32_t n, double dt, double half, double* x, double* v, const double* f,
+                   const double* m, const double* x_ref, double* moved)
+{
+    return guarded([&] {
+        require(ev, "evaluator"); require(x, "x"); require(v, "v"); require(f, "f"); require(m, "m"); require(x_ref, "x_ref");
+        require(moved, "moved");
+        *moved = ev->impl.md_advance(static_cast<cudaStream_t>(stream), n, dt, half, x, v, f, m, x_ref);
+    });
+}
+
+int sxb_md_finish(sxb_evaluator* ev, void* stream, int32_t n, double half, double* v, const double* m, double* f_out,
+                  double* twice_kinetic)
+{
+    return guarded([&] {
+        require(ev, "evaluator"); require(v, "v"); require(m, "m"); require(f_out, "f_out");
+        require(twice_kinetic, "twice_kinetic");
+        *twice_kinetic = ev->impl.md_finish(static_cast<cudaStream_t>(stream), n, half, v, m, f_out);
+    });
+}
+
 int sxb_compute_edge_vectors(sxb_evaluator* ev, uint64_t generation, const double* xyz)
 {
     return guarded([&] {

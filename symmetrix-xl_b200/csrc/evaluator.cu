@@ -20,6 +20,7 @@
 #include "edge_kernels_split.cuh"
 #include "edge_kernels_basis.cuh"
 #include "graph_kernels.cuh"
+#include "md_kernels.cuh"
 #include "node_kernels.cuh"
 #include "part_rules.hpp"
 #include "tc_gemm.cuh"
@@ -239,6 +240,7 @@ Evaluator::~Evaluator()
     if (stream_ && owns_stream_) cudaStreamDestroy(stream_);
     if (host_results_) cudaFreeHost(host_results_);
     if (host_stage_) cudaFreeHost(host_stage_);
+    if (md_host_) cudaFreeHost(md_host_);
 }
 
 void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num_receivers)
@@ -2103,6 +2105,41 @@ void Evaluator::synchronize()
         return;
     }
     SXB_CUDA(cudaStreamSynchronize(stream_));
+}
+
+void Evaluator::md_prepare()
+{
+    if (md_host_ != nullptr) return;
+    md_workspace_.reserve(sizeof(MdWorkspace));
+    SXB_CUDA(cudaMemset(md_workspace_.ptr, 0, sizeof(MdWorkspace)));
+    SXB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&md_host_), sizeof(double), cudaHostAllocMapped));
+}
+
+double Evaluator::md_advance(cudaStream_t stream, int n, double dt, double half, double* x, double* v, const double* f,
+                             const double* m, const double* x_ref)
+{
+    if (n < 1) throw std::invalid_argument("A molecular-dynamics step needs at least one atom.");
+    SXB_CUDA(cudaSetDevice(device_));
+    md_prepare();
+    md_advance_kernel<<<std::min<long>(blocks_for(n, kMdThreads), kMdBlocks), kMdThreads, 0, stream>>>(
+        n, dt, half, x, v, f, m, x_ref, reinterpret_cast<MdWorkspace*>(md_workspace_.ptr), md_host_);
+    SXB_CUDA(cudaGetLastError());
+    SXB_CUDA(cudaStreamSynchronize(stream));
+    return *static_cast<volatile double*>(md_host_);
+}
+
+double Evaluator::md_finish(cudaStream_t stream, int n, double half, double* v, const double* m, double* f_out)
+{
+    require_results();
+    if (n < 1 || n != num_nodes_ || n != num_receivers_)
+        throw std::invalid_argument("The molecular-dynamics step and the evaluated graph have different sizes.");
+    SXB_CUDA(cudaSetDevice(device_));
+    md_prepare();
+    md_finish_kernel<<<std::min<long>(blocks_for(n, kMdThreads), kMdBlocks), kMdThreads, 0, stream>>>(
+        n, half, v, m, forces_out_.ptr, f_out, reinterpret_cast<MdWorkspace*>(md_workspace_.ptr), md_host_);
+    SXB_CUDA(cudaGetLastError());
+    SXB_CUDA(cudaStreamSynchronize(stream));
+    return *static_cast<volatile double*>(md_host_);
 }
 
 void Evaluator::require_results() const

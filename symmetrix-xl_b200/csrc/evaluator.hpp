@@ -52,6 +52,10 @@ public:
 
     void compute_positions(std::uint64_t generation, const double* positions, bool on_device);
     void begin_positions(std::uint64_t generation, const double* positions, bool on_device);   // enqueues, does not wait
+    // the two halves of a velocity-Verlet step on the caller's stream; both wait for it
+    double md_advance(cudaStream_t stream, int n, double dt, double half, double* x, double* v, const double* f, const double* m,
+                      const double* x_ref);                                  // returns the largest squared displacement
+    double md_finish(cudaStream_t stream, int n, double half, double* v, const double* m, double* f_out);   // sum(m v^2)
     void finish_positions(std::uint64_t generation);                                           // waits and collects
     void compute_edge_vectors(std::uint64_t generation, const double* xyz);
     void synchronize();
@@ -164,6 +168,7 @@ private:
     };
     HaloPlan halo_plan_;
     bool use_graphs_ = true;
+    void md_prepare();
     void finish_compute();
     void collect_compute();     // waits for the evaluation whose end has been recorded, and reads status and totals
     void settle();              // waits for an evaluation that was begun and never finished
@@ -250,6 +255,8 @@ private:
     DeviceBuffer<int> source_offsets_, source_edges_;         // source schedule: edges sorted by source
     DeviceBuffer<int> det_sorted_sources_, det_edge_ids_, det_counts_;
     DeviceBuffer<double> det_partials_;
+    DeviceBuffer<unsigned char> md_workspace_;
+    double* md_host_ = nullptr;              // mapped: what one half of a molecular-dynamics step reports
     DeviceBuffer<float> halo_stage_;         // rows of H1 / H1_adj on their way to or from host buffers
     DeviceBuffer<double> edge_scratch_;      // [E][3]: caller edge vectors on the way in, un-permuted edge forces on the way out
     DeviceBuffer<int> error_flag_;

@@ -65,6 +65,9 @@ SIGNATURES = {
     "sxb_compute_positions_device": (ctypes.c_int, [_P, ctypes.c_uint64, _P]),
     "sxb_begin_positions": (ctypes.c_int, [_P, ctypes.c_uint64, _P]),
     "sxb_finish_positions": (ctypes.c_int, [_P, ctypes.c_uint64]),
+    "sxb_md_advance": (ctypes.c_int, [_P, _P, ctypes.c_int32, ctypes.c_double, ctypes.c_double, _P, _P, _P, _P, _P,
+                                      ctypes.POINTER(ctypes.c_double)]),
+    "sxb_md_finish": (ctypes.c_int, [_P, _P, ctypes.c_int32, ctypes.c_double, _P, _P, _P, ctypes.POINTER(ctypes.c_double)]),
     "sxb_compute_edge_vectors": (ctypes.c_int, [_P, ctypes.c_uint64, _P]),
     "sxb_synchronize": (ctypes.c_int, [_P]),
     "sxb_get_node_energies": (ctypes.c_int, [_P, _P, ctypes.c_int64]),
@@ -505,6 +508,18 @@ class MACEB200:
     def _finish_prepared_factorized_positions(self, graph_generation):
         """Second half: waits for the evaluation and collects its results."""
         _check(self._lib.sxb_finish_positions(self._h, int(graph_generation)))
+
+    def md_advance(self, stream, n, dt, half, x, v, f, m, x_ref):
+        """First half of a velocity-Verlet step on float64 device arrays; the largest squared displacement from ``x_ref``."""
+        moved = ctypes.c_double()
+        _check(self._lib.sxb_md_advance(self._h, stream, n, dt, half, x, v, f, m, x_ref, ctypes.byref(moved)))
+        return moved.value
+
+    def md_finish(self, stream, n, half, v, m, f_out):
+        """Second half, with the forces of the last evaluation, which are left in ``f_out``; the sum of ``m v^2``."""
+        total = ctypes.c_double()
+        _check(self._lib.sxb_md_finish(self._h, stream, n, half, v, m, f_out, ctypes.byref(total)))
+        return total.value
 
     def compute_positions_device(self, graph_generation, device_pointer: int):
         """Evaluation from float64 positions already resident on the evaluator's device."""

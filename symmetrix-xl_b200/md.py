@@ -1,6 +1,6 @@
 """Velocity-Verlet NVE molecular dynamics on the device, driven by the evaluator.
 
-Positions, velocities and forces stay in HBM; a step is two fused torch updates around one
+Positions, velocities and forces stay in HBM; a step is two kernels around one
 evaluation from device-resident positions.  The neighbor graph is built with a skin and rebuilt
 when the largest displacement since the last build exceeds skin/2, the reuse test of the
 reference's calculator (symmetrix/source/symmetrix/calculator.py:2894-2899).
@@ -53,13 +53,16 @@ class NVEIntegrator:
         self.x_ref = self.x.clone()
         self.rebuilds += 1
 
+    def _evaluate(self, moved):
+        if moved > (0.5 * self.skin) ** 2:
+            self._build()
+        self.ev.compute_positions_device(self.generation, self.x.data_ptr())
+
     def _forces(self):
         from .distributed import _as_tensor
 
         torch = self.torch
-        if float(((self.x - self.x_ref) ** 2).sum(dim=1).max()) > (0.5 * self.skin) ** 2:
-            self._build()
-        self.ev.compute_positions_device(self.generation, self.x.data_ptr())
+        self._evaluate(float(((self.x - self.x_ref) ** 2).sum(dim=1).max()))
         _e, f_ptr, _v = self.ev.device_results()
         forces = _as_tensor(torch, f_ptr, (self.n, 3), torch.float64, self.x.device).clone()
         return forces, self.ev.energy
@@ -67,8 +70,27 @@ class NVEIntegrator:
     def kinetic(self):
         return float(0.5 * KINETIC * (self.m * self.v * self.v).sum())
 
+    def _plain(self):
+        """The state is as it was set up here, and not tensors of another type, shape or layout put in its place, and no
+        subclass has its own forces or kinetic energy."""
+        torch, device, cls = self.torch, self.x_ref.device, type(self)
+        if cls._forces is not NVEIntegrator._forces or cls.kinetic is not NVEIntegrator.kinetic:
+            return False
+        return all(type(t) is torch.Tensor and t.dtype == torch.float64 and t.shape == shape and t.is_contiguous()
+                   and t.device == device and not t.requires_grad
+                   for t, shape in ((self.x, (self.n, 3)), (self.v, (self.n, 3)), (self.f, (self.n, 3)), (self.m, (self.n, 1)),
+                                    (self.x_ref, (self.n, 3))))
+
     def step(self):
         half = 0.5 * self.dt * ACCEL
+        if self._plain():
+            stream = self.torch.cuda.current_stream(self.x.device).cuda_stream
+            x, v, m = self.x.data_ptr(), self.v.data_ptr(), self.m.data_ptr()
+            self._evaluate(self.ev.md_advance(stream, self.n, self.dt, half, x, v, self.f.data_ptr(), m, self.x_ref.data_ptr()))
+            self.f = self.torch.empty_like(self.x)
+            twice_kinetic = self.ev.md_finish(stream, self.n, half, v, m, self.f.data_ptr())
+            self.potential = self.ev.energy
+            return self.potential + 0.5 * KINETIC * twice_kinetic
         self.v += half * self.f / self.m
         self.x += self.dt * self.v
         self.f, self.potential = self._forces()

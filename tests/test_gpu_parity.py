@@ -543,6 +543,56 @@ def test_nve_energy_conservation(pkg, model_path):
     assert md.kinetic() > 0
 
 
+@pytest.mark.parametrize("n", [1, 128, 129, 592 * 128 + 1])
+def test_advance_kernel_is_the_tensor_expression(pkg, model_path, n):
+    """Kick and drift bit for bit as the tensor expressions (one rounding per operation), a block's edge and more atoms than
+    the grid has threads; the largest squared displacement, also with a NaN among the atoms (it wins, as in max())."""
+    import torch
+
+    ev = pkg.MACEB200(model_path("small"))
+    gen = torch.Generator("cuda").manual_seed(n)
+    x, v, f, x_ref = (torch.randn((n, 3), dtype=torch.float64, device="cuda", generator=gen) for _ in range(4))
+    m = 1.0 + torch.rand((n, 1), dtype=torch.float64, device="cuda", generator=gen)
+    for bad in (False, True):
+        if bad:
+            f[n // 2, 1] = float("nan")
+        want_v = v + 0.37 * f / m
+        want_x = x + 0.9 * want_v
+        want = ((want_x - x_ref) ** 2).sum(dim=1).max().item()
+        got = ev.md_advance(torch.cuda.current_stream().cuda_stream, n, 0.9, 0.37, x.data_ptr(), v.data_ptr(), f.data_ptr(),
+                            m.data_ptr(), x_ref.data_ptr())
+        assert torch.equal(v.nan_to_num(7.0), want_v.nan_to_num(7.0)) and torch.equal(x.nan_to_num(7.0), want_x.nan_to_num(7.0))
+        assert np.isnan(got) if bad else abs(got - want) <= 4 * 2.0 ** -53 * want          # three squares, two sums
+
+
+@pytest.mark.parametrize("drop", [0, 6, 7, 8])
+def test_step_kernels_match_the_tensor_step(pkg, model_path, drop):
+    """The same trajectory from the two kernels and from tensor expressions, in the reproducible mode (equal forces for equal
+    positions): bit for bit, and the energies to the order of a sum of 3n squares.  127 to 135 atoms; lists are rebuilt."""
+    class Tensors(pkg.md.NVEIntegrator):
+        def kinetic(self):                      # a subclass with its own energy keeps the tensor step
+            return super().kinetic()
+
+    path = model_path("small")
+    pos, cell, types = pkg.modelgen.srtio3(3, 0.05, 3)
+    pos, types = pos[drop:], types[drop:]
+    masses = np.array([pkg.md.MASSES[z] for z in (8, 22, 38)])[types]
+    vel = pkg.md.maxwell_boltzmann(masses, 300.0, 3)
+    runs = []
+    for cls in (pkg.md.NVEIntegrator, Tensors):
+        ev = pkg.MACEB200(path)
+        ev.set_deterministic(True)
+        md = cls(ev, pos, cell, types, masses, vel, dt_fs=1.0, skin=0.02)
+        assert md._plain() == (cls is pkg.md.NVEIntegrator)
+        runs.append((md.run(8), md.x.cpu().numpy(), md.v.cpu().numpy(), md.f.cpu().numpy(), md.rebuilds, md.kinetic()))
+    for a, b in zip(runs[0][1:5], runs[1][1:5]):
+        assert np.array_equal(a, b)
+    assert runs[0][4] > 1
+    bound = 3 * len(pos) * 2.0 ** -53
+    assert abs(runs[0][5] - runs[1][5]) <= bound * runs[1][5]
+    assert np.abs(runs[0][0] - runs[1][0]).max() <= bound * runs[1][5] + 2.0 ** -52 * np.abs(runs[1][0]).max()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("arch,copies", [("medium", (2, 1, 1)), ("medium", (4, 2, 2)), ("small", (4, 2, 1)), ("large", (2, 2, 1))])
 def test_parts_of_a_receiver_add_up(pkg, model_path, arch, copies):
