@@ -58,10 +58,10 @@ __global__ void unpermute_edges_kernel(long num_edges, const int* __restrict__ e
     out[3 * o + 2] = in[3 * e + 2];
 }
 
-__global__ void narrow_offsets_kernel(int n, const long long* __restrict__ wide, int* __restrict__ narrow)
+__global__ void narrow_offsets_kernel(int n, int stride, const long long* __restrict__ wide, int* __restrict__ narrow)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= n) narrow[i] = static_cast<int>(wide[i]);
+    if (i <= n) narrow[i] = static_cast<int>(wide[static_cast<long>(i) * stride]);
 }
 
 inline int blocks_for(long n, int threads) { return static_cast<int>((n + threads - 1) / threads); }
@@ -245,12 +245,15 @@ Evaluator::~Evaluator()
 
 void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num_receivers)
 {
-    std::vector<int> requested(node_types);
-    std::sort(requested.begin(), requested.end());
-    requested.erase(std::unique(requested.begin(), requested.end()), requested.end());
-    if (requested.empty()) throw std::invalid_argument("MACE compact radial cache requires at least one active type.");
-    for (int t : requested)
+    if (node_types.empty()) throw std::invalid_argument("MACE compact radial cache requires at least one active type.");
+    std::vector<char> present(static_cast<std::size_t>(model_.num_elements), 0);
+    for (int t : node_types) {
         if (t < 0 || t >= model_.num_elements) throw std::invalid_argument("MACE active type index is out of range.");
+        present[t] = 1;
+    }
+    std::vector<int> requested;
+    for (int t = 0; t < model_.num_elements; ++t)
+        if (present[t]) requested.push_back(t);
     if (requested.size() > 255) throw std::invalid_argument("More than 255 active element types.");
     const int types = static_cast<int>(requested.size()), L = model_.l_max + 1;
     const bool changed = requested != active_types_;
@@ -262,7 +265,9 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num
     // built when a graph first asks for it
     basis_layer0_ = (model_.channels == 128 || model_.channels == 64) && radial_basis_width(model_, "R0") == kBasis
                     && PartRules{num_sms_, model_.channels, model_.shape_id, 0.0}.layer0_on_basis(num_receivers, types);
+    bool uploaded = changed;
     if (basis_layer0_ && !basis_ready_) {
+        uploaded = true;
         upload(basis_table_, build_r0_basis(model_, active_types_, &basis_pair_types_, false), stream_);
         upload(basis_steps_, build_r0_basis(model_, active_types_, &basis_pair_types_, true), stream_);
         s_a0_.resize(static_cast<std::size_t>(types) * L);
@@ -272,6 +277,7 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num
         basis_ready_ = true;
     }
     if (!basis_layer0_ && !table_ready_) {
+        uploaded = true;
         const auto table = fold_r0_table(model_, active_types_);
         if (table.size() > static_cast<std::size_t>(std::numeric_limits<int>::max()))
             throw std::length_error("Layer-0 spline table exceeds 32-bit indexing; too many active element types.");
@@ -279,7 +285,8 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num
         table_ready_ = true;
     }
     if (!changed) {
-        SXB_CUDA(cudaStreamSynchronize(stream_));
+        // with tables in place there is nothing to wait for: the neighbor search may still run while the host orders the nodes
+        if (uploaded) SXB_CUDA(cudaStreamSynchronize(stream_));
         return;
     }
     {
@@ -529,10 +536,18 @@ CellGrid finish_cell_grid(const double* inverse_cell, double cutoff)
             throw std::length_error("Cell list needs more bins along one axis than 32-bit indexing allows.");
         grid.bins[axis] = std::max(1, static_cast<int>(whole_bins));
         grid.reach[axis] = std::max(1, static_cast<int>(std::ceil(cutoff * inverse_spacing * grid.bins[axis]) + 1.0));
+        grid.range[axis] = cutoff * inverse_spacing * grid.bins[axis];
         total *= static_cast<std::size_t>(grid.bins[axis]);
         if (total >= static_cast<std::size_t>(std::numeric_limits<int>::max()))
             throw std::length_error("Cell list needs more bins than 32-bit indexing allows.");
     }
+    // The kernel passes over bins that lie beyond `range` along an axis.  Their distance is taken with the inverse cell, which
+    // may be off by 1e-9 of a period (validate_cell_pair): by that much of every period between two atoms, four times over, and
+    // by 1e-6 for the rounding of positions and distances, the range is widened.
+    double periods = 0.0;
+    for (int axis = 0; axis < 3; ++axis) periods += 1.0 + static_cast<double>(grid.reach[axis]) / grid.bins[axis];
+    for (int axis = 0; axis < 3; ++axis)
+        grid.range[axis] = grid.range[axis] * (1.0 + 1e-6) + 1e-6 + 4e-9 * periods * grid.bins[axis];
     grid.num_bins = static_cast<int>(total);
     grid.cutoff_squared = cutoff * cutoff;
     return grid;
@@ -565,19 +580,21 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
     nb_sorted_atoms_.reserve(n);
     nb_bin_sizes_.reserve(num_bins + 1);
     nb_bin_begin_.reserve(num_bins + 1);
-    nb_counts_.reserve(nr + 1);
-    nb_offsets_.reserve(nr + 1);
+    const int parts = stencil_parts(nr, num_sms_);
+    const int items = nr * parts;
+    nb_counts_.reserve(static_cast<std::size_t>(items) + 1);
+    nb_offsets_.reserve(static_cast<std::size_t>(items) + 1);
     int key_bits = 1;
     while ((1ll << key_bits) < static_cast<long long>(num_bins)) ++key_bits;
     std::size_t scan_bins_bytes = 0, scan_edges_bytes = 0, sort_bytes = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, scan_bins_bytes, nb_bin_sizes_.ptr, nb_bin_begin_.ptr, grid.num_bins + 1, stream_);
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_edges_bytes, nb_counts_.ptr, nb_offsets_.ptr, nr + 1, stream_);
+    cub::DeviceScan::ExclusiveSum(nullptr, scan_edges_bytes, nb_counts_.ptr, nb_offsets_.ptr, items + 1, stream_);
     cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, nb_atom_bin_.ptr, nb_sorted_bin_.ptr, nb_atom_index_.ptr, nb_sorted_atoms_.ptr, n,
                                     0, key_bits, stream_);
     nb_temp_.reserve(std::max(sort_bytes, std::max(scan_bins_bytes, scan_edges_bytes)));
 
     SXB_CUDA(cudaMemsetAsync(nb_bin_sizes_.ptr, 0, (num_bins + 1) * sizeof(int), stream_));
-    SXB_CUDA(cudaMemsetAsync(nb_counts_.ptr, 0, (nr + 1) * sizeof(long long), stream_));
+    SXB_CUDA(cudaMemsetAsync(nb_counts_.ptr, 0, (static_cast<std::size_t>(items) + 1) * sizeof(long long), stream_));
     SXB_CUDA(cudaMemsetAsync(error_flag_.ptr, 0, sizeof(int), stream_));
     wrap_and_bin_kernel<<<blocks_for(n, threads), threads, 0, stream_>>>(n, grid, positions_.ptr, inv_cell_.ptr, cell_.ptr,
                                                                           nb_wrapped_pos_.ptr, nb_wrap_count_.ptr, nb_atom_bin_.ptr,
@@ -588,14 +605,14 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
                                     nb_sorted_atoms_.ptr, n, 0, key_bits, stream_);
     gather_sorted_positions_kernel<<<blocks_for(n, threads), threads, 0, stream_>>>(n, nb_sorted_atoms_.ptr, nb_wrapped_pos_.ptr,
                                                                                      nb_sorted_pos_.ptr);
-    const int warp_blocks = blocks_for(static_cast<long>(nr) * 32, threads);
-    receiver_edges_kernel<false><<<warp_blocks, threads, 0, stream_>>>(nr, grid, nb_atom_bin_.ptr, nb_bin_begin_.ptr, nb_sorted_atoms_.ptr,
+    const int warp_blocks = blocks_for(static_cast<long>(items) * 32, threads);
+    receiver_edges_kernel<false><<<warp_blocks, threads, 0, stream_>>>(nr, parts, grid, nb_atom_bin_.ptr, nb_bin_begin_.ptr, nb_sorted_atoms_.ptr,
                                                                         nb_sorted_pos_.ptr, nb_wrapped_pos_.ptr, nb_wrap_count_.ptr,
-                                                                        cell_.ptr, nb_counts_.ptr, nullptr, nullptr, nullptr);
-    cub::DeviceScan::ExclusiveSum(nb_temp_.ptr, scan_edges_bytes, nb_counts_.ptr, nb_offsets_.ptr, nr + 1, stream_);
+                                                                        cell_.ptr, inv_cell_.ptr, nb_counts_.ptr, nullptr, nullptr, nullptr);
+    cub::DeviceScan::ExclusiveSum(nb_temp_.ptr, scan_edges_bytes, nb_counts_.ptr, nb_offsets_.ptr, items + 1, stream_);
     long long total = 0;
     int status = 0;
-    SXB_CUDA(cudaMemcpyAsync(&total, nb_offsets_.ptr + nr, sizeof(long long), cudaMemcpyDeviceToHost, stream_));
+    SXB_CUDA(cudaMemcpyAsync(&total, nb_offsets_.ptr + items, sizeof(long long), cudaMemcpyDeviceToHost, stream_));
     SXB_CUDA(cudaMemcpyAsync(&status, error_flag_.ptr, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     SXB_CUDA(cudaStreamSynchronize(stream_));
     if (status & 4) throw std::invalid_argument("Neighbor graph positions must be finite.");
@@ -605,10 +622,10 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
     first_caller_.reserve(nr + 1);
     sources_caller_.reserve_with_slack(static_cast<std::size_t>(total));
     shifts_caller_.reserve_with_slack(3 * static_cast<std::size_t>(total));
-    narrow_offsets_kernel<<<blocks_for(nr + 1, threads), threads, 0, stream_>>>(nr, nb_offsets_.ptr, first_caller_.ptr);
-    receiver_edges_kernel<true><<<warp_blocks, threads, 0, stream_>>>(nr, grid, nb_atom_bin_.ptr, nb_bin_begin_.ptr, nb_sorted_atoms_.ptr,
+    narrow_offsets_kernel<<<blocks_for(nr + 1, threads), threads, 0, stream_>>>(nr, parts, nb_offsets_.ptr, first_caller_.ptr);
+    receiver_edges_kernel<true><<<warp_blocks, threads, 0, stream_>>>(nr, parts, grid, nb_atom_bin_.ptr, nb_bin_begin_.ptr, nb_sorted_atoms_.ptr,
                                                                        nb_sorted_pos_.ptr, nb_wrapped_pos_.ptr, nb_wrap_count_.ptr,
-                                                                       cell_.ptr, nullptr, first_caller_.ptr, sources_caller_.ptr,
+                                                                       cell_.ptr, inv_cell_.ptr, nullptr, nb_offsets_.ptr, sources_caller_.ptr,
                                                                        shifts_caller_.ptr);
     launches_ += 5;
     SXB_CUDA(cudaGetLastError());
@@ -696,7 +713,7 @@ std::uint64_t Evaluator::prepare_graph_csr(int num_receivers, int num_nodes, con
     if (total > static_cast<long long>(std::numeric_limits<int>::max())) throw std::length_error("Graph exceeds 32-bit edge indexing.");
     const long E = static_cast<long>(total);
     first_caller_.reserve(R + 1);
-    narrow_offsets_kernel<<<blocks_for(R + 1, threads), threads, 0, stream_>>>(R, nb_offsets_.ptr, first_caller_.ptr);
+    narrow_offsets_kernel<<<blocks_for(R + 1, threads), threads, 0, stream_>>>(R, 1, nb_offsets_.ptr, first_caller_.ptr);
     sources_caller_.reserve_with_slack(static_cast<std::size_t>(E));
     if (E > 0) {
         SXB_CUDA(cudaMemcpyAsync(sources_caller_.ptr, neigh_indices, sizeof(int) * E, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream_));

@@ -4,7 +4,7 @@
 // (libsymmetrix/source/neighbor_graph_kokkos.cpp:39-405); the work split is different:
 //   * atoms are put in bin order by one stable radix sort of (bin, atom) pairs, so bins need no
 //     per-bin sort and the candidates of x-adjacent bins are contiguous in memory;
-//   * one warp owns a receiver; for each (z, y) row of the stencil it walks maximal runs of
+//   * one to eight warps own a receiver; for each (z, y) row of its share of the stencil a warp walks maximal runs of
 //     x-adjacent bins that share a periodic image, 32 candidates at a time, and compacts the accepted
 //     ones in order with a ballot and a prefix population count.
 // The distance test is evaluated in double with round-to-nearest adds and multiplies that are never
@@ -20,6 +20,7 @@ struct CellGrid {
     int bins[3];
     int reach[3];
     int num_bins;
+    double range[3];         // the cutoff in units of bins, a little more (see finish_cell_grid)
     double cutoff_squared;
 };
 
@@ -94,83 +95,105 @@ __device__ __forceinline__ int fold_bin(int raw, int extent, int& image)
     return raw - image * extent;
 }
 
-// kFill = false: counts[receiver] = number of accepted candidates.
-// kFill = true:  writes sources / shifts from offsets[receiver] on, in candidate order.
+// First and last bin offset along an axis that can hold a neighbor: a bin whose gap to the receiver, in units of bins, is beyond
+// `range` has none.  `inside` is where the receiver stands in its own bin, 0 to 1.
+__device__ __forceinline__ void stencil_extent(double inside, double range, int reach, int& low, int& high)
+{
+    high = static_cast<int>(fmin(static_cast<double>(reach), floor(range + inside)));
+    low = -static_cast<int>(fmin(static_cast<double>(reach), floor(range + 1.0 - inside)));
+}
+
+// kFill = false: counts[receiver * parts + part] = number of accepted candidates.
+// kFill = true:  writes sources / shifts from offsets[receiver * parts + part] on, in candidate order.
+// Both passes are serial chains of FP64 tests and ballots, 32 candidates a turn, so they are bound by the number of turns of a
+// warp.  The reference's stencil reaches one bin further than a neighbor can stand; the bins out of the receiver's range are
+// passed over (their candidates would all be rejected), and with few receivers the (z, y) rows are dealt to several warps.
+// From host positions to a ready graph, whole stencil by one warp, then as it is: 120 atoms 253 -> 143 us, 2,160: 270 -> 184,
+// 5,000: 373 -> 244, 20,480: 959 -> 485, 135,000: 4.55 -> 2.06 ms (6.5 A lists of about 99 neighbors; nodes sorted by a count).
 template <bool kFill>
 __global__ void __launch_bounds__(256)
-receiver_edges_kernel(int num_receivers, CellGrid grid, const int* __restrict__ atom_bin, const int* __restrict__ bin_begin,
+receiver_edges_kernel(int num_receivers, int parts, CellGrid grid, const int* __restrict__ atom_bin, const int* __restrict__ bin_begin,
                       const int* __restrict__ sorted_atoms, const double* __restrict__ sorted_pos,
                       const double* __restrict__ wrapped_pos, const int* __restrict__ wrap_count,
-                      const double* __restrict__ cell, long long* __restrict__ counts, const int* __restrict__ offsets,
-                      int* __restrict__ sources, int* __restrict__ shifts)
+                      const double* __restrict__ cell, const double* __restrict__ inv_cell, long long* __restrict__ counts,
+                      const long long* __restrict__ offsets, int* __restrict__ sources, int* __restrict__ shifts)
 {
-    const int receiver = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31u;
+    const int receiver = item / parts, part = item - receiver * parts;
     if (receiver >= num_receivers) return;
     const int nx = grid.bins[0], ny = grid.bins[1], nz = grid.bins[2];
     const int home = atom_bin[receiver];
     const int hx = home % nx, hy = (home / nx) % ny, hz = home / (nx * ny);
     const double rx = wrapped_pos[3 * receiver], ry = wrapped_pos[3 * receiver + 1], rz = wrapped_pos[3 * receiver + 2];
     const int wrx = wrap_count[3 * receiver], wry = wrap_count[3 * receiver + 1], wrz = wrap_count[3 * receiver + 2];
-    long long written = kFill ? offsets[receiver] : 0;
+    long long written = kFill ? offsets[item] : 0;
 
-    for (int dz = -grid.reach[2]; dz <= grid.reach[2]; ++dz) {
-        int iz;
-        const int bz = fold_bin(hz + dz, nz, iz);
+    int low[3], high[3];
+    const int own[3] = {hx, hy, hz};
+#pragma unroll
+    for (int axis = 0; axis < 3; ++axis) {
+        const double f = rx * inv_cell[axis] + ry * inv_cell[3 + axis] + rz * inv_cell[6 + axis];
+        const double inside = fmin(1.0, fmax(0.0, f * grid.bins[axis] - own[axis]));
+        stencil_extent(inside, grid.range[axis], grid.reach[axis], low[axis], high[axis]);
+    }
+    const int rows_y = high[1] - low[1] + 1;
+    const long rows = static_cast<long>(rows_y) * (high[2] - low[2] + 1);
+    const long row_begin = rows * part / parts, row_end = rows * (part + 1) / parts;
+    for (long t = row_begin; t < row_end; ++t) {
+        const int dz = low[2] + static_cast<int>(t / rows_y), dy = low[1] + static_cast<int>(t % rows_y);
+        int iz, iy;
+        const int bz = fold_bin(hz + dz, nz, iz), by = fold_bin(hy + dy, ny, iy);
         // image translation, one product per (axis, component); the sums below add them one at a time
         const double zx = __dmul_rn(static_cast<double>(iz), cell[6]), zy = __dmul_rn(static_cast<double>(iz), cell[7]),
                      zz = __dmul_rn(static_cast<double>(iz), cell[8]);
-        for (int dy = -grid.reach[1]; dy <= grid.reach[1]; ++dy) {
-            int iy;
-            const int by = fold_bin(hy + dy, ny, iy);
-            const double yx = __dmul_rn(static_cast<double>(iy), cell[3]), yy = __dmul_rn(static_cast<double>(iy), cell[4]),
-                         yz = __dmul_rn(static_cast<double>(iy), cell[5]);
-            const int row = (bz * ny + by) * nx;
-            int dx = -grid.reach[0];
-            while (dx <= grid.reach[0]) {
-                int ix;
-                const int bx = fold_bin(hx + dx, nx, ix);
-                // bins bx .. bx+run-1 of this row share the image ix and are contiguous in bin order
-                const int run = min(grid.reach[0] - dx + 1, nx - bx);
-                const double xx = __dmul_rn(static_cast<double>(ix), cell[0]), xy = __dmul_rn(static_cast<double>(ix), cell[1]),
-                             xz = __dmul_rn(static_cast<double>(ix), cell[2]);
-                const bool home_image = ix == 0 && iy == 0 && iz == 0;
-                const int first = bin_begin[row + bx], last = bin_begin[row + bx + run];
-                for (int k0 = first; k0 < last; k0 += 32) {
-                    const int k = k0 + static_cast<int>(lane);
-                    bool accept = false;
-                    int source = -1;
-                    if (k < last) {
-                        source = sorted_atoms[k];
-                        double d = __dadd_rn(sorted_pos[3 * k], -rx);
-                        d = __dadd_rn(__dadd_rn(__dadd_rn(d, xx), yx), zx);
-                        double d2 = __dmul_rn(d, d);
-                        d = __dadd_rn(sorted_pos[3 * k + 1], -ry);
-                        d = __dadd_rn(__dadd_rn(__dadd_rn(d, xy), yy), zy);
-                        d2 = __dadd_rn(d2, __dmul_rn(d, d));
-                        d = __dadd_rn(sorted_pos[3 * k + 2], -rz);
-                        d = __dadd_rn(__dadd_rn(__dadd_rn(d, xz), yz), zz);
-                        d2 = __dadd_rn(d2, __dmul_rn(d, d));
-                        accept = !(d2 > grid.cutoff_squared) && !(home_image && source == receiver);
-                    }
-                    const unsigned taken = __ballot_sync(0xffffffffu, accept);
-                    if constexpr (kFill) {
-                        if (accept) {
-                            const long long edge = written + __popc(taken & ((1u << lane) - 1u));
-                            sources[edge] = source;
-                            shifts[3 * edge] = ix - wrap_count[3 * source] + wrx;
-                            shifts[3 * edge + 1] = iy - wrap_count[3 * source + 1] + wry;
-                            shifts[3 * edge + 2] = iz - wrap_count[3 * source + 2] + wrz;
-                        }
-                    }
-                    written += __popc(taken);
+        const double yx = __dmul_rn(static_cast<double>(iy), cell[3]), yy = __dmul_rn(static_cast<double>(iy), cell[4]),
+                     yz = __dmul_rn(static_cast<double>(iy), cell[5]);
+        const int row = (bz * ny + by) * nx;
+        int dx = low[0];
+        while (dx <= high[0]) {
+            int ix;
+            const int bx = fold_bin(hx + dx, nx, ix);
+            // bins bx .. bx+run-1 of this row share the image ix and are contiguous in bin order
+            const int run = min(high[0] - dx + 1, nx - bx);
+            const double xx = __dmul_rn(static_cast<double>(ix), cell[0]), xy = __dmul_rn(static_cast<double>(ix), cell[1]),
+                         xz = __dmul_rn(static_cast<double>(ix), cell[2]);
+            const bool home_image = ix == 0 && iy == 0 && iz == 0;
+            const int first = bin_begin[row + bx], last = bin_begin[row + bx + run];
+            for (int k0 = first; k0 < last; k0 += 32) {
+                const int k = k0 + static_cast<int>(lane);
+                bool accept = false;
+                int source = -1;
+                if (k < last) {
+                    source = sorted_atoms[k];
+                    double d = __dadd_rn(sorted_pos[3 * k], -rx);
+                    d = __dadd_rn(__dadd_rn(__dadd_rn(d, xx), yx), zx);
+                    double d2 = __dmul_rn(d, d);
+                    d = __dadd_rn(sorted_pos[3 * k + 1], -ry);
+                    d = __dadd_rn(__dadd_rn(__dadd_rn(d, xy), yy), zy);
+                    d2 = __dadd_rn(d2, __dmul_rn(d, d));
+                    d = __dadd_rn(sorted_pos[3 * k + 2], -rz);
+                    d = __dadd_rn(__dadd_rn(__dadd_rn(d, xz), yz), zz);
+                    d2 = __dadd_rn(d2, __dmul_rn(d, d));
+                    accept = !(d2 > grid.cutoff_squared) && !(home_image && source == receiver);
                 }
-                dx += run;
+                const unsigned taken = __ballot_sync(0xffffffffu, accept);
+                if constexpr (kFill) {
+                    if (accept) {
+                        const long long edge = written + __popc(taken & ((1u << lane) - 1u));
+                        sources[edge] = source;
+                        shifts[3 * edge] = ix - wrap_count[3 * source] + wrx;
+                        shifts[3 * edge + 1] = iy - wrap_count[3 * source + 1] + wry;
+                        shifts[3 * edge + 2] = iz - wrap_count[3 * source + 2] + wrz;
+                    }
+                }
+                written += __popc(taken);
             }
+            dx += run;
         }
     }
     if constexpr (!kFill) {
-        if (lane == 0) counts[receiver] = written;
+        if (lane == 0) counts[item] = written;
     }
 }
 

@@ -8,8 +8,7 @@ namespace sxb {
 // The step moves 15 doubles per atom (260 KB for 2,160 atoms: far below a microsecond of HBM time); what it costs is
 // launches and waits.  As tensor expressions it took 17 launches and, with each result read by its own copy, two waits besides
 // that of the evaluation; here each half is one launch whose last block writes the one number that the host decides or reports
-// by into mapped memory: a step of 2,160 atoms
-// went from 1,451 to 1,283 µs, its neighbor lists included.
+// by into mapped memory: a step of 2,160 atoms went from 1,451 to 1,283 us, its neighbor lists included.
 // The operations and their rounding are those of the expressions  v += half * f / m;  x += dt * v  one by one (no FMA),
 // so a trajectory does not depend on which of the two forms ran.
 constexpr int kMdThreads = 128;

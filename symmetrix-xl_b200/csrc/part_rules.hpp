@@ -111,4 +111,15 @@ struct PartRules {
     }
 };
 
+// Warps that share a receiver's stencil in the neighbor search: as many as the chip holds at once, about half full.  The whole
+// build in us with 1 / 2 / 4 / 8 / 16: 40 receivers 179 / 173 / 138 / 136 / 133, 120: 162 / 144 / 138 / 138 / 136, 320: 167 / 153 /
+// 143 / 141 / 147, 1,080: 195 / 173 / 170 / 170 / 179, 2,160: 205 / 197 / 197 / 202 / 228, 5,000: 275 / 270 / 277 / 302 / 349,
+// 20,480: 597 / 617 / 671 / 774 / 985.
+inline int stencil_parts(long receivers, int num_sms)
+{
+    int parts = 1;
+    while (parts < 8 && 2 * parts * receivers <= 32l * num_sms) parts *= 2;
+    return parts;
+}
+
 }  // namespace sxb

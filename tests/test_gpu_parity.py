@@ -53,6 +53,33 @@ def test_neighbor_graph_triclinic_and_wrapped(pkg, model_path):
     assert mine == brute
 
 
+NEIGHBOR_EDGES = [("lattice", 8, 4.0), ("lattice", 10, 4.0), ("lattice", 12, 4.0), ("lattice", 14, 4.0), ("lattice", 8, 3.999),
+                  ("one", 1, 7.0), ("skewed", 1, 3.0), ("skewed", 40, 3.0), ("skewed", 700, 5.0), ("slab", 90, 6.5)]
+
+
+@pytest.mark.parametrize("kind,n,cutoff", NEIGHBOR_EDGES)
+def test_neighbor_graph_where_the_stencil_is_cut_short(pkg, model_path, kind, n, cutoff):
+    """Bins that a receiver's neighbors cannot reach are passed over and rows are dealt to 8, 4, 2 or 1 warps (592, 1,184 and
+    2,368 receivers): atoms exactly on the planes between bins with pairs exactly at the cutoff, cells far smaller than the
+    cutoff, strongly skewed cells, flat cells.  Bit for bit, order included."""
+    rng = np.random.default_rng(n)
+    if kind == "lattice":                    # spacing 2, bins of exactly one cutoff
+        pos = 2.0 * np.stack(np.meshgrid(*[np.arange(n)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+        cell = 2.0 * n * np.eye(3)
+    elif kind == "one":
+        pos, cell = np.array([[0.3, -0.2, 9.0]]), np.diag([2.0, 2.5, 30.0])
+    else:
+        cell = {"skewed": np.array([[6.0, 0.0, 0.0], [5.5, 7.0, 0.0], [-6.5, 5.0, 8.0]]) * max(1.0, (n / 40.0) ** (1 / 3)),
+                "slab": np.array([[22.0, 0.0, 0.0], [9.0, 18.0, 0.0], [1.0, 2.0, 3.5]])}[kind]
+        pos = rng.random((n, 3)) @ cell
+    types = rng.integers(0, 3, size=len(pos)).astype(np.int32)
+    ev = pkg.MACEB200(model_path("small"))
+    res = ev._prepare_periodic_factorized_graph(types, pos, cell, np.linalg.inv(cell), cutoff)
+    first, src, shifts = ev.graph(res["generation"])
+    ofirst, osrc, oshifts = neighbor.build_neighbor_graph(pos, cell, cutoff)
+    assert np.array_equal(first, ofirst) and np.array_equal(src, osrc) and np.array_equal(shifts, oshifts)
+
+
 @pytest.mark.parametrize("far", [1e12, -1e12, 1e300, -1e300, float("nan"), float("-inf")])
 def test_neighbor_graph_refuses_positions_it_cannot_wrap(pkg, model_path, far):
     """A coordinate whose count of cells does not fit 32 bits (a diverged trajectory is full of them) is an error like one that
