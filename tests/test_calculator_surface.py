@@ -131,6 +131,21 @@ def test_affine_cell_change_reuses_the_neighbor_list(pkg, model_path):
     assert calc.rebuilds == 2                      # a large strain rebuilds
 
 
+def test_short_lived_lists_are_launched_and_long_lived_ones_replayed(pkg, model_path):
+    """A list that follows one of fewer than eight evaluations is run kernel by kernel until its own eighth, then captured and
+    replayed.  In the reproducible mode all of them give the same bits, list after list."""
+    calc = pkg.Calculator(model_path("small"), skin=0.5)
+    calc.evaluator.set_deterministic(True)
+    structures = [pkg.modelgen.srtio3((2, 2, 1 + k % 2), 0.05, k) for k in range(4)]
+    want = {}
+    for evaluations in (1, 2, 7, 8, 9, 12, 1, 12):        # per list; crosses the eighth with short and with long ones before
+        for k, (pos, cell, types) in enumerate(structures):
+            for _ in range(evaluations):
+                out = calc.calculate(pos, cell, types)
+                first = want.setdefault(k, out)
+                assert out["energy"] == first["energy"] and np.array_equal(out["forces"], first["forces"])
+
+
 def test_members_in_flight_together_match_members_called_alone(pkg, model_path):
     """Members are begun before any is waited for: moving atoms, a member listed twice, and an input that the last
     step refuses (two atoms on one spot) leave every member usable.  The bound covers the order of the atomic sums
