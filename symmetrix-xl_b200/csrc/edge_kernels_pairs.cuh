@@ -11,8 +11,8 @@
 // Now FMA pipe 56 %, data pipe of L1 59 %, issue 52 %.  Reading 16 columns takes a warp 83 cycles with 16 warps on it, 390 bytes a
 // cycle and SM.  Other shapes measured: 16 channels x 4 edges a warp +13 % (every 32 bytes of another line cost a wavefront), L1
 // prefetch of the next edge's coefficients +15 %.
-// Rows without a coupling term are left out.  The reproducible mode keeps the register form, which leaves its records faster
-// (1,080 receivers: 0.295 against 0.469 ms).
+// Rows without a coupling term are left out.  In the reproducible mode the same kernel leaves records: every sum belongs to one
+// edge and has one order, whichever warp, chunk or part the edge falls to (1,080 receivers, register form / this: 293 / 180 us).
 //
 // Math and reference citations: see edge_kernels.cuh (layer 1 reverse).
 #pragma once
@@ -36,6 +36,15 @@ __device__ __forceinline__ void f2_red_split(float* address, f2 v)
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
     atomicAdd(address, lo);
     atomicAdd(address + kPairStep, hi);
+}
+
+// leaves a channel pair in a row of global memory that is read once, by another kernel
+__device__ __forceinline__ void f2_store_split(float* address, f2 v)
+{
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    address[0] = lo;
+    address[kPairStep] = hi;
 }
 
 // Harmonics in shared memory as pairs (Y, Y), each l starting on 16 bytes: l = 0 at 0, 1 at 2..4, 2 at 6..10, 3 at 12..18.
@@ -186,8 +195,9 @@ struct ChunkSums {
 };
 
 // Finishes the chunk's edges, one per thread of the first three warps: forces from the channel sums, pushed to the source atom;
-// leaves the receiver force and the virial of the chunk in totals[warp].
-template <int kGroups>
+// leaves the receiver force and the virial of the chunk in totals[warp].  With records (reproducible mode) each edge's force goes
+// to its place in out.edge_forces and nowhere else.
+template <int kGroups, bool kRecords>
 __device__ __forceinline__ void flush_active_chunk(const ActiveChunk& s, int count, const ChunkSums<kGroups>& sums, double (*__restrict__ totals)[kForceSums],
                                                    const ForceOutputs& out, float density_coef)
 {
@@ -215,9 +225,11 @@ __device__ __forceinline__ void flush_active_chunk(const ActiveChunk& s, int cou
         add_gradient_force(F, u.y, u.z, u.w, len.x, y, px, py, pz);
         const double ex = -static_cast<double>(px), ey = -static_cast<double>(py), ez = -static_cast<double>(pz);
         const int4 id = s.index[t];
-        atomicAdd(out.atom_forces + 3 * static_cast<size_t>(id.y), ex);
-        atomicAdd(out.atom_forces + 3 * static_cast<size_t>(id.y) + 1, ey);
-        atomicAdd(out.atom_forces + 3 * static_cast<size_t>(id.y) + 2, ez);
+        if constexpr (!kRecords) {
+            atomicAdd(out.atom_forces + 3 * static_cast<size_t>(id.y), ex);
+            atomicAdd(out.atom_forces + 3 * static_cast<size_t>(id.y) + 1, ey);
+            atomicAdd(out.atom_forces + 3 * static_cast<size_t>(id.y) + 2, ez);
+        }
         v[0] = -ex; v[1] = -ey; v[2] = -ez;
         const double rx = static_cast<double>(len.x) * u.y, ry = static_cast<double>(len.x) * u.z, rz = static_cast<double>(len.x) * u.w;
         v[3] = ex * rx; v[4] = ex * ry; v[5] = ex * rz;
@@ -229,6 +241,7 @@ __device__ __forceinline__ void flush_active_chunk(const ActiveChunk& s, int cou
             else { ef[0] = ex; ef[1] = ey; ef[2] = ez; }
         }
     }
+    if constexpr (kRecords) return;
     reduce_force_sums(v, lane);
     if ((lane & 7) == 0)
 #pragma unroll
@@ -303,7 +316,7 @@ static_assert(2 * kRowBatch * SXB_S2_ROW_BATCHES <= kPairColumnsS2 && kPairBlock
 static_assert(kPairBlocksS1 * pair_block_bytes(128) <= kSharedPerSM && kPairBlocksS2 * pair_block_bytes(128) <= kSharedPerSM, "shared memory");
 
 #define SXB_DEFINE_L1_PAIR_KERNEL(NAME)                                                                                 \
-template <int kC>                                                                                                       \
+template <int kC, bool kRecords = false>                                                                                \
 __global__ void __launch_bounds__(32 * kPairWarps##NAME, kPairBlocks##NAME)                                             \
 l1_reverse_pair_kernel_##NAME(int node0, const int* __restrict__ first, const int* __restrict__ sources,                \
                               const EdgeGeom* __restrict__ geom, const ActiveEdges active, SplineGrid grid,             \
@@ -375,20 +388,25 @@ l1_reverse_pair_kernel_##NAME(int node0, const int* __restrict__ first, const in
             f2 h[NH], hadj[NH], radial, rows[kRowBatch];                                                                \
             _Pragma("unroll") for (int b = 0; b < NH; ++b) h[b] = f2_pack(H1[source_row + b * kC], H1[source_row + b * kC + kPairStep]);\
             SXB_##NAME##_L1_REVERSE_EDGE_BODY                                                                           \
-            _Pragma("unroll") for (int b = 0; b < NH; ++b) f2_red_split(H1_adj + source_row + b * kC, hadj[b]);         \
+            /* kRecords: nothing is accumulated atomically; per-edge records are left for fixed-order passes */         \
+            float* adjoint = kRecords ? out.edge_source_adjoint + static_cast<size_t>(id.z) * NH * kC + k : H1_adj + source_row;\
+            _Pragma("unroll") for (int b = 0; b < NH; ++b) {                                                            \
+                if constexpr (kRecords) f2_store_split(adjoint + b * kC, hadj[b]);                                      \
+                else f2_red_split(adjoint + b * kC, hadj[b]);                                                           \
+            }                                                                                                           \
             f[0] = f2_sum(radial);                                                                                      \
             const float total_of = reduce16(f, lane);                                                                   \
             if ((lane & 1) == 0) channel_sums.f[t][16 * group + (lane >> 1)] = total_of;                                \
         }                                                                                                               \
         __syncthreads();                                                                                                \
-        flush_active_chunk<kGroups>(s, count, channel_sums, totals, out, density_coef);                                 \
+        flush_active_chunk<kGroups, kRecords>(s, count, channel_sums, totals, out, density_coef);                       \
     }                                                                                                                   \
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");                                                        \
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");                                                    \
     __syncthreads();                                                                                                    \
     if (warp == 0)                                                                                                      \
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(static_cast<unsigned>(kPairColumns##NAME)) : "memory");\
-    if (threadIdx.x < kForceSums) {                                                                                     \
+    if (!kRecords && threadIdx.x < kForceSums) {                                                                        \
         const double sum = totals[0][threadIdx.x] + totals[1][threadIdx.x] + totals[2][threadIdx.x];                    \
         if (threadIdx.x < 3) atomicAdd(out.atom_forces + 3 * static_cast<size_t>(i) + threadIdx.x, sum);                \
         else atomicAdd(out.virial_slots + (i % kVirialSlots) * 9 + threadIdx.x - 3, sum);                               \

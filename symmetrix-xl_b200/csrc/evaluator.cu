@@ -192,6 +192,7 @@ Evaluator::Evaluator(const std::string& json_path, int device_ordinal, const std
     SXB_ALLOW_POLY_SMEM(m1_forward_kernel_##NAME, SXB_##NAME##_M1_NUM_TERMS);                                           \
     SXB_ALLOW_POLY_SMEM(m1_reverse_kernel_##NAME, SXB_##NAME##_M1_NUM_TERMS)
 #define SXB_ALLOW_PAIR_CHUNK(NAME, WIDTH)                                                                                \
+    static_assert(SXB_##NAME##_NUM_HIDDEN > 4 || pair_dynamic_bytes(WIDTH) <= 48 * 1024, "records: no limit is set");     \
     SXB_CUDA(cudaFuncSetAttribute(l1_reverse_pair_kernel_##NAME<WIDTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pair_dynamic_bytes(WIDTH))))
     if (model_.shape_id == 0) {
         SXB_ALLOW_POLY_SMEM_SHAPE(S0);
@@ -1389,21 +1390,23 @@ void Evaluator::run_pipeline(int phases)
             }
             span_end();
             // hidden l > 0 at the common widths: channel pairs with the row adjoints in tensor memory; otherwise one channel per thread
-            // with the adjoints in registers (16 rows for hidden 0e), which also leaves the records of the reproducible mode.
-            const bool paired = !deterministic_ && (model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64)));
+            // with the adjoints in registers (16 rows for hidden 0e).  Both leave records in the reproducible mode.
+            const bool paired = model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64));
             span_begin("l1_reverse");
             if (paired && fo.edge_forces != nullptr && t0 == 0)   // edges at or beyond the cutoff are not visited
                 SXB_CUDA(cudaMemsetAsync(fo.edge_forces, 0, sizeof(double) * 3 * num_edges_, stream_));
             const int pair_blocks = model_.shape_id == 2 ? kPairBlocksS2 : kPairBlocksS1;
             const int reverse_parts = paired ? rules.l1_reverse_pairs(T, pair_blocks) : rules.l1_reverse(T);
             const dim3 reverse_grid(T, reverse_parts);
-#define SXB_PAIR_REVERSE(NAME, WIDTH)                                                                                     \
-            l1_reverse_pair_kernel_##NAME<WIDTH><<<reverse_grid, 32 * kPairWarps##NAME, pair_dynamic_bytes(WIDTH), stream_>>>(  \
+#define SXB_PAIR_REVERSE(NAME, WIDTH, ...)                                                                                \
+            l1_reverse_pair_kernel_##NAME<WIDTH, ##__VA_ARGS__><<<reverse_grid, 32 * kPairWarps##NAME, pair_dynamic_bytes(WIDTH), stream_>>>(  \
                 t0, first_.ptr, sources_.ptr, geom_.ptr, active_edges(), grid_, reinterpret_cast<const float4*>(r1_table_.ptr), \
                 H1_.ptr, dPhi1_.ptr, coupling_, H1_adj_.ptr, fo, density1, r1_pair_types_)
             if (paired) {
                 if (model_.shape_id == 2) SXB_PAIR_REVERSE(S2, 128);
+                else if (C == 128 && deterministic_) SXB_PAIR_REVERSE(S1, 128, true);
                 else if (C == 128) SXB_PAIR_REVERSE(S1, 128);
+                else if (deterministic_) SXB_PAIR_REVERSE(S1, 64, true);
                 else SXB_PAIR_REVERSE(S1, 64);
             } else if (deterministic_ && model_.shape_id == 0)
                 l1_reverse_kernel_S0<0, 3, true><<<reverse_grid, C, 0, stream_>>>(T, t0, C, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, grid_,

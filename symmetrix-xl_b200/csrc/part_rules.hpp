@@ -102,8 +102,8 @@ struct PartRules {
 
     // Layer-1 gradient with the row adjoints in registers.  Hidden 0e: 128 registers and 26 KB a block, eight blocks of up to two
     // warps, four of four.  1 / 2 / 4 / 8 parts, 32 channels (58 edges), 40 receivers: 31 / 21 / 15 / 13, 600: 35 / 33 / 33 / 35,
-    // 1,080: 37 / 39 / 45 / 56, 1,500: 60 / 54 / 60 / 72.  0e+1o (other widths, records): counted with 12 warps; records at 128
-    // channels, 40: 68 / 39 / 29 / 27, 600: 201 / 177 / 176 / 199, 1,080: 293 / 293 / 308 / 353.
+    // 1,080: 37 / 39 / 45 / 56, 1,500: 60 / 54 / 60 / 72.  0e+1o (widths without a paired kernel): counted with 12 warps; its
+    // records at 128 channels, 40: 68 / 39 / 29 / 27, 600: 201 / 177 / 176 / 199, 1,080: 293 / 293 / 308 / 353.
     int l1_reverse(long receivers) const
     {
         const int resident = shape == 0 ? std::min(8, 16 / block_warps()) : 12 / block_warps();

@@ -570,6 +570,26 @@ def test_nve_energy_conservation(pkg, model_path):
     assert md.kinetic() > 0
 
 
+@pytest.mark.parametrize("channels,scale", [(128, 1.0), (128, 0.9), (64, 0.9)])
+def test_records_of_the_paired_gradient_match_its_atomic_sums(pkg, model_path, channels, scale):
+    """The reproducible mode's records against the default build of the same kernel: one chunk of edges per receiver, and a
+    compressed cell with more than a chunk holds (96); in few parts and in many (40 and 320 receivers).  The two differ in the
+    order of FP32 sums of about 100 edges: bounds of 2^-24 times the terms of a sum times the largest row, with room for the
+    linears behind it.  Bits do not depend on the list's skin."""
+    for copies in (2, 4):
+        pos, cell, types = pkg.modelgen.srtio3(copies, 0.05, 8)
+        pos, cell = pos * scale, cell * scale
+        runs = []
+        for fixed, skin in ((False, 0.5), (True, 0.5), (True, 0.2)):
+            calc = pkg.Calculator(model_path("medium", seed=5, channels=channels), skin=skin)
+            calc.evaluator.set_deterministic(fixed)
+            runs.append(calc.calculate(pos, cell, types))
+        bound = 100 * 2.0 ** -24 * max(1.0, np.abs(runs[0]["forces"]).max())
+        assert np.abs(runs[1]["forces"] - runs[0]["forces"]).max() <= bound
+        assert np.abs(runs[1]["stress"] - runs[0]["stress"]).max() <= 0.1 * bound
+        assert np.array_equal(runs[1]["forces"], runs[2]["forces"]) and runs[1]["energy"] == runs[2]["energy"]
+
+
 @pytest.mark.parametrize("n", [1, 128, 129, 592 * 128 + 1])
 def test_advance_kernel_is_the_tensor_expression(pkg, model_path, n):
     """Kick and drift bit for bit as the tensor expressions (one rounding per operation), a block's edge and more atoms than
