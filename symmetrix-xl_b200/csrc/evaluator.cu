@@ -242,6 +242,7 @@ Evaluator::~Evaluator()
     if (host_results_) cudaFreeHost(host_results_);
     if (host_stage_) cudaFreeHost(host_stage_);
     if (md_host_) cudaFreeHost(md_host_);
+    if (search_host_) cudaFreeHost(search_host_);
 }
 
 void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num_receivers)
@@ -569,8 +570,6 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
 
     positions_.reserve(3 * static_cast<std::size_t>(n));
     SXB_CUDA(cudaMemcpyAsync(positions_.ptr, positions, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, stream_));
-    SXB_CUDA(cudaMemcpyAsync(cell_.ptr, cell, 9 * sizeof(double), cudaMemcpyHostToDevice, stream_));
-    SXB_CUDA(cudaMemcpyAsync(inv_cell_.ptr, inverse_cell, 9 * sizeof(double), cudaMemcpyHostToDevice, stream_));
     // cell-list scratch lives in members: a rebuild allocates nothing once the sizes have settled
     nb_wrapped_pos_.reserve(3 * static_cast<std::size_t>(n));
     nb_sorted_pos_.reserve(3 * static_cast<std::size_t>(n));
@@ -594,9 +593,12 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
                                     0, key_bits, stream_);
     nb_temp_.reserve(std::max(sort_bytes, std::max(scan_bins_bytes, scan_edges_bytes)));
 
-    SXB_CUDA(cudaMemsetAsync(nb_bin_sizes_.ptr, 0, (num_bins + 1) * sizeof(int), stream_));
-    SXB_CUDA(cudaMemsetAsync(nb_counts_.ptr, 0, (static_cast<std::size_t>(items) + 1) * sizeof(long long), stream_));
-    SXB_CUDA(cudaMemsetAsync(error_flag_.ptr, 0, sizeof(int), stream_));
+    if (search_host_ == nullptr) SXB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&search_host_), 2 * sizeof(long long), cudaHostAllocMapped));
+    CellPair pair;
+    std::copy(cell, cell + 9, pair.cell);
+    std::copy(inverse_cell, inverse_cell + 9, pair.inverse);
+    begin_search_kernel<<<blocks_for(static_cast<long>(num_bins) + 1, threads), threads, 0, stream_>>>(
+        pair, cell_.ptr, inv_cell_.ptr, grid.num_bins, nb_bin_sizes_.ptr, items, nb_counts_.ptr, error_flag_.ptr);
     wrap_and_bin_kernel<<<blocks_for(n, threads), threads, 0, stream_>>>(n, grid, positions_.ptr, inv_cell_.ptr, cell_.ptr,
                                                                           nb_wrapped_pos_.ptr, nb_wrap_count_.ptr, nb_atom_bin_.ptr,
                                                                           nb_atom_index_.ptr, nb_bin_sizes_.ptr, error_flag_.ptr);
@@ -611,11 +613,11 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
                                                                         nb_sorted_pos_.ptr, nb_wrapped_pos_.ptr, nb_wrap_count_.ptr,
                                                                         cell_.ptr, inv_cell_.ptr, nb_counts_.ptr, nullptr, nullptr, nullptr);
     cub::DeviceScan::ExclusiveSum(nb_temp_.ptr, scan_edges_bytes, nb_counts_.ptr, nb_offsets_.ptr, items + 1, stream_);
-    long long total = 0;
-    int status = 0;
-    SXB_CUDA(cudaMemcpyAsync(&total, nb_offsets_.ptr + items, sizeof(long long), cudaMemcpyDeviceToHost, stream_));
-    SXB_CUDA(cudaMemcpyAsync(&status, error_flag_.ptr, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    report_search_kernel<<<1, 1, 0, stream_>>>(nb_offsets_.ptr + items, error_flag_.ptr, search_host_);
+    SXB_CUDA(cudaGetLastError());
     SXB_CUDA(cudaStreamSynchronize(stream_));
+    const long long total = static_cast<volatile long long*>(search_host_)[0];
+    const int status = static_cast<int>(static_cast<volatile long long*>(search_host_)[1]);
     if (status & 4) throw std::invalid_argument("Neighbor graph positions must be finite.");
     if (status & 32) throw std::invalid_argument("Neighbor graph positions lie too many cells away from the periodic cell.");
     if (total > static_cast<long long>(std::numeric_limits<int>::max()))
@@ -628,7 +630,7 @@ std::pair<std::uint64_t, long> Evaluator::prepare_periodic_graph(int num_nodes, 
                                                                        nb_sorted_pos_.ptr, nb_wrapped_pos_.ptr, nb_wrap_count_.ptr,
                                                                        cell_.ptr, inv_cell_.ptr, nullptr, nb_offsets_.ptr, sources_caller_.ptr,
                                                                        shifts_caller_.ptr);
-    launches_ += 5;
+    launches_ += 7;
     SXB_CUDA(cudaGetLastError());
     std::vector<int> types(node_types, node_types + n);
     install_graph(nr, n, types, static_cast<long>(total), true);

@@ -256,6 +256,7 @@ private:
     DeviceBuffer<int> det_sorted_sources_, det_edge_ids_, det_counts_;
     DeviceBuffer<double> det_partials_;
     DeviceBuffer<unsigned char> md_workspace_;
+    long long* search_host_ = nullptr;       // mapped: number of edges and status of a neighbor search
     double* md_host_ = nullptr;              // mapped: what one half of a molecular-dynamics step reports
     DeviceBuffer<float> halo_stage_;         // rows of H1 / H1_adj on their way to or from host buffers
     DeviceBuffer<double> edge_scratch_;      // [E][3]: caller edge vectors on the way in, un-permuted edge forces on the way out

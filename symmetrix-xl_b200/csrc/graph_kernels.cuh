@@ -24,6 +24,34 @@ struct CellGrid {
     double cutoff_squared;
 };
 
+// What a search starts from, in one launch instead of three fills and two copies: the cell pair in its place, empty bins, a clear
+// status word.  For small graphs the launches and copies around the search cost more than the search: with this and the
+// report below a list of 120 atoms takes 118 instead of 143 us, of 2,160 atoms 152 instead of 184.
+struct CellPair {
+    double cell[9], inverse[9];
+};
+__global__ void begin_search_kernel(CellPair pair, double* __restrict__ cell, double* __restrict__ inv_cell, int num_bins,
+                                    int* __restrict__ bin_sizes, int items, long long* __restrict__ counts, int* __restrict__ status)
+{
+    const long k = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k < 9) {
+        cell[k] = pair.cell[k];
+        inv_cell[k] = pair.inverse[k];
+    }
+    if (k <= num_bins) bin_sizes[k] = 0;
+    if (k == 0) {
+        counts[items] = 0;
+        *status = 0;
+    }
+}
+
+// The number of edges and the status word, written to the host through its mapping.
+__global__ void report_search_kernel(const long long* __restrict__ total, const int* __restrict__ status, long long* __restrict__ host)
+{
+    host[0] = *total;
+    host[1] = *status;
+}
+
 // Fractional coordinates wrapped into [0, 1), the wrap count per axis, the wrapped Cartesian position
 // and the atom's bin; a non-finite coordinate raises bit 2 of the status word, one more than 2^31 - 1 cells
 // away bit 5.
@@ -109,7 +137,7 @@ __device__ __forceinline__ void stencil_extent(double inside, double range, int 
 // warp.  The reference's stencil reaches one bin further than a neighbor can stand; the bins out of the receiver's range are
 // passed over (their candidates would all be rejected), and with few receivers the (z, y) rows are dealt to several warps.
 // From host positions to a ready graph, whole stencil by one warp, then as it is: 120 atoms 253 -> 143 us, 2,160: 270 -> 184,
-// 5,000: 373 -> 244, 20,480: 959 -> 485, 135,000: 4.55 -> 2.06 ms (6.5 A lists of about 99 neighbors; nodes sorted by a count).
+// 5,000: 373 -> 244, 20,480: 959 -> 485, 135,000: 4.55 -> 2.06 ms, with the copies around it as they were (6.5 A lists of about 99 neighbors; nodes sorted by a count).
 template <bool kFill>
 __global__ void __launch_bounds__(256)
 receiver_edges_kernel(int num_receivers, int parts, CellGrid grid, const int* __restrict__ atom_bin, const int* __restrict__ bin_begin,
