@@ -1154,18 +1154,23 @@ void Evaluator::run_pipeline(int phases)
     if (phases & 1) {
         spans_.clear();
         events_used_ = 0;
-        SXB_CUDA(cudaMemsetAsync(forces_.ptr, 0, sizeof(double) * 3 * ALL, stream_));
-        SXB_CUDA(cudaMemsetAsync(H1_adj_.ptr, 0, sizeof(float) * static_cast<std::size_t>(ALL) * rowH, stream_));
+        ClearList clears;
+        clears.add(forces_.ptr, sizeof(double) * 3 * ALL);
+        clears.add(H1_adj_.ptr, sizeof(float) * static_cast<std::size_t>(ALL) * rowH);
+        clears.add(energy_slots_.ptr, sizeof(double) * kVirialSlots);
+        clears.add(virial_slots_.ptr, sizeof(double) * kVirialSlots * 9);
+        if (model_.a0_scaled) clears.add(dot0_.ptr, sizeof(float) * R);
+        if (model_.a1_scaled) clears.add(dot1_.ptr, sizeof(float) * R);
+        // one thread per 16 bytes of the largest region, up to eight blocks an SM
+        const long widest = std::max<long>(static_cast<long>(ALL) * static_cast<long>(rowH) / 4, 1);
+        clear_kernel<<<static_cast<int>(std::min<long>((widest + 255) / 256, 8l * num_sms_)), 256, 0, stream_>>>(clears);
+        launches_ += 1;
         if (model_.legacy_h1_basis) {   // old basis: dE/dH1 starts from the first readout's weights on the scalar block
             fill_scalar_block_kernel<<<blocks_for(static_cast<long>(R) * C, 256), 256, 0, stream_>>>(R, C, static_cast<long>(rowH),
                                                                                                     readout1_.ptr, H1_adj_.ptr);
             launches_ += 1;
         }
-        SXB_CUDA(cudaMemsetAsync(energy_slots_.ptr, 0, sizeof(double) * kVirialSlots, stream_));
-        SXB_CUDA(cudaMemsetAsync(virial_slots_.ptr, 0, sizeof(double) * kVirialSlots * 9, stream_));
         if (model_.a0_scaled || model_.a1_scaled) {
-            if (model_.a0_scaled) SXB_CUDA(cudaMemsetAsync(dot0_.ptr, 0, sizeof(float) * R, stream_));
-            if (model_.a1_scaled) SXB_CUDA(cudaMemsetAsync(dot1_.ptr, 0, sizeof(float) * R, stream_));
             span_begin("density_scales");
             density_scale_kernel<<<blocks_for(static_cast<long>(R) * 32, 256), 256, 0, stream_>>>(
                 R, first_.ptr, sources_.ptr, geom_.ptr, atype_.ptr, n_active, grid_, density0.table, density1.table, inv_scale0_.ptr,

@@ -572,6 +572,30 @@ SXB_DEFINE_NODE_READOUT(S1)
 SXB_DEFINE_NODE_READOUT(S2)
 #undef W
 
+// What an evaluation accumulates into, set to zero by one launch (a chain of four to six fills cost 1 to 2 us each, one after the
+// other: 40 atoms 193 -> 186 us, 320 atoms of the 32-channel model 166 -> 159, 5,000 atoms the same).  Regions of 4-byte words whose first lies on 16 bytes; the blocks stride over each in turn, 16 bytes a thread.
+constexpr int kMaxClears = 6;
+struct ClearList {
+    float* begin[kMaxClears];
+    long words[kMaxClears];
+    int count = 0;
+    void add(void* region, std::size_t bytes)
+    {
+        begin[count] = static_cast<float*>(region);
+        words[count++] = static_cast<long>(bytes / sizeof(float));
+    }
+};
+__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ClearList list)
+{
+    const long thread = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x, threads = static_cast<long>(gridDim.x) * blockDim.x;
+    for (int r = 0; r < list.count; ++r) {
+        const long vectors = list.words[r] >> 2;
+        for (long k = thread; k < vectors; k += threads)
+            reinterpret_cast<float4*>(list.begin[r])[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (thread < (list.words[r] & 3)) list.begin[r][4 * vectors + thread] = 0.0f;
+    }
+}
+
 // tensor[node][0][k] = values[k] for the first num_nodes nodes of a (node, component, channel) tensor.
 __global__ void fill_scalar_block_kernel(int num_nodes, int C, long node_stride, const float* __restrict__ values,
                                          float* __restrict__ tensor)
