@@ -249,10 +249,7 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num
 {
     if (node_types.empty()) throw std::invalid_argument("MACE compact radial cache requires at least one active type.");
     std::vector<char> present(static_cast<std::size_t>(model_.num_elements), 0);
-    for (int t : node_types) {
-        if (t < 0 || t >= model_.num_elements) throw std::invalid_argument("MACE active type index is out of range.");
-        present[t] = 1;
-    }
+    for (int t : node_types) present[t] = 1;
     std::vector<int> requested;
     for (int t = 0; t < model_.num_elements; ++t)
         if (present[t]) requested.push_back(t);
@@ -332,6 +329,15 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     // Receivers (nodes that own edges and readouts) come first in the caller's order; the nodes
     // after them are feature-only nodes (ghost atoms of a domain decomposition): they carry H1,
     // H1_adj, a type, a position and a force row, nothing else.
+    for (int t : node_types)
+        if (t < 0 || t >= model_.num_elements) throw std::invalid_argument("MACE active type index is out of range.");
+    // From here on tables, extents and buffers of the graph before are replaced one by one: its handle ends now, and not only
+    // when all of it has gone well.
+    generation_ += 1;
+    have_results_ = false;
+    mirror_valid_ = false;
+    pending_finish_ = false;
+    phase_ = 0;
     num_receivers_ = num_receivers;
     num_nodes_ = num_nodes;
     num_edges_ = num_edges;
@@ -484,13 +490,9 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
         host_results_ = host_stage_ = nullptr;
         host_results_capacity_ = 0;
     }
-    generation_ += 1;
     pending_ = false;             // the stream has been waited for above
     if (evaluations_ > 0) last_evaluations_ = evaluations_;
     evaluations_ = 0;
-    have_results_ = false;
-    mirror_valid_ = false;
-    phase_ = 0;
     halo_plan_ = HaloPlan{};      // buffers of a decomposed run belong to the previous graph
     geometry_mode_ = 0;           // a reference geometry belongs to the graph it was given for
 }

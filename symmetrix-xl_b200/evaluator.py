@@ -748,23 +748,27 @@ class Calculator:
             self.cell_updates += 1
         elif not reuse:
             cutoff = ev.r_cut + self.skin
-            if all(pbc):
-                result = ev._prepare_periodic_factorized_graph(node_types, positions, cell, np.linalg.inv(cell), cutoff)
-                self._generation = result["generation"]
-            else:
-                # axes that are not periodic get a stand-in cell vector long enough that nothing wraps
-                work_cell = cell.copy()
-                span = np.ptp(positions, axis=0).max() + 4.0 * cutoff + 1.0
-                for a in range(3):
-                    if not pbc[a]:
-                        work_cell[a] = 0.0
-                        work_cell[a, a] = span
-                self._work_cell, self._work_inverse = work_cell, np.linalg.inv(work_cell)
-                num_neigh, neigh, xyz = host_neighbor_list(positions, work_cell, pbc, cutoff)
-                ev._validate_graph_cardinality(len(positions), len(positions), len(neigh))
-                self._generation = ev._prepare_factorized_graph(len(positions), node_types, num_neigh, neigh, node_types[neigh])
-                ev._prepare_factorized_geometry(self._generation, positions, xyz, work_cell, np.linalg.inv(work_cell),
-                                                np.array(pbc, dtype=np.int32))
+            try:
+                if all(pbc):
+                    result = ev._prepare_periodic_factorized_graph(node_types, positions, cell, np.linalg.inv(cell), cutoff)
+                    self._generation = result["generation"]
+                else:
+                    # axes that are not periodic get a stand-in cell vector long enough that nothing wraps
+                    work_cell = cell.copy()
+                    span = np.ptp(positions, axis=0).max() + 4.0 * cutoff + 1.0
+                    for a in range(3):
+                        if not pbc[a]:
+                            work_cell[a] = 0.0
+                            work_cell[a, a] = span
+                    self._work_cell, self._work_inverse = work_cell, np.linalg.inv(work_cell)
+                    num_neigh, neigh, xyz = host_neighbor_list(positions, work_cell, pbc, cutoff)
+                    ev._validate_graph_cardinality(len(positions), len(positions), len(neigh))
+                    self._generation = ev._prepare_factorized_graph(len(positions), node_types, num_neigh, neigh, node_types[neigh])
+                    ev._prepare_factorized_geometry(self._generation, positions, xyz, work_cell, np.linalg.inv(work_cell),
+                                                    np.array(pbc, dtype=np.int32))
+            except Exception:
+                self._generation = 0         # the list before may have gone with the attempt: the next call builds its own
+                raise
             self._reference_positions = positions.copy()
             self._reference_cell = cell.copy()
             self._reference_fractional = positions @ np.linalg.inv(cell) if all(pbc) else None

@@ -761,3 +761,32 @@ def test_every_division_of_receivers(pkg, model_path, part_rule, arch, channels,
     out = calc.calculate(many, cell * np.array(copies)[:, None], np.tile(types, len(grid)))
     assert np.abs(out["energies"].reshape(len(grid), -1) - energies).max() <= TOL_E
     assert np.abs(out["forces"].reshape(len(grid), -1, 3) - forces).max() <= TOL_F
+
+
+@pytest.mark.gpu
+def test_a_graph_that_failed_to_install_ends_the_handle_before(pkg, model_path):
+    """Installation that throws after extents and tables have been replaced (the reproducible mode's records would take more than
+    16 GB): the handle before is refused, results are gone, and the calculator builds its list again, with the same bits.  Types
+    that are refused at once leave the handle as it was."""
+    calc = pkg.Calculator(model_path("medium"), skin=0.5)
+    calc.evaluator.set_deterministic(True)
+    ev = calc.evaluator
+    pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 6)
+    first = calc.calculate(pos, cell, types)
+    generation = calc._generation
+    bad = types.copy()
+    bad[3] = 3
+    with pytest.raises(ValueError):
+        ev._prepare_periodic_factorized_graph(bad, pos, cell, np.linalg.inv(cell), 6.5)
+    ev._compute_prepared_factorized_positions(generation, pos)
+    assert np.array_equal(ev.node_energies, first["energies"])
+    many, big, of = pkg.modelgen.srtio3((27, 26, 26), 0.05, 6)             # 91,260 atoms, 8.8 million edges
+    for _ in range(2):
+        with pytest.raises(ValueError, match="16 GB"):
+            calc.calculate(many, big, np.where(of == 2, 1, of).astype(np.int32))
+        with pytest.raises(ValueError, match="stale"):
+            ev._compute_prepared_factorized_positions(generation, pos)
+        with pytest.raises((RuntimeError, ValueError)):         # no results, or a buffer of the old extent
+            ev.node_energies
+    again = calc.calculate(pos, cell, types)
+    assert again["energy"] == first["energy"] and np.array_equal(again["forces"], first["forces"])
