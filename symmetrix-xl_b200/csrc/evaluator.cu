@@ -255,35 +255,31 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num
         if (present[t]) requested.push_back(t);
     if (requested.size() > 255) throw std::invalid_argument("More than 255 active element types.");
     const int types = static_cast<int>(requested.size()), L = model_.l_max + 1;
-    const bool changed = requested != active_types_;
-    if (changed) {
-        active_types_ = requested;
-        basis_ready_ = table_ready_ = false;
-    }
+    type_tables_.request(requested);
     // layer 0 on the functions of the radial network's last hidden layer, or on the folded table of every ordered pair: each
     // built when a graph first asks for it
     basis_layer0_ = (model_.channels == 128 || model_.channels == 64) && radial_basis_width(model_, "R0") == kBasis
                     && PartRules{num_sms_, model_.channels, model_.shape_id, 0.0}.layer0_on_basis(num_receivers, types);
-    bool uploaded = changed;
-    if (basis_layer0_ && !basis_ready_) {
+    bool uploaded = false;
+    if (basis_layer0_ && !type_tables_.basis) {
         uploaded = true;
-        upload(basis_table_, build_r0_basis(model_, active_types_, &basis_pair_types_, false), stream_);
-        upload(basis_steps_, build_r0_basis(model_, active_types_, &basis_pair_types_, true), stream_);
+        upload(basis_table_, build_r0_basis(model_, type_tables_.types, &basis_pair_types_, false), stream_);
+        upload(basis_steps_, build_r0_basis(model_, type_tables_.types, &basis_pair_types_, true), stream_);
         s_a0_.resize(static_cast<std::size_t>(types) * L);
         for (int a = 0; a < types; ++a)
             for (int l = 0; l < L; ++l)
-                upload_split(s_a0_[a * L + l], fold_r0_mixing(model_, active_types_, a, l).data(), types * kBasis, model_.channels);
-        basis_ready_ = true;
+                upload_split(s_a0_[a * L + l], fold_r0_mixing(model_, type_tables_.types, a, l).data(), types * kBasis, model_.channels);
+        type_tables_.basis = true;
     }
-    if (!basis_layer0_ && !table_ready_) {
+    if (!basis_layer0_ && !type_tables_.folded) {
         uploaded = true;
-        const auto table = fold_r0_table(model_, active_types_);
+        const auto table = fold_r0_table(model_, type_tables_.types);
         if (table.size() > static_cast<std::size_t>(std::numeric_limits<int>::max()))
             throw std::length_error("Layer-0 spline table exceeds 32-bit indexing; too many active element types.");
         upload(r0_table_, table, stream_);
-        table_ready_ = true;
+        type_tables_.folded = true;
     }
-    if (!changed) {
+    if (type_tables_.pairs) {
         // with tables in place there is nothing to wait for: the neighbor search may still run while the host orders the nodes
         if (uploaded) SXB_CUDA(cudaStreamSynchronize(stream_));
         return;
@@ -291,22 +287,22 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num
     {
         if (!model_.single_layer) {
             int pairs = 1;
-            const auto r1 = build_r1_table(model_, active_types_, &pairs);
+            const auto r1 = build_r1_table(model_, type_tables_.types, &pairs);
             if (r1.size() > static_cast<std::size_t>(std::numeric_limits<int>::max()))
                 throw std::length_error("Layer-1 spline table exceeds 32-bit indexing; too many active element types.");
             upload(r1_table_, r1, stream_);
         }
-        r1_pair_types_ = model_.agnesi ? static_cast<int>(active_types_.size()) : 1;
-        if (model_.a0_scaled) upload(density0_table_, build_density_table(model_, "A0", active_types_), stream_);
-        if (model_.a1_scaled) upload(density1_table_, build_density_table(model_, "A1", active_types_), stream_);
+        r1_pair_types_ = model_.agnesi ? static_cast<int>(type_tables_.types.size()) : 1;
+        if (model_.a0_scaled) upload(density0_table_, build_density_table(model_, "A0", type_tables_.types), stream_);
+        if (model_.a1_scaled) upload(density1_table_, build_density_table(model_, "A1", type_tables_.types), stream_);
     }
     if (model_.has_zbl) {
         // per-pair constants in the model precision, as the reference forms them (zbl.cpp:24-45)
-        const std::size_t n = active_types_.size();
+        const std::size_t n = type_tables_.types.size();
         std::vector<float> pairs(n * n * 4, 0.0f);
         for (std::size_t a = 0; a < n; ++a)
             for (std::size_t b = 0; b < n; ++b) {
-                const int Zu = model_.atomic_numbers[active_types_[a]], Zv = model_.atomic_numbers[active_types_[b]];
+                const int Zu = model_.atomic_numbers[type_tables_.types[a]], Zv = model_.atomic_numbers[type_tables_.types[b]];
                 if (Zu < 0 || Zv < 0 || static_cast<std::size_t>(std::max(Zu, Zv)) >= model_.zbl_covalent_radii.size())
                     throw std::invalid_argument("ZBL covalent radii do not cover the model's atomic numbers.");
                 const float zu = static_cast<float>(Zu), zv = static_cast<float>(Zv);
@@ -319,6 +315,7 @@ void Evaluator::prepare_active_types(const std::vector<int>& node_types, int num
             }
         upload(zbl_pairs_, pairs, stream_);
     }
+    type_tables_.pairs = true;
     SXB_CUDA(cudaStreamSynchronize(stream_));
 }
 
@@ -344,7 +341,7 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     has_shifts_ = has_shifts;
     prepare_active_types(node_types, num_receivers);
     std::vector<int> type_to_active(model_.num_elements, -1);
-    for (std::size_t a = 0; a < active_types_.size(); ++a) type_to_active[active_types_[a]] = static_cast<int>(a);
+    for (std::size_t a = 0; a < type_tables_.types.size(); ++a) type_to_active[type_tables_.types[a]] = static_cast<int>(a);
     // internal order: receivers stably grouped by element (a counting sort), feature-only nodes after them
     std::vector<int> original(num_nodes);
     std::iota(original.begin(), original.end(), 0);
@@ -356,14 +353,14 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     }
     std::vector<int> internal_of(num_nodes);
     std::vector<unsigned char> atype(num_nodes), element(num_nodes);
-    type_begin_.assign(active_types_.size() + 1, 0);
+    type_begin_.assign(type_tables_.types.size() + 1, 0);
     for (int i = 0; i < num_nodes; ++i) {
         internal_of[original[i]] = i;
         atype[i] = static_cast<unsigned char>(type_to_active[node_types[original[i]]]);
         element[i] = static_cast<unsigned char>(node_types[original[i]]);
         if (i < num_receivers) type_begin_[atype[i] + 1] += 1;
     }
-    for (std::size_t a = 0; a < active_types_.size(); ++a) type_begin_[a + 1] += type_begin_[a];
+    for (std::size_t a = 0; a < type_tables_.types.size(); ++a) type_begin_[a + 1] += type_begin_[a];
     if (model_.num_elements > 255) throw std::invalid_argument("More than 255 element types.");
     upload(original_, original, stream_);
     upload(internal_of_, internal_of, stream_);
@@ -402,7 +399,7 @@ void Evaluator::install_graph(int num_receivers, int num_nodes, const std::vecto
     active_ends_.reserve(N * edge_types());
     A0_.reserve(T * 16 * C);
     A0_adj_.reserve(T * 16 * C);
-    if (basis_layer0_) moments_.reserve(static_cast<std::size_t>(moment_receivers()) * 16 * kBasis * active_types_.size());
+    if (basis_layer0_) moments_.reserve(static_cast<std::size_t>(moment_receivers()) * 16 * kBasis * type_tables_.types.size());
     M0_.reserve(N * NH * C);
     M0_adj_.reserve(T * NH * C);
     H1_.reserve(ALL * NH * C);
@@ -1065,7 +1062,7 @@ ActiveEdges Evaluator::active_edges() const
 void Evaluator::run_pipeline(int phases)
 {
     const int R = num_receivers_, ALL = num_nodes_, C = model_.channels, NH = model_.num_hidden, NE = model_.num_lme;
-    const int n_active = static_cast<int>(active_types_.size());
+    const int n_active = static_cast<int>(type_tables_.types.size());
     const int tile_cap = tile_capacity();
     const bool tiled = tile_cap < R;
     const bool fused = fused_readout();
@@ -1203,7 +1200,7 @@ void Evaluator::run_pipeline(int phases)
             // one tile: the element-dependent skip term of H2 (x_i T_element) only needs M0, so it rides in this launch
             if (!fused && !tiled && !model_.legacy_h1_basis && !model_.pre_linear_up)
                 for_type_ranges(t0, T, [&](int a, int begin, int count) {
-                    calls.push_back({M0_.ptr + begin * rowH, scalar_rows, &s_h2_skip_[active_types_[a]], false,
+                    calls.push_back({M0_.ptr + begin * rowH, scalar_rows, &s_h2_skip_[type_tables_.types[a]], false,
                                      H2_.ptr + static_cast<std::size_t>(begin - t0) * C, flat_rows, 0, count, false, nullptr});
                 });
             if (model_.pre_linear_up)   // x = M0[l=0] P0, the scalar input of the first readout and the skip
@@ -1314,10 +1311,10 @@ void Evaluator::run_pipeline(int phases)
                     std::vector<TcCall> calls;
                     for_type_ranges(t0, T, [&](int a, int begin, int count) {
                         if (model_.pre_linear_up)
-                            calls.push_back({scalar_input_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[active_types_[a]],
+                            calls.push_back({scalar_input_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[type_tables_.types[a]],
                                              false, H2_.ptr + static_cast<std::size_t>(begin - t0) * C, flat_rows, 0, count, false, nullptr});
                         else
-                            calls.push_back({skip_input + begin * rowH, scalar_rows, &s_h2_skip_[active_types_[a]], false,
+                            calls.push_back({skip_input + begin * rowH, scalar_rows, &s_h2_skip_[type_tables_.types[a]], false,
                                              H2_.ptr + static_cast<std::size_t>(begin - t0) * C, flat_rows, 0, count, false, nullptr});
                     });
                     launch_tc(calls);
@@ -1356,12 +1353,12 @@ void Evaluator::run_pipeline(int phases)
                 // the reverse of the H1 linear adds to it later
                 if (model_.pre_linear_up)   // adjoint of x: q + S_element H2_adj, multiplied by P0^T in the last phase
                     for_type_ranges(t0, T, [&](int a, int begin, int count) {
-                        calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[active_types_[a]], true,
+                        calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[type_tables_.types[a]], true,
                                          scalar_adjoint_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, 0, count, false, readout1_.ptr});
                     });
                 else if (!tiled && !model_.legacy_h1_basis)
                     for_type_ranges(t0, T, [&](int a, int begin, int count) {
-                        calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[active_types_[a]], true,
+                        calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[type_tables_.types[a]], true,
                                          M0_adj_.ptr + (begin - t0) * rowH, scalar_rows, 0, count, false, readout1_.ptr});
                     });
                 launch_tc(calls);
@@ -1472,7 +1469,7 @@ void Evaluator::run_pipeline(int phases)
                 // old basis: the skip's adjoint S_element H2_adj joins H1_adj (which started from q) before the linear
                 std::vector<TcCall> calls;
                 for_type_ranges(t0, T, [&](int a, int begin, int count) {
-                    calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[active_types_[a]], true,
+                    calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[type_tables_.types[a]], true,
                                      H1_adj_.ptr + begin * rowH, scalar_rows, 0, count, true, nullptr});
                 });
                 launch_tc(calls);
@@ -1499,7 +1496,7 @@ void Evaluator::run_pipeline(int phases)
                 if (tiled && !fused) {
                     calls.clear();
                     for_type_ranges(t0, T, [&](int a, int begin, int count) {
-                        calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[active_types_[a]], true,
+                        calls.push_back({H2_adj_.ptr + static_cast<std::size_t>(begin) * C, flat_rows, &s_h2_skip_[type_tables_.types[a]], true,
                                          M0_adj_.ptr + (begin - t0) * rowH, scalar_rows, 0, count, true, nullptr});
                     });
                     launch_tc(calls);

@@ -14,6 +14,7 @@
 
 #include "model.hpp"
 #include "row_map.hpp"
+#include "type_tables.hpp"
 
 namespace sxb {
 
@@ -124,10 +125,10 @@ private:
     // (which stay in L2) / 0.8 GB: layer 0 7.9 / 6.8 ms; 20,000 with ten types 2.4 / 1.8 ms
     int moment_receivers() const
     {
-        const long fit = (1l << 30) / (16l * 64 * static_cast<long>(sizeof(float)) * static_cast<long>(std::max<std::size_t>(1, active_types_.size())));
+        const long fit = (1l << 30) / (16l * 64 * static_cast<long>(sizeof(float)) * static_cast<long>(std::max<std::size_t>(1, type_tables_.types.size())));
         return static_cast<int>(std::min<long>(tile_capacity(), std::max(1024l, fit)));
     }
-    int edge_types() const { return basis_layer0_ ? static_cast<int>(active_types_.size()) : 1; }   // types a receiver's edges are grouped by
+    int edge_types() const { return basis_layer0_ ? static_cast<int>(type_tables_.types.size()) : 1; }   // types a receiver's edges are grouped by
     // M1 to readout and back in one kernel (node_readout_kernel_*): the model has that form, and the graph is so small that short
     // dependent kernels cost more than the tensor cores gain.  By the receivers of the graph and not of the tile, so that tiles do
     // not change the arithmetic.  Five launches / one, us, 128 channels: 40 receivers 47 / 19, 320: 48 / 19, 1,080: 55 / 31, 5,000: 88 /
@@ -179,7 +180,7 @@ private:
     cudaStream_t stream_ = nullptr;
     cudaEvent_t event_begin_ = nullptr, event_end_ = nullptr;
     HostModel model_;
-    std::vector<int> active_types_;
+    TypeTables type_tables_;          // active element types and the tables that stand for them
     std::vector<int> type_begin_;
 
     // model tables on the device
@@ -204,7 +205,6 @@ private:
     std::vector<SplitWeight> s_a0_;   // [active type of the receiver][l]: radial functions of the network's last hidden layer to A0
     DeviceBuffer<float> basis_table_, basis_steps_, moments_;   // their splines in the order of either kernel; [slice][16][types * 64] sums over the edges, or their adjoints
     bool basis_layer0_ = false;       // layer 0 runs on those functions (chosen per graph)
-    bool basis_ready_ = false, table_ready_ = false;   // which of the two tables stands for the active types
     int basis_pair_types_ = 1;
     SplitWeight s_product0_;          // P0 of the pre_linear_up basis
     bool use_tensor_cores_ = true;

@@ -1,5 +1,11 @@
 """The rules that deal a receiver's edges to blocks and warps (csrc/part_rules.hpp), against measured kernel times."""
+import ctypes
+import subprocess
+from pathlib import Path
+
 import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
 
 # (hidden shape, channels, list edges, kernel, resident blocks of the shared-memory gradient): receivers -> us at 1, 2, 4, 8
 # parts (layer-0 sums: 1 and 4 parts) on 148 SMs, one launch of each kernel by CUDA events, medians of seven
@@ -51,3 +57,31 @@ def test_parts_stay_within_the_builds(part_rule):
                     for kernel in ("l1_forward", "l1_reverse", "l0_reverse"):
                         assert part_rule(kernel, *args, 0) in (1, 2, 4, 8)
                     assert part_rule("l1_forward", *args, 0) * receivers <= max(receivers, 148 * 5)
+
+
+def test_tables_of_a_preparation_that_threw_are_made_by_the_next(tmp_path):
+    """Bookkeeping of the type-dependent tables (csrc/type_tables.hpp): whichever of the uploads throws, the next preparation with
+    the same types makes what is missing, and other types make everything again."""
+    header = ROOT / "symmetrix-xl_b200" / "csrc" / "type_tables.hpp"
+    (tmp_path / "tables.cpp").write_text(
+        f'#include "{header}"\n#include <stdexcept>\n#include <string>\n'
+        "static sxb::TypeTables t;\nstatic int made[3];      // type that basis, folded table and pair tables were made for\n"
+        'extern "C" int prepare(int type, int on_basis, int fail)\n{\n    try {\n'
+        "        t.request({type});\n"
+        "        const auto make = [&](int table, bool& stands) {\n"
+        '            if (stands) return;\n            made[table] = -1;\n            if (fail == table) throw std::runtime_error("");\n'
+        "            made[table] = type;\n            stands = true;\n        };\n"
+        "        on_basis ? make(0, t.basis) : make(1, t.folded);\n        make(2, t.pairs);\n"
+        "    } catch (const std::runtime_error&) { return -1; }\n"
+        "    return made[on_basis ? 0 : 1] == type && made[2] == type;\n}\n")
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-shared", "-fPIC", "-o", str(tmp_path / "tables.so"),
+                    str(tmp_path / "tables.cpp")], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "tables.so"))
+    for on_basis in (0, 1):
+        for fail in (1 - on_basis, 2):
+            assert lib.prepare(7, on_basis, -1) == 1
+            assert lib.prepare(8, on_basis, fail) == -1
+            assert lib.prepare(8, on_basis, fail) == -1       # the same types again: not taken for prepared
+            assert lib.prepare(8, on_basis, -1) == 1
+            assert lib.prepare(8, 1 - on_basis, -1) == 1
+            assert lib.prepare(7, on_basis, fail) == -1 and lib.prepare(7, on_basis, -1) == 1
