@@ -1774,6 +1774,7 @@ void Evaluator::distributed_begin(std::uint64_t generation, const double* device
         throw std::logic_error("distributed evaluation: begin called while another evaluation is open.");
     }
     SXB_CUDA(cudaSetDevice(device_));
+    pending_ = false;         // an evaluation that was begun is dropped; its kernels come first on the stream
     have_results_ = false;
     mirror_valid_ = false;
     SXB_CUDA(cudaEventRecord(event_begin_, stream_));
@@ -1792,6 +1793,7 @@ void Evaluator::distributed_begin_edge_vectors(std::uint64_t generation, const d
         throw std::logic_error("distributed evaluation: begin called while another evaluation is open.");
     }
     SXB_CUDA(cudaSetDevice(device_));
+    pending_ = false;
     have_results_ = false;
     mirror_valid_ = false;
     SXB_CUDA(cudaEventRecord(event_begin_, stream_));
@@ -2094,6 +2096,7 @@ void Evaluator::set_halo_plan(const int* send_indices, long num_send, float* sen
 void Evaluator::mark_phases_replayed(std::uint64_t generation, long launches)
 {
     check_generation(generation);
+    pending_ = false;
     phase_ = 0;
     pending_finish_ = true;
     have_results_ = true;

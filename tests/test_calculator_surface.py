@@ -206,3 +206,36 @@ def test_ensemble_returns_mean_committee_and_variance(pkg, model_path):
         pkg.EnsembleCalculator(calculators=[ensemble.calculators[0], pkg.Calculator(model_path("medium", seed=31), skin=0.5)])
     with pytest.raises(TypeError):
         pkg.EnsembleCalculator(calculators=[ensemble.calculators[0], object()])
+
+
+@pytest.mark.parametrize("phases", ["device", "host", "vectors"])
+def test_an_evaluation_in_phases_drops_one_that_was_begun(pkg, model_path, phases):
+    """begin, then the first of three phases: finish is refused at every point of the phases, whose results are those of a whole
+    call (bound: the order of the atomic sums, as above)."""
+    import torch
+
+    pos, cell, types = pkg.modelgen.srtio3(2, 0.05, 8)
+    calc = pkg.Calculator(model_path("small", seed=31), skin=0.5)
+    want = calc.calculate(pos, cell, types)
+    ev, generation = calc.evaluator, calc._generation
+    first, src, shifts = ev.graph(generation)
+    receivers = np.repeat(np.arange(len(pos)), np.diff(first))
+    if phases == "vectors":
+        on_device = torch.from_numpy(pos[src] - pos[receivers] + shifts @ cell).cuda()
+    else:
+        on_device = torch.from_numpy(pos).cuda()
+    ev._begin_prepared_factorized_positions(generation, pos + 0.01)
+    if phases == "device":
+        ev.distributed_begin(generation, on_device.data_ptr())
+    elif phases == "host":
+        ev.distributed_begin_host(generation, pos)
+    else:
+        ev.distributed_begin_edge_vectors(generation, on_device.data_ptr())
+    for step in (ev.distributed_continue, ev.distributed_finish, ev.synchronize):
+        with pytest.raises(ValueError):
+            ev._finish_prepared_factorized_positions(generation)
+        step()
+    with pytest.raises(ValueError):
+        ev._finish_prepared_factorized_positions(generation)
+    assert np.abs(ev.node_energies - want["energies"]).max() <= 2e-6
+    assert np.abs(ev._reduce_atom_forces(len(pos), execution_graph_generation=generation) - want["forces"]).max() <= 2e-5
