@@ -681,6 +681,13 @@ def host_neighbor_list(positions, cell, pbc, cutoff):
     return num_neigh, neigh, xyz
 
 
+def runs_own(obj, cls, own):
+    """``obj`` is a ``cls`` that runs the methods ``own`` (name -> function, as ``cls`` defined them): no subclass, and nothing
+    set on the object or on the class, has put another in their place."""
+    return isinstance(obj, cls) and all(getattr(type(obj), name, None) is method and name not in vars(obj)
+                                        for name, method in own.items())
+
+
 class Calculator:
     """Minimal stand-in for the reference's ASE calculator hot path (``Symmetrix.calculate``,
     symmetrix/source/symmetrix/calculator.py:3934-4021): Verlet-skin neighbor cache (rebuild when
@@ -788,6 +795,11 @@ class Calculator:
         return out
 
 
+# what a member and its evaluator must run for the committee to begin and finish their evaluations itself
+_MEMBER_METHODS = {"calculate": Calculator.calculate}
+_EVALUATOR_METHODS = {"_compute_prepared_factorized_positions": MACEB200._compute_prepared_factorized_positions}
+
+
 class EnsembleCalculator:
     """Same-process committee of calculators, after the reference's ``SymmetrixEnsemble``
     (symmetrix/source/symmetrix/ensemble.py:65-212): members are evaluated on the same input, each on its
@@ -835,9 +847,10 @@ class EnsembleCalculator:
         return results
 
     def _member_results(self, positions, cell, node_types, pbc):
-        # a member that is listed twice, or whose class computes in its own way, is called as it stands
+        # when a member is listed twice, or computes in its own way (itself or its evaluator), all are called as they stand
         if len({id(m.evaluator) for m in self.calculators}) < self.num_models \
-                or any(type(m).calculate is not Calculator.calculate for m in self.calculators):
+                or not all(runs_own(m, Calculator, _MEMBER_METHODS) and runs_own(m.evaluator, MACEB200, _EVALUATOR_METHODS)
+                           for m in self.calculators):
             return [member.calculate(positions, cell, node_types, pbc) for member in self.calculators]
         begun, outputs = [], []
         try:

@@ -239,3 +239,57 @@ def test_an_evaluation_in_phases_drops_one_that_was_begun(pkg, model_path, phase
         ev._finish_prepared_factorized_positions(generation)
     assert np.abs(ev.node_energies - want["energies"]).max() <= 2e-6
     assert np.abs(ev._reduce_atom_forces(len(pos), execution_graph_generation=generation) - want["forces"]).max() <= 2e-5
+
+
+class _Restrained:
+    """An evaluator-like object around an evaluator: a harmonic term added to what it computes."""
+
+    def __init__(self, evaluator):
+        self._evaluator = evaluator
+
+    def __getattr__(self, name):
+        return getattr(self._evaluator, name)
+
+    @property
+    def node_energies(self):
+        return self._evaluator.node_energies + 1.0
+
+
+@pytest.mark.parametrize("way", ["evaluator subclass", "evaluator object", "evaluator instance", "evaluator class", "member subclass",
+                                 "member instance", "member class"])
+def test_members_that_compute_in_their_own_way_are_called(pkg, model_path, monkeypatch, way):
+    """Whatever a member or its evaluator has put in the place of its call is what the committee runs."""
+    pos, cell, types = pkg.modelgen.srtio3(1, 0.05, 8)
+    members = [pkg.Calculator(model_path("small", seed=s), skin=0.5) for s in (31, 32)]
+    plain = [m.calculate(pos, cell, types) for m in members]
+    last, calls = members[1], []
+    compute, calculate = pkg.MACEB200._compute_prepared_factorized_positions, pkg.Calculator.calculate
+
+    def compute_and_count(self, generation, positions):
+        calls.append(1)
+        return compute(self, generation, positions)
+
+    def shifted(self, *args, **kwargs):
+        calls.append(1)
+        out = calculate(self, *args, **kwargs)
+        out["energies"] = out["energies"] + 1.0
+        return out
+
+    kind, place = way.split()
+    if way == "evaluator object":
+        last.evaluator = _Restrained(last.evaluator)
+        calls.append(1)
+    else:
+        name, method = ("_compute_prepared_factorized_positions", compute_and_count) if kind == "evaluator" else ("calculate", shifted)
+        target = last.evaluator if kind == "evaluator" else last
+        if place == "subclass":
+            target.__class__ = type("Own", (type(target),), {name: method})
+        elif place == "instance":
+            setattr(target, name, method.__get__(target))
+        else:
+            monkeypatch.setattr(type(target), name, method)
+    out = pkg.EnsembleCalculator(calculators=members).calculate(pos, cell, types)
+    assert calls
+    shift = 1.0 if way == "evaluator object" or kind == "member" else 0.0
+    assert np.abs(out["energies_comm"][1] - plain[1]["energies"] - shift).max() <= 2e-6
+    assert np.abs(out["energies_comm"][0] - plain[0]["energies"] - (shift if place == "class" else 0.0)).max() <= 2e-6
