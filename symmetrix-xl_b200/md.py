@@ -10,6 +10,8 @@ from __future__ import annotations
 
 import numpy as np
 
+from .evaluator import MACEB200, runs_own
+
 ACCEL = 9.648533212331e-3      # (eV/A/amu) -> A/fs^2
 KINETIC = 103.642696562621     # amu*A^2/fs^2 -> eV
 KB = 8.617333262e-5            # eV/K
@@ -71,10 +73,12 @@ class NVEIntegrator:
         return float(0.5 * KINETIC * (self.m * self.v * self.v).sum())
 
     def _plain(self):
-        """The state is as it was set up here, and not tensors of another type, shape or layout put in its place, and no
-        subclass has its own forces or kinetic energy."""
-        torch, device, cls = self.torch, self.x_ref.device, type(self)
-        if cls._forces is not NVEIntegrator._forces or cls.kinetic is not NVEIntegrator.kinetic:
+        """The state is as it was set up here, and not tensors of another type, shape or layout put in its place, and neither the
+        integrator nor the evaluator has its own forces, kinetic energy or step (a restraint, a bias force)."""
+        torch, device = self.torch, self.x_ref.device
+        if not runs_own(self, NVEIntegrator, _STEP_METHODS) or not runs_own(self.ev, MACEB200, _EVALUATOR_METHODS):
+            return False
+        if not isinstance(self.dt, (int, float)):
             return False
         return all(type(t) is torch.Tensor and t.dtype == torch.float64 and t.shape == shape and t.is_contiguous()
                    and t.device == device and not t.requires_grad
@@ -87,8 +91,9 @@ class NVEIntegrator:
             stream = self.torch.cuda.current_stream(self.x.device).cuda_stream
             x, v, m = self.x.data_ptr(), self.v.data_ptr(), self.m.data_ptr()
             self._evaluate(self.ev.md_advance(stream, self.n, self.dt, half, x, v, self.f.data_ptr(), m, self.x_ref.data_ptr()))
-            self.f = self.torch.empty_like(self.x)
-            twice_kinetic = self.ev.md_finish(stream, self.n, half, v, m, self.f.data_ptr())
+            forces = self.torch.empty_like(self.x)
+            twice_kinetic = self.ev.md_finish(stream, self.n, half, v, m, forces.data_ptr())
+            self.f = forces
             self.potential = self.ev.energy
             return self.potential + 0.5 * KINETIC * twice_kinetic
         self.v += half * self.f / self.m
@@ -103,3 +108,8 @@ class NVEIntegrator:
         for _ in range(steps):
             energies.append(self.step())
         return np.array(energies)
+
+
+# what the integrator and its evaluator must run for the two step kernels to take the tensor expressions' place
+_STEP_METHODS = {"_forces": NVEIntegrator._forces, "kinetic": NVEIntegrator.kinetic}
+_EVALUATOR_METHODS = {name: getattr(MACEB200, name) for name in ("device_results", "md_advance", "md_finish")}

@@ -640,6 +640,67 @@ def test_step_kernels_match_the_tensor_step(pkg, model_path, drop):
     assert np.abs(runs[0][0] - runs[1][0]).max() <= bound * runs[1][5] + 2.0 ** -52 * np.abs(runs[1][0]).max()
 
 
+@pytest.mark.parametrize("way", ["evaluator subclass", "evaluator object", "evaluator instance", "evaluator class", "integrator subclass",
+                                 "integrator instance", "integrator class", "time step"])
+def test_forces_of_ones_own_steer_the_step(pkg, model_path, monkeypatch, way):
+    """Forces that an evaluator or an integrator puts in the place of the computed ones (here: none, the atoms fly straight) are
+    those of the step, as is a time step for each atom."""
+    import torch
+
+    pos, cell, types = pkg.modelgen.srtio3(1, 0.05, 3)
+    masses = np.array([pkg.md.MASSES[z] for z in (8, 22, 38)])[types]
+    vel = pkg.md.maxwell_boltzmann(masses, 300.0, 3)
+    zeros = torch.zeros((len(pos), 3), dtype=torch.float64, device="cuda")
+    results = pkg.MACEB200.device_results
+
+    def device_results(self):
+        energy, _forces, virial = results(getattr(self, "inner", self))
+        return energy, zeros.data_ptr(), virial
+
+    class Wrapper:
+        def __init__(self, inner):
+            self.inner = inner
+
+        def __getattr__(self, name):
+            if name.startswith("md_"):
+                raise AttributeError(name)
+            return getattr(self.inner, name)
+
+    Wrapper.device_results = device_results
+    ev = pkg.MACEB200(model_path("small"))
+    kind, place = way.split()
+    if way == "evaluator object":
+        ev = Wrapper(ev)
+    elif way == "evaluator subclass":
+        ev.__class__ = type("Own", (pkg.MACEB200,), {"device_results": device_results})
+    elif way == "evaluator instance":
+        ev.device_results = device_results.__get__(ev)
+    elif way == "evaluator class":
+        monkeypatch.setattr(pkg.MACEB200, "device_results", device_results)
+    md = pkg.md.NVEIntegrator(ev, pos, cell, types, masses, vel, dt_fs=1.0)
+    if kind == "integrator":
+        def forces(self):
+            self._evaluate(0.0)
+            return zeros.clone(), self.ev.energy
+
+        md.f = zeros.clone()
+        if place == "instance":
+            md._forces = forces.__get__(md)
+        elif place == "class":
+            monkeypatch.setattr(pkg.md.NVEIntegrator, "_forces", forces)
+        else:
+            md.__class__ = type("Own", (pkg.md.NVEIntegrator,), {"_forces": forces})
+    if way == "time step":
+        md.dt = torch.full((len(pos), 1), 0.5, dtype=torch.float64, device="cuda")
+        md.f = zeros.clone()
+    before, v = md.x.clone(), md.v.clone()
+    energy = md.step()
+    assert torch.equal(md.x, before + (0.5 if way == "time step" else 1.0) * v)
+    if way != "time step":
+        assert torch.equal(md.v, v) and torch.equal(md.f, zeros)
+    assert np.isfinite(energy)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("arch,copies", [("medium", (2, 1, 1)), ("medium", (4, 2, 2)), ("small", (4, 2, 1)), ("large", (2, 2, 1))])
 def test_parts_of_a_receiver_add_up(pkg, model_path, arch, copies):
