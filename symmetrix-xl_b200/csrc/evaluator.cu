@@ -2136,12 +2136,14 @@ void Evaluator::synchronize()
     SXB_CUDA(cudaStreamSynchronize(stream_));
 }
 
-void Evaluator::md_prepare()
+// The workspace is cleared on the caller's stream, where its first kernel follows.
+void Evaluator::md_prepare(cudaStream_t stream)
 {
     if (md_host_ != nullptr) return;
     md_workspace_.reserve(sizeof(MdWorkspace));
-    SXB_CUDA(cudaMemset(md_workspace_.ptr, 0, sizeof(MdWorkspace)));
+    SXB_CUDA(cudaMemsetAsync(md_workspace_.ptr, 0, sizeof(MdWorkspace), stream));
     SXB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&md_host_), sizeof(double), cudaHostAllocMapped));
+    *md_host_ = 0.0;
 }
 
 double Evaluator::md_advance(cudaStream_t stream, int n, double dt, double half, double* x, double* v, const double* f,
@@ -2149,7 +2151,7 @@ double Evaluator::md_advance(cudaStream_t stream, int n, double dt, double half,
 {
     if (n < 1) throw std::invalid_argument("A molecular-dynamics step needs at least one atom.");
     SXB_CUDA(cudaSetDevice(device_));
-    md_prepare();
+    md_prepare(stream);
     md_advance_kernel<<<std::min<long>(blocks_for(n, kMdThreads), kMdBlocks), kMdThreads, 0, stream>>>(
         n, dt, half, x, v, f, m, x_ref, reinterpret_cast<MdWorkspace*>(md_workspace_.ptr), md_host_);
     SXB_CUDA(cudaGetLastError());
@@ -2163,7 +2165,7 @@ double Evaluator::md_finish(cudaStream_t stream, int n, double half, double* v, 
     if (n < 1 || n != num_nodes_ || n != num_receivers_)
         throw std::invalid_argument("The molecular-dynamics step and the evaluated graph have different sizes.");
     SXB_CUDA(cudaSetDevice(device_));
-    md_prepare();
+    md_prepare(stream);
     md_finish_kernel<<<std::min<long>(blocks_for(n, kMdThreads), kMdBlocks), kMdThreads, 0, stream>>>(
         n, half, v, m, forces_out_.ptr, f_out, reinterpret_cast<MdWorkspace*>(md_workspace_.ptr), md_host_);
     SXB_CUDA(cudaGetLastError());

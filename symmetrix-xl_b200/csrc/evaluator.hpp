@@ -169,7 +169,7 @@ private:
     };
     HaloPlan halo_plan_;
     bool use_graphs_ = true;
-    void md_prepare();
+    void md_prepare(cudaStream_t stream);
     void finish_compute();
     void collect_compute();     // waits for the evaluation whose end has been recorded, and reads status and totals
     void settle();              // waits for an evaluation that was begun and never finished

@@ -612,6 +612,26 @@ def test_advance_kernel_is_the_tensor_expression(pkg, model_path, n):
         assert np.isnan(got) if bad else abs(got - want) <= 4 * 2.0 ** -53 * want          # three squares, two sums
 
 
+def test_first_step_of_an_evaluator_on_a_side_stream(pkg, model_path):
+    """The workspace of the step is cleared in the order of the caller's stream, which does not wait for the default one."""
+    import torch
+
+    n = 129
+    gen = torch.Generator("cuda").manual_seed(n)
+    x_ref, v, f = (torch.randn((n, 3), dtype=torch.float64, device="cuda", generator=gen) for _ in range(3))
+    m = torch.ones((n, 1), dtype=torch.float64, device="cuda")
+    x = x_ref + 0.01 * v
+    moved = ((x + 0.9 * (v + 0.37 * f) - x_ref) ** 2).sum(dim=1).max().item()
+    for _ in range(4):
+        ev = pkg.MACEB200(model_path("small"))
+        stream = torch.cuda.Stream()
+        state = [t.clone() for t in (x, v)]
+        stream.wait_stream(torch.cuda.current_stream())
+        got = ev.md_advance(stream.cuda_stream, n, 0.9, 0.37, state[0].data_ptr(), state[1].data_ptr(), f.data_ptr(), m.data_ptr(),
+                            x_ref.data_ptr())
+        assert abs(got - moved) <= 16 * 2.0 ** -53 * moved
+
+
 @pytest.mark.parametrize("drop", [0, 6, 7, 8])
 def test_step_kernels_match_the_tensor_step(pkg, model_path, drop):
     """The same trajectory from the two kernels and from tensor expressions, in the reproducible mode (equal forces for equal
