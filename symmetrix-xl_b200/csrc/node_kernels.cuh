@@ -5,6 +5,8 @@
 // 2516-2588, readout mace.cpp:2622-2657 with the MLP of multilayer_perceptron.cpp:34-80.
 #pragma once
 
+#include <cstddef>
+
 #include "common.cuh"
 #include "row_map.hpp"
 #include "generated/structures.h"
@@ -453,14 +455,28 @@ struct NodeReadoutArgs {
     double *node_energies, *energy_slots;
 };
 
+// Its vectors in shared memory, [channel][node] or [node][channel]; the partial sums are read in channel pairs.
+template <int kC>
+struct alignas(16) NodeReadoutShared {
+    static constexpr int G = 512 / kC, kParts = 256 / kC;
+    float m1[kC][G], xs[kC][G], adj_s[kC][G], h2[G][kC], sums[2][kParts][G][kC];
+    unsigned char types[G];
+};
+template <int kC>
+constexpr bool pairs_aligned()
+{
+    using S = NodeReadoutShared<kC>;
+    return alignof(S) % sizeof(float2) == 0 && offsetof(S, sums) % sizeof(float2) == 0 && kC % 2 == 0;
+}
+static_assert(pairs_aligned<32>() && pairs_aligned<64>() && pairs_aligned<128>(), "float2 reads of the partial sums");
+
 #define W(t) w[(t) * (kC / 2)]
 #define SXB_DEFINE_NODE_READOUT(NAME)                                                                               \
 template <int kC>                                                                                                   \
 __global__ void __launch_bounds__(256, 2) node_readout_kernel_##NAME(const NodeReadoutArgs a)                       \
 {                                                                                                                   \
     constexpr int NH = SXB_##NAME##_NUM_HIDDEN, NT = SXB_##NAME##_M1_NUM_TERMS, G = 512 / kC, kParts = 256 / kC;    \
-    __shared__ float m1[kC][G], xs[kC][G], adj_s[kC][G], h2[G][kC], sums[2][kParts][G][kC];                         \
-    __shared__ unsigned char types[G];                                                                              \
+    __shared__ NodeReadoutShared<kC> s;                                                                             \
     const int tid = threadIdx.x, base = blockIdx.x * G;                                                             \
     const int n = tid / (kC / 2), k = 2 * (tid % (kC / 2));             /* node and channel pair of the contractions */ \
     const bool valid = base + n < a.num_nodes;                                                                      \
@@ -476,10 +492,10 @@ __global__ void __launch_bounds__(256, 2) node_readout_kernel_##NAME(const NodeR
         SXB_##NAME##_M1_FORWARD_BODY                                                                                \
         const float2 value = *reinterpret_cast<const float2*>(&o[0]);                                               \
         const float2 scalar = *reinterpret_cast<const float2*>(a.M0 + node * NH * kC + k);                          \
-        m1[k][n] = value.x; m1[k + 1][n] = value.y;                                                                 \
-        xs[k][n] = scalar.x; xs[k + 1][n] = scalar.y;                                                               \
+        s.m1[k][n] = value.x; s.m1[k + 1][n] = value.y;                                                             \
+        s.xs[k][n] = scalar.x; s.xs[k + 1][n] = scalar.y;                                                           \
         if (valid) *reinterpret_cast<float2*>(a.M1 + node * kC + k) = value;                                        \
-        if (k == 0) types[n] = static_cast<unsigned char>(type);                                                    \
+        if (k == 0) s.types[n] = static_cast<unsigned char>(type);                                                  \
     }                                                                                                               \
     __syncthreads();                                                                                                \
     {                                                                                                               \
@@ -487,27 +503,27 @@ __global__ void __launch_bounds__(256, 2) node_readout_kernel_##NAME(const NodeR
         _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = 0.0f;                                                \
         _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {               \
             const float wv = a.W[c * kC + column];                                                                  \
-            _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(m1[c][r], wv, acc[r]);                      \
+            _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(s.m1[c][r], wv, acc[r]);                    \
         }                                                                                                           \
         for (int r0 = 0; r0 < G;) {   /* runs of equal elements: one in most blocks, receivers are sorted by element */ \
-            const int run = types[r0];                                                                              \
+            const int run = s.types[r0];                                                                            \
             int r1 = r0 + 1;                                                                                        \
-            while (r1 < G && types[r1] == run) ++r1;                                                                \
+            while (r1 < G && s.types[r1] == run) ++r1;                                                              \
             const float* const T = a.T + static_cast<size_t>(run) * kC * kC + column;                               \
             _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {           \
                 const float tv = T[c * kC];                                                                         \
-                _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(r >= r0 && r < r1 ? xs[c][r] : 0.0f, tv, acc[r]); \
+                _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(r >= r0 && r < r1 ? s.xs[c][r] : 0.0f, tv, acc[r]); \
             }                                                                                                       \
             r0 = r1;                                                                                                \
         }                                                                                                           \
-        _Pragma("unroll") for (int r = 0; r < G; ++r) sums[0][part][r][column] = acc[r];                            \
+        _Pragma("unroll") for (int r = 0; r < G; ++r) s.sums[0][part][r][column] = acc[r];                          \
     }                                                                                                               \
     __syncthreads();                                                                                                \
     for (int idx = tid; idx < G * kC; idx += 256) {                                                                 \
         const int r = idx / kC, c = idx % kC;                                                                       \
         float total = 0.0f;                                                                                         \
-        _Pragma("unroll") for (int p = 0; p < kParts; ++p) total += sums[0][p][r][c];                               \
-        h2[r][c] = total;                                                                                           \
+        _Pragma("unroll") for (int p = 0; p < kParts; ++p) total += s.sums[0][p][r][c];                             \
+        s.h2[r][c] = total;                                                                                         \
         if (base + r < a.num_nodes) a.H2[static_cast<size_t>(base + r) * kC + c] = total;                           \
     }                                                                                                               \
     __syncthreads();                                                                                                \
@@ -515,10 +531,10 @@ __global__ void __launch_bounds__(256, 2) node_readout_kernel_##NAME(const NodeR
         const int lane = tid & 31;                                                                                  \
         const size_t at = min(base + r, a.num_nodes - 1);                                                           \
         float g[kC / 32];                                                                                           \
-        const double e = a.atomic_energies[types[r]]                                                                \
-                         + readout16_node<kC / 32>(lane, a.act_scale, a.M0 + at * NH * kC, h2[r], a.q, a.W1, a.W2, g); \
+        const double e = a.atomic_energies[s.types[r]]                                                              \
+                         + readout16_node<kC / 32>(lane, a.act_scale, a.M0 + at * NH * kC, s.h2[r], a.q, a.W1, a.W2, g); \
         _Pragma("unroll") for (int c = 0; c < kC / 32; ++c) {                                                       \
-            adj_s[lane + 32 * c][r] = g[c];                                                                         \
+            s.adj_s[lane + 32 * c][r] = g[c];                                                                       \
             if (base + r < a.num_nodes) a.H2_adj[at * kC + lane + 32 * c] = g[c];                                   \
         }                                                                                                           \
         if (lane == 0 && base + r < a.num_nodes) {                                                                  \
@@ -532,32 +548,32 @@ __global__ void __launch_bounds__(256, 2) node_readout_kernel_##NAME(const NodeR
         _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = skip[r] = 0.0f;                                      \
         _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {               \
             const float wv = a.Wt[c * kC + column];                                                                 \
-            _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(adj_s[c][r], wv, acc[r]);                   \
+            _Pragma("unroll") for (int r = 0; r < G; ++r) acc[r] = fmaf(s.adj_s[c][r], wv, acc[r]);                 \
         }                                                                                                           \
         for (int r0 = 0; r0 < G;) {                                                                                 \
-            const int run = types[r0];                                                                              \
+            const int run = s.types[r0];                                                                            \
             int r1 = r0 + 1;                                                                                        \
-            while (r1 < G && types[r1] == run) ++r1;                                                                \
+            while (r1 < G && s.types[r1] == run) ++r1;                                                              \
             const float* const T = a.Tt + static_cast<size_t>(run) * kC * kC + column;                              \
             _Pragma("unroll 8") for (int c = part * (kC / kParts); c < (part + 1) * (kC / kParts); ++c) {           \
                 const float tv = T[c * kC];                                                                         \
-                _Pragma("unroll") for (int r = 0; r < G; ++r) skip[r] = fmaf(r >= r0 && r < r1 ? adj_s[c][r] : 0.0f, tv, skip[r]); \
+                _Pragma("unroll") for (int r = 0; r < G; ++r) skip[r] = fmaf(r >= r0 && r < r1 ? s.adj_s[c][r] : 0.0f, tv, skip[r]); \
             }                                                                                                       \
             r0 = r1;                                                                                                \
         }                                                                                                           \
-        _Pragma("unroll") for (int r = 0; r < G; ++r) { sums[0][part][r][column] = acc[r]; sums[1][part][r][column] = skip[r]; } \
+        _Pragma("unroll") for (int r = 0; r < G; ++r) { s.sums[0][part][r][column] = acc[r]; s.sums[1][part][r][column] = skip[r]; } \
     }                                                                                                               \
     __syncthreads();                                                                                                \
     {                                                                                                               \
         f2 x[16], g[16], adj[1];                                                                                    \
         float2 m1_adj = make_float2(0.0f, 0.0f), m0_adj = *reinterpret_cast<const float2*>(a.q + k);                \
         _Pragma("unroll") for (int p = 0; p < kParts; ++p) {                                                        \
-            const float2 u = *reinterpret_cast<const float2*>(&sums[0][p][n][k]), v = *reinterpret_cast<const float2*>(&sums[1][p][n][k]); \
+            const float2 u = *reinterpret_cast<const float2*>(&s.sums[0][p][n][k]), v = *reinterpret_cast<const float2*>(&s.sums[1][p][n][k]); \
             m1_adj.x += u.x; m1_adj.y += u.y; m0_adj.x += v.x; m0_adj.y += v.y;                                     \
         }                                                                                                           \
         if (valid) {                                                                                                \
             *reinterpret_cast<float2*>(a.M1_adj + node * kC + k) = m1_adj;                                          \
-            *reinterpret_cast<float2*>(a.M0_adj + node * a.M0_adj_stride + k) = m0_adj;                                    \
+            *reinterpret_cast<float2*>(a.M0_adj + node * a.M0_adj_stride + k) = m0_adj;                             \
         }                                                                                                           \
         _Pragma("unroll") for (int r = 0; r < 16; ++r) { x[r] = *reinterpret_cast<const f2*>(in + r * kC); g[r] = 0ull; } \
         adj[0] = *reinterpret_cast<const f2*>(&m1_adj);                                                             \
