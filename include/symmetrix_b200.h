@@ -376,6 +376,11 @@ int sxb_peer_destroy(sxb_peer_exchange_t* exchange);
  * invalidates the prepared graph; prepare again afterwards. */
 int sxb_set_tile_size(sxb_evaluator* evaluator, int32_t receivers_per_tile);
 
+/* Bound in bytes on one part of that workspace (2^30 to begin with): the sums over the radial functions, 4 KB per receiver and
+ * element type, which layer 0 of larger graphs makes for a slice of the receivers at a time (at least one).  The setting
+ * invalidates the prepared graph; prepare again afterwards. */
+int sxb_set_moment_bytes(sxb_evaluator* evaluator, int64_t bytes);
+
 /* Reproducible mode (off by default).  The default kernels add the source adjoint H1_adj and the forces
  * on source atoms with atomics, whose order -- and so the last bits of the results -- varies between
  * runs.  With this mode on, the kernels leave one record per edge and fixed-order passes sum them over a

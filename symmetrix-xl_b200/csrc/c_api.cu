@@ -611,6 +611,11 @@ int sxb_set_tile_size(sxb_evaluator* ev, int32_t receivers_per_tile)
     return guarded([&] { require(ev, "evaluator"); ev->impl.set_tile_size(receivers_per_tile); });
 }
 
+int sxb_set_moment_bytes(sxb_evaluator* ev, int64_t bytes)
+{
+    return guarded([&] { require(ev, "evaluator"); ev->impl.set_moment_bytes(static_cast<long>(bytes)); });
+}
+
 int sxb_set_stream(sxb_evaluator* ev, void* stream)
 {
     return guarded([&] { require(ev, "evaluator"); ev->impl.set_stream(static_cast<cudaStream_t>(stream)); });

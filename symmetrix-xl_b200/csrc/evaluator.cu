@@ -2257,6 +2257,15 @@ void Evaluator::set_tile_size(int receivers_per_tile)
     mirror_valid_ = false;
 }
 
+void Evaluator::set_moment_bytes(long bytes)
+{
+    if (bytes < 1) throw std::invalid_argument("The bound on the layer-0 sums must be positive.");
+    moment_bytes_ = bytes;
+    generation_ += 1;      // as for the tile size
+    have_results_ = false;
+    mirror_valid_ = false;
+}
+
 long Evaluator::get_stage(const std::string& name, double* out, long capacity)
 {
     require_results();

@@ -86,6 +86,9 @@ public:
     // Tiled streaming: receivers are processed in tiles of this many with one reusable workspace
     // (0 = one tile holding every receiver).  Takes effect at the next graph preparation.
     void set_tile_size(int receivers_per_tile);
+    // Bound on the sums over the radial functions, which layer 0 makes for a slice of the receivers at a time (at least one).
+    // Takes effect at the next graph preparation.
+    void set_moment_bytes(long bytes);
     // Reproducible mode: every accumulation in a fixed order (no atomics); takes effect at the next graph preparation.
     void set_deterministic(bool enabled);
     int tile_capacity() const;
@@ -121,12 +124,12 @@ private:
     void prepare_active_types(const std::vector<int>& node_types, int num_receivers);
     void install_graph(int num_receivers, int num_nodes, const std::vector<int>& node_types, long num_edges, bool has_shifts);
     ActiveEdges active_edges() const;
-    // receivers whose sums over the radial functions are kept at a time, 1 GB of them: 135,000 receivers, three types, in slices of 96 MB
-    // (which stay in L2) / 0.8 GB: layer 0 7.9 / 6.8 ms; 20,000 with ten types 2.4 / 1.8 ms
+    // receivers whose sums over the radial functions are kept at a time, 1 GB of them unless the caller asks for less: 135,000
+    // receivers, three types, in slices of 96 MB (which stay in L2) / 0.8 GB: layer 0 7.9 / 6.8 ms; 20,000 with ten types 2.4 / 1.8 ms
     int moment_receivers() const
     {
-        const long fit = (1l << 30) / (16l * 64 * static_cast<long>(sizeof(float)) * static_cast<long>(std::max<std::size_t>(1, type_tables_.types.size())));
-        return static_cast<int>(std::min<long>(tile_capacity(), std::max(1024l, fit)));
+        const long fit = moment_bytes_ / (16l * 64 * static_cast<long>(sizeof(float)) * static_cast<long>(std::max<std::size_t>(1, type_tables_.types.size())));
+        return static_cast<int>(std::min<long>(tile_capacity(), std::max(1l, fit)));
     }
     int edge_types() const { return basis_layer0_ ? static_cast<int>(type_tables_.types.size()) : 1; }   // types a receiver's edges are grouped by
     // M1 to readout and back in one kernel (node_readout_kernel_*): the model has that form, and the graph is so small that short
@@ -232,6 +235,7 @@ private:
     int num_nodes_ = 0, num_receivers_ = 0;
     int phase_ = 0;
     int tile_size_ = 0;
+    long moment_bytes_ = 1l << 30;
     bool owns_stream_ = true;
     bool pending_finish_ = false;
     long num_edges_ = 0;

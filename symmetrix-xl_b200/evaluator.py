@@ -120,6 +120,7 @@ SIGNATURES = {
     "sxb_peer_destroy": (ctypes.c_int, [_P]),
     "sxb_peer_set_wait_limit": (ctypes.c_int, [_P, ctypes.c_double]),
     "sxb_set_tile_size": (ctypes.c_int, [_P, ctypes.c_int32]),
+    "sxb_set_moment_bytes": (ctypes.c_int, [_P, ctypes.c_int64]),
     "sxb_set_deterministic": (ctypes.c_int, [_P, ctypes.c_int32]),
     "sxb_set_profiling": (ctypes.c_int, [_P, ctypes.c_int32]),
     "sxb_profile_entry": (ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_char_p, ctypes.c_int32, ctypes.POINTER(ctypes.c_float),
@@ -477,6 +478,11 @@ class MACEB200:
         """Tiled streaming with a reusable workspace (0 = off); prepare the graph again afterwards."""
         _check(self._lib.sxb_set_tile_size(self._h, int(receivers_per_tile)))
         self._tile_size = int(receivers_per_tile)
+
+    def set_moment_bytes(self, nbytes: int):
+        """Bound on the sums over the radial functions that layer 0 of larger graphs keeps at a time (1 GB to begin
+        with); prepare the graph again afterwards."""
+        _check(self._lib.sxb_set_moment_bytes(self._h, int(nbytes)))
 
     def set_stream(self, stream_ptr):
         _check(self._lib.sxb_set_stream(self._h, ctypes.c_void_p(stream_ptr)))

@@ -160,3 +160,30 @@ def test_forward_tensors_repeat_bit_for_bit(pkg, model_path):
             first = stages
         for name, tensor in stages.items():
             assert np.array_equal(tensor, first[name]), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,options,tile,receivers", [(128, {}, 0, 193), (128, {}, 0, 1), (128, {}, 320, 100),
+                                                             (64, dict(a0_scaled=True, a1_scaled=True, agnesi=True), 0, 211),
+                                                             (64, dict(a0_scaled=True), 450, 499)])
+def test_slices_of_the_sums_over_the_functions(pkg, model_path, channels, options, tile, receivers):
+    """Layer 0 in slices that end inside an element's run of receivers (750 atoms: 450, 150 and 150 of a type), of one receiver, smaller
+    and larger than a tile, against all at once.  A receiver's sums do not depend on the slice: A0 has the same bits.  Of the
+    gradient a slice decides how many warps take a run, and the order of the atomic sums has no fixed order in the first place: the
+    bounds of the tiled evaluation."""
+    path = model_path("medium", channels=channels, **options)
+    pos, cell, types = pkg.modelgen.srtio3((6, 5, 5), 0.05, 7)
+    whole, sliced = pkg.Calculator(path, skin=0.5), pkg.Calculator(path, skin=0.5)
+    with pytest.raises(ValueError):
+        sliced.evaluator.set_moment_bytes(0)
+    sliced.evaluator.set_moment_bytes(receivers * 3 * 16 * 64 * 4)
+    sliced.evaluator.set_tile_size(tile)
+    a = whole.calculate(pos, cell, types)
+    b = sliced.calculate(pos, cell, types)
+    used = [c.evaluator.execution_plan_report["candidates"][0]["estimated_bytes"] for c in (whole, sliced)]
+    assert used[0] - used[1] >= (len(pos) - receivers) * 3 * 16 * 64 * 4
+    if tile == 0:
+        assert np.array_equal(sliced.evaluator.stage("A0"), whole.evaluator.stage("A0"))
+    assert np.abs(a["energies"] - b["energies"]).max() <= 1e-6
+    assert np.abs(a["forces"] - b["forces"]).max() <= 1e-5
+    assert np.abs(a["stress"] - b["stress"]).max() <= 1e-8
