@@ -9,7 +9,7 @@
 // backwards, Badj = A0_adj G^T, and f_ij = -sum_(lm, h) Badj_i[type_j][lm][h] (rhat phi_h' Y_lm + phi_h grad Y_lm).
 // Reference statements of the same math: libsymmetrix/source/mace.cpp:1356-1403 and 1486-1559, compact_radial.cpp:291-366.
 //
-// 0e+1o, 5,000 atoms, three types, 128 channels, folded table / this (edges + linear): sums 172 / 43 + 42, gradient 243 / 93 + 47 us.
+// 0e+1o, 5,000 atoms, three types, 128 channels, folded table / this (edges + linear): sums 172 / 42 + 43, gradient 243 / 105 + 48 us.
 #pragma once
 
 #include "edge_kernels_warp.cuh"
@@ -109,12 +109,14 @@ l0_moments_kernel(int node0, int types, const int* __restrict__ first, const Edg
 
 // ---------------------------------------------------------------------------------------------
 // Gradient.  For the edges of a run, F[e][lm] = sum_h phi_h(r_e) Badj[lm][h] and D[e][lm] with the slopes phi_h' are two small
-// matrix products with the same right-hand side, 16 edges x 64 functions x 16 components: mma.sync, three TF32 passes, the small
-// products in accumulators of their own.  (tcgen05 wants 128 rows and its operands written to shared or tensor memory first; here
-// every lane computes the functions it feeds to the instruction, and Badj stays in its registers for the whole run.)  The FP32
-// form, a warp carrying one edge and reducing over its lanes, took 172 instructions per edge and 130 us (5,000 atoms).  A warp walks
-// all runs of a receiver (few receivers: one run or part of one): a warp's chain of dependent loads, first the edges, then their
-// coefficient rows, is what it waits for, 12 warps per SM; as warps of one run each 113 us.
+// matrix products with the same right-hand side, 16 edges x 64 functions x 16 components: mma.sync in FP64, where every product of
+// two floats is exact, the sums are rounded to float once.  (tcgen05 wants 128 rows and its operands written to shared or tensor
+// memory first; here every lane computes the functions it feeds to the instruction, and Badj stays in its registers for the whole
+// run.)  Three TF32 passes take 31 / 95 us at 1,080 / 5,000 receivers, this 31 / 105, but the TF32 unit truncates whenever it adds:
+// sums of 64 products of random sign were off by 1.1e-7 (2-norm) and pulled towards zero by 5e-8, in FP32 by 7e-8 and nothing.
+// The FP32 form, a warp carrying one edge and reducing over its lanes, took 172 instructions per edge and 130 us (5,000
+// receivers).  A warp walks all runs of a receiver (few receivers: one run or part of one): a warp's chain of dependent loads,
+// first the edges, then their coefficient rows, is what it waits for, 12 warps per SM; as warps of one run each 113 us (TF32).
 //
 // Fragments: lane = 4 g + t.  Rows g and g + 8 are edges; column t (t + 4) of step s is function 16 t + 2 s (16 t + 2 s + 1),
 // so that a lane reads 16 consecutive adjoints of a component, and the table lists the functions in the order of the steps.
@@ -123,18 +125,11 @@ struct alignas(16) MomentGradChunk {
     float2 point[32];     // x = offset inside the spline interval, y = table row (int)
 };
 
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1)
+__device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1)
 {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// x = hi + lo: hi the nearest TF32 value, lo what the instruction reads the leading bits of (of either sign, so without bias)
-__device__ __forceinline__ void tf32_split(float x, unsigned& hi, unsigned& lo)
-{
-    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(x - __uint_as_float(hi));
+    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
 }
 
 __global__ void __launch_bounds__(32, 12)
@@ -160,17 +155,17 @@ l0_moments_reverse_kernel(int node0, int types, const int* __restrict__ first, c
             run.y = min(run.y, begin + 16 * (steps * (part + 1) / parts));
         }
         if (run.x >= run.y) continue;
-        unsigned bhi[2][16], blo[2][16];      // [components g, g + 8][function 16 t + j]
+        double b[2][16];      // [components g, g + 8][function 16 t + j]
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             const float4* in = reinterpret_cast<const float4*>(Badj + (static_cast<size_t>(local) * 16 + 8 * n + g) * (kBasis * types) + type * kBasis + 16 * t);
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 const float4 w = in[m];
-                tf32_split(w.x * scale, bhi[n][4 * m], blo[n][4 * m]);
-                tf32_split(w.y * scale, bhi[n][4 * m + 1], blo[n][4 * m + 1]);
-                tf32_split(w.z * scale, bhi[n][4 * m + 2], blo[n][4 * m + 2]);
-                tf32_split(w.w * scale, bhi[n][4 * m + 3], blo[n][4 * m + 3]);
+                b[n][4 * m] = w.x * scale;
+                b[n][4 * m + 1] = w.y * scale;
+                b[n][4 * m + 2] = w.z * scale;
+                b[n][4 * m + 3] = w.w * scale;
             }
         }
         for (int chunk = run.x; chunk < run.y; chunk += 32) {
@@ -200,36 +195,22 @@ l0_moments_reverse_kernel(int node0, int types, const int* __restrict__ first, c
                     xxx[r] = xx[r] * x[r];
                     xx3[r] = 3.0f * xx[r];
                 }
-                float F[2][4] = {}, Fsmall[2][4] = {}, D[2][4] = {}, Dsmall[2][4] = {};   // [components 0-7, 8-15]
+                double F[2][4] = {}, D[2][4] = {};   // [components 0-7, 8-15]
 #pragma unroll
-                for (int pair = 0; pair < 4; ++pair) {
-                    // the instruction truncates when it adds: the large products of two steps at a time, their sums rounded to nearest
-                    float f[2][4] = {}, d[2][4] = {};
+                for (int step = 0; step < 8; ++step) {
+                    double value[4], slope[4];
 #pragma unroll
-                    for (int step = 2 * pair; step < 2 * pair + 2; ++step) {
-                        unsigned vhi[4], vlo[4], dhi[4], dlo[4];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const int r = q & 1;
-                            const float4 w = c[r][4 * (2 * step + (q >> 1))];
-                            tf32_split(cubic(w.x, w.y, w.z, w.w, x[r], xx[r], xxx[r]), vhi[q], vlo[q]);
-                            tf32_split(cubic_derivative(w.y, w.z, w.w, 2.0f * x[r], xx3[r]), dhi[q], dlo[q]);
-                        }
-#pragma unroll
-                        for (int n = 0; n < 2; ++n) {
-                            const unsigned b0 = bhi[n][2 * step], b1 = bhi[n][2 * step + 1];
-                            mma_tf32(Fsmall[n], vlo, b0, b1);
-                            mma_tf32(Dsmall[n], dlo, b0, b1);
-                            mma_tf32(f[n], vhi, b0, b1);
-                            mma_tf32(d[n], dhi, b0, b1);
-                            mma_tf32(Fsmall[n], vhi, blo[n][2 * step], blo[n][2 * step + 1]);
-                            mma_tf32(Dsmall[n], dhi, blo[n][2 * step], blo[n][2 * step + 1]);
-                        }
+                    for (int q = 0; q < 4; ++q) {
+                        const int r = q & 1;
+                        const float4 w = c[r][4 * (2 * step + (q >> 1))];
+                        value[q] = cubic(w.x, w.y, w.z, w.w, x[r], xx[r], xxx[r]);
+                        slope[q] = cubic_derivative(w.y, w.z, w.w, 2.0f * x[r], xx3[r]);
                     }
 #pragma unroll
-                    for (int n = 0; n < 2; ++n)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) { F[n][q] += f[n][q]; D[n][q] += d[n][q]; }
+                    for (int n = 0; n < 2; ++n) {
+                        mma_f64(F[n], value, b[n][2 * step], b[n][2 * step + 1]);
+                        mma_f64(D[n], slope, b[n][2 * step], b[n][2 * step + 1]);
+                    }
                 }
                 // a lane holds components 2 t, 2 t + 1 (+ 8) of its two edges
 #pragma unroll
@@ -238,8 +219,8 @@ l0_moments_reverse_kernel(int node0, int types, const int* __restrict__ first, c
 #pragma unroll
                     for (int n = 0; n < 2; ++n) {
                         float* o = s.fd[row[r]] + 8 * n + 2 * t;
-                        *reinterpret_cast<float2*>(o) = make_float2(F[n][2 * r] + Fsmall[n][2 * r], F[n][2 * r + 1] + Fsmall[n][2 * r + 1]);
-                        *reinterpret_cast<float2*>(o + 16) = make_float2(D[n][2 * r] + Dsmall[n][2 * r], D[n][2 * r + 1] + Dsmall[n][2 * r + 1]);
+                        *reinterpret_cast<float2*>(o) = make_float2(F[n][2 * r], F[n][2 * r + 1]);
+                        *reinterpret_cast<float2*>(o + 16) = make_float2(D[n][2 * r], D[n][2 * r + 1]);
                     }
                 }
             }

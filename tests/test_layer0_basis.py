@@ -187,3 +187,45 @@ def test_slices_of_the_sums_over_the_functions(pkg, model_path, channels, option
     assert np.abs(a["energies"] - b["energies"]).max() <= 1e-6
     assert np.abs(a["forces"] - b["forces"]).max() <= 1e-5
     assert np.abs(a["stress"] - b["stress"]).max() <= 1e-8
+
+
+def layer0_gradient_error(pkg, path, cells):
+    """Edge forces of a model with one interaction (nothing but layer 0) against float64 from the same adjoints of A0: the error's 2-norm
+    and its part along the forces, both over the 2-norm of the forces."""
+    from conftest import csr_from_positions
+    from oracle import mace_numpy
+
+    pos, cell, types = pkg.modelgen.srtio3(cells, 0.05, 11)
+    first, src, shifts, xyz = csr_from_positions(pos, cell, 6.0)
+    ev = pkg.MACEB200(path)
+    ev.compute_node_energies_forces(len(pos), types, np.diff(first), src, types[src], xyz)
+    oracle = mace_numpy.NumpyMACE(str(path))
+    C, l_of_lm = oracle.C, np.array([0] + [1] * 3 + [2] * 5 + [3] * 7)
+    adj = ev.stage("A0_adj").reshape(len(pos), 16, C)
+    mixed = np.empty(adj.shape)                   # adjoint of the sums before the receiver's mixing matrix (mace.cpp:1486-1503)
+    for a in range(oracle.A):
+        for lm in range(16):
+            mixed[types == a, lm] = adj[types == a, lm] @ oracle.WA0[a, l_of_lm[lm]].T
+    recv = np.repeat(np.arange(len(pos)), np.diff(first))
+    want = np.empty((len(src), 3))
+    for e0 in range(0, len(src), 2000):
+        e = slice(e0, e0 + 2000)
+        r = np.linalg.norm(xyz[e], axis=1)
+        Y, grad = mace_numpy.harmonics(3, xyz[e])
+        R, dR = (v.reshape(-1, 4, C)[:, l_of_lm] for v in oracle._radial("R0", types[recv[e]], types[src[e]], r))
+        weighted = mixed[recv[e]] * oracle.H0[types[src[e]]][:, None]
+        along = ((weighted * dR).sum(axis=2) * Y).sum(axis=1)
+        want[e] = -along[:, None] * xyz[e] / r[:, None] - np.einsum("em,edm->ed", (weighted * R).sum(axis=2), grad)
+    error = ev.node_forces.reshape(-1, 3) - want
+    return np.sqrt((error ** 2).sum() / (want ** 2).sum()), (error * want).sum() / (want ** 2).sum()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,cells", [(128, (6, 4, 4)), (64, (6, 6, 4))])
+def test_gradient_on_the_functions_is_not_pulled_towards_zero(pkg, model_path, channels, cells):
+    """A unit that truncates where FP32 rounds pulls each sum by 4e-8 an addition; errors that are rounded to nearest have no direction
+    (some 1e5 components of 4e-7: 1e-9, and a few 1e-8 for the coefficients of the tables, which are the same in every edge).  480 and
+    720 receivers are on the functions; without truncation in the products with the functions the linear before them is left."""
+    error, pull = layer0_gradient_error(pkg, model_path("medium", seed=1, channels=channels, single_layer=True), cells)
+    assert error <= 6e-7
+    assert abs(pull) <= 1.4e-7
