@@ -999,6 +999,7 @@ void Evaluator::launch_tc(const std::vector<TcCall>& calls)
                 p.map_c = make_activation_map(c.C, c.c_rows, c.first_node, c.num_nodes, N, p.nodes_per_tile);
                 p.bias = c.accumulate ? nullptr : c.bias;
                 p.accumulate = c.accumulate ? 1 : 0;
+                p.chunk_scale = c.unbiased ? kT3Truncated : 1.0f;
                 p.m_tiles = (c.num_nodes + p.nodes_per_tile - 1) / p.nodes_per_tile;
                 p.tile_begin = tiles;
                 tiles += p.m_tiles * p.n_tiles;
@@ -1114,7 +1115,9 @@ void Evaluator::run_pipeline(int phases)
             for (int l = 0; l <= model_.l_max; ++l) {
                 const RowMap moment_rows{16 * width, width, l * l * width, 2 * l + 1}, node_rows{16L * C, C, static_cast<long>(l) * l * C, 2 * l + 1};
                 const SplitWeight* w = &s_a0_[a * (model_.l_max + 1) + l];
-                if (reverse) calls.push_back({nodes, node_rows, w, true, moments, moment_rows, 0, count, false, nullptr});
+                // the sums were FP32 where this adjoint is now a linear of its own: its truncation is put back.  A0 is as near to float64
+                // as from the folded table either way (pull -4e-8, +5e-8 from the table, +8e-8 with the correction).
+                if (reverse) calls.push_back({nodes, node_rows, w, true, moments, moment_rows, 0, count, false, nullptr, true});
                 else calls.push_back({moments, moment_rows, w, false, nodes, node_rows, 0, count, false, nullptr});
             }
         });

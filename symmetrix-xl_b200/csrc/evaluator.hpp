@@ -224,6 +224,7 @@ private:
     struct TcCall {
         const float* A; RowMap a_rows; const SplitWeight* w; bool reverse; float* C; RowMap c_rows;
         int first_node, num_nodes; bool accumulate; const float* bias;
+        bool unbiased = false;    // kT3Truncated
     };
     void launch_tc(const std::vector<TcCall>& calls);
     DeviceBuffer<double> atomic_energies_;

@@ -13,11 +13,12 @@
 //   * the tensor core truncates whenever it adds to its accumulator, so a chain of K / 8 x 3 additions ends low by about one
 //     part in 10^7 for every six of them (K = 192: 2e-6 against 3e-7 for an FP32 sum).  Each chunk of 32 K therefore gets an
 //     accumulator of its own (two of 128 columns in tensor memory), its eight small products before its four large ones, and
-//     eight warps add the chunks up in registers, rounded to nearest: 1.5e-7;
+//     eight warps add the chunks up in registers, rounded to nearest: 1.5e-7; where a launch asks for it with what the truncations
+//     take on average put back (kT3Truncated);
 //   * the same warps leave tile i in shared memory, from where the TMA engine stores it, or adds it to the output, while they
 //     sum up tile i + 1.
 // A row tile holds floor(128 / components) whole nodes (128, 126, 125 or 126 rows); the remaining
-// accumulator lanes are never stored.  A column tile is 128, 64 or 32 columns wide, as the launch chooses.
+// accumulator lanes are never stored.  A column tile is 128, 96, 64 or 32 columns wide, as the launch chooses.
 // Thread roles: warps 0-3 split, warps 4-11 sums and epilogue, warp 12 lane 0 tcgen05.mma issue (warp 12 also
 // owns the tensor-memory allocation), warp 13 lane 0 weight TMA, warp 14 lane 0 activation TMA.  The
 // issuing thread is the narrow point of such a pipeline (every mbarrier or tcgen05 instruction costs
@@ -47,6 +48,12 @@ constexpr int kT3Columns = 512;               // allocated: accumulators, and 64
 static_assert(kT3SplitColumn + 64 * kT3SplitStages <= kT3Columns, "tensor memory");
 static_assert(kT3AStages <= kT3Ring && kT3Stages <= kT3Ring && kT3SplitStages <= kT3Ring, "rings of barriers");
 
+// What the truncations of a chunk take from its sum, on average, put back.  Only the four large products count; after each the unit
+// drops half a last place of the partial sum s_j, 0.72 x 2^-24 of it over mantissas spread evenly in their logarithm, and the s_j
+// make up (1 + 2 + 3 + 4) / 4 of the sum, whether the terms have one sign or random ones: 1.07e-7, nearly the last place of 1.
+// (Sums of 128 products emulated in double: 2-norm of the error 1.3e-7 -> 0.8e-7, pull -1.07e-7 -> +0.15e-7; FP32 in a chain 2.0e-7.)
+constexpr float kT3Truncated = 1.0f + 1.1920929e-7f;
+
 struct alignas(64) Tc3Problem {
     CUtensorMap map_a;       // activations [node][component][K], box [nodes_per_tile][components][32]
     CUtensorMap map_hi;      // Bt_hi [N][K], box [n_tile][32]
@@ -55,8 +62,9 @@ struct alignas(64) Tc3Problem {
     const float* bias;       // optional [N], added when not accumulating
     int K;                   // K % 32 == 0
     int accumulate;
+    float chunk_scale;       // 1, or kT3Truncated
     int rows_per_tile, nodes_per_tile;
-    int n_tile, n_tiles;     // 32, 64 or 128; N % n_tile == 0
+    int n_tile, n_tiles;     // 32, 64, 96 or 128; N % n_tile == 0
     int m_tiles;
     int tile_begin;          // first work item of this problem (items are m-major: m_tile * n_tiles + n)
 };
@@ -262,7 +270,7 @@ __global__ void __launch_bounds__(kT3Threads, 1) tc_gemm_tma_kernel(const __grid
 #pragma unroll
                     for (int q = 0; q < 32; ++q) asm volatile("" : "+r"(v[q]));   // no use of a register before the wait
 #pragma unroll
-                    for (int q = 0; q < 32; ++q) acc[32 * g + q] += __uint_as_float(v[q]);
+                    for (int q = 0; q < 32; ++q) acc[32 * g + q] = fmaf(__uint_as_float(v[q]), P.chunk_scale, acc[32 * g + q]);
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 mbar_arrive(&acc_empty[b]);

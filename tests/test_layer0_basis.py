@@ -221,11 +221,12 @@ def layer0_gradient_error(pkg, path, cells):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("channels,cells", [(128, (6, 4, 4)), (64, (6, 6, 4))])
-def test_gradient_on_the_functions_is_not_pulled_towards_zero(pkg, model_path, channels, cells):
-    """A unit that truncates where FP32 rounds pulls each sum by 4e-8 an addition; errors that are rounded to nearest have no direction
-    (some 1e5 components of 4e-7: 1e-9, and a few 1e-8 for the coefficients of the tables, which are the same in every edge).  480 and
-    720 receivers are on the functions; without truncation in the products with the functions the linear before them is left."""
-    error, pull = layer0_gradient_error(pkg, model_path("medium", seed=1, channels=channels, single_layer=True), cells)
+@pytest.mark.parametrize("channels,seed,cells,bound", [(128, 1, (6, 4, 4), 4e-8), (64, 2, (6, 6, 4), 1.2e-7)])
+def test_gradient_on_the_functions_is_not_pulled_towards_zero(pkg, model_path, channels, seed, cells, bound):
+    """A unit that truncates where FP32 rounds pulls each sum by 4e-8 an addition, in products with the functions and in the linear
+    before them 1.7e-7 and 2.3e-7 here; errors that are rounded to nearest have no direction (some 1e5 components of 4e-7: 1e-9).
+    Bounds: half a truncation for what the average in the linear leaves, and at 64 channels what the rounded coefficients of this model
+    do (-1e-7 on the folded table too).  480 and 720 receivers are on the functions."""
+    error, pull = layer0_gradient_error(pkg, model_path("medium", seed=seed, channels=channels, single_layer=True), cells)
     assert error <= 6e-7
-    assert abs(pull) <= 1.4e-7
+    assert abs(pull) <= bound
