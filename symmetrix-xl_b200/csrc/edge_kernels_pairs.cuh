@@ -5,8 +5,11 @@
 // channel pairs, in the packed instructions of sm_100a, they don't fit the registers; in shared memory (two edges per read) they
 // took a third of the wavefronts of a kernel that the shared-memory pipe bounded.  Tensor memory is read by a path of its own:
 // every warp reaches the 32 lanes of its quarter, so the rows of its 64 channels lie there as pairs, two columns a row, shared by the
-// warps of the same quarter, and come in batches of eight while the batch before is used.  Without the rows the registers suffice
-// for 16 warps per SM at one edge each (0e+1o; 12 warps for 0e+1o+2e).  Rows in registers one channel a thread / pairs with rows in
+// warps of the same quarter, and come in batches of eight while the batch before is used.  The first batch of an edge is asked for
+// along with its source row, not by the edge before: registers that a load has yet to fill are not carried round a loop, where a
+// copy of them may be placed (5,000 atoms, asked for by the edge before / this: 128 channels 701 / 695 us, 64 channels 388 / 392,
+// 0e+1o+2e 1,549 / 1,555).  Without the rows the registers suffice for 16 warps per SM at one edge each (0e+1o; 12 warps for
+// 0e+1o+2e).  Rows in registers one channel a thread / pairs with rows in
 // registers / rows in shared memory / this: 0e+1o, 5,000 atoms 1.00 / 0.94 / 0.90 / 0.70 ms; 0e+1o+2e, 20,000 atoms 10.5 / - / 8.9 / 6.6 ms.
 // Now FMA pipe 56 %, data pipe of L1 59 %, issue 52 %.  Reading 16 columns takes a warp 83 cycles with 16 warps on it, 390 bytes a
 // cycle and SM.  Other shapes measured: 16 channels x 4 edges a warp +13 % (every 32 bytes of another line cost a wavefront), L1
@@ -271,13 +274,17 @@ __device__ __forceinline__ void store_row_batch(unsigned taddr, const f2 (&rows)
           "r"(raw[9]), "r"(raw[10]), "r"(raw[11]), "r"(raw[12]), "r"(raw[13]), "r"(raw[14]), "r"(raw[15])
         : "memory");
 }
-// The batch asked for has arrived: its rows as channel pairs.  The moves are volatile like the wait, so that none is placed
-// before it; they cost nothing, the pairs being neighbouring registers already.
-__device__ __forceinline__ void take_row_batch(const unsigned (&raw)[2 * kRowBatch], f2 (&rows)[kRowBatch])
+// The batch asked for has arrived: its rows as channel pairs.  The registers go through the wait, so that whatever reads them
+// depends on it.
+__device__ __forceinline__ void take_row_batch(unsigned (&raw)[2 * kRowBatch], f2 (&rows)[kRowBatch])
 {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    asm volatile(
+        "tcgen05.wait::ld.sync.aligned;"
+        : "+r"(raw[0]), "+r"(raw[1]), "+r"(raw[2]), "+r"(raw[3]), "+r"(raw[4]), "+r"(raw[5]), "+r"(raw[6]), "+r"(raw[7]), "+r"(raw[8]),
+          "+r"(raw[9]), "+r"(raw[10]), "+r"(raw[11]), "+r"(raw[12]), "+r"(raw[13]), "+r"(raw[14]), "+r"(raw[15])
+        :: "memory");
 #pragma unroll
-    for (int q = 0; q < kRowBatch; ++q) asm volatile("mov.b64 %0, {%1, %2};" : "=l"(rows[q]) : "r"(raw[2 * q]), "r"(raw[2 * q + 1]));
+    for (int q = 0; q < kRowBatch; ++q) asm("mov.b64 %0, {%1, %2};" : "=l"(rows[q]) : "r"(raw[2 * q]), "r"(raw[2 * q + 1]));
 }
 
 #define RADIAL(p)                                                                                                   \
@@ -290,10 +297,11 @@ __device__ __forceinline__ void take_row_batch(const unsigned (&raw)[2 * kRowBat
 #define TERM(slot, term, lme) v[slot] = f2_mul(f2_pack(cgc.cg[term], cgc.cg[term]), DPHI(lme));
 #define TERM_ADD(slot, term, lme) v[slot] = f2_fma(f2_pack(cgc.cg[term], cgc.cg[term]), DPHI(lme), v[slot]);
 #define STORE(batch) store_row_batch(row_column + 2 * kRowBatch * (batch), v);
-/* takes batch b and asks for the next one; the last batch of an edge asks for the first one of the next edge */
+/* takes batch b and asks for the next one; what has been asked for is taken before the edge ends, so that no outstanding load is
+   carried round the loop */
 #define ROWS(b)                                                                                                     \
     take_row_batch(raw, rows);                                                                                      \
-    load_row_batch(row_column + 2 * kRowBatch * (((b) + 1) % kBatches), raw);
+    if constexpr ((b) + 1 < kBatches) load_row_batch(row_column + 2 * kRowBatch * ((b) + 1), raw);
 
 // Shared memory of a block with `channels` channels: edge state and channel sums; totals and the kilobyte that the system keeps.
 constexpr std::size_t pair_dynamic_bytes(int channels)
@@ -368,8 +376,6 @@ l1_reverse_pair_kernel_##NAME(int node0, const int* __restrict__ first, const in
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");                                                    \
     __syncthreads();                                                                                                    \
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");                                                     \
-    unsigned raw[2 * kRowBatch];                                                                                        \
-    load_row_batch(row_column, raw);                                                                                    \
     for (int chunk = 0; chunk < total; chunk += length) {                                                               \
         const int count = min(length, total - chunk);                                                                   \
         if (chunk > 0) {                                                                                                \
@@ -382,6 +388,8 @@ l1_reverse_pair_kernel_##NAME(int node0, const int* __restrict__ first, const in
             const int4 id = s.index[t];                                                                                 \
             const float2* yrow = s.y[t];                                                                                \
             float f[16];                                                                                                \
+            unsigned raw[2 * kRowBatch];                                                                                \
+            load_row_batch(row_column, raw);                                                                            \
             const float4 m = s.misc[t];                                                                                 \
             const float4* coef = table + id.x + k;                                                                      \
             const size_t source_row = static_cast<size_t>(id.y) * NH * kC + k;                                          \
@@ -401,7 +409,6 @@ l1_reverse_pair_kernel_##NAME(int node0, const int* __restrict__ first, const in
         __syncthreads();                                                                                                \
         flush_active_chunk<kGroups, kRecords>(s, count, channel_sums, totals, out, density_coef);                       \
     }                                                                                                                   \
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");                                                        \
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");                                                    \
     __syncthreads();                                                                                                    \
     if (warp == 0)                                                                                                      \

@@ -1,5 +1,6 @@
 """The rules that deal a receiver's edges to blocks and warps (csrc/part_rules.hpp), against measured kernel times."""
 import ctypes
+import re
 import subprocess
 from pathlib import Path
 
@@ -85,3 +86,15 @@ def test_tables_of_a_preparation_that_threw_are_made_by_the_next(tmp_path):
             assert lib.prepare(8, on_basis, -1) == 1
             assert lib.prepare(8, 1 - on_basis, -1) == 1
             assert lib.prepare(7, on_basis, fail) == -1 and lib.prepare(7, on_basis, -1) == 1
+
+
+def test_row_batches_are_taken_in_order():
+    """The layer-1 gradient on channel pairs asks for batch b + 1 of the row adjoints when it takes batch b (csrc/edge_kernels_pairs.cuh):
+    an edge's body takes every batch that is stored, once and in order, and leaves none outstanding."""
+    text = (ROOT / "symmetrix-xl_b200" / "csrc" / "generated" / "structures.h").read_text()
+    for name in ("S1", "S2"):
+        batches = int(re.search(rf"#define SXB_{name}_ROW_BATCHES (\d+)", text).group(1))
+        body = re.search(rf"#define SXB_{name}_L1_REVERSE_EDGE_BODY (.*?[^\\])\n(?!\s)", text, re.S).group(1)
+        stored = re.search(rf"#define SXB_{name}_L1_ADJOINT_ROWS (.*?[^\\])\n(?!\s)", text, re.S).group(1)
+        assert [int(b) for b in re.findall(r"\bROWS\((\d+)\)", body)] == list(range(batches))
+        assert [int(b) for b in re.findall(r"\bSTORE\((\d+)\)", stored)] == list(range(batches))
