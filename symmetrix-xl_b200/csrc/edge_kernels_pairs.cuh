@@ -21,6 +21,7 @@
 #pragma once
 
 #include "edge_kernels.cuh"
+#include "part_rules.hpp"
 
 namespace sxb {
 
@@ -314,10 +315,9 @@ constexpr std::size_t pair_block_bytes(int channels)
 }
 constexpr std::size_t kSharedPerSM = 228 * 1024;
 
-// warps of a block, resident blocks of an SM (what the launch bounds ask for and what the part rule counts with) and columns of
-// tensor memory a block allocates: the SM's 512 columns hold the rows of two receivers (0e+1o) or one
+// warps of a block and columns of tensor memory it allocates: the SM's 512 columns hold the rows of two receivers (0e+1o) or one,
+// the resident blocks that the part rule counts with (part_rules.hpp)
 constexpr int kPairWarpsS1 = 8, kPairWarpsS2 = 12;
-constexpr int kPairBlocksS1 = 2, kPairBlocksS2 = 1;
 constexpr int kPairColumnsS1 = 256, kPairColumnsS2 = 512;
 static_assert(2 * kRowBatch * SXB_S1_ROW_BATCHES <= kPairColumnsS1 && kPairBlocksS1 * kPairColumnsS1 <= 512, "tensor memory, 0e+1o");
 static_assert(2 * kRowBatch * SXB_S2_ROW_BATCHES <= kPairColumnsS2 && kPairBlocksS2 * kPairColumnsS2 <= 512, "tensor memory, 0e+1o+2e");

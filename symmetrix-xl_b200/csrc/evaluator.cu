@@ -1400,12 +1400,11 @@ void Evaluator::run_pipeline(int phases)
             span_end();
             // hidden l > 0 at the common widths: channel pairs with the row adjoints in tensor memory; otherwise one channel per thread
             // with the adjoints in registers (16 rows for hidden 0e).  Both leave records in the reproducible mode.
-            const bool paired = model_.shape_id == 2 || (model_.shape_id == 1 && (C == 128 || C == 64));
+            const bool paired = rules.l1_reverse_paired();
             span_begin("l1_reverse");
             if (paired && fo.edge_forces != nullptr && t0 == 0)   // edges at or beyond the cutoff are not visited
                 SXB_CUDA(cudaMemsetAsync(fo.edge_forces, 0, sizeof(double) * 3 * num_edges_, stream_));
-            const int pair_blocks = model_.shape_id == 2 ? kPairBlocksS2 : kPairBlocksS1;
-            const int reverse_parts = paired ? rules.l1_reverse_pairs(T, pair_blocks) : rules.l1_reverse(T);
+            const int reverse_parts = rules.l1_reverse(T);
             const dim3 reverse_grid(T, reverse_parts);
 #define SXB_PAIR_REVERSE(NAME, WIDTH, ...)                                                                                \
             l1_reverse_pair_kernel_##NAME<WIDTH, ##__VA_ARGS__><<<reverse_grid, 32 * kPairWarps##NAME, pair_dynamic_bytes(WIDTH), stream_>>>(  \

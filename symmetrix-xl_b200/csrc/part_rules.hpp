@@ -29,6 +29,9 @@ inline int edge_parts(long units, double slots, double edges, double overhead, d
     return best;
 }
 
+// Resident blocks of the layer-1 gradient on channel pairs: what its launch bounds ask for, 0e+1o and 0e+1o+2e.
+constexpr int kPairBlocksS1 = 2, kPairBlocksS2 = 1;
+
 struct PartRules {
     int num_sms, channels, shape;      // shape: 0 hidden 0e, 1 0e+1o, 2 0e+1o+2e
     double edges;                      // mean list edges of a receiver
@@ -82,30 +85,29 @@ struct PartRules {
         return parts;
     }
 
-    // Blocks that hold a receiver's row adjoints (the layer-1 gradient on channel pairs), `resident` of them on an SM.
-    int l1_reverse_shared(long receivers, int resident) const
-    {
-        return edge_parts(receivers, 1.0 * num_sms * resident, edges, 8.0, 0.95, 2, 8);
-    }
+    // Layer-1 gradient on channel pairs with the row adjoints in tensor memory (edge_kernels_pairs.cuh) at the common widths of
+    // hidden l > 0, or one channel per thread with the adjoints in registers.
+    bool l1_reverse_paired() const { return shape == 2 || (shape == 1 && (channels == 128 || channels == 64)); }
 
-    // Layer-1 gradient with the row adjoints in tensor memory.  A block of it has eight or twelve warps, a part costs more beside its
-    // edges than with a few warps: no more blocks than fill the chip about twice.  1 / 2 / 4 / 8 parts, 128 channels: 40 receivers
-    // 38 / 25 / 23 / 23, 160: 50 / 44 / 44 / 50, 320: 72 / 66 / 70 / 87, 600: 111 / 109 / 119 / 154, 1,080: 173 / 179 / 204 / 267, 5,000: 699 /
-    // 762 / 904 / 1,308; 64 channels, 40: 23 / 17 / 17 / 19, 320: 44 / 42 / 50 / 68, 1,080: 97 / 105 / 136 / 199; 0e+1o+2e, 40: 56 / 35 / 37 / 38,
-    // 160: 85 / 80 / 83 / 103, 600: 220 / 236 / 275 / 359.
+    // Parts of that gradient: on channel pairs, `resident` blocks of it on an SM.  A block has eight or twelve warps, a part costs more
+    // beside its edges than with a few warps: no more blocks than fill the chip about twice.  1 / 2 / 4 / 8 parts, 128 channels: 40
+    // receivers 38 / 25 / 23 / 23, 160: 50 / 44 / 44 / 50, 320: 72 / 66 / 70 / 87, 600: 111 / 109 / 119 / 154, 1,080: 173 / 179 / 204 /
+    // 267, 5,000: 699 / 762 / 904 / 1,308; 64 channels, 40: 23 / 17 / 17 / 19, 320: 44 / 42 / 50 / 68, 1,080: 97 / 105 / 136 / 199;
+    // 0e+1o+2e, 40: 56 / 35 / 37 / 38, 160: 85 / 80 / 83 / 103, 600: 220 / 236 / 275 / 359.
     int l1_reverse_pairs(long receivers, int resident) const
     {
-        int parts = l1_reverse_shared(receivers, resident);
+        int parts = edge_parts(receivers, 1.0 * num_sms * resident, edges, 8.0, 0.95, 2, 8);
         while (parts > 1 && 1.0 * receivers * parts > 2.2 * num_sms * resident) parts /= 2;
         return parts;
     }
 
-    // Layer-1 gradient with the row adjoints in registers.  Hidden 0e: 128 registers and 26 KB a block, eight blocks of up to two
+    // Either; with the adjoints in registers, hidden 0e: 128 registers and 26 KB a block, eight blocks of up to two
     // warps, four of four.  1 / 2 / 4 / 8 parts, 32 channels (58 edges), 40 receivers: 31 / 21 / 15 / 13, 600: 35 / 33 / 33 / 35,
     // 1,080: 37 / 39 / 45 / 56, 1,500: 60 / 54 / 60 / 72.  0e+1o (widths without a paired kernel): counted with 12 warps; its
     // records at 128 channels, 40: 68 / 39 / 29 / 27, 600: 201 / 177 / 176 / 199, 1,080: 293 / 293 / 308 / 353.
     int l1_reverse(long receivers) const
     {
+        if (l1_reverse_paired()) return l1_reverse_pairs(receivers, shape == 2 ? kPairBlocksS2 : kPairBlocksS1);
         const int resident = shape == 0 ? std::min(8, 16 / block_warps()) : 12 / block_warps();
         return edge_parts(receivers, 1.0 * num_sms * std::max(1, resident), edges, 5.0, 0.95, 2, 8);
     }

@@ -45,21 +45,23 @@ def model_path(pkg, model_dir):
 
 @pytest.fixture(scope="session")
 def part_rule(tmp_path_factory):
-    """rule(kernel, sms, channels, shape, edges, receivers, resident) -> parts, compiled from the library's header."""
+    """rule(kernel, sms, channels, shape, edges, receivers, types=3) -> parts, compiled from the library's header: the calls that the
+    launches make.  "layer0_on_basis" is 1 where layer 0 runs on the radial functions and "l0_moments_reverse" gives its parts."""
     folder = tmp_path_factory.mktemp("part_rules")
     header = ROOT / "symmetrix-xl_b200" / "csrc" / "part_rules.hpp"
+    kernels = {"l0_forward": "receivers", "l1_forward": "receivers", "l1_reverse": "receivers", "l0_reverse": "receivers",
+               "layer0_on_basis": "receivers, types", "l0_moments_reverse": "receivers, types"}
     (folder / "rules.cpp").write_text(
         f'#include "{header}"\n'
-        'extern "C" int rule(int kernel, int sms, int channels, int shape, double edges, long receivers, int resident)\n'
-        "{\n    const sxb::PartRules r{sms, channels, shape, edges};\n"
-        "    return kernel == 0 ? r.l0_forward(receivers) : kernel == 1 ? r.l1_forward(receivers) : kernel == 3 ? r.l0_reverse(receivers)\n"
-        "           : resident ? r.l1_reverse_shared(receivers, resident) : r.l1_reverse(receivers);\n}\n")
+        'extern "C" int rule(int kernel, int sms, int channels, int shape, double edges, long receivers, int types)\n'
+        "{\n    const sxb::PartRules r{sms, channels, shape, edges};\n    switch (kernel) {\n"
+        + "".join(f"    case {i}: return r.{name}({args});\n" for i, (name, args) in enumerate(kernels.items()))
+        + "    }\n    return 0 * types;\n}\n")
     subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-o", str(folder / "rules.so"),
                     str(folder / "rules.cpp")], check=True)
     lib = ctypes.CDLL(str(folder / "rules.so"))
     lib.rule.argtypes = [ctypes.c_int] * 4 + [ctypes.c_double, ctypes.c_long, ctypes.c_int]
-    kernels = ("l0_forward", "l1_forward", "l1_reverse", "l0_reverse")
-    return lambda kernel, *args: lib.rule(kernels.index(kernel), *args)
+    return lambda kernel, *args, types=3: lib.rule(list(kernels).index(kernel), *args, types)
 
 
 def csr_from_positions(positions, cell, cutoff):

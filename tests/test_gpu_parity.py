@@ -804,27 +804,32 @@ def test_layer1_gradient_widths_and_odd_edge_counts(pkg, model_path, channels, o
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("arch,channels,options,copies,parts", [
-    # parts of a receiver in the layer-0 sums, the layer-1 sums, the layer-1 and the layer-0 gradient
-    ("medium", 128, {}, (1, 1, 1), (4, 8, 8, 8)),
-    ("medium", 128, {}, (2, 2, 2), (4, 1, 4, 4)),
-    ("medium", 128, {}, (3, 3, 3), (4, 1, 1, 4)),
-    ("medium", 128, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 4), (4, 1, 2, 1)),
-    ("medium", 128, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 6), (1, 1, 1, 2)),
-    ("medium", 64, {}, (1, 1, 1), (4, 8, 8, 8)),
-    ("medium", 64, {}, (3, 3, 3), (4, 1, 1, 2)),
-    ("medium", 64, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 9), (1, 1, 1, 2)),
-    ("large", 128, {}, (1, 1, 1), (4, 8, 2, 8)),
-    ("large", 128, {}, (3, 3, 2), (4, 1, 1, 2)),
-    ("small", 32, {}, (1, 1, 1), (4, 8, 8, 8)),
-    ("small", 32, {}, (4, 3, 3), (4, 1, 2, 2)),
-    ("small", 32, {}, (6, 5, 4), (1, 1, 1, 1)),
+@pytest.mark.parametrize("arch,channels,options,copies,layer0,parts", [
+    # layer 0 on the folded table: parts of a receiver in the layer-0 sums, the layer-1 sums, the layer-1 and the layer-0 gradient; on
+    # the radial functions, whose sums are never divided: layer-1 sums, layer-1 and layer-0 gradient
+    ("medium", 128, {}, (1, 1, 1), "table", (4, 8, 4, 8)),
+    ("medium", 128, {}, (2, 2, 2), "table", (4, 1, 2, 4)),
+    ("medium", 128, {}, (3, 3, 3), "functions", (1, 1, 3)),
+    ("medium", 128, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 4), "functions", (1, 1, 3)),
+    ("medium", 128, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 6), "functions", (1, 1, 1)),
+    ("medium", 128, {"radial_hidden": (64, 64, 32)}, (3, 3, 3), "table", (4, 1, 1, 4)),
+    ("medium", 128, {"radial_hidden": (64, 64, 32), "a0_scaled": True}, (7, 4, 4), "table", (1, 1, 1, 1)),
+    ("medium", 64, {}, (1, 1, 1), "table", (4, 8, 4, 8)),
+    ("medium", 64, {}, (3, 3, 3), "functions", (1, 1, 3)),
+    ("medium", 64, {"a0_scaled": True, "a1_scaled": True}, (3, 3, 9), "functions", (1, 1, 1)),
+    ("medium", 64, {"radial_hidden": (64, 64, 32)}, (3, 3, 3), "table", (4, 1, 1, 2)),
+    ("medium", 64, {"radial_hidden": (64, 64, 32), "a0_scaled": True}, (7, 4, 4), "table", (1, 1, 1, 1)),
+    ("large", 128, {}, (1, 1, 1), "table", (4, 8, 2, 8)),
+    ("large", 128, {}, (3, 3, 2), "functions", (1, 1, 3)),
+    ("small", 32, {}, (1, 1, 1), "table", (4, 8, 8, 8)),
+    ("small", 32, {}, (4, 3, 3), "table", (4, 1, 2, 2)),
+    ("small", 32, {}, (6, 5, 4), "table", (1, 1, 1, 1)),
 ])
-def test_every_division_of_receivers(pkg, model_path, part_rule, arch, channels, options, copies, parts):
+def test_every_division_of_receivers(pkg, model_path, part_rule, arch, channels, options, copies, layer0, parts):
     """Each build that the part rules can choose, from the most parts to undivided receivers whose 97 list edges (small: 58)
     fill the 64-edge chunks of the layer-1 kernels and the 32-edge ones of layer 0 more than once: periodic copies of a 40-atom
-    cell, atom by atom against the oracle of the cell (bounds of the oracle comparison).  The parts are asserted, so that a
-    changed rule cannot leave a build out unnoticed."""
+    cell, atom by atom against the oracle of the cell (bounds of the oracle comparison).  The parts are asserted by the rules that the
+    launches call, so that a changed rule cannot leave a build out unnoticed."""
     import torch
 
     path = model_path(arch, 37, channels=channels, **options)
@@ -836,10 +841,13 @@ def test_every_division_of_receivers(pkg, model_path, part_rule, arch, channels,
     many = (pos[None] + (grid @ cell)[:, None]).reshape(-1, 3)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     shape = {"small": 0, "medium": 1, "large": 2}[arch]
-    resident = {(1, 128): 3, (1, 64): 4, (2, 128): 1}.get((shape, channels), 0)
-    assert parts == tuple(part_rule(kernel, sms, channels, shape, len(src) / len(pos), len(many), resident if kernel == "l1_reverse" else 0)
-                          for kernel in ("l0_forward", "l1_forward", "l1_reverse", "l0_reverse"))
+    rule = lambda kernel: part_rule(kernel, sms, channels, shape, len(src) / len(pos), len(many))
+    functions = channels in (64, 128) and "radial_hidden" not in options and rule("layer0_on_basis")
+    kernels = ("l1_forward", "l1_reverse", "l0_moments_reverse") if functions else ("l0_forward", "l1_forward", "l1_reverse", "l0_reverse")
+    assert (layer0, parts) == ("functions" if functions else "table", tuple(rule(kernel) for kernel in kernels))
+    calc.evaluator.set_profiling(True)
     out = calc.calculate(many, cell * np.array(copies)[:, None], np.tile(types, len(grid)))
+    assert ("gemm_a0" in {name for name, _ms, _launches in calc.evaluator.profile()}) == bool(functions)
     assert np.abs(out["energies"].reshape(len(grid), -1) - energies).max() <= TOL_E
     assert np.abs(out["forces"].reshape(len(grid), -1, 3) - forces).max() <= TOL_F
 
