@@ -1123,22 +1123,24 @@ void Evaluator::run_pipeline(int phases)
         });
         launch_tc(calls);
     };
-    auto l0_forward = [&](int t0, int T) {
+    // `again`: A0 of a tile made a second time, for the reverse sweep, under names of its own
+    auto l0_forward = [&](int t0, int T, bool again) {
+        const char* const edges_name = again ? "l0_forward_recompute" : "l0_forward";
         if (basis_layer0_) {
             for_moment_slices(t0, T, [&](int begin, int count) {
-                span_begin("l0_forward");
+                span_begin(edges_name);
                 l0_moments_kernel<<<count * n_active, 32, 0, stream_>>>(
                     begin, n_active, first_.ptr, geom_.ptr, active_edges(), basis_pair_types_, grid_,
                     reinterpret_cast<const float4*>(basis_table_.ptr), moments_.ptr, inv0);
                 launches_ += 1;
                 span_end();
-                span_begin("gemm_a0");
+                span_begin(again ? "gemm_a0_recompute" : "gemm_a0");
                 basis_linears(begin, count, t0, false);
                 span_end();
             });
             return;
         }
-        span_begin("l0_forward");
+        span_begin(edges_name);
         const int parts = sum_rules.l0_forward(sum_receivers(T)), warp_grid = blocks_for(static_cast<long>(T) * parts, kWarpsPerBlock);
         const std::size_t part_bytes = parts > 1 ? static_cast<std::size_t>(kWarpsPerBlock) * 16 * C * sizeof(float) : 0;
         if (C == 128)
@@ -1182,7 +1184,7 @@ void Evaluator::run_pipeline(int phases)
         }
         for (int t0 = 0; t0 < R; t0 += tile_cap) {
             const int T = std::min(tile_cap, R - t0);
-            l0_forward(t0, T);
+            l0_forward(t0, T, false);
             span_begin("m0_forward");
             float* m0 = M0_.ptr + t0 * rowH;
             if (model_.shape_id == 0)
@@ -1453,7 +1455,7 @@ void Evaluator::run_pipeline(int phases)
             const int T = std::min(tile_cap, R - t0);
             if (tiled) {
                 // the tile workspace no longer holds this tile's A0: regenerate it
-                l0_forward(t0, T);
+                l0_forward(t0, T, true);
             }
             span_begin("gemm_h1_reverse");
             // M0_adj_il = H1_adj_il W_l^T, then the direct adjoint q + T_element H2_adj on the scalar block

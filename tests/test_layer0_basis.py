@@ -178,10 +178,14 @@ def test_slices_of_the_sums_over_the_functions(pkg, model_path, channels, option
         sliced.evaluator.set_moment_bytes(0)
     sliced.evaluator.set_moment_bytes(receivers * 3 * 16 * 64 * 4)
     sliced.evaluator.set_tile_size(tile)
+    sliced.evaluator.set_profiling(True)
     a = whole.calculate(pos, cell, types)
     b = sliced.calculate(pos, cell, types)
     used = [c.evaluator.execution_plan_report["candidates"][0]["estimated_bytes"] for c in (whole, sliced)]
     assert used[0] - used[1] >= (len(pos) - receivers) * 3 * 16 * 64 * 4
+    names = {name for name, _ms, _launches in sliced.evaluator.profile()}     # A0 made again for the reverse sweep has names of its own
+    again = {"l0_forward_recompute", "gemm_a0_recompute"}
+    assert {"l0_forward", "gemm_a0"} <= names and names & again == (again if tile else set())
     if tile == 0:
         assert np.array_equal(sliced.evaluator.stage("A0"), whole.evaluator.stage("A0"))
     assert np.abs(a["energies"] - b["energies"]).max() <= 1e-6
