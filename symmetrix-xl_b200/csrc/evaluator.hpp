@@ -135,7 +135,10 @@ private:
     // M1 to readout and back in one kernel (node_readout_kernel_*): the model has that form, and the graph is so small that short
     // dependent kernels cost more than the tensor cores gain.  By the receivers of the graph and not of the tile, so that tiles do
     // not change the arithmetic.  Five launches / one, us, 128 channels: 40 receivers 47 / 19, 320: 48 / 19, 1,080: 55 / 31, 5,000: 88 /
-    // 99; 64 channels, 1,080: 60 / 17; hidden 0e at 32 channels, 320: 43 / 15.
+    // 99; 64 channels, 1,080: 60 / 17; hidden 0e at 32 channels, 320: 43 / 15.  With the linears of H1, in which the skip rides: 128
+    // channels, 3,000: 118 / 113, 4,000: 129 / 129; 64 channels, 6,050: 134 / 92, 7,200: 137 / 100; 32 channels, 12,000: 114 / 83,
+    // 15,360: 120 / 94; 0e+1o+2e, 320: 90 / 57, 1,080: 101 / 75, 3,000: 135 / 124, 4,000: 148 / 139.  The line is where 128 channels
+    // break even, the fewest nodes a block has; the others still gain there.
     bool fused_readout_model() const
     {
         const int C = model_.channels;

@@ -146,7 +146,6 @@ def reverse_edges_lines(paths, row_begin, fed):
     out, used, order = [], set(), []
 
     def put(target, a, b):
-        target, a, b = target.replace("[e]", ""), a.replace("[e]", ""), b.replace("[e]", "")
         out[-1] += f" {target} = f2_fma({a}, {b}, {target});" if target in used else f" {target} = f2_mul({a}, {b});"
         used.add(target)
 
@@ -166,19 +165,19 @@ def reverse_edges_lines(paths, row_begin, fed):
             if n2 < n1:
                 for b in range(n2):
                     out.append("     ")
-                    put(f"t[e][{b}]", "R[e]", f"h[e][{l2 * l2 + b}]")
+                    put(f"t[{b}]", "R", f"h[{l2 * l2 + b}]")
                 for a in range(n1):
                     for b in range(n2):
                         if row_begin[p] + a * n2 + b not in fed:
                             continue
                         take(row_begin[p] + a * n2 + b)
-                        put(f"ang[e][{a}]", f"t[e][{b}]", "w")
-                        put(f"v[e][{b}]", f"y[e][{a}]", "w")
+                        put(f"ang[{a}]", f"t[{b}]", "w")
+                        put(f"v[{b}]", f"y[{a}]", "w")
                         out[-1] += " }"
                 for b in range(n2):
                     out.append("     ")
-                    put(f"hadj[e][{l2 * l2 + b}]", "R[e]", f"v[e][{b}]")
-                    put("yw[e]", f"h[e][{l2 * l2 + b}]", f"v[e][{b}]")
+                    put(f"hadj[{l2 * l2 + b}]", "R", f"v[{b}]")
+                    put("yw", f"h[{l2 * l2 + b}]", f"v[{b}]")
             else:
                 for a in range(n1):
                     row = row_begin[p] + a * n2
@@ -190,15 +189,15 @@ def reverse_edges_lines(paths, row_begin, fed):
                         if row + b not in fed:
                             continue
                         take(row + b)
-                        put("v[e][0]", f"h[e][{l2 * l2 + b}]", "w")
-                        put(f"hadj[e][{l2 * l2 + b}]", "t[e][0]", "w")
+                        put("v[0]", f"h[{l2 * l2 + b}]", "w")
+                        put(f"hadj[{l2 * l2 + b}]", "t[0]", "w")
                         out[-1] += " }"
                     out.append("     ")
                     if l1:
-                        put(f"ang[e][{a}]", "R[e]", "v[e][0]")
-                    put("yw[e]", f"y[e][{a}]", "v[e][0]")
+                        put(f"ang[{a}]", "R", "v[0]")
+                    put("yw", f"y[{a}]", "v[0]")
             out.append("     ")
-            put("radial[e]", "dR[e]", "yw[e]")
+            put("radial", "dR", "yw")
             out.append("    }")
         if l1:
             out.append("     " + "".join(f" f[{l1 * l1 + a}] = f2_sum(ang[{a}]);" for a in range(n1)))
